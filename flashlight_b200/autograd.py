@@ -331,13 +331,14 @@ def _linear_bf16(x: Variable, w: Variable, b: Optional[Variable], gelu: bool = F
     xt, wt = x.tensor.contiguous(), w.tensor.contiguous()
     I, O = wt.shape
     rows = xt.numel() // I
+    mode = extension().math_mode  # bf16 products always run on the tensor cores
     fused = None
     if (b is not None or gelu) and LINEAR_FUSED_ON:
-        fused = F.linear_bias_act(xt, wt, b.tensor if b is not None else None, gelu)
+        fused = F.linear_bias_act(xt, wt, b.tensor if b is not None else None, gelu, math_mode=mode)
     if fused is not None:
         y, pre = fused
     else:
-        y = F.matmul(xt, wt, m=rows, n=O, k=I, a_strides=(I, 1), b_strides=(O, 1))
+        y = F.matmul(xt, wt, m=rows, n=O, k=I, a_strides=(I, 1), b_strides=(O, 1), math_mode=mode)
         y = y.reshape(tuple(xt.shape[:-1]) + (O,))
         if b is not None:
             F.channel_bias_add(y, b.tensor, rows, O, 1, out=y)
@@ -350,11 +351,12 @@ def _linear_bf16(x: Variable, w: Variable, b: Optional[Variable], gelu: bool = F
         if gelu:
             gy = F.gelu_backward(pre, gy)
         if inputs[0].isCalcGrad():   # dX (rows, I) = dY (rows, O) @ W^T (O, I)
-            gx = F.matmul(gy, wt, m=rows, n=I, k=O, a_strides=(O, 1), b_strides=(1, O))
+            gx = F.matmul(gy, wt, m=rows, n=I, k=O, a_strides=(O, 1), b_strides=(1, O),
+                          math_mode=mode)
             inputs[0].addGrad(gx.reshape(xt.shape))
         if inputs[1].isCalcGrad():   # dW (I, O) = X^T (I, rows) @ dY (rows, O)
             inputs[1].addGrad(F.matmul(xt, gy, m=I, n=O, k=rows, a_strides=(1, I),
-                                       b_strides=(O, 1)))
+                                       b_strides=(O, 1), math_mode=mode))
         if b is not None and inputs[2].isCalcGrad():
             inputs[2].addGrad(F.channel_sum(gy, rows, O, 1).reshape(b.tensor.shape))
 

@@ -116,7 +116,43 @@ def build_dist(force: bool = False) -> Path:
     return DIST_LIB
 
 
+NATIVE_SRC = CSRC / "py" / "native.cpp"
+NATIVE_LIB = CSRC / "py" / "_native.so"
+
+
+def build_native(force: bool = False) -> Path:
+    """Builds py/_native.so, the host path of the Python mirror (a CPython extension over torch's
+    C++ API and the C ABI; host code only).  Needs libflb200.so, which it links."""
+    import sysconfig
+
+    import torch
+    from torch.utils.cpp_extension import include_paths
+    h = hashlib.sha256(NATIVE_SRC.read_bytes() + torch.__version__.encode())
+    for hdr in sorted(INCLUDE.glob("*.h")):
+        h.update(hdr.read_bytes())
+    stamp_file = OBJ_DIR / "native.stamp"
+    OBJ_DIR.mkdir(exist_ok=True)
+    if (not force and NATIVE_LIB.exists() and stamp_file.exists()
+            and stamp_file.read_text() == h.hexdigest()):
+        return NATIVE_LIB
+    cuda = Path(_nvcc()).resolve().parent.parent
+    includes = [*include_paths(), sysconfig.get_paths()["include"], str(cuda / "include"), str(INCLUDE)]
+    torch_lib = Path(torch.__file__).resolve().parent / "lib"
+    cmd = ["g++", "-O2", "-std=c++17", "-fPIC", "-shared", "-fvisibility=hidden",
+           f"-D_GLIBCXX_USE_CXX11_ABI={int(torch._C._GLIBCXX_USE_CXX11_ABI)}",
+           *[f"-I{d}" for d in includes], str(NATIVE_SRC), "-o", str(NATIVE_LIB),
+           f"-L{torch_lib}", "-ltorch_python", "-ltorch", "-ltorch_cuda", "-ltorch_cpu", "-lc10_cuda",
+           "-lc10", f"-L{cuda / 'lib64'}", "-lcudart", f"-L{CSRC}", "-l:libflb200.so",
+           "-Wl,-rpath,$ORIGIN/.."]
+    res = subprocess.run(cmd, capture_output=True, text=True)
+    if res.returncode != 0:
+        raise RuntimeError(f"building {NATIVE_LIB.name} failed:\n{res.stdout}\n{res.stderr}")
+    stamp_file.write_text(h.hexdigest())
+    return NATIVE_LIB
+
+
 if __name__ == "__main__":
     path = build(force="--force" in sys.argv, verbose="--verbose" in sys.argv)
     print(path)
     print(build_dist(force="--force" in sys.argv))
+    print(build_native(force="--force" in sys.argv))

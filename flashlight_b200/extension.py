@@ -31,6 +31,7 @@ from typing import Optional, Sequence
 import torch
 
 from . import _lib as L
+from ._native import native as N
 
 _DTYPES = {torch.float32: L.F32, torch.float16: L.F16, torch.bfloat16: L.BF16}
 
@@ -69,13 +70,8 @@ def same_layout(a: torch.Tensor, b: torch.Tensor) -> bool:
     return a.shape == b.shape and is_channels_last(a) == is_channels_last(b)
 
 
-def empty_images(shape, like: torch.Tensor, channels_last: bool) -> torch.Tensor:
-    fmt = torch.channels_last if channels_last else torch.contiguous_format
-    return torch.empty(shape, dtype=like.dtype, device=like.device, memory_format=fmt)
-
-
 def stream_handle() -> int:
-    return torch.cuda.current_stream().cuda_stream
+    return torch._C._cuda_getCurrentRawStream(torch.cuda.current_device())
 
 
 _mask_offset = 0
@@ -88,15 +84,12 @@ def bernoulli_mask(shape, keep_prob: float, device, dtype=torch.float32, seed: O
     last call, seeded by torch's CUDA generator seed."""
     global _mask_offset
     out = torch.empty(shape, dtype=dtype, device=device)
-    n = out.numel()
     if seed is None:
         seed = torch.cuda.initial_seed() & ((1 << 64) - 1)
     if offset is None:
         offset = _mask_offset
-        _mask_offset += (n + 3) // 4
-    code = {torch.float32: L.F32, torch.float16: L.F16, torch.bfloat16: L.BF16}[dtype]
-    L.check(L.lib.flb200_bernoulli_mask(ptr(out), n, float(keep_prob), seed, offset, code,
-                                        stream_handle()))
+        _mask_offset += (out.numel() + 3) // 4
+    N.bernoulli_mask(out, keep_prob, seed, offset)
     return out
 
 
@@ -148,8 +141,8 @@ class _ConvLayoutCache:
         self.gy_key = None
         self.c.gy_cl, self.c.gy_cl_bytes, self.c.gy_cl_valid = None, 0, 0
 
-    def ref(self):
-        return C.byref(self.c)
+    def address(self) -> int:
+        return C.addressof(self.c)
 
 
 class AutogradPayload:
@@ -302,18 +295,19 @@ class B200AutogradExtension:
         return L.Conv2dDesc(W, H, Cin, N, kW, kH, Cout, sx, sy, px, py, dx, dy, groups,
                             dtype_code(input), self.math_mode, layout)
 
-    def _conv_cache(self, d, payload, like) -> Optional["_ConvLayoutCache"]:
+    def _conv_cache(self, payload, input, weights, args, y_cl, mode) -> Optional["_ConvLayoutCache"]:
         """The layout cache kept in the payload of one conv2d call site (None when the route
         keeps no channels-last copies, when there is no payload, or when caching is off)."""
         if payload is None or not self.cache_layouts:
             return None
         if isinstance(payload.data, _ConvLayoutCache):
             return payload.data
-        nx = L.lib.flb200_conv2d_cache_bytes(C.byref(d), 0)
-        ng = L.lib.flb200_conv2d_cache_bytes(C.byref(d), 1)
+        if mode == L.MATH_STRICT_F32:  # the fp32 kernels read either layout in place
+            return None
+        nx, ng = N.conv2d_cache_bytes(input, weights, *args, y_cl, mode)
         if nx == 0 and ng == 0:
             return None
-        payload.data = _ConvLayoutCache(nx, ng, like)
+        payload.data = _ConvLayoutCache(nx, ng, input)
         return payload.data
 
     def conv2d(self, input, weights, bias, sx, sy, px, py, dx, dy, groups, payload=None,
@@ -323,213 +317,93 @@ class B200AutogradExtension:
         stats_out: a list that receives (matrix, groups) — the batch-norm statistics of the result,
         taken in the convolution's epilogue (flb200_conv2d_forward_stats), for
         batchnorm(..., conv_stats=...) — where the library can do that; it stays empty otherwise."""
-        d = self._conv_desc(input, weights, sx, sy, px, py, dx, dy, groups, channels_last_out)
-        wo, ho = L.i32(), L.i32()
-        L.check(L.lib.flb200_conv2d_output_dims(C.byref(d), C.byref(wo), C.byref(ho)))
-        out = empty_images((d.N, d.Cout, ho.value, wo.value), input, d.layout != L.LAYOUT_NCHW)
-        if bias is not None and bias.numel() != d.Cout:
-            raise ValueError("conv2d: bias must have one element per output channel")
-        nbytes = L.lib.flb200_conv2d_workspace_bytes(C.byref(d), 0)
-        ws = workspace(nbytes, input)
-        cache = self._conv_cache(d, payload, input)
+        args = (sx, sy, px, py, dx, dy, groups)
+        y_cl = -1 if channels_last_out is None else int(bool(channels_last_out))
+        cache = self._conv_cache(payload, input, weights, args, y_cl, self.math_mode)
         if cache is not None:
             cache.bind_x(input)
-        if stats_out is not None:
-            groups = L.i64()
-            sbytes = L.lib.flb200_conv2d_stats_bytes(C.byref(d), C.byref(groups))
-            if sbytes and all(t is None or t.data_ptr() % 16 == 0
-                              for t in (input, weights, bias, out, ws)):
-                stats = torch.empty(sbytes // 4, dtype=torch.float32, device=input.device)
-                L.check(L.lib.flb200_conv2d_forward_stats(
-                    C.byref(d), ptr(input), ptr(weights), ptr(bias), ptr(out), ptr(stats), sbytes,
-                    ptr(ws), nbytes, cache.ref() if cache is not None else None, stream_handle()))
-                stats_out.append((stats, groups.value))
-                return out
-        L.check(L.lib.flb200_conv2d_forward_cached(
-            C.byref(d), ptr(input), ptr(weights), ptr(bias), ptr(out), ptr(ws), nbytes,
-            cache.ref() if cache is not None else None, stream_handle()))
+        out, stats, stat_groups = N.conv2d(input, weights, bias, *args, y_cl, self.math_mode,
+                                           cache.address() if cache is not None else None,
+                                           stats_out is not None)
+        if stats is not None:
+            stats_out.append((stats, stat_groups))
         return out
 
     def conv2dBackwardData(self, gradOutput, input, weight, sx, sy, px, py, dx, dy, groups,
                            dataGradBenchmark=None, payload=None):
-        grad_in = torch.empty_like(input)
+        args = (sx, sy, px, py, dx, dy, groups)
 
         def run(mode):
-            d = self._conv_desc(input, weight, sx, sy, px, py, dx, dy, groups,
-                                is_channels_last(gradOutput) or is_channels_last(input))
-            d.math_mode = mode
-            nbytes = L.lib.flb200_conv2d_workspace_bytes(C.byref(d), 1)
-            ws = workspace(nbytes, input)
-            cache = self._conv_cache(d, payload, input)
+            cache = self._conv_cache(payload, input, weight, args, self._y_cl(gradOutput, input), mode)
             if cache is not None:
                 cache.bind_gy(gradOutput)
-            L.check(L.lib.flb200_conv2d_backward_data_cached(
-                C.byref(d), ptr(gradOutput), ptr(weight), ptr(grad_in), ptr(ws), nbytes,
-                cache.ref() if cache is not None else None, stream_handle()))
+            return N.conv2d_backward_data(gradOutput, input, weight, *args, mode,
+                                          cache.address() if cache is not None else None)
 
-        self._audited(dataGradBenchmark, run)
-        return grad_in
+        return self._audited(dataGradBenchmark, run)
+
+    @staticmethod
+    def _y_cl(gradOutput, input) -> int:
+        return int(is_channels_last(gradOutput) or is_channels_last(input))
 
     def conv2dBackwardFilterBias(self, gradOutput, input, weights, bias, sx, sy, px, py, dx, dy,
                                  groups, filterBench=None, biasBench=None, autogradPayload=None):
-        grad_w = torch.empty_like(weights)
-        grad_b = torch.empty_like(bias) if bias is not None else None
+        args = (sx, sy, px, py, dx, dy, groups)
 
         def run(mode):
-            d = self._conv_desc(input, weights, sx, sy, px, py, dx, dy, groups,
-                                is_channels_last(gradOutput) or is_channels_last(input))
-            d.math_mode = mode
-            nbytes = L.lib.flb200_conv2d_workspace_bytes(C.byref(d), 2)
-            ws = workspace(nbytes, input)
-            cache = self._conv_cache(d, autogradPayload, input)
+            cache = self._conv_cache(autogradPayload, input, weights, args,
+                                     self._y_cl(gradOutput, input), mode)
             if cache is not None:
                 cache.check_x(input)
                 cache.check_gy(gradOutput)
-            L.check(L.lib.flb200_conv2d_backward_filter_bias_cached(
-                C.byref(d), ptr(gradOutput), ptr(input), ptr(grad_w), ptr(grad_b), ptr(ws), nbytes,
-                cache.ref() if cache is not None else None, stream_handle()))
+            grads = N.conv2d_backward_filter_bias(gradOutput, input, weights, bias, *args, mode,
+                                                  cache.address() if cache is not None else None)
             if cache is not None:
                 cache.release_gy()
+            return grads
 
-        self._audited(filterBench, run)   # the bias gradient is a reduction: nothing to choose
-        return grad_w, grad_b
+        # the bias gradient is a reduction: nothing to choose
+        return self._audited(filterBench, run)
 
     # --------------------------------------------------------------- pool2d
-    @staticmethod
-    def _pool_desc(input, wx, wy, sx, sy, px, py, mode) -> L.Pool2dDesc:
-        W, H, Cc, N = _shape4(input)
-        return L.Pool2dDesc(W, H, Cc, N, wx, wy, sx, sy, px, py, int(mode), dtype_code(input),
-                            L.LAYOUT_NHWC if is_channels_last(input) else L.LAYOUT_NCHW)
-
     def pool2d(self, input, wx, wy, sx, sy, px, py, mode, payload=None):
-        d = self._pool_desc(input, wx, wy, sx, sy, px, py, mode)
-        wo, ho = L.i32(), L.i32()
-        L.check(L.lib.flb200_pool2d_output_dims(C.byref(d), C.byref(wo), C.byref(ho)))
-        out = empty_images((d.N, d.C, ho.value, wo.value), input, d.layout == L.LAYOUT_NHWC)
-        argmax = None
-        if payload is not None and int(mode) == L.POOL_MAX:
-            argmax = torch.empty_like(out, dtype=torch.uint8)
+        out, argmax = N.pool2d(input, wx, wy, sx, sy, px, py, int(mode), payload is not None)
+        if argmax is not None:
             payload.data = _PoolPayload(argmax)
-        L.check(L.lib.flb200_pool2d_forward(C.byref(d), ptr(input), ptr(out), ptr(argmax),
-                                            stream_handle()))
         return out
 
     def pool2dBackward(self, gradOutput, input, poolOutput, wx, wy, sx, sy, px, py, mode,
                        payload=None):
-        d = self._pool_desc(input, wx, wy, sx, sy, px, py, mode)
         argmax = payload.data.argmax if payload is not None and payload.data is not None else None
-        grad_in = torch.empty_like(input)
-        L.check(L.lib.flb200_pool2d_backward(C.byref(d), ptr(gradOutput), ptr(input), ptr(argmax),
-                                             ptr(grad_in), stream_handle()))
-        return grad_in
+        return N.pool2d_backward(gradOutput, input, argmax, wx, wy, sx, sy, px, py, int(mode))
 
     # ------------------------------------------------------------ batchnorm
-    @staticmethod
-    def _bn_desc(input, axes: Sequence[int]) -> L.BatchnormDesc:
-        if is_channels_last(input):
-            # stored [N][H][W][C]: statistics per channel are column sums of a [pixels][C] matrix
-            if list(axes) != [2]:
-                raise ValueError("batchnorm: a channels-last tensor is normalised over fl axis 2 only")
-            n, c, h, w = input.shape
-            return L.BatchnormDesc(n * h * w, c, 1, dtype_code(input))
-        fl_shape = tuple(reversed(input.shape))
-        shape = (L.i64 * len(fl_shape))(*fl_shape)
-        ax = (L.i32 * len(axes))(*axes)
-        d = L.BatchnormDesc()
-        L.check(L.lib.flb200_batchnorm_geometry(shape, len(fl_shape), ax, len(axes), C.byref(d)))
-        d.dtype = dtype_code(input)
-        return d
-
     def batchnorm(self, input, weight, bias, runningMean, runningVar, axes, train, momentum,
                   epsilon, payload=None, relu=False, conv_stats=None):
         """Returns (output, saveMean, saveVar).  saveVar holds 1/sqrt(var + eps).
         runningMean / runningVar are updated in place when given.  relu=True returns
         relu(batchnorm(x)) from the same two passes (pair it with batchnormReluBackward)."""
-        d = self._bn_desc(input, axes)
-        for t in (weight, bias, runningMean, runningVar):
-            if t is not None and t.dtype != torch.float32:
-                raise ValueError("fl::batchnorm: non-input tensors must be of type f32")
-        if weight is not None and weight.numel() != d.channels:
-            raise ValueError("[BatchNorm] Invalid shape for weight.")
-        if bias is not None and bias.numel() != d.channels:
-            raise ValueError("[BatchNorm] Invalid shape for bias.")
-        out = torch.empty_like(input)
-        save_mean = save_var = None
-        if train:
-            save_mean = torch.empty(d.channels, dtype=torch.float32, device=input.device)
-            save_var = torch.empty(d.channels, dtype=torch.float32, device=input.device)
-        nbytes = L.lib.flb200_batchnorm_workspace_bytes(C.byref(d))
-        ws = workspace(nbytes, input)
-        if conv_stats is not None and train:
-            # statistics from what the producing convolution took: no pass over x for them
-            stats, groups = conv_stats
-            nbytes = L.lib.flb200_batchnorm_from_stats_workspace_bytes(C.byref(d), groups)
-            ws = workspace(nbytes, input)
-            L.check(L.lib.flb200_batchnorm_forward_from_stats(
-                C.byref(d), ptr(input), None, 1 if relu else 0, ptr(stats), groups, ptr(weight),
-                ptr(bias), ptr(runningMean), ptr(runningVar), ptr(save_mean), ptr(save_var),
-                float(momentum), float(epsilon), ptr(out), None, ptr(ws), nbytes, stream_handle()))
-            return out, save_mean, save_var
-        forward = L.lib.flb200_batchnorm_relu_forward if relu else L.lib.flb200_batchnorm_forward
-        L.check(forward(
-            C.byref(d), ptr(input), ptr(weight), ptr(bias), ptr(runningMean), ptr(runningVar),
-            ptr(save_mean), ptr(save_var), 1 if train else 0, float(momentum), float(epsilon),
-            ptr(out), ptr(ws), nbytes, stream_handle()))
-        return out, save_mean, save_var
+        stats, groups = conv_stats if conv_stats is not None else (None, 0)
+        return N.batchnorm(input, weight, bias, runningMean, runningVar, axes, train, momentum, epsilon,
+                           relu, stats, groups)
 
     def batchnormBackward(self, gradOutput, saveMean, saveVar, input, weight, axes, train, epsilon,
                           payload=None):
         if not train:
             # cudnn/BatchNorm.cpp:196-199
             raise RuntimeError("can't compute batchnorm grad when train was not specified")
-        d = self._bn_desc(input, axes)
-        grad_in = torch.empty_like(input)
-        grad_w = torch.empty(d.channels, dtype=torch.float32, device=input.device)
-        grad_b = torch.empty(d.channels, dtype=torch.float32, device=input.device)
-        nbytes = L.lib.flb200_batchnorm_workspace_bytes(C.byref(d))
-        ws = workspace(nbytes, input)
-        L.check(L.lib.flb200_batchnorm_backward(
-            C.byref(d), ptr(gradOutput), ptr(input), ptr(weight), ptr(saveMean), ptr(saveVar),
-            ptr(grad_in), ptr(grad_w), ptr(grad_b), ptr(ws), nbytes, stream_handle()))
-        return grad_in, grad_w, grad_b
+        return N.batchnorm_backward(gradOutput, saveMean, saveVar, input, weight, None, axes, False)
 
     def batchnormAddReluSupported(self, input, addend, axes) -> bool:
-        d = self._bn_desc(input, axes)
-        shape_ok = d.inner > 1 or (is_channels_last(input) and d.channels % 8 == 0)
-        return (input.dtype == torch.float32 and shape_ok and same_layout(input, addend)
-                and addend.dtype == input.dtype and is_dense(input)
-                and input.data_ptr() % 16 == 0 and addend.data_ptr() % 16 == 0)
+        return N.batchnorm_add_relu_supported(input, addend, axes)
 
     def batchnormAddRelu(self, input, addend, weight, bias, runningMean, runningVar, axes, train,
                          momentum, epsilon, payload=None, conv_stats=None):
         """relu(batchnorm(input) + addend) with the predicate's bit mask: returns
         (output, mask, saveMean, saveVar).  Check batchnormAddReluSupported first."""
-        d = self._bn_desc(input, axes)
-        out = torch.empty_like(input)
-        # elements per mask byte: 8 consecutive channels of a pixel for channels-last tensors
-        group = 8 if d.inner % 8 == 0 or d.inner == 1 else (4 if d.inner % 4 == 0 else 1)
-        mask = torch.empty((input.numel() + group - 1) // group, dtype=torch.uint8,
-                           device=input.device)
-        save_mean = save_var = None
-        if train:
-            save_mean = torch.empty(d.channels, dtype=torch.float32, device=input.device)
-            save_var = torch.empty(d.channels, dtype=torch.float32, device=input.device)
-        nbytes = L.lib.flb200_batchnorm_workspace_bytes(C.byref(d))
-        ws = workspace(nbytes, input)
-        if conv_stats is not None and train:
-            stats, groups = conv_stats
-            nbytes = L.lib.flb200_batchnorm_from_stats_workspace_bytes(C.byref(d), groups)
-            ws = workspace(nbytes, input)
-            L.check(L.lib.flb200_batchnorm_forward_from_stats(
-                C.byref(d), ptr(input), ptr(addend), 1, ptr(stats), groups, ptr(weight), ptr(bias),
-                ptr(runningMean), ptr(runningVar), ptr(save_mean), ptr(save_var), float(momentum),
-                float(epsilon), ptr(out), ptr(mask), ptr(ws), nbytes, stream_handle()))
-            return out, mask, save_mean, save_var
-        L.check(L.lib.flb200_batchnorm_add_relu_forward(
-            C.byref(d), ptr(input), ptr(addend), ptr(weight), ptr(bias), ptr(runningMean),
-            ptr(runningVar), ptr(save_mean), ptr(save_var), 1 if train else 0, float(momentum),
-            float(epsilon), ptr(out), ptr(mask), ptr(ws), nbytes, stream_handle()))
-        return out, mask, save_mean, save_var
+        stats, groups = conv_stats if conv_stats is not None else (None, 0)
+        return N.batchnorm_add_relu(input, addend, weight, bias, runningMean, runningVar, axes, train,
+                                    momentum, epsilon, stats, groups)
 
     def batchnormAddReluBackward(self, mask, gradA, gradB, saveMean, saveVar, input, weight, axes,
                                  train, epsilon, payload=None):
@@ -537,18 +411,7 @@ class B200AutogradExtension:
         gradSum = mask ? gradA + gradB : 0 is the addend's gradient (gradB may be None)."""
         if not train:
             raise RuntimeError("can't compute batchnorm grad when train was not specified")
-        d = self._bn_desc(input, axes)
-        grad_sum = torch.empty_like(input)
-        grad_in = torch.empty_like(input)
-        grad_w = torch.empty(d.channels, dtype=torch.float32, device=input.device)
-        grad_b = torch.empty(d.channels, dtype=torch.float32, device=input.device)
-        nbytes = L.lib.flb200_batchnorm_workspace_bytes(C.byref(d))
-        ws = workspace(nbytes, input)
-        L.check(L.lib.flb200_batchnorm_add_relu_backward(
-            C.byref(d), ptr(mask), ptr(gradA), ptr(gradB), ptr(input), ptr(weight), ptr(saveMean),
-            ptr(saveVar), ptr(grad_sum), ptr(grad_in), ptr(grad_w), ptr(grad_b), ptr(ws), nbytes,
-            stream_handle()))
-        return grad_sum, grad_in, grad_w, grad_b
+        return N.batchnorm_add_relu_backward(mask, gradA, gradB, saveMean, saveVar, input, weight, axes)
 
     def batchnormReluBackward(self, gradOutput, saveMean, saveVar, input, weight, bias, axes, train,
                               epsilon, payload=None):
@@ -556,16 +419,7 @@ class B200AutogradExtension:
         is rebuilt from the input, so no output tensor or mask is needed."""
         if not train:
             raise RuntimeError("can't compute batchnorm grad when train was not specified")
-        d = self._bn_desc(input, axes)
-        grad_in = torch.empty_like(input)
-        grad_w = torch.empty(d.channels, dtype=torch.float32, device=input.device)
-        grad_b = torch.empty(d.channels, dtype=torch.float32, device=input.device)
-        nbytes = L.lib.flb200_batchnorm_workspace_bytes(C.byref(d))
-        ws = workspace(nbytes, input)
-        L.check(L.lib.flb200_batchnorm_relu_backward(
-            C.byref(d), ptr(gradOutput), ptr(input), ptr(weight), ptr(bias), ptr(saveMean),
-            ptr(saveVar), ptr(grad_in), ptr(grad_w), ptr(grad_b), ptr(ws), nbytes, stream_handle()))
-        return grad_in, grad_w, grad_b
+        return N.batchnorm_backward(gradOutput, saveMean, saveVar, input, weight, bias, axes, True)
 
     # ------------------------------------------------------------------ rnn
     def _rnn_desc(self, input, hiddenSize, numLayers, mode, bidirectional) -> L.RnnDesc:
