@@ -156,9 +156,9 @@ attention_backward_kernel(const __grid_constant__ CUtensorMap map_q,
   const uint64_t dDO_mn = umma_desc(smem_u32(sDO), 8192, 1024, 2);   // one box of 64 d
   const uint64_t dQ_mn = umma_desc(smem_u32(sQ), 8192, 1024, 2);
   const uint64_t dK_mn = umma_desc(smem_u32(sK), 8192, 1024, 2);
-  const uint32_t id_s = umma_idesc_bf16(128, 0, 0);   // S, dP
-  const uint32_t id_t = umma_idesc_bf16(64, 1, 1);    // dV, dK: both operands MN-major
-  const uint32_t id_q = umma_idesc_bf16(64, 0, 1);    // dQ: dS K-major, K_j MN-major
+  const uint32_t id_s = umma_idesc_f16(kOperandBf16, 128, 0, 0);   // S, dP
+  const uint32_t id_t = umma_idesc_f16(kOperandBf16, 64, 1, 1);    // dV, dK: both operands MN-major
+  const uint32_t id_q = umma_idesc_f16(kOperandBf16, 64, 0, 1);    // dQ: dS K-major, K_j MN-major
 
   if (issuer) {
     mbar_expect_tx(bar_kv, 2 * kTile);
@@ -189,11 +189,11 @@ attention_backward_kernel(const __grid_constant__ CUtensorMap map_q,
       tc_fence_after();
 #pragma unroll
       for (int kk = 0; kk < 4; ++kk)  // K = 64 d in steps of 16
-        umma_bf16(tmem, umma_desc_advance(dQ_k, kk * 32), umma_desc_advance(dK_k, kk * 32), id_s,
+        umma_f16(tmem, umma_desc_advance(dQ_k, kk * 32), umma_desc_advance(dK_k, kk * 32), id_s,
                   kk > 0);
 #pragma unroll
       for (int kk = 0; kk < 4; ++kk)
-        umma_bf16(tmem + 128, umma_desc_advance(dDO_k, kk * 32), umma_desc_advance(dV_k, kk * 32),
+        umma_f16(tmem + 128, umma_desc_advance(dDO_k, kk * 32), umma_desc_advance(dV_k, kk * 32),
                   id_s, kk > 0);
       umma_commit(bar_s);
     }
@@ -238,14 +238,14 @@ attention_backward_kernel(const __grid_constant__ CUtensorMap map_q,
       tc_fence_after();
 #pragma unroll
       for (int kk = 0; kk < 8; ++kk) {  // K = 128 query rows in steps of 16
-        umma_bf16(tmem + 256, umma_desc_advance(dP_mn, kk * 2048),
+        umma_f16(tmem + 256, umma_desc_advance(dP_mn, kk * 2048),
                   umma_desc_advance(dDO_mn, kk * 2048), id_t, (it > 0 || kk > 0) ? 1u : 0u);
-        umma_bf16(tmem + 320, umma_desc_advance(dDS_mn, kk * 2048),
+        umma_f16(tmem + 320, umma_desc_advance(dDS_mn, kk * 2048),
                   umma_desc_advance(dQ_mn, kk * 2048), id_t, (it > 0 || kk > 0) ? 1u : 0u);
       }
 #pragma unroll
       for (int kk = 0; kk < 8; ++kk)  // K = 128 keys: two 64-key halves of dS, 16 key rows of K_j
-        umma_bf16(tmem + 384, umma_desc_advance(dDS_k, (kk >> 2) * kTile + (kk & 3) * 32),
+        umma_f16(tmem + 384, umma_desc_advance(dDS_k, (kk >> 2) * kTile + (kk & 3) * 32),
                   umma_desc_advance(dK_mn, kk * 2048), id_q, kk > 0);
       umma_commit(bar_o);
     }

@@ -139,6 +139,10 @@ int map3d(CUtensorMap* m, const float* base, long long inner, long long mid, lon
   const uint32_t box[3] = {32, (uint32_t)box_mid, 1};
   return tc::make_tensor_map(m, base, 3, dims, strides, box, mn_major);
 }
+tc::Launch gemm_plan(long long M, long long N, long long k_iters, bool a_mn, bool b_mn, bool split_k,
+                     long long Z = 1) {
+  return tc::plan_launch(M, N, k_iters, Z, a_mn, b_mn, tc::kOperandTf32, split_k);
+}
 tc::OperandPlan plan_k_major(int rank) {  // dims [K, rows, ...]
   tc::OperandPlan p{};
   p.rank = rank; p.mn_major = 0; p.mn_dim = 1; p.k_dim = 0; p.k2_dim = -1; p.z_dim = -1;
@@ -214,28 +218,32 @@ dim3 gather_grid(long long ld, int rows) {
 size_t tc_conv_workspace_bytes(const ConvGeo& g, int which) {
   if (g.groups != 1) return 0;
   if (cl_1x1(g)) {
-    if (which == 0) return 0;
-    if (which == 1) return up256((size_t)g.C * g.Cout * 4);
+    const long long M = (long long)g.N * g.HW;
+    if (which == 0)
+      return gemm_plan(M, g.Cout, (g.C + tc::kBK - 1) / tc::kBK, false, false, true).workspace_bytes;
+    if (which == 1)
+      return up256((size_t)g.C * g.Cout * 4) +
+             gemm_plan(M, g.C, (g.Cout + tc::kBK - 1) / tc::kBK, false, false, true).workspace_bytes;
     return patch_conv_supported(g) ? patch_conv_workspace_bytes(g, 2) : 0;
   }
   if (direct_1x1(g)) {
     if (which != 2) return 0;
     const long long k_iters = (long long)g.N * ((g.HW + tc::kBK - 1) / tc::kBK);
-    return tc::plan_launch(g.Cout, g.C, k_iters, 1).workspace_bytes;
+    return gemm_plan(g.Cout, g.C, k_iters, false, false, true).workspace_bytes;
   }
   if (patch_conv_supported(g)) return patch_conv_workspace_bytes(g, which);
   if (which != 1 && window_conv_supported(g)) return window_conv_workspace_bytes(g, which);
   const GeneralSizes s = general_sizes(g);
   if (which == 0) {
     return up256((size_t)s.kc * s.ld_out * 4) + up256((size_t)g.Cout * s.kp * 4) +
-           tc::plan_launch(s.ld_out, g.Cout, (s.kc + tc::kBK - 1) / tc::kBK, 1).workspace_bytes;
+           gemm_plan(s.ld_out, g.Cout, (s.kc + tc::kBK - 1) / tc::kBK, true, false, true).workspace_bytes;
   }
   if (which == 1) {
     return up256((size_t)s.k2 * s.ld_in * 4) + up256((size_t)g.C * s.k2p * 4) +
-           tc::plan_launch(s.ld_in, g.C, (s.k2 + tc::kBK - 1) / tc::kBK, 1).workspace_bytes;
+           gemm_plan(s.ld_in, g.C, (s.k2 + tc::kBK - 1) / tc::kBK, true, false, true).workspace_bytes;
   }
   return up256((size_t)s.kc * s.ld_out * 4) + up256((size_t)g.Cout * s.ld_out * 4) +
-         tc::plan_launch(g.Cout, s.kc, (s.ld_out + tc::kBK - 1) / tc::kBK, 1).workspace_bytes;
+         gemm_plan(g.Cout, s.kc, (s.ld_out + tc::kBK - 1) / tc::kBK, false, false, true).workspace_bytes;
 }
 
 size_t tc_conv_cache_bytes(const ConvGeo& g, int which) {
@@ -248,7 +256,8 @@ size_t tc_conv_cache_bytes(const ConvGeo& g, int which) {
 bool tc_conv_supported(const ConvGeo& g, int which, size_t workspace_bytes) {
   if (!flb200_has_tensor_core_path()) return false;
   if (g.groups != 1) return false;
-  if (cl_1x1(g) && which != 2) return workspace_bytes >= tc_conv_workspace_bytes(g, which);
+  if (cl_1x1(g) && which != 2)  // (more scratch than the transposed filter: split-K only)
+    return workspace_bytes >= (which == 1 ? up256((size_t)g.C * g.Cout * 4) : 0);
   // the other channels-last shapes run on the patch / row-window routes or not at all
   if ((g.x_cl || g.y_cl) && !patch_conv_supported(g) && !(which != 1 && window_conv_supported(g)))
     return false;
@@ -278,18 +287,16 @@ int tc_conv_forward(const ConvGeo& g, const float* x, const float* w, const floa
   ep.out = y;
   ep.alpha = 1.f;
   ep.bias_n = bias;
-  const int bn = tc::pick_bn(g.Cout);
   if (cl_1x1(g)) {
     const long long M = (long long)g.N * g.HW, k_iters = (g.C + tc::kBK - 1) / tc::kBK;
+    const tc::Launch L = gemm_plan(M, g.Cout, k_iters, false, false, !stats);
     if (int rc = map2d(&ma, x, g.C, M, g.C, tc::kBM, false)) return rc;
-    if (int rc = map2d(&mb, w, g.C, g.Cout, g.C, tc::b_box_rows(M, g.Cout, k_iters, false, false),
-                       false))
-      return rc;
+    if (int rc = map2d(&mb, w, g.C, g.Cout, g.C, L.b_box_rows(), false)) return rc;
     ep.m_stride = g.Cout;
     ep.n_stride = 1;
     ep.stats = stats ? stats->matrix : nullptr;
-    return tc::run(ma, mb, plan_k_major(2), plan_k_major(2), ep, M, g.Cout, k_iters, 1, nullptr, 0,
-                   st);
+    return tc::run(ma, mb, plan_k_major(2), plan_k_major(2), ep, M, g.Cout, k_iters, 1, L, ws,
+                   ws_bytes, st);
   }
   if (stats && tc_conv_stats_groups(g) == 0)
     return fail(FLB200_UNSUPPORTED, "conv2d_forward: this route takes no output statistics");
@@ -297,14 +304,14 @@ int tc_conv_forward(const ConvGeo& g, const float* x, const float* w, const floa
     if (int rc = map3d(&ma, x, g.HW, g.C, g.N, g.HW, (long long)g.C * g.HW, 32, true)) return rc;
     // a K-major B tile is one box of all the tile's rows, or of half of them on CTA pairs
     const long long k_iters = (g.C + tc::kBK - 1) / tc::kBK;
-    if (int rc = map2d(&mb, w, g.C, g.Cout, g.C, tc::b_box_rows(g.HW, g.Cout, k_iters, true, false), false)) return rc;
+    const tc::Launch L = gemm_plan(g.HW, g.Cout, k_iters, true, false, false, g.N);
+    if (int rc = map2d(&mb, w, g.C, g.Cout, g.C, L.b_box_rows(), false)) return rc;
     tc::OperandPlan pa = plan_mn_major(3), pb = plan_k_major(2);
     pa.z_dim = 2;
     ep.m_stride = 1;
     ep.n_stride = g.HW;
     ep.z_stride = (long long)g.Cout * g.HW;
-    return tc::run(ma, mb, pa, pb, ep, g.HW, g.Cout, (g.C + tc::kBK - 1) / tc::kBK, g.N, nullptr, 0,
-                   st);
+    return tc::run(ma, mb, pa, pb, ep, g.HW, g.Cout, k_iters, g.N, L, nullptr, 0, st);
   }
   if (patch_conv_supported(g))
     return patch_conv_forward(g, x, w, bias, y, ws, ws_bytes, st, cache, stats);
@@ -326,14 +333,16 @@ int tc_conv_forward(const ConvGeo& g, const float* x, const float* w, const floa
     wsrc = wp;
   }
   if (int rc = map2d(&ma, col, s.ld_out, s.kc, s.ld_out, 32, true)) return rc;
-  if (int rc = map2d(&mb, wsrc, s.kc, g.Cout, s.kp, tc::b_box_rows(s.ld_out, g.Cout, (s.kc + tc::kBK - 1) / tc::kBK, true, false), false)) return rc;
+  const long long k_iters = (s.kc + tc::kBK - 1) / tc::kBK;
+  const tc::Launch L = gemm_plan(s.ld_out, g.Cout, k_iters, true, false, true);
+  if (int rc = map2d(&mb, wsrc, s.kc, g.Cout, s.kp, L.b_box_rows(), false)) return rc;
   ep.m_div = s.hwp_out;
   ep.m_valid = g.HoWo;
   ep.m_outer = (long long)g.Cout * g.HoWo;
   ep.m_stride = 1;
   ep.n_stride = g.HoWo;
-  return tc::run(ma, mb, plan_mn_major(2), plan_k_major(2), ep, s.ld_out, g.Cout,
-                 (s.kc + tc::kBK - 1) / tc::kBK, 1, base + off, ws_bytes - off, st);
+  return tc::run(ma, mb, plan_mn_major(2), plan_k_major(2), ep, s.ld_out, g.Cout, k_iters, 1, L,
+                 base + off, ws_bytes - off, st);
 }
 
 int tc_conv_backward_data(const ConvGeo& g, const float* gy, const float* w, float* gx, void* ws,
@@ -343,20 +352,20 @@ int tc_conv_backward_data(const ConvGeo& g, const float* gy, const float* w, flo
   tc::EpiloguePlan ep{};
   ep.out = gx;
   ep.alpha = 1.f;
-  const int bn = tc::pick_bn(g.C);
   if (cl_1x1(g)) {
     const long long M = (long long)g.N * g.HW, k_iters = (g.Cout + tc::kBK - 1) / tc::kBK;
+    const tc::Launch L = gemm_plan(M, g.C, k_iters, false, false, true);
     float* wt = static_cast<float*>(ws);
+    const size_t wt_bytes = up256((size_t)g.C * g.Cout * 4);
     dim3 tgrid((unsigned)((g.C + 31) / 32), (unsigned)((g.Cout + 31) / 32));
     transpose_1x1_filter_kernel<<<tgrid, 256, 0, st>>>(w, wt, g.Cout, g.C);
     FLB200_AFTER_LAUNCH("transpose_1x1_filter");
     if (int rc = map2d(&ma, gy, g.Cout, M, g.Cout, tc::kBM, false)) return rc;
-    if (int rc = map2d(&mb, wt, g.Cout, g.C, g.Cout, tc::b_box_rows(M, g.C, k_iters, false, false),
-                       false))
-      return rc;
+    if (int rc = map2d(&mb, wt, g.Cout, g.C, g.Cout, L.b_box_rows(), false)) return rc;
     ep.m_stride = g.C;
     ep.n_stride = 1;
-    return tc::run(ma, mb, plan_k_major(2), plan_k_major(2), ep, M, g.C, k_iters, 1, nullptr, 0, st);
+    return tc::run(ma, mb, plan_k_major(2), plan_k_major(2), ep, M, g.C, k_iters, 1, L,
+                   static_cast<char*>(ws) + wt_bytes, ws_bytes - wt_bytes, st);
   }
   if (direct_1x1(g)) {
     if (int rc = map3d(&ma, gy, g.HW, g.Cout, g.N, g.HW, (long long)g.Cout * g.HW, 32, true))
@@ -364,10 +373,12 @@ int tc_conv_backward_data(const ConvGeo& g, const float* gy, const float* w, flo
     // B(k = co, n = ci) = w[co][ci]: the n index is contiguous.  With a multiple of 32 input
     // channels the map splits ci into (32, group) and the whole B tile is one copy.
     tc::OperandPlan pa = plan_mn_major(3), pb = plan_mn_major(2);
+    const long long k_iters = (g.Cout + tc::kBK - 1) / tc::kBK;
+    const tc::Launch L = gemm_plan(g.HW, g.C, k_iters, true, true, false, g.N);
     if (g.C % 32 == 0) {
       const uint64_t dims[3] = {32, (uint64_t)g.Cout, (uint64_t)(g.C / 32)};
       const uint64_t strides[2] = {(uint64_t)g.C * 4, 128};
-      const uint32_t box[3] = {32, 32, (uint32_t)(bn / 32)};
+      const uint32_t box[3] = {32, 32, (uint32_t)(L.bn / 32)};
       if (int rc = tc::make_tensor_map(&mb, w, 3, dims, strides, box, tc::kMapMnMajor)) return rc;
       pb.rank = 3; pb.mn_dim = 2; pb.k_dim = 1; pb.mn_grouped = 1;
     } else if (int rc = map2d(&mb, w, g.C, g.Cout, g.C, 32, true)) {
@@ -377,8 +388,7 @@ int tc_conv_backward_data(const ConvGeo& g, const float* gy, const float* w, flo
     ep.m_stride = 1;
     ep.n_stride = g.HW;
     ep.z_stride = (long long)g.C * g.HW;
-    return tc::run(ma, mb, pa, pb, ep, g.HW, g.C, (g.Cout + tc::kBK - 1) / tc::kBK, g.N, nullptr, 0,
-                   st);
+    return tc::run(ma, mb, pa, pb, ep, g.HW, g.C, k_iters, g.N, L, nullptr, 0, st);
   }
   if (patch_conv_supported(g)) return patch_conv_backward_data(g, gy, w, gx, ws, ws_bytes, st, cache);
   const GeneralSizes s = general_sizes(g);
@@ -392,14 +402,16 @@ int tc_conv_backward_data(const ConvGeo& g, const float* gy, const float* w, flo
   transpose_filter_kernel<<<grid_for((long long)g.C * s.k2p, 256), 256, 0, st>>>(w, wt, g, s.k2p);
   FLB200_AFTER_LAUNCH("transpose_filter");
   if (int rc = map2d(&ma, col, s.ld_in, s.k2, s.ld_in, 32, true)) return rc;
-  if (int rc = map2d(&mb, wt, s.k2, g.C, s.k2p, tc::b_box_rows(s.ld_in, g.C, (s.k2 + tc::kBK - 1) / tc::kBK, true, false), false)) return rc;
+  const long long k_iters = (s.k2 + tc::kBK - 1) / tc::kBK;
+  const tc::Launch L = gemm_plan(s.ld_in, g.C, k_iters, true, false, true);
+  if (int rc = map2d(&mb, wt, s.k2, g.C, s.k2p, L.b_box_rows(), false)) return rc;
   ep.m_div = s.hwp_in;
   ep.m_valid = g.HW;
   ep.m_outer = (long long)g.C * g.HW;
   ep.m_stride = 1;
   ep.n_stride = g.HW;
-  return tc::run(ma, mb, plan_mn_major(2), plan_k_major(2), ep, s.ld_in, g.C,
-                 (s.k2 + tc::kBK - 1) / tc::kBK, 1, base + off, ws_bytes - off, st);
+  return tc::run(ma, mb, plan_mn_major(2), plan_k_major(2), ep, s.ld_in, g.C, k_iters, 1, L,
+                 base + off, ws_bytes - off, st);
 }
 
 int tc_conv_backward_filter(const ConvGeo& g, const float* gy, const float* x, float* gw, void* ws,
@@ -411,23 +423,24 @@ int tc_conv_backward_filter(const ConvGeo& g, const float* gy, const float* x, f
   ep.alpha = 1.f;
   ep.n_stride = 1;
   if (direct_1x1(g)) {
-    const int bn = tc::pick_bn(g.C);
     const int k_inner = (g.HW + tc::kBK - 1) / tc::kBK;
     if (int rc = map3d(&ma, gy, g.HW, g.Cout, g.N, g.HW, (long long)g.Cout * g.HW, tc::kBM, false))
       return rc;
-    if (int rc = map3d(&mb, x, g.HW, g.C, g.N, g.HW, (long long)g.C * g.HW, tc::b_box_rows(g.Cout, g.C, (long long)g.N * k_inner, false, false), false)) return rc;
+    const tc::Launch L = gemm_plan(g.Cout, g.C, (long long)g.N * k_inner, false, false, true);
+    if (int rc = map3d(&mb, x, g.HW, g.C, g.N, g.HW, (long long)g.C * g.HW, L.b_box_rows(), false))
+      return rc;
     tc::OperandPlan pa = plan_k_major(3), pb = plan_k_major(3);
     pa.k2_dim = pb.k2_dim = 2;
     pa.k2_scale = pb.k2_scale = 1;
     pa.k_inner = pb.k_inner = k_inner;
     ep.m_stride = g.C;
-    return tc::run(ma, mb, pa, pb, ep, g.Cout, g.C, (long long)g.N * k_inner, 1, ws, ws_bytes, st);
+    return tc::run(ma, mb, pa, pb, ep, g.Cout, g.C, (long long)g.N * k_inner, 1, L, ws, ws_bytes,
+                   st);
   }
   if (patch_conv_supported(g)) return patch_conv_backward_filter(g, gy, x, gw, ws, ws_bytes, st, cache);
   if (window_conv_supported(g))
     return window_conv_backward_filter(g, gy, x, gw, ws, ws_bytes, st, cache);
   const GeneralSizes s = general_sizes(g);
-  const int bn = tc::pick_bn(s.kc);
   char* base = static_cast<char*>(ws);
   float* col = reinterpret_cast<float*>(base);
   size_t off = up256((size_t)s.kc * s.ld_out * 4);
@@ -439,10 +452,12 @@ int tc_conv_backward_filter(const ConvGeo& g, const float* gy, const float* x, f
                                                                       s.hwp_out, s.ld_out);
   FLB200_AFTER_LAUNCH("planes_to_rows");
   if (int rc = map2d(&ma, dyt, s.ld_out, g.Cout, s.ld_out, tc::kBM, false)) return rc;
-  if (int rc = map2d(&mb, col, s.ld_out, s.kc, s.ld_out, tc::b_box_rows(g.Cout, s.kc, (s.ld_out + tc::kBK - 1) / tc::kBK, false, false), false)) return rc;
+  const long long k_iters = (s.ld_out + tc::kBK - 1) / tc::kBK;
+  const tc::Launch L = gemm_plan(g.Cout, s.kc, k_iters, false, false, true);
+  if (int rc = map2d(&mb, col, s.ld_out, s.kc, s.ld_out, L.b_box_rows(), false)) return rc;
   ep.m_stride = s.kc;
-  return tc::run(ma, mb, plan_k_major(2), plan_k_major(2), ep, g.Cout, s.kc,
-                 (s.ld_out + tc::kBK - 1) / tc::kBK, 1, base + off, ws_bytes - off, st);
+  return tc::run(ma, mb, plan_k_major(2), plan_k_major(2), ep, g.Cout, s.kc, k_iters, 1, L,
+                 base + off, ws_bytes - off, st);
 }
 
 }  // namespace flb200

@@ -311,6 +311,7 @@ template <int BN>
 int run_patch(const CUtensorMap& ma, const CUtensorMap& mb, const PatchArgs& a, cudaStream_t st) {
   tc::PatchConvProblem<BN> p;
   p.a_mn_major = 0; p.b_mn_major = 0;
+  p.operand = tc::kOperandTf32;
   p.QW = a.patch.QW; p.PH = a.patch.PH; p.NB = a.patch.NB;
   p.qw_shift = a.patch.qw_shift; p.ph_shift = a.patch.ph_shift;
   p.tiles_q = (a.pix_w + p.QW - 1) / p.QW;
@@ -391,6 +392,7 @@ int run_wgrad(const CUtensorMap& ma, const CUtensorMap& mb, const ConvGeo& g, co
               const WgradPlan& w, float* partial, cudaStream_t st) {
   tc::PatchWgradProblem<BN> p;
   p.a_mn_major = 1; p.b_mn_major = 1;
+  p.operand = tc::kOperandTf32;
   p.QW = w.QW; p.PH = w.PH; p.tiles_q = w.tiles_q; p.tiles_p = w.tiles_p; p.images = g.N;
   p.M = g.Cout; p.N = tp.C;
   p.tiles_m = (g.Cout + tc::kBM - 1) / tc::kBM;

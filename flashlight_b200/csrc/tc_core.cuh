@@ -155,8 +155,8 @@ __device__ __forceinline__ void umma_tf32(uint32_t tmem_d, uint64_t adesc, uint6
       "l"(adesc), "l"(bdesc), "r"(idesc), "r"(accumulate)
       : "memory");
 }
-// bf16 operands (kind::f16), fp32 accumulate; K = 16 per instruction.
-__device__ __forceinline__ void umma_bf16(uint32_t tmem_d, uint64_t adesc, uint64_t bdesc,
+// bf16 or f16 operands (kind::f16), fp32 accumulate; K = 16 per instruction.
+__device__ __forceinline__ void umma_f16(uint32_t tmem_d, uint64_t adesc, uint64_t bdesc,
                                           uint32_t idesc, uint32_t accumulate) {
   asm volatile(
       "{\n\t.reg .pred p;\n\t"
@@ -225,9 +225,12 @@ __host__ __device__ inline uint32_t umma_idesc_tf32(int n, int a_mn_major, int b
          ((uint32_t)b_mn_major << 16) | ((uint32_t)(n >> 3) << 17) | ((uint32_t)(kBM >> 4) << 24);
 }
 
-// Instruction descriptor for kind::f16 with bf16 operands (format 1), fp32 accumulate, M = 128.
-__host__ __device__ inline uint32_t umma_idesc_bf16(int n, int a_mn_major, int b_mn_major) {
-  return (1u << 4) | (1u << 7) | (1u << 10) | ((uint32_t)a_mn_major << 15) |
+// Instruction descriptor for kind::f16 with bf16 (operand format 1) or f16 (0) operands, fp32
+// accumulate, M = 128.
+__host__ __device__ inline uint32_t umma_idesc_f16(int operand, int n, int a_mn_major,
+                                                   int b_mn_major) {
+  const uint32_t fmt = operand == kOperandBf16 ? 1u : 0u;
+  return (1u << 4) | (fmt << 7) | (fmt << 10) | ((uint32_t)a_mn_major << 15) |
          ((uint32_t)b_mn_major << 16) | ((uint32_t)(n >> 3) << 17) | ((uint32_t)(kBM >> 4) << 24);
 }
 
@@ -314,6 +317,15 @@ __device__ __forceinline__ void umma_tf32_pair(uint32_t tmem_d, uint64_t adesc, 
       "l"(adesc), "l"(bdesc), "r"(idesc), "r"(accumulate)
       : "memory");
 }
+__device__ __forceinline__ void umma_f16_pair(uint32_t tmem_d, uint64_t adesc, uint64_t bdesc,
+                                              uint32_t idesc, uint32_t accumulate) {
+  asm volatile(
+      "{\n\t.reg .pred p;\n\t"
+      "setp.ne.b32 p, %4, 0;\n\t"
+      "tcgen05.mma.cta_group::2.kind::f16 [%0], %1, %2, %3, p;\n\t}" ::"r"(tmem_d),
+      "l"(adesc), "l"(bdesc), "r"(idesc), "r"(accumulate)
+      : "memory");
+}
 // One arrival on the barrier at this shared-memory offset in BOTH CTAs of the pair once every
 // MMA issued so far by this thread has completed.
 __device__ __forceinline__ void umma_commit_pair(uint64_t* bar) {
@@ -328,6 +340,12 @@ __device__ __forceinline__ void umma_commit_pair(uint64_t* bar) {
 __host__ __device__ inline uint32_t umma_idesc_tf32_pair(int n, int a_mn_major, int b_mn_major) {
   return (1u << 4) | (2u << 7) | (2u << 10) | ((uint32_t)a_mn_major << 15) |
          ((uint32_t)b_mn_major << 16) | ((uint32_t)(n >> 3) << 17) |
+         ((uint32_t)((2 * kBM) >> 4) << 24);
+}
+// kind::f16 across the pair.
+__host__ __device__ inline uint32_t umma_idesc_f16_pair(int operand, int n, int a_mn_major,
+                                                        int b_mn_major) {
+  return (umma_idesc_f16(operand, n, a_mn_major, b_mn_major) & 0x00ffffffu) |
          ((uint32_t)((2 * kBM) >> 4) << 24);
 }
 

@@ -40,7 +40,7 @@ static EncodeTiledFn encode_tiled_fn() {
 // 128-byte swizzle of 16-byte chunks, MN-major ones the swizzle of 32-byte chunks.
 int make_tensor_map(CUtensorMap* map, const void* base, int rank, const uint64_t* dims,
                     const uint64_t* strides_bytes, const uint32_t* box, int mode,
-                    const uint32_t* elem_strides, bool bf16) {
+                    const uint32_t* elem_strides, int operand) {
   EncodeTiledFn fn = encode_tiled_fn();
   if (!fn) return fail(FLB200_UNSUPPORTED, "cuTensorMapEncodeTiled is not available");
   cuuint64_t gd[5];
@@ -52,7 +52,10 @@ int make_tensor_map(CUtensorMap* map, const void* base, int rank, const uint64_t
     es[i] = elem_strides ? elem_strides[i] : 1;
     if (i > 0) gs[i - 1] = strides_bytes[i - 1];
   }
-  CUresult r = fn(map, bf16 ? CU_TENSOR_MAP_DATA_TYPE_BFLOAT16 : CU_TENSOR_MAP_DATA_TYPE_FLOAT32,
+  CUresult r = fn(map,
+                  operand == kOperandBf16   ? CU_TENSOR_MAP_DATA_TYPE_BFLOAT16
+                  : operand == kOperandF16 ? CU_TENSOR_MAP_DATA_TYPE_FLOAT16
+                                           : CU_TENSOR_MAP_DATA_TYPE_FLOAT32,
                   (cuuint32_t)rank, const_cast<void*>(base),
                   gd, gs, bx, es, CU_TENSOR_MAP_INTERLEAVE_NONE,
                   mode == kMapStaging ? CU_TENSOR_MAP_SWIZZLE_NONE
@@ -112,10 +115,14 @@ tc_splitk_reduce_kernel(const float* __restrict__ partial, EpiloguePlan ep, int 
     const long long off = epi_off(m, ep.m_div, ep.m_stride, ep.m_outer) +
                           epi_off(n, ep.n_div, ep.n_stride, ep.n_outer) + (long long)z * ep.z_stride;
     float v = ep.alpha * s + (ep.bias_m ? ep.bias_m[m] : 0.f) + (ep.bias_n ? ep.bias_n[n] : 0.f);
-    if (ep.out_bf16) {
+    if (ep.out16 == kOperandBf16) {
       __nv_bfloat16* dst = reinterpret_cast<__nv_bfloat16*>(ep.out) + off;
       if (ep.beta != 0.f) v += ep.beta * __bfloat162float(*dst);
       *dst = __float2bfloat16(v);
+    } else if (ep.out16 == kOperandF16) {
+      __half* dst = reinterpret_cast<__half*>(ep.out) + off;
+      if (ep.beta != 0.f) v += ep.beta * __half2float(*dst);
+      *dst = __float2half_rn(v);
     } else {
       float* dst = ep.out + off;
       if (ep.beta != 0.f) v += ep.beta * *dst;
@@ -125,7 +132,10 @@ tc_splitk_reduce_kernel(const float* __restrict__ partial, EpiloguePlan ep, int 
 }
 
 // The same for a row-major result (unit column stride, no row / column regrouping) of a
-// multiple of 4 columns: four columns per thread, 16-byte loads of every split's partial sums.
+// multiple of 4 columns: four columns per thread, 16-byte loads of every split's partial sums,
+// and the activation of a fused linear layer (pre-activation rounded to T first, as the store
+// of an unsplit product does).
+template <typename T>
 static __global__ void __launch_bounds__(256)
 tc_splitk_reduce_vec_kernel(const float4* __restrict__ partial, EpiloguePlan ep, int M, int N4,
                             int Z, int splits) {
@@ -136,37 +146,32 @@ tc_splitk_reduce_vec_kernel(const float4* __restrict__ partial, EpiloguePlan ep,
     const int z = (int)(i / mn4);
     const long long r = i - (long long)z * mn4;
     const int m = (int)(r / N4), n = 4 * (int)(r - (long long)m * N4);
+    const float4* src = partial + (long long)z * splits * mn4 + r;
     float4 s = make_float4(0.f, 0.f, 0.f, 0.f);
+#pragma unroll 4
     for (int sp = 0; sp < splits; ++sp) {
-      const float4 p = partial[((long long)z * splits + sp) * mn4 + r];
+      const float4 p = src[(long long)sp * mn4];
       s.x += p.x; s.y += p.y; s.z += p.z; s.w += p.w;
     }
     const long long off = (long long)m * ep.m_stride + n + (long long)z * ep.z_stride;
     const float bm = ep.bias_m ? ep.bias_m[m] : 0.f;
-    float v[4] = {ep.alpha * s.x + bm, ep.alpha * s.y + bm, ep.alpha * s.z + bm,
-                  ep.alpha * s.w + bm};
+    float4 v = make_float4(ep.alpha * s.x + bm, ep.alpha * s.y + bm, ep.alpha * s.z + bm,
+                           ep.alpha * s.w + bm);
     if (ep.bias_n) {
       const float4 b = *reinterpret_cast<const float4*>(ep.bias_n + n);
-      v[0] += b.x; v[1] += b.y; v[2] += b.z; v[3] += b.w;
+      v.x += b.x; v.y += b.y; v.z += b.z; v.w += b.w;
     }
-    if (ep.out_bf16) {
-      __nv_bfloat162* dst = reinterpret_cast<__nv_bfloat162*>(
-          reinterpret_cast<__nv_bfloat16*>(ep.out) + off);
-      if (ep.beta != 0.f) {
-        const float2 d0 = __bfloat1622float2(dst[0]), d1 = __bfloat1622float2(dst[1]);
-        v[0] += ep.beta * d0.x; v[1] += ep.beta * d0.y;
-        v[2] += ep.beta * d1.x; v[3] += ep.beta * d1.y;
-      }
-      __nv_bfloat162 h[2] = {__floats2bfloat162_rn(v[0], v[1]), __floats2bfloat162_rn(v[2], v[3])};
-      *reinterpret_cast<uint2*>(dst) = *reinterpret_cast<uint2*>(h);
-    } else {
-      float4* dst = reinterpret_cast<float4*>(ep.out + off);
-      if (ep.beta != 0.f) {
-        const float4 d = *dst;
-        v[0] += ep.beta * d.x; v[1] += ep.beta * d.y; v[2] += ep.beta * d.z; v[3] += ep.beta * d.w;
-      }
-      *dst = make_float4(v[0], v[1], v[2], v[3]);
+    T* dst = reinterpret_cast<T*>(ep.out) + off;
+    if (ep.beta != 0.f) {
+      v.x += ep.beta * Num<T>::to_f(dst[0]); v.y += ep.beta * Num<T>::to_f(dst[1]);
+      v.z += ep.beta * Num<T>::to_f(dst[2]); v.w += ep.beta * Num<T>::to_f(dst[3]);
     }
+    if (ep.act) {
+      v = epi_round<T>(v);
+      if (ep.pre) epi_store4(static_cast<T*>(ep.pre) + off, v);
+      v = make_float4(epi_gelu(v.x), epi_gelu(v.y), epi_gelu(v.z), epi_gelu(v.w));
+    }
+    epi_store4(dst, v);
   }
 }
 
@@ -179,9 +184,9 @@ template <int BN>
 static int launch_gemm(const CUtensorMap& ma, const CUtensorMap& mb, const OperandPlan& pa,
                        const OperandPlan& pb, const EpiloguePlan& ep, long long M, long long N,
                        long long k_iters, long long Z, const Launch& L, float* partial,
-                       cudaStream_t st, bool bf16) {
+                       cudaStream_t st, int operand) {
   GemmProblem<BN> p;
-  p.bf16 = bf16 ? 1 : 0;
+  p.operand = operand;
   p.a = make_coords(pa); p.b = make_coords(pb); p.ep = ep;
   p.a_mn_major = pa.mn_major; p.b_mn_major = pb.mn_major;
   p.M = (int)M; p.N = (int)N; p.k_iters = (int)k_iters;
@@ -196,11 +201,11 @@ static int launch_gemm(const CUtensorMap& ma, const CUtensorMap& mb, const Opera
   p.tiles_n = (int)((N + BN - 1) / BN);
   p.Z = (int)Z;
   p.partial = partial;
+  p.set_store_mode();
   const long long tiles = (long long)p.tiles_m * p.tiles_n * Z * L.splits;
   FLB200_REQUIRE(tiles < 0x7fffffffLL, "tc_gemm: too many tiles");
-  if constexpr (BN >= 128) {
-    if (!bf16 && !x3_enabled() &&
-        gemm_uses_pairs(M, N, k_iters, pa.mn_major != 0, pb.mn_major != 0)) {
+  if constexpr (BN >= 256) {
+    if (L.pairs) {
       const long long pair_tiles = (long long)((p.tiles_m + 1) / 2) * p.tiles_n * Z * L.splits;
       return launch_pair_problem<GemmProblem<BN>, BN>("tc_gemm_pair", ma, mb, p, pair_tiles, st);
     }
@@ -215,27 +220,6 @@ int pick_bn(long long N) {
   if (N <= 64) return 64;
   if (N < 192) return 128;
   return 256;
-}
-
-bool gemm_uses_pairs(long long M, long long N, long long k_iters, bool a_mn_major,
-                     bool b_mn_major) {
-  if (x3_enabled()) return false;  // the CTA-pair kernel has no 3xTF32 instantiation
-  // 1x1 forward layers (activation planes MN-major, filter K-major): 5-9 % faster on pairs
-  // with 256-column tiles; with both operands MN-major (1x1 backward data: 8 copies per CTA
-  // and stage) pairs measured between 7 % faster and 11 % slower and are not used.
-  if (a_mn_major && !b_mn_major) return pick_bn(N) >= 256 && M > kBM && k_iters >= 8;
-  if (a_mn_major || b_mn_major) return false;
-  // both K-major: long K loops (backward-filter of 1 x 1 layers) ...
-  if (pick_bn(N) >= 128 && M > kBM && k_iters >= 64) return true;
-  // ... and tall products with wide rows (1 x 1 layers over channels-last tensors, linear
-  // layers): every 128-row tile re-reads the whole B panel out of L2, a pair halves that
-  static const long long min_k = env_ll("FLB200_PAIR_MIN_K", 4);
-  static const long long min_bn = env_ll("FLB200_PAIR_MIN_BN", 256);
-  return pick_bn(N) >= min_bn && M >= 8 * kBM && k_iters >= min_k;
-}
-int b_box_rows(long long M, long long N, long long k_iters, bool a_mn_major, bool b_mn_major) {
-  const int bn = pick_bn(N);
-  return gemm_uses_pairs(M, N, k_iters, a_mn_major, b_mn_major) ? bn / 2 : bn;
 }
 
 void plan_splits(long long tiles, long long k_iters, long long min_ips, int* splits_out,
@@ -268,46 +252,107 @@ void plan_splits(long long tiles, long long k_iters, long long min_ips, int* spl
   *ips_out = (int)best_ips;
 }
 
-Launch plan_launch(long long M, long long N, long long k_iters, long long Z) {
-  Launch L;
-  L.bn = pick_bn(N);
-  const long long tiles = ((M + kBM - 1) / kBM) * ((N + L.bn - 1) / L.bn) * Z;
-  plan_splits(tiles, k_iters, 8, &L.splits, &L.iters_per_split);
-  L.workspace_bytes = L.splits > 1 ? (size_t)(Z * L.splits * M * N) * sizeof(float) : 0;
-  return L;
+// The launch lasts `rounds` tiles per CTA (or CTA pair), so the plan weighs the clocks of a tile
+// against how evenly the tiles fill the 148 SMs.  Clocks of one stage (128 bytes of K), measured:
+// a tile sits at the shared-memory port, 2 x (16 KB + BN x 128 B) per stage at 128 B/clock, and
+// above ~420 of barrier hand-over; a pair halves the B half of that and runs at the tensor
+// pipe's own 512.  A small product wants narrow tiles and a split of K for the sake of the
+// idle SMs: a 128-row bf16 product of 2304 columns ran on 9 CTAs of 148 with 256-column tiles,
+// 17 us; on 72 with 32-column ones, 7 us.
+Launch plan_launch(long long M, long long N, long long k_iters, long long Z, bool a_mn_major,
+                   bool b_mn_major, int operand, bool split_k) {
+  const long long sm = device_info().sm_count > 0 ? device_info().sm_count : 148;
+  const bool x3 = x3_enabled();
+  if (k_iters < 1) k_iters = 1;
+  const int box = operand == kOperandTf32 ? 32 : 64;
+  const long long tiles_m = (M + kBM - 1) / kBM;
+  Launch best{};
+  double best_cost = -1.0;
+  struct Width { int bn, pairs, clocks; };
+  static const Width widths[5] = {
+      {256, 1, 530}, {256, 0, 780}, {128, 0, 520}, {64, 0, 440}, {32, 0, 420}};
+  int widest = pick_bn(N);
+  if (operand != kOperandTf32 && b_mn_major && widest < box) widest = box;
+  for (const Width& w : widths) {
+    if (w.bn > widest) continue;
+    if (operand != kOperandTf32 && b_mn_major && w.bn < box) continue;  // one box at least
+    if (w.pairs) {
+      if (x3 || M <= kBM) continue;
+      // TF32 pairs, measured: both operands MN-major (12 copies a stage) win nothing, and a
+      // short K loop loses more to the cross-CTA hand-offs than it gains
+      if (operand == kOperandTf32 && (b_mn_major || k_iters < (a_mn_major ? 8 : 4))) continue;
+      if (k_iters < 4) continue;
+    }
+    double clocks = w.clocks * (x3 ? 2.5 : 1.0);
+    // issuing a TMA copy takes a producer warp ~120 clocks, and there are two of them
+    const int copies = (a_mn_major ? kBM / box : 1) +
+                       (b_mn_major ? (w.pairs ? w.bn / 2 : w.bn) / box : 1);
+    if (clocks < copies * 65.0) clocks = copies * 65.0;
+    const double drain = 600.0 + 8.0 * w.bn;  // storing one tile, hidden behind the next
+    const long long units = w.pairs ? sm / 2 : sm;
+    const long long tiles = (w.pairs ? (tiles_m + 1) / 2 : tiles_m) * ((N + w.bn - 1) / w.bn) * Z;
+    const long long by_k = k_iters / 4;
+    long long tries[3] = {1, units / (tiles > 0 ? tiles : 1), 2 * units / (tiles > 0 ? tiles : 1)};
+    for (int i = 0; i < 3; ++i) {
+      long long s = tries[i] < by_k ? tries[i] : by_k;
+      if (i > 0 && (!split_k || s < 2)) continue;
+      if (s < 1) s = 1;
+      const long long ips = (k_iters + s - 1) / s;
+      s = (k_iters + ips - 1) / ips;
+      const long long rounds = (tiles * s + units - 1) / units;
+      const double loop = ips * clocks > drain ? ips * clocks : drain;
+      double cost = 4000.0 + rounds * loop + drain;
+      // the partial sums and the second launch that adds them
+      if (s > 1) cost += 4500.0 + (double)M * N * Z * 4.0 * (2 * s + 1) / 2500.0;
+      if (best_cost < 0 || cost < best_cost) {
+        best_cost = cost;
+        best.bn = w.bn;
+        best.pairs = w.pairs;
+        best.splits = (int)s;
+        best.iters_per_split = (int)ips;
+      }
+    }
+  }
+  best.workspace_bytes = best.splits > 1 ? (size_t)(Z * best.splits * M * N) * sizeof(float) : 0;
+  return best;
 }
 
 int run(const CUtensorMap& ma, const CUtensorMap& mb, const OperandPlan& pa, const OperandPlan& pb,
-        const EpiloguePlan& ep, long long M, long long N, long long k_iters, long long Z, void* ws,
-        size_t ws_bytes, cudaStream_t st, bool bf16) {
-  Launch L = plan_launch(M, N, k_iters, Z);
-  // an MN-major bf16 B tile is made of 64-column boxes: no narrower tile than one box
-  if (bf16 && pb.mn_major && L.bn < 64) L.bn = 64;
-  // split-K partials are written with 16-byte vectors: an unaligned workspace is not used
-  // (nor are the column statistics of the output taken from partial sums)
-  if (L.splits > 1 && (!ws || !aligned16(ws) || ws_bytes < L.workspace_bytes || ep.stats || ep.act ||
-                       ep.pre)) {
-    L.splits = 1;
-    L.iters_per_split = (int)k_iters;
+        const EpiloguePlan& ep, long long M, long long N, long long k_iters, long long Z, Launch L,
+        void* ws, size_t ws_bytes, cudaStream_t st, int operand) {
+  const uintptr_t out_addr = reinterpret_cast<uintptr_t>(ep.out);
+  const bool rows_of_4 = ep.m_div == 0 && ep.n_div == 0 && ep.m_valid == 0 && ep.n_stride == 1 &&
+                         N % 4 == 0 && ep.m_stride % 4 == 0 && ep.z_stride % 4 == 0 &&
+                         out_addr % (ep.out16 ? 8 : 16) == 0 &&
+                         (!ep.bias_n || aligned16(ep.bias_n));
+  if (L.splits > 1) {
+    // split-K partials are written with 16-byte vectors: an unaligned workspace is not used
+    // (nor are the column statistics of the output taken from partial sums)
+    const size_t one = (size_t)(Z * M * N) * sizeof(float);
+    long long s = ws && aligned16(ws) ? (long long)(ws_bytes / one) : 0;
+    if (s > L.splits) s = L.splits;
+    if (s < 2 || ep.stats || (ep.act && !rows_of_4)) s = 1;
+    L.iters_per_split = (int)((k_iters + s - 1) / s);
+    L.splits = (int)((k_iters + L.iters_per_split - 1) / L.iters_per_split);
   }
   float* partial = static_cast<float*>(ws);
   int rc;
-  if (L.bn == 32) rc = launch_gemm<32>(ma, mb, pa, pb, ep, M, N, k_iters, Z, L, partial, st, bf16);
-  else if (L.bn == 64) rc = launch_gemm<64>(ma, mb, pa, pb, ep, M, N, k_iters, Z, L, partial, st, bf16);
-  else if (L.bn == 128) rc = launch_gemm<128>(ma, mb, pa, pb, ep, M, N, k_iters, Z, L, partial, st, bf16);
-  else rc = launch_gemm<256>(ma, mb, pa, pb, ep, M, N, k_iters, Z, L, partial, st, bf16);
+  if (L.bn == 32) rc = launch_gemm<32>(ma, mb, pa, pb, ep, M, N, k_iters, Z, L, partial, st, operand);
+  else if (L.bn == 64) rc = launch_gemm<64>(ma, mb, pa, pb, ep, M, N, k_iters, Z, L, partial, st, operand);
+  else if (L.bn == 128) rc = launch_gemm<128>(ma, mb, pa, pb, ep, M, N, k_iters, Z, L, partial, st, operand);
+  else rc = launch_gemm<256>(ma, mb, pa, pb, ep, M, N, k_iters, Z, L, partial, st, operand);
   if (rc) return rc;
   if (L.splits > 1) {
-    const uintptr_t out_addr = reinterpret_cast<uintptr_t>(ep.out);
-    const bool rows_of_4 = ep.m_div == 0 && ep.n_div == 0 && ep.m_valid == 0 && ep.n_stride == 1 &&
-                           N % 4 == 0 && ep.m_stride % 4 == 0 && ep.z_stride % 4 == 0 &&
-                           out_addr % (ep.out_bf16 ? 8 : 16) == 0 &&
-                           (!ep.bias_n || aligned16(ep.bias_n));
     if (rows_of_4) {
       const int rgrid = grid_for(M * (N / 4) * Z, 256);
-      tc_splitk_reduce_vec_kernel<<<rgrid, 256, 0, st>>>(reinterpret_cast<const float4*>(partial),
-                                                         ep, (int)M, (int)(N / 4), (int)Z,
-                                                         L.splits);
+      const float4* p4 = reinterpret_cast<const float4*>(partial);
+      const int n4 = (int)(N / 4);
+      if (ep.out16 == kOperandBf16)
+        tc_splitk_reduce_vec_kernel<__nv_bfloat16><<<rgrid, 256, 0, st>>>(p4, ep, (int)M, n4, (int)Z, L.splits);
+      else if (ep.out16 == kOperandF16)
+        tc_splitk_reduce_vec_kernel<__half><<<rgrid, 256, 0, st>>>(p4, ep, (int)M, n4, (int)Z, L.splits);
+      else
+        tc_splitk_reduce_vec_kernel<float><<<rgrid, 256, 0, st>>>(p4, ep, (int)M, n4, (int)Z, L.splits);
     } else {
       const int rgrid = grid_for(M * N * Z, 256);
       tc_splitk_reduce_kernel<<<rgrid, 256, 0, st>>>(partial, ep, (int)M, (int)N, (int)Z,
@@ -369,9 +414,10 @@ Prepared prepare(const flb200_matmul_desc* d, const void* a, const void* b, cons
 // Tensor map + plan of one operand: rows x K matrix (+ batch).
 int build_operand(const Side& s, const void* base, long long rows, long long K, long long batch,
                   long long batch_stride, int tile_rows, CUtensorMap* map, tc::OperandPlan* plan,
-                  bool bf16) {
-  const uint32_t kstage = bf16 ? 64 : tc::kBK;   // elements of K per stage (128 bytes)
-  const uint64_t esize = bf16 ? 2 : 4;
+                  int operand) {
+  const bool half = operand != tc::kOperandTf32;
+  const uint32_t kstage = tc::stage_k(operand);  // elements of K per stage (128 bytes)
+  const uint64_t esize = half ? 2 : 4;
   uint64_t dims[3], strides[2];
   uint32_t box[3];
   *plan = tc::OperandPlan{};
@@ -379,7 +425,7 @@ int build_operand(const Side& s, const void* base, long long rows, long long K, 
   plan->k2_dim = -1;
   if (s.mn_major) {
     dims[0] = (uint64_t)rows; dims[1] = (uint64_t)K;
-    box[0] = bf16 ? 64 : 32; box[1] = kstage;
+    box[0] = half ? 64 : 32; box[1] = kstage;
     plan->mn_major = 1; plan->mn_dim = 0; plan->k_dim = 1;
   } else {
     dims[0] = (uint64_t)K; dims[1] = (uint64_t)rows;
@@ -398,10 +444,10 @@ int build_operand(const Side& s, const void* base, long long rows, long long K, 
     plan->z_dim = 2;
   }
   plan->rank = rank;
-  // bf16 tiles use the plain 128-byte swizzle for both majors
+  // 16-bit tiles use the plain 128-byte swizzle for both majors
   return tc::make_tensor_map(map, base, rank, dims, strides, box,
-                             s.mn_major && !bf16 ? tc::kMapMnMajor : tc::kMapKMajor, nullptr,
-                             bf16);
+                             s.mn_major && !half ? tc::kMapMnMajor : tc::kMapKMajor, nullptr,
+                             operand);
 }
 
 }  // namespace
@@ -414,12 +460,20 @@ bool tc_gemm_supported(const flb200_matmul_desc* d, const void* a, const void* b
 
 size_t tc_gemm_workspace_bytes(const flb200_matmul_desc* d) {
   if (!d || d->m < 1 || d->n < 1 || d->k < 1) return 0;
-  const long long kstage = d->dtype == FLB200_BF16 ? 64 : tc::kBK;
-  const long long k_iters = (d->k + kstage - 1) / kstage;
-  // the swapped orientation has the same M*N; take the larger split count of both
-  const size_t w1 = tc::plan_launch(d->m, d->n, k_iters, d->batch).workspace_bytes;
-  const size_t w2 = tc::plan_launch(d->n, d->m, k_iters, d->batch).workspace_bytes;
-  return w1 > w2 ? w1 : w2;
+  // What the call will want depends on things that this query does not know (operand alignment,
+  // and for the linear layers the type): the largest of the plans it may choose.
+  size_t need = 0;
+  for (int operand : {(int)tc::kOperandTf32, (int)tc::kOperandBf16}) {
+    const long long k_iters = (d->k + tc::stage_k(operand) - 1) / tc::stage_k(operand);
+    for (int mn = 0; mn < 2; ++mn)
+      for (int swap = 0; swap < 2; ++swap) {
+        const size_t w = tc::plan_launch(swap ? d->n : d->m, swap ? d->m : d->n, k_iters, d->batch,
+                                         mn != 0, mn != 0, operand, true)
+                             .workspace_bytes;
+        if (w > need) need = w;
+      }
+  }
+  return need;
 }
 
 int tc_gemm_run(const flb200_matmul_desc* d, const void* a, const void* b, void* c, void* ws,
@@ -432,42 +486,34 @@ int tc_gemm_run(const flb200_matmul_desc* d, const void* a, const void* b, void*
     return fail(FLB200_UNSUPPORTED,
                 "tc_gemm: bias / activation are fused only into a row-major, 16-byte aligned "
                 "result of a multiple of 32 columns");
-  const bool bf16 = d->dtype == FLB200_BF16;
-  const long long kstage = bf16 ? 64 : tc::kBK;
+  const int operand = tc::operand_of(d->dtype);
+  const long long kstage = tc::stage_k(operand);
   const long long k_iters = (d->k + kstage - 1) / kstage;
   CUtensorMap ma, mb;
   tc::OperandPlan pa, pb;
   tc::EpiloguePlan ep{};
   ep.out = static_cast<float*>(c);
-  ep.out_bf16 = bf16 ? 1 : 0;
+  ep.out16 = operand;
   ep.alpha = d->alpha;
   ep.beta = d->beta;
   ep.z_stride = d->c_batch;
   ep.bias_n = bias_n;
   ep.act = act;
   ep.pre = pre;
-  long long M, N;
-  if (!p.swap) {
-    M = d->m; N = d->n;
-    const int bn = tc::pick_bn(N);
-    if (int rc = build_operand(p.a, a, d->m, d->k, d->batch, d->a_batch, tc::kBM, &ma, &pa, bf16)) return rc;
-    if (int rc = build_operand(p.b, b, d->n, d->k, d->batch, d->b_batch,
-                               bf16 ? bn : tc::b_box_rows(M, N, k_iters, p.a.mn_major, p.b.mn_major), &mb,
-                               &pb, bf16)) return rc;
-    ep.m_stride = d->c_row;
-    ep.n_stride = d->c_col;
-  } else {
-    // C^T = B^T A^T: the kernel's rows are the caller's columns
-    M = d->n; N = d->m;
-    const int bn = tc::pick_bn(N);
-    if (int rc = build_operand(p.b, b, d->n, d->k, d->batch, d->b_batch, tc::kBM, &ma, &pa, bf16)) return rc;
-    if (int rc = build_operand(p.a, a, d->m, d->k, d->batch, d->a_batch,
-                               bf16 ? bn : tc::b_box_rows(M, N, k_iters, p.b.mn_major, p.a.mn_major), &mb,
-                               &pb, bf16)) return rc;
-    ep.m_stride = d->c_col;
-    ep.n_stride = d->c_row;
-  }
-  return tc::run(ma, mb, pa, pb, ep, M, N, k_iters, d->batch, ws, ws_bytes, st, bf16);
+  // swapped, C^T = B^T A^T: the kernel's rows are the caller's columns
+  const Side &sa = p.swap ? p.b : p.a, &sb = p.swap ? p.a : p.b;
+  const long long M = p.swap ? d->n : d->m, N = p.swap ? d->m : d->n;
+  ep.m_stride = p.swap ? d->c_col : d->c_row;
+  ep.n_stride = p.swap ? d->c_row : d->c_col;
+  const tc::Launch L =
+      tc::plan_launch(M, N, k_iters, d->batch, sa.mn_major, sb.mn_major, operand, ws != nullptr);
+  if (int rc = build_operand(sa, p.swap ? b : a, M, d->k, d->batch, p.swap ? d->b_batch : d->a_batch,
+                             tc::kBM, &ma, &pa, operand))
+    return rc;
+  if (int rc = build_operand(sb, p.swap ? a : b, N, d->k, d->batch, p.swap ? d->a_batch : d->b_batch,
+                             L.b_box_rows(), &mb, &pb, operand))
+    return rc;
+  return tc::run(ma, mb, pa, pb, ep, M, N, k_iters, d->batch, L, ws, ws_bytes, st, operand);
 }
 
 }  // namespace flb200

@@ -24,6 +24,14 @@ namespace tc {
 constexpr int kBM = 128;  // rows of one output tile (UMMA M)
 constexpr int kBK = 32;   // fp32 elements per pipeline stage along K (= 128 bytes)
 
+// Operand types of a contraction: fp32 read as TF32, or 16-bit (twice the elements per stage).
+enum { kOperandTf32 = 0, kOperandBf16 = 1, kOperandF16 = 2 };
+inline int operand_of(int dtype) {
+  return dtype == FLB200_BF16 ? kOperandBf16 : (dtype == FLB200_F16 ? kOperandF16 : kOperandTf32);
+}
+// elements of K per 128-byte stage row
+inline int stage_k(int operand) { return operand == kOperandTf32 ? kBK : 2 * kBK; }
+
 // How one operand's TMA coordinates advance.  coord[d] for dimension d of the
 // tensor map is  base[d] + mn * (d == mn_dim) + k_lo * (d == k_dim)
 //                + k_hi * k2_scale * (d == k2_dim) + z * (d == z_dim)
@@ -73,32 +81,31 @@ struct EpiloguePlan {
   const float* bias_m;  // added per row (may be null)
   const float* bias_n;  // added per column (may be null)
   float alpha, beta;
-  int out_bf16;         // `out` points at __nv_bfloat16 (offsets are in elements either way)
+  int out16;            // `out` points at kOperandBf16 / kOperandF16 elements (offsets are in
+                        // elements either way); 0: fp32
   int act;              // 0 none, 1 GELU (tanh form): applied after alpha and the biases, on the
-                        // row-major fp32 (staged) and bf16 (vector) store paths only
+                        // staged row-major store path and in the split-K reduction only
   void* pre;            // with act: where the value BEFORE the activation goes too (same type
                         // and layout as `out`; what the activation's gradient needs), or null
   float* stats;         // EpiStats matrix [ceil(M / 128) * 4][2 * N] (tc_kernel.cuh) or null:
                         // per-column sums and sums of squares of a row-major fp32 output
 };
 
+// How an M x N contraction over k_iters stages and Z batches runs: tile width, whether CTA pairs
+// (tc_pair.cuh) or single CTAs, split-K factor and the scratch that takes.
 struct Launch {
-  int bn, splits, iters_per_split;
+  int bn, pairs, splits, iters_per_split;
   size_t workspace_bytes;
+  // rows a K-major B map must put in one box: a pair's CTAs load half of the tile's columns each
+  int b_box_rows() const { return pairs ? bn / 2 : bn; }
 };
 
+// tile width by the number of columns alone (the convolution policies' starting point)
 int pick_bn(long long N);
-// Whether an M x N contraction runs on CTA pairs (two SMs per 256 x BN tile, each loading half
-// of the B tile), and the number of rows a K-major B map must put in one box accordingly.
-// Pairs pay off when both operands are K-major single boxes and the K loop is long (the
-// backward-filter shapes), and for an MN-major A with a K-major B at 256 columns (the 1x1
-// forward layers); tiles with a short K loop lose more to the cross-CTA hand-offs per tile
-// than they gain (measured).  Every K-major B map must take its box rows from b_box_rows.
-bool gemm_uses_pairs(long long M, long long N, long long k_iters, bool a_mn_major,
-                     bool b_mn_major);
-int b_box_rows(long long M, long long N, long long k_iters, bool a_mn_major, bool b_mn_major);
-// Tile width, split-K factor and scratch size for an M x N output over k_iters stages, Z batches.
-Launch plan_launch(long long M, long long N, long long k_iters, long long Z);
+// Every map of a run must be made for the plan it runs with (b_box_rows).  split_k: the caller
+// has scratch and an epilogue that the split-K reduction can apply.
+Launch plan_launch(long long M, long long N, long long k_iters, long long Z, bool a_mn_major,
+                   bool b_mn_major, int operand, bool split_k);
 // Split-K factor for `tiles` output tiles of k_iters stage iterations each, at least min_ips
 // iterations per split, chosen so that tiles * splits fills whole rounds of the persistent grid.
 void plan_splits(long long tiles, long long k_iters, long long min_ips, int* splits, int* ips);
@@ -112,7 +119,7 @@ void plan_splits(long long tiles, long long k_iters, long long min_ips, int* spl
 enum { kMapKMajor = 0, kMapMnMajor = 1, kMapStaging = 2 };
 int make_tensor_map(CUtensorMap* map, const void* base, int rank, const uint64_t* dims,
                     const uint64_t* strides_bytes, const uint32_t* box, int mode,
-                    const uint32_t* elem_strides = nullptr, bool bf16 = false);
+                    const uint32_t* elem_strides = nullptr, int operand = kOperandTf32);
 
 // 3xTF32 ("fp32-grade") mode of the current host thread: set by the C entry points around a
 // call (X3Scope), read where kernels are launched.
@@ -127,11 +134,11 @@ struct X3Scope {
 int* status_ptr();
 void count_tc_launch();
 
-// Launches the contraction (and the split-K reduction when the plan splits K).  Without
-// enough scratch the contraction runs unsplit.
+// Launches the contraction as planned (and the split-K reduction when the plan splits K).  With
+// less scratch than the plan wants, fewer splits run; with none, one.
 int run(const CUtensorMap& ma, const CUtensorMap& mb, const OperandPlan& pa, const OperandPlan& pb,
-        const EpiloguePlan& ep, long long M, long long N, long long k_iters, long long Z, void* ws,
-        size_t ws_bytes, cudaStream_t st, bool bf16 = false);
+        const EpiloguePlan& ep, long long M, long long N, long long k_iters, long long Z, Launch L,
+        void* ws, size_t ws_bytes, cudaStream_t st, int operand = kOperandTf32);
 
 }  // namespace tc
 }  // namespace flb200

@@ -25,7 +25,7 @@
 // drain and the CTA frees its TMEM and returns (the host then reports FLB200_TIMEOUT).
 //
 // A problem policy P tells the skeleton what a tile is:
-//   int  a_mn_major, b_mn_major;
+//   int  a_mn_major, b_mn_major, operand;   // operand: kOperandTf32 / kOperandBf16 / kOperandF16
 //   static constexpr bool kWarpProducer;  // load() is called by the whole warp (else lane 0)
 //   static constexpr int kMinBlocks;      // second argument of tc_persistent_kernel's launch
 //                                         // bounds: 1 = the register allocator may use the whole
@@ -47,6 +47,8 @@
 //                         // warp's 4 KB staging tile for policies that store through it
 #pragma once
 #include <cuda_bf16.h>
+
+#include <type_traits>
 
 #include "tc_core.cuh"
 
@@ -108,6 +110,19 @@ struct EpiStats {
     }
   }
 };
+
+// Four consecutive elements of a row-major output, rounded to its type.
+__device__ __forceinline__ void epi_store4(float* p, float4 v) { *reinterpret_cast<float4*>(p) = v; }
+template <typename T>
+__device__ __forceinline__ void epi_store4(T* p, float4 v) {
+  T h[4] = {Num<T>::from_f(v.x), Num<T>::from_f(v.y), Num<T>::from_f(v.z), Num<T>::from_f(v.w)};
+  *reinterpret_cast<uint2*>(p) = *reinterpret_cast<const uint2*>(h);
+}
+template <typename T>
+__device__ __forceinline__ float4 epi_round(float4 v) {
+  return make_float4(Num<T>::to_f(Num<T>::from_f(v.x)), Num<T>::to_f(Num<T>::from_f(v.y)),
+                     Num<T>::to_f(Num<T>::from_f(v.z)), Num<T>::to_f(Num<T>::from_f(v.w)));
+}
 
 // gelu in the tanh form of flashlight/fl/autograd/Functions.cpp:1791-1796 (the constants of
 // flb200_gelu_forward)
@@ -191,8 +206,9 @@ tc_persistent_kernel(const __grid_constant__ CUtensorMap map_a,
   static_assert(STAGES % KSUB == 0 && (X3 == 0 || KSUB == 1), "ring must be whole groups");
   constexpr int NG = STAGES / KSUB;
   extern __shared__ char smem_raw[];
-  char* tiles = reinterpret_cast<char*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) &
-                                        ~static_cast<uintptr_t>(1023));
+  // (an offset rather than a rounded address: the compiler keeps knowing that the tiles are
+  // shared memory, and may move the epilogue's reads of them ahead of its stores)
+  char* tiles = smem_raw + ((1024u - (smem_u32(smem_raw) & 1023u)) & 1023u);
   uint64_t* full_bar = reinterpret_cast<uint64_t*>(tiles + SL::kTileBytes);
   uint64_t* empty_bar = full_bar + STAGES;
   uint64_t* tfull_bar = empty_bar + STAGES;   // [2] accumulator ready for the epilogue
@@ -305,15 +321,15 @@ tc_persistent_kernel(const __grid_constant__ CUtensorMap map_a,
     }
   } else if (warp == 1) {
     if (lane == 0) {
-      bool bf16 = false;
-      if constexpr (P::kBf16Capable) bf16 = prob.bf16 != 0;
-      const uint32_t idesc = bf16 ? umma_idesc_bf16(BN, prob.a_mn_major, prob.b_mn_major)
-                                  : umma_idesc_tf32(BN, prob.a_mn_major, prob.b_mn_major);
+      const bool half = prob.operand != kOperandTf32;
+      const uint32_t idesc =
+          half ? umma_idesc_f16(prob.operand, BN, prob.a_mn_major, prob.b_mn_major)
+               : umma_idesc_tf32(BN, prob.a_mn_major, prob.b_mn_major);
       // MN-major tiles: fp32 in 32 x 32 boxes with the 32-byte-chunk swizzle (4 KB apart, k
-      // atoms 512 B apart, 8 k-rows = 1 KB per MMA); bf16 in 64 x 64 boxes with the plain
+      // atoms 512 B apart, 8 k-rows = 1 KB per MMA); 16-bit in 64 x 64 boxes with the plain
       // 128-byte swizzle (8 KB apart, k atoms 1 KB apart, 16 k-rows = 2 KB per MMA)
-      const uint32_t mn_lbo = bf16 ? 8192 : kBK * 128, mn_sbo = bf16 ? 1024 : 512;
-      const uint32_t mn_step = bf16 ? 2048 : 1024, mn_layout = bf16 ? 2 : 1;
+      const uint32_t mn_lbo = half ? 8192 : kBK * 128, mn_sbo = half ? 1024 : 512;
+      const uint32_t mn_step = half ? 2048 : 1024, mn_layout = half ? 2 : 1;
       // descriptors of the ring's first sub-stage; every MMA offsets them (umma_desc_advance)
       const uint32_t ring = smem_u32(tiles);
       const uint64_t a_desc0 = prob.a_mn_major ? umma_desc(ring, mn_lbo, mn_sbo, mn_layout)
@@ -325,68 +341,76 @@ tc_persistent_kernel(const __grid_constant__ CUtensorMap map_a,
       // MN-major: step 8 (bf16: 16) k-rows = 1024 (2048) bytes inside each box.
       const uint32_t a_jstep = prob.a_mn_major ? mn_step : 32;
       const uint32_t b_jstep = prob.b_mn_major ? mn_step : 32;
-      uint32_t s = 0, round = 0, nt = 0;
-      typename P::Tile t;
       TC_PROF_VAR(m_full);
       TC_PROF_VAR(m_acc);
       TC_PROF_NOW(m_t0);
-      for (int tile = blockIdx.x; tile < n_tiles && *failed == 0; tile += gridDim.x, ++nt) {
-        prob.decode(tile, t);
-        const uint32_t acc = nt & 1, around = nt >> 1;
-        TC_PROF_NOW(w0);
-        if (around > 0 && !mbar_wait(&tempty_bar[acc], (around - 1) & 1)) {
-          *failed = 4;
-          break;
-        }
-        TC_PROF_ADD(m_acc, w0);
-        tc_fence_after();
-        const uint32_t d_tmem = tmem_base + acc * BN;
-        const int k0 = prob.k_begin(t), k1 = prob.k_end(t);
-        for (int k = k0; k < k1; k += KSUB) {
-          TC_PROF_NOW(w1);
-          if (!mbar_wait(X3 ? &split_bar[s] : &full_bar[s], round & 1)) {
-            *failed = 2;
+      // One copy of the loop per operand kind: with the kind tested between two MMAs the chains
+      // that feed their descriptors to the tensor core no longer overlap, and every MMA took
+      // 200 clocks to issue whatever its shape (bf16 4096 x 3072 x 768: 27.7 us, now 17.5).
+      auto mma_tiles = [&](auto half_kind) {
+        constexpr bool kHalf = decltype(half_kind)::value;
+        uint32_t s = 0, round = 0, nt = 0;
+        typename P::Tile t;
+        for (int tile = blockIdx.x; tile < n_tiles && *failed == 0; tile += gridDim.x, ++nt) {
+          prob.decode(tile, t);
+          const uint32_t acc = nt & 1, around = nt >> 1;
+          TC_PROF_NOW(w0);
+          if (around > 0 && !mbar_wait(&tempty_bar[acc], (around - 1) & 1)) {
+            *failed = 4;
             break;
           }
-          TC_PROF_ADD(m_full, w1);
+          TC_PROF_ADD(m_acc, w0);
           tc_fence_after();
-          if constexpr (X3 != 0) {
-            // a * b ~ a_hi * b_hi + a_lo * b_hi + a_hi * b_lo with x = x_hi + x_lo, x_hi exact
-            // in TF32: fp32-grade products out of three tensor-core passes
-            const uint32_t off = s * SL::kStageBytes;
-#pragma unroll
-            for (int j = 0; j < kBK / kUmmaK; ++j) {
-              const uint64_t ah = umma_desc_advance(a_desc0, off + j * a_jstep);
-              const uint64_t bh = umma_desc_advance(b_desc0, off + j * b_jstep);
-              const uint64_t al = umma_desc_advance(a_desc0, off + SL::kLoOffset + j * a_jstep);
-              const uint64_t bl = umma_desc_advance(b_desc0, off + SL::kLoOffset + j * b_jstep);
-              umma_tf32(d_tmem, al, bh, idesc, (k > k0 || j > 0) ? 1u : 0u);
-              umma_tf32(d_tmem, ah, bl, idesc, 1u);
-              umma_tf32(d_tmem, ah, bh, idesc, 1u);
+          const uint32_t d_tmem = tmem_base + acc * BN;
+          const int k0 = prob.k_begin(t), k1 = prob.k_end(t);
+          for (int k = k0; k < k1; k += KSUB) {
+            TC_PROF_NOW(w1);
+            if (!mbar_wait(X3 ? &split_bar[s] : &full_bar[s], round & 1)) {
+              *failed = 2;
+              break;
             }
-            umma_commit(&empty_bar[s]);
+            TC_PROF_ADD(m_full, w1);
+            tc_fence_after();
+            if constexpr (X3 != 0) {
+              // a * b ~ a_hi * b_hi + a_lo * b_hi + a_hi * b_lo with x = x_hi + x_lo, x_hi exact
+              // in TF32: fp32-grade products out of three tensor-core passes
+              const uint32_t off = s * SL::kStageBytes;
+  #pragma unroll
+              for (int j = 0; j < kBK / kUmmaK; ++j) {
+                const uint64_t ah = umma_desc_advance(a_desc0, off + j * a_jstep);
+                const uint64_t bh = umma_desc_advance(b_desc0, off + j * b_jstep);
+                const uint64_t al = umma_desc_advance(a_desc0, off + SL::kLoOffset + j * a_jstep);
+                const uint64_t bl = umma_desc_advance(b_desc0, off + SL::kLoOffset + j * b_jstep);
+                umma_tf32(d_tmem, al, bh, idesc, (k > k0 || j > 0) ? 1u : 0u);
+                umma_tf32(d_tmem, ah, bl, idesc, 1u);
+                umma_tf32(d_tmem, ah, bh, idesc, 1u);
+              }
+              umma_commit(&empty_bar[s]);
+              if (++s == NG) { s = 0; ++round; }
+              continue;
+            }
+            const int kn = min(KSUB, k1 - k);
+  #pragma unroll
+            for (int sub = 0; sub < KSUB; ++sub) {
+              if (sub >= kn) break;
+              const uint32_t off = (s * KSUB + sub) * SL::kStageBytes;
+  #pragma unroll
+              for (int j = 0; j < kBK / kUmmaK; ++j) {
+                const uint64_t ad = umma_desc_advance(a_desc0, off + j * a_jstep);
+                const uint64_t bd = umma_desc_advance(b_desc0, off + j * b_jstep);
+                const uint32_t accumulate = (k > k0 || sub > 0 || j > 0) ? 1u : 0u;
+                if constexpr (kHalf) umma_f16(d_tmem, ad, bd, idesc, accumulate);
+                else umma_tf32(d_tmem, ad, bd, idesc, accumulate);
+              }
+            }
+            umma_commit(&empty_bar[s]);  // frees the group once these MMAs have read it
             if (++s == NG) { s = 0; ++round; }
-            continue;
           }
-          const int kn = min(KSUB, k1 - k);
-#pragma unroll
-          for (int sub = 0; sub < KSUB; ++sub) {
-            if (sub >= kn) break;
-            const uint32_t off = (s * KSUB + sub) * SL::kStageBytes;
-#pragma unroll
-            for (int j = 0; j < kBK / kUmmaK; ++j) {
-              const uint64_t ad = umma_desc_advance(a_desc0, off + j * a_jstep);
-              const uint64_t bd = umma_desc_advance(b_desc0, off + j * b_jstep);
-              const uint32_t accumulate = (k > k0 || sub > 0 || j > 0) ? 1u : 0u;
-              if (bf16) umma_bf16(d_tmem, ad, bd, idesc, accumulate);
-              else umma_tf32(d_tmem, ad, bd, idesc, accumulate);
-            }
-          }
-          umma_commit(&empty_bar[s]);  // frees the group once these MMAs have read it
-          if (++s == NG) { s = 0; ++round; }
+          umma_commit(&tfull_bar[acc]);  // accumulator complete
         }
-        umma_commit(&tfull_bar[acc]);  // accumulator complete
-      }
+      };
+      if (half) mma_tiles(std::true_type{});
+      else mma_tiles(std::false_type{});
 #ifdef FLB200_TC_PROFILE
       TC_PROF_PUT(2, m_full); TC_PROF_PUT(3, m_acc); TC_PROF_PUT(4, clock64() - m_t0);
 #endif
@@ -492,9 +516,8 @@ tc_persistent_kernel(const __grid_constant__ CUtensorMap map_a,
 template <int BN>
 struct GemmProblem {
   static constexpr bool kWarpProducer = true;
-  static constexpr int kMinBlocks = 0;
-  static constexpr bool kBf16Capable = true;
-  int bf16;  // operands are bf16 (64 elements per stage), else fp32 read as TF32
+  static constexpr int kMinBlocks = 1;
+  int operand;  // kOperandTf32, or 16-bit (64 elements per stage)
   OperandCoords a, b;
   EpiloguePlan ep;
   int a_mn_major, b_mn_major;
@@ -532,7 +555,7 @@ struct GemmProblem {
     __syncwarp();
     // a K-major operand is one box, an MN-major one a box per 32 rows: copies [0, na) are A,
     // [na, na + nb) are B; copy i is issued by lane i / parts of producer warp i % parts
-    const int box_mn = bf16 ? 64 : 32, box_bytes = bf16 ? 8192 : kBK * 128;
+    const int box_mn = operand ? 64 : 32, box_bytes = operand ? 8192 : kBK * 128;
     const int na = a_mn_major && !a.mn_shift ? kBM / box_mn : 1;
     const int nb = b_mn_major && !b.mn_shift ? BN / box_mn : 1;  // grouped: one copy
     const int copy = lane * parts + part;
@@ -577,16 +600,17 @@ struct GemmProblem {
                                             char* a_dst, char* b_dst, int rank, int copy) const {
     // this CTA's 128 rows of A and its BN/2 columns of B; `copy` = which of the stage's copies
     // the calling lane issues
-    const int na = a_mn_major ? kBM / 32 : 1, nb = b_mn_major ? BN / 64 : 1;
+    const int box_mn = operand ? 64 : 32, box_bytes = operand ? 8192 : kBK * 128;
+    const int na = a_mn_major ? kBM / box_mn : 1, nb = b_mn_major ? (BN / 2) / box_mn : 1;
     if (copy < na) {
       int c[4];
-      operand_coords(a, t.m0 + 32 * copy, ls.a_lo, ls.a_hi, t.z, c);
-      tma_load_pair(ma, full_bar, a_dst + copy * (kBK * 128), a.rank, c);
+      operand_coords(a, t.m0 + box_mn * copy, ls.a_lo, ls.a_hi, t.z, c);
+      tma_load_pair(ma, full_bar, a_dst + copy * box_bytes, a.rank, c);
     } else if (copy < na + nb) {
       const int j = copy - na;
       int c[4];
-      operand_coords(b, t.n0 + rank * (BN / 2) + 32 * j, ls.b_lo, ls.b_hi, t.z, c);
-      tma_load_pair(mb, full_bar, b_dst + j * (kBK * 128), b.rank, c);
+      operand_coords(b, t.n0 + rank * (BN / 2) + box_mn * j, ls.b_lo, ls.b_hi, t.z, c);
+      tma_load_pair(mb, full_bar, b_dst + j * box_bytes, b.rank, c);
     }
     if (++ls.a_lo == a.k_inner) { ls.a_lo = 0; ++ls.a_hi; }
     if (++ls.b_lo == b.k_inner) { ls.b_lo = 0; ++ls.b_hi; }
@@ -595,171 +619,185 @@ struct GemmProblem {
     return t.n0 + c0 < N;
   }
 
-  // Rows 4k + lane / 8 (k = 0..7) of the warp's staged 32 x 32 chunk to a row-major output,
-  // 16 bytes per lane.  MODE 0: the values as staged; 1: + bias_n; 2: + bias_n, then gelu, the
-  // pre-activation kept in ep.pre when that is set.  STATS: per-channel sums of the stored
-  // values into row `group` of ep.stats.
-  template <int MODE, bool STATS>
-  __device__ __forceinline__ void staged_rows(float* stage, int lane, int m_first, float* out_row,
+  // How store() writes a chunk of 32 whole columns; decided once on the host (see set_store_mode),
+  // so that a chunk costs one test and not the chain of them.
+  enum {
+    kStoreGeneral = 0,  // element offsets of any kind, one row per lane
+    kStorePartial,      // split-K partial sums, row-major fp32
+    kStoreF32,          // row-major result: + 1 bias_n, + 2 bias_n and gelu, + 3 statistics too
+    kStoreF32Bias,
+    kStoreF32Gelu,
+    kStoreF32Stats,
+    kStoreBf16,
+    kStoreBf16Bias,
+    kStoreBf16Gelu,
+    kStoreBf16Stats,
+    kStoreF16,
+    kStoreF16Bias,
+    kStoreF16Gelu,
+    kStoreF16Stats,
+  };
+  int store_mode;
+
+  void set_store_mode() {
+    store_mode = kStoreGeneral;
+    if (splits > 1) {
+      if ((N & 3) == 0) store_mode = kStorePartial;
+      return;
+    }
+    if (ep.beta != 0.f || ep.n_div != 0 || ep.m_div != 0 || ep.n_stride != 1 ||
+        ep.bias_m != nullptr || (ep.m_stride & 3) != 0 || (ep.z_stride & 3) != 0 ||
+        (reinterpret_cast<uintptr_t>(ep.out) & 15) != 0)
+      return;
+    const int base = ep.out16 == 0 ? kStoreF32 : (ep.out16 == kOperandBf16 ? kStoreBf16 : kStoreF16);
+    store_mode = base + (ep.stats ? 3 : (ep.act ? 2 : (ep.bias_n ? 1 : 0)));
+  }
+
+  // The warp's staged 32 x 32 chunk to a row-major output of type T: lane i stores columns
+  // 4 (i % 8) .. + 3 of rows 4 k + i / 8, k = 0..7 (whole 128-byte rows of fp32, 64-byte rows of
+  // 16-bit values).  All eight reads are issued before the first store; `rows` < 32 only at the
+  // ragged end.  MODE 0: the values times alpha; 1: + bias_n; 2: + bias_n, then gelu, the
+  // pre-activation kept in ep.pre when that is set; 3: + bias_n, and per-channel sums of the
+  // stored values into row `group` of ep.stats.
+  template <typename T, int MODE>
+  __device__ __forceinline__ void staged_rows(float* stage, int lane, int rows, T* dst, T* pre,
                                               long long ld, int nb, long long group) const {
     float4 bq = make_float4(0.f, 0.f, 0.f, 0.f);
     if (MODE != 0 && ep.bias_n)
       bq = *reinterpret_cast<const float4*>(ep.bias_n + nb + 4 * (lane & 7));
-    float* pre_row = nullptr;
-    if (MODE == 2 && ep.pre)
-      pre_row = static_cast<float*>(ep.pre) + (out_row - ep.out);
-    EpiStats acc;
+    float4 val[8];
 #pragma unroll
-    for (int k = 0; k < 8; ++k) {
-      const int mr = m_first + 4 * k + (lane >> 3);
-      float4 val = epi_stage_read(stage, lane, k);
-      if (MODE != 0) { val.x += bq.x; val.y += bq.y; val.z += bq.z; val.w += bq.w; }
-      if (mr < M) {
-        const long long off = (long long)mr * ld;
-        if (MODE == 2) {
-          if (pre_row) *reinterpret_cast<float4*>(pre_row + off) = val;
-          val = make_float4(epi_gelu(val.x), epi_gelu(val.y), epi_gelu(val.z), epi_gelu(val.w));
+    for (int k = 0; k < 8; ++k) val[k] = epi_stage_read(stage, lane, k);
+    EpiStats acc;
+    const long long step = 4 * ld;
+    const int r0 = lane >> 3;
+    if (MODE == 0) {
+      if (rows >= 32) {
+#pragma unroll
+        for (int k = 0; k < 8; ++k, dst += step) epi_store4(dst, val[k]);
+      } else {
+#pragma unroll
+        for (int k = 0; k < 8; ++k, dst += step)
+          if (4 * k + r0 < rows) epi_store4(dst, val[k]);
+      }
+      return;
+    }
+#pragma unroll
+    for (int k = 0; k < 8; ++k, dst += step) {
+      float4 v = val[k];
+      v.x += bq.x; v.y += bq.y; v.z += bq.z; v.w += bq.w;
+      const bool live = 4 * k + r0 < rows;
+      if (MODE == 2) {
+        // the activation sees the value that the pre-activation tensor holds (rounded to T)
+        v = epi_round<T>(v);
+        if (pre) {
+          if (live) epi_store4(pre, v);
+          pre += step;
         }
-        *reinterpret_cast<float4*>(out_row + off) = val;
-        if (STATS) acc.add(val);
+        v = make_float4(epi_gelu(v.x), epi_gelu(v.y), epi_gelu(v.z), epi_gelu(v.w));
+      }
+      if (MODE == 3) {
+        v = epi_round<T>(v);
+        if (live) acc.add(v);
+      }
+      if (live) epi_store4(dst, v);
+    }
+    if (MODE == 3) acc.flush(ep.stats, group, N, nb, lane, stage);
+  }
+  template <typename T, int MODE>
+  __device__ __forceinline__ void staged_result(float* stage, int lane, int m_first, int nb,
+                                                const Tile& t) const {
+    const long long off = (long long)(m_first + (lane >> 3)) * ep.m_stride +
+                          (long long)t.z * ep.z_stride + nb + 4 * (lane & 7);
+    T* pre = MODE == 2 && ep.pre ? static_cast<T*>(ep.pre) + off : nullptr;
+    staged_rows<T, MODE>(stage, lane, M - m_first, reinterpret_cast<T*>(ep.out) + off, pre,
+                         ep.m_stride, nb, m_first >> 5);
+  }
+
+  // a row's 32 columns one by one: column tails, strided and accumulating 16-bit results
+  template <typename T>
+  __device__ __forceinline__ void store_16(long long m_off, int nb, float bm, const float* v) const {
+    T* out16 = reinterpret_cast<T*>(ep.out);
+#pragma unroll
+    for (int j = 0; j < 32; ++j) {
+      const int n = nb + j;
+      if (n < N) {
+        T* dst = out16 + m_off + epi_off(n, ep.n_div, ep.n_stride, ep.n_outer);
+        float r = ep.alpha * v[j] + bm + (ep.bias_n ? ep.bias_n[n] : 0.f);
+        if (ep.beta != 0.f) r += ep.beta * Num<T>::to_f(*dst);
+        *dst = Num<T>::from_f(r);
       }
     }
-    if (STATS) acc.flush(ep.stats, group, N, nb, lane, stage);
   }
 
   __device__ __forceinline__ void store(const Tile& t, int row, int c0, const float* v,
                                         float* stage, int lane) const {
     const int m = t.m0 + row;
     const int nb = t.n0 + c0;
-    // Row-major fp32 output with nothing but alpha to apply (a linear layer's product, a 1 x 1
-    // convolution over channels-last tensors, split-K partial sums): through the staging tile,
-    // whole 128-byte rows per store instruction.  The condition is uniform across the warp.
-    {
-      float* base = nullptr;
-      long long ld = 0;
-      float scale = 1.f;
-      if (splits > 1) {
-        if ((N & 3) == 0) {
-          base = partial + ((long long)(t.z * splits + t.split) * M) * N;
-          ld = N;
-        }
-      } else if (!ep.out_bf16 && ep.beta == 0.f && ep.n_div == 0 && ep.m_div == 0 &&
-                 ep.n_stride == 1 && ep.bias_m == nullptr &&
-                 (ep.m_stride & 3) == 0 && ((ep.z_stride * t.z) & 3) == 0 &&
-                 (reinterpret_cast<uintptr_t>(ep.out) & 15) == 0) {
-        base = ep.out + (long long)t.z * ep.z_stride;
-        ld = ep.m_stride;
-        scale = ep.alpha;
-      }
-      if (base != nullptr && nb + 32 <= N) {
+    if (store_mode != kStoreGeneral && nb + 32 <= N) {
+      // through the staging tile, whole row segments per store instruction
+      const int m_first = m - lane;  // first row of this warp
+      if (m_first >= M && store_mode != kStoreF32Stats && store_mode != kStoreBf16Stats &&
+          store_mode != kStoreF16Stats)
+        return;  // (statistics of a phantom tile are zeros that somebody adds up)
+      if (store_mode == kStorePartial || ep.alpha == 1.f) {
+        epi_stage_write(stage, lane, v);
+      } else {
         float w[32];
 #pragma unroll
-        for (int j = 0; j < 32; ++j) w[j] = scale * v[j];
+        for (int j = 0; j < 32; ++j) w[j] = ep.alpha * v[j];
         epi_stage_write(stage, lane, w);
-        const int m_first = m - lane;  // first row of this warp
-        // The flags are uniform across the grid: each combination has its own copy of the
-        // store loop, so the plain one stays eight loads followed by eight stores.
-        const bool fused = splits == 1 && (ep.bias_n != nullptr || ep.act != 0);
-        const bool stats = splits == 1 && ep.stats != nullptr;
-        float* out_row = base + nb + 4 * (lane & 7);
-        const long long group = (long long)(t.m0 >> 7) * 4 + (row >> 5);
-        if (!fused) {
-          if (!stats) staged_rows<0, false>(stage, lane, m_first, out_row, ld, nb, group);
-          else staged_rows<0, true>(stage, lane, m_first, out_row, ld, nb, group);
-        } else if (ep.act == 0) {
-          if (!stats) staged_rows<1, false>(stage, lane, m_first, out_row, ld, nb, group);
-          else staged_rows<1, true>(stage, lane, m_first, out_row, ld, nb, group);
-        } else {
-          if (!stats) staged_rows<2, false>(stage, lane, m_first, out_row, ld, nb, group);
-          else staged_rows<2, true>(stage, lane, m_first, out_row, ld, nb, group);
-        }
-        __syncwarp();  // the tile is rewritten by the next chunk
-        return;
       }
+      switch (store_mode) {
+        case kStorePartial: {
+          float* dst = partial + ((long long)(t.z * splits + t.split) * M + m_first + (lane >> 3)) * N +
+                       nb + 4 * (lane & 7);
+          staged_rows<float, 0>(stage, lane, M - m_first, dst, nullptr, N, nb, 0);
+          break;
+        }
+        case kStoreF32: staged_result<float, 0>(stage, lane, m_first, nb, t); break;
+        case kStoreF32Bias: staged_result<float, 1>(stage, lane, m_first, nb, t); break;
+        case kStoreF32Gelu: staged_result<float, 2>(stage, lane, m_first, nb, t); break;
+        case kStoreF32Stats: staged_result<float, 3>(stage, lane, m_first, nb, t); break;
+        case kStoreBf16: staged_result<__nv_bfloat16, 0>(stage, lane, m_first, nb, t); break;
+        case kStoreBf16Bias: staged_result<__nv_bfloat16, 1>(stage, lane, m_first, nb, t); break;
+        case kStoreBf16Gelu: staged_result<__nv_bfloat16, 2>(stage, lane, m_first, nb, t); break;
+        case kStoreBf16Stats: staged_result<__nv_bfloat16, 3>(stage, lane, m_first, nb, t); break;
+        case kStoreF16: staged_result<__half, 0>(stage, lane, m_first, nb, t); break;
+        case kStoreF16Bias: staged_result<__half, 1>(stage, lane, m_first, nb, t); break;
+        case kStoreF16Gelu: staged_result<__half, 2>(stage, lane, m_first, nb, t); break;
+        default: staged_result<__half, 3>(stage, lane, m_first, nb, t); break;
+      }
+      __syncwarp();  // the tile is rewritten by the next chunk
+      return;
     }
     if (m >= M) return;
     if (splits > 1) {
       float* dst = partial + ((long long)(t.z * splits + t.split) * M + m) * N + nb;
-      if (nb + 32 <= N && (N & 3) == 0) {
 #pragma unroll
-        for (int j = 0; j < 32; j += 4)
-          *reinterpret_cast<float4*>(dst + j) = make_float4(v[j], v[j + 1], v[j + 2], v[j + 3]);
-      } else {
-#pragma unroll
-        for (int j = 0; j < 32; ++j)
-          if (nb + j < N) dst[j] = v[j];
-      }
+      for (int j = 0; j < 32; ++j)
+        if (nb + j < N) dst[j] = v[j];
       return;
     }
     if (ep.m_valid != 0 && ep.m_div != 0 && (m % ep.m_div) >= ep.m_valid) return;
     const long long m_off =
         epi_off(m, ep.m_div, ep.m_stride, ep.m_outer) + (long long)t.z * ep.z_stride;
     const float bm = ep.bias_m ? ep.bias_m[m] : 0.f;
-    if (ep.out_bf16) {
-      __nv_bfloat16* outb = reinterpret_cast<__nv_bfloat16*>(ep.out);
-      if (ep.beta == 0.f && ep.n_div == 0 && ep.n_stride == 1 && nb + 32 <= N &&
-          ((m_off + nb) & 7) == 0 && (reinterpret_cast<uintptr_t>(ep.out) & 15) == 0) {
-        uint4* dst = reinterpret_cast<uint4*>(outb + m_off + nb);
-        uint4* dpre = ep.act && ep.pre
-                          ? reinterpret_cast<uint4*>(static_cast<__nv_bfloat16*>(ep.pre) + m_off + nb)
-                          : nullptr;
-        const float* bn = ep.bias_n ? ep.bias_n + nb : nullptr;
-#pragma unroll
-        for (int j = 0; j < 32; j += 8) {
-          float r[8];
-#pragma unroll
-          for (int q = 0; q < 8; ++q) r[q] = ep.alpha * v[j + q] + bm + (bn ? bn[j + q] : 0.f);
-          __nv_bfloat162 h[4];
-          if (ep.act) {
-            if (dpre) {
-#pragma unroll
-              for (int q = 0; q < 4; ++q) h[q] = __floats2bfloat162_rn(r[2 * q], r[2 * q + 1]);
-              dpre[j >> 3] = *reinterpret_cast<uint4*>(h);
-            }
-            // the activation sees the value the pre-activation tensor holds (rounded to bf16),
-            // as the unfused chain does
-#pragma unroll
-            for (int q = 0; q < 8; ++q) r[q] = epi_gelu(__bfloat162float(__float2bfloat16(r[q])));
-          }
-#pragma unroll
-          for (int q = 0; q < 4; ++q) h[q] = __floats2bfloat162_rn(r[2 * q], r[2 * q + 1]);
-          dst[j >> 3] = *reinterpret_cast<uint4*>(h);
-        }
-        return;
-      }
-#pragma unroll
-      for (int j = 0; j < 32; ++j) {
-        const int n = nb + j;
-        if (n < N) {
-          __nv_bfloat16* dst = outb + m_off + epi_off(n, ep.n_div, ep.n_stride, ep.n_outer);
-          float r = ep.alpha * v[j] + bm + (ep.bias_n ? ep.bias_n[n] : 0.f);
-          if (ep.beta != 0.f) r += ep.beta * __bfloat162float(*dst);
-          *dst = __float2bfloat16(r);
-        }
-      }
+    if (ep.out16) {
+      if (ep.out16 == kOperandBf16) store_16<__nv_bfloat16>(m_off, nb, bm, v);
+      else store_16<__half>(m_off, nb, bm, v);
       return;
     }
     const bool simple = ep.beta == 0.f && ep.n_div == 0;
-    if (simple && nb + 32 <= N && ep.bias_n != nullptr) {
-      // strided columns with a per-column bias (convolution output planes)
+    if (simple && nb + 32 <= N) {
+      // strided columns (convolution output planes): the rows of a warp are contiguous
       float* dst = ep.out + m_off + (long long)nb * ep.n_stride;
       const long long ns = ep.n_stride;
-      const float* bn = ep.bias_n + nb;
+      if (ep.bias_n != nullptr) {
+        const float* bn = ep.bias_n + nb;
 #pragma unroll
-      for (int j = 0; j < 32; ++j) dst[j * ns] = ep.alpha * v[j] + bm + bn[j];
-      return;
-    }
-    if (simple && nb + 32 <= N) {
-      float* dst = ep.out + m_off + (long long)nb * ep.n_stride;
-      if (ep.n_stride == 1 && ((m_off + nb) & 3) == 0 &&
-          (reinterpret_cast<uintptr_t>(ep.out) & 15) == 0) {
-#pragma unroll
-        for (int j = 0; j < 32; j += 4)
-          *reinterpret_cast<float4*>(dst + j) =
-              make_float4(ep.alpha * v[j] + bm, ep.alpha * v[j + 1] + bm,
-                          ep.alpha * v[j + 2] + bm, ep.alpha * v[j + 3] + bm);
+        for (int j = 0; j < 32; ++j) dst[j * ns] = ep.alpha * v[j] + bm + bn[j];
       } else {
-        const long long ns = ep.n_stride;
 #pragma unroll
         for (int j = 0; j < 32; ++j) dst[j * ns] = ep.alpha * v[j] + bm;
       }

@@ -65,8 +65,7 @@ tc_pair_kernel(const __grid_constant__ CUtensorMap map_a,
   static_assert(STAGES % KSUB == 0, "ring must be whole groups");
   constexpr int NG = STAGES / KSUB;
   extern __shared__ char smem_raw[];
-  char* tiles = reinterpret_cast<char*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) &
-                                        ~static_cast<uintptr_t>(1023));
+  char* tiles = smem_raw + ((1024u - (smem_u32(smem_raw) & 1023u)) & 1023u);  // (tc_kernel.cuh)
   uint64_t* full_bar = reinterpret_cast<uint64_t*>(tiles + SL::kTileBytes);
   uint64_t* empty_bar = full_bar + STAGES;
   uint64_t* tfull_bar = empty_bar + STAGES;
@@ -165,57 +164,70 @@ tc_pair_kernel(const __grid_constant__ CUtensorMap map_a,
     }
   } else if (warp == 1) {
     if (lane == 0 && rank == 0) {
-      const uint32_t idesc = umma_idesc_tf32_pair(BN, prob.a_mn_major, prob.b_mn_major);
-      // descriptors of the ring's first stage; every MMA offsets them
+      const bool half = prob.operand != kOperandTf32;
+      const uint32_t idesc =
+          half ? umma_idesc_f16_pair(prob.operand, BN, prob.a_mn_major, prob.b_mn_major)
+               : umma_idesc_tf32_pair(BN, prob.a_mn_major, prob.b_mn_major);
+      // descriptors of the ring's first stage; every MMA offsets them (tc_kernel.cuh)
+      const uint32_t mn_lbo = half ? 8192 : kBK * 128, mn_sbo = half ? 1024 : 512;
+      const uint32_t mn_step = half ? 2048 : 1024, mn_layout = half ? 2 : 1;
       const uint32_t ring = smem_u32(tiles);
-      const uint64_t a_desc0 = prob.a_mn_major ? umma_desc(ring, kBK * 128, 512, 1)
+      const uint64_t a_desc0 = prob.a_mn_major ? umma_desc(ring, mn_lbo, mn_sbo, mn_layout)
                                                : umma_desc(ring, 16, 1024, 2);
       const uint64_t b_desc0 = prob.b_mn_major
-                                   ? umma_desc(ring + SL::kABytes, kBK * 128, 512, 1)
+                                   ? umma_desc(ring + SL::kABytes, mn_lbo, mn_sbo, mn_layout)
                                    : umma_desc(ring + SL::kABytes, 16, 1024, 2);
-      const uint32_t a_jstep = prob.a_mn_major ? 1024 : 32, b_jstep = prob.b_mn_major ? 1024 : 32;
-      uint32_t s = 0, round = 0, nt = 0;
-      typename P::Tile t;
+      const uint32_t a_jstep = prob.a_mn_major ? mn_step : 32;
+      const uint32_t b_jstep = prob.b_mn_major ? mn_step : 32;
       TC_PROF_VAR(m_full);
       TC_PROF_VAR(m_acc);
       TC_PROF_NOW(m_t0);
-      for (int tile = pair; tile < n_tiles && *failed == 0; tile += n_pairs, ++nt) {
-        prob.decode_pair(tile, 0, t);
-        const uint32_t acc = nt & 1, around = nt >> 1;
-        TC_PROF_NOW(w0);
-        if (around > 0 && !mbar_wait(&tempty_bar[acc], (around - 1) & 1)) {
-          *failed = 4;
-          break;
-        }
-        TC_PROF_ADD(m_acc, w0);
-        tc_fence_after();
-        const uint32_t d_tmem = tmem_base + acc * BN;
-        const int k0 = prob.k_begin(t), k1 = prob.k_end(t);
-        for (int k = k0; k < k1; k += KSUB) {
-          const int kn = min(KSUB, k1 - k);
-          TC_PROF_NOW(w1);
-          if (!mbar_wait(&full_bar[s], round & 1)) {
-            *failed = 2;
+      auto mma_tiles = [&](auto half_kind) {  // one copy per operand kind (see tc_kernel.cuh)
+        constexpr bool kHalf = decltype(half_kind)::value;
+        uint32_t s = 0, round = 0, nt = 0;
+        typename P::Tile t;
+        for (int tile = pair; tile < n_tiles && *failed == 0; tile += n_pairs, ++nt) {
+          prob.decode_pair(tile, 0, t);
+          const uint32_t acc = nt & 1, around = nt >> 1;
+          TC_PROF_NOW(w0);
+          if (around > 0 && !mbar_wait(&tempty_bar[acc], (around - 1) & 1)) {
+            *failed = 4;
             break;
           }
-          TC_PROF_ADD(m_full, w1);
+          TC_PROF_ADD(m_acc, w0);
           tc_fence_after();
-#pragma unroll
-          for (int sub = 0; sub < KSUB; ++sub) {
-            if (sub >= kn) break;
-            const uint32_t off = (s * KSUB + sub) * SL::kStageBytes;
-#pragma unroll
-            for (int j = 0; j < kBK / kUmmaK; ++j) {
-              const uint64_t ad = umma_desc_advance(a_desc0, off + j * a_jstep);
-              const uint64_t bd = umma_desc_advance(b_desc0, off + j * b_jstep);
-              umma_tf32_pair(d_tmem, ad, bd, idesc, (k > k0 || sub > 0 || j > 0) ? 1u : 0u);
+          const uint32_t d_tmem = tmem_base + acc * BN;
+          const int k0 = prob.k_begin(t), k1 = prob.k_end(t);
+          for (int k = k0; k < k1; k += KSUB) {
+            const int kn = min(KSUB, k1 - k);
+            TC_PROF_NOW(w1);
+            if (!mbar_wait(&full_bar[s], round & 1)) {
+              *failed = 2;
+              break;
             }
+            TC_PROF_ADD(m_full, w1);
+            tc_fence_after();
+  #pragma unroll
+            for (int sub = 0; sub < KSUB; ++sub) {
+              if (sub >= kn) break;
+              const uint32_t off = (s * KSUB + sub) * SL::kStageBytes;
+  #pragma unroll
+              for (int j = 0; j < kBK / kUmmaK; ++j) {
+                const uint64_t ad = umma_desc_advance(a_desc0, off + j * a_jstep);
+                const uint64_t bd = umma_desc_advance(b_desc0, off + j * b_jstep);
+                const uint32_t accumulate = (k > k0 || sub > 0 || j > 0) ? 1u : 0u;
+                if constexpr (kHalf) umma_f16_pair(d_tmem, ad, bd, idesc, accumulate);
+                else umma_tf32_pair(d_tmem, ad, bd, idesc, accumulate);
+              }
+            }
+            umma_commit_pair(&empty_bar[s]);  // frees the group in both CTAs
+            if (++s == NG) { s = 0; ++round; }
           }
-          umma_commit_pair(&empty_bar[s]);  // frees the group in both CTAs
-          if (++s == NG) { s = 0; ++round; }
+          umma_commit_pair(&tfull_bar[acc]);  // both CTAs' halves of the accumulator complete
         }
-        umma_commit_pair(&tfull_bar[acc]);  // both CTAs' halves of the accumulator complete
-      }
+      };
+      if (half) mma_tiles(std::true_type{});
+      else mma_tiles(std::false_type{});
 #ifdef FLB200_TC_PROFILE
       TC_PROF_PUT(2, m_full); TC_PROF_PUT(3, m_acc); TC_PROF_PUT(4, clock64() - m_t0);
 #endif

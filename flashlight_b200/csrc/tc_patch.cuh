@@ -51,8 +51,8 @@ template <int BN>
 struct PatchConvProblem {
   static constexpr bool kWarpProducer = false;
   static constexpr int kMinBlocks = 1;
-  static constexpr bool kBf16Capable = false;
   int a_mn_major, b_mn_major;  // 0, 0
+  int operand;
   // patch geometry (all powers of two, NB * PH * QW == 128)
   int QW, PH, NB, qw_shift, ph_shift;
   int tiles_q, tiles_p, tiles_b, tiles_n;
@@ -159,16 +159,15 @@ struct PatchConvProblem {
   __device__ __forceinline__ bool chunk_live(const Tile& t, int c0) const {
     return t.n0 + c0 < n_out;
   }
-  // output address of row `r` of the tile (channels-last output, class offsets applied), or
-  // null for a row outside the image
-  __device__ __forceinline__ float* cl_row(const Tile& t, int r) const {
+  // pixel index (in the whole output) of row `r` of the tile, class offsets applied, or -1 for a
+  // row outside the image
+  __device__ __forceinline__ long long cl_pixel(const Tile& t, int r) const {
     const int q = t.q0 + (r & (QW - 1));
     const int p = t.p0 + ((r >> qw_shift) & (PH - 1));
     const int img = t.b0 + (r >> (qw_shift + ph_shift));
-    if (q >= pix_w || p >= pix_h || img >= images) return nullptr;
+    if (q >= pix_w || p >= pix_h || img >= images) return -1;
     const int oh_add = fill_cell ? 0 : cls[t.c].oh_add, ow_add = fill_cell ? 0 : cls[t.c].ow_add;
-    return out + (((long long)img * out_H + p * oh_mul + oh_add) * out_W + q * ow_mul + ow_add) *
-                     out_C;
+    return ((long long)img * out_H + p * oh_mul + oh_add) * out_W + q * ow_mul + ow_add;
   }
   // Pixel rows 4k + lane / 8 (k = 0..7) of the warp's staged chunk, 16 bytes per lane, bias
   // added; STATS (uniform across the grid, so a copy of the loop each): per-channel sums of
@@ -181,15 +180,21 @@ struct PatchConvProblem {
     float4 bq = make_float4(0.f, 0.f, 0.f, 0.f);
     if (bias) bq = *reinterpret_cast<const float4*>(bias + nb + 4 * (lane & 7));
     const int r_first = row - lane;
+    // every lane works out the address of its own row; the rows it stores come by shuffle
+    const long long own = cl_pixel(t, row);
+    float4 val[8];
+#pragma unroll
+    for (int k = 0; k < 8; ++k) val[k] = epi_stage_read(stage, lane, k);
     EpiStats acc;
 #pragma unroll
     for (int k = 0; k < 8; ++k) {
-      float* dst = cl_row(t, r_first + 4 * k + (lane >> 3));
-      float4 val = epi_stage_read(stage, lane, k);
-      val.x += bq.x; val.y += bq.y; val.z += bq.z; val.w += bq.w;
-      if (dst) {
-        *reinterpret_cast<float4*>(dst + nb + 4 * (lane & 7)) = val;
-        if (STATS) acc.add(val);
+      const long long pix = __shfl_sync(0xffffffffu, own, 4 * k + (lane >> 3));
+      float4 v = val[k];
+      v.x += bq.x; v.y += bq.y; v.z += bq.z; v.w += bq.w;
+      if (pix >= 0) {
+        float* dst = out + pix * out_C + nb + 4 * (lane & 7);
+        *reinterpret_cast<float4*>(dst) = v;
+        if (STATS) acc.add(v);
         if (FILL) {
           // this pixel owns its whole oh_mul x ow_mul cell: the other pixels receive zeros
           const int r = r_first + 4 * k + (lane >> 3);
@@ -197,8 +202,8 @@ struct PatchConvProblem {
           const int oh0 = (t.p0 + ((r >> qw_shift) & (PH - 1))) * oh_mul;
           for (int a = 0; a < oh_mul && oh0 + a < out_H; ++a)
             for (int b = a == 0 ? 1 : 0; b < ow_mul && ow0 + b < out_W; ++b)
-              *reinterpret_cast<float4*>(dst + ((long long)a * out_W + b) * out_C + nb +
-                                         4 * (lane & 7)) = make_float4(0.f, 0.f, 0.f, 0.f);
+              *reinterpret_cast<float4*>(dst + ((long long)a * out_W + b) * out_C) =
+                  make_float4(0.f, 0.f, 0.f, 0.f);
         }
       }
     }
@@ -307,8 +312,8 @@ template <int BN>
 struct PatchWgradProblem {
   static constexpr bool kWarpProducer = true;
   static constexpr int kMinBlocks = 1;
-  static constexpr bool kBf16Capable = false;
   int a_mn_major, b_mn_major;  // 1, 1
+  int operand;
   int QW, PH;                  // 32-pixel patch: QW * PH == 32
   int tiles_q, tiles_p, images;
   int tiles_m, tiles_n, M, N;  // M = output channels, N = input channels
