@@ -8,12 +8,16 @@
 // dilation (dx,dy), groups.
 //
 // GEMM views (per group):
-//   forward   M = Cout/g, N = batch*Ho*Wo, K = (C/g)*kH*kW
-//   bwd data  M = C/g,    N = batch*H*W,   K = (Cout/g)*kH*kW
-//   bwd filt  M = Cout/g, N = (C/g)*kH*kW, K = batch*Ho*Wo   (split-K)
-// STRICT mode: the fp32-FMA kernel of simt_gemm.cuh with im2col loaders below.
+//   forward   M = batch*Ho*Wo, N = Cout/g,        K = (C/g)*kH*kW
+//   bwd data  M = batch*H*W,   N = C/g,           K = (Cout/g)*kH*kW
+//   bwd filt  M = Cout/g,      N = (C/g)*kH*kW,   K = batch*Ho*Wo   (split-K)
+// STRICT mode: the fp32-FMA kernel of simt_gemm.cuh with the loaders below.  Channels-last images
+// of a multiple of 4 channels are read in 16-byte runs of channels, K ordered (tap, channel),
+// against a filter repacked to that order; anything else element by element with the lanes along
+// the pixels, K in the filter's own order (channel, tap).
 // TF32 mode: shapes covered by the tensor-core kernels go to tc_conv, the rest
 // fall through to the fp32 kernel.
+#include "filter_permute.cuh"
 #include "simt_gemm.cuh"
 #include "tc_conv.cuh"
 #include "tc_gemm.cuh"
@@ -61,181 +65,354 @@ int make_conv_geo(const char* name, const flb200_conv2d_desc* d, ConvGeo* g) {
 
 namespace {
 
-// ------------------------------------------------------------- forward
-// B(k=(ci,r,s), n=(img,p,q)) = x[img][g*Cg+ci][p*sy-py+r*dy][q*sx-px+s*dx]
-struct FpropB {
-  static constexpr bool kAlongK = false;
-  const float* x;
+// Pixel index and filter tap of the two image views: the forward pass reads x at
+// (p*sy - py + r*dy, q*sx - px + s*dx), backward-data reads dy where h + py - r*dy and
+// w + px - s*dx divide by the stride.
+struct PixelRow { long long base; int h0, w0; };
+
+// ---- images read channel-run-wise (channels-last, a multiple of 4 channels per group)
+template <bool DGRAD>
+struct ImageVec {
+  static constexpr int kKind = kVecK;
+  const float* p;
   ConvGeo g;
-  long long n_total;
-  struct Row { long long base; int h0, w0; };
-  struct Kk { int off, dh, dw; };
+  int n_total, c4;  // pixels, 4-channel runs per tap
+  typedef PixelRow Row;
+  struct Iter { int cq, r, s; };
+  __device__ const float* base() const { return p; }
   __device__ Row row(int n, int z) const {
     if (n >= n_total) return Row{-1, 0, 0};
-    const int img = n / g.HoWo, pq = n - img * g.HoWo;
-    const int p = pq / g.Wo, q = pq - p * g.Wo;
-    return Row{(long long)img * g.C * g.HW + (long long)z * g.Cg * g.x_cs, p * g.sy - g.py,
+    if (DGRAD) {
+      const int img = n / g.HW, hw = n - img * g.HW, h = hw / g.W, w = hw - h * g.W;
+      return Row{(long long)img * g.Cout * g.HoWo + (long long)z * g.Coutg, h + g.py, w + g.px};
+    }
+    const int img = n / g.HoWo, pq = n - img * g.HoWo, y = pq / g.Wo, q = pq - y * g.Wo;
+    return Row{(long long)img * g.C * g.HW + (long long)z * g.Cg, y * g.sy - g.py, q * g.sx - g.px};
+  }
+  __device__ Iter iter(int k, int) const {
+    const int run = k >> 2, tap = run / c4, r = tap / g.kW;
+    return Iter{run - tap * c4, r, tap - r * g.kW};
+  }
+  __device__ void advance(Iter& it) const {
+    it.cq += kBKf / 4;
+    while (it.cq >= c4) {
+      it.cq -= c4;
+      if (++it.s == g.kW) { it.s = 0; ++it.r; }
+    }
+  }
+  __device__ const float* at(const Row& row, const Iter& it) const {
+    if (row.base < 0) return nullptr;
+    if (DGRAD) {
+      const int th = row.h0 - it.r * g.dy, tw = row.w0 - it.s * g.dx;
+      if (th < 0 || tw < 0) return nullptr;
+      int y = th, q = tw;
+      if (g.sy != 1) { y = th / g.sy; if (y * g.sy != th) return nullptr; }
+      if (g.sx != 1) { q = tw / g.sx; if (q * g.sx != tw) return nullptr; }
+      if (y >= g.Ho || q >= g.Wo) return nullptr;
+      return p + row.base + (long long)(y * g.Wo + q) * g.Cout + 4 * it.cq;
+    }
+    const int h = row.h0 + it.r * g.dy, w = row.w0 + it.s * g.dx;
+    if (h < 0 || h >= g.H || w < 0 || w >= g.W) return nullptr;
+    return p + row.base + (long long)(h * g.W + w) * g.C + 4 * it.cq;
+  }
+};
+
+// ---- images read element by element, K = (channel, tap)
+template <bool DGRAD>
+struct ImageElem {
+  static constexpr int kKind = kElemRows;
+  const float* p;
+  ConvGeo g;
+  int n_total;
+  typedef PixelRow Row;
+  struct Kk { int off, dh, dw; };
+  __device__ const float* base() const { return p; }
+  __device__ Row row(int n, int z) const {
+    if (n >= n_total) return Row{-1, 0, 0};
+    if (DGRAD) {
+      const int img = n / g.HW, hw = n - img * g.HW, h = hw / g.W, w = hw - h * g.W;
+      return Row{(long long)img * g.Cout * g.HoWo + (long long)z * g.Coutg * g.y_cs, h + g.py, w + g.px};
+    }
+    const int img = n / g.HoWo, pq = n - img * g.HoWo, y = pq / g.Wo, q = pq - y * g.Wo;
+    return Row{(long long)img * g.C * g.HW + (long long)z * g.Cg * g.x_cs, y * g.sy - g.py,
                q * g.sx - g.px};
   }
-  __device__ Kk kk(long long k, int) const {
-    const int ki = (int)k;
-    const int ci = ki / g.RS, rs = ki - ci * g.RS;
-    const int r = rs / g.kW, s = rs - r * g.kW;
-    return Kk{ci * g.x_cs, r * g.dy, s * g.dx};
+  __device__ Kk kk(int k, int) const {
+    const int c = k / g.RS, rs = k - c * g.RS, r = rs / g.kW, s = rs - r * g.kW;
+    return Kk{c * (DGRAD ? g.y_cs : g.x_cs), r * g.dy, s * g.dx};
   }
-  __device__ float load(const Row& r, const Kk& k) const {
-    const int h = r.h0 + k.dh, w = r.w0 + k.dw;
-    if (r.base < 0 || h < 0 || h >= g.H || w < 0 || w >= g.W) return 0.f;
-    return x[r.base + k.off + (long long)(h * g.W + w) * g.x_ps];
-  }
-};
-
-struct FpropEpilogue {
-  float* y;
-  const float* bias;
-  ConvGeo g;
-  struct Row { long long off; float b; };
-  struct Col { long long off; };
-  __device__ Row row(int m, int z) const {
-    const int co = z * g.Coutg + m;
-    return Row{(long long)co * g.y_cs, bias ? bias[co] : 0.f};
-  }
-  __device__ Col col(int n, int) const {
-    const int img = n / g.HoWo, pq = n - img * g.HoWo;
-    return Col{(long long)img * g.Cout * g.HoWo + (long long)pq * g.y_ps};
-  }
-  __device__ void store(const Row& r, const Col& c, float acc) const {
-    y[r.off + c.off] = acc + r.b;
+  __device__ const float* at(const Row& row, const Kk& k) const {
+    if (row.base < 0) return nullptr;
+    if (DGRAD) {
+      const int th = row.h0 - k.dh, tw = row.w0 - k.dw;
+      if (th < 0 || tw < 0) return nullptr;
+      int y = th, q = tw;
+      if (g.sy != 1) { y = th / g.sy; if (y * g.sy != th) return nullptr; }
+      if (g.sx != 1) { q = tw / g.sx; if (q * g.sx != tw) return nullptr; }
+      if (y >= g.Ho || q >= g.Wo) return nullptr;
+      return p + row.base + k.off + (long long)(y * g.Wo + q) * g.y_ps;
+    }
+    const int h = row.h0 + k.dh, w = row.w0 + k.dw;
+    if (h < 0 || h >= g.H || w < 0 || w >= g.W) return nullptr;
+    return p + row.base + k.off + (long long)(h * g.W + w) * g.x_ps;
   }
 };
 
-// ------------------------------------------------------- backward data
-// A(m=ci, k=(co,r,s)) = w[g*Coutg+co][ci][r][s]
-struct DgradA {
-  static constexpr bool kAlongK = true;
+// ---- filters.  The filter in the K order of the image view: row = co (forward) or ci
+// (backward-data), tap_major: k = (tap, channel) else (channel, tap).
+struct FilterElem {
+  static constexpr int kKind = kElemK;
   const float* w;
   ConvGeo g;
+  int dgrad, tap_major, rows;
   struct Row { long long off; };
   struct Kk { long long off; };
-  __device__ Row row(int m, int z) const {
-    if (m >= g.Cg) return Row{-1};
-    return Row{(long long)m * g.RS + (long long)z * g.Coutg * g.Cg * g.RS};
+  __device__ const float* base() const { return w; }
+  __device__ Row row(int r, int z) const {
+    if (r >= rows) return Row{-1};
+    const long long group = (long long)z * g.Coutg * g.Cg * g.RS;
+    return Row{group + (long long)r * g.RS * (dgrad ? 1 : g.Cg)};
   }
-  __device__ Kk kk(long long k, int) const {
-    const int ki = (int)k;
-    const int co = ki / g.RS, rs = ki - co * g.RS;
-    return Kk{(long long)co * g.Cg * g.RS + rs};
+  __device__ Kk kk(int k, int) const {
+    const int ch = dgrad ? g.Coutg : g.Cg;
+    const int c = tap_major ? k % ch : k / g.RS, tap = tap_major ? k / ch : k - c * g.RS;
+    return Kk{(long long)c * g.RS * (dgrad ? g.Cg : 1) + tap};
   }
-  __device__ float load(const Row& r, const Kk& k) const {
-    return r.off >= 0 ? w[r.off + k.off] : 0.f;
+  __device__ const float* at(const Row& r, const Kk& k) const {
+    return r.off >= 0 ? w + r.off + k.off : nullptr;
   }
 };
+// ---- image-shaped results: rows are pixels, columns channels
+struct PixelOut {
+  float* out;
+  const float* bias;
+  float alpha, beta;
+  int along_m, vec;
+  long long image, chan, pix;  // element strides
+  int pixels, per_group;       // pixels per image, columns per group
+  __device__ long long row(int m, int) const {
+    const int img = m / pixels;
+    return img * image + (m - img * pixels) * pix;
+  }
+  __device__ long long col(int n, int z) const { return (long long)(z * per_group + n) * chan; }
+  __device__ int bias_at(int n, int z) const { return z * per_group + n; }
+};
+PixelOut pixel_out(float* out, const float* bias, const ConvGeo& g, bool dgrad) {
+  PixelOut o{out, bias, 1.f, 0.f, 0, 0, 0, 0, 0, 0, 0};
+  o.image = dgrad ? (long long)g.C * g.HW : (long long)g.Cout * g.HoWo;
+  o.chan = dgrad ? g.x_cs : g.y_cs;
+  o.pix = dgrad ? g.x_ps : g.y_ps;
+  o.pixels = dgrad ? g.HW : g.HoWo;
+  o.per_group = dgrad ? g.Cg : g.Coutg;
+  o.along_m = o.pix == 1;
+  o.vec = o.chan == 1 && o.per_group % 4 == 0 && o.pix % 4 == 0 && aligned16(out);
+  return o;
+}
 
-// B(k=(co,r,s), n=(img,h,w)) = gy[img][g*Coutg+co][p][q] with p*sy = h+py-r*dy, q*sx = w+px-s*dx
-struct DgradB {
-  static constexpr bool kAlongK = false;
-  const float* gy;
+// ---- backward filter: K = pixels of the output
+// x around output pixel k, 16-byte runs of channels, n = (tap, channel)
+struct WindowVec {
+  static constexpr int kKind = kVecRow;
+  const float* x;
   ConvGeo g;
-  long long n_total;
-  struct Row { long long base; int hh, ww; };
-  struct Kk { int off, dh, dw; };
+  int n_total;
+  struct Row { int off, dh, dw; };
+  struct Iter { long long img; int y, q; };
+  __device__ const float* base() const { return x; }
   __device__ Row row(int n, int z) const {
     if (n >= n_total) return Row{-1, 0, 0};
-    const int img = n / g.HW, hw = n - img * g.HW;
-    const int h = hw / g.W, w = hw - h * g.W;
-    return Row{(long long)img * g.Cout * g.HoWo + (long long)z * g.Coutg * g.y_cs, h + g.py,
-               w + g.px};
+    const int tap = n / g.Cg, c = n - tap * g.Cg, r = tap / g.kW, s = tap - r * g.kW;
+    return Row{z * g.Cg + c, r * g.dy - g.py, s * g.dx - g.px};
   }
-  __device__ Kk kk(long long k, int) const {
-    const int ki = (int)k;
-    const int co = ki / g.RS, rs = ki - co * g.RS;
-    const int r = rs / g.kW, s = rs - r * g.kW;
-    return Kk{co * g.y_cs, r * g.dy, s * g.dx};
+  __device__ Iter iter(int k, int) const {
+    const int img = k / g.HoWo, pq = k - img * g.HoWo, y = pq / g.Wo;
+    return Iter{(long long)img * g.C * g.HW, y, pq - y * g.Wo};
   }
-  __device__ float load(const Row& r, const Kk& k) const {
-    const int th = r.hh - k.dh, tw = r.ww - k.dw;
-    if (r.base < 0 || th < 0 || tw < 0) return 0.f;
-    int p = th, q = tw;
-    if (g.sy != 1) { p = th / g.sy; if (p * g.sy != th) return 0.f; }
-    if (g.sx != 1) { q = tw / g.sx; if (q * g.sx != tw) return 0.f; }
-    if (p >= g.Ho || q >= g.Wo) return 0.f;
-    return gy[r.base + k.off + (long long)(p * g.Wo + q) * g.y_ps];
+  __device__ void advance(Iter& it) const {
+    it.q += kBKf;
+    while (it.q >= g.Wo) {
+      it.q -= g.Wo;
+      if (++it.y == g.Ho) { it.y = 0; it.img += (long long)g.C * g.HW; }
+    }
   }
-};
-
-struct DgradEpilogue {
-  float* gx;
-  ConvGeo g;
-  struct Row { long long off; };
-  struct Col { long long off; };
-  __device__ Row row(int m, int z) const { return Row{((long long)z * g.Cg + m) * g.x_cs}; }
-  __device__ Col col(int n, int) const {
-    const int img = n / g.HW, hw = n - img * g.HW;
-    return Col{(long long)img * g.C * g.HW + (long long)hw * g.x_ps};
-  }
-  __device__ void store(const Row& r, const Col& c, float acc) const { gx[r.off + c.off] = acc; }
-};
-
-// ----------------------------------------------------- backward filter
-// A(m=co, k=(img,p,q)) = gy[img][g*Coutg+co][p][q]
-struct WgradA {
-  static constexpr bool kAlongK = true;
-  const float* gy;
-  ConvGeo g;
-  struct Row { long long off; };
-  struct Kk { long long off; };
-  __device__ Row row(int m, int z) const {
-    if (m >= g.Coutg) return Row{-1};
-    return Row{((long long)z * g.Coutg + m) * g.y_cs};
-  }
-  __device__ Kk kk(long long k, int) const {
-    const long long img = k / g.HoWo;
-    const int pq = (int)(k - img * g.HoWo);
-    return Kk{img * g.Cout * g.HoWo + (long long)pq * g.y_ps};
-  }
-  __device__ float load(const Row& r, const Kk& k) const {
-    return r.off >= 0 ? gy[r.off + k.off] : 0.f;
+  __device__ const float* at(const Row& r, const Iter& it) const {
+    const int h = it.y * g.sy + r.dh, w = it.q * g.sx + r.dw;
+    if (r.off < 0 || h < 0 || h >= g.H || w < 0 || w >= g.W) return nullptr;
+    return x + it.img + (long long)(h * g.W + w) * g.C + r.off;
   }
 };
-
-// B(k=(img,p,q), n=(ci,r,s)) = x[img][g*Cg+ci][p*sy-py+r*dy][q*sx-px+s*dx]
-struct WgradB {
-  static constexpr bool kAlongK = true;
+// element by element, n = (channel, tap)
+struct WindowElem {
+  static constexpr int kKind = kElemK;
   const float* x;
   ConvGeo g;
   int n_total;
   struct Row { long long off; int dh, dw; };
   struct Kk { long long base; int h0, w0; };
+  __device__ const float* base() const { return x; }
   __device__ Row row(int n, int z) const {
     if (n >= n_total) return Row{-1, 0, 0};
-    const int ci = n / g.RS, rs = n - ci * g.RS;
-    const int r = rs / g.kW, s = rs - r * g.kW;
-    return Row{((long long)z * g.Cg + ci) * g.x_cs, r * g.dy - g.py, s * g.dx - g.px};
+    const int c = n / g.RS, rs = n - c * g.RS, r = rs / g.kW, s = rs - r * g.kW;
+    return Row{((long long)z * g.Cg + c) * g.x_cs, r * g.dy - g.py, s * g.dx - g.px};
   }
-  __device__ Kk kk(long long k, int) const {
-    const long long img = k / g.HoWo;
-    const int pq = (int)(k - img * g.HoWo);
-    const int p = pq / g.Wo, q = pq - p * g.Wo;
-    return Kk{img * g.C * g.HW, p * g.sy, q * g.sx};
+  __device__ Kk kk(int k, int) const {
+    const int img = k / g.HoWo, pq = k - img * g.HoWo, y = pq / g.Wo, q = pq - y * g.Wo;
+    return Kk{(long long)img * g.C * g.HW, y * g.sy, q * g.sx};
   }
-  __device__ float load(const Row& r, const Kk& k) const {
+  __device__ const float* at(const Row& r, const Kk& k) const {
     const int h = k.h0 + r.dh, w = k.w0 + r.dw;
-    if (r.off < 0 || h < 0 || h >= g.H || w < 0 || w >= g.W) return 0.f;
-    return x[k.base + r.off + (long long)(h * g.W + w) * g.x_ps];
+    if (r.off < 0 || h < 0 || h >= g.H || w < 0 || w >= g.W) return nullptr;
+    return x + k.base + r.off + (long long)(h * g.W + w) * g.x_ps;
   }
 };
-
-struct WgradEpilogue {
-  float* gw;
+// dy element by element, lanes along the pixels
+struct GradElem {
+  static constexpr int kKind = kElemK;
+  const float* gy;
   ConvGeo g;
   struct Row { long long off; };
-  struct Col { long long off; };
+  struct Kk { long long off; };
+  __device__ const float* base() const { return gy; }
   __device__ Row row(int m, int z) const {
-    return Row{((long long)z * g.Coutg + m) * ((long long)g.Cg * g.RS)};
+    return Row{m < g.Coutg ? ((long long)z * g.Coutg + m) * g.y_cs : -1};
   }
-  __device__ Col col(int n, int) const { return Col{(long long)n}; }
-  __device__ void store(const Row& r, const Col& c, float acc) const { gw[r.off + c.off] = acc; }
+  __device__ Kk kk(int k, int) const {
+    const int img = k / g.HoWo;
+    return Kk{(long long)img * g.Cout * g.HoWo + (long long)(k - img * g.HoWo) * g.y_ps};
+  }
+  __device__ const float* at(const Row& r, const Kk& k) const {
+    return r.off >= 0 ? gy + r.off + k.off : nullptr;
+  }
 };
+struct FilterOut {
+  float* out;
+  const float* bias;
+  float alpha, beta;
+  int along_m, vec;
+  ConvGeo g;
+  int tap_major;
+  __device__ long long row(int m, int z) const {
+    return ((long long)z * g.Coutg + m) * ((long long)g.Cg * g.RS);
+  }
+  __device__ long long col(int n, int) const {
+    return tap_major ? (long long)(n % g.Cg) * g.RS + n / g.Cg : n;
+  }
+  __device__ int bias_at(int n, int) const { return n; }
+};
+
+// ---- the three passes on the fp32 kernel
+inline size_t up256c(size_t v) { return (v + 255) / 256 * 256; }
+
+// Products of some size first bring their operands into the order that the 16-byte loaders read:
+// the filter with its rows contiguous, an image in fl's order as a channels-last copy.  Below this
+// many multiply-adds a copy and its launch cost more than the element-wise loads they replace.
+constexpr double kStrictCopyWork = 3.2e7;
+struct StrictScratch { size_t filter, x, gy; };
+StrictScratch strict_scratch(const ConvGeo& g, int which) {
+  StrictScratch s{0, 0, 0};
+  if ((double)g.N * (which == 1 ? g.HW : g.HoWo) * g.Cout * g.Cg * g.RS < kStrictCopyWork) return s;
+  const size_t x = up256c((size_t)g.N * g.C * g.HW * 4), gy = up256c((size_t)g.N * g.Cout * g.HoWo * 4);
+  const bool x_copy = !g.x_cl && g.Cg % 4 == 0 && g.C >= 8;
+  const bool gy_copy = !g.y_cl && g.Coutg % 4 == 0 && g.Cout >= 8;
+  if (which != 2) s.filter = up256c((size_t)g.Cout * g.Cg * g.RS * 4);
+  if (which == 0 && x_copy) s.x = x;
+  if (which == 1 && gy_copy) s.gy = gy;
+  if (which == 2 && (g.x_cl || x_copy) && (g.y_cl || gy_copy)) {
+    if (!g.x_cl) s.x = x;
+    if (!g.y_cl) s.gy = gy;
+  }
+  return s;
+}
+size_t strict_scratch_bytes(const ConvGeo& g, int which) {
+  const StrictScratch s = strict_scratch(g, which);
+  return s.filter + s.x + s.gy;
+}
+
+// forward (DGRAD = false) and backward-data: an image against the filter
+template <bool DGRAD>
+int strict_image_pass(const char* name, const ConvGeo& g0, const float* src, const float* w,
+                      const float* bias, float* dst, void* ws, size_t ws_bytes, cudaStream_t st) {
+  ConvGeo g = g0;
+  const long long M = (long long)g.N * (DGRAD ? g.HW : g.HoWo);
+  FLB200_REQUIRE(M < 0x7fffffffLL, "%s: too many pixels", name);
+  const int ch = DGRAD ? g.Coutg : g.Cg, N = DGRAD ? g.Cg : g.Coutg;
+  const long long K = (long long)ch * g.RS;
+  FLB200_REQUIRE(K < 0x7fffff00LL, "%s: filter too large", name);
+  const PixelOut ep = pixel_out(dst, bias, g, DGRAD);
+  const StrictScratch need = strict_scratch(g, DGRAD ? 1 : 0);
+  const bool scratch = ws && aligned16(ws) && ws_bytes >= need.filter + need.x + need.gy;
+  char* at = static_cast<char*>(ws);
+  if (scratch && need.x + need.gy) {
+    float* copy = reinterpret_cast<float*>(at);
+    const int C = DGRAD ? g.Cout : g.C, pixels = DGRAD ? g.HoWo : g.HW;
+    if (int rc = to_channels_last(src, copy, g.N, C, pixels, st)) return rc;
+    at += need.x + need.gy;
+    src = copy;
+    if (DGRAD) { g.y_cl = 1; g.y_cs = 1; g.y_ps = g.Cout; }
+    else { g.x_cl = 1; g.x_cs = 1; g.x_ps = g.C; }
+  }
+  const bool vec = (DGRAD ? g.y_cl : g.x_cl) && ch % 4 == 0 && aligned16(src);
+  const FilterElem f{w, g, DGRAD ? 1 : 0, vec ? 1 : 0, N};
+  const float* packed = nullptr;
+  if (scratch && need.filter && N % 4 == 0) {
+    // out[z][k][row], k = (tap, channel) for channel runs, else (channel, tap)
+    float* out = reinterpret_cast<float*>(at);
+    const long long s_tap = (long long)N * (vec ? ch : 1), s_ch = (long long)N * (vec ? 1 : g.RS);
+    for (int z = 0; z < g.groups; ++z) {
+      const long long group = (long long)z * g.Coutg * g.Cg * g.RS;
+      if (int rc = filter_permute(w + group, out + group, g.Coutg, g.Cg, g.RS, s_tap, DGRAD ? s_ch : 1,
+                                  DGRAD ? 1 : s_ch, st))
+        return rc;
+    }
+    packed = out;
+    at += need.filter;
+  }
+  ws_bytes -= at - static_cast<char*>(ws);
+  const StridedLoader<kVecRow> fv{packed, 1, N, (long long)N * K, N};
+  if (vec) {
+    const ImageVec<DGRAD> iv{src, g, (int)M, ch / 4};
+    if (packed) return launch_simt_gemm(name, iv, fv, ep, M, N, K, g.groups, at, ws_bytes, st);
+    return launch_simt_gemm(name, iv, f, ep, M, N, K, g.groups, at, ws_bytes, st);
+  }
+  const ImageElem<DGRAD> ie{src, g, (int)M};
+  if (packed) return launch_simt_gemm(name, ie, fv, ep, M, N, K, g.groups, at, ws_bytes, st);
+  return launch_simt_gemm(name, ie, f, ep, M, N, K, g.groups, at, ws_bytes, st);
+}
+
+int strict_filter_pass(const char* name, const ConvGeo& g0, const float* gy, const float* x, float* gw,
+                       void* ws, size_t ws_bytes, cudaStream_t st) {
+  ConvGeo g = g0;
+  const long long N = (long long)g.Cg * g.RS, K = (long long)g.N * g.HoWo;
+  FLB200_REQUIRE(N < 0x7fffffffLL && K < 0x7fffff00LL, "%s: extent out of range", name);
+  const StrictScratch need = strict_scratch(g, 2);
+  char* at = static_cast<char*>(ws);
+  if (ws && aligned16(ws) && ws_bytes >= need.x + need.gy) {
+    if (need.x) {
+      if (int rc = to_channels_last(x, reinterpret_cast<float*>(at), g.N, g.C, g.HW, st)) return rc;
+      x = reinterpret_cast<const float*>(at);
+      at += need.x;
+      g.x_cl = 1; g.x_cs = 1; g.x_ps = g.C;
+    }
+    if (need.gy) {
+      if (int rc = to_channels_last(gy, reinterpret_cast<float*>(at), g.N, g.Cout, g.HoWo, st)) return rc;
+      gy = reinterpret_cast<const float*>(at);
+      at += need.gy;
+      g.y_cl = 1; g.y_cs = 1; g.y_ps = g.Cout;
+    }
+    ws_bytes -= need.x + need.gy;
+  }
+  FilterOut ep{gw, nullptr, 1.f, 0.f, 0, 0, g, 0};
+  if (g.x_cl && g.y_cl && g.Cg % 4 == 0 && g.Coutg % 4 == 0 && aligned16(x) && aligned16(gy)) {
+    const StridedLoader<kVecRow> gl{gy, 1, g.Cout, g.Coutg, g.Coutg};
+    ep.tap_major = 1;
+    ep.vec = g.RS == 1 && aligned16(gw);
+    return launch_simt_gemm(name, gl, WindowVec{x, g, (int)N}, ep, g.Coutg, N, K, g.groups, at, ws_bytes,
+                            st);
+  }
+  ep.vec = N % 4 == 0 && aligned16(gw);
+  return launch_simt_gemm(name, GradElem{gy, g}, WindowElem{x, g, (int)N}, ep, g.Coutg, N, K, g.groups, at,
+                          ws_bytes, st);
+}
 
 inline size_t max_sz(size_t a, size_t b) { return a > b ? a : b; }
 
@@ -310,7 +487,6 @@ struct WideCopies {
   long long n[4];
   size_t off[4], total;
 };
-inline size_t up256c(size_t v) { return (v + 255) / 256 * 256; }
 WideCopies wide_copies(const ConvGeo& g, int which) {
   const long long x = (long long)g.N * g.C * g.HW, w = (long long)g.Cout * g.Cg * g.RS,
                   y = (long long)g.N * g.Cout * g.HoWo, b = g.Cout;
@@ -346,14 +522,14 @@ size_t flb200_conv2d_workspace_bytes(const flb200_conv2d_desc* d, int which) {
   if (make_conv_geo("conv2d_workspace_bytes", d, &g)) return 0;
   size_t need = 0;
   if (which == 0) {
-    need = plan_simt(g.Coutg, (long long)g.N * g.HoWo, (long long)g.Cg * g.RS, g.groups)
-               .workspace_bytes;
+    need = strict_scratch_bytes(g, 0) +
+           plan_simt((long long)g.N * g.HoWo, g.Coutg, (long long)g.Cg * g.RS, g.groups).workspace_bytes;
   } else if (which == 1) {
-    need = plan_simt(g.Cg, (long long)g.N * g.HW, (long long)g.Coutg * g.RS, g.groups)
-               .workspace_bytes;
+    need = strict_scratch_bytes(g, 1) +
+           plan_simt((long long)g.N * g.HW, g.Cg, (long long)g.Coutg * g.RS, g.groups).workspace_bytes;
   } else {
-    need = plan_simt(g.Coutg, (long long)g.Cg * g.RS, (long long)g.N * g.HoWo, g.groups)
-               .workspace_bytes;
+    need = strict_scratch_bytes(g, 2) +
+           plan_simt(g.Coutg, (long long)g.Cg * g.RS, (long long)g.N * g.HoWo, g.groups).workspace_bytes;
     need = max_sz(need, g.y_cl ? flb200_channel_sum_workspace_bytes((int64_t)g.N * g.HoWo, g.Cout, 1)
                                : flb200_channel_sum_workspace_bytes(g.N, g.Cout, g.HoWo));
   }
@@ -413,14 +589,7 @@ int flb200_conv2d_forward_cached(const flb200_conv2d_desc* d, const void* x, con
   if (d->math_mode != FLB200_MATH_STRICT_F32 && tc_operands_aligned(x, w, y, bias, workspace) &&
       tc_conv_supported(g, 0, workspace_bytes))
     return tc_conv_forward(g, xf, wf, bf, yf, workspace, workspace_bytes, st, cache);
-  const long long n_total = (long long)g.N * g.HoWo;
-  FLB200_REQUIRE(n_total < 0x7fffffffLL, "conv2d_forward: too many output pixels");
-  const long long K = (long long)g.Cg * g.RS;
-  StridedLoader<true> al{wf, K, 1, (long long)g.Coutg * K, g.Coutg};
-  FpropB bl{xf, g, n_total};
-  FpropEpilogue ep{yf, bf, g};
-  return launch_simt_gemm("conv2d_forward", al, bl, ep, g.Coutg, n_total, K, g.groups, workspace,
-                          workspace_bytes, st);
+  return strict_image_pass<false>("conv2d_forward", g, xf, wf, bf, yf, workspace, workspace_bytes, st);
 }
 
 size_t flb200_conv2d_stats_bytes(const flb200_conv2d_desc* d, int64_t* groups) {
@@ -499,13 +668,8 @@ int flb200_conv2d_backward_data_cached(const flb200_conv2d_desc* d, const void* 
       tc_operands_aligned(grad_y, w, grad_x, nullptr, workspace) &&
       tc_conv_supported(g, 1, workspace_bytes))
     return tc_conv_backward_data(g, gyf, wf, gxf, workspace, workspace_bytes, st, cache);
-  const long long n_total = (long long)g.N * g.HW;
-  FLB200_REQUIRE(n_total < 0x7fffffffLL, "conv2d_backward_data: too many input pixels");
-  DgradA al{wf, g};
-  DgradB bl{gyf, g, n_total};
-  DgradEpilogue ep{gxf, g};
-  return launch_simt_gemm("conv2d_backward_data", al, bl, ep, g.Cg, n_total,
-                          (long long)g.Coutg * g.RS, g.groups, workspace, workspace_bytes, st);
+  return strict_image_pass<true>("conv2d_backward_data", g, gyf, wf, nullptr, gxf, workspace,
+                                 workspace_bytes, st);
 }
 
 int flb200_conv2d_backward_filter_bias(const flb200_conv2d_desc* d, const void* grad_y,
@@ -554,12 +718,7 @@ int flb200_conv2d_backward_filter_bias_cached(const flb200_conv2d_desc* d, const
       tc_conv_supported(g, 2, workspace_bytes)) {
     rc = tc_conv_backward_filter(g, gyf, xf, gwf, workspace, workspace_bytes, st, cache);
   } else {
-    const int n_total = g.Cg * g.RS;
-    WgradA al{gyf, g};
-    WgradB bl{xf, g, n_total};
-    WgradEpilogue ep{gwf, g};
-    rc = launch_simt_gemm("conv2d_backward_filter", al, bl, ep, g.Coutg, n_total,
-                          (long long)g.N * g.HoWo, g.groups, workspace, workspace_bytes, st);
+    rc = strict_filter_pass("conv2d_backward_filter", g, gyf, xf, gwf, workspace, workspace_bytes, st);
   }
   if (rc) return rc;
   if (grad_bias) {

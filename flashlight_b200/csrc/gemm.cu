@@ -10,23 +10,48 @@
 namespace flb200 {
 namespace {
 
+// Which way an operand is read: 16-byte chunks along its unit stride where base, strides and
+// extent allow it, single elements otherwise.
+int loader_kind(const void* p, long long row, long long col, long long z, long long rows, long long K,
+                long long batch) {
+  const bool vec = aligned16(p) && (batch == 1 || z % 4 == 0);
+  if (col == 1 && vec && row % 4 == 0 && K % 4 == 0) return kVecK;
+  if (row == 1 && vec && col % 4 == 0 && rows % 4 == 0) return kVecRow;
+  return row == 1 && col != 1 ? kElemRows : kElemK;
+}
+
+template <int AKIND, int BKIND>
+int matmul_simt_as(const flb200_matmul_desc* d, const float* a, const float* b,
+                   const StridedEpilogue& ep, void* ws, size_t ws_bytes, cudaStream_t st) {
+  // Operand B is indexed (row = n, k): row stride is b_col, k stride is b_row.
+  return launch_simt_gemm("matmul", StridedLoader<AKIND>{a, d->a_row, d->a_col, d->a_batch, (int)d->m},
+                          StridedLoader<BKIND>{b, d->b_col, d->b_row, d->b_batch, (int)d->n}, ep, d->m,
+                          d->n, d->k, d->batch, ws, ws_bytes, st);
+}
+template <int AKIND>
+int matmul_simt_b(int bkind, const flb200_matmul_desc* d, const float* a, const float* b,
+                  const StridedEpilogue& ep, void* ws, size_t ws_bytes, cudaStream_t st) {
+  if (bkind == kVecK) return matmul_simt_as<AKIND, kVecK>(d, a, b, ep, ws, ws_bytes, st);
+  if (bkind == kVecRow) return matmul_simt_as<AKIND, kVecRow>(d, a, b, ep, ws, ws_bytes, st);
+  if (bkind == kElemRows) return matmul_simt_as<AKIND, kElemRows>(d, a, b, ep, ws, ws_bytes, st);
+  return matmul_simt_as<AKIND, kElemK>(d, a, b, ep, ws, ws_bytes, st);
+}
+
 int matmul_simt(const flb200_matmul_desc* d, const void* a, const void* b, void* c, void* ws,
                 size_t ws_bytes, cudaStream_t st) {
-  StridedEpilogue ep{static_cast<float*>(c), d->c_row, d->c_col, d->c_batch, d->alpha, d->beta};
-  const bool a_k = d->a_col == 1 || d->a_row != 1;  // read A along k unless m is the unit stride
-  const bool b_k = d->b_row == 1 && d->b_col != 1;  // read B along k only when k is the unit stride
+  StridedEpilogue ep{static_cast<float*>(c), nullptr, d->alpha, d->beta, 0, 0, d->c_row, d->c_col,
+                     d->c_batch};
+  ep.along_m = d->c_row == 1 && d->c_col != 1;
+  ep.vec = d->c_col == 1 && d->n % 4 == 0 && d->c_row % 4 == 0 &&
+           (d->batch == 1 || d->c_batch % 4 == 0) && aligned16(c);
+  const int ak = loader_kind(a, d->a_row, d->a_col, d->a_batch, d->m, d->k, d->batch);
+  const int bk = loader_kind(b, d->b_col, d->b_row, d->b_batch, d->n, d->k, d->batch);
   const float* ap = static_cast<const float*>(a);
   const float* bp = static_cast<const float*>(b);
-  // Operand B is indexed (row = n, k): row stride is b_col, k stride is b_row.
-#define FLB200_MM(AK, BK_)                                                                     \
-  return launch_simt_gemm("matmul", StridedLoader<AK>{ap, d->a_row, d->a_col, d->a_batch, (int)d->m}, \
-                          StridedLoader<BK_>{bp, d->b_col, d->b_row, d->b_batch, (int)d->n}, ep, \
-                          d->m, d->n, d->k, d->batch, ws, ws_bytes, st)
-  if (a_k && b_k) FLB200_MM(true, true);
-  if (a_k && !b_k) FLB200_MM(true, false);
-  if (!a_k && b_k) FLB200_MM(false, true);
-  FLB200_MM(false, false);
-#undef FLB200_MM
+  if (ak == kVecK) return matmul_simt_b<kVecK>(bk, d, ap, bp, ep, ws, ws_bytes, st);
+  if (ak == kVecRow) return matmul_simt_b<kVecRow>(bk, d, ap, bp, ep, ws, ws_bytes, st);
+  if (ak == kElemRows) return matmul_simt_b<kElemRows>(bk, d, ap, bp, ep, ws, ws_bytes, st);
+  return matmul_simt_b<kElemK>(bk, d, ap, bp, ep, ws, ws_bytes, st);
 }
 
 int check_desc(const flb200_matmul_desc* d, const void* a, const void* b, const void* c) {

@@ -24,6 +24,8 @@
 // Algorithmic flops 2*M*N*K of the implicit GEMM; copies and gathers are overhead.
 #include "tc_conv.cuh"
 
+#include "filter_permute.cuh"
+
 #include "tc_gemm.cuh"
 
 namespace flb200 {
@@ -167,25 +169,6 @@ bool cl_1x1(const ConvGeo& g) {
   return g.x_cl && g.y_cl && g.kW == 1 && g.kH == 1 && g.sx == 1 && g.sy == 1 && g.px == 0 &&
          g.py == 0 && g.groups == 1 && g.C % 4 == 0 && g.Cout % 4 == 0 &&
          (long long)g.N * g.HW < 0x7fffffffLL;
-}
-
-// wt[ci][co] = w[co][ci] (1 x 1 filters), row stride Cout.
-__global__ void transpose_1x1_filter_kernel(const float* __restrict__ w, float* __restrict__ wt,
-                                            int Cout, int C) {
-  __shared__ float tile[32][33];
-  const int tx = threadIdx.x & 31, ty = threadIdx.x >> 5;
-  const int ci0 = blockIdx.x * 32, co0 = blockIdx.y * 32;
-#pragma unroll
-  for (int i = 0; i < 4; ++i) {
-    const int co = co0 + ty + 8 * i, ci = ci0 + tx;
-    tile[ty + 8 * i][tx] = (co < Cout && ci < C) ? w[(long long)co * C + ci] : 0.f;
-  }
-  __syncthreads();
-#pragma unroll
-  for (int i = 0; i < 4; ++i) {
-    const int ci = ci0 + ty + 8 * i, co = co0 + tx;
-    if (ci < C && co < Cout) wt[(long long)ci * Cout + co] = tile[tx][ty + 8 * i];
-  }
 }
 
 struct GeneralSizes {
@@ -357,9 +340,8 @@ int tc_conv_backward_data(const ConvGeo& g, const float* gy, const float* w, flo
     const tc::Launch L = gemm_plan(M, g.C, k_iters, false, false, true);
     float* wt = static_cast<float*>(ws);
     const size_t wt_bytes = up256((size_t)g.C * g.Cout * 4);
-    dim3 tgrid((unsigned)((g.C + 31) / 32), (unsigned)((g.Cout + 31) / 32));
-    transpose_1x1_filter_kernel<<<tgrid, 256, 0, st>>>(w, wt, g.Cout, g.C);
-    FLB200_AFTER_LAUNCH("transpose_1x1_filter");
+    // wt[ci][co] = w[co][ci]
+    if (int rc = filter_permute(w, wt, g.Cout, g.C, 1, 0, 1, g.Cout, st)) return rc;
     if (int rc = map2d(&ma, gy, g.Cout, M, g.Cout, tc::kBM, false)) return rc;
     if (int rc = map2d(&mb, wt, g.Cout, g.C, g.Cout, L.b_box_rows(), false)) return rc;
     ep.m_stride = g.C;

@@ -45,6 +45,9 @@ int tc_conv_backward_filter(const ConvGeo& g, const float* gy, const float* x, f
                             size_t ws_bytes, cudaStream_t st,
     flb200_conv2d_cache* cache = nullptr);
 
+// dst[n][pixel][c] = src[n][c][pixel]
+int to_channels_last(const float* src, float* dst, int N, int C, int pixels, cudaStream_t st);
+
 // Channels-last implicit-GEMM route (tc_conv_patch.cu): no im2col matrix, one NHWC copy of the
 // activation operand per pass.
 bool patch_conv_supported(const ConvGeo& g);

@@ -4,6 +4,7 @@
 // Scratch traffic per pass: one transposed copy of the activation operand (8 bytes per
 // element) and a repacked filter; there is no im2col matrix.
 
+#include "filter_permute.cuh"
 #include "tc_conv.cuh"
 #include "tc_patch.cuh"
 
@@ -165,21 +166,13 @@ int x_to_nhwc(const ConvGeo& g, const float* x, float* xt, int cp, cudaStream_t 
 
 // Filter w[co][ci][tap] repacked to out[tap][rows][kp] with (rows, k) = (co, ci) for the
 // forward pass and (ci, co) for backward-data; k >= its extent is zero.
-__global__ void pack_filter_kernel(const float* __restrict__ w, float* __restrict__ out, int Cout,
-                                   int C, int RS, int rows, int kext, int kp, int rows_are_co) {
-  const long long total = (long long)RS * rows * kp;
-  for (long long t = (long long)blockIdx.x * blockDim.x + threadIdx.x; t < total;
-       t += (long long)gridDim.x * blockDim.x) {
-    const int k = (int)(t % kp);
-    const long long r2 = t / kp;
-    const int row = (int)(r2 % rows), tap = (int)(r2 / rows);
-    float v = 0.f;
-    if (k < kext) {
-      const int co = rows_are_co ? row : k, ci = rows_are_co ? k : row;
-      v = w[((long long)co * C + ci) * RS + tap];
-    }
-    out[t] = v;
-  }
+int pack_filter(const float* w, float* out, int Cout, int C, int RS, int kp, bool rows_are_co,
+                cudaStream_t st) {
+  const int rows = rows_are_co ? Cout : C;
+  if (kp != (rows_are_co ? C : Cout))  // (the copies of fl-order images are padded to 4 channels)
+    FLB200_CUDA_CHECK(cudaMemsetAsync(out, 0, (size_t)RS * rows * kp * 4, st));
+  return filter_permute(w, out, Cout, C, RS, (long long)rows * kp, rows_are_co ? kp : 1,
+                        rows_are_co ? 1 : kp, st);
 }
 
 // gw[co][ci][tap] = sum over splits of partial[split][tap][co][ci]
@@ -508,6 +501,10 @@ int window_rows_map(CUtensorMap* m, const float* base, const WindowGeo& wg, int 
 
 }  // namespace
 
+int to_channels_last(const float* src, float* dst, int N, int C, int pixels, cudaStream_t st) {
+  return to_nhwc(src, dst, N, C, C, pixels, st);
+}
+
 // ---------------------------------------------------------------- interface
 bool patch_conv_supported(const ConvGeo& g) {
   // small channel counts would waste most of each 32-wide K chunk: those stay on the gather route
@@ -564,9 +561,7 @@ int patch_conv_forward(const ConvGeo& g0, const float* x, const float* w, const 
     }
     xt = xs.buf;
   }
-  pack_filter_kernel<<<grid_for((long long)g.RS * g.Cout * cp, 256), 256, 0, st>>>(
-      w, wp, g.Cout, g.C, g.RS, g.Cout, g.C, cp, 1);
-  FLB200_AFTER_LAUNCH("pack_filter");
+  if (int rc = pack_filter(w, wp, g.Cout, g.C, g.RS, cp, true, st)) return rc;
   PatchArgs a{};
   a.patch = pick_patch(g.Wo, g.Ho, g.N);
   a.pix_w = g.Wo; a.pix_h = g.Ho; a.images = g.N; a.n_out = g.Cout;
@@ -605,9 +600,7 @@ int patch_conv_backward_data(const ConvGeo& g, const float* gy, const float* w, 
     if (gs.flag) *gs.flag = 1;  // backward-filter of the same grad_y can take it from here
     gyt = gs.buf;
   }
-  pack_filter_kernel<<<grid_for((long long)g.RS * g.C * cop, 256), 256, 0, st>>>(
-      w, wd, g.Cout, g.C, g.RS, g.C, g.Cout, cop, 0);
-  FLB200_AFTER_LAUNCH("pack_filter");
+  if (int rc = pack_filter(w, wd, g.Cout, g.C, g.RS, cop, false, st)) return rc;
   const int bn = tc::pick_bn(g.C);
   CUtensorMap mb;
   if (int rc = filter_map(&mb, wd, g.Cout, cop, g.C, g.RS, filter_box_rows(bn))) return rc;

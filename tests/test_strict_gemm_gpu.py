@@ -1,0 +1,61 @@
+"""The fp32-FMA contraction kernel at the edges of its tiles, splits and operand loaders, against
+fp64 products and the CPU oracle (strict bound)."""
+import pytest
+import torch
+
+from oracle import flref as R
+from tests.parity import STRICT_TOL, assert_close, randn
+
+pytestmark = pytest.mark.gpu
+
+
+# (m, n, k): one element; below, at and past the 32 / 64 / 128 tiles; K below a stage, with a tail,
+# split over a cluster of CTAs, and over clusters and scratch
+@pytest.mark.parametrize("mnk", [(1, 1, 1), (31, 33, 15), (64, 64, 16), (129, 65, 36), (1, 1024, 3136),
+                                 (130, 260, 20), (32, 28, 20000), (3000, 30, 72), (257, 128, 516)])
+@pytest.mark.parametrize("a_k", [True, False])
+@pytest.mark.parametrize("b_k", [True, False])
+@pytest.mark.parametrize("offset", [0, 1])
+def test_matmul_strict_loaders(mnk, a_k, b_k, offset):
+    """a_k / b_k: k contiguous (else the rows); offset 1: base not 16-byte aligned, so that the
+    element loaders read what the vector loaders would."""
+    from flashlight_b200 import _lib as L
+    from flashlight_b200 import functions as F
+    m, n, k = mnk
+    a, b = randn(m, k, seed=1), randn(k, n, seed=2)
+    store = lambda t: torch.cat([torch.zeros(offset), t.reshape(-1)]).cuda()[offset:]
+    ad, bd = store(a if a_k else a.t().contiguous()), store(b.t().contiguous() if b_k else b)
+    c = F.matmul(ad, bd, m=m, n=n, k=k, a_strides=(k, 1) if a_k else (1, m),
+                 b_strides=(1, k) if b_k else (n, 1), math_mode=L.MATH_STRICT_F32)
+    assert_close(c, a.double() @ b.double(), STRICT_TOL, f"matmul {mnk}")
+
+
+# N, C, H, W, Cout, kH, kW, stride, pad, groups: element loaders; repacked filter and channels-last
+# copy; channels not a multiple of 4; groups; a filter of many taps; stride with empty classes
+@pytest.mark.parametrize("case", [(2, 1, 9, 9, 8, 5, 5, 1, 2, 1), (16, 32, 14, 14, 64, 5, 5, 1, 2, 1),
+                                  (8, 36, 13, 15, 44, 3, 3, 2, 1, 1), (16, 30, 14, 14, 66, 3, 3, 1, 1, 1),
+                                  (16, 64, 12, 12, 64, 3, 3, 1, 1, 4), (2, 16, 1, 70, 24, 1, 13, 1, 0, 1),
+                                  (40, 64, 17, 17, 256, 1, 1, 2, 0, 1), (8, 64, 30, 30, 64, 1, 1, 1, 0, 1)])
+@pytest.mark.parametrize("channels_last", [False, True])
+def test_conv_strict_routes(case, channels_last):
+    from flashlight_b200 import _lib as L
+    from flashlight_b200.extension import B200AutogradExtension
+    N, C, H, W, Co, kH, kW, s, p, groups = case
+    if channels_last and C == 1:
+        pytest.skip("one channel has one layout")
+    ext = B200AutogradExtension(math_mode=L.MATH_STRICT_F32)
+    x = randn(N, C, H, W, seed=3)
+    w = randn(Co, C // groups, kH, kW, seed=4) * (1.0 / (C // groups * kH * kW) ** 0.5)
+    b = randn(Co, seed=5)
+    args = (s, s, p, p, 1, 1, groups)
+    put = lambda t: t.cuda().contiguous(memory_format=torch.channels_last) if channels_last else t.cuda()
+    y = ext.conv2d(put(x), w.cuda(), b.cuda(), *args)
+    want = R.conv2d(x.double(), w.double(), b.double(), *args)
+    assert_close(y, want, STRICT_TOL, "conv forward")
+    gy = randn(*want.shape, seed=6)
+    gx = ext.conv2dBackwardData(put(gy), put(x), w.cuda(), *args)
+    assert_close(gx, R.conv2d_backward_data(gy.double(), x.shape, w.double(), *args), STRICT_TOL, "conv dx")
+    gw, gb = ext.conv2dBackwardFilterBias(put(gy), put(x), w.cuda(), b.cuda(), *args)
+    wgw, wgb = R.conv2d_backward_filter_bias(gy.double(), x.double(), w.shape, True, *args)
+    assert_close(gw, wgw, STRICT_TOL, "conv dw")
+    assert_close(gb, wgb, STRICT_TOL, "conv db")
