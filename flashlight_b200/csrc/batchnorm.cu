@@ -68,13 +68,27 @@ __device__ __forceinline__ float bn_scale(float invstd, const float* weight, lon
   return (float)((double)invstd * (weight ? (double)weight[c] : 1.0));
 }
 
+// invstd * gamma per channel: what the statistics pass left, or (evaluation mode) straight from the
+// running variance, which saves the small kernel that would prepare it.
+struct BnScale {
+  const float* scale;
+  const float* running_var;  // evaluation mode when set
+  const float* weight;
+  double eps;
+  __device__ float at(long long c) const {
+    if (!running_var) return scale[c];
+    const double invstd = 1.0 / sqrt((double)running_var[c] + eps);
+    return (float)(invstd * (weight ? (double)weight[c] : 1.0));
+  }
+};
+
 template <bool RELU>
 struct BnFwdApplyF {  // y = (x - mean) * scale + shift, then max(., 0) when RELU
   const float* mean;
-  const float* scale;  // invstd * gamma
+  BnScale scale;
   const float* shift;  // beta
   struct K { float mean, scale, shift; };
-  __device__ K channel(long long c) const { return K{mean[c], scale[c], shift ? shift[c] : 0.f}; }
+  __device__ K channel(long long c) const { return K{mean[c], scale.at(c), shift ? shift[c] : 0.f}; }
   __device__ float apply(const K& k, float a, float) const {
     const float z = bn_value(a, k.mean, k.scale, k.shift);
     return RELU ? (z > 0.f ? z : (z != z ? z : 0.f)) : z;
@@ -135,11 +149,11 @@ template <int G>
 __global__ void __launch_bounds__(kChanThreads)
 bn_add_relu_apply_kernel(const float* __restrict__ x, const float* __restrict__ addend,
                          float* __restrict__ y, uint8_t* __restrict__ mask, ChannelGeo g,
-                         const float* __restrict__ mean, const float* __restrict__ scale,
+                         const float* __restrict__ mean, const BnScale scale,
                          const float* __restrict__ shift) {
   constexpr int NV = G / 4;
   const long long c = blockIdx.x;
-  const float m = mean[c], sc = scale[c], sh = shift ? shift[c] : 0.f;
+  const float m = mean[c], sc = scale.at(c), sh = shift ? shift[c] : 0.f;
   long long begin = (long long)blockIdx.y * g.chunk;
   long long end = begin + g.chunk;
   if (end > g.per_channel) end = g.per_channel;
@@ -222,10 +236,10 @@ bn_tail_backward_reduce_kernel(const float* __restrict__ x, const float* __restr
 __global__ void __launch_bounds__(kChanThreads)
 bn_add_relu_apply_scalar_kernel(const float* __restrict__ x, const float* __restrict__ addend,
                                 float* __restrict__ y, uint8_t* __restrict__ mask, ChannelGeo g,
-                                const float* __restrict__ mean, const float* __restrict__ scale,
+                                const float* __restrict__ mean, const BnScale scale,
                                 const float* __restrict__ shift) {
   const long long c = blockIdx.x;
-  const float m = mean[c], sc = scale[c], sh = shift ? shift[c] : 0.f;
+  const float m = mean[c], sc = scale.at(c), sh = shift ? shift[c] : 0.f;
   long long begin = (long long)blockIdx.y * g.chunk;
   long long end = begin + g.chunk;
   if (end > g.per_channel) end = g.per_channel;
@@ -273,11 +287,26 @@ inline OctetTiling octet_tiling(long long channels) {
   return OctetTiling{shift, (int)((octs + (1LL << shift) - 1) >> shift)};
 }
 
+// eight consecutive values of a tensor as fp32: two 16-byte vectors or one
+template <typename T>
+__device__ __forceinline__ void load8(const T* p, float* v) {
+  constexpr int V = Vec16<T>::N;
+#pragma unroll
+  for (int h = 0; h < 8 / V; ++h) unpack16(load16(p + h * V), v + h * V);
+}
+template <typename T>
+__device__ __forceinline__ void store8(T* p, const float* v) {
+  constexpr int V = Vec16<T>::N;
+#pragma unroll
+  for (int h = 0; h < 8 / V; ++h) store16(p + h * V, pack16<T>(v + h * V));
+}
+
+template <typename T>
 __global__ void __launch_bounds__(256)
-bn_add_relu_apply_cl_kernel(const float* __restrict__ x, const float* __restrict__ addend,
-                            float* __restrict__ y, uint8_t* __restrict__ mask, long long rows,
+bn_add_relu_apply_cl_kernel(const T* __restrict__ x, const T* __restrict__ addend,
+                            T* __restrict__ y, uint8_t* __restrict__ mask, long long rows,
                             long long channels, long long rows_per_split, int co_shift,
-                            const float* __restrict__ mean, const float* __restrict__ scale,
+                            const float* __restrict__ mean, const BnScale scale,
                             const float* __restrict__ shift) {
   const int co = 1 << co_shift, rl = 256 >> co_shift;
   const int tq = threadIdx.x & (co - 1), tr = threadIdx.x >> co_shift;
@@ -287,7 +316,7 @@ bn_add_relu_apply_cl_kernel(const float* __restrict__ x, const float* __restrict
 #pragma unroll
   for (int j = 0; j < 8; ++j) {
     m[j] = mean[c + j];
-    sc[j] = scale[c + j];
+    sc[j] = scale.at(c + j);
     sh[j] = shift ? shift[c + j] : 0.f;
   }
   const long long r0 = (long long)blockIdx.y * rows_per_split;
@@ -296,10 +325,8 @@ bn_add_relu_apply_cl_kernel(const float* __restrict__ x, const float* __restrict
   for (long long r = r0 + tr; r < r1; r += rl) {
     const long long off = r * channels + c;
     float a[8], s[8], z[8];
-    *reinterpret_cast<float4*>(a) = *reinterpret_cast<const float4*>(x + off);
-    *reinterpret_cast<float4*>(a + 4) = *reinterpret_cast<const float4*>(x + off + 4);
-    *reinterpret_cast<float4*>(s) = *reinterpret_cast<const float4*>(addend + off);
-    *reinterpret_cast<float4*>(s + 4) = *reinterpret_cast<const float4*>(addend + off + 4);
+    load8(x + off, a);
+    load8(addend + off, s);
     unsigned bits = 0;
 #pragma unroll
     for (int j = 0; j < 8; ++j) {
@@ -307,16 +334,29 @@ bn_add_relu_apply_cl_kernel(const float* __restrict__ x, const float* __restrict
       z[j] = v > 0.f ? v : (v != v ? v : 0.f);
       bits |= (v > 0.f ? 1u : 0u) << j;
     }
-    *reinterpret_cast<float4*>(y + off) = make_float4(z[0], z[1], z[2], z[3]);
-    *reinterpret_cast<float4*>(y + off + 4) = make_float4(z[4], z[5], z[6], z[7]);
+    store8(y + off, z);
     mask[off >> 3] = (uint8_t)bits;
   }
 }
 
-__global__ void __launch_bounds__(256)
-bn_tail_backward_reduce_cl_kernel(const float* __restrict__ x, const float* __restrict__ ga,
-                                  const float* __restrict__ gb, const uint8_t* __restrict__ mask,
-                                  float* __restrict__ gz, float2* __restrict__ partial,
+template <typename T>
+void launch_add_relu_cl(const void* x, const void* addend, void* y, uint8_t* mask, long long rows,
+                        long long channels, const float* mean, const BnScale& scale, const float* shift,
+                        cudaStream_t st) {
+  const OctetTiling ot = octet_tiling(channels);
+  const long long rps = apply_rows_per_split(rows, ot.col_blocks, 256 >> ot.co_shift,
+                                             sizeof(T) == 4 ? 16 : 4);  // registers: 4 per SM
+  const dim3 grid((unsigned)ot.col_blocks, (unsigned)((rows + rps - 1) / rps));
+  bn_add_relu_apply_cl_kernel<T><<<grid, 256, 0, st>>>(
+      static_cast<const T*>(x), static_cast<const T*>(addend), static_cast<T*>(y), mask, rows, channels,
+      rps, ot.co_shift, mean, scale, shift);
+}
+
+template <typename T>
+__global__ void __launch_bounds__(256, 3)
+bn_tail_backward_reduce_cl_kernel(const T* __restrict__ x, const T* __restrict__ ga,
+                                  const T* __restrict__ gb, const uint8_t* __restrict__ mask,
+                                  T* __restrict__ gz, float2* __restrict__ partial,
                                   long long rows, long long channels, int splits,
                                   long long rows_per_split, int co_shift,
                                   const float* __restrict__ mean) {
@@ -335,17 +375,15 @@ bn_tail_backward_reduce_cl_kernel(const float* __restrict__ x, const float* __re
     const long long r0 = (long long)blockIdx.y * rows_per_split;
     long long r1 = r0 + rows_per_split;
     if (r1 > rows) r1 = rows;
+#pragma unroll 2
     for (long long r = r0 + tr; r < r1; r += rl) {
       const long long off = r * channels + c;
       float xv[8], av[8];
-      *reinterpret_cast<float4*>(xv) = *reinterpret_cast<const float4*>(x + off);
-      *reinterpret_cast<float4*>(xv + 4) = *reinterpret_cast<const float4*>(x + off + 4);
-      *reinterpret_cast<float4*>(av) = *reinterpret_cast<const float4*>(ga + off);
-      *reinterpret_cast<float4*>(av + 4) = *reinterpret_cast<const float4*>(ga + off + 4);
+      load8(x + off, xv);
+      load8(ga + off, av);
       if (gb) {
         float bv[8];
-        *reinterpret_cast<float4*>(bv) = *reinterpret_cast<const float4*>(gb + off);
-        *reinterpret_cast<float4*>(bv + 4) = *reinterpret_cast<const float4*>(gb + off + 4);
+        load8(gb + off, bv);
 #pragma unroll
         for (int j = 0; j < 8; ++j) av[j] += bv[j];
       }
@@ -353,12 +391,12 @@ bn_tail_backward_reduce_cl_kernel(const float* __restrict__ x, const float* __re
       float rv[8];
 #pragma unroll
       for (int j = 0; j < 8; ++j) {
-        rv[j] = (bits >> j) & 1u ? av[j] : 0.f;
+        // what is reduced is what the tensor holds
+        rv[j] = Num<T>::to_f(Num<T>::from_f((bits >> j) & 1u ? av[j] : 0.f));
         s0[j] += rv[j];
         s1[j] += rv[j] * (xv[j] - m[j]);
       }
-      *reinterpret_cast<float4*>(gz + off) = make_float4(rv[0], rv[1], rv[2], rv[3]);
-      *reinterpret_cast<float4*>(gz + off + 4) = make_float4(rv[4], rv[5], rv[6], rv[7]);
+      store8(gz + off, rv);
     }
   }
 #pragma unroll
@@ -521,15 +559,6 @@ __global__ void affine_bwd_finalize_kernel(const float2* __restrict__ partial, i
   if (grad_weight) grad_weight[c] = (float)s1;
 }
 
-__global__ void bn_infer_prepare_kernel(long long channels, const float* __restrict__ weight,
-                                        const float* __restrict__ running_var, double eps,
-                                        float* __restrict__ scale) {
-  const long long c = (long long)blockIdx.x * blockDim.x + threadIdx.x;
-  if (c >= channels) return;
-  const double invstd = 1.0 / sqrt((double)running_var[c] + eps);
-  scale[c] = (float)(invstd * (weight ? (double)weight[c] : 1.0));
-}
-
 __global__ void bn_bwd_finalize_kernel(const float2* __restrict__ partial, int splits,
                                        long long channels, double count,
                                        const float* __restrict__ weight,
@@ -557,17 +586,15 @@ int launch_reduce(const char* name, const void* a, const void* b, float2* partia
   if (inner == 1) {
     const int splits = column_splits(outer, channels);
     const long long rps = (outer + splits - 1) / splits;
-    if constexpr (std::is_same<T, float>::value) {
-      if (channels % 4 == 0 && aligned16(a) && (NIN == 1 || aligned16(b))) {
-        const ColumnTiling ct = column_tiling(channels);
-        dim3 vgrid((unsigned)ct.col_blocks, (unsigned)splits);
-        column_reduce_vec_kernel<NIN, F><<<vgrid, 256, 0, st>>>(
-            static_cast<const float*>(a), static_cast<const float*>(b), partial, outer, channels,
-            splits, rps, ct.cq_shift, f);
-        FLB200_AFTER_LAUNCH(name);
-        *splits_out = splits;
-        return FLB200_OK;
-      }
+    if (channels % Vec16<T>::N == 0 && aligned16(a) && (NIN == 1 || aligned16(b))) {
+      const ColumnTiling ct = column_tiling(channels, Vec16<T>::N);
+      dim3 vgrid((unsigned)ct.col_blocks, (unsigned)splits);
+      column_reduce_vec_kernel<T, NIN, F><<<vgrid, 256, 0, st>>>(
+          static_cast<const T*>(a), static_cast<const T*>(b), partial, outer, channels,
+          splits, rps, ct.cq_shift, f);
+      FLB200_AFTER_LAUNCH(name);
+      *splits_out = splits;
+      return FLB200_OK;
     }
     dim3 grid((unsigned)((channels + 31) / 32), (unsigned)splits);
     column_reduce_kernel<T, NIN, F><<<grid, 256, 0, st>>>(
@@ -595,22 +622,16 @@ template <typename T, int NIN, typename F>
 int launch_apply(const char* name, const void* a, const void* b, void* out, long long outer,
                  long long channels, long long inner, F f, cudaStream_t st) {
   if (inner == 1) {
-    if constexpr (std::is_same<T, float>::value) {
-      if (channels % 4 == 0 && aligned16(a) && aligned16(out) && (NIN == 1 || aligned16(b))) {
-        const ColumnTiling ct = column_tiling(channels);
-        // about 16 CTAs per SM, at least 32 rows each
-        long long splits = (16LL * device_info().sm_count + ct.col_blocks - 1) / ct.col_blocks;
-        if (splits > (outer + 31) / 32) splits = (outer + 31) / 32;
-        if (splits > 65535) splits = 65535;
-        if (splits < 1) splits = 1;
-        const long long rps = (outer + splits - 1) / splits;
-        dim3 vgrid((unsigned)ct.col_blocks, (unsigned)splits);
-        column_apply_vec_kernel<NIN, F><<<vgrid, 256, 0, st>>>(
-            static_cast<const float*>(a), static_cast<const float*>(b), static_cast<float*>(out),
-            outer, channels, rps, ct.cq_shift, f);
-        FLB200_AFTER_LAUNCH(name);
-        return FLB200_OK;
-      }
+    if (channels % Vec16<T>::N == 0 && aligned16(a) && aligned16(out) && (NIN == 1 || aligned16(b))) {
+      const ColumnTiling ct = column_tiling(channels, Vec16<T>::N);
+      const long long rps = apply_rows_per_split(outer, ct.col_blocks, 256 >> ct.cq_shift,
+                                                 sizeof(T) == 4 ? 16 : 6);
+      dim3 vgrid((unsigned)ct.col_blocks, (unsigned)((outer + rps - 1) / rps));
+      column_apply_vec_kernel<T, NIN, F><<<vgrid, 256, 0, st>>>(
+          static_cast<const T*>(a), static_cast<const T*>(b), static_cast<T*>(out),
+          outer, channels, rps, ct.cq_shift, f);
+      FLB200_AFTER_LAUNCH(name);
+      return FLB200_OK;
     }
     const int grid = grid_for(outer * channels, 256 * 4);
     column_apply_kernel<T, NIN, F><<<grid, 256, 0, st>>>(
@@ -645,6 +666,12 @@ int check_geo(const char* name, long long outer, long long channels, long long i
   FLB200_REQUIRE(outer >= 1 && channels >= 1 && inner >= 1, "%s: empty geometry", name);
   FLB200_REQUIRE(channels < 0x7fffffffLL, "%s: too many channels", name);
   return FLB200_OK;
+}
+
+// Shapes of the fused batch-norm + shortcut + relu passes: channels-last rows of whole 8-channel
+// groups in any type, fl's own order in f32.
+bool add_relu_supported(const flb200_batchnorm_desc* d) {
+  return d->inner < 2 ? d->channels % 8 == 0 : d->dtype == FLB200_F32;
 }
 
 inline size_t align_up(size_t v, size_t a) { return (v + a - 1) / a * a; }
@@ -862,6 +889,7 @@ static int batchnorm_forward_impl(bool relu, const void* addend, uint8_t* mask,
       reinterpret_cast<float*>(ws + align_up(channel_partial_bytes(d->outer, C, d->inner), 256));
   int rc = FLB200_OK;
   const float* mean_ptr;
+  BnScale bs{scale, nullptr, nullptr, 0.0};
   if (train) {
     FLB200_REQUIRE(save_mean && save_invstd, "batchnorm_forward: training needs save_mean/save_invstd");
     if (stats) {
@@ -891,21 +919,12 @@ static int batchnorm_forward_impl(bool relu, const void* addend, uint8_t* mask,
   } else {
     FLB200_REQUIRE(running_mean && running_var,
                    "batchnorm_forward: inference needs running_mean/running_var");
-    bn_infer_prepare_kernel<<<(unsigned)((C + 127) / 128), 128, 0, st>>>(C, weight, running_var,
-                                                                         epsilon, scale);
-    FLB200_AFTER_LAUNCH("batchnorm_infer_prepare");
+    bs = BnScale{nullptr, running_var, weight, epsilon};
     mean_ptr = running_mean;
   }
   if (addend && d->inner == 1) {
-    const OctetTiling ot = octet_tiling(C);
-    long long splits = (16LL * device_info().sm_count + ot.col_blocks - 1) / ot.col_blocks;
-    if (splits > (d->outer + 31) / 32) splits = (d->outer + 31) / 32;
-    if (splits > 65535) splits = 65535;
-    if (splits < 1) splits = 1;
-    const long long rps = (d->outer + splits - 1) / splits;
-    bn_add_relu_apply_cl_kernel<<<dim3((unsigned)ot.col_blocks, (unsigned)splits), 256, 0, st>>>(
-        static_cast<const float*>(x), static_cast<const float*>(addend), static_cast<float*>(y),
-        mask, d->outer, C, rps, ot.co_shift, mean_ptr, scale, bias);
+    FLB200_DISPATCH_DTYPE(d->dtype, "batchnorm_add_relu_forward",
+                          (launch_add_relu_cl<T>(x, addend, y, mask, d->outer, C, mean_ptr, bs, bias, st)));
     FLB200_AFTER_LAUNCH("batchnorm_add_relu_apply_channels_last");
   } else if (addend) {
     const ChannelGeo g = make_channel_geo(d->outer, C, d->inner);
@@ -913,23 +932,23 @@ static int batchnorm_forward_impl(bool relu, const void* addend, uint8_t* mask,
     if (d->inner % 8 == 0)
       bn_add_relu_apply_kernel<8><<<grid, kChanThreads, 0, st>>>(
           static_cast<const float*>(x), static_cast<const float*>(addend), static_cast<float*>(y),
-          mask, g, mean_ptr, scale, bias);
+          mask, g, mean_ptr, bs, bias);
     else if (d->inner % 4 != 0)
       bn_add_relu_apply_scalar_kernel<<<grid, kChanThreads, 0, st>>>(
           static_cast<const float*>(x), static_cast<const float*>(addend), static_cast<float*>(y),
-          mask, g, mean_ptr, scale, bias);
+          mask, g, mean_ptr, bs, bias);
     else
       bn_add_relu_apply_kernel<4><<<grid, kChanThreads, 0, st>>>(
           static_cast<const float*>(x), static_cast<const float*>(addend), static_cast<float*>(y),
-          mask, g, mean_ptr, scale, bias);
+          mask, g, mean_ptr, bs, bias);
     FLB200_AFTER_LAUNCH("batchnorm_add_relu_apply");
   } else if (relu) {
-    BnFwdApplyF<true> af{mean_ptr, scale, bias};
+    BnFwdApplyF<true> af{mean_ptr, bs, bias};
     FLB200_DISPATCH_DTYPE(d->dtype, "batchnorm_relu_forward",
                           rc = (launch_apply<T, 1>("batchnorm_relu_apply", x, nullptr, y, d->outer,
                                                    C, d->inner, af, st)));
   } else {
-    BnFwdApplyF<false> af{mean_ptr, scale, bias};
+    BnFwdApplyF<false> af{mean_ptr, bs, bias};
     FLB200_DISPATCH_DTYPE(d->dtype, "batchnorm_forward",
                           rc = (launch_apply<T, 1>("batchnorm_apply", x, nullptr, y, d->outer, C,
                                                    d->inner, af, st)));
@@ -965,11 +984,10 @@ int flb200_batchnorm_add_relu_forward(const flb200_batchnorm_desc* d, const void
                                       double epsilon, void* y, uint8_t* mask, void* workspace,
                                       size_t workspace_bytes, void* stream) {
   FLB200_REQUIRE(d && addend && mask, "batchnorm_add_relu_forward: null argument");
-  if (d->dtype != FLB200_F32 || (d->inner < 2 && d->channels % 8 != 0) || !aligned16(x) ||
-      !aligned16(addend) || !aligned16(y))
+  if (!add_relu_supported(d) || !aligned16(x) || !aligned16(addend) || !aligned16(y))
     return fail(FLB200_UNSUPPORTED,
-                "batchnorm_add_relu_forward: f32, 16-byte aligned tensors, in a spatial layout or "
-                "channels-last with a multiple of 8 channels, only");
+                "batchnorm_add_relu_forward: 16-byte aligned tensors, channels-last with a multiple "
+                "of 8 channels or (f32) in a spatial layout, only");
   return batchnorm_forward_impl(true, addend, mask, d, x, weight, bias, running_mean, running_var,
                                 save_mean, save_invstd, train, momentum, epsilon, y, workspace,
                                 workspace_bytes, stream);
@@ -990,12 +1008,11 @@ int flb200_batchnorm_forward_from_stats(const flb200_batchnorm_desc* d, const vo
                                         double epsilon, void* y, uint8_t* mask, void* workspace,
                                         size_t workspace_bytes, void* stream) {
   FLB200_REQUIRE(d && stats && groups >= 1, "batchnorm_forward_from_stats: null argument");
-  FLB200_REQUIRE(d->dtype == FLB200_F32 && aligned16(stats) && d->channels % 4 == 0,
-                 "batchnorm_forward_from_stats: f32 tensors, channels a multiple of 4");
+  FLB200_REQUIRE(aligned16(stats) && d->channels % 4 == 0,
+                 "batchnorm_forward_from_stats: channels a multiple of 4");
   if (addend) {
     FLB200_REQUIRE(mask, "batchnorm_forward_from_stats: the add + relu form writes a mask");
-    if ((d->inner < 2 && d->channels % 8 != 0) || !aligned16(x) || !aligned16(addend) ||
-        !aligned16(y))
+    if (!add_relu_supported(d) || !aligned16(x) || !aligned16(addend) || !aligned16(y))
       return fail(FLB200_UNSUPPORTED,
                   "batchnorm_forward_from_stats: the add + relu form needs 16-byte aligned "
                   "tensors, in a spatial layout or channels-last with a multiple of 8 channels");
@@ -1034,11 +1051,13 @@ static int batchnorm_backward_impl(bool relu, const uint8_t* tail_mask, const vo
     const OctetTiling ot = octet_tiling(C);
     splits = column_splits(d->outer, C);
     const long long rps = (d->outer + splits - 1) / splits;
-    bn_tail_backward_reduce_cl_kernel<<<dim3((unsigned)ot.col_blocks, (unsigned)splits), 256, 0,
-                                        st>>>(
-        static_cast<const float*>(x), static_cast<const float*>(grad_y),
-        static_cast<const float*>(tail_gb), tail_mask, static_cast<float*>(tail_sum), partial,
-        d->outer, C, splits, rps, ot.co_shift, save_mean);
+    FLB200_DISPATCH_DTYPE(
+        d->dtype, "batchnorm_add_relu_backward",
+        (bn_tail_backward_reduce_cl_kernel<T>
+         <<<dim3((unsigned)ot.col_blocks, (unsigned)splits), 256, 0, st>>>(
+             static_cast<const T*>(x), static_cast<const T*>(grad_y), static_cast<const T*>(tail_gb),
+             tail_mask, static_cast<T*>(tail_sum), partial, d->outer, C, splits, rps, ot.co_shift,
+             save_mean)));
     FLB200_AFTER_LAUNCH("batchnorm_tail_backward_reduce_channels_last");
     grad_y = tail_sum;
   } else if (tail_mask) {
@@ -1120,11 +1139,11 @@ int flb200_batchnorm_add_relu_backward(const flb200_batchnorm_desc* d, const uin
                                        float* grad_weight, float* grad_bias, void* workspace,
                                        size_t workspace_bytes, void* stream) {
   FLB200_REQUIRE(d && mask && grad_y_a && grad_sum, "batchnorm_add_relu_backward: null argument");
-  if (d->dtype != FLB200_F32 || (d->inner < 2 && d->channels % 8 != 0) || !aligned16(x) ||
+  if (!add_relu_supported(d) || !aligned16(x) ||
       !aligned16(grad_y_a) || !aligned16(grad_sum) || (grad_y_b && !aligned16(grad_y_b)))
     return fail(FLB200_UNSUPPORTED,
-                "batchnorm_add_relu_backward: f32, 16-byte aligned tensors, in a spatial layout or "
-                "channels-last with a multiple of 8 channels, only");
+                "batchnorm_add_relu_backward: 16-byte aligned tensors, channels-last with a multiple "
+                "of 8 channels or (f32) in a spatial layout, only");
   return batchnorm_backward_impl(false, mask, grad_y_b, grad_sum, d, grad_y_a, x, weight, nullptr,
                                  save_mean, save_invstd, grad_x, grad_weight, grad_bias, workspace,
                                  workspace_bytes, stream);

@@ -10,6 +10,8 @@
 // per-channel kernel finishes in double precision.  The channel is constant per
 // CTA, so the per-channel constants live in registers.
 #pragma once
+#include <algorithm>
+
 #include "common.cuh"
 
 namespace flb200 {
@@ -212,151 +214,172 @@ column_apply_kernel(const T* __restrict__ a, const T* __restrict__ b, T* __restr
 }
 
 // ------------------------------------------------------------------------------------------
-// inner == 1 with fp32 data, channels a multiple of 4 and 16-byte aligned tensors (the
-// channels-last image tensors, [pixels][channels]): the same column reduction and per-channel
-// pass with 16-byte accesses.  A CTA of 256 threads is CQ column quads (4 channels each, CQ a
-// power of two <= 64) x 256 / CQ row lanes; a thread keeps the constants of its four channels in
-// registers and walks the rows of its split with four independent loads in flight.
+// inner == 1 with channels a multiple of the 16-byte vector (4 fp32, 8 16-bit values) and 16-byte
+// aligned tensors (channels-last image tensors [pixels][channels], rows of features): the same
+// column reduction and per-channel pass with 16-byte accesses.  A CTA of 256 threads is CQ column
+// vectors (CQ a power of two <= 64) x 256 / CQ row lanes; a thread keeps the constants of its
+// channels in registers and walks the rows of its split with several independent loads in flight.
+// (Element by element, 16-bit tensors ran at a quarter to half of the bandwidth of fp32 ones: the
+// three reductions for relu(batch-norm) gradients in a block of 64 x 56 x 56 x 256 f16 took 166 us,
+// with vectors 76; its statistics passes 40 us each, now 23.)
 struct ColumnTiling {
   int cq_shift;    // log2(CQ)
-  int col_blocks;  // ceil(channels / (4 * CQ))
+  int col_blocks;  // ceil(channels / (V * CQ))
 };
-inline ColumnTiling column_tiling(long long channels) {
-  const long long quads = (channels + 3) / 4;
+inline ColumnTiling column_tiling(long long channels, int v = 4) {
+  const long long vecs = (channels + v - 1) / v;
   int shift = 0;
-  while ((2LL << shift) <= quads && shift < 6) ++shift;
+  while ((2LL << shift) <= vecs && shift < 6) ++shift;
   ColumnTiling t;
   t.cq_shift = shift;
-  t.col_blocks = (int)((quads + (1LL << shift) - 1) >> shift);
+  t.col_blocks = (int)((vecs + (1LL << shift) - 1) >> shift);
   return t;
 }
 
-template <int NIN, typename F>
-__global__ void __launch_bounds__(256)
-column_reduce_vec_kernel(const float* __restrict__ a, const float* __restrict__ b,
+template <typename T, int NIN, typename F>
+__global__ void __launch_bounds__(256, 3)
+column_reduce_vec_kernel(const T* __restrict__ a, const T* __restrict__ b,
                          float2* __restrict__ partial, long long rows, long long channels,
                          int splits, long long rows_per_split, int cq_shift, F f) {
-  __shared__ float sh0[1024];
-  __shared__ float sh1[1024];
+  constexpr int V = Vec16<T>::N;
+  __shared__ float sh0[256 * V];
+  __shared__ float sh1[256 * V];
   const int cq = 1 << cq_shift, rl = 256 >> cq_shift;
   const int tq = threadIdx.x & (cq - 1), tr = threadIdx.x >> cq_shift;
-  const long long c = ((long long)blockIdx.x * cq + tq) * 4;
+  const long long c = ((long long)blockIdx.x * cq + tq) * V;
   const int s = blockIdx.y;
-  float s0[4] = {0.f, 0.f, 0.f, 0.f}, s1[4] = {0.f, 0.f, 0.f, 0.f};
-  const bool live = c < channels;
-  if (live) {
-    typename F::K k[4];
+  float s0[V], s1[V];
 #pragma unroll
-    for (int j = 0; j < 4; ++j) k[j] = f.channel(c + j);
+  for (int j = 0; j < V; ++j) s0[j] = s1[j] = 0.f;
+  if (c < channels) {
+    typename F::K k[V];
+#pragma unroll
+    for (int j = 0; j < V; ++j) k[j] = f.channel(c + j);
     const long long r0 = (long long)s * rows_per_split;
     long long r1 = r0 + rows_per_split;
     if (r1 > rows) r1 = rows;
     long long r = r0 + tr;
+    auto take = [&](const Vec16<T>& ra, const Vec16<T>& rb) {
+      float va[V], vb[V];
+      unpack16(ra, va);
+      if (NIN == 2) unpack16(rb, vb);
+#pragma unroll
+      for (int j = 0; j < V; ++j) f.accumulate(k[j], va[j], NIN == 2 ? vb[j] : 0.f, s0[j], s1[j]);
+    };
     // eight 16-byte loads in flight per thread: 8 rows of one tensor or 4 rows of two
     constexpr int U = NIN == 2 ? 4 : 8;
     for (; r + (long long)(U - 1) * rl < r1; r += (long long)U * rl) {
-      float4 va[U], vb[U];
+      Vec16<T> va[U], vb[U];
 #pragma unroll
       for (int u = 0; u < U; ++u) {
         const long long off = (r + (long long)u * rl) * channels + c;
-        va[u] = *reinterpret_cast<const float4*>(a + off);
-        if (NIN == 2) vb[u] = *reinterpret_cast<const float4*>(b + off);
+        va[u] = load16(a + off);
+        if (NIN == 2) vb[u] = load16(b + off);
       }
 #pragma unroll
-      for (int u = 0; u < U; ++u) {
-        f.accumulate(k[0], va[u].x, NIN == 2 ? vb[u].x : 0.f, s0[0], s1[0]);
-        f.accumulate(k[1], va[u].y, NIN == 2 ? vb[u].y : 0.f, s0[1], s1[1]);
-        f.accumulate(k[2], va[u].z, NIN == 2 ? vb[u].z : 0.f, s0[2], s1[2]);
-        f.accumulate(k[3], va[u].w, NIN == 2 ? vb[u].w : 0.f, s0[3], s1[3]);
-      }
+      for (int u = 0; u < U; ++u) take(va[u], vb[u]);
     }
     for (; r < r1; r += rl) {
       const long long off = r * channels + c;
-      const float4 va = *reinterpret_cast<const float4*>(a + off);
-      float4 vb = make_float4(0.f, 0.f, 0.f, 0.f);
-      if (NIN == 2) vb = *reinterpret_cast<const float4*>(b + off);
-      f.accumulate(k[0], va.x, vb.x, s0[0], s1[0]);
-      f.accumulate(k[1], va.y, vb.y, s0[1], s1[1]);
-      f.accumulate(k[2], va.z, vb.z, s0[2], s1[2]);
-      f.accumulate(k[3], va.w, vb.w, s0[3], s1[3]);
+      const Vec16<T> va = load16(a + off);
+      Vec16<T> vb;
+      if (NIN == 2) vb = load16(b + off);
+      take(va, vb);
     }
   }
-  // sh[tr][tq * 4 + j]: 256 threads x 4 values
+  // sh[tr][tq * V + j]: 256 threads x V values
 #pragma unroll
-  for (int j = 0; j < 4; ++j) {
-    sh0[(tr << (cq_shift + 2)) + tq * 4 + j] = s0[j];
-    sh1[(tr << (cq_shift + 2)) + tq * 4 + j] = s1[j];
+  for (int j = 0; j < V; ++j) {
+    sh0[(tr * cq + tq) * V + j] = s0[j];
+    sh1[(tr * cq + tq) * V + j] = s1[j];
   }
   __syncthreads();
-  // thread t < 4 * CQ finishes column t of the block
-  if ((int)threadIdx.x < 4 * cq) {
-    const long long cc = (long long)blockIdx.x * cq * 4 + threadIdx.x;
+  // the block's V * CQ columns, each finished by one thread
+  for (int t = threadIdx.x; t < V * cq; t += 256) {
+    const long long cc = (long long)blockIdx.x * cq * V + t;
     if (cc < channels) {
       float t0 = 0.f, t1 = 0.f;
       for (int i = 0; i < rl; ++i) {
-        t0 += sh0[(i << (cq_shift + 2)) + threadIdx.x];
-        t1 += sh1[(i << (cq_shift + 2)) + threadIdx.x];
+        t0 += sh0[i * cq * V + t];
+        t1 += sh1[i * cq * V + t];
       }
       partial[cc * splits + s] = make_float2(t0, t1);
     }
   }
 }
 
-template <int NIN, typename F>
-__global__ void __launch_bounds__(256)
-column_apply_vec_kernel(const float* __restrict__ a, const float* __restrict__ b,
-                        float* __restrict__ out, long long rows, long long channels,
+template <typename T, int NIN, typename F>
+__global__ void __launch_bounds__(256, sizeof(T) == 4 ? 4 : NIN == 2 ? 2 : 3)
+column_apply_vec_kernel(const T* __restrict__ a, const T* __restrict__ b,
+                        T* __restrict__ out, long long rows, long long channels,
                         long long rows_per_split, int cq_shift, F f) {
+  constexpr int V = Vec16<T>::N;
   const int cq = 1 << cq_shift, rl = 256 >> cq_shift;
   const int tq = threadIdx.x & (cq - 1), tr = threadIdx.x >> cq_shift;
-  const long long c = ((long long)blockIdx.x * cq + tq) * 4;
+  const long long c = ((long long)blockIdx.x * cq + tq) * V;
   if (c >= channels) return;
-  typename F::K k[4];
+  typename F::K k[V];
 #pragma unroll
-  for (int j = 0; j < 4; ++j) k[j] = f.channel(c + j);
+  for (int j = 0; j < V; ++j) k[j] = f.channel(c + j);
   const long long r0 = (long long)blockIdx.y * rows_per_split;
   long long r1 = r0 + rows_per_split;
   if (r1 > rows) r1 = rows;
   long long r = r0 + tr;
+  auto apply = [&](const Vec16<T>& ra, const Vec16<T>& rb) {
+    float va[V], vb[V], o[V];
+    unpack16(ra, va);
+    if (NIN == 2) unpack16(rb, vb);
+#pragma unroll
+    for (int j = 0; j < V; ++j) o[j] = f.apply(k[j], va[j], NIN == 2 ? vb[j] : 0.f);
+    return pack16<T>(o);
+  };
   for (; r + 3LL * rl < r1; r += 4LL * rl) {
-    float4 va[4], vb[4];
+    Vec16<T> va[4], vb[4];
 #pragma unroll
     for (int u = 0; u < 4; ++u) {
       const long long off = (r + (long long)u * rl) * channels + c;
-      va[u] = *reinterpret_cast<const float4*>(a + off);
-      if (NIN == 2) vb[u] = *reinterpret_cast<const float4*>(b + off);
+      va[u] = load16(a + off);
+      if (NIN == 2) vb[u] = load16(b + off);
     }
 #pragma unroll
-    for (int u = 0; u < 4; ++u) {
-      const long long off = (r + (long long)u * rl) * channels + c;
-      *reinterpret_cast<float4*>(out + off) =
-          make_float4(f.apply(k[0], va[u].x, NIN == 2 ? vb[u].x : 0.f),
-                      f.apply(k[1], va[u].y, NIN == 2 ? vb[u].y : 0.f),
-                      f.apply(k[2], va[u].z, NIN == 2 ? vb[u].z : 0.f),
-                      f.apply(k[3], va[u].w, NIN == 2 ? vb[u].w : 0.f));
-    }
+    for (int u = 0; u < 4; ++u)
+      store16(out + (r + (long long)u * rl) * channels + c, apply(va[u], vb[u]));
   }
   for (; r < r1; r += rl) {
     const long long off = r * channels + c;
-    const float4 va = *reinterpret_cast<const float4*>(a + off);
-    float4 vb = make_float4(0.f, 0.f, 0.f, 0.f);
-    if (NIN == 2) vb = *reinterpret_cast<const float4*>(b + off);
-    *reinterpret_cast<float4*>(out + off) =
-        make_float4(f.apply(k[0], va.x, vb.x), f.apply(k[1], va.y, vb.y), f.apply(k[2], va.z, vb.z),
-                    f.apply(k[3], va.w, vb.w));
+    const Vec16<T> va = load16(a + off);
+    Vec16<T> vb;
+    if (NIN == 2) vb = load16(b + off);
+    store16(out + off, apply(va, vb));
   }
 }
 
-// Splits of the column path (rows handled per CTA): about six CTAs per SM over the vector
-// tiling's column blocks, at least 64 rows each, at most 512 splits.
+// Splits of the column path (rows handled per CTA): one wave of three CTAs per SM (the kernel's
+// registers allow that many with 16-bit data) over the vector tiling's column blocks, at least 32
+// rows each, at most 512 splits.  Where that would round to a few splits, two waves of them.
 inline int column_splits(long long rows, long long channels) {
   const long long col_blocks = column_tiling(channels).col_blocks;
-  long long splits = (6LL * device_info().sm_count + col_blocks - 1) / col_blocks;
-  const long long max_by_work = (rows + 63) / 64;
+  long long splits = 3LL * device_info().sm_count / col_blocks;
+  if (splits < 8) splits = (6LL * device_info().sm_count + col_blocks - 1) / col_blocks;
+  const long long max_by_work = (rows + 31) / 32;
   if (splits > max_by_work) splits = max_by_work;
   if (splits > 512) splits = 512;
   if (splits < 1) splits = 1;
   return static_cast<int>(splits);
+}
+
+// Rows of one CTA of a per-channel pass with `per_sm` CTAs per SM that walk `lanes` rows at once, a
+// multiple of the four rows that a thread has in flight.  Every thread first loads the constants of
+// its channels: with eight 16-bit channels per thread those cost as much as a few rows, so 16-bit
+// passes are six CTAs per SM (two waves of three, or three of two; the three relu(batch-norm)
+// gradient passes of a 64 x 56 x 56 x 256 f16 block took 155 us at 16 per SM, 97 so); fp32 ones keep
+// 16, which measured 4 to 8 % faster than one wave.
+inline long long apply_rows_per_split(long long rows, long long col_blocks, long long lanes,
+                                      long long per_sm) {
+  const long long ctas = per_sm * device_info().sm_count;
+  const long long splits = std::max(1LL, std::min(65535LL, ctas / col_blocks));
+  const long long unit = 4 * lanes;
+  return ((rows + splits - 1) / splits + unit - 1) / unit * unit;
 }
 
 // Scratch bytes for the (channel, split) partial sums of any op built on these.

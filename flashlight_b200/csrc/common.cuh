@@ -1,6 +1,7 @@
 // Shared host/device helpers of the flb200 kernel library (sm_100a only).
 #pragma once
 
+#include <type_traits>
 #include <cuda_runtime.h>
 #include <cuda_fp16.h>
 #include <cuda_bf16.h>
@@ -94,6 +95,43 @@ __device__ __forceinline__ Vec16<T> load16(const T* p) {
 template <typename T>
 __device__ __forceinline__ void store16(T* p, const Vec16<T>& r) {
   *reinterpret_cast<uint4*>(p) = *reinterpret_cast<const uint4*>(&r);
+}
+
+// Its values as fp32 and back; 16-bit values are converted two at a time.
+template <typename T>
+__device__ __forceinline__ void unpack16(const Vec16<T>& r, float* v) {
+  if constexpr (sizeof(T) == 4) {
+#pragma unroll
+    for (int j = 0; j < 4; ++j) v[j] = r.v[j];
+  } else {
+#pragma unroll
+    for (int j = 0; j < 8; j += 2) {
+      float2 f;
+      if constexpr (std::is_same<T, __half>::value)
+        f = __half22float2(*reinterpret_cast<const __half2*>(r.v + j));
+      else
+        f = __bfloat1622float2(*reinterpret_cast<const __nv_bfloat162*>(r.v + j));
+      v[j] = f.x;
+      v[j + 1] = f.y;
+    }
+  }
+}
+template <typename T>
+__device__ __forceinline__ Vec16<T> pack16(const float* v) {
+  Vec16<T> r;
+  if constexpr (sizeof(T) == 4) {
+#pragma unroll
+    for (int j = 0; j < 4; ++j) r.v[j] = v[j];
+  } else {
+#pragma unroll
+    for (int j = 0; j < 8; j += 2) {
+      if constexpr (std::is_same<T, __half>::value)
+        *reinterpret_cast<__half2*>(r.v + j) = __floats2half2_rn(v[j], v[j + 1]);
+      else
+        *reinterpret_cast<__nv_bfloat162*>(r.v + j) = __floats2bfloat162_rn(v[j], v[j + 1]);
+    }
+  }
+  return r;
 }
 
 __device__ __forceinline__ float warp_sum(float v) {

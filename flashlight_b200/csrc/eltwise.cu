@@ -23,24 +23,21 @@ __global__ void __launch_bounds__(kThreads) unary_vec_kernel(const T* __restrict
   const int64_t nvec = n / V;
   const int64_t stride = (int64_t)gridDim.x * kThreads;
   int64_t i = (int64_t)blockIdx.x * kThreads + threadIdx.x;
+  auto map = [&](const Vec16<T>& r) {
+    float v[V];
+    unpack16(r, v);
+#pragma unroll
+    for (int j = 0; j < V; ++j) v[j] = op(v[j]);
+    return pack16<T>(v);
+  };
   for (; i + (kUnroll - 1) * stride < nvec; i += kUnroll * stride) {
     Vec16<T> va[kUnroll];
 #pragma unroll
     for (int u = 0; u < kUnroll; ++u) va[u] = load16(a + (i + u * stride) * V);
 #pragma unroll
-    for (int u = 0; u < kUnroll; ++u) {
-      Vec16<T> vo;
-#pragma unroll
-      for (int j = 0; j < V; ++j) vo.v[j] = Num<T>::from_f(op(Num<T>::to_f(va[u].v[j])));
-      store16(out + (i + u * stride) * V, vo);
-    }
+    for (int u = 0; u < kUnroll; ++u) store16(out + (i + u * stride) * V, map(va[u]));
   }
-  for (; i < nvec; i += stride) {
-    Vec16<T> va = load16(a + i * V), vo;
-#pragma unroll
-    for (int j = 0; j < V; ++j) vo.v[j] = Num<T>::from_f(op(Num<T>::to_f(va.v[j])));
-    store16(out + i * V, vo);
-  }
+  for (; i < nvec; i += stride) store16(out + i * V, map(load16(a + i * V)));
   for (int64_t t = nvec * V + (int64_t)blockIdx.x * kThreads + threadIdx.x; t < n; t += stride)
     out[t] = Num<T>::from_f(op(Num<T>::to_f(a[t])));
 }
@@ -63,6 +60,14 @@ __global__ void __launch_bounds__(kThreads) binary_vec_kernel(const T* __restric
   const int64_t nvec = n / V;
   const int64_t stride = (int64_t)gridDim.x * kThreads;
   int64_t i = (int64_t)blockIdx.x * kThreads + threadIdx.x;
+  auto map = [&](const Vec16<T>& ra, const Vec16<T>& rb) {
+    float va[V], vb[V];
+    unpack16(ra, va);
+    unpack16(rb, vb);
+#pragma unroll
+    for (int j = 0; j < V; ++j) va[j] = op(va[j], vb[j]);
+    return pack16<T>(va);
+  };
   for (; i + (kUnroll - 1) * stride < nvec; i += kUnroll * stride) {
     Vec16<T> va[kUnroll], vb[kUnroll];
 #pragma unroll
@@ -71,21 +76,9 @@ __global__ void __launch_bounds__(kThreads) binary_vec_kernel(const T* __restric
       vb[u] = load16(b + (i + u * stride) * V);
     }
 #pragma unroll
-    for (int u = 0; u < kUnroll; ++u) {
-      Vec16<T> vo;
-#pragma unroll
-      for (int j = 0; j < V; ++j)
-        vo.v[j] = Num<T>::from_f(op(Num<T>::to_f(va[u].v[j]), Num<T>::to_f(vb[u].v[j])));
-      store16(out + (i + u * stride) * V, vo);
-    }
+    for (int u = 0; u < kUnroll; ++u) store16(out + (i + u * stride) * V, map(va[u], vb[u]));
   }
-  for (; i < nvec; i += stride) {
-    Vec16<T> va = load16(a + i * V), vb = load16(b + i * V), vo;
-#pragma unroll
-    for (int j = 0; j < V; ++j)
-      vo.v[j] = Num<T>::from_f(op(Num<T>::to_f(va.v[j]), Num<T>::to_f(vb.v[j])));
-    store16(out + i * V, vo);
-  }
+  for (; i < nvec; i += stride) store16(out + i * V, map(load16(a + i * V), load16(b + i * V)));
   for (int64_t t = nvec * V + (int64_t)blockIdx.x * kThreads + threadIdx.x; t < n; t += stride)
     out[t] = Num<T>::from_f(op(Num<T>::to_f(a[t]), Num<T>::to_f(b[t])));
 }

@@ -756,8 +756,9 @@ NATIVE(batchnorm) {
 NATIVE(batchnorm_add_relu_supported) {  // (input, addend, axes)
   const Tensor &in = x.tensor(0), &add = x.tensor(1);
   const flb200_batchnorm_desc d = bn_desc(in, x.at(2));
-  const bool shape_ok = d.inner > 1 || (channels_last(in) && d.channels % 8 == 0);
-  return PyBool_FromLong(in.scalar_type() == ScalarType::Float && shape_ok && same_layout(in, add) &&
+  const bool shape_ok = d.inner > 1 ? in.scalar_type() == ScalarType::Float
+                                    : channels_last(in) && d.channels % 8 == 0;
+  return PyBool_FromLong(shape_ok && same_layout(in, add) &&
                          add.scalar_type() == in.scalar_type() && dense(in) && aligned16(&in) && aligned16(&add));
 }
 // (input, addend, weight, bias, running_mean, running_var, axes, train, momentum, epsilon, stats or
