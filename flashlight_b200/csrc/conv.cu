@@ -60,6 +60,7 @@ int make_conv_geo(const char* name, const flb200_conv2d_desc* d, ConvGeo* g) {
   g->x_ps = g->x_cl ? d->C : 1;
   g->y_cs = g->y_cl ? 1 : g->HoWo;
   g->y_ps = g->y_cl ? d->Cout : 1;
+  g->operand = tc::kOperandTf32;
   return FLB200_OK;
 }
 
@@ -481,6 +482,18 @@ int narrow(const float* in, void* out, long long n, int dtype, cudaStream_t st) 
   FLB200_AFTER_LAUNCH("conv_narrow");
   return FLB200_OK;
 }
+// Channels-last 16-bit convolutions of a multiple of 8 channels need none of this in the tensor-core
+// modes: their operands go to the tensor cores as they are (products of 16-bit values are exact
+// in either case, the sums are fp32 in tensor memory, the result is rounded once).  The copies of a
+// residual block of 64 x 56 x 56 x 256 f16 alone took 0.84 of its 2.8 ms.
+bool native16(const flb200_conv2d_desc* d, ConvGeo* g, int which) {
+  if (d->dtype == FLB200_F32 || d->math_mode == FLB200_MATH_STRICT_F32) return false;
+  g->operand = tc::operand_of(d->dtype);
+  if (tc_conv_native16(*g, which)) return true;
+  g->operand = tc::kOperandTf32;
+  return false;
+}
+
 // byte offsets of the fp32 copies pass `which` needs, in the order of its tensors:
 // 0: x, w, bias, y | 1: grad_y, w, grad_x | 2: grad_y, x, grad_w, grad_bias
 struct WideCopies {
@@ -533,6 +546,9 @@ size_t flb200_conv2d_workspace_bytes(const flb200_conv2d_desc* d, int which) {
     need = max_sz(need, g.y_cl ? flb200_channel_sum_workspace_bytes((int64_t)g.N * g.HoWo, g.Cout, 1)
                                : flb200_channel_sum_workspace_bytes(g.N, g.Cout, g.HoWo));
   }
+  if (native16(d, &g, which))  // + the fp32 bias or its gradient
+    return up256c(max_sz(need, tc_conv_workspace_bytes(g, which))) + up256c((size_t)g.Cout * 4) +
+           wide_copies(g, which).total;
   if (d->math_mode != FLB200_MATH_STRICT_F32) need = max_sz(need, tc_conv_workspace_bytes(g, which));
   if (d->dtype != FLB200_F32 && which >= 0 && which <= 2)
     need = up256c(need) + wide_copies(g, which).total;  // fp32 copies of the 16-bit tensors
@@ -561,6 +577,18 @@ int flb200_conv2d_forward_cached(const flb200_conv2d_desc* d, const void* x, con
   if (int st = make_conv_geo("conv2d_forward", d, &g)) return st;
   FLB200_REQUIRE(x && w && y, "conv2d_forward: null tensor");
   cudaStream_t st = as_stream(stream);
+  if (native16(d, &g, 0)) {
+    const size_t bias_bytes = bias ? up256c((size_t)g.Cout * 4) : 0;
+    if (tc_operands_aligned(x, w, y, nullptr, workspace) && workspace_bytes >= bias_bytes &&
+        tc_conv_supported(g, 0, workspace_bytes - bias_bytes)) {
+      float* b32 = bias ? static_cast<float*>(workspace) : nullptr;
+      if (int rc = widen(bias, b32, g.Cout, d->dtype, st)) return rc;
+      return tc_conv_forward(g, static_cast<const float*>(x), static_cast<const float*>(w), b32,
+                             static_cast<float*>(y), static_cast<char*>(workspace) + bias_bytes,
+                             workspace_bytes - bias_bytes, st, nullptr);
+    }
+    g.operand = tc::kOperandTf32;
+  }
   if (d->dtype != FLB200_F32) {
     const WideCopies c = wide_copies(g, 0);
     if (!workspace || workspace_bytes < c.total)
@@ -596,7 +624,7 @@ size_t flb200_conv2d_stats_bytes(const flb200_conv2d_desc* d, int64_t* groups) {
   ConvGeo g;
   if (groups) *groups = 0;
   if (make_conv_geo("conv2d_stats_bytes", d, &g)) return 0;
-  if (d->math_mode == FLB200_MATH_STRICT_F32 || d->dtype != FLB200_F32) return 0;
+  if (d->math_mode == FLB200_MATH_STRICT_F32 || (d->dtype != FLB200_F32 && !native16(d, &g, 0))) return 0;
   const long long n = tc_conv_stats_groups(g);
   if (n == 0 || !tc_conv_supported(g, 0, tc_conv_workspace_bytes(g, 0))) return 0;
   if (groups) *groups = n;
@@ -612,19 +640,26 @@ int flb200_conv2d_forward_stats(const flb200_conv2d_desc* d, const void* x, cons
   if (int st = make_conv_geo("conv2d_forward_stats", d, &g)) return st;
   FLB200_REQUIRE(x && w && y && stats, "conv2d_forward_stats: null tensor");
   const size_t need = flb200_conv2d_stats_bytes(d, nullptr);
-  if (need == 0 || !tc_operands_aligned(x, w, y, bias, workspace) || !aligned16(stats) ||
-      !tc_conv_supported(g, 0, workspace_bytes))
+  const bool half = native16(d, &g, 0);
+  const size_t bias_bytes = half && bias ? up256c((size_t)g.Cout * 4) : 0;
+  if (need == 0 || workspace_bytes < bias_bytes || !tc_operands_aligned(x, w, y, bias, workspace) || !aligned16(stats) ||
+      !tc_conv_supported(g, 0, workspace_bytes - bias_bytes))
     return fail(FLB200_UNSUPPORTED,
-                "conv2d_forward_stats: needs a tensor-core route with a channels-last fp32 output "
+                "conv2d_forward_stats: needs a tensor-core route with a channels-last output "
                 "of a multiple of 32 channels, 16-byte aligned tensors and the forward workspace");
   if (stats_bytes < need)
     return fail(FLB200_WORKSPACE_TOO_SMALL, "conv2d_forward_stats: statistics buffer %zu < %zu",
                 stats_bytes, need);
   ConvStats cs{stats};
-  tc::X3Scope x3(d->math_mode == FLB200_MATH_F32X3);
-  return tc_conv_forward(g, static_cast<const float*>(x), static_cast<const float*>(w),
-                         static_cast<const float*>(bias), static_cast<float*>(y), workspace,
-                         workspace_bytes, as_stream(stream), cache, &cs);
+  tc::X3Scope x3(!half && d->math_mode == FLB200_MATH_F32X3);
+  const float* b32 = static_cast<const float*>(bias);
+  if (bias_bytes) {
+    if (int rc = widen(bias, static_cast<float*>(workspace), g.Cout, d->dtype, as_stream(stream))) return rc;
+    b32 = static_cast<const float*>(workspace);
+  }
+  return tc_conv_forward(g, static_cast<const float*>(x), static_cast<const float*>(w), b32,
+                         static_cast<float*>(y), workspace ? static_cast<char*>(workspace) + bias_bytes : nullptr,
+                         workspace_bytes - bias_bytes, as_stream(stream), cache, &cs);
 }
 
 int flb200_conv2d_backward_data(const flb200_conv2d_desc* d, const void* grad_y, const void* w,
@@ -642,6 +677,13 @@ int flb200_conv2d_backward_data_cached(const flb200_conv2d_desc* d, const void* 
   if (int st = make_conv_geo("conv2d_backward_data", d, &g)) return st;
   FLB200_REQUIRE(grad_y && w && grad_x, "conv2d_backward_data: null tensor");
   cudaStream_t st = as_stream(stream);
+  if (native16(d, &g, 1)) {
+    if (tc_operands_aligned(grad_y, w, grad_x, nullptr, workspace) &&
+        tc_conv_supported(g, 1, workspace_bytes))
+      return tc_conv_backward_data(g, static_cast<const float*>(grad_y), static_cast<const float*>(w),
+                                   static_cast<float*>(grad_x), workspace, workspace_bytes, st, nullptr);
+    g.operand = tc::kOperandTf32;
+  }
   if (d->dtype != FLB200_F32) {
     const WideCopies c = wide_copies(g, 1);
     if (!workspace || workspace_bytes < c.total)
@@ -687,6 +729,24 @@ int flb200_conv2d_backward_filter_bias_cached(const flb200_conv2d_desc* d, const
   if (int st = make_conv_geo("conv2d_backward_filter_bias", d, &g)) return st;
   FLB200_REQUIRE(grad_y && x && grad_w, "conv2d_backward_filter_bias: null tensor");
   cudaStream_t st = as_stream(stream);
+  if (native16(d, &g, 2)) {
+    if (tc_operands_aligned(grad_y, x, grad_w, nullptr, workspace) &&
+        tc_conv_supported(g, 2, workspace_bytes)) {
+      if (int rc = tc_conv_backward_filter(g, static_cast<const float*>(grad_y),
+                                           static_cast<const float*>(x), static_cast<float*>(grad_w),
+                                           workspace, workspace_bytes, st, nullptr))
+        return rc;
+      if (!grad_bias) return FLB200_OK;
+      float* gb32 = static_cast<float*>(workspace);
+      const size_t gb_bytes = up256c((size_t)g.Cout * 4);
+      if (int rc = flb200_channel_sum(grad_y, gb32, (int64_t)g.N * g.HoWo, g.Cout, 1, d->dtype,
+                                      static_cast<char*>(workspace) + gb_bytes,
+                                      workspace_bytes - gb_bytes, stream))
+        return rc;
+      return narrow(gb32, grad_bias, g.Cout, d->dtype, st);
+    }
+    g.operand = tc::kOperandTf32;
+  }
   if (d->dtype != FLB200_F32) {
     const WideCopies c = wide_copies(g, 2);
     if (!workspace || workspace_bytes < c.total)

@@ -128,11 +128,11 @@ __global__ void transpose_filter_kernel(const float* __restrict__ w, float* __re
 
 // ------------------------------------------------------------- map helpers
 int map2d(CUtensorMap* m, const float* base, long long inner, long long outer, long long ld,
-          int box_outer, bool mn_major) {
+          int box_outer, bool mn_major, int operand = tc::kOperandTf32) {
   const uint64_t dims[2] = {(uint64_t)inner, (uint64_t)outer};
-  const uint64_t strides[1] = {(uint64_t)ld * 4};
-  const uint32_t box[2] = {32, (uint32_t)box_outer};
-  return tc::make_tensor_map(m, base, 2, dims, strides, box, mn_major);
+  const uint64_t strides[1] = {(uint64_t)ld * (operand ? 2 : 4)};
+  const uint32_t box[2] = {(uint32_t)tc::stage_k(operand), (uint32_t)box_outer};
+  return tc::make_tensor_map(m, base, 2, dims, strides, box, mn_major, nullptr, operand);
 }
 int map3d(CUtensorMap* m, const float* base, long long inner, long long mid, long long outer,
           long long stride1, long long stride2, int box_mid, bool mn_major) {
@@ -142,11 +142,12 @@ int map3d(CUtensorMap* m, const float* base, long long inner, long long mid, lon
   return tc::make_tensor_map(m, base, 3, dims, strides, box, mn_major);
 }
 tc::Launch gemm_plan(long long M, long long N, long long k_iters, bool a_mn, bool b_mn, bool split_k,
-                     long long Z = 1) {
-  return tc::plan_launch(M, N, k_iters, Z, a_mn, b_mn, tc::kOperandTf32, split_k);
+                     long long Z = 1, int operand = tc::kOperandTf32) {
+  return tc::plan_launch(M, N, k_iters, Z, a_mn, b_mn, operand, split_k);
 }
-tc::OperandPlan plan_k_major(int rank) {  // dims [K, rows, ...]
+tc::OperandPlan plan_k_major(int rank, int operand = tc::kOperandTf32) {  // dims [K, rows, ...]
   tc::OperandPlan p{};
+  p.k_elems = tc::stage_k(operand);
   p.rank = rank; p.mn_major = 0; p.mn_dim = 1; p.k_dim = 0; p.k2_dim = -1; p.z_dim = -1;
   return p;
 }
@@ -167,8 +168,11 @@ bool direct_1x1(const ConvGeo& g) {
 //   backward filt  the channels-last patch route over the batch as one row of pixels
 bool cl_1x1(const ConvGeo& g) {
   return g.x_cl && g.y_cl && g.kW == 1 && g.kH == 1 && g.sx == 1 && g.sy == 1 && g.px == 0 &&
-         g.py == 0 && g.groups == 1 && g.C % 4 == 0 && g.Cout % 4 == 0 &&
-         (long long)g.N * g.HW < 0x7fffffffLL;
+         g.py == 0 && g.groups == 1 && g.C % (g.operand ? 8 : 4) == 0 &&
+         g.Cout % (g.operand ? 8 : 4) == 0 && (long long)g.N * g.HW < 0x7fffffffLL;
+}
+inline long long stages(long long k, const ConvGeo& g) {
+  return (k + tc::stage_k(g.operand) - 1) / tc::stage_k(g.operand);
 }
 
 struct GeneralSizes {
@@ -198,15 +202,22 @@ dim3 gather_grid(long long ld, int rows) {
 }  // namespace
 
 // -------------------------------------------------------------- interface
+bool tc_conv_native16(const ConvGeo& g, int which) {
+  // the boxes of the backward-filter pass are whole 64-channel groups (nhwc_map5)
+  if (which == 2 && ((g.C > 64 && g.C % 64 != 0) || (g.Cout > 64 && g.Cout % 64 != 0))) return false;
+  return g.operand != tc::kOperandTf32 && g.x_cl && g.y_cl && flb200_has_tensor_core_path() &&
+         patch_conv_supported(g);
+}
+
 size_t tc_conv_workspace_bytes(const ConvGeo& g, int which) {
   if (g.groups != 1) return 0;
   if (cl_1x1(g)) {
     const long long M = (long long)g.N * g.HW;
     if (which == 0)
-      return gemm_plan(M, g.Cout, (g.C + tc::kBK - 1) / tc::kBK, false, false, true).workspace_bytes;
+      return gemm_plan(M, g.Cout, stages(g.C, g), false, false, true, 1, g.operand).workspace_bytes;
     if (which == 1)
       return up256((size_t)g.C * g.Cout * 4) +
-             gemm_plan(M, g.C, (g.Cout + tc::kBK - 1) / tc::kBK, false, false, true).workspace_bytes;
+             gemm_plan(M, g.C, stages(g.Cout, g), false, false, true, 1, g.operand).workspace_bytes;
     return patch_conv_supported(g) ? patch_conv_workspace_bytes(g, 2) : 0;
   }
   if (direct_1x1(g)) {
@@ -271,15 +282,16 @@ int tc_conv_forward(const ConvGeo& g, const float* x, const float* w, const floa
   ep.alpha = 1.f;
   ep.bias_n = bias;
   if (cl_1x1(g)) {
-    const long long M = (long long)g.N * g.HW, k_iters = (g.C + tc::kBK - 1) / tc::kBK;
-    const tc::Launch L = gemm_plan(M, g.Cout, k_iters, false, false, !stats);
-    if (int rc = map2d(&ma, x, g.C, M, g.C, tc::kBM, false)) return rc;
-    if (int rc = map2d(&mb, w, g.C, g.Cout, g.C, L.b_box_rows(), false)) return rc;
+    const long long M = (long long)g.N * g.HW, k_iters = stages(g.C, g);
+    const tc::Launch L = gemm_plan(M, g.Cout, k_iters, false, false, !stats, 1, g.operand);
+    if (int rc = map2d(&ma, x, g.C, M, g.C, tc::kBM, false, g.operand)) return rc;
+    if (int rc = map2d(&mb, w, g.C, g.Cout, g.C, L.b_box_rows(), false, g.operand)) return rc;
+    ep.out16 = g.operand;
     ep.m_stride = g.Cout;
     ep.n_stride = 1;
     ep.stats = stats ? stats->matrix : nullptr;
-    return tc::run(ma, mb, plan_k_major(2), plan_k_major(2), ep, M, g.Cout, k_iters, 1, L, ws,
-                   ws_bytes, st);
+    return tc::run(ma, mb, plan_k_major(2, g.operand), plan_k_major(2, g.operand), ep, M, g.Cout,
+                   k_iters, 1, L, ws, ws_bytes, st, g.operand);
   }
   if (stats && tc_conv_stats_groups(g) == 0)
     return fail(FLB200_UNSUPPORTED, "conv2d_forward: this route takes no output statistics");
@@ -336,18 +348,23 @@ int tc_conv_backward_data(const ConvGeo& g, const float* gy, const float* w, flo
   ep.out = gx;
   ep.alpha = 1.f;
   if (cl_1x1(g)) {
-    const long long M = (long long)g.N * g.HW, k_iters = (g.Cout + tc::kBK - 1) / tc::kBK;
-    const tc::Launch L = gemm_plan(M, g.C, k_iters, false, false, true);
+    const long long M = (long long)g.N * g.HW, k_iters = stages(g.Cout, g);
+    const tc::Launch L = gemm_plan(M, g.C, k_iters, false, false, true, 1, g.operand);
     float* wt = static_cast<float*>(ws);
     const size_t wt_bytes = up256((size_t)g.C * g.Cout * 4);
     // wt[ci][co] = w[co][ci]
-    if (int rc = filter_permute(w, wt, g.Cout, g.C, 1, 0, 1, g.Cout, st)) return rc;
-    if (int rc = map2d(&ma, gy, g.Cout, M, g.Cout, tc::kBM, false)) return rc;
-    if (int rc = map2d(&mb, wt, g.Cout, g.C, g.Cout, L.b_box_rows(), false)) return rc;
+    if (int rc = g.operand ? filter_permute(reinterpret_cast<const uint16_t*>(w),
+                                            reinterpret_cast<uint16_t*>(wt), g.Cout, g.C, 1, 0, 1,
+                                            g.Cout, st)
+                           : filter_permute(w, wt, g.Cout, g.C, 1, 0, 1, g.Cout, st))
+      return rc;
+    if (int rc = map2d(&ma, gy, g.Cout, M, g.Cout, tc::kBM, false, g.operand)) return rc;
+    if (int rc = map2d(&mb, wt, g.Cout, g.C, g.Cout, L.b_box_rows(), false, g.operand)) return rc;
+    ep.out16 = g.operand;
     ep.m_stride = g.C;
     ep.n_stride = 1;
-    return tc::run(ma, mb, plan_k_major(2), plan_k_major(2), ep, M, g.C, k_iters, 1, L,
-                   static_cast<char*>(ws) + wt_bytes, ws_bytes - wt_bytes, st);
+    return tc::run(ma, mb, plan_k_major(2, g.operand), plan_k_major(2, g.operand), ep, M, g.C, k_iters,
+                   1, L, static_cast<char*>(ws) + wt_bytes, ws_bytes - wt_bytes, st, g.operand);
   }
   if (direct_1x1(g)) {
     if (int rc = map3d(&ma, gy, g.HW, g.Cout, g.N, g.HW, (long long)g.Cout * g.HW, 32, true))

@@ -16,9 +16,17 @@ struct ConvGeo {
   // img * C * HW + c * x_cs + pixel * x_ps; likewise y with Cout, HoWo, y_cs, y_ps.
   int x_cl, y_cl;
   int x_cs, x_ps, y_cs, y_ps;
+  int operand;  // tc::kOperandTf32: fp32 tensors; kOperandBf16 / kOperandF16: 16-bit tensors read
+                // by the tensor cores as they are (tc_conv_native16)
 };
 
 int make_conv_geo(const char* name, const flb200_conv2d_desc* d, ConvGeo* g);
+
+// Whether the tensor-core routes take this geometry on 16-bit tensors without fp32 copies:
+// channels-last on both sides, channels a multiple of 8 (16-byte pixels), for the filter gradient
+// of 64 from there on.  x, w, y and their
+// gradients are then of the 16-bit type behind the float pointers below; bias stays fp32.
+bool tc_conv_native16(const ConvGeo& g, int which);
 
 // which: 0 forward, 1 backward-data, 2 backward-filter.
 bool tc_conv_supported(const ConvGeo& g, int which, size_t workspace_bytes);

@@ -166,17 +166,21 @@ int x_to_nhwc(const ConvGeo& g, const float* x, float* xt, int cp, cudaStream_t 
 
 // Filter w[co][ci][tap] repacked to out[tap][rows][kp] with (rows, k) = (co, ci) for the
 // forward pass and (ci, co) for backward-data; k >= its extent is zero.
-int pack_filter(const float* w, float* out, int Cout, int C, int RS, int kp, bool rows_are_co,
+int pack_filter(const ConvGeo& g, const float* w, float* out, int kp, bool rows_are_co,
                 cudaStream_t st) {
-  const int rows = rows_are_co ? Cout : C;
-  if (kp != (rows_are_co ? C : Cout))  // (the copies of fl-order images are padded to 4 channels)
-    FLB200_CUDA_CHECK(cudaMemsetAsync(out, 0, (size_t)RS * rows * kp * 4, st));
-  return filter_permute(w, out, Cout, C, RS, (long long)rows * kp, rows_are_co ? kp : 1,
-                        rows_are_co ? 1 : kp, st);
+  const int rows = rows_are_co ? g.Cout : g.C;
+  const long long s_tap = (long long)rows * kp, s_co = rows_are_co ? kp : 1, s_ci = rows_are_co ? 1 : kp;
+  if (g.operand != tc::kOperandTf32)
+    return filter_permute(reinterpret_cast<const uint16_t*>(w), reinterpret_cast<uint16_t*>(out), g.Cout,
+                          g.C, g.RS, s_tap, s_co, s_ci, st);
+  if (kp != (rows_are_co ? g.C : g.Cout))  // (the copies of fl-order images are padded to 4 channels)
+    FLB200_CUDA_CHECK(cudaMemsetAsync(out, 0, (size_t)g.RS * rows * kp * 4, st));
+  return filter_permute(w, out, g.Cout, g.C, g.RS, s_tap, s_co, s_ci, st);
 }
 
 // gw[co][ci][tap] = sum over splits of partial[split][tap][co][ci]
-__global__ void wgrad_reduce_kernel(const float* __restrict__ partial, float* __restrict__ gw,
+template <typename T>
+__global__ void wgrad_reduce_kernel(const float* __restrict__ partial, T* __restrict__ gw,
                                     int Cout, int C, int RS, int splits) {
   const long long per_split = (long long)RS * Cout * C;
   for (long long t = (long long)blockIdx.x * blockDim.x + threadIdx.x; t < per_split;
@@ -186,32 +190,52 @@ __global__ void wgrad_reduce_kernel(const float* __restrict__ partial, float* __
     const int co = (int)(r2 % Cout), tap = (int)(r2 / Cout);
     float s = 0.f;
     for (int sp = 0; sp < splits; ++sp) s += partial[(long long)sp * per_split + t];
-    gw[((long long)co * C + ci) * RS + tap] = s;
+    gw[((long long)co * C + ci) * RS + tap] = Num<T>::from_f(s);
   }
 }
 
-// The same, four input channels per thread (C a multiple of 4, 16-byte aligned partial sums):
-// 16-byte loads of every split's slice, same order of additions.
-__global__ void wgrad_reduce_vec_kernel(const float4* __restrict__ partial, float* __restrict__ gw,
-                                        int Cout, int C4, int RS, int splits) {
+// The same for C a multiple of 4 and 16-byte aligned partial sums: a CTA owns 32 consecutive input
+// channels of one output channel and all taps; 16-byte loads of every split's slice (same order of
+// additions), and the result leaves through shared memory in the filter's own contiguous order,
+// instead of one word per tap stride.
+template <typename T>
+__global__ void __launch_bounds__(128)
+wgrad_reduce_vec_kernel(const float4* __restrict__ partial, T* __restrict__ gw, int Cout, int C4,
+                        int RS, int splits) {
+  extern __shared__ float red_tile[];  // [tap][32 channels + 1]
+  const int q0 = blockIdx.x * 8, co = blockIdx.y;
+  const int nq = min(8, C4 - q0);
   const long long per_split = (long long)RS * Cout * C4;
-  for (long long t = (long long)blockIdx.x * blockDim.x + threadIdx.x; t < per_split;
-       t += (long long)gridDim.x * blockDim.x) {
-    const int ci = 4 * (int)(t % C4);
-    const long long r2 = t / C4;
-    const int co = (int)(r2 % Cout), tap = (int)(r2 / Cout);
+  for (int i = threadIdx.x; i < RS * 8; i += 128) {
+    const int tap = i >> 3, q = i & 7;
+    if (q >= nq) continue;
+    const float4* src = partial + ((long long)tap * Cout + co) * C4 + q0 + q;
     float4 s = make_float4(0.f, 0.f, 0.f, 0.f);
+#pragma unroll 4
     for (int sp = 0; sp < splits; ++sp) {
-      const float4 v = partial[(long long)sp * per_split + t];
+      const float4 v = src[(long long)sp * per_split];
       s.x += v.x; s.y += v.y; s.z += v.z; s.w += v.w;
     }
-    float* dst = gw + ((long long)co * (4 * C4) + ci) * RS + tap;
-    if (RS == 1) {
-      *reinterpret_cast<float4*>(dst) = s;
-    } else {
-      dst[0] = s.x; dst[RS] = s.y; dst[2 * RS] = s.z; dst[3 * RS] = s.w;
-    }
+    float* t = red_tile + tap * 33 + 4 * q;
+    t[0] = s.x; t[1] = s.y; t[2] = s.z; t[3] = s.w;
   }
+  __syncthreads();
+  T* dst = gw + ((long long)co * (4 * C4) + 4 * q0) * RS;
+  for (int i = threadIdx.x; i < 4 * nq * RS; i += 128)
+    dst[i] = Num<T>::from_f(red_tile[(i % RS) * 33 + i / RS]);
+}
+template <typename T>
+int wgrad_reduce(const float* partial, T* gw, const ConvGeo& g, int splits, cudaStream_t st) {
+  const size_t smem = (size_t)g.RS * 33 * sizeof(float);
+  if (g.C % 4 == 0 && (reinterpret_cast<uintptr_t>(partial) & 15) == 0 && g.Cout <= 65535 &&
+      smem <= 48 * 1024)
+    wgrad_reduce_vec_kernel<T><<<dim3((unsigned)((g.C / 4 + 7) / 8), (unsigned)g.Cout), 128, smem, st>>>(
+        reinterpret_cast<const float4*>(partial), gw, g.Cout, g.C / 4, g.RS, splits);
+  else
+    wgrad_reduce_kernel<T><<<grid_for((long long)g.RS * g.Cout * g.C, 256), 256, 0, st>>>(
+        partial, gw, g.Cout, g.C, g.RS, splits);
+  FLB200_AFTER_LAUNCH("wgrad_reduce");
+  return FLB200_OK;
 }
 
 struct Patch { int QW, PH, NB, qw_shift, ph_shift; };
@@ -237,58 +261,63 @@ Patch pick_patch(int Wq, int Hq, int images) {
   p.ph_shift = log2i(p.PH);
   return p;
 }
-// 32-pixel patch (the K extent of one stage) for the backward-filter pass.
-void pick_k_patch(int Wq, int Hq, int* QW, int* PH) {
+// Patch of `pixels` (the K extent of one stage: 32, or 64 with 16-bit operands) for the
+// backward-filter pass.
+void pick_k_patch(int Wq, int pixels, int* QW, int* PH) {
   int q = 4;
-  while (q < Wq && q < 32) q *= 2;
-  int ph = 32 / q;
-  (void)Hq;
+  while (q < Wq && q < pixels) q *= 2;
   *QW = q;
-  *PH = ph;
+  *PH = pixels / q;
 }
 
 // 4-D NHWC map [c, w, h, n] of a tensor with cp channels per pixel.
-int nhwc_map(CUtensorMap* m, const float* base, int C, int cp, int W, int H, int N, int box_w,
-             int box_h, int box_n, int sx, int sy, int mode) {
+int nhwc_map(CUtensorMap* m, const float* base, int operand, int C, int cp, int W, int H, int N,
+             int box_w, int box_h, int box_n, int sx, int sy, int mode) {
+  const uint64_t es_ = operand ? 2 : 4;
   const uint64_t dims[4] = {(uint64_t)C, (uint64_t)W, (uint64_t)H, (uint64_t)N};
-  const uint64_t strides[3] = {(uint64_t)cp * 4, (uint64_t)W * cp * 4, (uint64_t)H * W * cp * 4};
-  const uint32_t box[4] = {32, (uint32_t)(box_w * sx), (uint32_t)(box_h * sy), (uint32_t)box_n};
+  const uint64_t strides[3] = {cp * es_, (uint64_t)W * cp * es_, (uint64_t)H * W * cp * es_};
+  const uint32_t box[4] = {(uint32_t)tc::stage_k(operand), (uint32_t)(box_w * sx),
+                           (uint32_t)(box_h * sy), (uint32_t)box_n};
   const uint32_t es[4] = {1, (uint32_t)sx, (uint32_t)sy, 1};
-  return tc::make_tensor_map(m, base, 4, dims, strides, box, mode, es);
+  return tc::make_tensor_map(m, base, 4, dims, strides, box, mode, es, operand);
 }
 
-// The same tensor with the channel index split into (32 contiguous channels, group of 32):
-// [32, w, h, n, ceil(C / 32)].  One box of nbox groups lands in shared memory as nbox
-// consecutive [pixels][32 channels] blocks, the layout of an MN-major operand.  Channels past
-// C of the last group read the neighbouring pixel (or the bytes after the tensor, which the
+// The same tensor with the channel index split into (one 128-byte run of channels, group):
+// [32 or 64, w, h, n, groups].  One box of nbox groups lands in shared memory as nbox
+// consecutive [pixels][channels of a group] blocks, the layout of an MN-major operand.  Channels
+// past C of the last group read the neighbouring pixel (or the bytes after the tensor, which the
 // callers keep inside their workspace); such rows / columns of the product are never stored.
-int nhwc_map5(CUtensorMap* m, const float* base, int C, int cp, int W, int H, int N, int box_w,
-              int box_h, int nbox, int sx, int sy) {
-  const uint64_t dims[5] = {32, (uint64_t)W, (uint64_t)H, (uint64_t)N, (uint64_t)((C + 31) / 32)};
-  const uint64_t strides[4] = {(uint64_t)cp * 4, (uint64_t)W * cp * 4, (uint64_t)H * W * cp * 4,
-                               128};
-  const uint32_t box[5] = {32, (uint32_t)(box_w * sx), (uint32_t)(box_h * sy), 1, (uint32_t)nbox};
+int nhwc_map5(CUtensorMap* m, const float* base, int operand, int C, int cp, int W, int H, int N,
+              int box_w, int box_h, int nbox, int sx, int sy) {
+  const uint64_t es_ = operand ? 2 : 4, run = (uint64_t)tc::stage_k(operand);
+  const uint64_t dims[5] = {(uint64_t)C < run ? (uint64_t)C : run, (uint64_t)W, (uint64_t)H, (uint64_t)N, (C + run - 1) / run};
+  const uint64_t strides[4] = {cp * es_, (uint64_t)W * cp * es_, (uint64_t)H * W * cp * es_, 128};
+  const uint32_t box[5] = {(uint32_t)run, (uint32_t)(box_w * sx), (uint32_t)(box_h * sy), 1,
+                           (uint32_t)nbox};
   const uint32_t es[5] = {1, (uint32_t)sx, (uint32_t)sy, 1, 1};
-  return tc::make_tensor_map(m, base, 5, dims, strides, box, tc::kMapMnMajor, es);
+  return tc::make_tensor_map(m, base, 5, dims, strides, box,
+                             operand ? tc::kMapKMajor : tc::kMapMnMajor, es, operand);
 }
 
 // Packed filter map [k, rows, taps].
-int filter_map(CUtensorMap* m, const float* base, int kext, int kp, int rows, int taps, int bn) {
+int filter_map(CUtensorMap* m, const float* base, int operand, int kext, int kp, int rows, int taps,
+               int box_rows) {
+  const uint64_t es_ = operand ? 2 : 4;
   const uint64_t dims[3] = {(uint64_t)kext, (uint64_t)rows, (uint64_t)taps};
-  const uint64_t strides[2] = {(uint64_t)kp * 4, (uint64_t)rows * kp * 4};
-  const uint32_t box[3] = {32, (uint32_t)bn, 1};
-  return tc::make_tensor_map(m, base, 3, dims, strides, box, tc::kMapKMajor);
+  const uint64_t strides[2] = {kp * es_, (uint64_t)rows * kp * es_};
+  const uint32_t box[3] = {(uint32_t)tc::stage_k(operand), (uint32_t)box_rows, 1};
+  return tc::make_tensor_map(m, base, 3, dims, strides, box, tc::kMapKMajor, nullptr, operand);
 }
 
-// CTA pairs (tc_pair.cuh) for 256-column tiles: each CTA then loads half of the filter tile.
-// Measured: 3x3 layers with 256-column tiles run 14 % faster on pairs (with the ring handed
-// over two sub-stages at a time); at 128 and 64 columns pairs are slower than single CTAs.
+// CTA pairs (tc_pair.cuh) for 256-column tiles: 3x3 layers 14 % faster, with the ring handed over
+// two sub-stages at a time; at 128 and 64 columns pairs measured slower than single CTAs.
 bool patch_uses_pairs(int bn) { return bn >= 256 && !tc::x3_enabled(); }
 
 // Fills the parts of the problem that do not depend on BN and launches with the BN that fits
 // the number of output channels.  The filter map must have been made with
 // filter_box_rows(bn) rows per box.
 struct PatchArgs {
+  int operand;
   Patch patch;
   int pix_w, pix_h, images, n_out, cchunks, a_w_mul, a_h_mul;
   int ncls;                                   // parity classes in this launch (1 = forward)
@@ -304,7 +333,8 @@ template <int BN>
 int run_patch(const CUtensorMap& ma, const CUtensorMap& mb, const PatchArgs& a, cudaStream_t st) {
   tc::PatchConvProblem<BN> p;
   p.a_mn_major = 0; p.b_mn_major = 0;
-  p.operand = tc::kOperandTf32;
+  p.operand = a.operand;
+  p.kel = tc::stage_k(a.operand);
   p.QW = a.patch.QW; p.PH = a.patch.PH; p.NB = a.patch.NB;
   p.qw_shift = a.patch.qw_shift; p.ph_shift = a.patch.ph_shift;
   p.tiles_q = (a.pix_w + p.QW - 1) / p.QW;
@@ -348,21 +378,22 @@ struct WgradPlan {
 // C = columns per tap, taps = number of taps (the window route passes 32 and kH).
 WgradPlan plan_wgrad(const ConvGeo& g, int C, int taps) {
   WgradPlan w;
-  pick_k_patch(g.Wo, g.Ho, &w.QW, &w.PH);
+  pick_k_patch(g.Wo, tc::stage_k(g.operand), &w.QW, &w.PH);
   w.tiles_q = (g.Wo + w.QW - 1) / w.QW;
   w.tiles_p = (g.Ho + w.PH - 1) / w.PH;
   w.k_iters = g.N * w.tiles_p * w.tiles_q;
-  const int cboxes = (C + 31) / 32;
-  if (cboxes >= 8) {
-    w.cn_shift = 3; w.tg = 1; w.tap_groups = taps; w.bn = 256;
+  const int box = tc::stage_k(g.operand), most = 256 / box;  // channels of a box, boxes of a tile
+  const int cboxes = (C + box - 1) / box;
+  if (cboxes >= most) {
+    w.cn_shift = log2i(most); w.tg = 1; w.tap_groups = taps; w.bn = 256;
     w.tiles_n = (C + 255) / 256;
   } else {
     w.cn_shift = log2i(cboxes);
-    const int tg_max = 8 >> w.cn_shift;
+    const int tg_max = most >> w.cn_shift;
     w.tap_groups = (taps + tg_max - 1) / tg_max;
     w.tg = (taps + w.tap_groups - 1) / w.tap_groups;
-    w.bn = tc::pick_bn(32 * (w.tg << w.cn_shift));
-    if (w.bn == 128 && 32 * (w.tg << w.cn_shift) > 128) w.bn = 256;
+    const int cols = box * (w.tg << w.cn_shift);
+    w.bn = cols <= 64 ? tc::pick_bn(cols) : (cols <= 128 ? 128 : 256);
     w.tiles_n = 1;
   }
   const long long out_tiles =
@@ -374,7 +405,10 @@ WgradPlan plan_wgrad(const ConvGeo& g, int C, int taps) {
 }
 WgradPlan plan_wgrad(const ConvGeo& g) { return plan_wgrad(g, g.C, g.RS); }
 
-inline int wgrad_a_boxes(int Cout) { return Cout >= tc::kBM ? tc::kBM / 32 : (Cout + 31) / 32; }
+inline int wgrad_a_boxes(const ConvGeo& g) {
+  const int box = tc::stage_k(g.operand);
+  return g.Cout >= tc::kBM ? tc::kBM / box : (g.Cout + box - 1) / box;
+}
 
 // Tap geometry of a backward-filter launch: tap t = (t / kW, t % kW) reads x at
 // (s * dil_x - pad_x, r * dil_y - pad_y) from the output pixel's origin.
@@ -385,13 +419,14 @@ int run_wgrad(const CUtensorMap& ma, const CUtensorMap& mb, const ConvGeo& g, co
               const WgradPlan& w, float* partial, cudaStream_t st) {
   tc::PatchWgradProblem<BN> p;
   p.a_mn_major = 1; p.b_mn_major = 1;
-  p.operand = tc::kOperandTf32;
+  p.operand = g.operand;
+  p.cb_shift = g.operand ? 6 : 5;
   p.QW = w.QW; p.PH = w.PH; p.tiles_q = w.tiles_q; p.tiles_p = w.tiles_p; p.images = g.N;
   p.M = g.Cout; p.N = tp.C;
   p.tiles_m = (g.Cout + tc::kBM - 1) / tc::kBM;
   p.tiles_n = w.tiles_n;
   p.ntaps = tp.ntaps; p.tap_groups = w.tap_groups; p.tg = w.tg; p.cn_shift = w.cn_shift;
-  p.a_nbox = wgrad_a_boxes(g.Cout);
+  p.a_nbox = wgrad_a_boxes(g);
   p.splits = w.splits; p.iters_per_split = w.ips; p.k_iters = w.k_iters;
   p.b_w_mul = g.sx; p.b_h_mul = g.sy;
   p.kW = tp.kW; p.dil_x = tp.dil_x; p.dil_y = tp.dil_y; p.pad_x = tp.pad_x; p.pad_y = tp.pad_y;
@@ -512,8 +547,9 @@ bool patch_conv_supported(const ConvGeo& g) {
         g.N <= 65535))
     return false;
   // channels-last tensors are read in place: their pixel stride must be a multiple of 16 bytes
-  if (g.x_cl && g.C % 4 != 0) return false;
-  if (g.y_cl && g.Cout % 4 != 0) return false;
+  const int vec = g.operand ? 8 : 4;
+  if (g.x_cl && g.C % vec != 0) return false;
+  if (g.y_cl && g.Cout % vec != 0) return false;
   return g.x_cl == g.y_cl;
 }
 
@@ -561,11 +597,12 @@ int patch_conv_forward(const ConvGeo& g0, const float* x, const float* w, const 
     }
     xt = xs.buf;
   }
-  if (int rc = pack_filter(w, wp, g.Cout, g.C, g.RS, cp, true, st)) return rc;
+  if (int rc = pack_filter(g, w, wp, cp, true, st)) return rc;
   PatchArgs a{};
   a.patch = pick_patch(g.Wo, g.Ho, g.N);
   a.pix_w = g.Wo; a.pix_h = g.Ho; a.images = g.N; a.n_out = g.Cout;
-  a.cchunks = (g.C + tc::kBK - 1) / tc::kBK;
+  a.operand = g.operand;
+  a.cchunks = (g.C + tc::stage_k(g.operand) - 1) / tc::stage_k(g.operand);
   a.a_w_mul = g.sx; a.a_h_mul = g.sy;
   a.ncls = 1;
   a.cls[0] = tc::PatchClass{tc::TapGrid{g.kH, g.kW, -g.py, g.dy, -g.px, g.dx, 0, 1, 0, 1, g.kW},
@@ -577,10 +614,10 @@ int patch_conv_forward(const ConvGeo& g0, const float* x, const float* w, const 
   a.stats = stats && g.y_cl ? stats->matrix : nullptr;
   const int bn = tc::pick_bn(g.Cout);
   CUtensorMap ma, mb;
-  if (int rc = nhwc_map(&ma, xt, g.C, cp, g.W, g.H, g.N, a.patch.QW, a.patch.PH, a.patch.NB, g.sx,
+  if (int rc = nhwc_map(&ma, xt, g.operand, g.C, cp, g.W, g.H, g.N, a.patch.QW, a.patch.PH, a.patch.NB, g.sx,
                         g.sy, tc::kMapKMajor))
     return rc;
-  if (int rc = filter_map(&mb, wp, g.C, cp, g.Cout, g.RS, filter_box_rows(bn))) return rc;
+  if (int rc = filter_map(&mb, wp, g.operand, g.C, cp, g.Cout, g.RS, filter_box_rows(bn))) return rc;
   return run_patch_any(bn, ma, mb, a, st);
 }
 
@@ -600,12 +637,11 @@ int patch_conv_backward_data(const ConvGeo& g, const float* gy, const float* w, 
     if (gs.flag) *gs.flag = 1;  // backward-filter of the same grad_y can take it from here
     gyt = gs.buf;
   }
-  if (int rc = pack_filter(w, wd, g.Cout, g.C, g.RS, cop, false, st)) return rc;
+  if (int rc = pack_filter(g, w, wd, cop, false, st)) return rc;
+  const int cchunks = (g.Cout + tc::stage_k(g.operand) - 1) / tc::stage_k(g.operand);
   const int bn = tc::pick_bn(g.C);
   CUtensorMap mb;
-  if (int rc = filter_map(&mb, wd, g.Cout, cop, g.C, g.RS, filter_box_rows(bn))) return rc;
-  // One launch per parity class (a, b) of the input pixel: h = p*sy + a, w = q*sx + b.  Only
-  // the taps with (a + py - r*dy) divisible by sy reach that class.
+  if (int rc = filter_map(&mb, wd, g.operand, g.Cout, cop, g.C, g.RS, filter_box_rows(bn))) return rc;
   // One launch per parity class (a, b) of the input pixel: h = p*sy + a, w = q*sx + b.  Only
   // the taps with (a + py - r*dy) divisible by sy reach that class; they form an arithmetic
   // progression in r (and likewise in s).  Classes that no tap reaches keep a zero gradient.
@@ -640,7 +676,7 @@ int patch_conv_backward_data(const ConvGeo& g, const float* gy, const float* w, 
   // launch writes the zeros of the other classes itself; otherwise clear gx first.
   const bool fill_cell = live == 1 && origin_live && empty > 0;
   if (empty > 0 && !fill_cell)
-    FLB200_CUDA_CHECK(cudaMemsetAsync(gx, 0, (size_t)g.N * g.C * g.HW * 4, st));
+    FLB200_CUDA_CHECK(cudaMemsetAsync(gx, 0, (size_t)g.N * g.C * g.HW * (g.operand ? 2 : 4), st));
   // The classes of one launch must have the same pixel extent (H, W multiples of the stride)
   // and fit the policy's class table; then ONE launch walks all of them, the classes of a
   // pixel patch as consecutive tiles, so that their interleaved stores meet in L2.  Otherwise
@@ -650,7 +686,8 @@ int patch_conv_backward_data(const ConvGeo& g, const float* gy, const float* w, 
                      g.W % g.sx == 0 && bn >= 256;
   PatchArgs a{};
   a.images = g.N; a.n_out = g.C;
-  a.cchunks = (g.Cout + tc::kBK - 1) / tc::kBK;
+  a.operand = g.operand;
+  a.cchunks = cchunks;
   a.a_w_mul = 1; a.a_h_mul = 1;
   a.out = gx; a.bias = nullptr;
   a.out_H = g.H; a.out_W = g.W; a.out_C = g.C;
@@ -660,7 +697,7 @@ int patch_conv_backward_data(const ConvGeo& g, const float* gy, const float* w, 
   auto launch = [&](PatchArgs& args) -> int {
     args.patch = pick_patch(args.pix_w, args.pix_h, g.N);
     CUtensorMap ma;
-    if (int rc = nhwc_map(&ma, gyt, g.Cout, cop, g.Wo, g.Ho, g.N, args.patch.QW, args.patch.PH,
+    if (int rc = nhwc_map(&ma, gyt, g.operand, g.Cout, cop, g.Wo, g.Ho, g.N, args.patch.QW, args.patch.PH,
                           args.patch.NB, 1, 1, tc::kMapKMajor))
       return rc;
     return run_patch_any(bn, ma, mb, args, st);
@@ -724,23 +761,19 @@ int patch_conv_backward_filter(const ConvGeo& g0, const float* gy, const float* 
   }
   float* partial = reinterpret_cast<float*>(base + off);
   CUtensorMap ma, mb;
-  if (int rc = nhwc_map5(&ma, gyt, g.Cout, cop, g.Wo, g.Ho, g.N, wp.QW, wp.PH,
-                         wgrad_a_boxes(g.Cout), 1, 1))
+  if (int rc = nhwc_map5(&ma, gyt, g.operand, g.Cout, cop, g.Wo, g.Ho, g.N, wp.QW, wp.PH,
+                         wgrad_a_boxes(g), 1, 1))
     return rc;
-  if (int rc = nhwc_map5(&mb, xt, g.C, cp, g.W, g.H, g.N, wp.QW, wp.PH, 1 << wp.cn_shift, g.sx,
+  if (int rc = nhwc_map5(&mb, xt, g.operand, g.C, cp, g.W, g.H, g.N, wp.QW, wp.PH, 1 << wp.cn_shift, g.sx,
                          g.sy))
     return rc;
   const WgradTaps tp{g.C, g.RS, g.kW, g.dx, g.dy, g.px, g.py};
   if (int rc = run_wgrad_any(ma, mb, g, tp, wp, partial, st)) return rc;
-  if (g.C % 4 == 0 && (reinterpret_cast<uintptr_t>(partial) & 15) == 0 &&
-      (g.RS != 1 || (reinterpret_cast<uintptr_t>(gw) & 15) == 0))
-    wgrad_reduce_vec_kernel<<<grid_for((long long)g.RS * g.Cout * (g.C / 4), 256), 256, 0, st>>>(
-        reinterpret_cast<const float4*>(partial), gw, g.Cout, g.C / 4, g.RS, wp.splits);
-  else
-    wgrad_reduce_kernel<<<grid_for((long long)g.RS * g.Cout * g.C, 256), 256, 0, st>>>(
-        partial, gw, g.Cout, g.C, g.RS, wp.splits);
-  FLB200_AFTER_LAUNCH("wgrad_reduce");
-  return FLB200_OK;
+  if (g.operand == tc::kOperandBf16)
+    return wgrad_reduce(partial, reinterpret_cast<__nv_bfloat16*>(gw), g, wp.splits, st);
+  if (g.operand == tc::kOperandF16)
+    return wgrad_reduce(partial, reinterpret_cast<__half*>(gw), g, wp.splits, st);
+  return wgrad_reduce(partial, gw, g, wp.splits, st);
 }
 
 // ------------------------------------------------------- row-window interface
@@ -757,7 +790,7 @@ bool window_conv_supported(const ConvGeo& g) {
   const WindowGeo wg = window_geo(g);
   const Patch pt = pick_patch(g.Wo, g.Ho, g.N);
   int qw, ph;
-  pick_k_patch(g.Wo, g.Ho, &qw, &ph);
+  pick_k_patch(g.Wo, tc::kBK, &qw, &ph);
   CUtensorMap m;
   const float* placeholder = reinterpret_cast<const float*>(uintptr_t(1) << 30);
   return window_map(&m, placeholder, wg, g.N, pt.QW, pt.PH, pt.NB, g.sx, g.sy) == 0 &&
@@ -797,7 +830,7 @@ int window_conv_forward(const ConvGeo& g, const float* x, const float* w, const 
   if (int rc = window_map(&ma, xtp, wg, g.N, a.patch.QW, a.patch.PH, a.patch.NB, g.sx, g.sy))
     return rc;
   const int bn = tc::pick_bn(g.Cout);
-  if (int rc = filter_map(&mb, wr, 32, 32, g.Cout, g.kH, filter_box_rows(bn))) return rc;
+  if (int rc = filter_map(&mb, wr, g.operand, 32, 32, g.Cout, g.kH, filter_box_rows(bn))) return rc;
   if (!xs.valid) {
     const long long total = (long long)g.N * wg.Hp * wg.Wp;
     nchw_to_nhwc4_pad_kernel<<<grid_for(total, 256), 256, 0, st>>>(
@@ -844,8 +877,8 @@ int window_conv_backward_filter(const ConvGeo& g, const float* gy, const float* 
   CUtensorMap ma, mb;
   if (int rc = window_rows_map(&mb, xtp, wg, g.N, wp.QW, wp.PH, 1 << wp.cn_shift, g.sx, g.sy, g.kH,
                                g.dy)) return rc;
-  if (int rc = nhwc_map5(&ma, gyt, g.Cout, cop, g.Wo, g.Ho, g.N, wp.QW, wp.PH,
-                         wgrad_a_boxes(g.Cout), 1, 1))
+  if (int rc = nhwc_map5(&ma, gyt, g.operand, g.Cout, cop, g.Wo, g.Ho, g.N, wp.QW, wp.PH,
+                         wgrad_a_boxes(g), 1, 1))
     return rc;
   if (!xs.valid) {
     const long long total = (long long)g.N * wg.Hp * wg.Wp;

@@ -53,6 +53,7 @@ struct PatchConvProblem {
   static constexpr int kMinBlocks = 1;
   int a_mn_major, b_mn_major;  // 0, 0
   int operand;
+  int kel;                     // channels per stage: 32 fp32, 64 16-bit
   // patch geometry (all powers of two, NB * PH * QW == 128)
   int QW, PH, NB, qw_shift, ph_shift;
   int tiles_q, tiles_p, tiles_b, tiles_n;
@@ -67,7 +68,7 @@ struct PatchConvProblem {
   int ncls;
   PatchClass cls[kMaxPatchClasses];
   // output: out[img][co][oh][ow], oh = p * oh_mul + oh_add, ow = q * ow_mul + ow_add
-  float* out;
+  float* out;                // 16-bit elements where operand says so (channels-last only)
   const float* bias;
   int out_H, out_W, out_C;
   int oh_mul, ow_mul;
@@ -111,10 +112,10 @@ struct PatchConvProblem {
                                             const Tile& t, LoadState& ls, uint32_t full_bar,
                                             char* a_dst, char* b_dst, int rank, int lane) const {
     if (lane == 0) {
-      int ca[4] = {ls.cc * kBK, ls.aw, ls.ah, t.b0};
+      int ca[4] = {ls.cc * kel, ls.aw, ls.ah, t.b0};
       tma_load_pair(ma, full_bar, a_dst, 4, ca);
     } else if (lane == 1) {
-      int cb[4] = {ls.cc * kBK, t.n0 + rank * (BN / 2), ls.wtap, 0};  // this CTA's half of B
+      int cb[4] = {ls.cc * kel, t.n0 + rank * (BN / 2), ls.wtap, 0};  // this CTA's half of B
       tma_load_pair(mb, full_bar, b_dst, 3, cb);
     }
     advance(ls);
@@ -150,9 +151,9 @@ struct PatchConvProblem {
                                        const Tile& t, LoadState& ls, uint64_t* bar, char* a_dst,
                                        char* b_dst, int, bool last, int, int) const {
     mbar_post_tx(bar, (kBM + BN) * kBK * 4, last);  // NB*PH*QW == 128 rows of 128 bytes + B tile
-    int ca[4] = {ls.cc * kBK, ls.aw, ls.ah, t.b0};
+    int ca[4] = {ls.cc * kel, ls.aw, ls.ah, t.b0};
     tma_load(ma, bar, a_dst, 4, ca);
-    int cb[4] = {ls.cc * kBK, t.n0, ls.wtap, 0};
+    int cb[4] = {ls.cc * kel, t.n0, ls.wtap, 0};
     tma_load(mb, bar, b_dst, 3, cb);
     advance(ls);
   }
@@ -169,12 +170,12 @@ struct PatchConvProblem {
     const int oh_add = fill_cell ? 0 : cls[t.c].oh_add, ow_add = fill_cell ? 0 : cls[t.c].ow_add;
     return ((long long)img * out_H + p * oh_mul + oh_add) * out_W + q * ow_mul + ow_add;
   }
-  // Pixel rows 4k + lane / 8 (k = 0..7) of the warp's staged chunk, 16 bytes per lane, bias
-  // added; STATS (uniform across the grid, so a copy of the loop each): per-channel sums of
-  // the stored values into the statistics matrix.  FILL: the strided backward-data whose only
-  // class with taps is (0, 0) — every pixel also writes the zeros of its cell, whole 128-byte
+  // Pixel rows 4k + lane / 8 (k = 0..7) of the warp's staged chunk, 4 channels per lane, bias
+  // added; STATS (uniform across the grid, so a copy of the loop each): per-channel sums of the
+  // stored values into the statistics matrix.  FILL: the strided backward-data whose only
+  // class with taps is (0, 0) — every pixel also writes the zeros of its cell, whole
   // rows like its own values, so the tensor needs no clearing pass.
-  template <bool STATS, bool FILL>
+  template <typename T, bool STATS, bool FILL>
   __device__ __forceinline__ void staged_pixels(const Tile& t, int row, int nb, float* stage,
                                                 int lane) const {
     float4 bq = make_float4(0.f, 0.f, 0.f, 0.f);
@@ -192,9 +193,12 @@ struct PatchConvProblem {
       float4 v = val[k];
       v.x += bq.x; v.y += bq.y; v.z += bq.z; v.w += bq.w;
       if (pix >= 0) {
-        float* dst = out + pix * out_C + nb + 4 * (lane & 7);
-        *reinterpret_cast<float4*>(dst) = v;
-        if (STATS) acc.add(v);
+        T* dst = reinterpret_cast<T*>(out) + pix * out_C + nb + 4 * (lane & 7);
+        if (STATS) {
+          v = epi_round<T>(v);
+          acc.add(v);
+        }
+        epi_store4(dst, v);
         if (FILL) {
           // this pixel owns its whole oh_mul x ow_mul cell: the other pixels receive zeros
           const int r = r_first + 4 * k + (lane >> 3);
@@ -202,8 +206,7 @@ struct PatchConvProblem {
           const int oh0 = (t.p0 + ((r >> qw_shift) & (PH - 1))) * oh_mul;
           for (int a = 0; a < oh_mul && oh0 + a < out_H; ++a)
             for (int b = a == 0 ? 1 : 0; b < ow_mul && ow0 + b < out_W; ++b)
-              *reinterpret_cast<float4*>(dst + ((long long)a * out_W + b) * out_C) =
-                  make_float4(0.f, 0.f, 0.f, 0.f);
+              epi_store4(dst + ((long long)a * out_W + b) * out_C, make_float4(0.f, 0.f, 0.f, 0.f));
         }
       }
     }
@@ -213,17 +216,40 @@ struct PatchConvProblem {
       acc.flush(stats, tile_m * 4 + (row >> 5), n_out, nb, lane, stage);
     }
   }
+  template <typename T>
+  __device__ __forceinline__ void store_cl(const Tile& t, int row, int nb, const float* v,
+                                           float* stage, int lane) const {
+    if (nb + 32 <= n_out && (out_C & 3) == 0) {
+      // through the warp's staging tile, 4 whole pixel rows per store instruction (tc_kernel.cuh)
+      epi_stage_write(stage, lane, v);
+      if (fill_cell) staged_pixels<T, false, true>(t, row, nb, stage, lane);
+      else if (stats) staged_pixels<T, true, false>(t, row, nb, stage, lane);
+      else staged_pixels<T, false, false>(t, row, nb, stage, lane);
+      __syncwarp();
+      return;
+    }
+    // the channel tail, one pixel per lane; the other pixels of a cell receive zeros
+    const long long pix = cl_pixel(t, row);
+    if (pix < 0) return;
+    const int q = t.q0 + (row & (QW - 1)), p = t.p0 + ((row >> qw_shift) & (PH - 1));
+    const int cell_h = fill_cell ? min(oh_mul, out_H - p * oh_mul) : 1;
+    const int cell_w = fill_cell ? min(ow_mul, out_W - q * ow_mul) : 1;
+    for (int a = 0; a < cell_h; ++a)
+      for (int b = 0; b < cell_w; ++b) {
+        T* dst = reinterpret_cast<T*>(out) + (pix + (long long)a * out_W + b) * out_C + nb;
+#pragma unroll
+        for (int j = 0; j < 32; ++j)
+          if (nb + j < n_out)
+            dst[j] = Num<T>::from_f(a == 0 && b == 0 ? v[j] + (bias ? bias[nb + j] : 0.f) : 0.f);
+      }
+  }
   __device__ __forceinline__ void store(const Tile& t, int row, int c0, const float* v,
                                         float* stage, int lane) const {
     const int nb = t.n0 + c0;
-    if (out_cl && nb + 32 <= n_out && (out_C & 3) == 0) {
-      // channels-last output: through the warp's staging tile, 4 whole 128-byte pixel rows per
-      // store instruction (see tc_kernel.cuh)
-      epi_stage_write(stage, lane, v);
-      if (fill_cell) staged_pixels<false, true>(t, row, nb, stage, lane);
-      else if (stats) staged_pixels<true, false>(t, row, nb, stage, lane);
-      else staged_pixels<false, false>(t, row, nb, stage, lane);
-      __syncwarp();
+    if (out_cl) {
+      if (operand == kOperandTf32) store_cl<float>(t, row, nb, v, stage, lane);
+      else if (operand == kOperandBf16) store_cl<__nv_bfloat16>(t, row, nb, v, stage, lane);
+      else store_cl<__half>(t, row, nb, v, stage, lane);
       return;
     }
     // row -> (image, p, q) inside the patch
@@ -231,39 +257,6 @@ struct PatchConvProblem {
     const int p = t.p0 + ((row >> qw_shift) & (PH - 1));
     const int img = t.b0 + (row >> (qw_shift + ph_shift));
     if (q >= pix_w || p >= pix_h || img >= images) return;
-    if (out_cl) {
-      // channels-last: the 32 columns of this chunk are 128 contiguous bytes of one pixel
-      const int oh0 = p * oh_mul + (fill_cell ? 0 : cls[t.c].oh_add);
-      const int ow0 = q * ow_mul + (fill_cell ? 0 : cls[t.c].ow_add);
-      const int cell_h = fill_cell ? oh_mul : 1, cell_w = fill_cell ? ow_mul : 1;
-      for (int a = 0; a < cell_h; ++a) {
-        if (oh0 + a >= out_H) break;
-        for (int b = 0; b < cell_w; ++b) {
-          if (ow0 + b >= out_W) break;
-          float* dst = out + (((long long)img * out_H + oh0 + a) * out_W + ow0 + b) * out_C + nb;
-          const bool mine = a == 0 && b == 0;  // the other pixels of a cell receive zeros
-          if (nb + 32 <= n_out && (out_C & 3) == 0) {
-#pragma unroll
-            for (int j = 0; j < 32; j += 4) {
-              float4 val = make_float4(0.f, 0.f, 0.f, 0.f);
-              if (mine) {
-                val = make_float4(v[j], v[j + 1], v[j + 2], v[j + 3]);
-                if (bias) {
-                  val.x += bias[nb + j]; val.y += bias[nb + j + 1];
-                  val.z += bias[nb + j + 2]; val.w += bias[nb + j + 3];
-                }
-              }
-              *reinterpret_cast<float4*>(dst + j) = val;
-            }
-          } else {
-#pragma unroll
-            for (int j = 0; j < 32; ++j)
-              if (nb + j < n_out) dst[j] = mine ? v[j] + (bias ? bias[nb + j] : 0.f) : 0.f;
-          }
-        }
-      }
-      return;
-    }
     const long long plane = (long long)out_H * out_W;
     if (fill_cell) {
       // Strided backward-data whose only class with taps is (0, 0): this pixel owns the whole
@@ -314,7 +307,8 @@ struct PatchWgradProblem {
   static constexpr int kMinBlocks = 1;
   int a_mn_major, b_mn_major;  // 1, 1
   int operand;
-  int QW, PH;                  // 32-pixel patch: QW * PH == 32
+  int QW, PH;                  // pixel patch of one stage: QW * PH == 32 (16-bit operands: 64)
+  int cb_shift;                // log2 of the channels of one box: 5 (16-bit operands: 6)
   int tiles_q, tiles_p, images;
   int tiles_m, tiles_n, M, N;  // M = output channels, N = input channels
   // The BN columns of a tile are tg taps x (1 << cn_shift) boxes of 32 input channels, so a
@@ -339,7 +333,7 @@ struct PatchWgradProblem {
     t.m0 = (r % tiles_m) * kBM; r /= tiles_m;
     t.tap0 = r * tg;
     t.ntap = min(tg, ntaps - t.tap0);
-    t.cn_live = min(1 << cn_shift, (N - t.n0 + 31) >> 5);
+    t.cn_live = min(1 << cn_shift, (N - t.n0 + (1 << cb_shift) - 1) >> cb_shift);
     t.k0 = t.split * iters_per_split;
     t.k1 = min(t.k0 + iters_per_split, k_iters);
   }
@@ -367,15 +361,16 @@ struct PatchWgradProblem {
     // 1 << cn_shift boxes of x.  Boxes past the last channel are zero-filled or hold a
     // neighbouring pixel's channels; they only reach accumulator rows / columns that the
     // epilogue never stores.
+    const int box_bytes = 128 << cb_shift;  // 32 pixels x 32 fp32 or 64 pixels x 64 16-bit channels
     if (lane == 0 && part == 0)
-      mbar_post_tx(bar, (a_nbox + (t.ntap << cn_shift)) * (kBK * 128), last);
+      mbar_post_tx(bar, (a_nbox + (t.ntap << cn_shift)) * box_bytes, last);
     __syncwarp();
     if (copy == 0) {
-      int ca[5] = {0, q0, p0, ls.img, t.m0 >> 5};
+      int ca[5] = {0, q0, p0, ls.img, t.m0 >> cb_shift};
       tma_load(ma, bar, a_dst, 5, ca);
     } else if (copy <= t.ntap) {
-      int cb[5] = {0, q0 * b_w_mul + ls.dw, p0 * b_h_mul + ls.dh, ls.img, t.n0 >> 5};
-      tma_load(mb, bar, b_dst + ((copy - 1) << cn_shift) * (kBK * 128), 5, cb);
+      int cb[5] = {0, q0 * b_w_mul + ls.dw, p0 * b_h_mul + ls.dh, ls.img, t.n0 >> cb_shift};
+      tma_load(mb, bar, b_dst + ((copy - 1) << cn_shift) * box_bytes, 5, cb);
     }
     if (++ls.qi == tiles_q) {
       ls.qi = 0;
@@ -383,27 +378,36 @@ struct PatchWgradProblem {
     }
   }
   __device__ __forceinline__ bool chunk_live(const Tile& t, int c0) const {
-    const int j = c0 >> 5;
+    const int j = c0 >> cb_shift;
     return (j >> cn_shift) < t.ntap && (j & ((1 << cn_shift) - 1)) < t.cn_live;
   }
-  __device__ __forceinline__ void store(const Tile& t, int row, int c0, const float* v, float*,
-                                        int) const {
-    const int m = t.m0 + row;
-    if (m >= M) return;
-    const int j = c0 >> 5;
+  __device__ __forceinline__ void store(const Tile& t, int row, int c0, const float* v,
+                                        float* stage, int lane) const {
+    const int m = t.m0 + row, m_first = m - lane;
+    const int j = c0 >> cb_shift;
     const int tap = t.tap0 + (j >> cn_shift);
-    const int nb = t.n0 + ((j & ((1 << cn_shift) - 1)) << 5);
-    float* dst = partial + (((long long)t.split * ntaps + tap) * M + m) * N + nb;
+    const int nb = t.n0 + ((j & ((1 << cn_shift) - 1)) << cb_shift) + (c0 & ((1 << cb_shift) - 1));
+    if (nb >= N || m_first >= M) return;
+    float* base = partial + (((long long)t.split * ntaps + tap) * M + m_first) * N + nb;
     if (nb + 32 <= N && (N & 3) == 0) {
+      // whole 128-byte rows per store instruction (tc_kernel.cuh)
+      epi_stage_write(stage, lane, v);
+      float4 val[8];
 #pragma unroll
-      for (int jj = 0; jj < 32; jj += 4)
-        *reinterpret_cast<float4*>(dst + jj) =
-            make_float4(v[jj], v[jj + 1], v[jj + 2], v[jj + 3]);
-    } else {
+      for (int k = 0; k < 8; ++k) val[k] = epi_stage_read(stage, lane, k);
+      float* dst = base + (long long)(lane >> 3) * N + 4 * (lane & 7);
 #pragma unroll
-      for (int jj = 0; jj < 32; ++jj)
-        if (nb + jj < N) dst[jj] = v[jj];
+      for (int k = 0; k < 8; ++k)
+        if (m_first + 4 * k + (lane >> 3) < M)
+          *reinterpret_cast<float4*>(dst + 4LL * k * N) = val[k];
+      __syncwarp();
+      return;
     }
+    if (m >= M) return;
+    float* dst = base + (long long)lane * N;
+#pragma unroll
+    for (int jj = 0; jj < 32; ++jj)
+      if (nb + jj < N) dst[jj] = v[jj];
   }
 };
 

@@ -50,3 +50,42 @@ def test_batchnorm_16bit_channels_last(dtype, shape):
         gz = tot * (y.detach().cpu().double() > 0)
         for g, want in zip(got, (gz,) + tuple(R.batchnorm_backward(gz, x.double(), w.double(), [2], 1e-5))):
             assert_close_scaled(g.float(), want, tol, "tail gradient")
+
+
+# N, C, H, W, Cout, k, stride, pad, dilation: 1 x 1 GEMM with K and N tails; one 64-channel stage and
+# one past it; fewer than 64 channels; 72 channels (the filter gradient widens); strided 1 x 1 and
+# 3 x 3 (classes of backward-data); more taps than a filter-gradient tile; a pixel count past the
+# patch; all tile widths
+@pytest.mark.parametrize("dtype", [torch.float16, torch.bfloat16])
+@pytest.mark.parametrize("case", [(2, 8, 5, 5, 32, 1, 1, 0, 1), (3, 64, 9, 9, 256, 1, 1, 0, 1),
+                                  (2, 128, 14, 14, 64, 3, 1, 1, 1), (2, 40, 13, 11, 24, 3, 1, 1, 1),
+                                  (2, 72, 7, 7, 136, 3, 1, 1, 1), (2, 128, 15, 14, 192, 1, 2, 0, 1),
+                                  (3, 64, 17, 18, 64, 3, 2, 1, 1), (2, 16, 12, 12, 32, 5, 1, 2, 1),
+                                  (4, 64, 33, 40, 128, 3, 1, 2, 2), (40, 256, 14, 14, 256, 3, 1, 1, 1),
+                                  (9, 512, 7, 7, 512, 3, 1, 1, 1)])
+def test_conv_16bit_channels_last(dtype, case):
+    from flashlight_b200 import _lib as L
+    from flashlight_b200.extension import B200AutogradExtension
+    N, C, H, W, Co, k, s, p, d = case
+    ext, tol = B200AutogradExtension(math_mode=L.MATH_TF32), TOL[dtype]
+    x = randn(N, C, H, W, seed=80).to(dtype)
+    w = (randn(Co, C, k, k, seed=81) * (1.0 / (C * k * k) ** 0.5)).to(dtype)
+    b = randn(Co, seed=82).to(dtype)
+    args = (s, s, p, p, d, d, 1)
+    stats = []
+    y = ext.conv2d(cl(x), w.cuda(), b.cuda(), *args, stats_out=stats)
+    want = R.conv2d(x.double(), w.double(), b.double(), *args)
+    assert y.dtype == dtype
+    assert_close_scaled(y.float(), want, tol, "conv y")
+    if stats:  # statistics of the stored values, taken in the epilogue
+        weight, bias = randn(Co, seed=84).abs() + 0.5, randn(Co, seed=85)
+        z = ext.batchnorm(y, weight.cuda(), bias.cuda(), None, None, [2], True, 0.0, 1e-5, conv_stats=stats[0])[0]
+        wz = R.batchnorm(y.cpu().double(), weight.double(), bias.double(), None, None, [2], True, 0.0, 1e-5)[0]
+        assert_close_scaled(z.float(), wz, tol, "bn from conv statistics")
+    gy = randn(*want.shape, seed=83).to(dtype)
+    gx = ext.conv2dBackwardData(cl(gy), cl(x), w.cuda(), *args)
+    assert_close_scaled(gx.float(), R.conv2d_backward_data(gy.double(), x.shape, w.double(), *args), tol, "conv dx")
+    gw, gb = ext.conv2dBackwardFilterBias(cl(gy), cl(x), w.cuda(), b.cuda(), *args)
+    wgw, wgb = R.conv2d_backward_filter_bias(gy.double(), x.double(), w.shape, True, *args)
+    assert_close_scaled(gw.float(), wgw, tol, "conv dw")
+    assert_close_scaled(gb.float(), wgb, tol, "conv db")
