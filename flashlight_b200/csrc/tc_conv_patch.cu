@@ -309,8 +309,33 @@ int filter_map(CUtensorMap* m, const float* base, int operand, int kext, int kp,
   return tc::make_tensor_map(m, base, 3, dims, strides, box, tc::kMapKMajor, nullptr, operand);
 }
 
-// CTA pairs (tc_pair.cuh) for 256-column tiles: 3x3 layers 14 % faster, with the ring handed over
-// two sub-stages at a time; at 128 and 64 columns pairs measured slower than single CTAs.
+// Tile width of a patch convolution over m_tiles pixel patches of k_iters stages each: the clocks
+// of a tile against how evenly the tiles fill the SMs, as in tc::plan_launch.  256-column tiles run
+// on CTA pairs (tc_pair.cuh; 3x3 layers 14 % faster, with the ring handed over two sub-stages at a
+// time); at 128 and 64 columns pairs measured slower than single CTAs.  A few images on 14 x 14
+// planes leave most of the chip idle at 256 columns.
+int pick_patch_bn(long long n_out, long long m_tiles, long long k_iters) {
+  struct Width { int bn, clocks; };
+  static const Width widths[4] = {{256, 530}, {128, 520}, {64, 440}, {32, 420}};
+  const int widest = tc::pick_bn(n_out);
+  const bool x3 = tc::x3_enabled();
+  const long long sm = device_info().sm_count > 0 ? device_info().sm_count : 148;
+  int best = widest;
+  double best_cost = -1.0;
+  for (const Width& w : widths) {
+    if (w.bn > widest) continue;
+    const bool pair = w.bn >= 256 && !x3;
+    const long long tiles = (pair ? (m_tiles + 1) / 2 : m_tiles) * ((n_out + w.bn - 1) / w.bn);
+    const long long units = pair ? sm / 2 : sm;
+    const double drain = 600.0 + 8.0 * w.bn, loop = (double)k_iters * w.clocks;
+    const double cost = (double)((tiles + units - 1) / units) * (loop > drain ? loop : drain) + drain;
+    if (best_cost < 0 || cost < best_cost) {
+      best_cost = cost;
+      best = w.bn;
+    }
+  }
+  return best;
+}
 bool patch_uses_pairs(int bn) { return bn >= 256 && !tc::x3_enabled(); }
 
 // Fills the parts of the problem that do not depend on BN and launches with the BN that fits
@@ -612,7 +637,7 @@ int patch_conv_forward(const ConvGeo& g0, const float* x, const float* w, const 
   a.oh_mul = 1; a.ow_mul = 1;
   a.out_cl = g.y_cl;
   a.stats = stats && g.y_cl ? stats->matrix : nullptr;
-  const int bn = tc::pick_bn(g.Cout);
+  const int bn = pick_patch_bn(g.Cout, patch_conv_stats_groups(g0) / 4, (long long)g.RS * a.cchunks);
   CUtensorMap ma, mb;
   if (int rc = nhwc_map(&ma, xt, g.operand, g.C, cp, g.W, g.H, g.N, a.patch.QW, a.patch.PH, a.patch.NB, g.sx,
                         g.sy, tc::kMapKMajor))
@@ -639,7 +664,11 @@ int patch_conv_backward_data(const ConvGeo& g, const float* gy, const float* w, 
   }
   if (int rc = pack_filter(g, w, wd, cop, false, st)) return rc;
   const int cchunks = (g.Cout + tc::stage_k(g.operand) - 1) / tc::stage_k(g.operand);
-  const int bn = tc::pick_bn(g.C);
+  const Patch whole = pick_patch((g.W + g.sx - 1) / g.sx, (g.H + g.sy - 1) / g.sy, g.N);
+  const long long m_tiles = (long long)g.sx * g.sy * (((g.W + g.sx - 1) / g.sx + whole.QW - 1) / whole.QW) *
+                            (((g.H + g.sy - 1) / g.sy + whole.PH - 1) / whole.PH) *
+                            ((g.N + whole.NB - 1) / whole.NB);
+  const int bn = pick_patch_bn(g.C, m_tiles, ((long long)g.RS * cchunks + g.sx * g.sy - 1) / (g.sx * g.sy));
   CUtensorMap mb;
   if (int rc = filter_map(&mb, wd, g.operand, g.Cout, cop, g.C, g.RS, filter_box_rows(bn))) return rc;
   // One launch per parity class (a, b) of the input pixel: h = p*sy + a, w = q*sx + b.  Only
