@@ -17,8 +17,10 @@
 // The reserve space (forward -> backward payload) holds the activated gates,
 // cell states, GRU candidates' recurrent part and the outputs of inner layers.
 #include <cstdlib>
+#include <vector>
 
 #include "common.cuh"
+#include "rnn_sequence.cuh"
 #include "rnn_step.cuh"
 
 namespace flb200 {
@@ -220,14 +222,31 @@ __global__ void copy_rows_kernel(const float* __restrict__ src, long long src_st
   dst[(long long)b * dst_stride + j] = src ? src[(long long)b * src_stride + j] : 0.f;
 }
 
-struct FwdWs { size_t zero, gh, bias, sync, mm, total; };
+// Shape and batch of a layer for the persistent kernels (rnn_sequence.cu).
+SeqShape seq_shape(const RnnDims& r) {
+  SeqShape s{};
+  s.T = r.T; s.B = r.B; s.H = r.H; s.G = r.G; s.dirs = r.dirs;
+  s.act = r.mode == FLB200_RNN_RELU ? 0 : 1;
+  s.out_stride = s.dy_stride = (long long)r.H * r.dirs;
+  return s;
+}
+// FLB200_RNN_PERSISTENT=0: a kernel per step
+bool persistent_off() {
+  static const bool off = [] {
+    const char* v = getenv("FLB200_RNN_PERSISTENT");
+    return v && v[0] == '0';
+  }();
+  return off;
+}
+
+struct FwdWs { size_t zero, gh, bias, seq, mm, total; };
 FwdWs fwd_ws(const RnnDims& r) {
   FwdWs w{};
   size_t off = 0;
   w.zero = off; off += up256((size_t)r.B * r.H * 4);
   w.gh = off; off += up256((size_t)r.B * r.GH * 4);
   w.bias = off; off += up256((size_t)r.GH * 4);
-  w.sync = off; off += 256;  // grid-barrier counter of the persistent recurrence kernel
+  w.seq = off; off += up256(rnn_sequence_scratch_bytes(seq_shape(r), false));
   w.mm = off;
   size_t m = 0;
   for (int l = 0; l < r.L; ++l) {
@@ -241,21 +260,21 @@ FwdWs fwd_ws(const RnnDims& r) {
   return w;
 }
 
-struct BwdWs { size_t dgx, dgh, dya, dyb, dh, dc, zero, sync, xbuf, red, mm, mm_bytes, red_bytes, total; };
+// dgx, dgh, dh, dc: one per direction, gx_stride / h_stride bytes apart
+struct BwdWs { size_t dgx, dgh, dya, dyb, dh, dc, zero, seq, red, mm, mm_bytes, red_bytes, gx_stride, h_stride, total; };
 BwdWs bwd_ws(const RnnDims& r) {
   BwdWs w{};
   size_t off = 0;
-  w.dgx = off; off += up256((size_t)r.TB * r.GH * 4);
-  w.dgh = off; if (r.mode == FLB200_RNN_GRU) off += up256((size_t)r.TB * r.GH * 4);
+  w.gx_stride = up256((size_t)r.TB * r.GH * 4);
+  w.h_stride = up256((size_t)r.B * r.H * 4);
+  w.dgx = off; off += w.gx_stride * r.dirs;
+  w.dgh = off; if (r.mode == FLB200_RNN_GRU) off += w.gx_stride * r.dirs;
   w.dya = off; off += up256((size_t)r.TB * r.H * r.dirs * 4);
   w.dyb = off; off += up256((size_t)r.TB * r.H * r.dirs * 4);
-  w.dh = off; off += up256((size_t)r.B * r.H * 4);
-  w.dc = off; off += up256((size_t)r.B * r.H * 4);
+  w.dh = off; off += w.h_stride * r.dirs;
+  w.dc = off; off += w.h_stride * r.dirs;
   w.zero = off; off += up256((size_t)r.B * r.H * 4);
-  w.sync = off; off += 256;  // grid-barrier counter of the persistent recurrence kernel
-  w.xbuf = off;              // its per-step exchange of partial sums
-  if (r.H == 256 || r.H == 512 || r.H == 1024)
-    off += up256(lstm_sequence_backward_scratch_bytes(r.H));
+  w.seq = off; off += up256(rnn_sequence_scratch_bytes(seq_shape(r), true));
   w.red = off;
   w.red_bytes = flb200_channel_sum_workspace_bytes(r.TB, r.GH, 1);
   off += up256(w.red_bytes);
@@ -358,6 +377,11 @@ static int rnn_forward_impl(const flb200_rnn_desc* d, const void* x, const void*
                               : reinterpret_cast<float*>(rs + RL.inner_y_off +
                                                          RL.inner_y_stride * (size_t)l);
     const long long out_stride = (long long)H * r.dirs;
+    // TF32 mode, where the device can hold it: the recurrences of the layer's directions in one
+    // persistent kernel for all T steps, W_hh resident in shared memory
+    SeqShape shape = seq_shape(r);
+    int rows = persistent_off() ? 0 : B;
+    std::vector<SeqJob> jobs;
     for (int dir = 0; dir < r.dirs; ++dir) {
       const int p = l * r.dirs + dir;
       const ParamOffsets po = param_offsets(r, p);
@@ -373,48 +397,41 @@ static int rnn_forward_impl(const flb200_rnn_desc* d, const void* x, const void*
         return rc;
       if (int rc = flb200_channel_bias_add(gates, bias, gates, r.TB, GH, 1, FLB200_F32, stream))
         return rc;
+      if (rows > 0) rows = rnn_sequence_rows(d->math_mode, shape, wf + po.w_hh, false);
+      // (GRU: the reserve tensor q takes the place of the cell states)
+      for (int b = 0; rows > 0 && b < B; b += rows)
+        jobs.push_back(SeqJob{wf + po.w_hh, gates + b * GH,
+                              (r.mode == FLB200_RNN_GRU ? qbuf : cells) + (long long)b * H,
+                              wf + po.b_hh + 2 * H, out + b * out_stride + (long long)dir * H,
+                              (hxf ? hxf + (long long)p * BH : zero) + (long long)b * H,
+                              (cxf ? cxf + (long long)p * BH : zero) + (long long)b * H,
+                              B - b < rows ? B - b : rows, dir});
+    }
+    if (rows > 0)
+      if (int rc = rnn_sequence_forward(shape, jobs.data(), (int)jobs.size(), ws + W.seq, st)) return rc;
+    for (int dir = 0; dir < r.dirs; ++dir) {
+      const int p = l * r.dirs + dir;
+      const ParamOffsets po = param_offsets(r, p);
+      float* gates = reinterpret_cast<float*>(rs + RL.per_p * (size_t)p);
+      float* cells = reinterpret_cast<float*>(rs + RL.per_p * (size_t)p + RL.cell_off);
+      float* qbuf = reinterpret_cast<float*>(rs + RL.per_p * (size_t)p + RL.q_off);
       const float* h_prev = hxf ? hxf + (long long)p * BH : zero;
       long long hp_stride = H;
       const float* c_prev = cxf ? cxf + (long long)p * BH : zero;
-      // LSTM in TF32 mode: one fused kernel per step (contraction + reduction + cell)
-      const bool fused = r.mode == FLB200_RNN_LSTM && lstm_step_supported(d->math_mode, B, H);
-      CUtensorMap map_whh;
-      if (fused)
-        if (int rc = lstm_step_weight_map(&map_whh, wf + po.w_hh, H)) return rc;
-      // ... or, where the device can hold the whole launch at once, ONE persistent kernel for
-      // all T steps with W_hh resident in shared memory (FLB200_RNN_PERSISTENT=0: per step)
-      static const bool persistent_off = [] {
-        const char* v = getenv("FLB200_RNN_PERSISTENT");
-        return v && v[0] == '0';
-      }();
       int first_step = 0;
-      if (r.mode != FLB200_RNN_LSTM && !persistent_off &&
-          lstm_sequence_supported(d->math_mode, B, H, r.G)) {
-        // GRU and the plain cells: the same persistent kernel with three gates / one; the
-        // GRU's reserve tensor q takes the place of the cell states
-        const bool gru = r.mode == FLB200_RNN_GRU;
-        if (int rc = lstm_step_weight_map(&map_whh, wf + po.w_hh, H, r.G)) return rc;
-        if (int rc = lstm_sequence_forward(
-                map_whh, gates, gru ? qbuf : nullptr, out + (long long)dir * H, out_stride, h_prev,
-                nullptr, reinterpret_cast<unsigned*>(ws + W.sync), T, B, H, dir, 0, -1, st, r.G,
-                gru ? wf + po.b_hh + 2 * H : nullptr, r.mode == FLB200_RNN_RELU ? 0 : 1))
-          return rc;
-        const int t_last = dir == 0 ? T - 1 : 0;
-        h_prev = out + (long long)t_last * B * out_stride + (long long)dir * H;
-        hp_stride = out_stride;
-        first_step = T;
-      }
-      if (fused && !persistent_off && lstm_sequence_supported(d->math_mode, B, H)) {
-        if (int rc = lstm_sequence_forward(
-                map_whh, gates, cells, out + (long long)dir * H, out_stride, h_prev, c_prev,
-                reinterpret_cast<unsigned*>(ws + W.sync), T, B, H, dir, 0, -1, st))
-          return rc;
+      if (rows > 0) {
         const int t_last = dir == 0 ? T - 1 : 0;
         h_prev = out + (long long)t_last * B * out_stride + (long long)dir * H;
         hp_stride = out_stride;
         c_prev = cells + (long long)t_last * BH;
         first_step = T;
       }
+      // otherwise an LSTM in TF32 mode: one fused kernel per step (contraction + reduction + cell)
+      const bool fused = first_step < T && r.mode == FLB200_RNN_LSTM &&
+                         lstm_step_supported(d->math_mode, B, H);
+      CUtensorMap map_whh;
+      if (fused)
+        if (int rc = lstm_step_weight_map(&map_whh, wf + po.w_hh, H)) return rc;
       for (int step = first_step; step < T; ++step) {
         const int t = dir == 0 ? step : T - 1 - step;
         float* g_t = gates + (long long)t * B * GH;
@@ -498,11 +515,11 @@ static int rnn_backward_impl(const flb200_rnn_desc* d, const void* x, const void
   float* gwf = static_cast<float*>(grad_w);
   const float* hxf = static_cast<const float*>(hx);
   const float* cxf = static_cast<const float*>(cx);
-  float* dgx = reinterpret_cast<float*>(ws + W.dgx);
-  float* dgh = r.mode == FLB200_RNN_GRU ? reinterpret_cast<float*>(ws + W.dgh) : dgx;
   float* dy_bufs[2] = {reinterpret_cast<float*>(ws + W.dya), reinterpret_cast<float*>(ws + W.dyb)};
-  float* dh = reinterpret_cast<float*>(ws + W.dh);
-  float* dc = reinterpret_cast<float*>(ws + W.dc);
+  auto dgx_of = [&](int dir) { return reinterpret_cast<float*>(ws + W.dgx + W.gx_stride * dir); };
+  auto dgh_of = [&](int dir) {
+    return r.mode == FLB200_RNN_GRU ? reinterpret_cast<float*>(ws + W.dgh + W.gx_stride * dir) : dgx_of(dir);
+  };
   float* zero = reinterpret_cast<float*>(ws + W.zero);
   void* red = ws + W.red;
   void* mmws = ws + W.mm;
@@ -527,38 +544,48 @@ static int rnn_backward_impl(const flb200_rnn_desc* d, const void* x, const void
     // layer, else what the layer above left in the ping-pong buffer.
     const float* dy_l = l == r.L - 1 ? static_cast<const float*>(grad_y) : dy_bufs[(l + 1) & 1];
     float* din = l == 0 ? static_cast<float*>(grad_x) : dy_bufs[l & 1];
+    // TF32 mode, where the device can hold it: the recurrences of the layer's directions in one
+    // persistent kernel (GRU: q in the place of the cell states, h0 in the place of c0, the recurrent
+    // side's gate gradients in dgh; plain cells: gates only)
+    const bool lstm = r.mode == FLB200_RNN_LSTM, gru = r.mode == FLB200_RNN_GRU;
+    SeqShape shape = seq_shape(r);
+    int rows = persistent_off() ? 0 : B;
+    for (int dir = 0; dir < r.dirs && rows > 0; ++dir)
+      rows = rnn_sequence_rows(d->math_mode, shape, wf + param_offsets(r, l * r.dirs + dir).w_hh, true);
+    const bool persistent = rows > 0;
+    std::vector<SeqBwdJob> jobs;
+    for (int dir = 0; dir < r.dirs && persistent; ++dir) {
+      const int p = l * r.dirs + dir;
+      const float* cells = reinterpret_cast<const float*>(rs + RL.per_p * (size_t)p +
+                                                          (gru ? RL.q_off : RL.cell_off));
+      const float* gates = reinterpret_cast<const float*>(rs + RL.per_p * (size_t)p);
+      const float* first = lstm ? cxf : hxf;
+      const float* ghy = static_cast<const float*>(grad_hy);
+      const float* gcy = lstm ? static_cast<const float*>(grad_cy) : nullptr;
+      float* dh = reinterpret_cast<float*>(ws + W.dh + W.h_stride * dir);
+      float* dc = reinterpret_cast<float*>(ws + W.dc + W.h_stride * dir);
+      for (int b = 0; b < B; b += rows) {
+        const long long at = (long long)p * BH + (long long)b * H, bh = (long long)b * H;
+        jobs.push_back(SeqBwdJob{wf + param_offsets(r, p).w_hh, gates + b * GH, cells + bh,
+                                 first ? first + at : zero + bh, out + b * ys + (long long)dir * H,
+                                 dy_l ? dy_l + b * ys + (long long)dir * H : nullptr,
+                                 ghy ? ghy + at : nullptr, gcy ? gcy + at : nullptr,
+                                 dgx_of(dir) + b * GH, dgh_of(dir) + b * GH, dh + bh, dc + bh,
+                                 B - b < rows ? B - b : rows, dir});
+      }
+    }
+    if (persistent)
+      if (int rc = rnn_sequence_backward(shape, jobs.data(), (int)jobs.size(), ws + W.seq, st)) return rc;
     for (int dir = 0; dir < r.dirs; ++dir) {
       const int p = l * r.dirs + dir;
       const ParamOffsets po = param_offsets(r, p);
       const float* gates = reinterpret_cast<const float*>(rs + RL.per_p * (size_t)p);
       const float* cells = reinterpret_cast<const float*>(rs + RL.per_p * (size_t)p + RL.cell_off);
       const float* qbuf = reinterpret_cast<const float*>(rs + RL.per_p * (size_t)p + RL.q_off);
-      // LSTM in TF32 mode on a device that holds the whole launch at once: the recurrence of
-      // all T steps in ONE persistent kernel (FLB200_RNN_PERSISTENT=0: kernels per step)
-      static const bool persistent_off = [] {
-        const char* v = getenv("FLB200_RNN_PERSISTENT");
-        return v && v[0] == '0';
-      }();
-      const bool lstm = r.mode == FLB200_RNN_LSTM, gru = r.mode == FLB200_RNN_GRU;
-      const bool persistent = !persistent_off &&
-                              lstm_sequence_backward_supported(d->math_mode, B, H, r.G);
-      if (persistent) {
-        // (GRU: q in the place of the cell states, h0 in the place of c0, no cell-state
-        // gradients, the recurrent side's gate gradients in dgh; plain cells: gates only)
-        CUtensorMap map_wt;
-        if (int rc = lstm_sequence_weight_map_transposed(&map_wt, wf + po.w_hh, H, r.G)) return rc;
-        const float* first_state = lstm ? (cxf ? cxf + (long long)p * BH : zero)
-                                        : (hxf ? hxf + (long long)p * BH : zero);
-        if (int rc = lstm_sequence_backward(
-                map_wt, gates, lstm ? cells : qbuf, first_state,
-                dy_l ? dy_l + (long long)dir * H : nullptr, ys,
-                grad_hy ? static_cast<const float*>(grad_hy) + (long long)p * BH : nullptr,
-                lstm && grad_cy ? static_cast<const float*>(grad_cy) + (long long)p * BH : nullptr,
-                dgx, dh, dc, reinterpret_cast<float*>(ws + W.xbuf),
-                reinterpret_cast<unsigned*>(ws + W.sync), T, B, H, dir, st, r.G, dgh,
-                out + (long long)dir * H, ys, r.mode == FLB200_RNN_RELU ? 0 : 1))
-          return rc;
-      }
+      float* dgx = dgx_of(dir);
+      float* dgh = dgh_of(dir);
+      float* dh = reinterpret_cast<float*>(ws + W.dh + W.h_stride * dir);
+      float* dc = reinterpret_cast<float*>(ws + W.dc + W.h_stride * dir);
       if (!persistent) {
       copy_rows_kernel<<<cell_grid, 256, 0, st>>>(
           grad_hy ? static_cast<const float*>(grad_hy) + (long long)p * BH : nullptr, H, dh, H, B,
@@ -700,35 +727,43 @@ int flb200_rnn_backward_dropout(const flb200_rnn_desc* d, const void* x, const v
 }
 
 // ---- self-test of the bounded waits -------------------------------------------------------
+static SeqShape selftest_shape() {
+  SeqShape s{};
+  s.T = 3; s.B = 4; s.H = 256; s.G = 4; s.dirs = 1;
+  s.out_stride = s.H;
+  return s;
+}
 size_t flb200_selftest_bounded_wait_workspace_bytes(void) {
-  // W_hh [4H][H], gates [T][B][4H], cells and output [T][B][H], h0 / c0 [B][H], the counter
-  const size_t H = 256, B = 4, T = 3;
-  return (4 * H * H + T * B * 4 * H + 2 * T * B * H + 2 * B * H) * 4 + 256;
+  // W_hh [4H][H], gates [T][B][4H], cells and output [T][B][H], h0 / c0 [B][H], the exchange buffer
+  const SeqShape s = selftest_shape();
+  const size_t H = s.H, B = s.B, T = s.T;
+  return (4 * H * H + T * B * 4 * H + 2 * T * B * H + 2 * B * H) * 4 + rnn_sequence_scratch_bytes(s, false);
 }
 
 int flb200_selftest_bounded_wait(double budget_ms, void* workspace, size_t workspace_bytes,
                                  void* stream) {
-  const int H = 256, B = 4, T = 3;
+  const SeqShape s = selftest_shape();
+  const int H = s.H, B = s.B, T = s.T;
   FLB200_REQUIRE(workspace && workspace_bytes >= flb200_selftest_bounded_wait_workspace_bytes(),
                  "selftest_bounded_wait: workspace too small");
   FLB200_REQUIRE(budget_ms > 0.0 && budget_ms <= 1000.0, "selftest_bounded_wait: budget in (0, 1000] ms");
-  if (!lstm_sequence_supported(FLB200_MATH_TF32, B, H))
+  float* w = static_cast<float*>(workspace);
+  if (rnn_sequence_rows(FLB200_MATH_TF32, s, w, false) < B)
     return fail(FLB200_UNSUPPORTED, "selftest_bounded_wait: the persistent kernel cannot run here");
   cudaStream_t st = as_stream(stream);
   FLB200_CUDA_CHECK(cudaMemsetAsync(workspace, 0, flb200_selftest_bounded_wait_workspace_bytes(), st));
-  float* w = static_cast<float*>(workspace);
-  float* gates = w + 4 * H * H;
-  float* cells = gates + T * B * 4 * H;
-  float* out = cells + T * B * H;
-  float* h0 = out + T * B * H;
-  float* c0 = h0 + B * H;
-  unsigned* sync = reinterpret_cast<unsigned*>(c0 + B * H);
-  CUtensorMap map;
-  if (int rc = lstm_step_weight_map(&map, w, H)) return rc;
-  // CTA 0 never arrives at the grid barrier: every CTA's wait for step 1 runs out after
-  // budget_ms (at ~2 GHz), raises the status flag and the kernel still ends by itself
-  return lstm_sequence_forward(map, gates, cells, out, H, h0, c0, sync, T, B, H, 0,
-                               (long long)(budget_ms * 2.0e6), 0, st);
+  SeqJob job{};
+  job.w_hh = w;
+  job.gates = w + 4 * H * H;
+  job.cells = job.gates + T * B * 4 * H;
+  job.out = job.cells + T * B * H;
+  float* h0 = job.out + T * B * H;
+  job.h0 = h0;
+  job.c0 = h0 + B * H;
+  job.B = B;
+  // CTA 0 never publishes its states: every CTA's wait in step 1 runs out after budget_ms (at
+  // ~2 GHz), raises the status flag and the kernel still ends by itself
+  return rnn_sequence_forward(s, &job, 1, h0 + 2 * B * H, st, (long long)(budget_ms * 2.0e6), 0);
 }
 
 }  // extern "C"
