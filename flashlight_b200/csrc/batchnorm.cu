@@ -330,7 +330,9 @@ bn_add_relu_apply_cl_kernel(const T* __restrict__ x, const T* __restrict__ adden
     unsigned bits = 0;
 #pragma unroll
     for (int j = 0; j < 8; ++j) {
-      const float v = bn_value(a[j], m[j], sc[j], sh[j]) + s[j];
+      // rounded to the tensor's type like the result of batchnorm alone: of values within a rounding
+      // error of zero, relu must keep the same ones as the chain of operators does
+      const float v = Num<T>::to_f(Num<T>::from_f(bn_value(a[j], m[j], sc[j], sh[j]))) + s[j];
       z[j] = v > 0.f ? v : (v != v ? v : 0.f);
       bits |= (v > 0.f ? 1u : 0u) << j;
     }

@@ -42,6 +42,9 @@ def test_batchnorm_16bit_channels_last(dtype, shape):
         return
     y, mask, sm, sv = ext.batchnormAddRelu(cl(x), cl(s), w.cuda(), b.cuda(), None, None, [2], True, 0.0, 1e-5)
     assert_close_scaled(y.float(), torch.relu(wy + s.double()), tol, "tail y")
+    from flashlight_b200 import functions as F
+    chain = F.relu(F.add(ext.batchnorm(cl(x), w.cuda(), b.cuda(), None, None, [2], True, 0.0, 1e-5)[0], cl(s)))
+    assert torch.equal(y, chain)  # the same values, so the same relu predicate, as the operators
     ga, gb = randn(*shape, seed=98).to(dtype), randn(*shape, seed=99).to(dtype)
     for second in (gb, None):
         got = ext.batchnormAddReluBackward(mask, cl(ga), None if second is None else cl(second), sm, sv, cl(x),
