@@ -377,8 +377,7 @@ bn_tail_backward_reduce_cl_kernel(const T* __restrict__ x, const T* __restrict__
     const long long r0 = (long long)blockIdx.y * rows_per_split;
     long long r1 = r0 + rows_per_split;
     if (r1 > rows) r1 = rows;
-#pragma unroll 2
-    for (long long r = r0 + tr; r < r1; r += rl) {
+    auto row = [&](long long r, float* t0, float* t1) {
       const long long off = r * channels + c;
       float xv[8], av[8];
       load8(x + off, xv);
@@ -395,11 +394,25 @@ bn_tail_backward_reduce_cl_kernel(const T* __restrict__ x, const T* __restrict__
       for (int j = 0; j < 8; ++j) {
         // what is reduced is what the tensor holds
         rv[j] = Num<T>::to_f(Num<T>::from_f((bits >> j) & 1u ? av[j] : 0.f));
-        s0[j] += rv[j];
-        s1[j] += rv[j] * (xv[j] - m[j]);
+        t0[j] += rv[j];
+        t1[j] += rv[j] * (xv[j] - m[j]);
       }
       store8(gz + off, rv);
+    };
+    long long r = r0 + tr;
+    for (; r + rl < r1; r += 2 * rl) {  // two rows by themselves first: shorter chains of additions
+      float g0[8], g1[8];
+#pragma unroll
+      for (int j = 0; j < 8; ++j) g0[j] = g1[j] = 0.f;
+      row(r, g0, g1);
+      row(r + rl, g0, g1);
+#pragma unroll
+      for (int j = 0; j < 8; ++j) {
+        s0[j] += g0[j];
+        s1[j] += g1[j];
+      }
     }
+    if (r < r1) row(r, s0, s1);
   }
 #pragma unroll
   for (int j = 0; j < 8; ++j) {

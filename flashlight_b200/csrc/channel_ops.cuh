@@ -259,12 +259,12 @@ column_reduce_vec_kernel(const T* __restrict__ a, const T* __restrict__ b,
     long long r1 = r0 + rows_per_split;
     if (r1 > rows) r1 = rows;
     long long r = r0 + tr;
-    auto take = [&](const Vec16<T>& ra, const Vec16<T>& rb) {
+    auto take = [&](const Vec16<T>& ra, const Vec16<T>& rb, float* t0, float* t1) {
       float va[V], vb[V];
       unpack16(ra, va);
       if (NIN == 2) unpack16(rb, vb);
 #pragma unroll
-      for (int j = 0; j < V; ++j) f.accumulate(k[j], va[j], NIN == 2 ? vb[j] : 0.f, s0[j], s1[j]);
+      for (int j = 0; j < V; ++j) f.accumulate(k[j], va[j], NIN == 2 ? vb[j] : 0.f, t0[j], t1[j]);
     };
     // eight 16-byte loads in flight per thread: 8 rows of one tensor or 4 rows of two
     constexpr int U = NIN == 2 ? 4 : 8;
@@ -276,15 +276,25 @@ column_reduce_vec_kernel(const T* __restrict__ a, const T* __restrict__ b,
         va[u] = load16(a + off);
         if (NIN == 2) vb[u] = load16(b + off);
       }
+      // the rows in flight are summed by themselves first: a long chain of positive fp32 terms is
+      // biased (variance of 104000 bf16 rows, 117 to a thread: 1.4e-6 off, in groups of 8 4e-8)
+      float g0[V], g1[V];
 #pragma unroll
-      for (int u = 0; u < U; ++u) take(va[u], vb[u]);
+      for (int j = 0; j < V; ++j) g0[j] = g1[j] = 0.f;
+#pragma unroll
+      for (int u = 0; u < U; ++u) take(va[u], vb[u], g0, g1);
+#pragma unroll
+      for (int j = 0; j < V; ++j) {
+        s0[j] += g0[j];
+        s1[j] += g1[j];
+      }
     }
     for (; r < r1; r += rl) {
       const long long off = r * channels + c;
       const Vec16<T> va = load16(a + off);
       Vec16<T> vb;
       if (NIN == 2) vb = load16(b + off);
-      take(va, vb);
+      take(va, vb, s0, s1);
     }
   }
   // sh[tr][tq * V + j]: 256 threads x V values
