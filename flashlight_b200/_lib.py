@@ -112,6 +112,7 @@ SIGNATURES = {
                                                  vp, vp, sz, vp]),
     "flb200_matmul_workspace_bytes": (sz, [P(MatmulDesc)]),
     "flb200_matmul": (C.c_int, [P(MatmulDesc), vp, vp, vp, vp, sz, vp]),
+    "flb200_matmul_wide": (C.c_int, [P(MatmulDesc), vp, vp, vp, vp, sz, vp]),
     "flb200_linear_workspace_bytes": (sz, [i64, i64, i64, C.c_int]),
     "flb200_linear_forward": (C.c_int, [i64, i64, i64, vp, vp, vp, vp, C.c_int, vp, sz, vp]),
     "flb200_linear_bias_act_forward": (C.c_int, [i64, i64, i64, vp, vp, vp, vp, vp, C.c_int, C.c_int,

@@ -46,21 +46,34 @@ def set_math_mode(mode: int) -> None:
     extension().math_mode = mode
 
 
+def _as(t: torch.Tensor, shape) -> torch.Tensor:
+    return t if t.shape == shape else t.reshape(shape)
+
+
 class Variable:
+    # what most Variables never set lives on the class: an operator makes one on every call
+    _grad: Optional[torch.Tensor] = None
+    _grad_owned = False
+    # A second gradient contribution is kept apart until somebody reads `grad`: a
+    # grad_func that can take two addends (grad_func2) then sums them inside its own
+    # kernel instead of paying a whole-tensor addition first.
+    _grad_second: Optional[torch.Tensor] = None
+    grad_func2: Optional[Callable] = None
+    grad_hook: Optional[Callable[["Variable"], None]] = None
+    # the type its gradient is wanted in, where that is not the tensor's (cast)
+    grad_dtype = None
+
     def __init__(self, tensor: torch.Tensor, calc_grad: bool = False,
                  inputs: Sequence["Variable"] = (), grad_func: Optional[Callable] = None):
         self.tensor = tensor
         self.inputs: List[Variable] = list(inputs)
         self.grad_func = grad_func
-        self.calc_grad = calc_grad or any(i.calc_grad for i in self.inputs)
-        self._grad: Optional[torch.Tensor] = None
-        self._grad_owned = False
-        # A second gradient contribution is kept apart until somebody reads `grad`: a
-        # grad_func that can take two addends (grad_func2) then sums them inside its own
-        # kernel instead of paying a whole-tensor addition first.
-        self._grad_second: Optional[torch.Tensor] = None
-        self.grad_func2: Optional[Callable] = None
-        self.grad_hook: Optional[Callable[["Variable"], None]] = None
+        self.calc_grad = calc_grad
+        if not calc_grad:
+            for i in self.inputs:
+                if i.calc_grad:
+                    self.calc_grad = True
+                    break
 
     @property
     def grad(self) -> Optional[torch.Tensor]:
@@ -88,6 +101,10 @@ class Variable:
                              f"dimensions: {tuple(g.shape)} vs {tuple(self.tensor.shape)}")
         if self._grad is None:
             self._grad, self._grad_owned = g, False
+            return
+        if g.dtype != self._grad.dtype:  # a wide contribution (grad_dtype) and a plain one
+            total = self.grad.to(torch.float32)
+            self._grad, self._grad_owned = F.add(total, g.to(torch.float32)), True
         elif self._grad_second is None and self.grad_func2 is not None:
             self._grad_second = g
         else:
@@ -124,19 +141,22 @@ class Variable:
                 if id(inp) not in seen:
                     stack.append((inp, False))
         for node in reversed(order):
-            if node.grad_func2 is not None and node._grad_second is not None:
+            func = node.grad_func
+            if node._grad_second is not None and node.grad_func2 is not None:
                 first, second = node._grad, node._grad_second
                 node._grad_second = None
                 node.grad_func2(node.inputs, first, second)
-            elif node.grad_func is not None and node.grad is not None:
-                node.grad_func(node.inputs, node.grad)
+            elif func is not None:
+                g = node.grad
+                if g is not None:
+                    func(node.inputs, g)
             if node.grad_hook is not None and node.grad is not None:
                 node.grad_hook(node)
-            if not retain_graph and node.grad_func is not None:
+            if not retain_graph and func is not None:
                 node.grad_func = None
                 node.grad_func2 = None
                 node.inputs = []
-                node.grad = None
+                node._grad, node._grad_second, node._grad_owned = None, None, False
 
 
 # ------------------------------------------------------------------ functions
@@ -321,7 +341,12 @@ def cast(x: Variable, dtype) -> Variable:
         out = F.astype(t, d) if t.is_cuda else None
         return out if out is not None else t.to(d)
 
-    return glue(x, lambda t: to(t, dtype), lambda g: to(g, src))
+    def grad_func(inputs, gy):
+        inputs[0].addGrad(gy if gy.dtype == src else to(gy, src))
+
+    y = Variable(to(x.tensor, dtype), False, [x], grad_func)
+    y.grad_dtype = src
+    return y
 
 
 def _linear_bf16(x: Variable, w: Variable, b: Optional[Variable], gelu: bool = False) -> Variable:
@@ -339,7 +364,7 @@ def _linear_bf16(x: Variable, w: Variable, b: Optional[Variable], gelu: bool = F
         y, pre = fused
     else:
         y = F.matmul(xt, wt, m=rows, n=O, k=I, a_strides=(I, 1), b_strides=(O, 1), math_mode=mode)
-        y = y.reshape(tuple(xt.shape[:-1]) + (O,))
+        y = _as(y, xt.shape[:-1] + (O,))
         if b is not None:
             F.channel_bias_add(y, b.tensor, rows, O, 1, out=y)
         pre = y
@@ -353,12 +378,14 @@ def _linear_bf16(x: Variable, w: Variable, b: Optional[Variable], gelu: bool = F
         if inputs[0].isCalcGrad():   # dX (rows, I) = dY (rows, O) @ W^T (O, I)
             gx = F.matmul(gy, wt, m=rows, n=I, k=O, a_strides=(O, 1), b_strides=(1, O),
                           math_mode=mode)
-            inputs[0].addGrad(gx.reshape(xt.shape))
+            inputs[0].addGrad(_as(gx, xt.shape))
         if inputs[1].isCalcGrad():   # dW (I, O) = X^T (I, rows) @ dY (rows, O)
+            # (straight into fp32 where that is what the master weights take)
             inputs[1].addGrad(F.matmul(xt, gy, m=I, n=O, k=rows, a_strides=(1, I),
-                                       b_strides=(O, 1), math_mode=mode))
+                                       b_strides=(O, 1), math_mode=mode,
+                                       wide=w.grad_dtype == torch.float32))
         if b is not None and inputs[2].isCalcGrad():
-            inputs[2].addGrad(F.channel_sum(gy, rows, O, 1).reshape(b.tensor.shape))
+            inputs[2].addGrad(_as(F.channel_sum(gy, rows, O, 1), b.tensor.shape))
 
     return Variable(y, False, [x, w] + ([b] if b is not None else []), grad_func)
 
@@ -545,22 +572,31 @@ def unbind(x: Variable, fwd, bwd, n: int) -> List[Variable]:
     hands each part out as a Variable of its own — the q, k, v of a packed projection.  The
     reference indexes the packed tensor three times, and each index gradient is a zero tensor
     of the full size with one slice filled, summed by addGrad
-    (flashlight/fl/autograd/Functions.cpp:1233-1263 `index`); here the parts' gradients are
-    written into one buffer and `bwd` maps it back once, when the last of them has arrived.
-    Every part must take part in the loss (a part without a gradient would leave the buffer
-    waiting).  Data movement only: torch glue."""
+    (flashlight/fl/autograd/Functions.cpp:1233-1263 `index`); here the parts' gradients go into
+    one buffer (unless they arrive in one) and `bwd` maps it back once, when the last of them is
+    there.  Every part must take part in the loss (a part without a gradient would leave the
+    others waiting).  Data movement only: torch glue."""
     stacked = fwd(x.tensor)
-    state = {"buf": None, "seen": 0}
+    parts: List[Optional[torch.Tensor]] = [None] * n
 
     def part_grad(i):
         def grad_func(inputs, gy):
-            if state["buf"] is None:
-                state["buf"] = torch.empty_like(stacked)
-            state["buf"][i].copy_(gy)
-            state["seen"] += 1
-            if state["seen"] == n:
-                full, state["buf"], state["seen"] = state["buf"], None, 0
-                inputs[0].addGrad(bwd(full))
+            parts[i] = gy
+            if any(p is None for p in parts):
+                return
+            first, step = parts[0], stacked[0].numel()
+            if all(p.is_contiguous() and p.dtype == stacked.dtype and
+                   p.data_ptr() == first.data_ptr() + k * step * p.element_size() and
+                   p.untyped_storage().data_ptr() == first.untyped_storage().data_ptr()
+                   for k, p in enumerate(parts)):
+                # already one after another in one buffer (functions.attention_backward)
+                full = first.as_strided(stacked.shape, stacked.stride(), first.storage_offset())
+            else:
+                full = torch.empty_like(stacked)
+                for k, p in enumerate(parts):
+                    full[k].copy_(p)
+            parts[:] = [None] * n
+            inputs[0].addGrad(bwd(full))
         return grad_func
 
     return [Variable(stacked[i], False, [x], part_grad(i)) for i in range(n)]
@@ -678,13 +714,13 @@ def layernorm(x: Variable, w: Variable, b: Variable, eps: float = 1e-5) -> Varia
         need_p = inputs[1].isCalcGrad() or inputs[2].isCalcGrad()
         gx, gw, gb = F.layernorm_backward(gy, xhat, wt, invstd, inputs[0].isCalcGrad(), need_p)
         if inputs[0].isCalcGrad():
-            inputs[0].addGrad(gx.reshape(xt.shape))
+            inputs[0].addGrad(_as(gx, xt.shape))
         if inputs[1].isCalcGrad():
-            inputs[1].addGrad(gw.reshape(wt.shape))
+            inputs[1].addGrad(_as(gw, wt.shape))
         if inputs[2].isCalcGrad():
-            inputs[2].addGrad(gb.reshape(bt.shape))
+            inputs[2].addGrad(_as(gb, bt.shape))
 
-    return Variable(y.reshape(xt.shape), False, [x, w, b], grad_func)
+    return Variable(_as(y, xt.shape), False, [x, w, b], grad_func)
 
 
 def embedding(table: Variable, ids: torch.Tensor) -> Variable:

@@ -104,6 +104,17 @@ int flb200_matmul(const flb200_matmul_desc* d, const void* a, const void* b, voi
   return run_matmul(d, a, b, c, workspace, workspace_bytes, stream);
 }
 
+int flb200_matmul_wide(const flb200_matmul_desc* d, const void* a, const void* b, float* c,
+                       void* workspace, size_t workspace_bytes, void* stream) {
+  if (int st = check_desc(d, a, b, c)) return st;
+  if (d->dtype == FLB200_F32) return run_matmul(d, a, b, c, workspace, workspace_bytes, stream);
+  if (d->m == 0 || d->n == 0) return FLB200_OK;
+  if (!tc_gemm_supported(d, a, b, c))
+    return fail(FLB200_UNSUPPORTED, "matmul_wide: bf16 needs the tensor-core path");
+  return tc_gemm_run(d, a, b, c, workspace, workspace_bytes, as_stream(stream), nullptr, 0, nullptr,
+                     true);
+}
+
 // which: 0 forward, 1 backward-input, 2 backward-weight.  A NULL / short
 // workspace is accepted by the three calls: the contraction then runs unsplit.
 size_t flb200_linear_workspace_bytes(int64_t O, int64_t I, int64_t cols, int which) {

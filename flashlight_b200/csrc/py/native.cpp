@@ -425,6 +425,8 @@ NATIVE(linear_backward) {  // (x, weight, grad_y, has_bias, need_x, need_w, mode
 NATIVE(matmul) {
   const Tensor &a = x.tensor(0), &b = x.tensor(1);
   const Tensor* given = x.t(2);
+  const bool wide = x.b(19);  // an f32 result of 16-bit operands
+  if (wide && given && given->scalar_type() != ScalarType::Float) value_error("matmul: a wide result is float32");
   flb200_matmul_desc d = {};
   d.m = x.i(3); d.n = x.i(4); d.k = x.i(5);
   d.a_row = x.i(6); d.a_col = x.i(7); d.b_row = x.i(8); d.b_col = x.i(9);
@@ -435,14 +437,16 @@ NATIVE(matmul) {
     c = *given;
     d.c_row = x.i(10); d.c_col = x.i(11); d.c_batch = x.i(15);
   } else {
-    if (d.batch > 1) c = empty({d.batch, d.m, d.n}, a.scalar_type(), a);
-    else c = empty({d.m, d.n}, a.scalar_type(), a);
+    const ScalarType type = wide ? ScalarType::Float : a.scalar_type();
+    if (d.batch > 1) c = empty({d.batch, d.m, d.n}, type, a);
+    else c = empty({d.m, d.n}, type, a);
     d.c_row = d.n; d.c_col = 1; d.c_batch = d.m * d.n;
   }
   d.alpha = (float)x.d(16); d.beta = (float)x.d(17);
   d.dtype = code_of(a); d.math_mode = x.n32(18);
   Workspace ws(flb200_matmul_workspace_bytes(&d), a);
-  check(flb200_matmul(&d, P(a), P(b), P(c), ws.p(), ws.bytes, stream()));
+  check(wide ? flb200_matmul_wide(&d, P(a), P(b), Pf(&c), ws.p(), ws.bytes, stream())
+             : flb200_matmul(&d, P(a), P(b), P(c), ws.p(), ws.bytes, stream()));
   return wrap(c);
 }
 
@@ -530,7 +534,8 @@ NATIVE(attention_backward) {  // (q, k, v, o, grad_o, lse, scale, causal) -> (dq
       value_error("attention_backward: q, k, v, o and grad_o must be dense and alike");
   }
   const int64_t Z = q.size(0), T = q.size(1), hd = q.size(2);
-  Tensor dq = empty_like(q), dk = empty_like(q), dv = empty_like(q);
+  const Tensor all = empty({3, Z, T, hd}, q.scalar_type(), q);  // one after another (autograd.unbind)
+  const Tensor dq = all.select(0, 0), dk = all.select(0, 1), dv = all.select(0, 2);
   Workspace ws(flb200_attention_backward_workspace_bytes(Z, T, hd), q);
   check(flb200_attention_backward(P(q), P(x.t(1)), P(x.t(2)), P(x.t(3)), P(x.t(4)), Pf(x.t(5)), P(dq), P(dk), P(dv),
                                   Z, T, hd, (float)x.d(6), x.b(7) ? 1 : 0, code_of(q), ws.p(), ws.bytes, stream()));

@@ -7,6 +7,7 @@
 #include "tc_gemm.cuh"
 
 #include <cstdlib>
+#include <cstring>
 #include <mutex>
 
 #include "tc_pair.cuh"
@@ -52,6 +53,31 @@ int make_tensor_map(CUtensorMap* map, const void* base, int rank, const uint64_t
     es[i] = elem_strides ? elem_strides[i] : 1;
     if (i > 0) gs[i - 1] = strides_bytes[i - 1];
   }
+  // Encoding a map is work of the host alone and depends on these values only: each thread keeps the
+  // last ones that it made.
+  struct Key {
+    const void* base;
+    cuuint64_t gd[5], gs[4];
+    cuuint32_t bx[5], es[5];
+    int rank, mode, operand, used;
+  };
+  struct Entry { Key key; CUtensorMap map; };
+  static thread_local Entry known[128] = {};
+  Key key;
+  memset(&key, 0, sizeof(key));
+  key.base = base;
+  key.rank = rank; key.mode = mode; key.operand = operand; key.used = 1;
+  unsigned long long h = reinterpret_cast<uintptr_t>(base) >> 4;
+  for (int i = 0; i < rank; ++i) {
+    key.gd[i] = gd[i]; key.bx[i] = bx[i]; key.es[i] = es[i];
+    if (i > 0) key.gs[i - 1] = gs[i - 1];
+    h = h * 31 + gd[i] + 17 * bx[i];
+  }
+  Entry& e = known[(h * 0x9e3779b97f4a7c15ull) >> 57];
+  if (memcmp(&e.key, &key, sizeof(key)) == 0) {
+    *map = e.map;
+    return FLB200_OK;
+  }
   CUresult r = fn(map,
                   operand == kOperandBf16   ? CU_TENSOR_MAP_DATA_TYPE_BFLOAT16
                   : operand == kOperandF16 ? CU_TENSOR_MAP_DATA_TYPE_FLOAT16
@@ -65,6 +91,8 @@ int make_tensor_map(CUtensorMap* map, const void* base, int rank, const uint64_t
   if (r != CUDA_SUCCESS)
     return fail(FLB200_INVALID_ARG, "cuTensorMapEncodeTiled failed with code %d (rank %d)", (int)r,
                 rank);
+  e.key = key;
+  e.map = *map;
   return FLB200_OK;
 }
 
@@ -259,11 +287,8 @@ void plan_splits(long long tiles, long long k_iters, long long min_ips, int* spl
 // pipe's own 512.  A small product wants narrow tiles and a split of K for the sake of the
 // idle SMs: a 128-row bf16 product of 2304 columns ran on 9 CTAs of 148 with 256-column tiles,
 // 17 us; on 72 with 32-column ones, 7 us.
-Launch plan_launch(long long M, long long N, long long k_iters, long long Z, bool a_mn_major,
-                   bool b_mn_major, int operand, bool split_k) {
-  const long long sm = device_info().sm_count > 0 ? device_info().sm_count : 148;
-  const bool x3 = x3_enabled();
-  if (k_iters < 1) k_iters = 1;
+static Launch compute_launch(long long M, long long N, long long k_iters, long long Z, bool a_mn_major,
+                             bool b_mn_major, int operand, bool split_k, long long sm, bool x3) {
   const int box = operand == kOperandTf32 ? 32 : 64;
   const long long tiles_m = (M + kBM - 1) / kBM;
   Launch best{};
@@ -315,6 +340,25 @@ Launch plan_launch(long long M, long long N, long long k_iters, long long Z, boo
   }
   best.workspace_bytes = best.splits > 1 ? (size_t)(Z * best.splits * M * N) * sizeof(float) : 0;
   return best;
+}
+
+// Weighing a plan takes 0.3 us and an operator asks for several (its workspace, its launch): each
+// thread remembers the plans of the last sizes it saw.
+Launch plan_launch(long long M, long long N, long long k_iters, long long Z, bool a_mn_major,
+                   bool b_mn_major, int operand, bool split_k) {
+  struct Entry { long long m, n, k, z, rest; Launch plan; };
+  static thread_local Entry known[64] = {};
+  const long long sm = device_info().sm_count > 0 ? device_info().sm_count : 148;
+  const bool x3 = x3_enabled();
+  if (k_iters < 1) k_iters = 1;
+  const long long rest = 1 + (a_mn_major ? 2 : 0) + (b_mn_major ? 4 : 0) + (split_k ? 8 : 0) +
+                         (x3 ? 16 : 0) + operand * 32LL + sm * 256;
+  const unsigned long long h = ((unsigned long long)(M * 31 + N) * 31 + k_iters * 7 + Z) * 31 + rest;
+  Entry& e = known[(h * 0x9e3779b97f4a7c15ull) >> 58];
+  if (e.m != M || e.n != N || e.k != k_iters || e.z != Z || e.rest != rest)
+    e = Entry{M, N, k_iters, Z, rest,
+              compute_launch(M, N, k_iters, Z, a_mn_major, b_mn_major, operand, split_k, sm, x3)};
+  return e.plan;
 }
 
 int run(const CUtensorMap& ma, const CUtensorMap& mb, const OperandPlan& pa, const OperandPlan& pb,
@@ -477,7 +521,8 @@ size_t tc_gemm_workspace_bytes(const flb200_matmul_desc* d) {
 }
 
 int tc_gemm_run(const flb200_matmul_desc* d, const void* a, const void* b, void* c, void* ws,
-                size_t ws_bytes, cudaStream_t st, const float* bias_n, int act, void* pre) {
+                size_t ws_bytes, cudaStream_t st, const float* bias_n, int act, void* pre,
+                bool wide) {
   const Prepared p = prepare(d, a, b, c);
   if (!p.ok) return fail(FLB200_UNSUPPORTED, "tc_gemm: layout not covered");
   const bool fused = bias_n != nullptr || act != 0 || pre != nullptr;
@@ -493,7 +538,7 @@ int tc_gemm_run(const flb200_matmul_desc* d, const void* a, const void* b, void*
   tc::OperandPlan pa, pb;
   tc::EpiloguePlan ep{};
   ep.out = static_cast<float*>(c);
-  ep.out16 = operand;
+  ep.out16 = wide ? 0 : operand;
   ep.alpha = d->alpha;
   ep.beta = d->beta;
   ep.z_stride = d->c_batch;

@@ -17,7 +17,7 @@ size_t tc_gemm_workspace_bytes(const flb200_matmul_desc* d);
 // (FLB200_UNSUPPORTED otherwise, so that the caller can run the operators one by one).
 int tc_gemm_run(const flb200_matmul_desc* d, const void* a, const void* b, void* c, void* ws,
                 size_t ws_bytes, cudaStream_t st, const float* bias_n = nullptr, int act = 0,
-                void* pre = nullptr);
+                void* pre = nullptr, bool wide = false);  // wide: fp32 result of 16-bit operands
 
 namespace tc {
 

@@ -172,12 +172,14 @@ def linear_backward(x, weight, grad_y, has_bias: bool, need_input_grad=True, nee
 
 
 def matmul(a, b, c=None, *, m, n, k, a_strides, b_strides, c_strides=None, batch=1,
-           batch_strides=(0, 0, 0), alpha=1.0, beta=0.0, math_mode: Optional[int] = None):
-    """C[m,n] = alpha * A(m,k) B(k,n) + beta * C on strided row-major views (flb200_matmul)."""
+           batch_strides=(0, 0, 0), alpha=1.0, beta=0.0, math_mode: Optional[int] = None,
+           wide: bool = False):
+    """C[m,n] = alpha * A(m,k) B(k,n) + beta * C on strided row-major views (flb200_matmul); wide: an
+    f32 result whatever the operands' type."""
     c_row, c_col = c_strides if c is not None else (0, 0)
     return N.matmul(a, b, c, m, n, k, a_strides[0], a_strides[1], b_strides[0], b_strides[1], c_row,
                     c_col, batch, batch_strides[0], batch_strides[1], batch_strides[2], alpha, beta,
-                    default_math_mode() if math_mode is None else math_mode)
+                    default_math_mode() if math_mode is None else math_mode, wide)
 
 
 # --------------------------------------------------- logSoftmax and CE loss

@@ -324,6 +324,10 @@ typedef struct flb200_matmul_desc {
 size_t flb200_matmul_workspace_bytes(const flb200_matmul_desc* d);
 int flb200_matmul(const flb200_matmul_desc* d, const void* a, const void* b, void* c,
                   void* workspace, size_t workspace_bytes, void* stream);
+/* The same with an f32 C whatever the operands' type: the gradient of fp32 master weights from bf16
+ * activations, without a bf16 copy in between. */
+int flb200_matmul_wide(const flb200_matmul_desc* d, const void* a, const void* b, float* c,
+                       void* workspace, size_t workspace_bytes, void* stream);
 
 /* fl::linear gradFunc pieces (Functions.cpp:1255-1309) on fl-layout buffers:
  * weight [O,I], x [I,cols], y / grad_y [O,cols] (all column-major).  which:
