@@ -129,6 +129,10 @@ SIGNATURES = {
     "flb200_softmax_backward": (C.c_int, [vp, vp, vp, i64, i64, f32, C.c_int, vp]),
     "flb200_softmax_forward_lse": (C.c_int, [vp, vp, vp, i64, i64, f32, i64, C.c_int, vp]),
     "flb200_attention_backward_supported": (C.c_int, [i64, i64, C.c_int]),
+    "flb200_attention_packed_supported": (C.c_int, [i64, i64, C.c_int]),
+    "flb200_attention_packed_forward": (C.c_int, [vp, vp, vp, i64, i64, i64, i64, f32, C.c_int, C.c_int, vp]),
+    "flb200_attention_packed_backward": (C.c_int, [vp, vp, vp, vp, vp, i64, i64, i64, i64, f32, C.c_int,
+                                                   C.c_int, vp, sz, vp]),
     "flb200_attention_backward_workspace_bytes": (sz, [i64, i64, i64]),
     "flb200_attention_backward": (C.c_int, [vp, vp, vp, vp, vp, vp, vp, vp, vp, i64, i64, i64, f32,
                                             C.c_int, C.c_int, vp, sz, vp]),

@@ -666,6 +666,25 @@ def attention(q: Variable, k: Variable, v: Variable, scale: float, causal: bool)
     return Variable(out, False, [q, k, v], grad_func)
 
 
+def attention_packed(qkv: Variable, B: int, T: int, heads: int, scale: float,
+                     causal: bool) -> Optional[Variable]:
+    """attention() on the packed projection (B * T, 3 * heads * head dim), result (B * T, heads * head
+    dim): one kernel forward, which reads q, k and v where the projection left them, and the fused
+    gradient, which writes theirs there.  None where the kernels are not built for the tensor."""
+    if FUSED_ATTENTION_OFF or qkv.tensor.dtype != torch.bfloat16:
+        return None
+    qt = qkv.tensor.contiguous()
+    fused = F.attention_packed(qt, B, T, heads, scale, causal)
+    if fused is None:
+        return None
+    out, lse = fused
+
+    def grad_func(inputs, gy):
+        inputs[0].addGrad(F.attention_packed_backward(qt, out, gy.contiguous(), lse, B, T, heads, scale, causal))
+
+    return Variable(out, False, [qkv], grad_func)
+
+
 def softmax_rows(x: Variable, scale: float = 1.0, causal_period: int = 0) -> Variable:
     """softmax over the last dimension (Functions.cpp:1021-1042) of scale * x, with the causal
     mask of attention scores folded in when causal_period = T (x is a stack of T-row score

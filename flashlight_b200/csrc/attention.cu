@@ -1,12 +1,15 @@
-// Fused attention backward (flash style): dq, dk, dv of  o = softmax(scale * q k^T [+ causal
-// mask]) v  without materialising the T x T score tensors in device memory.  The reference
+// Fused attention, forward and backward (flash style):  o = softmax(scale * q k^T [+ causal mask]) v
+// and dq, dk, dv, without materialising the T x T score tensors in device memory.  The reference
 // builds the chain out of whole-tensor operators and keeps the probabilities for the gradient
 // (flashlight/fl/autograd/Functions.cpp:1828-1891, 1021-1042); here the forward pass keeps only
-// the row-wise log-sum-exp of the scaled scores, and this kernel recomputes the probabilities of
-// one 128 x 128 block at a time in tensor memory.
+// the row-wise log-sum-exp of the scaled scores, and the backward kernel recomputes the
+// probabilities of // one 128 x 128 block at a time in tensor memory.
 //
-// bf16 tensors [batch * heads][T][64], T a multiple of 128.  One CTA per (batch-head, block of
-// 128 keys): K_j and V_j stay in shared memory, the CTA walks the query blocks i (i >= j with
+// bf16 tensors of head dimension 64 and any length T, read and written in place through strides:
+// [batch * heads][T][64], or the packed projection [batch][T][3][heads][64] as its contraction left
+// it, which saves a reordering copy on each side.  Rows past T arrive as zeros from TMA, are masked
+// and never stored.
+// Backward: one CTA per (batch-head, block of 128 keys): K_j and V_j stay in shared memory, the CTA walks the query blocks i (i >= j with
 // the causal mask) and per block issues five tcgen05 contractions with fp32 accumulators in
 // tensor memory:
 //     S  = Q_i K_j^T                    (128 x 128, K = 64)   columns   0..127
@@ -28,6 +31,11 @@
 #include <cuda_bf16.h>
 #include <cuda_runtime.h>
 
+#include <algorithm>
+#include <mutex>
+#include <set>
+#include <utility>
+
 #include "common.cuh"
 #include "flb200.h"
 #include "tc_core.cuh"
@@ -43,8 +51,13 @@ constexpr int kAttnThreads = 288;      // warps 0..7: two threads per query row 
 constexpr int kTile = 128 * 128;       // bytes of a [128 rows][64 bf16] tile
 constexpr int kAttnSmem = 4 * kTile + 2 * 2 * kTile + 1024 + 256;  // K V Q dO, P dS, align, bars
 
+// element (batch b, head h, position t, d) of a tensor is at b * batch + h * head + t * row + d
+struct HeadStrides { long long batch, head, row; };
+
 struct AttnArgs {
-  const float* dsum;  // rowsum(dO * O), from attention_dsum_kernel
+  HeadStrides gs;     // of dq, dk and dv
+  int heads;
+  const float* dsum;  // rowsum(dO * O), from attention_dsum_kernel, [batch * heads][T]
   const float* lse;
   float* dq_acc;
   __nv_bfloat16* dk;
@@ -121,10 +134,11 @@ attention_backward_kernel(const __grid_constant__ CUtensorMap map_q,
   int* failed = reinterpret_cast<int*>(bars + 5);
 
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  const int nblk = a.T / 128;
+  const int nblk = (a.T + 127) / 128;
   const int j = blockIdx.x % nblk;        // key block
   const int bh = blockIdx.x / nblk;       // batch * heads index
-  const long long row0 = (long long)bh * a.T;  // first row of this head in the [BH * T][64] views
+  const int batch = bh / a.heads, head = bh - batch * a.heads;
+  const long long row0 = (long long)bh * a.T;  // first row of this head in lse, dsum and dq_acc
 
   if (threadIdx.x == 0) {
     mbar_init(bar_kv, 1);
@@ -162,9 +176,9 @@ attention_backward_kernel(const __grid_constant__ CUtensorMap map_q,
 
   if (issuer) {
     mbar_expect_tx(bar_kv, 2 * kTile);
-    int c[2] = {0, (int)(row0 + (long long)j * 128)};
-    tma_load(&map_k, bar_kv, sK, 2, c);
-    tma_load(&map_v, bar_kv, sV, 2, c);
+    int c[4] = {0, j * 128, head, batch};
+    tma_load(&map_k, bar_kv, sK, 4, c);
+    tma_load(&map_v, bar_kv, sV, 4, c);
   }
 
 #ifdef FLB200_ATTN_PROFILE
@@ -181,9 +195,9 @@ attention_backward_kernel(const __grid_constant__ CUtensorMap map_q,
     const long long qrow = row0 + (long long)i * 128;
     if (issuer) {
       mbar_expect_tx(bar_q, 2 * kTile);
-      int c[2] = {0, (int)qrow};
-      tma_load(&map_q, bar_q, sQ, 2, c);
-      tma_load(&map_do, bar_q, sDO, 2, c);
+      int c[4] = {0, i * 128, head, batch};
+      tma_load(&map_q, bar_q, sQ, 4, c);
+      tma_load(&map_do, bar_q, sDO, 4, c);
       if (it == 0 && *failed == 0 && !mbar_wait(bar_kv, 0)) *failed = 1;
       if (*failed == 0 && !mbar_wait(bar_q, ph)) *failed = 2;
       tc_fence_after();
@@ -199,8 +213,10 @@ attention_backward_kernel(const __grid_constant__ CUtensorMap map_q,
     }
     float lse = 0.f, dsum = 0.f;
     if (row_thread) {
-      dsum = a.dsum[qrow + r];
-      lse = a.lse[qrow + r];
+      if (i * 128 + r < a.T) {
+        dsum = a.dsum[qrow + r];
+        lse = a.lse[qrow + r];
+      }
       ATTN_MARK(0, tp);
       if (*failed == 0 && !mbar_wait(bar_s, ph)) *failed = 3;
       tc_fence_after();
@@ -213,7 +229,8 @@ attention_backward_kernel(const __grid_constant__ CUtensorMap map_q,
         tmem_ld32_pair(lane_addr + (uint32_t)c0, s, lane_addr + 128u + (uint32_t)c0, dp);
 #pragma unroll
         for (int e = 0; e < 32; ++e) {
-          const bool masked = a.causal && (j * 128 + c0 + e > q_pos);
+          const int key = j * 128 + c0 + e;
+          const bool masked = (a.causal && key > q_pos) || key >= a.T || q_pos >= a.T;
           const float p = masked ? 0.f : __expf(a.scale * s[e] - lse);
           s[e] = p;
           dp[e] = a.scale * p * (dp[e] - dsum);
@@ -257,7 +274,8 @@ attention_backward_kernel(const __grid_constant__ CUtensorMap map_q,
       float v[32];
       tmem_ld32(tmem + ((uint32_t)((warp & 3) * 32) << 16) + 384u + 32u * half, v);
 #pragma unroll
-      for (int e = 0; e < 32; e += 4) red_add_v4(dst + e, v[e], v[e + 1], v[e + 2], v[e + 3]);
+      for (int e = 0; e < 32; e += 4)
+        if (i * 128 + r < a.T) red_add_v4(dst + e, v[e], v[e + 1], v[e + 2], v[e + 3]);
       ATTN_MARK(4, tp);
     }
     // the next block's loads and contractions overwrite Q_i, dO_i, S, dP, P, dS and dQ
@@ -276,13 +294,15 @@ attention_backward_kernel(const __grid_constant__ CUtensorMap map_q,
 
   if (row_thread) {
     // the first half of the row threads stores dV_j, the second dK_j
-    const long long krow = row0 + (long long)j * 128 + r;
+    const int key = j * 128 + r;
     const uint32_t lane_addr = tmem + ((uint32_t)((warp & 3) * 32) << 16) + 256u + 64u * half;
-    __nv_bfloat16* out = (half == 0 ? a.dv : a.dk) + krow * 64;
+    __nv_bfloat16* out = (half == 0 ? a.dv : a.dk) + batch * a.gs.batch + head * a.gs.head +
+                         (long long)key * a.gs.row;
 #pragma unroll 1
     for (int c0 = 0; c0 < 64; c0 += 32) {
       float v[32];
       tmem_ld32(lane_addr + (uint32_t)c0, v);
+      if (key >= a.T) continue;
 #pragma unroll
       for (int u = 0; u < 4; ++u)
         *reinterpret_cast<uint4*>(out + c0 + 8 * u) =
@@ -299,10 +319,12 @@ attention_backward_kernel(const __grid_constant__ CUtensorMap map_q,
   }
 }
 
-// D[row] = sum_d dO[row][d] * O[row][d]: eight lanes per row, one 16-byte load each
+// D[row] = sum_d dO[row][d] * O[row][d]: eight lanes per row, one 16-byte load each.  Rows in the
+// order [batch][T][heads] of o, results in [batch][heads][T].
 __global__ void attention_dsum_kernel(const __nv_bfloat16* __restrict__ o,
                                       const __nv_bfloat16* __restrict__ d_o,
-                                      float* __restrict__ dsum, long long rows) {
+                                      float* __restrict__ dsum, long long rows, int T,
+                                      int heads) {
   const long long t = blockIdx.x * (long long)blockDim.x + threadIdx.x;
   const long long row = t >> 3;
   float acc = 0.f;
@@ -320,18 +342,276 @@ __global__ void attention_dsum_kernel(const __nv_bfloat16* __restrict__ o,
   acc += __shfl_xor_sync(0xffffffffu, acc, 1);
   acc += __shfl_xor_sync(0xffffffffu, acc, 2);
   acc += __shfl_xor_sync(0xffffffffu, acc, 4);
-  if (row < rows && (threadIdx.x & 7) == 0) dsum[row] = acc;
+  if (row < rows && (threadIdx.x & 7) == 0) {
+    const long long bt = row / heads, b = bt / T;
+    dsum[(b * heads + row - bt * heads) * T + bt - b * T] = acc;
+  }
 }
 
 __global__ void narrow_dq_kernel(const float* __restrict__ acc, __nv_bfloat16* __restrict__ dq,
-                                 long long n8) {
+                                 long long n8, int T, int heads, HeadStrides gs) {
   for (long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x; i < n8;
        i += (long long)gridDim.x * blockDim.x) {
     const float4 lo = reinterpret_cast<const float4*>(acc)[2 * i];
     const float4 hi = reinterpret_cast<const float4*>(acc)[2 * i + 1];
-    reinterpret_cast<uint4*>(dq)[i] = make_uint4(pack_bf16(lo.x, lo.y), pack_bf16(lo.z, lo.w),
+    const long long row = i >> 3, bh = row / T, b = bh / heads;
+    __nv_bfloat16* to = dq + b * gs.batch + (bh - b * heads) * gs.head + (row - bh * T) * gs.row + 8 * (i & 7);
+    *reinterpret_cast<uint4*>(to) = make_uint4(pack_bf16(lo.x, lo.y), pack_bf16(lo.z, lo.w),
                                                  pack_bf16(hi.x, hi.y), pack_bf16(hi.z, hi.w));
   }
+}
+
+// ---------------------------------------------------------------------------------- forward
+// One CTA per (batch-head, block of 128 queries), largest blocks of a causal head first; it walks the
+// key blocks j with two contractions each:
+//     S  = Q_i K_j^T   (128 x 128, K = 64)    columns   0..127
+//     O  = P V_j       (128 x  64, K = 128)   columns 128..191
+// Two threads per query row (half of the columns each) read S, agree on the new row maximum m through
+// shared memory, write P = exp(scale * S - m) as a bf16 operand tile, and keep the row's sum and its
+// output in fp32 registers, rescaled by exp(m_old - m) per block.  K_{j+1} is fetched while the
+// probabilities of block j are computed, S_{j+1} runs behind O_j.  What bounds it is that chain from
+// contraction to contraction, not the tensor pipe: two CTAs share an SM and fill each other's waits.
+// (scores, softmax and context as three operators, with a reordering copy before and after: five
+// launches and three T x T passes per layer.)
+constexpr int kFwdSmem = 5 * kTile + 1024 + 1024 + 256;  // Q K V P(2), row exchange, align, bars
+struct AttnFwdArgs {
+  __nv_bfloat16* out;
+  HeadStrides os;
+  float* lse;  // [batch * heads][T], or null
+  int T, heads, causal;
+  float scale;
+  int* status;
+};
+
+__global__ void __launch_bounds__(kAttnThreads, 2)
+attention_forward_kernel(const __grid_constant__ CUtensorMap map_q,
+                         const __grid_constant__ CUtensorMap map_k,
+                         const __grid_constant__ CUtensorMap map_v, const AttnFwdArgs a) {
+  extern __shared__ __align__(1024) char smem_raw[];
+  char* base = smem_raw + ((1024 - (smem_u32(smem_raw) & 1023)) & 1023);
+  char* sQ = base;
+  char* sK = base + kTile;
+  char* sV = base + 2 * kTile;
+  char* sP = base + 3 * kTile;  // two 64-key halves
+  float* row_x = reinterpret_cast<float*>(base + 5 * kTile);  // [2 halves][128 rows]
+  uint64_t* bars = reinterpret_cast<uint64_t*>(row_x + 256);
+  uint64_t* bar_q = bars;
+  uint64_t* bar_k = bars + 1;
+  uint64_t* bar_v = bars + 2;
+  uint64_t* bar_s = bars + 3;
+  uint64_t* bar_o = bars + 4;
+  uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(bars + 5);
+  volatile int* failed = reinterpret_cast<volatile int*>(bars + 6);
+
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const int nblk = (a.T + 127) / 128;
+  const int i = nblk - 1 - (int)blockIdx.x % nblk;  // query block
+  const int bh = blockIdx.x / nblk;
+  const int batch = bh / a.heads, head = bh - batch * a.heads;
+
+  if (threadIdx.x == 0) {
+    for (int k = 0; k < 5; ++k) mbar_init(bars + k, 1);
+    *failed = 0;
+    fence_barrier_init();
+  }
+  if (warp == 8) tmem_alloc(tmem_slot, 256);
+  tc_fence_before();
+  __syncthreads();
+  tc_fence_after();
+  const uint32_t tmem = *tmem_slot;
+  const bool issuer = warp == 8 && lane == 0;
+  const int r = (warp & 3) * 32 + lane, half = warp >> 2;
+  const int q_pos = i * 128 + r;
+  const int blocks = a.causal ? i + 1 : nblk;
+
+  const uint64_t dQ = umma_desc(smem_u32(sQ), 16, 1024, 2);
+  const uint64_t dK = umma_desc(smem_u32(sK), 16, 1024, 2);
+  const uint64_t dP = umma_desc(smem_u32(sP), 16, 1024, 2);
+  const uint64_t dV = umma_desc(smem_u32(sV), 8192, 1024, 2);  // one box of 64 d, rows = keys
+  const uint32_t id_s = umma_idesc_f16(kOperandBf16, 128, 0, 0);
+  const uint32_t id_o = umma_idesc_f16(kOperandBf16, 64, 0, 1);
+  auto load = [&](const CUtensorMap* m, uint64_t* bar, char* to, int block) {
+    mbar_expect_tx(bar, kTile);
+    int c[4] = {0, block * 128, head, batch};
+    tma_load(m, bar, to, 4, c);
+  };
+  auto wait = [&](uint64_t* bar, uint32_t phase, int code) {
+    if (*failed == 0 && !mbar_wait(bar, phase)) *failed = code;
+    tc_fence_after();
+  };
+  auto scores = [&](uint32_t phase) {
+    wait(bar_k, phase, 2);
+#pragma unroll
+    for (int kk = 0; kk < 4; ++kk)  // K = 64 d in steps of 16
+      umma_f16(tmem, umma_desc_advance(dQ, kk * 32), umma_desc_advance(dK, kk * 32), id_s, kk > 0);
+    umma_commit(bar_s);
+  };
+  if (issuer) {
+    load(&map_q, bar_q, sQ, i);
+    load(&map_k, bar_k, sK, 0);
+    load(&map_v, bar_v, sV, 0);
+    wait(bar_q, 0, 1);
+    scores(0);
+  }
+  float m = -INFINITY, sum = 0.f, o[32];
+#pragma unroll
+  for (int e = 0; e < 32; ++e) o[e] = 0.f;
+  const uint32_t lane_addr = tmem + ((uint32_t)((warp & 3) * 32) << 16);
+
+  for (int j = 0; j < blocks; ++j) {
+    const uint32_t ph = j & 1;
+    float alpha = 1.f;
+    if (warp < 8) {
+      wait(bar_s, ph, 3);
+      // this thread's 64 keys; those in front of `live` count
+      const int k0 = j * 128 + 64 * half;
+      const int live = min(a.T, a.causal ? q_pos + 1 : a.T) - k0;
+      float mx = -INFINITY;
+#pragma unroll 1
+      for (int c0 = 0; c0 < 64; c0 += 32) {
+        float s[32];
+        tmem_ld32(lane_addr + 64u * half + c0, s);
+#pragma unroll
+        for (int e = 0; e < 32; ++e) mx = fmaxf(mx, c0 + e < live ? a.scale * s[e] : -INFINITY);
+      }
+      row_x[half * 128 + r] = mx;
+      // the two warps that share these rows
+      asm volatile("bar.sync %0, 64;" ::"r"(1 + (warp & 3)) : "memory");
+      mx = fmaxf(mx, row_x[(half ^ 1) * 128 + r]);
+      const float m_new = fmaxf(m, mx);
+      alpha = __expf(m - m_new);
+      m = m_new;
+      sum *= alpha;
+#pragma unroll 1
+      for (int c0 = 0; c0 < 64; c0 += 32) {
+        float s[32];
+        tmem_ld32(lane_addr + 64u * half + c0, s);
+#pragma unroll
+        for (int e = 0; e < 32; ++e) {
+          s[e] = c0 + e < live ? __expf(a.scale * s[e] - m) : 0.f;
+          sum += s[e];
+        }
+#pragma unroll
+        for (int u = 0; u < 4; ++u)
+          *reinterpret_cast<uint4*>(sP + score_chunk(r, 64 * half + c0 + 8 * u)) =
+              make_uint4(pack_bf16(s[8 * u], s[8 * u + 1]), pack_bf16(s[8 * u + 2], s[8 * u + 3]),
+                         pack_bf16(s[8 * u + 4], s[8 * u + 5]), pack_bf16(s[8 * u + 6], s[8 * u + 7]));
+      }
+      fence_proxy_async();
+    } else if (issuer) {
+      wait(bar_s, ph, 3);
+      if (j + 1 < blocks) load(&map_k, bar_k, sK, j + 1);
+    }
+    tc_fence_before();
+    __syncthreads();  // P is complete, S and the last block's O have been read
+    if (issuer) {
+      wait(bar_v, ph, 4);
+#pragma unroll
+      for (int kk = 0; kk < 8; ++kk)  // K = 128 keys: two 64-key halves of P, 16 key rows of V_j
+        umma_f16(tmem + 128, umma_desc_advance(dP, (kk >> 2) * kTile + (kk & 3) * 32),
+                 umma_desc_advance(dV, kk * 2048), id_o, kk > 0);
+      umma_commit(bar_o);
+      if (j + 1 < blocks) scores(ph ^ 1);
+      wait(bar_o, ph, 5);
+      if (j + 1 < blocks) load(&map_v, bar_v, sV, j + 1);
+    } else if (warp < 8) {
+      wait(bar_o, ph, 5);
+      float v[32];
+      tmem_ld32(lane_addr + 128u + 32u * half, v);
+#pragma unroll
+      for (int e = 0; e < 32; ++e) o[e] = o[e] * alpha + v[e];
+    }
+    __syncwarp();
+  }
+  if (warp < 8) {
+    asm volatile("bar.sync %0, 64;" ::"r"(1 + (warp & 3)) : "memory");  // row_x has been read
+    row_x[half * 128 + r] = sum;
+    asm volatile("bar.sync %0, 64;" ::"r"(1 + (warp & 3)) : "memory");
+    sum = half == 0 ? sum + row_x[128 + r] : row_x[r] + sum;
+    if (q_pos < a.T) {
+      const float inv = 1.f / sum;
+      __nv_bfloat16* to = a.out + batch * a.os.batch + head * a.os.head + (long long)q_pos * a.os.row + 32 * half;
+#pragma unroll
+      for (int u = 0; u < 4; ++u)
+        *reinterpret_cast<uint4*>(to + 8 * u) = make_uint4(
+            pack_bf16(o[8 * u] * inv, o[8 * u + 1] * inv), pack_bf16(o[8 * u + 2] * inv, o[8 * u + 3] * inv),
+            pack_bf16(o[8 * u + 4] * inv, o[8 * u + 5] * inv), pack_bf16(o[8 * u + 6] * inv, o[8 * u + 7] * inv));
+      if (half == 0 && a.lse) a.lse[(long long)bh * a.T + q_pos] = m + logf(sum);
+    }
+  }
+  tc_fence_before();
+  __syncthreads();
+  if (threadIdx.x == 0 && *failed != 0 && a.status) atomicExch(a.status, *failed);
+  if (warp == 8) {
+    tc_fence_after();
+    tmem_dealloc(tmem, 256);
+  }
+}
+
+// Blocks of 128 positions of one head of a strided tensor; positions past T are zeros.
+int head_map(CUtensorMap* m, const void* base, const HeadStrides& s, long long batch, long long heads,
+             long long T) {
+  const uint64_t dims[4] = {64, (uint64_t)T, (uint64_t)heads, (uint64_t)batch};
+  const uint64_t strides[3] = {(uint64_t)s.row * 2, (uint64_t)s.head * 2, (uint64_t)s.batch * 2};
+  const uint32_t box[4] = {64, 128, 1, 1};
+  return tc::make_tensor_map(m, base, 4, dims, strides, box, tc::kMapKMajor, nullptr, tc::kOperandBf16);
+}
+int configure(const void* kernel, int smem) {
+  static std::mutex mu;
+  static std::set<std::pair<int, const void*>> done;
+  int dev = 0;
+  FLB200_CUDA_CHECK(cudaGetDevice(&dev));
+  std::lock_guard<std::mutex> lock(mu);
+  if (done.count({dev, kernel})) return FLB200_OK;
+  FLB200_CUDA_CHECK(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, smem));
+  done.insert({dev, kernel});
+  return FLB200_OK;
+}
+bool head_shape_ok(long long T, long long head_dim, int dtype) {
+  return flb200_has_tensor_core_path() && dtype == FLB200_BF16 && head_dim == 64 && T > 0 && T < (1 << 24);
+}
+
+// is: strides of q, k, v; os: of o and grad_o; gs: of the gradients
+int run_attention_backward(const void* q, const void* k, const void* v, const HeadStrides& is, const void* o,
+                           const void* grad_o, const HeadStrides& os, const float* lse, void* grad_q,
+                           void* grad_k, void* grad_v, const HeadStrides& gs, long long batch,
+                           long long heads, long long T, float scale, int causal, void* workspace,
+                           cudaStream_t st) {
+  const long long rows = batch * heads * T;
+  CUtensorMap mq, mk, mv, mg;
+  if (int rc = head_map(&mq, q, is, batch, heads, T)) return rc;
+  if (int rc = head_map(&mk, k, is, batch, heads, T)) return rc;
+  if (int rc = head_map(&mv, v, is, batch, heads, T)) return rc;
+  if (int rc = head_map(&mg, grad_o, os, batch, heads, T)) return rc;
+  if (int rc = configure(reinterpret_cast<const void*>(attention_backward_kernel), kAttnSmem)) return rc;
+  const size_t acc_bytes = (size_t)rows * 64 * sizeof(float);
+  FLB200_CUDA_CHECK(cudaMemsetAsync(workspace, 0, acc_bytes, st));
+  float* dsum = reinterpret_cast<float*>(static_cast<char*>(workspace) + acc_bytes);
+  attention_dsum_kernel<<<(unsigned)((rows * 8 + 255) / 256), 256, 0, st>>>(
+      static_cast<const __nv_bfloat16*>(o), static_cast<const __nv_bfloat16*>(grad_o), dsum, rows, (int)T,
+      (int)heads);
+  FLB200_AFTER_LAUNCH("attention_dsum");
+  AttnArgs a{};
+  a.gs = gs;
+  a.heads = (int)heads;
+  a.dsum = dsum;
+  a.lse = lse;
+  a.dq_acc = static_cast<float*>(workspace);
+  a.dk = static_cast<__nv_bfloat16*>(grad_k);
+  a.dv = static_cast<__nv_bfloat16*>(grad_v);
+  a.T = (int)T;
+  a.causal = causal ? 1 : 0;
+  a.scale = scale;
+  a.status = tc::status_ptr();
+  const unsigned grid = (unsigned)(batch * heads * ((T + 127) / 128));
+  attention_backward_kernel<<<grid, kAttnThreads, kAttnSmem, st>>>(mq, mk, mv, mg, a);
+  FLB200_AFTER_LAUNCH("attention_backward");
+  tc::count_tc_launch();
+  const long long n8 = rows * 64 / 8;
+  narrow_dq_kernel<<<(unsigned)std::min<long long>((n8 + 255) / 256, 148 * 8), 256, 0, st>>>(
+      a.dq_acc, static_cast<__nv_bfloat16*>(grad_q), n8, (int)T, (int)heads, gs);
+  FLB200_AFTER_LAUNCH("attention_narrow_dq");
+  return FLB200_OK;
 }
 
 }  // namespace
@@ -378,48 +658,72 @@ int flb200_attention_backward(const void* q, const void* k, const void* v, const
   const void* ptrs[] = {q, k, v, o, grad_o, grad_q, grad_k, grad_v, workspace};
   for (const void* p : ptrs)
     FLB200_REQUIRE(aligned16(p), "attention_backward: tensors must be 16-byte aligned");
-  cudaStream_t st = as_stream(stream);
-  CUtensorMap mq, mk, mv, mg;
-  const uint64_t dims[2] = {64, (uint64_t)rows};
-  const uint64_t strides[1] = {128};
-  const uint32_t box[2] = {64, 128};
-  if (int rc = tc::make_tensor_map(&mq, q, 2, dims, strides, box, tc::kMapKMajor, nullptr, true)) return rc;
-  if (int rc = tc::make_tensor_map(&mk, k, 2, dims, strides, box, tc::kMapKMajor, nullptr, true)) return rc;
-  if (int rc = tc::make_tensor_map(&mv, v, 2, dims, strides, box, tc::kMapKMajor, nullptr, true)) return rc;
-  if (int rc = tc::make_tensor_map(&mg, grad_o, 2, dims, strides, box, tc::kMapKMajor, nullptr, true)) return rc;
-  static bool configured[64] = {false};
-  int dev = 0;
-  FLB200_CUDA_CHECK(cudaGetDevice(&dev));
-  if (dev >= 0 && dev < 64 && !configured[dev]) {
-    FLB200_CUDA_CHECK(cudaFuncSetAttribute(attention_backward_kernel,
-                                           cudaFuncAttributeMaxDynamicSharedMemorySize, kAttnSmem));
-    configured[dev] = true;
-  }
-  const size_t acc_bytes = (size_t)rows * 64 * sizeof(float);
-  FLB200_CUDA_CHECK(cudaMemsetAsync(workspace, 0, acc_bytes, st));
-  float* dsum = reinterpret_cast<float*>(static_cast<char*>(workspace) + acc_bytes);
-  attention_dsum_kernel<<<(unsigned)((rows * 8 + 255) / 256), 256, 0, st>>>(
-      static_cast<const __nv_bfloat16*>(o), static_cast<const __nv_bfloat16*>(grad_o), dsum, rows);
-  FLB200_AFTER_LAUNCH("attention_dsum");
-  AttnArgs a{};
-  a.dsum = dsum;
+  const HeadStrides dense{seq_len * 64, seq_len * 64, 64};
+  return run_attention_backward(q, k, v, dense, o, grad_o, dense, lse, grad_q, grad_k, grad_v, dense,
+                                batch_heads, 1, seq_len, scale, causal, workspace, as_stream(stream));
+}
+
+int flb200_attention_packed_supported(int64_t seq_len, int64_t head_dim, int dtype) {
+  return head_shape_ok(seq_len, head_dim, dtype) ? 1 : 0;
+}
+
+int flb200_attention_packed_forward(const void* qkv, void* out, float* lse, int64_t batch, int64_t heads,
+                                    int64_t seq_len, int64_t head_dim, float scale, int causal, int dtype,
+                                    void* stream) {
+  FLB200_REQUIRE(qkv && out, "attention_packed_forward: null tensor");
+  FLB200_REQUIRE(batch > 0 && heads > 0 && batch * heads * seq_len < 0x7fffffffLL,
+                 "attention_packed_forward: bad extents");
+  if (!head_shape_ok(seq_len, head_dim, dtype) || !aligned16(qkv) || !aligned16(out))
+    return fail(FLB200_UNSUPPORTED,
+                "attention_packed_forward: built for 16-byte aligned bf16 tensors of head dimension 64");
+  const long long width = heads * 64;
+  const HeadStrides is{seq_len * 3 * width, 64, 3 * width}, os{seq_len * width, 64, width};
+  const __nv_bfloat16* q = static_cast<const __nv_bfloat16*>(qkv);
+  CUtensorMap mq, mk, mv;
+  if (int rc = head_map(&mq, q, is, batch, heads, seq_len)) return rc;
+  if (int rc = head_map(&mk, q + width, is, batch, heads, seq_len)) return rc;
+  if (int rc = head_map(&mv, q + 2 * width, is, batch, heads, seq_len)) return rc;
+  if (int rc = configure(reinterpret_cast<const void*>(attention_forward_kernel), kFwdSmem)) return rc;
+  AttnFwdArgs a{};
+  a.out = static_cast<__nv_bfloat16*>(out);
+  a.os = os;
   a.lse = lse;
-  a.dq_acc = static_cast<float*>(workspace);
-  a.dk = static_cast<__nv_bfloat16*>(grad_k);
-  a.dv = static_cast<__nv_bfloat16*>(grad_v);
   a.T = (int)seq_len;
+  a.heads = (int)heads;
   a.causal = causal ? 1 : 0;
   a.scale = scale;
   a.status = tc::status_ptr();
-  const unsigned grid = (unsigned)(batch_heads * (seq_len / 128));
-  attention_backward_kernel<<<grid, kAttnThreads, kAttnSmem, st>>>(mq, mk, mv, mg, a);
-  FLB200_AFTER_LAUNCH("attention_backward");
+  const unsigned grid = (unsigned)(batch * heads * ((seq_len + 127) / 128));
+  attention_forward_kernel<<<grid, kAttnThreads, kFwdSmem, as_stream(stream)>>>(mq, mk, mv, a);
+  FLB200_AFTER_LAUNCH("attention_forward");
   tc::count_tc_launch();
-  const long long n8 = rows * 64 / 8;
-  narrow_dq_kernel<<<(unsigned)std::min<long long>((n8 + 255) / 256, 148 * 8), 256, 0, st>>>(
-      a.dq_acc, static_cast<__nv_bfloat16*>(grad_q), n8);
-  FLB200_AFTER_LAUNCH("attention_narrow_dq");
   return FLB200_OK;
+}
+
+int flb200_attention_packed_backward(const void* qkv, const void* out, const void* grad_out, const float* lse,
+                                     void* grad_qkv, int64_t batch, int64_t heads, int64_t seq_len,
+                                     int64_t head_dim, float scale, int causal, int dtype, void* workspace,
+                                     size_t workspace_bytes, void* stream) {
+  FLB200_REQUIRE(qkv && out && grad_out && lse && grad_qkv, "attention_packed_backward: null tensor");
+  FLB200_REQUIRE(batch > 0 && heads > 0 && batch * heads * seq_len < 0x7fffffffLL,
+                 "attention_packed_backward: bad extents");
+  const void* ptrs[] = {qkv, out, grad_out, grad_qkv, workspace};
+  bool aligned = true;
+  for (const void* p : ptrs) aligned = aligned && aligned16(p);
+  if (!head_shape_ok(seq_len, head_dim, dtype) || !aligned)
+    return fail(FLB200_UNSUPPORTED,
+                "attention_packed_backward: built for 16-byte aligned bf16 tensors of head dimension 64");
+  const size_t need = flb200_attention_backward_workspace_bytes(batch * heads, seq_len, head_dim);
+  if (!workspace || workspace_bytes < need)
+    return fail(FLB200_WORKSPACE_TOO_SMALL, "attention_packed_backward: workspace %zu < %zu",
+                workspace_bytes, need);
+  const long long width = heads * 64;
+  const HeadStrides is{seq_len * 3 * width, 64, 3 * width}, os{seq_len * width, 64, width};
+  const __nv_bfloat16* q = static_cast<const __nv_bfloat16*>(qkv);
+  __nv_bfloat16* g = static_cast<__nv_bfloat16*>(grad_qkv);
+  return run_attention_backward(q, q + width, q + 2 * width, is, out, grad_out, os, lse, g, g + width,
+                                g + 2 * width, is, batch, heads, seq_len, scale, causal, workspace,
+                                as_stream(stream));
 }
 
 }  // extern "C"

@@ -542,6 +542,34 @@ NATIVE(attention_backward) {  // (q, k, v, o, grad_o, lse, scale, causal) -> (dq
   return wrap({dq, dk, dv});
 }
 
+// (qkv [B * T, 3 * heads * hd] contiguous, B, T, heads, scale, causal) -> (out [B * T, heads * hd], lse), or
+// None where the fused kernel is not built for it
+NATIVE(attention_packed) {
+  const Tensor& qkv = x.tensor(0);
+  const int64_t B = x.i(1), T = x.i(2), h = x.i(3);
+  if (qkv.dim() != 2 || !qkv.is_contiguous() || B < 1 || T < 1 || h < 1 || qkv.size(0) != B * T ||
+      qkv.size(1) % (3 * h) != 0)
+    value_error("attention_packed: qkv must be a dense (B * T, 3 * heads * head dim) tensor");
+  const int64_t hd = qkv.size(1) / (3 * h);
+  if (!flb200_attention_packed_supported(T, hd, code_of(qkv)) || (reinterpret_cast<uintptr_t>(P(qkv)) & 15))
+    Py_RETURN_NONE;
+  Tensor out = empty({B * T, h * hd}, qkv.scalar_type(), qkv), lse = floats(B * h * T, qkv);
+  check(flb200_attention_packed_forward(P(qkv), P(out), Pf(&lse), B, h, T, hd, (float)x.d(4), x.b(5) ? 1 : 0,
+                                        code_of(qkv), stream()));
+  return wrap({out, lse});
+}
+NATIVE(attention_packed_backward) {  // (qkv, out, grad_out contiguous, lse, B, T, heads, scale, causal)
+  const Tensor &qkv = x.tensor(0), &out = x.tensor(1), &gy = x.tensor(2);
+  const int64_t B = x.i(4), T = x.i(5), h = x.i(6), hd = out.size(1) / h;
+  if (gy.sizes() != out.sizes() || !gy.is_contiguous() || gy.scalar_type() != qkv.scalar_type())
+    value_error("attention_packed_backward: grad_out must be dense and like out");
+  Tensor g = empty_like(qkv);
+  Workspace ws(flb200_attention_backward_workspace_bytes(B * h, T, hd), qkv);
+  check(flb200_attention_packed_backward(P(qkv), P(out), P(gy), Pf(x.t(3)), P(g), B, h, T, hd, (float)x.d(7),
+                                         x.b(8) ? 1 : 0, code_of(qkv), ws.p(), ws.bytes, stream()));
+  return wrap(g);
+}
+
 // ---------------------------------------------------------------- embedding
 int id_code(const Tensor& ids) {
   if (ids.scalar_type() == ScalarType::Long) return FLB200_IDS_I64;
@@ -835,7 +863,8 @@ PyMethodDef methods[] = {
     ENTRY(linear_bias_act), ENTRY(linear_backward), ENTRY(matmul), ENTRY(log_softmax),
     ENTRY(log_softmax_backward), ENTRY(cce_forward), ENTRY(cce_backward),
     ENTRY(log_softmax_cce_backward), ENTRY(softmax), ENTRY(softmax_backward),
-    ENTRY(attention_backward), ENTRY(embedding), ENTRY(embedding_backward),
+    ENTRY(attention_backward), ENTRY(attention_packed), ENTRY(attention_packed_backward),
+    ENTRY(embedding), ENTRY(embedding_backward),
     ENTRY(conv2d_cache_bytes), ENTRY(conv2d), ENTRY(conv2d_backward_data),
     ENTRY(conv2d_backward_filter_bias), ENTRY(pool2d), ENTRY(pool2d_backward), ENTRY(batchnorm),
     ENTRY(batchnorm_add_relu_supported), ENTRY(batchnorm_add_relu), ENTRY(batchnorm_backward),

@@ -264,5 +264,17 @@ def attention_backward(q, k, v, o, grad_o, lse, scale: float, causal: bool):
     return N.attention_backward(q, k, v, o, grad_o, lse, scale, causal)
 
 
+def attention_packed(qkv, B: int, T: int, heads: int, scale: float, causal: bool):
+    """softmax(scale * q k^T [+ causal mask]) v from the packed projection (B * T, 3 * heads * head
+    dim) in one kernel: returns (out (B * T, heads * head dim), lse), or None where it is not built
+    (bf16 tensors of head dimension 64 only)."""
+    return N.attention_packed(qkv, B, T, heads, scale, causal)
+
+
+def attention_packed_backward(qkv, out, grad_out, lse, B: int, T: int, heads: int, scale: float, causal: bool):
+    """Gradient of attention_packed with respect to the packed projection."""
+    return N.attention_packed_backward(qkv, out, grad_out, lse, B, T, heads, scale, causal)
+
+
 def softmax_backward(y, grad_y, scale: float = 1.0):
     return N.softmax_backward(y, grad_y, scale)

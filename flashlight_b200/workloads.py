@@ -296,6 +296,10 @@ class TransformerLM(nn.Module):
         d, h = self.d, self.heads
         hd = d // h
         qkv = self._lin(blk["qkv"], x)  # (B*T, 3d)
+        # one kernel each way on the packed projection where it is built (bf16, head dim 64)
+        ctx = A.attention_packed(qkv, B, T, h, 1.0 / math.sqrt(hd), True)
+        if ctx is not None:
+            return self._lin(blk["proj"], ctx)
 
         # pure data movement (fl::reorder with the head vectors kept whole): one copy brings the
         # head index forward for q, k and v together, (B*T, 3d) -> (3, B*h, T, hd); their
@@ -305,8 +309,7 @@ class TransformerLM(nn.Module):
             lambda t: _reorder(t, (B, T, 3, h, hd), (2, 0, 3, 1, 4)).reshape(3, B * h, T, hd),
             lambda g: _reorder(g, (3, B, h, T, hd), (1, 3, 0, 2, 4)).reshape(B * T, 3 * d), 3)
         # scores (B*h, T, T) -> softmax with the scale 1/sqrt(head dim) and the causal mask folded
-        # in -> context (B*h, T, hd); the gradient is the fused kernel where it is built (bf16,
-        # head dim 64, T a multiple of 128), which keeps no T x T tensor for the backward pass
+        # in -> context (B*h, T, hd)
         ctx = A.attention(q, k, v, 1.0 / math.sqrt(hd), causal=True)
         merged = A.glue(
             ctx, lambda t: _reorder(t, (B, h, T, hd), (0, 2, 1, 3)).reshape(B * T, d),

@@ -533,6 +533,20 @@ int flb200_attention_backward(const void* q, const void* k, const void* v, const
                               int64_t head_dim, float scale, int causal, int dtype,
                               void* workspace, size_t workspace_bytes, void* stream);
 
+/* The same operator, both ways, on the packed projection [batch][seq_len][3][heads][64] as its
+ * contraction leaves it (q, k, v of a position one after another): out and grad_out are
+ * [batch][seq_len][heads][64], grad_qkv has the layout of qkv, lse is [batch][heads][seq_len] (the
+ * forward pass writes it, or takes null).  bf16, head dimension 64, any seq_len.  Workspace of the
+ * gradient: flb200_attention_backward_workspace_bytes(batch * heads, ...). */
+int flb200_attention_packed_supported(int64_t seq_len, int64_t head_dim, int dtype);
+int flb200_attention_packed_forward(const void* qkv, void* out, float* lse, int64_t batch, int64_t heads,
+                                    int64_t seq_len, int64_t head_dim, float scale, int causal, int dtype,
+                                    void* stream);
+int flb200_attention_packed_backward(const void* qkv, const void* out, const void* grad_out,
+                                     const float* lse, void* grad_qkv, int64_t batch, int64_t heads,
+                                     int64_t seq_len, int64_t head_dim, float scale, int causal, int dtype,
+                                     void* workspace, size_t workspace_bytes, void* stream);
+
 /* logSoftmax over fl dim 0: x, y [C, X] column-major (Functions.cpp:1044-1070). */
 int flb200_log_softmax_forward(const void* x, void* y, int64_t C, int64_t X, int dtype,
                                void* stream);
