@@ -428,43 +428,59 @@ inline bool tc_operands_aligned(const void* a, const void* b, const void* c, con
 
 
 // ---- 16-bit tensors ---------------------------------------------------------------------------
-// f16 / bf16 convolutions (the reference accepts f16, backend/cudnn/Conv2D.cpp:231,266,321) run
-// as: widen the operands into fp32 copies at the front of the workspace, run the fp32 operator
+// Casts between fp32 and 16-bit tensors, and f16 / bf16 convolutions (the reference accepts f16,
+// backend/cudnn/Conv2D.cpp:231,266,321) that the tensor cores do not read as they are: widen the operands into fp32 copies at the front of the workspace, run the fp32 operator
 // in the call's math mode (TF32 tensor cores keep 10 mantissa bits, as many as f16 has and more
 // than bf16), round the result once to the 16-bit type.  Accumulation is fp32 throughout.
+// Eight elements of 16-byte aligned tensors, or what is left of them, one by one elsewhere.
+template <typename T>
+__device__ __forceinline__ void widen8(const T* in, float* out) {
+  float v[8];
+  unpack16(load16(in), v);
+#pragma unroll
+  for (int j = 0; j < 8; j += 4)
+    *reinterpret_cast<float4*>(out + j) = make_float4(v[j], v[j + 1], v[j + 2], v[j + 3]);
+}
+// Both kernels are bound by memory, on a weight matrix by their launch: 16-byte accesses, two groups
+// of a thread in flight.  (51 bf16 copies of 134 M weights: 387 us with 4-byte loads, 348 so; 131 M
+// scores to fp32: 165 and 152.)
 template <typename T>
 __global__ void widen_kernel(const T* __restrict__ in, float* __restrict__ out, long long n) {
   const long long stride = (long long)gridDim.x * blockDim.x * 8;
-  for (long long i = ((long long)blockIdx.x * blockDim.x + threadIdx.x) * 8; i < n; i += stride) {
-    if (i + 8 <= n && (reinterpret_cast<uintptr_t>(in + i) & 15) == 0) {
-      const Vec16<T> v = *reinterpret_cast<const Vec16<T>*>(in + i);
-#pragma unroll
-      for (int j = 0; j < 8; j += 4)
-        *reinterpret_cast<float4*>(out + i + j) =
-            make_float4(Num<T>::to_f(v.v[j]), Num<T>::to_f(v.v[j + 1]), Num<T>::to_f(v.v[j + 2]),
-                        Num<T>::to_f(v.v[j + 3]));
-    } else {
-      for (long long j = i; j < n && j < i + 8; ++j) out[j] = Num<T>::to_f(in[j]);
+  long long i = ((long long)blockIdx.x * blockDim.x + threadIdx.x) * 8;
+  if (((reinterpret_cast<uintptr_t>(in) | reinterpret_cast<uintptr_t>(out)) & 15) == 0) {
+    for (; i + stride + 8 <= n; i += 2 * stride) {
+      widen8(in + i, out + i);
+      widen8(in + i + stride, out + i + stride);
     }
+    for (; i + 8 <= n; i += stride) widen8(in + i, out + i);
   }
+  for (; i < n; i += stride)
+    for (long long j = i; j < n && j < i + 8; ++j) out[j] = Num<T>::to_f(in[j]);
 }
 template <typename T>
 __global__ void narrow_kernel(const float* __restrict__ in, T* __restrict__ out, long long n) {
   const long long stride = (long long)gridDim.x * blockDim.x * 8;
-  for (long long i = ((long long)blockIdx.x * blockDim.x + threadIdx.x) * 8; i < n; i += stride) {
-    if (i + 8 <= n && (reinterpret_cast<uintptr_t>(out + i) & 15) == 0) {
-      Vec16<T> v;
-#pragma unroll
-      for (int j = 0; j < 8; ++j) v.v[j] = Num<T>::from_f(in[i + j]);
-      *reinterpret_cast<Vec16<T>*>(out + i) = v;
-    } else {
-      for (long long j = i; j < n && j < i + 8; ++j) out[j] = Num<T>::from_f(in[j]);
+  long long i = ((long long)blockIdx.x * blockDim.x + threadIdx.x) * 8;
+  if (((reinterpret_cast<uintptr_t>(in) | reinterpret_cast<uintptr_t>(out)) & 15) == 0) {
+    const auto group = [&](const float4& lo, const float4& hi) {
+      const float v[8] = {lo.x, lo.y, lo.z, lo.w, hi.x, hi.y, hi.z, hi.w};
+      return pack16<T>(v);
+    };
+    const auto at = [&](long long k) { return *reinterpret_cast<const float4*>(in + k); };
+    for (; i + stride + 8 <= n; i += 2 * stride) {
+      const float4 a = at(i), b = at(i + 4), c = at(i + stride), d = at(i + stride + 4);
+      store16(out + i, group(a, b));
+      store16(out + i + stride, group(c, d));
     }
+    for (; i + 8 <= n; i += stride) store16(out + i, group(at(i), at(i + 4)));
   }
+  for (; i < n; i += stride)
+    for (long long j = i; j < n && j < i + 8; ++j) out[j] = Num<T>::from_f(in[j]);
 }
 int widen(const void* in, float* out, long long n, int dtype, cudaStream_t st) {
   if (n == 0 || !in) return FLB200_OK;
-  const unsigned grid = (unsigned)std::min<long long>((n / 8 + 255) / 256 + 1, 148 * 8);
+  const unsigned grid = (unsigned)std::min<long long>(n / 8 / 256 + 1, 16LL * device_info().sm_count);
   if (dtype == FLB200_F16)
     widen_kernel<__half><<<grid, 256, 0, st>>>(static_cast<const __half*>(in), out, n);
   else
@@ -474,7 +490,7 @@ int widen(const void* in, float* out, long long n, int dtype, cudaStream_t st) {
 }
 int narrow(const float* in, void* out, long long n, int dtype, cudaStream_t st) {
   if (n == 0 || !out) return FLB200_OK;
-  const unsigned grid = (unsigned)std::min<long long>((n / 8 + 255) / 256 + 1, 148 * 8);
+  const unsigned grid = (unsigned)std::min<long long>(n / 8 / 256 + 1, 16LL * device_info().sm_count);
   if (dtype == FLB200_F16)
     narrow_kernel<__half><<<grid, 256, 0, st>>>(in, static_cast<__half*>(out), n);
   else
