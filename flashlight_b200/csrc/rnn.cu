@@ -22,6 +22,7 @@
 #include "common.cuh"
 #include "rnn_sequence.cuh"
 #include "rnn_step.cuh"
+#include "tc_gemm.cuh"
 
 namespace flb200 {
 namespace {
@@ -105,6 +106,27 @@ int mm(int math_mode, long long m, long long n, long long k, const float* a, lon
   d.alpha = 1.f; d.beta = beta;
   d.dtype = FLB200_F32; d.math_mode = math_mode;
   return flb200_matmul(&d, a, b, c, ws, ws_bytes, stream);
+}
+
+// gates[TB][GH] = in * W_ih^T + bias: the bias in the contraction's epilogue where the tensor cores run
+// it (as a pass of its own over 16000 x 4096 gates it took 85 us), else by the channel kernel.
+int project_input(int math_mode, const RnnDims& r, const float* in, long long In, const float* w_ih,
+                  const float* bias, float* gates, void* ws, size_t ws_bytes, void* stream) {
+  flb200_matmul_desc d = {};
+  d.m = r.TB; d.n = r.GH; d.k = In; d.batch = 1;
+  d.a_row = In; d.a_col = 1;
+  d.b_row = 1; d.b_col = In;
+  d.c_row = r.GH; d.c_col = 1;
+  d.alpha = 1.f; d.beta = 0.f;
+  d.dtype = FLB200_F32; d.math_mode = math_mode;
+  if (math_mode != FLB200_MATH_STRICT_F32 && r.GH % 32 == 0 && aligned16(gates) && aligned16(bias) &&
+      tc_gemm_supported(&d, in, w_ih, gates)) {
+    tc::X3Scope x3(math_mode == FLB200_MATH_F32X3);
+    const int rc = tc_gemm_run(&d, in, w_ih, gates, ws, ws_bytes, as_stream(stream), bias);
+    if (rc != FLB200_UNSUPPORTED) return rc;
+  }
+  if (int rc = flb200_matmul(&d, in, w_ih, gates, ws, ws_bytes, stream)) return rc;
+  return flb200_channel_bias_add(gates, bias, gates, r.TB, r.GH, 1, FLB200_F32, stream);
 }
 
 size_t mm_ws(long long m, long long n, long long k) {
@@ -391,11 +413,8 @@ static int rnn_forward_impl(const flb200_rnn_desc* d, const void* x, const void*
       combine_bias_kernel<<<(unsigned)((GH + 255) / 256), 256, 0, st>>>(wf + po.b_ih, wf + po.b_hh,
                                                                         bias, H, r.G, r.mode);
       FLB200_AFTER_LAUNCH("rnn_combine_bias");
-      // all input projections of this pseudo-layer: gates[TB][GH] = in * W_ih^T + bias
-      if (int rc = mm(d->math_mode, r.TB, GH, In, in, In, 1, wf + po.w_ih, 1, In, gates, GH, 0.f,
-                      mmws, mmws_bytes, stream))
-        return rc;
-      if (int rc = flb200_channel_bias_add(gates, bias, gates, r.TB, GH, 1, FLB200_F32, stream))
+      // all input projections of this pseudo-layer
+      if (int rc = project_input(d->math_mode, r, in, In, wf + po.w_ih, bias, gates, mmws, mmws_bytes, stream))
         return rc;
       if (rows > 0) rows = rnn_sequence_rows(d->math_mode, shape, wf + po.w_hh, false);
       // (GRU: the reserve tensor q takes the place of the cell states)
@@ -654,9 +673,13 @@ static int rnn_backward_impl(const flb200_rnn_desc* d, const void* x, const void
       if (int rc = flb200_channel_sum(dgx, gwf + po.b_ih, r.TB, GH, 1, FLB200_F32, red,
                                       W.red_bytes, stream))
         return rc;
-      if (int rc = flb200_channel_sum(dgh, gwf + po.b_hh, r.TB, GH, 1, FLB200_F32, red,
-                                      W.red_bytes, stream))
+      if (dgh == dgx) {  // every cell but the GRU: the same sums
+        FLB200_CUDA_CHECK(cudaMemcpyAsync(gwf + po.b_hh, gwf + po.b_ih, (size_t)GH * 4,
+                                          cudaMemcpyDeviceToDevice, st));
+      } else if (int rc = flb200_channel_sum(dgh, gwf + po.b_hh, r.TB, GH, 1, FLB200_F32, red,
+                                             W.red_bytes, stream)) {
         return rc;
+      }
       // gradient of the layer input: din[TB][In] (+)= dgx * W_ih
       if (int rc = mm(d->math_mode, r.TB, In, GH, dgx, GH, 1, wf + po.w_ih, In, 1, din, In,
                       dir == 0 ? 0.f : 1.f, mmws, mmws_bytes, stream))
