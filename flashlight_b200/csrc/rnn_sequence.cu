@@ -11,8 +11,8 @@
 // enough: a CTA can only be asked to write step s + 2 once everybody has consumed step s, which the
 // data dependence itself ensures (each state needs all states of the step before).
 // With a grid-wide barrier per step (release counter, fence, cluster barrier) a step of a 1024-unit
-// LSTM over 32 rows took 7.2 us forward and 8.0 us backward; now 3.9 and 7.0, and the two directions
-// of a 512-unit one run together in 4.4 and 6.2.  Loads complete in order, yet neither prefetching
+// LSTM over 32 rows took 7.2 us forward and 8.0 us backward; now 3.9 and 6.9, and the two directions
+// of a 512-unit one run together in 4.4 and 6.0.  Loads complete in order, yet neither prefetching
 // the next step's gates nor loading them after the polls measured faster.
 //
 // All CTAs of a launch must be resident at once; the host asks the occupancy calculator and launches
