@@ -526,7 +526,7 @@ inline SimtPlan plan_simt(long long M, long long N, long long K, long long Z) {
     const Tile& t = tiles[i];
     const long long n = ((M + t.bm - 1) / t.bm) * ((N + t.bn - 1) / t.bn) * Z;
     for (int c = 1; c <= 8; c *= 2) {
-      if (c > 1 && K < 64LL * c) break;
+      if (c > 1 && (K < 64LL * c || Z * c > 65535)) break;  // batches and splits share grid z
       for (int p = 1; p <= 64; p *= 4) {
         if (p > 1 && (c < 8 || K < 256LL * c * p || Z * c * p > 65535)) break;
         const long long kps = (K + (long long)c * p - 1) / ((long long)c * p);

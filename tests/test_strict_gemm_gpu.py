@@ -30,6 +30,18 @@ def test_matmul_strict_loaders(mnk, a_k, b_k, offset):
     assert_close(c, a.double() @ b.double(), STRICT_TOL, f"matmul {mnk}")
 
 
+# batches that fill grid z with and without a split of K beside them (65535 is the most)
+@pytest.mark.parametrize("zmnk", [(8192, 4, 4, 512), (9000, 5, 3, 1024), (40000, 1, 2, 128), (65535, 1, 1, 256)])
+def test_matmul_strict_many_batches(zmnk):
+    from flashlight_b200 import _lib as L
+    from flashlight_b200 import functions as F
+    z, m, n, k = zmnk
+    a, b = randn(z, m, k, seed=8), randn(z, k, n, seed=9)
+    c = F.matmul(a.cuda(), b.cuda(), m=m, n=n, k=k, batch=z, a_strides=(k, 1), b_strides=(n, 1),
+                 batch_strides=(m * k, k * n, 0), math_mode=L.MATH_STRICT_F32)
+    assert_close(c, a.double() @ b.double(), STRICT_TOL, f"batched matmul {zmnk}")
+
+
 # N, C, H, W, Cout, kH, kW, stride, pad, groups: element loaders; repacked filter and channels-last
 # copy; channels not a multiple of 4; groups; a filter of many taps; stride with empty classes
 @pytest.mark.parametrize("case", [(2, 1, 9, 9, 8, 5, 5, 1, 2, 1), (16, 32, 14, 14, 64, 5, 5, 1, 2, 1),
