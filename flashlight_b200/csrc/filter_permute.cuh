@@ -11,6 +11,9 @@
 namespace flb200 {
 
 constexpr int kPermuteCo = 32;
+// The most taps of a filter whose tile fits in shared memory at one input channel per CTA (32 rows of
+// up to 1816 words: 227 KB); longer filters are left as they are.
+constexpr int kPermuteMaxTaps = 1815;
 // log2 of the input channels per CTA
 inline int permute_ci_shift(int RS) { return RS == 1 ? 5 : (RS <= 40 ? 3 : (RS <= 80 ? 2 : 0)); }
 
@@ -56,6 +59,7 @@ filter_permute_kernel(const T* __restrict__ w, T* __restrict__ out, int Cout, in
 template <typename T>
 int filter_permute(const T* w, T* out, int Cout, int C, int RS, long long s_tap, long long s_co,
                    long long s_ci, cudaStream_t st) {
+  FLB200_REQUIRE(RS <= kPermuteMaxTaps, "filter_permute: %d taps do not fit", RS);
   const int shift = permute_ci_shift(RS), run = 1 << shift;
   const size_t smem = (size_t)kPermuteCo * ((run * RS) | 1) * sizeof(T);
   if (smem > 48 * 1024)  // more than 380 taps
