@@ -359,12 +359,9 @@ int strict_image_pass(const char* name, const ConvGeo& g0, const float* src, con
     // out[z][k][row], k = (tap, channel) for channel runs, else (channel, tap)
     float* out = reinterpret_cast<float*>(at);
     const long long s_tap = (long long)N * (vec ? ch : 1), s_ch = (long long)N * (vec ? 1 : g.RS);
-    for (int z = 0; z < g.groups; ++z) {
-      const long long group = (long long)z * g.Coutg * g.Cg * g.RS;
-      if (int rc = filter_permute(w + group, out + group, g.Coutg, g.Cg, g.RS, s_tap, DGRAD ? s_ch : 1,
-                                  DGRAD ? 1 : s_ch, st))
-        return rc;
-    }
+    if (int rc = filter_permute(w, out, g.Coutg, g.Cg, g.RS, s_tap, DGRAD ? s_ch : 1, DGRAD ? 1 : s_ch, st,
+                                g.groups))
+      return rc;
     packed = out;
     at += need.filter;
   }

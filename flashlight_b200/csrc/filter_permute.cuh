@@ -1,10 +1,11 @@
 // Repacking of convolution filters: w[co][ci][tap] to out[tap * s_tap + co * s_co + ci * s_ci],
-// where one of s_co, s_ci is 1.  A CTA brings 32 output channels x a short run of input channels x
-// all taps into shared memory along the filter's own contiguous order and writes it out along the
-// contiguous index of the target, so both sides move whole sectors; the runs are short (8 input
-// channels) because most filters are small and a few CTAs would be bound by their own latency.
-// (A thread per target element read the filter kH * kW elements apart: 57 us for a 13-tap
-// 1024 x 1024 filter, 54 MB; now 37.)
+// where one of s_co, s_ci is 1; the grid's z walks groups of Cout * C * RS words on both sides.  A
+// CTA brings 32 output channels x a short run of input channels x all taps into shared memory along
+// the filter's own contiguous order and writes it out along the contiguous index of the target, so
+// both sides move whole sectors; the runs are short (8 input channels) because most filters are
+// small and a few CTAs would be bound by their own latency.  (A thread per target element read the
+// filter kH * kW elements apart: 57 us for a 13-tap 1024 x 1024 filter, 54 MB; now 37.  With a
+// launch per group, 256 groups of 4 x 4 channels took 1 ms.)
 #pragma once
 #include "common.cuh"
 
@@ -28,6 +29,9 @@ filter_permute_kernel(const T* __restrict__ w, T* __restrict__ out, int Cout, in
   const int nco = min(kPermuteCo, Cout - co0), nci = min(ci_run, C - ci0);
   const int run = nci * RS, pitch = (ci_run * RS) | 1;
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  const long long group = (long long)blockIdx.z * Cout * C * RS;
+  w += group;
+  out += group;
   // i / RS for the small i of a tile (rs_magic = ceil(2^32 / RS), 0 for RS == 1)
   auto over_rs = [&](int i) { return rs_magic ? (int)__umulhi((unsigned)i, rs_magic) : i; };
 #pragma unroll
@@ -58,15 +62,16 @@ filter_permute_kernel(const T* __restrict__ w, T* __restrict__ out, int Cout, in
 
 template <typename T>
 int filter_permute(const T* w, T* out, int Cout, int C, int RS, long long s_tap, long long s_co,
-                   long long s_ci, cudaStream_t st) {
+                   long long s_ci, cudaStream_t st, int groups = 1) {
   FLB200_REQUIRE(RS <= kPermuteMaxTaps, "filter_permute: %d taps do not fit", RS);
   const int shift = permute_ci_shift(RS), run = 1 << shift;
   const size_t smem = (size_t)kPermuteCo * ((run * RS) | 1) * sizeof(T);
   if (smem > 48 * 1024)  // more than 380 taps
     FLB200_CUDA_CHECK(cudaFuncSetAttribute(filter_permute_kernel<T>,
                                            cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
-  dim3 grid((unsigned)((C + run - 1) / run), (unsigned)((Cout + kPermuteCo - 1) / kPermuteCo));
-  FLB200_REQUIRE(grid.y <= 65535, "filter_permute: too many channels");
+  dim3 grid((unsigned)((C + run - 1) / run), (unsigned)((Cout + kPermuteCo - 1) / kPermuteCo),
+            (unsigned)groups);
+  FLB200_REQUIRE(grid.y <= 65535 && groups <= 65535, "filter_permute: too many channels");
   const unsigned magic = RS == 1 ? 0u : (unsigned)(((1ull << 32) + RS - 1) / RS);
   filter_permute_kernel<T><<<grid, 256, smem, st>>>(w, out, Cout, C, RS, magic, shift, s_tap, s_co, s_ci);
   FLB200_AFTER_LAUNCH("filter_permute");

@@ -73,3 +73,21 @@ def test_conv_strict_routes(case, channels_last):
     wgw, wgb = R.conv2d_backward_filter_bias(gy.double(), x.double(), w.shape, True, *args)
     assert_close(gw, wgw, STRICT_TOL, "conv dw")
     assert_close(gb, wgb, STRICT_TOL, "conv db")
+
+
+def test_conv_strict_groups_launch_once():
+    """The filters of all groups are repacked by one launch, and the results are those of the groups
+    one by one."""
+    from flashlight_b200 import _lib as L
+    from flashlight_b200.extension import B200AutogradExtension
+    ext = B200AutogradExtension(math_mode=L.MATH_STRICT_F32)
+    N, C, H, groups = 8, 256, 20, 64
+    args = (1, 1, 1, 1, 1, 1, groups)
+    x, w = randn(N, C, H, H, seed=21), randn(C, C // groups, 3, 3, seed=22) / 6
+    gy = randn(N, C, H, H, seed=23)
+    before = L.kernel_launches()
+    y = ext.conv2d(x.cuda(), w.cuda(), None, *args)
+    gx = ext.conv2dBackwardData(gy.cuda(), x.cuda(), w.cuda(), *args)
+    assert L.kernel_launches() - before <= 8
+    assert_close(y, R.conv2d(x.double(), w.double(), None, *args), STRICT_TOL, "conv forward")
+    assert_close(gx, R.conv2d_backward_data(gy.double(), x.shape, w.double(), *args), STRICT_TOL, "conv dx")
