@@ -313,8 +313,9 @@ StrictScratch strict_scratch(const ConvGeo& g, int which) {
   StrictScratch s{0, 0, 0};
   if ((double)g.N * (which == 1 ? g.HW : g.HoWo) * g.Cout * g.Cg * g.RS < kStrictCopyWork) return s;
   const size_t x = up256c((size_t)g.N * g.C * g.HW * 4), gy = up256c((size_t)g.N * g.Cout * g.HoWo * 4);
-  const bool x_copy = !g.x_cl && g.Cg % 4 == 0 && g.C >= 8;
-  const bool gy_copy = !g.y_cl && g.Coutg % 4 == 0 && g.Cout >= 8;
+  const bool images = g.N <= 65535;  // the copying kernels put them in the grid's third extent
+  const bool x_copy = !g.x_cl && g.Cg % 4 == 0 && g.C >= 8 && images;
+  const bool gy_copy = !g.y_cl && g.Coutg % 4 == 0 && g.Cout >= 8 && images;
   if (which != 2 && g.RS <= kPermuteMaxTaps) s.filter = up256c((size_t)g.Cout * g.Cg * g.RS * 4);
   if (which == 0 && x_copy) s.x = x;
   if (which == 1 && gy_copy) s.gy = gy;

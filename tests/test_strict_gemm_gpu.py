@@ -44,12 +44,14 @@ def test_matmul_strict_many_batches(zmnk):
 
 # N, C, H, W, Cout, kH, kW, stride, pad, groups: element loaders; repacked filter and channels-last
 # copy; channels not a multiple of 4; groups; a filter of many taps; stride with empty classes;
-# filters whose repacking needs more than the default shared memory, and more than there is
+# filters whose repacking needs more than the default shared memory, and more than there is; more
+# images than a grid's third extent
 @pytest.mark.parametrize("case", [(2, 1, 9, 9, 8, 5, 5, 1, 2, 1), (16, 32, 14, 14, 64, 5, 5, 1, 2, 1),
                                   (8, 36, 13, 15, 44, 3, 3, 2, 1, 1), (16, 30, 14, 14, 66, 3, 3, 1, 1, 1),
                                   (16, 64, 12, 12, 64, 3, 3, 1, 1, 4), (2, 16, 1, 70, 24, 1, 13, 1, 0, 1),
                                   (40, 64, 17, 17, 256, 1, 1, 2, 0, 1), (8, 64, 30, 30, 64, 1, 1, 1, 0, 1),
-                                  (2, 8, 1, 900, 16, 1, 401, 1, 0, 1), (2, 4, 1, 2500, 8, 1, 2001, 1, 0, 1)])
+                                  (2, 8, 1, 900, 16, 1, 401, 1, 0, 1), (2, 4, 1, 2500, 8, 1, 2001, 1, 0, 1),
+                                  (70000, 8, 1, 6, 16, 1, 3, 1, 0, 1)])
 @pytest.mark.parametrize("channels_last", [False, True])
 def test_conv_strict_routes(case, channels_last):
     from flashlight_b200 import _lib as L
