@@ -200,16 +200,26 @@ column_reduce_kernel(const T* __restrict__ a, const T* __restrict__ b,
   }
 }
 
+// Element by element.  The threads walk in steps of a multiple of the channels, so that each stays on
+// one channel and makes its constants once, the batch-norm scale in fp64 among them (64 x 30 x 112 x 112
+// f16 in evaluation mode: 95 us with a scale per element, 61 with scales from a kernel before, 37 so).
+// Only where the channels outnumber the threads does a thread change them.
 template <typename T, int NIN, typename F>
 __global__ void __launch_bounds__(256)
 column_apply_kernel(const T* __restrict__ a, const T* __restrict__ b, T* __restrict__ out,
                     long long rows, long long channels, F f) {
   const long long total = rows * channels;
-  const long long stride = (long long)gridDim.x * blockDim.x;
-  for (long long t = (long long)blockIdx.x * blockDim.x + threadIdx.x; t < total; t += stride) {
-    const long long c = t % channels;
-    const typename F::K k = f.channel(c);
+  const long long threads = (long long)gridDim.x * blockDim.x;
+  const bool fixed = threads >= channels;
+  const long long stride = fixed ? threads - threads % channels : threads;
+  long long t = (long long)blockIdx.x * blockDim.x + threadIdx.x;
+  if (t >= stride || t >= total) return;
+  typename F::K k = f.channel(t % channels);
+  while (true) {
     out[t] = Num<T>::from_f(f.apply(k, Num<T>::to_f(a[t]), NIN == 2 ? Num<T>::to_f(b[t]) : 0.f));
+    t += stride;
+    if (t >= total) return;
+    if (!fixed) k = f.channel(t % channels);
   }
 }
 

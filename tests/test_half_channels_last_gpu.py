@@ -92,3 +92,25 @@ def test_conv_16bit_channels_last(dtype, case):
     wgw, wgb = R.conv2d_backward_filter_bias(gy.double(), x.double(), w.shape, True, *args)
     assert_close_scaled(gw.float(), wgw, tol, "conv dw")
     assert_close_scaled(gb.float(), wgb, tol, "conv db")
+
+
+# channels off the vectors: a thread keeps to one channel, unless there are more channels than threads
+@pytest.mark.parametrize("dtype", [torch.float32, torch.float16])
+@pytest.mark.parametrize("shape", [(3, 30, 20, 21), (1, 5, 2, 1), (1, 2051, 1, 2), (64, 33, 30, 30)])
+def test_batchnorm_element_kernels(dtype, shape):
+    from flashlight_b200 import _lib as L
+    from flashlight_b200.extension import B200AutogradExtension
+    ext, tol = B200AutogradExtension(math_mode=L.MATH_TF32), TOL.get(dtype, 1e-4)
+    ch = shape[1]
+    x, gy = (randn(*shape, seed=191) * 1.7 + 0.4).to(dtype), randn(*shape, seed=192).to(dtype)
+    w, b = randn(ch, seed=193).abs() + 0.5, randn(ch, seed=194)
+    rm, rv = randn(ch, seed=195), randn(ch, seed=196).abs() + 0.3
+    y = ext.batchnorm(cl(x), w.cuda(), b.cuda(), rm.cuda(), rv.cuda(), [2], False, 0.0, 1e-5)[0]
+    want = R.batchnorm(x.double(), w.double(), b.double(), rm.double(), rv.double(), [2], False, 0.0, 1e-5)[0]
+    assert_close_scaled(y.float(), want, tol, "bn evaluation")
+    if x.numel() < 64 * ch:  # the gradient of two rows per channel is what their cancellation leaves
+        return
+    _, sm, sv = ext.batchnorm(cl(x), w.cuda(), b.cuda(), None, None, [2], True, 0.0, 1e-5)
+    got = ext.batchnormBackward(cl(gy), sm, sv, cl(x), w.cuda(), [2], True, 1e-5)
+    for g, v in zip(got, R.batchnorm_backward(gy.double(), x.double(), w.double(), [2], 1e-5)):
+        assert_close_scaled(g.float(), v, tol, "bn gradient")
