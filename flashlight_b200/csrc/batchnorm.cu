@@ -599,9 +599,10 @@ int launch_reduce(const char* name, const void* a, const void* b, float2* partia
                   long long outer, long long channels, long long inner, F f, int* splits_out,
                   cudaStream_t st) {
   if (inner == 1) {
-    const int splits = column_splits(outer, channels);
+    const bool vec = channels % Vec16<T>::N == 0 && aligned16(a) && (NIN == 1 || aligned16(b));
+    const int splits = column_splits(outer, channels, vec);
     const long long rps = (outer + splits - 1) / splits;
-    if (channels % Vec16<T>::N == 0 && aligned16(a) && (NIN == 1 || aligned16(b))) {
+    if (vec) {
       const ColumnTiling ct = column_tiling(channels, Vec16<T>::N);
       dim3 vgrid((unsigned)ct.col_blocks, (unsigned)splits);
       column_reduce_vec_kernel<T, NIN, F><<<vgrid, 256, 0, st>>>(
@@ -1064,7 +1065,7 @@ static int batchnorm_backward_impl(bool relu, const uint8_t* tail_mask, const vo
   int rc = FLB200_OK, splits = 0;
   if (tail_mask && d->inner == 1) {
     const OctetTiling ot = octet_tiling(C);
-    splits = column_splits(d->outer, C);
+    splits = column_splits(d->outer, C, true);
     const long long rps = (d->outer + splits - 1) / splits;
     FLB200_DISPATCH_DTYPE(
         d->dtype, "batchnorm_add_relu_backward",

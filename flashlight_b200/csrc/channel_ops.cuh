@@ -319,9 +319,15 @@ column_reduce_vec_kernel(const T* __restrict__ a, const T* __restrict__ b,
     const long long cc = (long long)blockIdx.x * cq * V + t;
     if (cc < channels) {
       float t0 = 0.f, t1 = 0.f;
-      for (int i = 0; i < rl; ++i) {
-        t0 += sh0[i * cq * V + t];
-        t1 += sh1[i * cq * V + t];
+      for (int i0 = 0; i0 < rl; i0 += 4) {  // (rl is 4 or a multiple of it; short chains as above)
+        float g0 = 0.f, g1 = 0.f;
+#pragma unroll
+        for (int i = 0; i < 4; ++i) {
+          g0 += sh0[(i0 + i) * cq * V + t];
+          g1 += sh1[(i0 + i) * cq * V + t];
+        }
+        t0 += g0;
+        t1 += g1;
       }
       partial[cc * splits + s] = make_float2(t0, t1);
     }
@@ -374,14 +380,17 @@ column_apply_vec_kernel(const T* __restrict__ a, const T* __restrict__ b,
   }
 }
 
-// Splits of the column path (rows handled per CTA): one wave of three CTAs per SM (the kernel's
-// registers allow that many with 16-bit data) over the vector tiling's column blocks, at least 32
-// rows each, at most 512 splits.  Where that would round to a few splits, two waves of them.
-inline int column_splits(long long rows, long long channels) {
-  const long long col_blocks = column_tiling(channels).col_blocks;
-  long long splits = 3LL * device_info().sm_count / col_blocks;
-  if (splits < 8) splits = (6LL * device_info().sm_count + col_blocks - 1) / col_blocks;
-  const long long max_by_work = (rows + 31) / 32;
+// Splits of the column path (rows handled per CTA), at most 512.  The vector kernel: one wave of three
+// CTAs per SM (its registers allow that many with 16-bit data) over its column blocks, at least 32 rows
+// each; where that would round to a few splits, two waves of them.  The element kernel has fewer loads
+// in flight per thread: two waves, at least 64 rows each (the gradient sums of 64 x 33 x 56 x 56 f32:
+// 57 us with the vector kernel's splits, 43 so, and shorter chains of additions).
+inline int column_splits(long long rows, long long channels, bool vec) {
+  const long long sm = device_info().sm_count, col_blocks = column_tiling(channels).col_blocks;
+  const long long two_waves = (6 * sm + col_blocks - 1) / col_blocks;
+  long long splits = vec ? 3 * sm / col_blocks : two_waves;
+  if (splits < 8) splits = two_waves;
+  const long long least = vec ? 32 : 64, max_by_work = (rows + least - 1) / least;
   if (splits > max_by_work) splits = max_by_work;
   if (splits > 512) splits = 512;
   if (splits < 1) splits = 1;
@@ -402,11 +411,12 @@ inline long long apply_rows_per_split(long long rows, long long col_blocks, long
   return ((rows + splits - 1) / splits + unit - 1) / unit * unit;
 }
 
-// Scratch bytes for the (channel, split) partial sums of any op built on these.
+// Scratch bytes for the (channel, split) partial sums of any op built on these, whichever kernel
+// the alignment of its tensors leads to.
 inline size_t channel_partial_bytes(long long outer, long long channels, long long inner) {
   long long splits;
   if (inner == 1) {
-    splits = column_splits(outer, channels);
+    splits = std::max(column_splits(outer, channels, true), column_splits(outer, channels, false));
   } else {
     splits = make_channel_geo(outer, channels, inner).splits;
   }
