@@ -597,10 +597,10 @@ __global__ void bn_bwd_finalize_kernel(const float2* __restrict__ partial, int s
 template <typename T, int NIN, typename F>
 int launch_reduce(const char* name, const void* a, const void* b, float2* partial,
                   long long outer, long long channels, long long inner, F f, int* splits_out,
-                  cudaStream_t st) {
+                  cudaStream_t st, int most_splits = 512) {
   if (inner == 1) {
     const bool vec = channels % Vec16<T>::N == 0 && aligned16(a) && (NIN == 1 || aligned16(b));
-    const int splits = column_splits(outer, channels, vec);
+    const int splits = std::min(column_splits(outer, channels, vec), most_splits);
     const long long rps = (outer + splits - 1) / splits;
     if (vec) {
       const ColumnTiling ct = column_tiling(channels, Vec16<T>::N);
@@ -704,6 +704,21 @@ size_t flb200_channel_sum_workspace_bytes(int64_t outer, int64_t channels, int64
   return channel_partial_bytes(outer, channels, inner);
 }
 
+static int channel_sum_impl(const void* in, float* out, long long outer, long long channels, long long inner,
+                            int dtype, void* workspace, int most_splits, void* stream) {
+  cudaStream_t st = as_stream(stream);
+  float2* partial = static_cast<float2*>(workspace);
+  int splits = 0;
+  int rc = FLB200_OK;
+  FLB200_DISPATCH_DTYPE(dtype, "channel_sum",
+                        rc = (launch_reduce<T, 1>("channel_sum", in, nullptr, partial, outer, channels, inner,
+                                                  SumF{}, &splits, st, most_splits)));
+  if (rc) return rc;
+  sum_finalize_kernel<<<fin_grid(channels), kFinThreads, 0, st>>>(partial, splits, channels, out);
+  FLB200_AFTER_LAUNCH("channel_sum_finalize");
+  return FLB200_OK;
+}
+
 int flb200_channel_sum(const void* in, float* out, int64_t outer, int64_t channels, int64_t inner,
                        int dtype, void* workspace, size_t workspace_bytes, void* stream) {
   if (int st = check_geo("channel_sum", outer, channels, inner)) return st;
@@ -711,17 +726,7 @@ int flb200_channel_sum(const void* in, float* out, int64_t outer, int64_t channe
   if (workspace_bytes < channel_partial_bytes(outer, channels, inner) || !workspace)
     return fail(FLB200_WORKSPACE_TOO_SMALL, "channel_sum: workspace %zu < %zu", workspace_bytes,
                 channel_partial_bytes(outer, channels, inner));
-  cudaStream_t st = as_stream(stream);
-  float2* partial = static_cast<float2*>(workspace);
-  int splits = 0;
-  int rc = FLB200_OK;
-  FLB200_DISPATCH_DTYPE(dtype, "channel_sum",
-                        rc = (launch_reduce<T, 1>("channel_sum", in, nullptr, partial, outer,
-                                                  channels, inner, SumF{}, &splits, st)));
-  if (rc) return rc;
-  sum_finalize_kernel<<<fin_grid(channels), kFinThreads, 0, st>>>(partial, splits, channels, out);
-  FLB200_AFTER_LAUNCH("channel_sum_finalize");
-  return FLB200_OK;
+  return channel_sum_impl(in, out, outer, channels, inner, dtype, workspace, 512, stream);
 }
 
 // ---- channel sum for callers that cannot hand over scratch memory ------------------------
@@ -737,7 +742,11 @@ static __device__ __align__(256) unsigned char g_channel_sum_scratch[kStaticScra
 int flb200_channel_sum_static_scratch(const void* in, float* out, int64_t outer, int64_t channels,
                                       int64_t inner, int dtype, void* stream) {
   if (int st = check_geo("channel_sum_static_scratch", outer, channels, inner)) return st;
-  const size_t need = channel_partial_bytes(outer, channels, inner);
+  FLB200_REQUIRE(in && out, "channel_sum_static_scratch: null pointer");
+  // The shapes that fit are those whose partial sums fit with the element kernel's splits; the vector
+  // kernel, which likes more of them for few rows, then makes do with what the array holds.
+  const size_t need = inner == 1 ? (size_t)channels * column_splits(outer, channels, false) * sizeof(float2)
+                                 : channel_partial_bytes(outer, channels, inner);
   if (need > kStaticScratchBytes)
     return fail(FLB200_INVALID_ARG,
                 "channel_sum_static_scratch: this shape needs %zu bytes of partial sums, the "
@@ -768,8 +777,8 @@ int flb200_channel_sum_static_scratch(const void* in, float* out, int64_t outer,
                 cudaGetErrorString(lookup_error[dev]));
   }
   // Every partial is written before it is read, so stale contents of earlier calls do no harm.
-  return flb200_channel_sum(in, out, outer, channels, inner, dtype, device_addr[dev],
-                            kStaticScratchBytes, stream);
+  return channel_sum_impl(in, out, outer, channels, inner, dtype, device_addr[dev],
+                          (int)std::min<size_t>(512, kStaticScratchBytes / (channels * sizeof(float2))), stream);
 }
 
 int flb200_channel_bias_add(const void* x, const float* bias, void* y, int64_t outer,

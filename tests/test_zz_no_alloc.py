@@ -44,6 +44,19 @@ def test_static_scratch_matches_caller_scratch_on_two_calls_in_a_row():
         assert err <= 1e-4
 
 
+@pytest.mark.parametrize("outer, channels", [(256, 20000), (512, 16384), (64, 131072)])
+def test_static_scratch_takes_few_rows_of_many_channels(outer, channels):
+    """Their partial sums fit at a split per 64 rows, although flb200_channel_sum would split more."""
+    from flashlight_b200 import _lib as L
+    x = torch.randn(outer, channels, generator=torch.Generator().manual_seed(6)).cuda()
+    out = torch.empty(channels, device="cuda")
+    L.check(L.lib.flb200_channel_sum_static_scratch(x.data_ptr(), out.data_ptr(), outer, channels, 1, L.F32,
+                                                    torch.cuda.current_stream().cuda_stream))
+    torch.cuda.synchronize()
+    ref = x.double().sum(0)
+    assert float((out.double() - ref).abs().max() / ref.abs().max()) <= 1e-5
+
+
 def test_static_scratch_refuses_shapes_beyond_its_array():
     from flashlight_b200 import _lib as L
     outer, channels, inner = 4096, 40000, 1   # 40000 channels x 64 splits x 8 B > 1 MiB
