@@ -96,6 +96,18 @@ void check(int status) {
   throw PyRaised();
 }
 
+// Other threads run while the library or the allocator does: a launch waits where the device's queue
+// is full, an allocation may wait for the device.  The arguments are made before, with the lock held.
+struct Unlocked {
+  PyThreadState* state = PyEval_SaveThread();
+  ~Unlocked() { PyEval_RestoreThread(state); }
+};
+template <class R, class... Params, class... A>
+R unlocked(R (*f)(Params...), A... a) {
+  const Unlocked u;
+  return f(a...);
+}
+
 template <class F>
 PyObject* guarded(F f) {
   HANDLE_TH_ERRORS
@@ -155,6 +167,7 @@ void* stream() { return c10::cuda::getCurrentCUDAStream().stream(); }
 
 Tensor empty(at::IntArrayRef shape, ScalarType type, const Tensor& like, bool cl = false) {
   if (!like.is_cuda()) value_error("the B200 autograd extension needs device (CUDA) tensors");
+  const Unlocked u;
   return at::detail::empty_cuda(shape, type, like.device(),
                                 cl ? std::optional<at::MemoryFormat>(at::MemoryFormat::ChannelsLast)
                                    : std::nullopt);
@@ -194,9 +207,9 @@ NATIVE(unary) {  // (op, x)
   Tensor out = empty_like(in);
   const int64_t n = in.numel();
   switch (x.n32(0)) {
-    case U_RELU: check(flb200_relu_forward(P(in), P(out), n, dt, stream())); break;
-    case U_GELU: check(flb200_gelu_forward(P(in), P(out), n, dt, stream())); break;
-    default: check(flb200_tanh_forward(P(in), P(out), n, dt, stream()));
+    case U_RELU: check(unlocked(flb200_relu_forward, P(in), P(out), n, dt, stream())); break;
+    case U_GELU: check(unlocked(flb200_gelu_forward, P(in), P(out), n, dt, stream())); break;
+    default: check(unlocked(flb200_tanh_forward, P(in), P(out), n, dt, stream()));
   }
   return wrap(out);
 }
@@ -210,10 +223,10 @@ NATIVE(binary) {  // (op, a, b, out or None)
   Tensor out = given ? *given : empty_like(a);
   const int64_t n = a.numel();
   switch (x.n32(0)) {
-    case B_RELU: check(flb200_relu_backward(P(a), P(b), P(out), n, dt, stream())); break;
-    case B_GELU: check(flb200_gelu_backward(P(a), P(b), P(out), n, dt, stream())); break;
-    case B_TANH: check(flb200_tanh_backward(P(a), P(b), P(out), n, dt, stream())); break;
-    default: check(flb200_add(P(a), P(b), P(out), n, dt, stream()));
+    case B_RELU: check(unlocked(flb200_relu_backward, P(a), P(b), P(out), n, dt, stream())); break;
+    case B_GELU: check(unlocked(flb200_gelu_backward, P(a), P(b), P(out), n, dt, stream())); break;
+    case B_TANH: check(unlocked(flb200_tanh_backward, P(a), P(b), P(out), n, dt, stream())); break;
+    default: check(unlocked(flb200_add, P(a), P(b), P(out), n, dt, stream()));
   }
   return wrap(out);
 }
@@ -227,9 +240,9 @@ NATIVE(relu_mask) {  // (a, b) -> (y, mask)
   Tensor y = empty_like(a), mask = empty({(a.numel() + 7) / 8}, ScalarType::Byte, a);
   uint8_t* m = static_cast<uint8_t*>(mask.data_ptr());
   if (b)
-    check(flb200_add_relu_forward_mask(P(a), P(*b), P(y), m, a.numel(), dt, stream()));
+    check(unlocked(flb200_add_relu_forward_mask, P(a), P(*b), P(y), m, a.numel(), dt, stream()));
   else
-    check(flb200_relu_forward_mask(P(a), P(y), m, a.numel(), dt, stream()));
+    check(unlocked(flb200_relu_forward_mask, P(a), P(y), m, a.numel(), dt, stream()));
   return wrap({y, mask});
 }
 NATIVE(relu_mask_backward) {  // (mask, ga, gb or None)
@@ -240,9 +253,9 @@ NATIVE(relu_mask_backward) {  // (mask, ga, gb or None)
   Tensor gx = empty_like(ga);
   const uint8_t* m = static_cast<const uint8_t*>(P(x.tensor(0)));
   if (gb)
-    check(flb200_relu_backward_mask_sum(m, P(ga), P(*gb), P(gx), ga.numel(), dt, stream()));
+    check(unlocked(flb200_relu_backward_mask_sum, m, P(ga), P(*gb), P(gx), ga.numel(), dt, stream()));
   else
-    check(flb200_relu_backward_mask(m, P(ga), P(gx), ga.numel(), dt, stream()));
+    check(unlocked(flb200_relu_backward_mask, m, P(ga), P(gx), ga.numel(), dt, stream()));
   return wrap(gx);
 }
 
@@ -251,7 +264,7 @@ NATIVE(dropout_apply) {  // (x, mask, scale)
   if (!same_layout(in, mask) || in.scalar_type() != mask.scalar_type())
     value_error("mask must match the tensor's shape, memory layout and dtype");
   Tensor out = empty_like(in);
-  check(flb200_dropout_apply(P(in), P(mask), P(out), (float)x.d(2), in.numel(), code_of(in), stream()));
+  check(unlocked(flb200_dropout_apply, P(in), P(mask), P(out), (float)x.d(2), in.numel(), code_of(in), stream()));
   return wrap(out);
 }
 
@@ -259,7 +272,7 @@ NATIVE(astype) {  // (x, dtype code)
   const Tensor& in = x.tensor(0);
   const int dst = x.n32(1);
   Tensor out = empty(in.sizes(), type_of(dst), in);
-  check(flb200_astype(P(in), code_of(in), P(out), dst, in.numel(), stream()));
+  check(unlocked(flb200_astype, P(in), code_of(in), P(out), dst, in.numel(), stream()));
   return wrap(out);
 }
 
@@ -297,7 +310,7 @@ NATIVE(reorder) {  // (x, shape tuple, perm tuple)
     }
   }
   Tensor out = empty(at::IntArrayRef(out_shape, n), in.scalar_type(), in);
-  check(flb200_reorder(P(in), P(out), dims, st, inner, code_of(in), stream()));
+  check(unlocked(flb200_reorder, P(in), P(out), dims, st, inner, code_of(in), stream()));
   return wrap(out);
 }
 
@@ -306,7 +319,7 @@ NATIVE(bernoulli_mask) {  // (out, keep_prob, seed, offset)
   const uint64_t seed = PyLong_AsUnsignedLongLongMask(x.at(2));
   const uint64_t off = PyLong_AsUnsignedLongLongMask(x.at(3));
   if (PyErr_Occurred()) throw PyRaised();
-  check(flb200_bernoulli_mask(P(out), out.numel(), (float)x.d(1), seed, off, code_of(out), stream()));
+  check(unlocked(flb200_bernoulli_mask, P(out), out.numel(), (float)x.d(1), seed, off, code_of(out), stream()));
   Py_RETURN_NONE;
 }
 
@@ -316,14 +329,14 @@ NATIVE(channel_sum) {  // (x, outer, channels, inner)
   if (in.numel() != o * c * n) value_error("channel_sum: geometry does not match the tensor");
   Tensor out = floats(c, in);
   Workspace ws(flb200_channel_sum_workspace_bytes(o, c, n), in);
-  check(flb200_channel_sum(P(in), Pf(&out), o, c, n, code_of(in), ws.p(), ws.bytes, stream()));
+  check(unlocked(flb200_channel_sum, P(in), Pf(&out), o, c, n, code_of(in), ws.p(), ws.bytes, stream()));
   return wrap(out);
 }
 NATIVE(channel_bias_add) {  // (x, bias, outer, channels, inner, out or None)
   const Tensor& in = x.tensor(0);
   const Tensor* given = x.t(5);
   Tensor out = given ? *given : empty_like(in);
-  check(flb200_channel_bias_add(P(in), Pf(x.t(1)), P(out), x.i(2), x.i(3), x.i(4), code_of(in), stream()));
+  check(unlocked(flb200_channel_bias_add, P(in), Pf(x.t(1)), P(out), x.i(2), x.i(3), x.i(4), code_of(in), stream()));
   return wrap(out);
 }
 
@@ -332,7 +345,7 @@ NATIVE(layernorm) {  // (x contiguous, weight, bias, eps) -> (y, xhat, invstd)
   const Tensor& in = x.tensor(0);
   const int64_t feat = in.size(-1), rows = feat ? in.numel() / feat : 0;
   Tensor y = empty_like(in), xhat = empty_like(in), invstd = floats(rows, in);
-  check(flb200_layernorm_forward(P(in), Pf(x.t(1)), Pf(x.t(2)), P(y), P(xhat), nullptr, Pf(&invstd), rows,
+  check(unlocked(flb200_layernorm_forward, P(in), Pf(x.t(1)), Pf(x.t(2)), P(y), P(xhat), nullptr, Pf(&invstd), rows,
                                  feat, x.d(3), code_of(in), stream()));
   return wrap({y, xhat, invstd});
 }
@@ -343,7 +356,7 @@ NATIVE(layernorm_backward) {  // (grad_y contiguous, xhat, weight, invstd, need_
   if (x.b(4)) gx = empty_like(xhat);
   if (x.b(5)) { gw = floats(feat, xhat); gb = floats(feat, xhat); }
   Workspace ws(flb200_layernorm_backward_workspace_bytes(rows, feat), xhat);
-  check(flb200_layernorm_backward(P(gy), P(xhat), Pf(x.t(2)), Pf(x.t(3)), gx.defined() ? P(gx) : nullptr,
+  check(unlocked(flb200_layernorm_backward, P(gy), P(xhat), Pf(x.t(2)), Pf(x.t(3)), gx.defined() ? P(gx) : nullptr,
                                   gw.defined() ? Pf(&gw) : nullptr, gb.defined() ? Pf(&gb) : nullptr, rows,
                                   feat, code_of(xhat), ws.p(), ws.bytes, stream()));
   return wrap({gx, gw, gb});
@@ -374,7 +387,7 @@ NATIVE(linear) {  // (x, weight, bias or None, mode)
   const LinearDims d = linear_dims(w, in);
   Tensor y = rows_of(in, d.O);
   Workspace ws(flb200_linear_workspace_bytes(d.O, d.I, d.cols, 0), in);
-  check(flb200_linear_forward(d.O, d.I, d.cols, P(w), P(in), P(x.t(2)), P(y), x.n32(3), ws.p(), ws.bytes,
+  check(unlocked(flb200_linear_forward, d.O, d.I, d.cols, P(w), P(in), P(x.t(2)), P(y), x.n32(3), ws.p(), ws.bytes,
                               stream()));
   return wrap(y);
 }
@@ -390,8 +403,8 @@ NATIVE(linear_bias_act) {  // (x, weight, bias or None, gelu, mode) -> (y, pre) 
   Tensor y = rows_of(in, d.O), pre;
   if (gelu) pre = empty_like(y);
   Workspace ws(flb200_linear_workspace_bytes(d.O, d.I, d.cols, 0), in);
-  const int st = flb200_linear_bias_act_forward(
-      d.O, d.I, d.cols, P(w), P(in), Pf(bias), P(y), gelu ? P(pre) : nullptr,
+  const int st = unlocked(
+      flb200_linear_bias_act_forward, d.O, d.I, d.cols, P(w), P(in), Pf(bias), P(y), gelu ? P(pre) : nullptr,
       gelu ? FLB200_ACT_GELU : FLB200_ACT_NONE, code_of(in), mode, ws.p(), ws.bytes, stream());
   if (st == FLB200_UNSUPPORTED) Py_RETURN_NONE;
   check(st);
@@ -406,17 +419,19 @@ NATIVE(linear_backward) {  // (x, weight, grad_y, has_bias, need_x, need_w, mode
     if (gy.numel() != d.cols * d.O) value_error("channel_sum: geometry does not match the tensor");
     gb = floats(d.O, gy);
     Workspace ws(flb200_channel_sum_workspace_bytes(d.cols, d.O, 1), in);
-    check(flb200_channel_sum(P(gy), Pf(&gb), d.cols, d.O, 1, code_of(gy), ws.p(), ws.bytes, stream()));
+    check(unlocked(flb200_channel_sum, P(gy), Pf(&gb), d.cols, d.O, 1, code_of(gy), ws.p(), ws.bytes, stream()));
   }
   if (x.b(4)) {
     gx = empty_like(in);
     Workspace ws(flb200_linear_workspace_bytes(d.O, d.I, d.cols, 1), in);
-    check(flb200_linear_backward_input(d.O, d.I, d.cols, P(w), P(gy), P(gx), mode, ws.p(), ws.bytes, stream()));
+    check(unlocked(flb200_linear_backward_input, d.O, d.I, d.cols, P(w), P(gy), P(gx), mode, ws.p(), ws.bytes,
+                   stream()));
   }
   if (x.b(5)) {
     gw = empty_like(w);
     Workspace ws(flb200_linear_workspace_bytes(d.O, d.I, d.cols, 2), in);
-    check(flb200_linear_backward_weight(d.O, d.I, d.cols, P(gy), P(in), P(gw), mode, ws.p(), ws.bytes, stream()));
+    check(unlocked(flb200_linear_backward_weight, d.O, d.I, d.cols, P(gy), P(in), P(gw), mode, ws.p(), ws.bytes,
+                   stream()));
   }
   return wrap({gx, gw, gb});
 }
@@ -445,8 +460,8 @@ NATIVE(matmul) {
   d.alpha = (float)x.d(16); d.beta = (float)x.d(17);
   d.dtype = code_of(a); d.math_mode = x.n32(18);
   Workspace ws(flb200_matmul_workspace_bytes(&d), a);
-  check(wide ? flb200_matmul_wide(&d, P(a), P(b), Pf(&c), ws.p(), ws.bytes, stream())
-             : flb200_matmul(&d, P(a), P(b), P(c), ws.p(), ws.bytes, stream()));
+  check(wide ? unlocked(flb200_matmul_wide, &d, P(a), P(b), Pf(&c), ws.p(), ws.bytes, stream())
+             : unlocked(flb200_matmul, &d, P(a), P(b), P(c), ws.p(), ws.bytes, stream()));
   return wrap(c);
 }
 
@@ -460,7 +475,7 @@ NATIVE(log_softmax) {  // (x)
   int64_t C, X;
   classes(in, &C, &X);
   Tensor y = empty_like(in);
-  check(flb200_log_softmax_forward(P(in), P(y), C, X, code_of(in), stream()));
+  check(unlocked(flb200_log_softmax_forward, P(in), P(y), C, X, code_of(in), stream()));
   return wrap(y);
 }
 NATIVE(log_softmax_backward) {  // (y, grad_y)
@@ -468,7 +483,7 @@ NATIVE(log_softmax_backward) {  // (y, grad_y)
   int64_t C, X;
   classes(y, &C, &X);
   Tensor gx = empty_like(y);
-  check(flb200_log_softmax_backward(P(y), P(x.tensor(1)), P(gx), C, X, code_of(y), stream()));
+  check(unlocked(flb200_log_softmax_backward, P(y), P(x.tensor(1)), P(gx), C, X, code_of(y), stream()));
   return wrap(gx);
 }
 NATIVE(cce_forward) {  // (logp, targets int32, reduction, ignore_index) -> (loss, meta)
@@ -480,16 +495,18 @@ NATIVE(cce_forward) {  // (logp, targets int32, reduction, ignore_index) -> (los
   Tensor meta = empty({2}, ScalarType::Int, logp);  // [count, bad-target flag]
   int32_t* m = static_cast<int32_t*>(meta.data_ptr());
   void* st = stream();
-  if (cudaMemsetAsync(m, 0, 8, static_cast<cudaStream_t>(st)) != cudaSuccess) check(FLB200_LAUNCH_FAILURE);
+  if (unlocked(cudaMemsetAsync, m, 0, (size_t)8,
+               static_cast<cudaStream_t>(st)) != cudaSuccess) check(FLB200_LAUNCH_FAILURE);
   Workspace ws(flb200_cce_workspace_bytes(X), logp);
-  check(flb200_cce_forward(P(logp), static_cast<const int32_t*>(P(tg)), Pf(&loss), m, m + 1, C, X, red, x.n32(3),
+  check(unlocked(flb200_cce_forward, P(logp), static_cast<const int32_t*>(P(tg)), Pf(&loss), m, m + 1, C, X, red,
+                 x.n32(3),
                            code_of(logp), ws.p(), ws.bytes, st));
   return wrap({loss, meta});
 }
 NATIVE(cce_backward) {  // (grad_loss, targets, meta, C, reduction, ignore_index, like)
   const Tensor &tg = x.tensor(1), &meta = x.tensor(2), &like = x.tensor(6);
   Tensor gx = empty_like(like);
-  check(flb200_cce_backward(Pf(x.t(0)), static_cast<const int32_t*>(P(tg)),
+  check(unlocked(flb200_cce_backward, Pf(x.t(0)), static_cast<const int32_t*>(P(tg)),
                             static_cast<const int32_t*>(P(meta)), P(gx), x.i(3), tg.numel(), x.n32(4), x.n32(5),
                             code_of(like), stream()));
   return wrap(gx);
@@ -499,7 +516,7 @@ NATIVE(log_softmax_cce_backward) {  // (y, grad_loss, targets, meta, reduction, 
   int64_t C, X;
   classes(y, &C, &X);
   Tensor gx = empty_like(y);
-  check(flb200_log_softmax_cce_backward(P(y), Pf(x.t(1)), static_cast<const int32_t*>(P(tg)),
+  check(unlocked(flb200_log_softmax_cce_backward, P(y), Pf(x.t(1)), static_cast<const int32_t*>(P(tg)),
                                         static_cast<const int32_t*>(P(meta)), P(gx), C, X, x.n32(4), x.n32(5),
                                         code_of(y), stream()));
   return wrap(gx);
@@ -511,11 +528,11 @@ NATIVE(softmax) {  // (x, scale, causal_period, with_lse) -> y or (y, lse)
   const float scale = (float)x.d(1);
   Tensor y = empty_like(in);
   if (!x.b(3)) {
-    check(flb200_softmax_forward(P(in), P(y), C, X, scale, x.i(2), code_of(in), stream()));
+    check(unlocked(flb200_softmax_forward, P(in), P(y), C, X, scale, x.i(2), code_of(in), stream()));
     return wrap(y);
   }
   Tensor lse = floats(X, in);
-  check(flb200_softmax_forward_lse(P(in), P(y), Pf(&lse), C, X, scale, x.i(2), code_of(in), stream()));
+  check(unlocked(flb200_softmax_forward_lse, P(in), P(y), Pf(&lse), C, X, scale, x.i(2), code_of(in), stream()));
   return wrap({y, lse});
 }
 NATIVE(softmax_backward) {  // (y, grad_y, scale)
@@ -523,7 +540,7 @@ NATIVE(softmax_backward) {  // (y, grad_y, scale)
   int64_t C, X;
   classes(y, &C, &X);
   Tensor gx = empty_like(y);
-  check(flb200_softmax_backward(P(y), P(x.tensor(1)), P(gx), C, X, (float)x.d(2), code_of(y), stream()));
+  check(unlocked(flb200_softmax_backward, P(y), P(x.tensor(1)), P(gx), C, X, (float)x.d(2), code_of(y), stream()));
   return wrap(gx);
 }
 NATIVE(attention_backward) {  // (q, k, v, o, grad_o, lse, scale, causal) -> (dq, dk, dv)
@@ -537,7 +554,8 @@ NATIVE(attention_backward) {  // (q, k, v, o, grad_o, lse, scale, causal) -> (dq
   const Tensor all = empty({3, Z, T, hd}, q.scalar_type(), q);  // one after another (autograd.unbind)
   const Tensor dq = all.select(0, 0), dk = all.select(0, 1), dv = all.select(0, 2);
   Workspace ws(flb200_attention_backward_workspace_bytes(Z, T, hd), q);
-  check(flb200_attention_backward(P(q), P(x.t(1)), P(x.t(2)), P(x.t(3)), P(x.t(4)), Pf(x.t(5)), P(dq), P(dk), P(dv),
+  check(unlocked(flb200_attention_backward, P(q), P(x.t(1)), P(x.t(2)), P(x.t(3)), P(x.t(4)), Pf(x.t(5)), P(dq),
+                 P(dk), P(dv),
                                   Z, T, hd, (float)x.d(6), x.b(7) ? 1 : 0, code_of(q), ws.p(), ws.bytes, stream()));
   return wrap({dq, dk, dv});
 }
@@ -554,7 +572,7 @@ NATIVE(attention_packed) {
   if (!flb200_attention_packed_supported(T, hd, code_of(qkv)) || (reinterpret_cast<uintptr_t>(P(qkv)) & 15))
     Py_RETURN_NONE;
   Tensor out = empty({B * T, h * hd}, qkv.scalar_type(), qkv), lse = floats(B * h * T, qkv);
-  check(flb200_attention_packed_forward(P(qkv), P(out), Pf(&lse), B, h, T, hd, (float)x.d(4), x.b(5) ? 1 : 0,
+  check(unlocked(flb200_attention_packed_forward, P(qkv), P(out), Pf(&lse), B, h, T, hd, (float)x.d(4), x.b(5) ? 1 : 0,
                                         code_of(qkv), stream()));
   return wrap({out, lse});
 }
@@ -565,7 +583,7 @@ NATIVE(attention_packed_backward) {  // (qkv, out, grad_out contiguous, lse, B, 
     value_error("attention_packed_backward: grad_out must be dense and like out");
   Tensor g = empty_like(qkv);
   Workspace ws(flb200_attention_backward_workspace_bytes(B * h, T, hd), qkv);
-  check(flb200_attention_packed_backward(P(qkv), P(out), P(gy), Pf(x.t(3)), P(g), B, h, T, hd, (float)x.d(7),
+  check(unlocked(flb200_attention_packed_backward, P(qkv), P(out), P(gy), Pf(x.t(3)), P(g), B, h, T, hd, (float)x.d(7),
                                          x.b(8) ? 1 : 0, code_of(qkv), ws.p(), ws.bytes, stream()));
   return wrap(g);
 }
@@ -581,7 +599,7 @@ NATIVE(embedding) {  // (table, ids contiguous)
   const int code = id_code(ids);
   const int64_t vocab = table.size(0), dim = table.size(1), rows = ids.numel();
   Tensor out = empty({rows, dim}, table.scalar_type(), table);
-  check(flb200_embedding_forward(P(table), P(ids), code, P(out), rows, dim, vocab, code_of(table), stream()));
+  check(unlocked(flb200_embedding_forward, P(table), P(ids), code, P(out), rows, dim, vocab, code_of(table), stream()));
   return wrap(out);
 }
 NATIVE(embedding_backward) {  // (grad_out contiguous, ids contiguous, vocab)
@@ -589,7 +607,8 @@ NATIVE(embedding_backward) {  // (grad_out contiguous, ids contiguous, vocab)
   const int code = id_code(ids);
   const int64_t vocab = x.i(2), dim = g.size(-1);
   Tensor out = empty({vocab, dim}, ScalarType::Float, g);
-  check(flb200_embedding_backward(P(g), P(ids), code, Pf(&out), ids.numel(), dim, vocab, code_of(g), stream()));
+  check(unlocked(flb200_embedding_backward, P(g), P(ids), code, Pf(&out), ids.numel(), dim, vocab, code_of(g),
+                 stream()));
   return wrap(out);
 }
 
@@ -661,10 +680,11 @@ NATIVE(conv2d) {
   }
   if (sbytes) {
     stats = floats((int64_t)(sbytes / 4), in);
-    check(flb200_conv2d_forward_stats(&d, P(in), P(w), P(bias), P(out), Pf(&stats), sbytes, ws.p(), ws.bytes, cache,
+    check(unlocked(flb200_conv2d_forward_stats, &d, P(in), P(w), P(bias), P(out), Pf(&stats), sbytes, ws.p(),
+                   ws.bytes, cache,
                                       stream()));
   } else {
-    check(flb200_conv2d_forward_cached(&d, P(in), P(w), P(bias), P(out), ws.p(), ws.bytes, cache, stream()));
+    check(unlocked(flb200_conv2d_forward_cached, &d, P(in), P(w), P(bias), P(out), ws.p(), ws.bytes, cache, stream()));
   }
   PyObject* r = PyTuple_New(3);
   PyTuple_SET_ITEM(r, 0, wrap(out));
@@ -678,7 +698,8 @@ NATIVE(conv2d_backward_data) {
   const flb200_conv2d_desc d = conv_desc(in, w, x, 3, channels_last(gy) || channels_last(in), x.n32(10));
   Tensor gx = empty_like(in);
   Workspace ws(flb200_conv2d_workspace_bytes(&d, 1), in);
-  check(flb200_conv2d_backward_data_cached(&d, P(gy), P(w), P(gx), ws.p(), ws.bytes, cache_of(x.at(11)), stream()));
+  check(unlocked(flb200_conv2d_backward_data_cached, &d, P(gy), P(w), P(gx), ws.p(), ws.bytes, cache_of(x.at(11)),
+                 stream()));
   return wrap(gx);
 }
 // (grad_y, input, weights, bias or None, sx sy px py dx dy groups, mode, cache) -> (grad_w, grad_b)
@@ -689,7 +710,8 @@ NATIVE(conv2d_backward_filter_bias) {
   Tensor gw = empty_like(w), gb;
   if (bias) gb = empty_like(*bias);
   Workspace ws(flb200_conv2d_workspace_bytes(&d, 2), in);
-  check(flb200_conv2d_backward_filter_bias_cached(&d, P(gy), P(in), P(gw), bias ? P(gb) : nullptr, ws.p(), ws.bytes,
+  check(unlocked(flb200_conv2d_backward_filter_bias_cached, &d, P(gy), P(in), P(gw), bias ? P(gb) : nullptr, ws.p(),
+                 ws.bytes,
                                                   cache_of(x.at(12)), stream()));
   return wrap({gw, gb});
 }
@@ -713,7 +735,8 @@ NATIVE(pool2d) {  // (input, wx wy sx sy px py mode, want_argmax) -> (y, argmax 
   const bool cl = d.layout == FLB200_LAYOUT_NHWC;
   Tensor out = empty({d.N, d.C, ho, wo}, in.scalar_type(), in, cl), arg;
   if (x.b(8) && d.mode == FLB200_POOL_MAX) arg = empty({d.N, d.C, ho, wo}, ScalarType::Byte, in, cl);
-  check(flb200_pool2d_forward(&d, P(in), P(out), arg.defined() ? static_cast<uint8_t*>(arg.data_ptr()) : nullptr,
+  check(unlocked(flb200_pool2d_forward, &d, P(in), P(out),
+                 arg.defined() ? static_cast<uint8_t*>(arg.data_ptr()) : nullptr,
                               stream()));
   return wrap({out, arg});
 }
@@ -721,7 +744,7 @@ NATIVE(pool2d_backward) {  // (grad_y, input, argmax or None, wx wy sx sy px py 
   const Tensor &gy = x.tensor(0), &in = x.tensor(1);
   const flb200_pool2d_desc d = pool_desc(in, x, 3);
   Tensor gx = empty_like(in);
-  check(flb200_pool2d_backward(&d, P(gy), P(in), static_cast<const uint8_t*>(P(x.t(2))), P(gx), stream()));
+  check(unlocked(flb200_pool2d_backward, &d, P(gy), P(in), static_cast<const uint8_t*>(P(x.t(2))), P(gx), stream()));
   return wrap(gx);
 }
 
@@ -777,12 +800,13 @@ NATIVE(batchnorm) {
   if (stats && train) {  // statistics from what the producing convolution took: no pass over x for them
     const int64_t groups = x.i(11);
     Workspace ws(flb200_batchnorm_from_stats_workspace_bytes(&d, groups), in);
-    check(flb200_batchnorm_forward_from_stats(&d, P(in), nullptr, relu ? 1 : 0, Pf(stats), groups, w, b, rm, rv, pm, pv,
+    check(unlocked(flb200_batchnorm_forward_from_stats, &d, P(in), nullptr, relu ? 1 : 0, Pf(stats), groups, w, b,
+                   rm, rv, pm, pv,
                                               mom, eps, P(out), nullptr, ws.p(), ws.bytes, stream()));
   } else {
     Workspace ws(flb200_batchnorm_workspace_bytes(&d), in);
-    check((relu ? flb200_batchnorm_relu_forward : flb200_batchnorm_forward)(
-        &d, P(in), w, b, rm, rv, pm, pv, train ? 1 : 0, mom, eps, P(out), ws.p(), ws.bytes, stream()));
+    check(unlocked(
+        relu ? flb200_batchnorm_relu_forward : flb200_batchnorm_forward, &d, P(in), w, b, rm, rv, pm, pv, train ? 1 : 0, mom, eps, P(out), ws.p(), ws.bytes, stream()));
   }
   return wrap({out, sm, sv});
 }
@@ -812,11 +836,13 @@ NATIVE(batchnorm_add_relu) {
   if (stats && train) {
     const int64_t groups = x.i(11);
     Workspace ws(flb200_batchnorm_from_stats_workspace_bytes(&d, groups), in);
-    check(flb200_batchnorm_forward_from_stats(&d, P(in), P(add), 1, Pf(stats), groups, w, b, rm, rv, pm, pv, mom, eps,
+    check(unlocked(flb200_batchnorm_forward_from_stats, &d, P(in), P(add), 1, Pf(stats), groups, w, b, rm, rv, pm,
+                   pv, mom, eps,
                                               P(out), m, ws.p(), ws.bytes, stream()));
   } else {
     Workspace ws(flb200_batchnorm_workspace_bytes(&d), in);
-    check(flb200_batchnorm_add_relu_forward(&d, P(in), P(add), w, b, rm, rv, pm, pv, train ? 1 : 0, mom, eps, P(out), m,
+    check(unlocked(flb200_batchnorm_add_relu_forward, &d, P(in), P(add), w, b, rm, rv, pm, pv, train ? 1 : 0, mom,
+                   eps, P(out), m,
                                             ws.p(), ws.bytes, stream()));
   }
   return wrap({out, mask, sm, sv});
@@ -829,10 +855,12 @@ NATIVE(batchnorm_backward) {
   Tensor gx = empty_like(in), gw = floats(d.channels, in), gb = floats(d.channels, in);
   Workspace ws(flb200_batchnorm_workspace_bytes(&d), in);
   if (x.b(7))
-    check(flb200_batchnorm_relu_backward(&d, P(gy), P(in), w, Pf(x.t(5)), sm, sv, P(gx), Pf(&gw), Pf(&gb), ws.p(),
+    check(unlocked(flb200_batchnorm_relu_backward, &d, P(gy), P(in), w, Pf(x.t(5)), sm, sv, P(gx), Pf(&gw), Pf(&gb),
+                   ws.p(),
                                          ws.bytes, stream()));
   else
-    check(flb200_batchnorm_backward(&d, P(gy), P(in), w, sm, sv, P(gx), Pf(&gw), Pf(&gb), ws.p(), ws.bytes, stream()));
+    check(unlocked(flb200_batchnorm_backward, &d, P(gy), P(in), w, sm, sv, P(gx), Pf(&gw), Pf(&gb), ws.p(), ws.bytes,
+                   stream()));
   return wrap({gx, gw, gb});
 }
 // (mask, grad_a, grad_b or None, save_mean, save_invstd, input, weight, axes)
@@ -842,7 +870,8 @@ NATIVE(batchnorm_add_relu_backward) {
   const flb200_batchnorm_desc d = bn_desc(in, x.at(7));
   Tensor gs = empty_like(in), gx = empty_like(in), gw = floats(d.channels, in), gb = floats(d.channels, in);
   Workspace ws(flb200_batchnorm_workspace_bytes(&d), in);
-  check(flb200_batchnorm_add_relu_backward(&d, static_cast<const uint8_t*>(P(x.t(0))), P(x.t(1)), P(x.t(2)), P(in),
+  check(unlocked(flb200_batchnorm_add_relu_backward, &d, static_cast<const uint8_t*>(P(x.t(0))), P(x.t(1)),
+                 P(x.t(2)), P(in),
                                            Pf(x.t(6)), Pf(x.t(3)), Pf(x.t(4)), P(gs), P(gx), Pf(&gw), Pf(&gb), ws.p(),
                                            ws.bytes, stream()));
   return wrap({gs, gx, gw, gb});
