@@ -345,8 +345,15 @@ rnn_sequence_kernel(const __grid_constant__ Launch<SeqJob> a) {
         (uint32_t)owner);
     const uint32_t push_bar = mapa_u32(smem_u32(recv_bar), (uint32_t)owner);
     const uint32_t recv_bytes = (uint32_t)(kUnits * G * quads * 16);
+    // A warp that loads no tile, pushes no row and updates no pair takes no part: nobody waits for it,
+    // so it could fall two phases behind a barrier that it only follows, and miss one.
+    const bool pushes = (warp & 3) < G && (warp >> 2) * (kHalf / 4) < quads;
+    bool updates = false;
+#pragma unroll
+    for (int it = 0; it < kItems; ++it) updates = updates || live[it];
+    const bool role = warp < stages || pushes || __any_sync(0xffffffffu, updates);
 
-    for (int step = 0; step < a.T && waits.warp_goes_on(); ++step) {
+    for (int step = 0; role && step < a.T && waits.warp_goes_on(); ++step) {
       const int t = job.reverse ? a.T - 1 - step : step;
       const int slot = step & 1;
       float* g_t = job.gates + (long long)t * a.B_total * G * H + group * kUnits + rank * kOwn;
@@ -381,7 +388,7 @@ rnn_sequence_kernel(const __grid_constant__ Launch<SeqJob> a) {
         if (lane == 0) issue_tile<false, NB>(tmem_base, a_desc0, b_desc0, warp, done_bar);
         __syncwarp();
       }
-      if ((warp & 3) < G && waits.warp_bar<false>(done_bar, step & 1)) {
+      if (pushes && waits.warp_bar<false>(done_bar, step & 1)) {
         tc_fence_after();
         const uint32_t at = push_at + (uint32_t)(slot * Recv<G, NB>::kFloats * 4);
         const uint32_t bar = push_bar + (uint32_t)(slot * 8);
@@ -580,7 +587,13 @@ rnn_sequence_backward_kernel(const __grid_constant__ Launch<SeqBwdJob> a) {
     unsigned long long* push = a.part[ji] + tile_at + ((long long)(row / units) * SL + rank) * block + 2 * (row % units);
     const unsigned long long* pull = a.part[ji] + tile_at + (long long)rank * SL * block;
 
-    for (int sb = 0; sb < a.T && waits.warp_goes_on(); ++sb) {
+    // (a warp with no part in the steps stays out of them, as in the forward kernel)
+    bool updates = false;
+#pragma unroll
+    for (int it = 0; it < kItems; ++it) updates = updates || live[it];
+    const bool role = warp < stages || warp_live || __any_sync(0xffffffffu, updates);
+
+    for (int sb = 0; role && sb < a.T && waits.warp_goes_on(); ++sb) {
       const int step = a.T - 1 - sb;
       const int t = job.reverse ? a.T - 1 - step : step;
       const int slot = sb & 1;
