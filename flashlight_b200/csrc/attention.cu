@@ -301,13 +301,15 @@ attention_backward_kernel(const __grid_constant__ CUtensorMap map_q,
 #pragma unroll 1
     for (int c0 = 0; c0 < 64; c0 += 32) {
       float v[32];
+      __syncwarp();  // the lanes past the end store nothing, and are back for the next load
       tmem_ld32(lane_addr + (uint32_t)c0, v);
-      if (key >= a.T) continue;
+      if (key < a.T) {
 #pragma unroll
-      for (int u = 0; u < 4; ++u)
-        *reinterpret_cast<uint4*>(out + c0 + 8 * u) =
-            make_uint4(pack_bf16(v[8 * u], v[8 * u + 1]), pack_bf16(v[8 * u + 2], v[8 * u + 3]),
-                       pack_bf16(v[8 * u + 4], v[8 * u + 5]), pack_bf16(v[8 * u + 6], v[8 * u + 7]));
+        for (int u = 0; u < 4; ++u)
+          *reinterpret_cast<uint4*>(out + c0 + 8 * u) =
+              make_uint4(pack_bf16(v[8 * u], v[8 * u + 1]), pack_bf16(v[8 * u + 2], v[8 * u + 3]),
+                         pack_bf16(v[8 * u + 4], v[8 * u + 5]), pack_bf16(v[8 * u + 6], v[8 * u + 7]));
+      }
     }
   }
   tc_fence_before();
