@@ -32,6 +32,7 @@
 #include <cuda_runtime.h>
 
 #include <algorithm>
+#include <cfloat>
 #include <mutex>
 #include <set>
 #include <utility>
@@ -456,7 +457,9 @@ attention_forward_kernel(const __grid_constant__ CUtensorMap map_q,
     wait(bar_q, 0, 1);
     scores(0);
   }
-  float m = -INFINITY, sum = 0.f, o[32];
+  // the running maximum starts at the lowest finite value: keys whose scores are all -inf then count
+  // as zeros, where -inf - (-inf) would leave NaN to every later block of the row
+  float m = -FLT_MAX, sum = 0.f, o[32];
 #pragma unroll
   for (int e = 0; e < 32; ++e) o[e] = 0.f;
   const uint32_t lane_addr = tmem + ((uint32_t)((warp & 3) * 32) << 16);

@@ -32,6 +32,27 @@ def test_attention_packed(shape, causal):
     assert_close_scaled(g.float(), ref.grad, 1.6e-2, "attention gradient")
 
 
+@pytest.mark.parametrize("causal", [True, False])
+def test_attention_packed_infinite_scores(causal):
+    """Keys of score -inf weigh nothing, even where they fill the first blocks of a row; rows that see
+    no other keys are NaN, as softmax makes them."""
+    from flashlight_b200 import functions as F
+    B, T, h, lead = 1, 400, 2, 260
+    qkv = randn(B * T, 3, h, 64, seed=3).bfloat16()
+    qkv[:, 0, :, 0] = 1.0
+    qkv[:lead, 1, :, 0] = float("-inf")
+    out, lse = F.attention_packed(qkv.reshape(B * T, 3 * h * 64).cuda(), B, T, h, 0.125, causal)
+    q, k, v = qkv.double().reshape(B, T, 3, h, 64).permute(2, 0, 3, 1, 4)
+    s = 0.125 * q @ k.transpose(-1, -2)
+    if causal:
+        s = s.masked_fill(torch.ones(T, T).triu(1).bool(), float("-inf"))
+    want = (torch.softmax(s, -1) @ v).permute(0, 2, 1, 3).reshape(B * T, h * 64)
+    first = lead if causal else 0
+    assert out[:first].isnan().all()
+    assert_close_scaled(out[first:].float(), want[first:], 1.2e-2, "attention output")
+    assert_close_scaled(lse.reshape(B, h, T)[:, :, first:], torch.logsumexp(s, -1)[:, :, first:], 1e-3, "attention lse")
+
+
 def test_attention_packed_declines_what_it_is_not_built_for():
     from flashlight_b200 import functions as F
     assert F.attention_packed(randn(8, 96, seed=1).bfloat16().cuda(), 1, 8, 1, 1.0, True) is None
