@@ -103,6 +103,8 @@ class Variable:
             self._grad, self._grad_owned = g, False
             return
         if g.dtype != self._grad.dtype:  # a wide contribution (grad_dtype) and a plain one
+            if {g.dtype, self._grad.dtype} != {self.tensor.dtype, torch.float32}:
+                raise ValueError("addGrad: gradients of different types")
             total = self.grad.to(torch.float32)
             self._grad, self._grad_owned = F.add(total, g.to(torch.float32)), True
         elif self._grad_second is None and self.grad_func2 is not None:
