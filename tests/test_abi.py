@@ -172,16 +172,3 @@ def test_unbind_returns_one_gradient_for_all_parts():
         for i in range(3):
             want[:, :, i] = float(i + 1)
         assert torch.equal(x.grad, want.reshape(B * T, 3 * d))
-
-
-def test_add_grad_refuses_gradients_of_unrelated_types():
-    """Two types meet in one gradient only where one is the tensor's and the other fp32."""
-    import torch
-    from flashlight_b200.autograd import Variable
-    for own, first, second in ((torch.bfloat16, torch.bfloat16, torch.float16),
-                               (torch.float16, torch.float32, torch.bfloat16),
-                               (torch.float32, torch.float32, torch.bfloat16)):
-        v = Variable(torch.zeros(4, dtype=own), True)
-        v.addGrad(torch.ones(4, dtype=first))
-        with pytest.raises(ValueError):
-            v.addGrad(torch.ones(4, dtype=second))

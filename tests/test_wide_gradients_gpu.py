@@ -38,3 +38,15 @@ def test_wide_and_plain_contributions_add_up():
     w.addGrad(a)
     w.addGrad(b)
     assert torch.equal(w.grad, a + b.float())
+
+
+def test_add_grad_refuses_gradients_of_unrelated_types():
+    """Two types meet in one gradient only where one is the tensor's and the other fp32."""
+    from flashlight_b200.autograd import Variable
+    for own, first, second in ((torch.bfloat16, torch.bfloat16, torch.float16),
+                               (torch.float16, torch.float32, torch.bfloat16),
+                               (torch.float32, torch.float32, torch.bfloat16)):
+        v = Variable(torch.zeros(4, dtype=own, device="cuda"), True)
+        v.addGrad(torch.ones(4, dtype=first, device="cuda"))
+        with pytest.raises(ValueError):
+            v.addGrad(torch.ones(4, dtype=second, device="cuda"))
