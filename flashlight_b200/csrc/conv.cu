@@ -378,11 +378,24 @@ int strict_image_pass(const char* name, const ConvGeo& g0, const float* src, con
   return launch_simt_gemm(name, ie, f, ep, M, N, K, g.groups, at, ws_bytes, st);
 }
 
+// (beta: what of gw's own values stays)
 int strict_filter_pass(const char* name, const ConvGeo& g0, const float* gy, const float* x, float* gw,
-                       void* ws, size_t ws_bytes, cudaStream_t st) {
+                       void* ws, size_t ws_bytes, cudaStream_t st, float beta = 0.f) {
   ConvGeo g = g0;
   const long long N = (long long)g.Cg * g.RS, K = (long long)g.N * g.HoWo;
-  FLB200_REQUIRE(N < 0x7fffffffLL && K < 0x7fffff00LL, "%s: extent out of range", name);
+  FLB200_REQUIRE(N < 0x7fffffffLL, "%s: extent out of range", name);
+  constexpr long long kMostK = 1LL << 30;  // the kernel counts k in 32 bits: more pixels in pieces
+  if (K > kMostK && g.N > 1) {
+    const int most = (int)std::max(1LL, kMostK / g.HoWo);
+    for (int n = 0; n < g0.N; n += most) {
+      g.N = std::min(most, g0.N - n);
+      if (int rc = strict_filter_pass(name, g, gy + (long long)n * g.Cout * g.HoWo, x + (long long)n * g.C * g.HW,
+                                      gw, ws, ws_bytes, st, n ? 1.f : 0.f))
+        return rc;
+    }
+    return FLB200_OK;
+  }
+  FLB200_REQUIRE(K < 0x7fffff00LL, "%s: extent out of range", name);
   const StrictScratch need = strict_scratch(g, 2);
   char* at = static_cast<char*>(ws);
   if (ws && aligned16(ws) && ws_bytes >= need.x + need.gy) {
@@ -400,7 +413,7 @@ int strict_filter_pass(const char* name, const ConvGeo& g0, const float* gy, con
     }
     ws_bytes -= need.x + need.gy;
   }
-  FilterOut ep{gw, nullptr, 1.f, 0.f, 0, 0, g, 0};
+  FilterOut ep{gw, nullptr, 1.f, beta, 0, 0, g, 0};
   if (g.x_cl && g.y_cl && g.Cg % 4 == 0 && g.Coutg % 4 == 0 && aligned16(x) && aligned16(gy)) {
     const StridedLoader<kVecRow> gl{gy, 1, g.Cout, g.Coutg, g.Coutg};
     ep.tap_major = 1;

@@ -39,6 +39,18 @@ int matmul_simt_b(int bkind, const flb200_matmul_desc* d, const float* a, const 
 
 int matmul_simt(const flb200_matmul_desc* d, const void* a, const void* b, void* c, void* ws,
                 size_t ws_bytes, cudaStream_t st) {
+  constexpr long long kMostK = 1LL << 30;  // the kernel counts k in 32 bits: longer sums in pieces
+  if (d->k > kMostK) {
+    flb200_matmul_desc part = *d;
+    for (long long k0 = 0; k0 < d->k; k0 += kMostK) {
+      part.k = d->k - k0 < kMostK ? d->k - k0 : kMostK;
+      if (int rc = matmul_simt(&part, static_cast<const float*>(a) + k0 * d->a_col,
+                               static_cast<const float*>(b) + k0 * d->b_row, c, ws, ws_bytes, st))
+        return rc;
+      part.beta = 1.f;
+    }
+    return FLB200_OK;
+  }
   StridedEpilogue ep{static_cast<float*>(c), nullptr, d->alpha, d->beta, 0, 0, d->c_row, d->c_col,
                      d->c_batch};
   ep.along_m = d->c_row == 1 && d->c_col != 1;

@@ -42,6 +42,27 @@ def test_matmul_strict_many_batches(zmnk):
     assert_close(c, a.double() @ b.double(), STRICT_TOL, f"batched matmul {zmnk}")
 
 
+def test_matmul_strict_k_past_32_bits():
+    """2^31 + 37 products of 2 and 0.5 (strides of 0 read one element of each): all partial sums are
+    whole numbers below 2^24 or sums of a few of them."""
+    from flashlight_b200 import _lib as L
+    from flashlight_b200 import functions as F
+    k = 2 ** 31 + 37
+    c = F.matmul(torch.full((4,), 2.0).cuda(), torch.full((4,), 0.5).cuda(), m=1, n=1, k=k, a_strides=(1, 0),
+                 b_strides=(0, 1), math_mode=L.MATH_STRICT_F32)
+    assert abs(float(c) / k - 1.0) <= 1e-6
+
+
+def test_conv_strict_filter_gradient_of_many_pixels():
+    """More output pixels than one sum takes: 1025 images of 2^20, every product 0.5."""
+    from flashlight_b200 import _lib as L
+    from flashlight_b200.extension import B200AutogradExtension
+    ext = B200AutogradExtension(math_mode=L.MATH_STRICT_F32)
+    x, gy = torch.ones(1025, 1, 1024, 1024, device="cuda"), torch.full((1025, 1, 1024, 1024), 0.5, device="cuda")
+    gw, _ = ext.conv2dBackwardFilterBias(gy, x, torch.ones(1, 1, 1, 1, device="cuda"), None, 1, 1, 0, 0, 1, 1, 1)
+    assert float(gw) == 1025 * 2.0 ** 19
+
+
 # N, C, H, W, Cout, kH, kW, stride, pad, groups: element loaders; repacked filter and channels-last
 # copy; channels not a multiple of 4; groups; a filter of many taps; stride with empty classes;
 # filters whose repacking needs more than the default shared memory, and more than there is; more
