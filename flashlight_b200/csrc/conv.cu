@@ -576,6 +576,7 @@ size_t flb200_conv2d_workspace_bytes(const flb200_conv2d_desc* d, int which) {
   if (native16(d, &g, which))  // + the fp32 bias or its gradient
     return up256c(max_sz(need, tc_conv_workspace_bytes(g, which))) + up256c((size_t)g.Cout * 4) +
            wide_copies(g, which).total;
+  tc::X3Scope x3(d->math_mode == FLB200_MATH_F32X3);  // plans differ by mode
   if (d->math_mode != FLB200_MATH_STRICT_F32) need = max_sz(need, tc_conv_workspace_bytes(g, which));
   if (d->dtype != FLB200_F32 && which >= 0 && which <= 2)
     need = up256c(need) + wide_copies(g, which).total;  // fp32 copies of the 16-bit tensors
@@ -652,6 +653,7 @@ size_t flb200_conv2d_stats_bytes(const flb200_conv2d_desc* d, int64_t* groups) {
   if (groups) *groups = 0;
   if (make_conv_geo("conv2d_stats_bytes", d, &g)) return 0;
   if (d->math_mode == FLB200_MATH_STRICT_F32 || (d->dtype != FLB200_F32 && !native16(d, &g, 0))) return 0;
+  tc::X3Scope x3(g.operand == tc::kOperandTf32 && d->math_mode == FLB200_MATH_F32X3);
   const long long n = tc_conv_stats_groups(g);
   if (n == 0 || !tc_conv_supported(g, 0, tc_conv_workspace_bytes(g, 0))) return 0;
   if (groups) *groups = n;

@@ -135,7 +135,11 @@ size_t flb200_linear_workspace_bytes(int64_t O, int64_t I, int64_t cols, int whi
   if (which == 0) { d.m = cols; d.n = O; d.k = I; }
   else if (which == 1) { d.m = cols; d.n = I; d.k = O; }
   else { d.m = I; d.n = O; d.k = cols; }
-  return flb200_matmul_workspace_bytes(&d);
+  d.math_mode = FLB200_MATH_TF32;  // (the call may come in either tensor-core mode)
+  const size_t tf32 = flb200_matmul_workspace_bytes(&d);
+  d.math_mode = FLB200_MATH_F32X3;
+  const size_t x3 = flb200_matmul_workspace_bytes(&d);
+  return tf32 > x3 ? tf32 : x3;
 }
 
 // fl layout (column-major): weight (o,i) at o + i*O; x (i,col) at i + col*I;

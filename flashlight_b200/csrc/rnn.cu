@@ -129,11 +129,8 @@ int project_input(int math_mode, const RnnDims& r, const float* in, long long In
   return flb200_channel_bias_add(gates, bias, gates, r.TB, r.GH, 1, FLB200_F32, stream);
 }
 
-size_t mm_ws(long long m, long long n, long long k) {
-  flb200_matmul_desc d = {};
-  d.m = m; d.n = n; d.k = k; d.batch = 1;
-  d.math_mode = FLB200_MATH_TF32;
-  return flb200_matmul_workspace_bytes(&d);
+size_t mm_ws(long long m, long long n, long long k) {  // in either tensor-core mode
+  return flb200_linear_workspace_bytes(n, k, m, 0);
 }
 
 __device__ __forceinline__ float sigmoidf_(float v) { return 1.f / (1.f + expf(-v)); }

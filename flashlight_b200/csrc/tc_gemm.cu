@@ -505,9 +505,10 @@ bool tc_gemm_supported(const flb200_matmul_desc* d, const void* a, const void* b
 size_t tc_gemm_workspace_bytes(const flb200_matmul_desc* d) {
   if (!d || d->m < 1 || d->n < 1 || d->k < 1) return 0;
   // What the call will want depends on things that this query does not know (operand alignment,
-  // and for the linear layers the type): the largest of the plans it may choose.
+  // and for the linear layers the type): the largest of the plans it may choose in this mode.
   size_t need = 0;
   for (int operand : {(int)tc::kOperandTf32, (int)tc::kOperandBf16}) {
+    tc::X3Scope x3(operand == tc::kOperandTf32 && d->math_mode == FLB200_MATH_F32X3);
     const long long k_iters = (d->k + tc::stage_k(operand) - 1) / tc::stage_k(operand);
     for (int mn = 0; mn < 2; ++mn)
       for (int swap = 0; swap < 2; ++swap) {

@@ -93,3 +93,23 @@ def test_resnet_step_f32x3(L):
         gg = p.grad.detach().cpu().double().reshape(wg.shape)
         err = float((gg - wg).abs().max()) / (float(wg.abs().max()) or 1.0)
         assert err <= 1e-3, f"parameter {i}: {err:.3e}"
+
+
+@pytest.mark.parametrize("case", [(1, 64, 16, 16, 128, 9, 4), (1, 128, 9, 9, 256, 9, 4)])
+def test_conv_takes_the_tensor_cores_with_the_workspace_it_asks_for(case):
+    """Long sums over few pixels, whose plans split K further in this mode than in TF32."""
+    from flashlight_b200 import _lib as L
+    from flashlight_b200.extension import B200AutogradExtension
+    N, C, H, W, Co, k, p = case
+    ext = B200AutogradExtension(math_mode=L.MATH_F32X3)
+    x, w = randn(N, C, H, W, seed=60), randn(Co, C, k, k, seed=61) / (C * k * k) ** 0.5
+    args = (1, 1, p, p, 1, 1, 1)
+    want = R.conv2d(x.double(), w.double(), None, *args)
+    gy = randn(*want.shape, seed=62)
+    before = L.lib.flb200_tc_kernel_launches()
+    y = ext.conv2d(x.cuda(), w.cuda(), None, *args)
+    forward = L.lib.flb200_tc_kernel_launches()
+    gx = ext.conv2dBackwardData(gy.cuda(), x.cuda(), w.cuda(), *args)
+    assert forward > before and L.lib.flb200_tc_kernel_launches() > forward
+    assert_close(y, want, F32X3_TOL, "conv forward")
+    assert_close(gx, R.conv2d_backward_data(gy.double(), x.shape, w.double(), *args), F32X3_TOL, "conv dx")
