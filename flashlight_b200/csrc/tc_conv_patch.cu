@@ -285,8 +285,8 @@ int nhwc_map(CUtensorMap* m, const float* base, int operand, int C, int cp, int 
 // The same tensor with the channel index split into (one 128-byte run of channels, group):
 // [32 or 64, w, h, n, groups].  One box of nbox groups lands in shared memory as nbox
 // consecutive [pixels][channels of a group] blocks, the layout of an MN-major operand.  Channels
-// past C of the last group read the neighbouring pixel (or the bytes after the tensor, which the
-// callers keep inside their workspace); such rows / columns of the product are never stored.
+// past C of the last group read the neighbouring pixel, or up to 112 bytes after the tensor; such
+// rows / columns of the product are never stored.
 int nhwc_map5(CUtensorMap* m, const float* base, int operand, int C, int cp, int W, int H, int N,
               int box_w, int box_h, int nbox, int sx, int sy) {
   const uint64_t es_ = operand ? 2 : 4, run = (uint64_t)tc::stage_k(operand);
@@ -297,6 +297,27 @@ int nhwc_map5(CUtensorMap* m, const float* base, int operand, int C, int cp, int
   const uint32_t es[5] = {1, (uint32_t)sx, (uint32_t)sy, 1, 1};
   return tc::make_tensor_map(m, base, 5, dims, strides, box,
                              operand ? tc::kMapKMajor : tc::kMapMnMajor, es, operand);
+}
+
+// Whether such a map reads past the end of the tensor.
+bool reads_past_end(const ConvGeo& g, int C) {
+  const int run = tc::stage_k(g.operand);
+  return C > run && C % run != 0;
+}
+// The map of dy or x for the backward-filter pass.  A copy in scratch has room behind it; of the
+// caller's own tensor nothing may be read past its end (the memory after it need not be mapped), so
+// one that is no whole number of groups is mapped with its channels as they are, and *each says that
+// every box is a copy of its own.
+int nhwc_operand(CUtensorMap* m, int* each, const ConvGeo& g, const float* base, bool own, int C, int cp,
+                 int W, int H, int box_w, int box_h, int nbox, int sx, int sy) {
+  *each = own && reads_past_end(g, C) ? 1 : 0;
+  if (!*each) return nhwc_map5(m, base, g.operand, C, cp, W, H, g.N, box_w, box_h, nbox, sx, sy);
+  return nhwc_map(m, base, g.operand, C, cp, W, H, g.N, box_w, box_h, 1, sx, sy,
+                  g.operand ? tc::kMapKMajor : tc::kMapMnMajor);
+}
+// Bytes of a cached copy [pixels][cp] of C channels, room for what nhwc_map5 reads behind it included.
+size_t copy_bytes(const ConvGeo& g, long long pixels, int C, int cp) {
+  return (size_t)pixels * cp * 4 + (reads_past_end(g, C) ? 128 : 0);
 }
 
 // Packed filter map [k, rows, taps].
@@ -440,8 +461,8 @@ inline int wgrad_a_boxes(const ConvGeo& g) {
 struct WgradTaps { int C, ntaps, kW, dil_x, dil_y, pad_x, pad_y; };
 
 template <int BN>
-int run_wgrad(const CUtensorMap& ma, const CUtensorMap& mb, const ConvGeo& g, const WgradTaps& tp,
-              const WgradPlan& w, float* partial, cudaStream_t st) {
+int run_wgrad(const CUtensorMap& ma, const CUtensorMap& mb, int a_each, int b_each, const ConvGeo& g,
+              const WgradTaps& tp, const WgradPlan& w, float* partial, cudaStream_t st) {
   tc::PatchWgradProblem<BN> p;
   p.a_mn_major = 1; p.b_mn_major = 1;
   p.operand = g.operand;
@@ -452,6 +473,7 @@ int run_wgrad(const CUtensorMap& ma, const CUtensorMap& mb, const ConvGeo& g, co
   p.tiles_n = w.tiles_n;
   p.ntaps = tp.ntaps; p.tap_groups = w.tap_groups; p.tg = w.tg; p.cn_shift = w.cn_shift;
   p.a_nbox = wgrad_a_boxes(g);
+  p.a_each = a_each; p.b_each = b_each;
   p.splits = w.splits; p.iters_per_split = w.ips; p.k_iters = w.k_iters;
   p.b_w_mul = g.sx; p.b_h_mul = g.sy;
   p.kW = tp.kW; p.dil_x = tp.dil_x; p.dil_y = tp.dil_y; p.pad_x = tp.pad_x; p.pad_y = tp.pad_y;
@@ -460,12 +482,12 @@ int run_wgrad(const CUtensorMap& ma, const CUtensorMap& mb, const ConvGeo& g, co
   return tc::launch_problem<tc::PatchWgradProblem<BN>, BN>("tc_patch_wgrad", ma, mb, p, tiles,
                                                           st);
 }
-int run_wgrad_any(const CUtensorMap& ma, const CUtensorMap& mb, const ConvGeo& g,
+int run_wgrad_any(const CUtensorMap& ma, const CUtensorMap& mb, int a_each, int b_each, const ConvGeo& g,
                   const WgradTaps& tp, const WgradPlan& w, float* partial, cudaStream_t st) {
-  if (w.bn == 32) return run_wgrad<32>(ma, mb, g, tp, w, partial, st);
-  if (w.bn == 64) return run_wgrad<64>(ma, mb, g, tp, w, partial, st);
-  if (w.bn == 128) return run_wgrad<128>(ma, mb, g, tp, w, partial, st);
-  return run_wgrad<256>(ma, mb, g, tp, w, partial, st);
+  if (w.bn == 32) return run_wgrad<32>(ma, mb, a_each, b_each, g, tp, w, partial, st);
+  if (w.bn == 64) return run_wgrad<64>(ma, mb, a_each, b_each, g, tp, w, partial, st);
+  if (w.bn == 128) return run_wgrad<128>(ma, mb, a_each, b_each, g, tp, w, partial, st);
+  return run_wgrad<256>(ma, mb, a_each, b_each, g, tp, w, partial, st);
 }
 
 // ------------------------------------------------ few-channel "row window" route
@@ -591,8 +613,8 @@ size_t patch_conv_workspace_bytes(const ConvGeo& g0, int which) {
 }
 
 size_t patch_conv_cache_bytes(const ConvGeo& g, int which) {
-  if (which == 0) return g.x_cl ? 0 : up256((size_t)g.N * sampled_geo(g).HW * up4(g.C) * 4);
-  return g.y_cl ? 0 : up256((size_t)g.N * g.HoWo * up4(g.Cout) * 4);
+  if (which == 0) return g.x_cl ? 0 : up256(copy_bytes(g, (long long)g.N * sampled_geo(g).HW, g.C, up4(g.C)));
+  return g.y_cl ? 0 : up256(copy_bytes(g, (long long)g.N * g.HoWo, g.Cout, up4(g.Cout)));
 }
 
 // rows of the statistics matrix: four per pixel patch (one per 32-row quarter of a tile)
@@ -614,7 +636,7 @@ int patch_conv_forward(const ConvGeo& g0, const float* x, const float* w, const 
   float* wp = reinterpret_cast<float*>(base);
   if (!g.x_cl) {
     const ClSlot xs =
-        cl_slot(cache, 0, (size_t)g.N * g.HW * cp * 4, reinterpret_cast<float*>(base));
+        cl_slot(cache, 0, copy_bytes(g, (long long)g.N * g.HW, g.C, cp), reinterpret_cast<float*>(base));
     wp = reinterpret_cast<float*>(base + up256((size_t)g.N * g.HW * cp * 4));
     if (!xs.valid) {
       if (int rc = x_to_nhwc(g0, x, xs.buf, cp, st)) return rc;
@@ -656,7 +678,7 @@ int patch_conv_backward_data(const ConvGeo& g, const float* gy, const float* w, 
   float* wd = reinterpret_cast<float*>(base);
   if (!g.y_cl) {
     const ClSlot gs =
-        cl_slot(cache, 1, (size_t)g.N * g.HoWo * cop * 4, reinterpret_cast<float*>(base));
+        cl_slot(cache, 1, copy_bytes(g, (long long)g.N * g.HoWo, g.Cout, cop), reinterpret_cast<float*>(base));
     wd = reinterpret_cast<float*>(base + up256((size_t)g.N * g.HoWo * cop * 4));
     if (int rc = to_nhwc(gy, gs.buf, g.N, g.Cout, cop, g.HoWo, st)) return rc;
     if (gs.flag) *gs.flag = 1;  // backward-filter of the same grad_y can take it from here
@@ -768,7 +790,7 @@ int patch_conv_backward_filter(const ConvGeo& g0, const float* gy, const float* 
   const float* xt = x;
   if (!g.x_cl) {
     const ClSlot xs =
-        cl_slot(cache, 0, (size_t)g.N * g.HW * cp * 4, reinterpret_cast<float*>(base));
+        cl_slot(cache, 0, copy_bytes(g, (long long)g.N * g.HW, g.C, cp), reinterpret_cast<float*>(base));
     off += up256((size_t)g.N * g.HW * cp * 4);
     if (!xs.valid) {
       if (int rc = x_to_nhwc(g0, x, xs.buf, cp, st)) return rc;
@@ -779,7 +801,8 @@ int patch_conv_backward_filter(const ConvGeo& g0, const float* gy, const float* 
   const float* gyt = gy;
   if (!g.y_cl) {
     const ClSlot gs =
-        cl_slot(cache, 1, (size_t)g.N * g.HoWo * cop * 4, reinterpret_cast<float*>(base + off));
+        cl_slot(cache, 1, copy_bytes(g, (long long)g.N * g.HoWo, g.Cout, cop),
+                reinterpret_cast<float*>(base + off));
     off += up256((size_t)g.N * g.HoWo * cop * 4);
     if (gs.valid) {
       *gs.flag = 0;  // consumed: the next backward pass brings another grad_y
@@ -790,14 +813,15 @@ int patch_conv_backward_filter(const ConvGeo& g0, const float* gy, const float* 
   }
   float* partial = reinterpret_cast<float*>(base + off);
   CUtensorMap ma, mb;
-  if (int rc = nhwc_map5(&ma, gyt, g.operand, g.Cout, cop, g.Wo, g.Ho, g.N, wp.QW, wp.PH,
-                         wgrad_a_boxes(g), 1, 1))
+  int a_each, b_each;
+  if (int rc = nhwc_operand(&ma, &a_each, g, gyt, g.y_cl, g.Cout, cop, g.Wo, g.Ho, wp.QW, wp.PH,
+                            wgrad_a_boxes(g), 1, 1))
     return rc;
-  if (int rc = nhwc_map5(&mb, xt, g.operand, g.C, cp, g.W, g.H, g.N, wp.QW, wp.PH, 1 << wp.cn_shift, g.sx,
-                         g.sy))
+  if (int rc = nhwc_operand(&mb, &b_each, g, xt, g.x_cl, g.C, cp, g.W, g.H, wp.QW, wp.PH, 1 << wp.cn_shift,
+                            g.sx, g.sy))
     return rc;
   const WgradTaps tp{g.C, g.RS, g.kW, g.dx, g.dy, g.px, g.py};
-  if (int rc = run_wgrad_any(ma, mb, g, tp, wp, partial, st)) return rc;
+  if (int rc = run_wgrad_any(ma, mb, a_each, b_each, g, tp, wp, partial, st)) return rc;
   if (g.operand == tc::kOperandBf16)
     return wgrad_reduce(partial, reinterpret_cast<__nv_bfloat16*>(gw), g, wp.splits, st);
   if (g.operand == tc::kOperandF16)
@@ -906,8 +930,9 @@ int window_conv_backward_filter(const ConvGeo& g, const float* gy, const float* 
   CUtensorMap ma, mb;
   if (int rc = window_rows_map(&mb, xtp, wg, g.N, wp.QW, wp.PH, 1 << wp.cn_shift, g.sx, g.sy, g.kH,
                                g.dy)) return rc;
-  if (int rc = nhwc_map5(&ma, gyt, g.operand, g.Cout, cop, g.Wo, g.Ho, g.N, wp.QW, wp.PH,
-                         wgrad_a_boxes(g), 1, 1))
+  int a_each;
+  if (int rc = nhwc_operand(&ma, &a_each, g, gyt, g.y_cl, g.Cout, cop, g.Wo, g.Ho, wp.QW, wp.PH,
+                            wgrad_a_boxes(g), 1, 1))
     return rc;
   if (!xs.valid) {
     const long long total = (long long)g.N * wg.Hp * wg.Wp;
@@ -921,7 +946,7 @@ int window_conv_backward_filter(const ConvGeo& g, const float* gy, const float* 
   // One GEMM: M = Cout, N = kH blocks of 32 window floats, K = pixels.  The filter rows are
   // the channel groups of the view, so the launch has a single tap at offset zero.
   const WgradTaps tp{32 * g.kH, 1, 1, 1, 1, 0, 0};
-  if (int rc = run_wgrad_any(ma, mb, g, tp, wp, partial, st)) return rc;
+  if (int rc = run_wgrad_any(ma, mb, a_each, 0, g, tp, wp, partial, st)) return rc;
   window_wgrad_reduce_kernel<<<grid_for((long long)g.Cout * g.C * g.RS, 256), 256, 0, st>>>(
       partial, gw, g.Cout, g.C, g.kH, g.kW, wp.splits);
   FLB200_AFTER_LAUNCH("window_wgrad_reduce");

@@ -314,7 +314,8 @@ struct PatchWgradProblem {
   // The BN columns of a tile are tg taps x (1 << cn_shift) boxes of 32 input channels, so a
   // narrow layer shares one load of dy between several taps.
   int ntaps, tap_groups, tg, cn_shift;
-  int a_nbox;                  // 32-channel boxes of dy per copy: min(4, ceil(M / 32))
+  int a_nbox;                  // 32-channel boxes of dy per stage: min(4, ceil(M / 32))
+  int a_each, b_each;          // 1: a copy per box (nhwc_operand), else one copy of all of them
   int splits, iters_per_split, k_iters;  // k_iters = images * tiles_p * tiles_q
   int b_w_mul, b_h_mul;        // B box origin = (q0 * b_w_mul + dw, p0 * b_h_mul + dh)
   int kW, dil_x, dil_y, pad_x, pad_y;  // tap t = (r, s) = (t / kW, t % kW): dw = s*dil_x - pad_x
@@ -344,8 +345,9 @@ struct PatchWgradProblem {
     ls.qi = r % tiles_q; r /= tiles_q;
     ls.pi = r % tiles_p; r /= tiles_p;
     ls.img = r;
-    // copy 0 is dy, copy j >= 1 the x box of tap tap0 + j - 1
-    const int tap = t.tap0 + max(copy - 1, 0);
+    // the first copies are dy, the others x, tap after tap
+    const int na = a_each ? a_nbox : 1;
+    const int tap = t.tap0 + (max(copy - na, 0) >> (b_each ? cn_shift : 0));
     const int tr = tap / kW, ts = tap - tr * kW;
     ls.dw = ts * dil_x - pad_x;
     ls.dh = tr * dil_y - pad_y;
@@ -356,21 +358,33 @@ struct PatchWgradProblem {
                                        int parts) const {
     const int q0 = ls.qi * QW, p0 = ls.pi * PH;
     const int copy = lane * parts + part;
-    // The channel index is split into (32 contiguous channels, group of 32) in both maps, so
-    // one copy brings every 32 x 32 box of an operand: a_nbox boxes of dy, and per tap
-    // 1 << cn_shift boxes of x.  Boxes past the last channel are zero-filled or hold a
-    // neighbouring pixel's channels; they only reach accumulator rows / columns that the
-    // epilogue never stores.
+    // With the channel index of a map split into (32 contiguous channels, group of 32) one copy
+    // brings every 32 x 32 box of an operand: a_nbox boxes of dy, and per tap 1 << cn_shift boxes
+    // of x.  Boxes past the last channel are zero-filled or hold a neighbouring pixel's channels;
+    // they only reach accumulator rows / columns that the epilogue never stores.  Over whole
+    // channels each box is a copy of its own, zero-filled past the last channel.
     const int box_bytes = 128 << cb_shift;  // 32 pixels x 32 fp32 or 64 pixels x 64 16-bit channels
     if (lane == 0 && part == 0)
       mbar_post_tx(bar, (a_nbox + (t.ntap << cn_shift)) * box_bytes, last);
     __syncwarp();
-    if (copy == 0) {
-      int ca[5] = {0, q0, p0, ls.img, t.m0 >> cb_shift};
-      tma_load(ma, bar, a_dst, 5, ca);
-    } else if (copy <= t.ntap) {
-      int cb[5] = {0, q0 * b_w_mul + ls.dw, p0 * b_h_mul + ls.dh, ls.img, t.n0 >> cb_shift};
-      tma_load(mb, bar, b_dst + ((copy - 1) << cn_shift) * box_bytes, 5, cb);
+    const int na = a_each ? a_nbox : 1, j = copy - na;
+    if (j < 0) {
+      if (a_each) {
+        int ca[5] = {t.m0 + (copy << cb_shift), q0, p0, ls.img, 0};
+        tma_load(ma, bar, a_dst + copy * box_bytes, 4, ca);
+      } else {
+        int ca[5] = {0, q0, p0, ls.img, t.m0 >> cb_shift};
+        tma_load(ma, bar, a_dst, 5, ca);
+      }
+    } else if (j < (b_each ? t.ntap << cn_shift : t.ntap)) {
+      const int w = q0 * b_w_mul + ls.dw, h = p0 * b_h_mul + ls.dh;
+      if (b_each) {
+        int cb[5] = {t.n0 + ((j & ((1 << cn_shift) - 1)) << cb_shift), w, h, ls.img, 0};
+        tma_load(mb, bar, b_dst + j * box_bytes, 4, cb);
+      } else {
+        int cb[5] = {0, w, h, ls.img, t.n0 >> cb_shift};
+        tma_load(mb, bar, b_dst + (j << cn_shift) * box_bytes, 5, cb);
+      }
     }
     if (++ls.qi == tiles_q) {
       ls.qi = 0;

@@ -337,3 +337,35 @@ def test_conv_statistics_are_declined_where_not_built():
         sums = []
         y = ext.conv2d(xin, w, None, 1, 1, 1, 1, 1, 1, 1, None, stats_out=sums)
         assert sums == [] and y.shape == (2, 48, 8, 8)
+
+
+# channels past one 32-channel box that fill no whole number of them, on either side: the filter
+# gradient then maps the caller's tensors box by box (fl's order: copies, kept in the payload)
+RAGGED = [(2, 36, 9, 10, 48, 3, 1), (2, 48, 8, 8, 36, 1, 1), (1, 100, 7, 7, 164, 3, 2), (3, 292, 6, 6, 68, 1, 1),
+          (2, 64, 9, 9, 40, 5, 1), (2, 44, 12, 5, 64, 3, 1), (4, 3, 20, 22, 100, 7, 2)]
+
+
+@pytest.mark.parametrize("channels_last", [True, False])
+@pytest.mark.parametrize("mode", ["tf32", "f32x3"])
+@pytest.mark.parametrize("case", RAGGED)
+def test_filter_gradient_of_ragged_channels(L, case, mode, channels_last):
+    from flashlight_b200.extension import AutogradPayload, B200AutogradExtension
+    N, Cin, H, W, Cout, k, s = case
+    ext = B200AutogradExtension(math_mode=L.MATH_BY_NAME[mode])
+    p = k // 2
+    args = (s, s, p, p, 1, 1, 1)
+    x, w = randn(N, Cin, H, W, seed=71), randn(Cout, Cin, k, k, seed=72) / (Cin * k * k) ** 0.5
+    out_only = Cin < 16  # a first convolution: x in fl's order
+    xd = cl(x) if channels_last and not out_only else x.cuda()
+    payload = None if channels_last else AutogradPayload()
+    ext.conv2d(xd, w.cuda(), None, *args, payload=payload, channels_last_out=True if channels_last and out_only else None)
+    want = R.conv2d(x.double(), w.double(), None, *args)
+    gy = randn(*want.shape, seed=73)
+    gd = cl(gy) if channels_last else gy.cuda()
+    before = L.lib.flb200_tc_kernel_launches()
+    if payload is not None:
+        ext.conv2dBackwardData(gd, xd, w.cuda(), *args, payload=payload)
+    gw, _ = ext.conv2dBackwardFilterBias(gd, xd, w.cuda(), None, *args, autogradPayload=payload)
+    assert L.lib.flb200_tc_kernel_launches() > before
+    wgw, _ = R.conv2d_backward_filter_bias(gy.double(), x.double(), w.shape, False, *args)
+    assert_close_scaled(gw, wgw, TF32_SCALED_TOL if mode == "tf32" else 2e-5, "conv backward filter")
