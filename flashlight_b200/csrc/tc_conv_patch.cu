@@ -499,9 +499,10 @@ int run_wgrad_any(const CUtensorMap& ma, const CUtensorMap& mb, int a_each, int 
 // the window extent.  The filter rows r are the taps of the implicit GEMM (k_iters = kH).
 constexpr int kWinPixels = 8;  // 32 floats / 4 channels
 
-// dst[n][hp][wp] = (x[n][0..C)[hp-py][wp-px], 0...) as one float4, zero outside the image.
+// dst[n][hp][wp] = (x[n][0..C)[hp-py][wp-px], 0...) as one float4, zero outside the image and in the
+// rows behind the last of the N images.
 __global__ void __launch_bounds__(256)
-nchw_to_nhwc4_pad_kernel(const float* __restrict__ x, float4* __restrict__ dst, int C, int H,
+nchw_to_nhwc4_pad_kernel(const float* __restrict__ x, float4* __restrict__ dst, int N, int C, int H,
                          int W, int Hp, int Wp, int py, int px, long long total) {
   for (long long t = (long long)blockIdx.x * blockDim.x + threadIdx.x; t < total;
        t += (long long)gridDim.x * blockDim.x) {
@@ -511,7 +512,7 @@ nchw_to_nhwc4_pad_kernel(const float* __restrict__ x, float4* __restrict__ dst, 
     const long long n = r2 / Hp;
     const int h = hp - py, w = wp - px;
     float v[4] = {0.f, 0.f, 0.f, 0.f};
-    if (h >= 0 && h < H && w >= 0 && w < W) {
+    if (n < N && h >= 0 && h < H && w >= 0 && w < W) {
       for (int c = 0; c < C; ++c) v[c] = x[((n * C + c) * H + h) * W + w];
     }
     dst[t] = make_float4(v[0], v[1], v[2], v[3]);
@@ -555,6 +556,11 @@ WindowGeo window_geo(const ConvGeo& g) {
   return w;
 }
 
+// Pixels of the padded copy: its images, and the rows behind the last one that window_rows_map reaches.
+long long window_pixels(const ConvGeo& g, const WindowGeo& w) {
+  return ((long long)g.N * w.Hp + (long long)(g.kH - 1) * g.dy) * w.Wp;
+}
+
 // [32-float window, window start pixel, padded row, image]: the pixel stride (16 bytes) is
 // smaller than the window, i.e. the rows of the view overlap.
 int window_map(CUtensorMap* m, const float* base, const WindowGeo& wg, int N, int box_w, int box_h,
@@ -569,8 +575,8 @@ int window_map(CUtensorMap* m, const float* base, const WindowGeo& wg, int N, in
 // Backward-filter view: a fifth index r (the filter row) steps dy padded rows, so one copy
 // of nbox >= kH groups brings the windows of every filter row of a 32-pixel patch as the
 // [pixels][32] blocks of an MN-major operand.  Row p*sy + r*dy can pass the image's last
-// padded row only for patch rows p >= Ho, where dy is zero and what is read instead (the next
-// image, or the bytes after the tensor inside the workspace) is finite.
+// padded row only for patch rows p >= Ho, where dy is zero and what is read instead is the next
+// image, or the zeros behind the last one.
 int window_rows_map(CUtensorMap* m, const float* base, const WindowGeo& wg, int N, int box_w,
                     int box_h, int nbox, int sx, int sy, int kH, int dil_y) {
   const uint64_t dims[5] = {32, (uint64_t)wg.starts, (uint64_t)wg.Hp, (uint64_t)N, (uint64_t)kH};
@@ -852,7 +858,7 @@ bool window_conv_supported(const ConvGeo& g) {
 
 size_t window_conv_workspace_bytes(const ConvGeo& g, int which) {
   const WindowGeo wg = window_geo(g);
-  const size_t xtp = up256((size_t)g.N * wg.Hp * wg.Wp * 16);
+  const size_t xtp = up256((size_t)window_pixels(g, wg) * 16);
   if (which == 0) return xtp + up256((size_t)g.kH * g.Cout * 32 * 4);
   const int cop = up4(g.Cout);
   // the backward-filter GEMM has 32 columns per tap and kH taps
@@ -863,7 +869,7 @@ size_t window_conv_workspace_bytes(const ConvGeo& g, int which) {
 size_t window_conv_cache_bytes(const ConvGeo& g, int which) {
   if (which != 0) return 0;  // this route has no backward-data pass to share grad_y with
   const WindowGeo wg = window_geo(g);
-  return up256((size_t)g.N * wg.Hp * wg.Wp * 16);
+  return up256((size_t)window_pixels(g, wg) * 16);
 }
 
 int window_conv_forward(const ConvGeo& g, const float* x, const float* w, const float* bias,
@@ -873,9 +879,9 @@ int window_conv_forward(const ConvGeo& g, const float* x, const float* w, const 
   const WindowGeo wg = window_geo(g);
   char* base = static_cast<char*>(ws);
   const ClSlot xs =
-      cl_slot(cache, 0, (size_t)g.N * wg.Hp * wg.Wp * 16, reinterpret_cast<float*>(base));
+      cl_slot(cache, 0, (size_t)window_pixels(g, wg) * 16, reinterpret_cast<float*>(base));
   float* xtp = xs.buf;
-  float* wr = reinterpret_cast<float*>(base + up256((size_t)g.N * wg.Hp * wg.Wp * 16));
+  float* wr = reinterpret_cast<float*>(base + up256((size_t)window_pixels(g, wg) * 16));
   PatchArgs a{};
   a.patch = pick_patch(g.Wo, g.Ho, g.N);
   CUtensorMap ma, mb;
@@ -885,9 +891,9 @@ int window_conv_forward(const ConvGeo& g, const float* x, const float* w, const 
   const int bn = tc::pick_bn(g.Cout);
   if (int rc = filter_map(&mb, wr, g.operand, 32, 32, g.Cout, g.kH, filter_box_rows(bn))) return rc;
   if (!xs.valid) {
-    const long long total = (long long)g.N * wg.Hp * wg.Wp;
+    const long long total = window_pixels(g, wg);
     nchw_to_nhwc4_pad_kernel<<<grid_for(total, 256), 256, 0, st>>>(
-        x, reinterpret_cast<float4*>(xtp), g.C, g.H, g.W, wg.Hp, wg.Wp, g.py, g.px, total);
+        x, reinterpret_cast<float4*>(xtp), g.N, g.C, g.H, g.W, wg.Hp, wg.Wp, g.py, g.px, total);
     FLB200_AFTER_LAUNCH("nchw_to_nhwc4_pad");
     if (xs.flag) *xs.flag = 1;
   }
@@ -916,9 +922,9 @@ int window_conv_backward_filter(const ConvGeo& g, const float* gy, const float* 
   const WgradPlan wp = plan_wgrad(g, 32 * g.kH, 1);
   char* base = static_cast<char*>(ws);
   const ClSlot xs =
-      cl_slot(cache, 0, (size_t)g.N * wg.Hp * wg.Wp * 16, reinterpret_cast<float*>(base));
+      cl_slot(cache, 0, (size_t)window_pixels(g, wg) * 16, reinterpret_cast<float*>(base));
   float* xtp = xs.buf;
-  size_t off = up256((size_t)g.N * wg.Hp * wg.Wp * 16);
+  size_t off = up256((size_t)window_pixels(g, wg) * 16);
   const float* gyt = gy;
   float* gy_copy = nullptr;
   if (!g.y_cl) {
@@ -935,9 +941,9 @@ int window_conv_backward_filter(const ConvGeo& g, const float* gy, const float* 
                             wgrad_a_boxes(g), 1, 1))
     return rc;
   if (!xs.valid) {
-    const long long total = (long long)g.N * wg.Hp * wg.Wp;
+    const long long total = window_pixels(g, wg);
     nchw_to_nhwc4_pad_kernel<<<grid_for(total, 256), 256, 0, st>>>(
-        x, reinterpret_cast<float4*>(xtp), g.C, g.H, g.W, wg.Hp, wg.Wp, g.py, g.px, total);
+        x, reinterpret_cast<float4*>(xtp), g.N, g.C, g.H, g.W, wg.Hp, wg.Wp, g.py, g.px, total);
     FLB200_AFTER_LAUNCH("nchw_to_nhwc4_pad");
     if (xs.flag) *xs.flag = 1;
   }

@@ -369,3 +369,24 @@ def test_filter_gradient_of_ragged_channels(L, case, mode, channels_last):
     assert L.lib.flb200_tc_kernel_launches() > before
     wgw, _ = R.conv2d_backward_filter_bias(gy.double(), x.double(), w.shape, False, *args)
     assert_close_scaled(gw, wgw, TF32_SCALED_TOL if mode == "tf32" else 2e-5, "conv backward filter")
+
+
+@pytest.mark.parametrize("case", [(2, 3, 13, 14, 32, 3, 1), (3, 1, 9, 7, 48, 5, 1), (1, 4, 21, 20, 64, 7, 2)])
+def test_first_convolution_ignores_what_scratch_held(L, case):
+    """Rows of the pixel patches past the image meet zeros behind the padded copy, not what the memory
+    held before (NaN here)."""
+    from flashlight_b200.extension import B200AutogradExtension
+    N, C, H, W, Cout, k, s = case
+    ext = B200AutogradExtension(math_mode=L.MATH_TF32, cache_layouts=False)
+    args = (s, s, k // 2, k // 2, 1, 1, 1)
+    x, w = randn(N, C, H, W, seed=74), randn(Cout, C, k, k, seed=75)
+    want = R.conv2d(x.double(), w.double(), None, *args)
+    gy = randn(*want.shape, seed=76)
+    xd, gd, wd = x.cuda(), gy.cuda(), w.cuda()
+    blocks = [torch.full((n,), float("nan"), device="cuda") for n in [1 << b for b in range(8, 23)] * 3]
+    del blocks
+    before = L.lib.flb200_tc_kernel_launches()
+    gw, _ = ext.conv2dBackwardFilterBias(gd, xd, wd, None, *args)
+    assert L.lib.flb200_tc_kernel_launches() > before
+    wgw, _ = R.conv2d_backward_filter_bias(gy.double(), x.double(), w.shape, False, *args)
+    assert_close_scaled(gw, wgw, TF32_SCALED_TOL, "conv backward filter")
