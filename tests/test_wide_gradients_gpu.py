@@ -8,8 +8,10 @@ from tests.parity import assert_close, randn
 pytestmark = pytest.mark.gpu
 
 
-# m, n, k: single tiles with tails, pairs, few tiles of a long K (split, reduced by a second kernel)
-@pytest.mark.parametrize("mnk", [(8, 8, 8), (72, 40, 200), (512, 1536, 600), (768, 768, 4096), (136, 264, 8200)])
+# m, n, k: single tiles with tails, pairs, few tiles of a long K (split, reduced by a second kernel;
+# many splits of a small result, which share a CTA there)
+@pytest.mark.parametrize("mnk", [(8, 8, 8), (72, 40, 200), (512, 1536, 600), (768, 768, 4096), (136, 264, 8200), (8, 32, 20000),
+                                 (72, 40, 12544)])
 def test_matmul_wide(mnk):
     from flashlight_b200 import functions as F
     m, n, k = mnk
