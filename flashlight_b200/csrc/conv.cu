@@ -118,44 +118,61 @@ struct ImageVec {
   }
 };
 
-// ---- images read element by element, K = (channel, tap)
+// ---- images read element by element, K = (channel, tap).  Row and k carry their part of the offset
+// whether or not they meet inside the image, so that an element costs two additions, the test of its
+// position and one address; only backward-data with a stride has to divide.
+constexpr int kNowhere = -(1 << 30);  // a position that no tap brings inside
 template <bool DGRAD>
 struct ImageElem {
   static constexpr int kKind = kElemRows;
   const float* p;
   ConvGeo g;
   int n_total;
-  typedef PixelRow Row;
-  struct Kk { int off, dh, dw; };
+  struct Row { long long off; int h0, w0; };
+  struct Kk { long long off; int dh, dw; };
   __device__ const float* base() const { return p; }
+  __device__ bool divides() const { return DGRAD && (g.sx != 1 || g.sy != 1); }
   __device__ Row row(int n, int z) const {
-    if (n >= n_total) return Row{-1, 0, 0};
+    if (n >= n_total) return Row{0, kNowhere, kNowhere};
+    Row r;
     if (DGRAD) {
       const int img = n / g.HW, hw = n - img * g.HW, h = hw / g.W, w = hw - h * g.W;
-      return Row{(long long)img * g.Cout * g.HoWo + (long long)z * g.Coutg * g.y_cs, h + g.py, w + g.px};
+      r.off = (long long)img * g.Cout * g.HoWo + (long long)z * g.Coutg * g.y_cs;
+      r.h0 = h + g.py;
+      r.w0 = w + g.px;
+      if (!divides()) r.off += ((long long)r.h0 * g.Wo + r.w0) * g.y_ps;
+    } else {
+      const int img = n / g.HoWo, pq = n - img * g.HoWo, y = pq / g.Wo, q = pq - y * g.Wo;
+      r.h0 = y * g.sy - g.py;
+      r.w0 = q * g.sx - g.px;
+      r.off = (long long)img * g.C * g.HW + (long long)z * g.Cg * g.x_cs +
+              ((long long)r.h0 * g.W + r.w0) * g.x_ps;
     }
-    const int img = n / g.HoWo, pq = n - img * g.HoWo, y = pq / g.Wo, q = pq - y * g.Wo;
-    return Row{(long long)img * g.C * g.HW + (long long)z * g.Cg * g.x_cs, y * g.sy - g.py,
-               q * g.sx - g.px};
+    return r;
   }
   __device__ Kk kk(int k, int) const {
     const int c = k / g.RS, rs = k - c * g.RS, r = rs / g.kW, s = rs - r * g.kW;
-    return Kk{c * (DGRAD ? g.y_cs : g.x_cs), r * g.dy, s * g.dx};
+    Kk v{(long long)c * (DGRAD ? g.y_cs : g.x_cs), r * g.dy, s * g.dx};
+    if (DGRAD) {
+      v.dh = -v.dh;
+      v.dw = -v.dw;
+    }
+    if (!divides()) v.off += ((long long)v.dh * (DGRAD ? g.Wo : g.W) + v.dw) * (DGRAD ? g.y_ps : g.x_ps);
+    return v;
   }
   __device__ const float* at(const Row& row, const Kk& k) const {
-    if (row.base < 0) return nullptr;
-    if (DGRAD) {
-      const int th = row.h0 - k.dh, tw = row.w0 - k.dw;
-      if (th < 0 || tw < 0) return nullptr;
-      int y = th, q = tw;
-      if (g.sy != 1) { y = th / g.sy; if (y * g.sy != th) return nullptr; }
-      if (g.sx != 1) { q = tw / g.sx; if (q * g.sx != tw) return nullptr; }
-      if (y >= g.Ho || q >= g.Wo) return nullptr;
-      return p + row.base + k.off + (long long)(y * g.Wo + q) * g.y_ps;
+    int h = row.h0 + k.dh, w = row.w0 + k.dw;
+    long long off = row.off + k.off;
+    if (divides()) {
+      if (h < 0 || w < 0) return nullptr;
+      const int y = h / g.sy, q = w / g.sx;
+      if (y * g.sy != h || q * g.sx != w) return nullptr;
+      h = y;
+      w = q;
+      off += ((long long)y * g.Wo + q) * g.y_ps;
     }
-    const int h = row.h0 + k.dh, w = row.w0 + k.dw;
-    if (h < 0 || h >= g.H || w < 0 || w >= g.W) return nullptr;
-    return p + row.base + k.off + (long long)(h * g.W + w) * g.x_ps;
+    const bool inside = (unsigned)h < (unsigned)(DGRAD ? g.Ho : g.H) && (unsigned)w < (unsigned)(DGRAD ? g.Wo : g.W);
+    return inside ? p + off : nullptr;
   }
 };
 
@@ -206,7 +223,8 @@ PixelOut pixel_out(float* out, const float* bias, const ConvGeo& g, bool dgrad) 
   o.pixels = dgrad ? g.HW : g.HoWo;
   o.per_group = dgrad ? g.Cg : g.Coutg;
   o.along_m = o.pix == 1;
-  o.vec = o.chan == 1 && o.per_group % 4 == 0 && o.pix % 4 == 0 && aligned16(out);
+  o.vec = (o.along_m ? o.pixels % 4 == 0 && o.chan % 4 == 0
+                     : o.chan == 1 && o.per_group % 4 == 0 && o.pix % 4 == 0) && aligned16(out);
   return o;
 }
 
@@ -242,28 +260,30 @@ struct WindowVec {
     return x + it.img + (long long)(h * g.W + w) * g.C + r.off;
   }
 };
-// element by element, n = (channel, tap)
+// element by element, n = (channel, tap); offsets split as in ImageElem
 struct WindowElem {
   static constexpr int kKind = kElemK;
   const float* x;
   ConvGeo g;
   int n_total;
   struct Row { long long off; int dh, dw; };
-  struct Kk { long long base; int h0, w0; };
+  struct Kk { long long off; int h0, w0; };
   __device__ const float* base() const { return x; }
   __device__ Row row(int n, int z) const {
-    if (n >= n_total) return Row{-1, 0, 0};
+    if (n >= n_total) return Row{0, kNowhere, kNowhere};
     const int c = n / g.RS, rs = n - c * g.RS, r = rs / g.kW, s = rs - r * g.kW;
-    return Row{((long long)z * g.Cg + c) * g.x_cs, r * g.dy - g.py, s * g.dx - g.px};
+    const int dh = r * g.dy - g.py, dw = s * g.dx - g.px;
+    return Row{((long long)z * g.Cg + c) * g.x_cs + ((long long)dh * g.W + dw) * g.x_ps, dh, dw};
   }
   __device__ Kk kk(int k, int) const {
     const int img = k / g.HoWo, pq = k - img * g.HoWo, y = pq / g.Wo, q = pq - y * g.Wo;
-    return Kk{(long long)img * g.C * g.HW, y * g.sy, q * g.sx};
+    const int h0 = y * g.sy, w0 = q * g.sx;
+    return Kk{(long long)img * g.C * g.HW + ((long long)h0 * g.W + w0) * g.x_ps, h0, w0};
   }
   __device__ const float* at(const Row& r, const Kk& k) const {
     const int h = k.h0 + r.dh, w = k.w0 + r.dw;
-    if (r.off < 0 || h < 0 || h >= g.H || w < 0 || w >= g.W) return nullptr;
-    return x + k.base + r.off + (long long)(h * g.W + w) * g.x_ps;
+    const bool inside = (unsigned)h < (unsigned)g.H && (unsigned)w < (unsigned)g.W;
+    return inside ? x + k.off + r.off : nullptr;
   }
 };
 // dy element by element, lanes along the pixels

@@ -54,7 +54,7 @@ int matmul_simt(const flb200_matmul_desc* d, const void* a, const void* b, void*
   StridedEpilogue ep{static_cast<float*>(c), nullptr, d->alpha, d->beta, 0, 0, d->c_row, d->c_col,
                      d->c_batch};
   ep.along_m = d->c_row == 1 && d->c_col != 1;
-  ep.vec = d->c_col == 1 && d->n % 4 == 0 && d->c_row % 4 == 0 &&
+  ep.vec = (ep.along_m ? d->m % 4 == 0 && d->c_col % 4 == 0 : d->c_col == 1 && d->n % 4 == 0 && d->c_row % 4 == 0) &&
            (d->batch == 1 || d->c_batch % 4 == 0) && aligned16(c);
   const int ak = loader_kind(a, d->a_row, d->a_col, d->a_batch, d->m, d->k, d->batch);
   const int bk = loader_kind(b, d->b_col, d->b_row, d->b_batch, d->n, d->k, d->batch);

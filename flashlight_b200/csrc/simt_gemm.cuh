@@ -36,7 +36,7 @@
 // Epilogue concept: element offsets of a row and of a column (-1: not stored) and
 //   float* out; const float* bias (per column, may be null); float alpha, beta;
 //   int along_m (consecutive rows are adjacent in memory, else consecutive columns);
-//   int vec (columns may be stored four at a time).
+//   int vec (the adjacent ones may be stored four at a time).
 #pragma once
 #include "common.cuh"
 #include "tc_core.cuh"
@@ -100,7 +100,7 @@ struct Feeder<L, ROWS, THREADS, kVecK> {
   typename L::Row rows[PASSES];
   typename L::Iter it;
   int k;
-  __device__ void begin(const L& l, char*, int r0, int k0, int z) {
+  __device__ void begin(const L& l, char*, int r0, int, int k0, int z) {
     const int t = threadIdx.x;
 #pragma unroll
     for (int p = 0; p < PASSES; ++p) rows[p] = l.row(r0 + t / 4 + STEP * p, z);
@@ -127,7 +127,7 @@ struct Feeder<L, ROWS, THREADS, kVecRow> {
   typename L::Row row;
   typename L::Iter it[PASSES];
   int k;
-  __device__ void begin(const L& l, char*, int r0, int k0, int z) {
+  __device__ void begin(const L& l, char*, int r0, int, int k0, int z) {
     const int t = threadIdx.x;
     row = l.row(r0 + 4 * (t % CHUNKS), z);
     k = k0 + t / CHUNKS;
@@ -148,20 +148,24 @@ struct Feeder<L, ROWS, THREADS, kVecRow> {
 };
 
 // Single elements.  The decoded k of a stage (lanes along rows: 16 of them, made by 16 threads one
-// stage ahead) or the decoded rows (lanes along k) sit in a shared table.
+// stage ahead) or the decoded rows (lanes along k) sit in a shared table.  Rows past the last one are
+// left as they are: nothing that they meet is stored.
 template <class L, int ROWS, int THREADS>
 struct Feeder<L, ROWS, THREADS, kElemRows> {
   static constexpr int KSTEP = THREADS / ROWS, PASSES = kBKf / KSTEP;
   static constexpr int kTableBytes = 2 * kBKf * (int)sizeof(typename L::Kk);
   typename L::Row row;
-  __device__ void begin(const L& l, char* table, int r0, int k0, int z) {
+  bool live;
+  __device__ void begin(const L& l, char*, int r0, int rows, int, int z) {
     row = l.row(r0 + threadIdx.x % ROWS, z);
+    live = (int)(threadIdx.x % ROWS) < rows;
   }
   __device__ void prepare(const L& l, char* table, int k0, int slot, int kend, int z) {
     if (threadIdx.x < kBKf && k0 + (int)threadIdx.x < kend)
       reinterpret_cast<typename L::Kk*>(table)[(slot & 1) * kBKf + threadIdx.x] = l.kk(k0 + threadIdx.x, z);
   }
   __device__ void issue(const L& l, char* table, float* dst, int slot, int kleft) {
+    if (!live) return;
     const int t = threadIdx.x;
     const typename L::Kk* kt = reinterpret_cast<const typename L::Kk*>(table) + (slot & 1) * kBKf;
 #pragma unroll
@@ -176,9 +180,10 @@ template <class L, int ROWS, int THREADS>
 struct Feeder<L, ROWS, THREADS, kElemK> {
   static constexpr int RSTEP = THREADS / kBKf, PASSES = ROWS / RSTEP;
   static constexpr int kTableBytes = ROWS * (int)sizeof(typename L::Row);
-  int k, z;
-  __device__ void begin(const L& l, char* table, int r0, int k0, int z_) {
-    for (int r = threadIdx.x; r < ROWS; r += THREADS)
+  int k, z, live_rows;
+  __device__ void begin(const L& l, char* table, int r0, int rows, int k0, int z_) {
+    live_rows = rows < ROWS ? rows : ROWS;
+    for (int r = threadIdx.x; r < live_rows; r += THREADS)
       reinterpret_cast<typename L::Row*>(table)[r] = l.row(r0 + r, z_);
     k = k0 + threadIdx.x % kBKf;
     z = z_;
@@ -192,6 +197,7 @@ struct Feeder<L, ROWS, THREADS, kElemK> {
 #pragma unroll
     for (int p = 0; p < PASSES; ++p) {
       const int r = t / kBKf + RSTEP * p;
+      if (r >= live_rows) break;
       const float* src = live ? l.at(rows[r], kk) : nullptr;
       cp_async4(dst + r * kRowPitch + t % kBKf, src ? src : l.base(), src != nullptr);
     }
@@ -205,6 +211,7 @@ struct FfmaSmem {
   static constexpr int kB = k_layout(BL::kKind) ? T::BN * kRowPitch : T::BN * kBKf;
   static constexpr int kRing = kRingStages * (kA + kB) * 4;
   static constexpr int kTile = T::BM * (T::BN + 8) * 4;
+  static_assert(kTile >= T::BN * (T::BM + 4) * 4, "both orders of the tile fit");
   static constexpr int kMain = kRing > kTile ? kRing : kTile;
   static constexpr int kTabA = (Feeder<AL, T::BM, T::kThreads>::kTableBytes + 15) / 16 * 16;
   static constexpr int kTabB = (Feeder<BL, T::BN, T::kThreads>::kTableBytes + 15) / 16 * 16;
@@ -237,8 +244,8 @@ ffma_gemm_kernel(const AL al, const BL bl, const EP ep, int M, int N, int K, int
   Feeder<AL, BM, T::kThreads> fa;
   Feeder<BL, BN, T::kThreads> fb;
   constexpr bool kTables = AL::kKind >= kElemRows || BL::kKind >= kElemRows;
-  fa.begin(al, tab_a, m0, kbeg, z);
-  fb.begin(bl, tab_b, n0, kbeg, z);
+  fa.begin(al, tab_a, m0, M - m0, kbeg, z);
+  fb.begin(bl, tab_b, n0, N - n0, kbeg, z);
   for (int r = t; r < BM; r += T::kThreads) roff[r] = m0 + r < M ? ep.row(m0 + r, z) : -1;
   for (int c = t; c < BN; c += T::kThreads) coff[c] = n0 + c < N ? ep.col(n0 + c, z) : -1;
   // the element feeders take what is left of the stage, the vector feeders their own k
@@ -261,7 +268,7 @@ ffma_gemm_kernel(const AL al, const BL bl, const EP ep, int M, int N, int K, int
 #pragma unroll
   for (int b = 0; b < kRingStages - 1; ++b) {
     issue(b);
-    if (kTables) { prepare(b + 1); __syncthreads(); }
+    if (kTables && b + 1 < blocks) { prepare(b + 1); __syncthreads(); }
   }
 
   // acc: even / odd k of (i, j) when both operands are [row][k]; else neighbouring columns (B
@@ -358,7 +365,8 @@ ffma_gemm_kernel(const AL al, const BL bl, const EP ep, int M, int N, int K, int
   // ---- the tile through shared memory: summed over the cluster, stored in memory order
   cp_async_wait<0>();
   __syncthreads();
-  const int pitch = ep.along_m ? BN + 1 : BN + 8;
+  // (column after column where consecutive rows are adjacent in memory)
+  const int pitch_r = ep.along_m ? 1 : BN + 8, pitch_c = ep.along_m ? BM + 4 : 1;
   float* tile = ring;
 #pragma unroll
   for (int i = 0; i < TM; ++i)
@@ -377,7 +385,7 @@ ffma_gemm_kernel(const AL al, const BL bl, const EP ep, int M, int N, int K, int
         const float2 h = halves(acc[(j * TM + i) / 2]);
         v = i % 2 ? h.y : h.x;
       }
-      tile[r * pitch + c] = v;
+      tile[r * pitch_r + c * pitch_c] = v;
     }
   if (csplits > 1) tc::cluster_sync_all();
   else __syncthreads();
@@ -386,53 +394,76 @@ ffma_gemm_kernel(const AL al, const BL bl, const EP ep, int M, int N, int K, int
   const uint32_t tile_u = tc::smem_u32(tile);
   const bool raw = psplits > 1;
   float* pbase = raw ? partial + ((long long)(z * psplits + ps) * M) * N : nullptr;
-  if (!ep.along_m && (raw ? (N & 3) == 0 : ep.vec != 0)) {
+  // one or four adjacent values of the tile, summed over the cluster in rank order
+  auto sum1 = [&](int at) {
+    if (csplits == 1) return tile[at];
+    float v = 0.f;
+    for (int q = 0; q < csplits; ++q) {
+      float u;
+      asm volatile("ld.shared::cluster.f32 %0, [%1];"
+                   : "=f"(u)
+                   : "r"(tc::mapa_u32(tile_u + at * 4, (uint32_t)q)));
+      v += u;
+    }
+    return v;
+  };
+  auto sum4 = [&](int at) {
+    if (csplits == 1) return *reinterpret_cast<const float4*>(tile + at);
+    float4 v = make_float4(0.f, 0.f, 0.f, 0.f);
+    for (int q = 0; q < csplits; ++q) {
+      float4 u;
+      asm volatile("ld.shared::cluster.v4.f32 {%0, %1, %2, %3}, [%4];"
+                   : "=f"(u.x), "=f"(u.y), "=f"(u.z), "=f"(u.w)
+                   : "r"(tc::mapa_u32(tile_u + at * 4, (uint32_t)q)));
+      v.x += u.x; v.y += u.y; v.z += u.z; v.w += u.w;
+    }
+    return v;
+  };
+  auto store4 = [&](float* to, float4 v, float4 bias) {
+    float4* dst = reinterpret_cast<float4*>(to);
+    v.x = ep.alpha * v.x + bias.x; v.y = ep.alpha * v.y + bias.y;
+    v.z = ep.alpha * v.z + bias.z; v.w = ep.alpha * v.w + bias.w;
+    if (ep.beta != 0.f) {
+      const float4 o = *dst;
+      v.x += ep.beta * o.x; v.y += ep.beta * o.y; v.z += ep.beta * o.z; v.w += ep.beta * o.w;
+    }
+    *dst = v;
+  };
+  if (raw ? !ep.along_m && (N & 3) == 0 : !ep.along_m && ep.vec != 0) {
     for (int idx = t; idx < rows_here * (BN / 4); idx += T::kThreads) {
       const int r = r_first + idx / (BN / 4), c = 4 * (idx % (BN / 4));
-      float4 v;
-      if (csplits == 1) {
-        v = *reinterpret_cast<const float4*>(tile + r * pitch + c);
-      } else {
-        v = make_float4(0.f, 0.f, 0.f, 0.f);
-        for (int q = 0; q < csplits; ++q) {
-          float4 u;
-          asm volatile("ld.shared::cluster.v4.f32 {%0, %1, %2, %3}, [%4];"
-                       : "=f"(u.x), "=f"(u.y), "=f"(u.z), "=f"(u.w)
-                       : "r"(tc::mapa_u32(tile_u + (r * pitch + c) * 4, (uint32_t)q)));
-          v.x += u.x; v.y += u.y; v.z += u.z; v.w += u.w;
-        }
-      }
+      const float4 v = sum4(r * pitch_r + c);
       if (roff[r] < 0 || coff[c] < 0) continue;
       if (raw) {
         *reinterpret_cast<float4*>(pbase + (long long)(m0 + r) * N + n0 + c) = v;
         continue;
       }
-      float4* dst = reinterpret_cast<float4*>(ep.out + roff[r] + coff[c]);
-      v.x *= ep.alpha; v.y *= ep.alpha; v.z *= ep.alpha; v.w *= ep.alpha;
+      float4 bias = make_float4(0.f, 0.f, 0.f, 0.f);
       if (ep.bias) {
         const float* bp = ep.bias + ep.bias_at(n0 + c, z);
-        v.x += bp[0]; v.y += bp[1]; v.z += bp[2]; v.w += bp[3];
+        bias = make_float4(bp[0], bp[1], bp[2], bp[3]);
       }
-      if (ep.beta != 0.f) {
-        const float4 o = *dst;
-        v.x += ep.beta * o.x; v.y += ep.beta * o.y; v.z += ep.beta * o.z; v.w += ep.beta * o.w;
-      }
-      *dst = v;
+      store4(ep.out + roff[r] + coff[c], v, bias);
+    }
+  } else if (!raw && ep.along_m && ep.vec != 0) {
+    // four rows of a column per thread (one at a time, 16 x 28 x 28 x 256 -> 512 channels in fl's order
+    // took 153 us, so 100)
+    const int quads = rows_here / 4, shift = __ffs(quads) - 1;
+    for (int idx = t; idx < quads * BN; idx += T::kThreads) {
+      const int r = r_first + 4 * (idx & (quads - 1)), c = idx >> shift;
+      const float4 v = sum4(r + c * pitch_c);
+      if (roff[r] < 0 || coff[c] < 0) continue;
+      const float b = ep.bias ? ep.bias[ep.bias_at(n0 + c, z)] : 0.f;
+      store4(ep.out + roff[r] + coff[c], v, make_float4(b, b, b, b));
     }
   } else {
-    for (int idx = t; idx < rows_here * BN; idx += T::kThreads) {
-      const int r = r_first + (ep.along_m ? idx % rows_here : idx / BN);
-      const int c = ep.along_m ? idx / rows_here : idx % BN;
-      float v = 0.f;
-      for (int q = 0; q < csplits; ++q) {
-        float u;
-        if (csplits == 1) u = tile[r * pitch + c];
-        else
-          asm volatile("ld.shared::cluster.f32 %0, [%1];"
-                       : "=f"(u)
-                       : "r"(tc::mapa_u32(tile_u + (r * pitch + c) * 4, (uint32_t)q)));
-        v += u;
-      }
+    // lanes along the rows where those are adjacent, or the columns too few to fill a warp
+    const int cols = min(BN, N - n0), shift = __ffs(rows_here) - 1;
+    const bool by_row = ep.along_m || cols < 16;
+    for (int idx = t; idx < rows_here * (by_row ? cols : BN); idx += T::kThreads) {
+      const int r = r_first + (by_row ? idx & (rows_here - 1) : idx / BN);
+      const int c = by_row ? idx >> shift : idx % BN;
+      float v = sum1(r * pitch_r + c * pitch_c);
       if (roff[r] < 0 || coff[c] < 0) continue;
       if (raw) {
         pbase[(long long)(m0 + r) * N + n0 + c] = v;
@@ -527,7 +558,7 @@ inline SimtPlan plan_simt(long long M, long long N, long long K, long long Z) {
     const long long n = ((M + t.bm - 1) / t.bm) * ((N + t.bn - 1) / t.bn) * Z;
     for (int c = 1; c <= 8; c *= 2) {
       if (c > 1 && (K < 64LL * c || Z * c > 65535)) break;  // batches and splits share grid z
-      for (int p = 1; p <= 64; p *= 4) {
+      for (int p = 1; p <= 64; p *= 2) {
         if (p > 1 && (c < 8 || K < 256LL * c * p || Z * c * p > 65535)) break;
         const long long kps = (K + (long long)c * p - 1) / ((long long)c * p);
         const long long ctas = n * c * p;
@@ -592,6 +623,7 @@ int launch_simt_gemm(const char* name, const AL& al, const BL& bl, const EP& ep,
   FLB200_REQUIRE(M < 0x7fffffffLL && N < 0x7fffffffLL && K >= 0 && K < 0x7fffff00LL,
                  "%s: extent out of range", name);
   constexpr bool kBothK = k_layout(AL::kKind) && k_layout(BL::kKind);
+  constexpr bool kElem = AL::kKind >= kElemRows || BL::kKind >= kElemRows;
   SimtPlan p = plan_simt(M, N, K, Z);
   if (p.psplits > 1 && (!workspace || !aligned16(workspace) || workspace_bytes < p.workspace_bytes)) {
     // no scratch from the caller: the clusters alone share the K range
@@ -602,7 +634,17 @@ int launch_simt_gemm(const char* name, const AL& al, const BL& bl, const EP& ep,
   FLB200_REQUIRE(Z * p.csplits * p.psplits <= 65535, "%s: too many batches", name);
   float* partial = static_cast<float*>(workspace);
   int rc;
-  if (p.tile == 2) {
+  if constexpr (kElem) {
+    // more threads for the same tile: single elements cost a dozen instructions each, and half as many
+    // per thread hide twice the latency
+    if (p.tile == 2)
+      rc = launch_ffma<std::conditional_t<AL::kKind == kVecRow, FfmaTile<32, 32, 4, 2, 6>, FfmaTile<32, 32, 2, 4, 6>>>(
+          name, al, bl, ep, M, N, K, Z, p, partial, st);
+    else if (p.tile == 1)
+      rc = launch_ffma<FfmaTile<64, 64, 8, 4, 4>>(name, al, bl, ep, M, N, K, Z, p, partial, st);
+    else
+      rc = launch_ffma<FfmaTile<128, 64, 8, 4, 2>>(name, al, bl, ep, M, N, K, Z, p, partial, st);
+  } else if (p.tile == 2) {
     rc = launch_ffma<FfmaTile<32, 32, 4, 4, 8>>(name, al, bl, ep, M, N, K, Z, p, partial, st);
   } else if constexpr (kBothK) {
     rc = p.tile == 1

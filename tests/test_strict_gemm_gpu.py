@@ -30,6 +30,21 @@ def test_matmul_strict_loaders(mnk, a_k, b_k, offset):
     assert_close(c, a.double() @ b.double(), STRICT_TOL, f"matmul {mnk}")
 
 
+# results stored along their rows (four at a time where m and the strides allow it), with and without
+# a split of K, and added to
+@pytest.mark.parametrize("mnk", [(64, 33, 40), (36, 5, 2100), (130, 70, 100), (33, 20, 3000), (1, 40, 17), (128, 64, 20000)])
+@pytest.mark.parametrize("beta", [0.0, 0.5])
+def test_matmul_strict_transposed_result(mnk, beta):
+    from flashlight_b200 import _lib as L
+    from flashlight_b200 import functions as F
+    m, n, k = mnk
+    a, b, c = randn(m, k, seed=14), randn(k, n, seed=15), randn(n, m, seed=16)
+    got = c.cuda()
+    F.matmul(a.cuda(), b.cuda(), got, m=m, n=n, k=k, a_strides=(k, 1), b_strides=(n, 1), c_strides=(1, m), beta=beta,
+             math_mode=L.MATH_STRICT_F32)
+    assert_close(got, (a.double() @ b.double()).t() + beta * c.double(), STRICT_TOL, f"matmul {mnk}")
+
+
 # batches that fill grid z with and without a split of K beside them (65535 is the most)
 @pytest.mark.parametrize("zmnk", [(8192, 4, 4, 512), (9000, 5, 3, 1024), (40000, 1, 2, 128), (65535, 1, 1, 256)])
 def test_matmul_strict_many_batches(zmnk):
@@ -66,13 +81,16 @@ def test_conv_strict_filter_gradient_of_many_pixels():
 # N, C, H, W, Cout, kH, kW, stride, pad, groups: element loaders; repacked filter and channels-last
 # copy; channels not a multiple of 4; groups; a filter of many taps; stride with empty classes;
 # filters whose repacking needs more than the default shared memory, and more than there is; more
-# images than a grid's third extent
+# images than a grid's third extent; a channel per group; long sums of few pixels, in whole quads and
+# not; one output channel
 @pytest.mark.parametrize("case", [(2, 1, 9, 9, 8, 5, 5, 1, 2, 1), (16, 32, 14, 14, 64, 5, 5, 1, 2, 1),
                                   (8, 36, 13, 15, 44, 3, 3, 2, 1, 1), (16, 30, 14, 14, 66, 3, 3, 1, 1, 1),
                                   (16, 64, 12, 12, 64, 3, 3, 1, 1, 4), (2, 16, 1, 70, 24, 1, 13, 1, 0, 1),
                                   (40, 64, 17, 17, 256, 1, 1, 2, 0, 1), (8, 64, 30, 30, 64, 1, 1, 1, 0, 1),
                                   (2, 8, 1, 900, 16, 1, 401, 1, 0, 1), (2, 4, 1, 2500, 8, 1, 2001, 1, 0, 1),
-                                  (70000, 8, 1, 6, 16, 1, 3, 1, 0, 1)])
+                                  (70000, 8, 1, 6, 16, 1, 3, 1, 0, 1), (3, 24, 9, 11, 24, 3, 3, 1, 1, 24),
+                                  (5, 6, 17, 19, 6, 5, 5, 2, 2, 6), (1, 256, 4, 4, 64, 3, 3, 1, 1, 1),
+                                  (1, 130, 5, 3, 70, 3, 3, 1, 1, 1), (2, 20, 33, 31, 1, 3, 3, 1, 1, 1)])
 @pytest.mark.parametrize("channels_last", [False, True])
 def test_conv_strict_routes(case, channels_last):
     from flashlight_b200 import _lib as L
