@@ -1,5 +1,6 @@
 // Repacking of convolution filters: w[co][ci][tap] to out[tap * s_tap + co * s_co + ci * s_ci],
-// where one of s_co, s_ci is 1; the grid's z walks groups of Cout * C * RS words on both sides.  A
+// where one of s_co, s_ci is 1; the grid's z walks groups of Cout * C * RS words on both sides; `pad`
+// (at most 3) zeros follow each contiguous run of the target.  A
 // CTA brings 32 output channels x a short run of input channels x all taps into shared memory along
 // the filter's own contiguous order and writes it out along the contiguous index of the target, so
 // both sides move whole sectors; the runs are short (8 input channels) because most filters are
@@ -21,7 +22,7 @@ inline int permute_ci_shift(int RS) { return RS == 1 ? 5 : (RS <= 40 ? 3 : (RS <
 template <typename T>
 __global__ void __launch_bounds__(256)
 filter_permute_kernel(const T* __restrict__ w, T* __restrict__ out, int Cout, int C, int RS,
-                      unsigned rs_magic, int ci_shift, long long s_tap, long long s_co, long long s_ci) {
+                      unsigned rs_magic, int ci_shift, long long s_tap, long long s_co, long long s_ci, int pad) {
   extern __shared__ char permute_smem[];
   T* tile = reinterpret_cast<T*>(permute_smem);
   const int ci_run = 1 << ci_shift;
@@ -49,6 +50,7 @@ filter_permute_kernel(const T* __restrict__ w, T* __restrict__ out, int Cout, in
     for (int i = warp; i < run; i += 8) {  // one (ci, tap) per warp, lanes along co
       const int ci = over_rs(i), tap = i - ci * RS;
       if (lane < nco) out[tap * s_tap + lane + ci * s_ci] = tile[lane * pitch + i];
+      if (lane < pad && co0 + nco == Cout) out[tap * s_tap + nco + lane + ci * s_ci] = T(0);
     }
   } else {
     const int total = nco * RS << ci_shift;  // (co, tap, ci), ci fastest
@@ -56,15 +58,21 @@ filter_permute_kernel(const T* __restrict__ w, T* __restrict__ out, int Cout, in
     for (int e = threadIdx.x; e < total; e += 256) {
       const int ci = e & (ci_run - 1), i = e >> ci_shift, r = over_rs(i), tap = i - r * RS;
       if (ci < nci) out[tap * s_tap + r * s_co + ci] = tile[r * pitch + ci * RS + tap];
+      if (ci < pad && ci0 + nci == C) out[tap * s_tap + r * s_co + nci + ci] = T(0);
     }
   }
 }
 
 template <typename T>
 int filter_permute(const T* w, T* out, int Cout, int C, int RS, long long s_tap, long long s_co,
-                   long long s_ci, cudaStream_t st, int groups = 1) {
+                   long long s_ci, cudaStream_t st, int groups = 1, int pad = 0) {
   FLB200_REQUIRE(RS <= kPermuteMaxTaps, "filter_permute: %d taps do not fit", RS);
-  const int shift = permute_ci_shift(RS), run = 1 << shift;
+  int shift = permute_ci_shift(RS);
+  // few CTAs: shorter runs (64 x 64 filters of 31 taps: 8.6 us in 16 CTAs, 2.6 in 128), as long as the
+  // stores stay together, and `pad` threads are there for the zeros
+  const long long over_co = (Cout + kPermuteCo - 1) / kPermuteCo;
+  while (shift > (s_co == 1 ? 0 : 2) && over_co * ((C + (1 << shift) - 1) >> shift) * groups < 148) --shift;
+  const int run = 1 << shift;
   const size_t smem = (size_t)kPermuteCo * ((run * RS) | 1) * sizeof(T);
   if (smem > 48 * 1024)  // more than 380 taps
     FLB200_CUDA_CHECK(cudaFuncSetAttribute(filter_permute_kernel<T>,
@@ -73,7 +81,7 @@ int filter_permute(const T* w, T* out, int Cout, int C, int RS, long long s_tap,
             (unsigned)groups);
   FLB200_REQUIRE(grid.y <= 65535 && groups <= 65535, "filter_permute: too many channels");
   const unsigned magic = RS == 1 ? 0u : (unsigned)(((1ull << 32) + RS - 1) / RS);
-  filter_permute_kernel<T><<<grid, 256, smem, st>>>(w, out, Cout, C, RS, magic, shift, s_tap, s_co, s_ci);
+  filter_permute_kernel<T><<<grid, 256, smem, st>>>(w, out, Cout, C, RS, magic, shift, s_tap, s_co, s_ci, pad);
   FLB200_AFTER_LAUNCH("filter_permute");
   return FLB200_OK;
 }

@@ -173,9 +173,8 @@ int pack_filter(const ConvGeo& g, const float* w, float* out, int kp, bool rows_
   if (g.operand != tc::kOperandTf32)
     return filter_permute(reinterpret_cast<const uint16_t*>(w), reinterpret_cast<uint16_t*>(out), g.Cout,
                           g.C, g.RS, s_tap, s_co, s_ci, st);
-  if (kp != (rows_are_co ? g.C : g.Cout))  // (the copies of fl-order images are padded to 4 channels)
-    FLB200_CUDA_CHECK(cudaMemsetAsync(out, 0, (size_t)g.RS * rows * kp * 4, st));
-  return filter_permute(w, out, g.Cout, g.C, g.RS, s_tap, s_co, s_ci, st);
+  // (the copies of fl-order images are padded to 4 channels)
+  return filter_permute(w, out, g.Cout, g.C, g.RS, s_tap, s_co, s_ci, st, 1, kp - (rows_are_co ? g.C : g.Cout));
 }
 
 // gw[co][ci][tap] = sum over splits of partial[split][tap][co][ci]
