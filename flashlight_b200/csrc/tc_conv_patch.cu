@@ -193,19 +193,34 @@ __global__ void wgrad_reduce_kernel(const float* __restrict__ partial, T* __rest
   }
 }
 
-// The same for C a multiple of 4 and 16-byte aligned partial sums: a CTA owns 32 consecutive input
-// channels of one output channel and all taps; 16-byte loads of every split's slice (same order of
-// additions), and the result leaves through shared memory in the filter's own contiguous order,
-// instead of one word per tap stride.
+// The same for C a multiple of 4 and 16-byte aligned partial sums, 16-byte loads of every split's
+// slice (same order of additions).  One tap: the sums are in the filter's order.
 template <typename T>
-__global__ void __launch_bounds__(128)
+__global__ void __launch_bounds__(256)
+wgrad_reduce_flat_kernel(const float4* __restrict__ partial, T* __restrict__ gw, long long n4, int splits) {
+  for (long long t = (long long)blockIdx.x * blockDim.x + threadIdx.x; t < n4;
+       t += (long long)gridDim.x * blockDim.x) {
+    float4 s = make_float4(0.f, 0.f, 0.f, 0.f);
+#pragma unroll 4
+    for (int sp = 0; sp < splits; ++sp) {
+      const float4 v = partial[(long long)sp * n4 + t];
+      s.x += v.x; s.y += v.y; s.z += v.z; s.w += v.w;
+    }
+    tc::epi_store4(gw + 4 * t, s);
+  }
+}
+// Several taps: a CTA owns 32 consecutive input channels of one output channel and all taps, and the
+// result leaves through shared memory in the filter's own contiguous order, instead of one word per
+// tap stride.  (2048 x 512 filters of one tap: 22 us this way, 2.6 in the order they have.)
+template <typename T>
+__global__ void __launch_bounds__(256)
 wgrad_reduce_vec_kernel(const float4* __restrict__ partial, T* __restrict__ gw, int Cout, int C4,
                         int RS, int splits) {
   extern __shared__ float red_tile[];  // [tap][32 channels + 1]
   const int q0 = blockIdx.x * 8, co = blockIdx.y;
   const int nq = min(8, C4 - q0);
   const long long per_split = (long long)RS * Cout * C4;
-  for (int i = threadIdx.x; i < RS * 8; i += 128) {
+  for (int i = threadIdx.x; i < RS * 8; i += blockDim.x) {
     const int tap = i >> 3, q = i & 7;
     if (q >= nq) continue;
     const float4* src = partial + ((long long)tap * Cout + co) * C4 + q0 + q;
@@ -220,16 +235,21 @@ wgrad_reduce_vec_kernel(const float4* __restrict__ partial, T* __restrict__ gw, 
   }
   __syncthreads();
   T* dst = gw + ((long long)co * (4 * C4) + 4 * q0) * RS;
-  for (int i = threadIdx.x; i < 4 * nq * RS; i += 128)
+  for (int i = threadIdx.x; i < 4 * nq * RS; i += blockDim.x)
     dst[i] = Num<T>::from_f(red_tile[(i % RS) * 33 + i / RS]);
 }
 template <typename T>
 int wgrad_reduce(const float* partial, T* gw, const ConvGeo& g, int splits, cudaStream_t st) {
   const size_t smem = (size_t)g.RS * 33 * sizeof(float);
-  if (g.C % 4 == 0 && (reinterpret_cast<uintptr_t>(partial) & 15) == 0 && g.Cout <= 65535 &&
-      smem <= 48 * 1024)
-    wgrad_reduce_vec_kernel<T><<<dim3((unsigned)((g.C / 4 + 7) / 8), (unsigned)g.Cout), 128, smem, st>>>(
-        reinterpret_cast<const float4*>(partial), gw, g.Cout, g.C / 4, g.RS, splits);
+  const bool vec = g.C % 4 == 0 && (reinterpret_cast<uintptr_t>(partial) & 15) == 0;
+  const float4* p4 = reinterpret_cast<const float4*>(partial);
+  const long long n4 = (long long)g.Cout * g.C / 4;
+  if (vec && g.RS == 1 && (reinterpret_cast<uintptr_t>(gw) & (4 * sizeof(T) - 1)) == 0)
+    wgrad_reduce_flat_kernel<T><<<grid_for(n4, 256), 256, 0, st>>>(p4, gw, n4, splits);
+  else if (vec && g.Cout <= 65535 && smem <= 48 * 1024)
+    wgrad_reduce_vec_kernel<T><<<dim3((unsigned)((g.C / 4 + 7) / 8), (unsigned)g.Cout),
+                                 std::min(256, (g.RS * 8 + 31) / 32 * 32), smem, st>>>(
+        p4, gw, g.Cout, g.C / 4, g.RS, splits);
   else
     wgrad_reduce_kernel<T><<<grid_for((long long)g.RS * g.Cout * g.C, 256), 256, 0, st>>>(
         partial, gw, g.Cout, g.C, g.RS, splits);

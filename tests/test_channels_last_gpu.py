@@ -390,3 +390,38 @@ def test_first_convolution_ignores_what_scratch_held(L, case):
     assert L.lib.flb200_tc_kernel_launches() > before
     wgw, _ = R.conv2d_backward_filter_bias(gy.double(), x.double(), w.shape, False, *args)
     assert_close_scaled(gw, wgw, TF32_SCALED_TOL, "conv backward filter")
+
+
+@pytest.mark.parametrize("case", [(2, 17, 9, 10, 33, 3), (1, 31, 8, 8, 70, 1), (2, 18, 7, 9, 16, 5)])
+def test_padded_filters_ignore_what_scratch_held(L, case):
+    """fl's order with channels that are no multiple of 4: the repacked filter ends in zeros, whatever
+    the memory held (NaN here)."""
+    from flashlight_b200.extension import B200AutogradExtension
+    N, C, H, W, Cout, k = case
+    ext = B200AutogradExtension(math_mode=L.MATH_TF32, cache_layouts=False)
+    args = (1, 1, k // 2, k // 2, 1, 1, 1)
+    x, w = randn(N, C, H, W, seed=77), randn(Cout, C, k, k, seed=78)
+    want = R.conv2d(x.double(), w.double(), None, *args)
+    gy = randn(*want.shape, seed=79)
+    xd, gd, wd = x.cuda(), gy.cuda(), w.cuda()
+    for what, call, ref in (("conv forward", lambda: ext.conv2d(xd, wd, None, *args), want),
+                            ("conv dx", lambda: ext.conv2dBackwardData(gd, xd, wd, *args),
+                             R.conv2d_backward_data(gy.double(), x.shape, w.double(), *args))):
+        blocks = [torch.full((n,), float("nan"), device="cuda") for n in [1 << b for b in range(8, 22)] * 3]
+        del blocks
+        assert_close_scaled(call(), ref, TF32_SCALED_TOL, what)
+
+
+# one tap: the sums of the splits are in the filter's order already
+@pytest.mark.parametrize("dtype", [torch.float32, torch.float16])
+@pytest.mark.parametrize("case", [(9, 64, 20, 20, 24), (1, 128, 3, 3, 200), (4, 16, 30, 30, 16)])
+def test_filter_gradient_of_one_tap(L, case, dtype):
+    from flashlight_b200.extension import B200AutogradExtension
+    N, C, H, W, Cout = case
+    ext = B200AutogradExtension(math_mode=L.MATH_TF32)
+    args = (1, 1, 0, 0, 1, 1, 1)
+    x, gy = randn(N, C, H, W, seed=87).to(dtype), randn(N, Cout, H, W, seed=88).to(dtype)
+    w = torch.zeros(Cout, C, 1, 1, dtype=dtype, device="cuda")
+    gw, _ = ext.conv2dBackwardFilterBias(cl(gy), cl(x), w, None, *args)
+    wgw, _ = R.conv2d_backward_filter_bias(gy.double(), x.double(), w.shape, False, *args)
+    assert_close_scaled(gw.float(), wgw, TF32_SCALED_TOL, "conv backward filter")
