@@ -3,15 +3,15 @@
 // builds the chain out of whole-tensor operators and keeps the probabilities for the gradient
 // (flashlight/fl/autograd/Functions.cpp:1828-1891, 1021-1042); here the forward pass keeps only
 // the row-wise log-sum-exp of the scaled scores, and the backward kernel recomputes the
-// probabilities of // one 128 x 128 block at a time in tensor memory.
+// probabilities of one 128 x 128 block at a time in tensor memory.
 //
 // bf16 tensors of head dimension 64 and any length T, read and written in place through strides:
 // [batch * heads][T][64], or the packed projection [batch][T][3][heads][64] as its contraction left
 // it, which saves a reordering copy on each side.  Rows past T arrive as zeros from TMA, are masked
 // and never stored.
-// Backward: one CTA per (batch-head, block of 128 keys): K_j and V_j stay in shared memory, the CTA walks the query blocks i (i >= j with
-// the causal mask) and per block issues five tcgen05 contractions with fp32 accumulators in
-// tensor memory:
+// Backward: one CTA per (batch-head, block of 128 keys): K_j and V_j stay in shared memory, the CTA
+// walks the query blocks i (i >= j with the causal mask) and per block issues five tcgen05
+// contractions with fp32 accumulators in tensor memory:
 //     S  = Q_i K_j^T                    (128 x 128, K = 64)   columns   0..127
 //     dP = dO_i V_j^T                   (128 x 128, K = 64)   columns 128..255
 //     dV_j += P^T dO_i                  (128 x  64, K = 128)  columns 256..319   (kept over i)

@@ -460,9 +460,10 @@ inline bool tc_operands_aligned(const void* a, const void* b, const void* c, con
 
 // ---- 16-bit tensors ---------------------------------------------------------------------------
 // Casts between fp32 and 16-bit tensors, and f16 / bf16 convolutions (the reference accepts f16,
-// backend/cudnn/Conv2D.cpp:231,266,321) that the tensor cores do not read as they are: widen the operands into fp32 copies at the front of the workspace, run the fp32 operator
-// in the call's math mode (TF32 tensor cores keep 10 mantissa bits, as many as f16 has and more
-// than bf16), round the result once to the 16-bit type.  Accumulation is fp32 throughout.
+// backend/cudnn/Conv2D.cpp:231,266,321) that the tensor cores do not read as they are: widen the
+// operands into fp32 copies at the front of the workspace, run the fp32 operator in the call's math
+// mode (TF32 tensor cores keep 10 mantissa bits, as many as f16 has and more than bf16), round the
+// result once to the 16-bit type.  Accumulation is fp32 throughout.
 // Eight elements of 16-byte aligned tensors, or what is left of them, one by one elsewhere.
 template <typename T>
 __device__ __forceinline__ void widen8(const T* in, float* out) {

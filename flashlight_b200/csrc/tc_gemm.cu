@@ -36,8 +36,8 @@ static EncodeTiledFn encode_tiled_fn() {
   return fn;
 }
 
-// fp32 tensor map; dims[0] is the contiguous dimension, strides_bytes[i] belongs to
-// dims[i+1], box[0] must be 32 elements (128 bytes).  K-major operand tiles use the
+// Tensor map of fp32 or 16-bit elements (`operand`); dims[0] is the contiguous dimension,
+// strides_bytes[i] belongs to dims[i+1], box[0] is 128 bytes.  K-major operand tiles use the
 // 128-byte swizzle of 16-byte chunks, MN-major ones the swizzle of 32-byte chunks.
 int make_tensor_map(CUtensorMap* map, const void* base, int rank, const uint64_t* dims,
                     const uint64_t* strides_bytes, const uint32_t* box, int mode,

@@ -88,7 +88,8 @@ struct EpiloguePlan {
   void* pre;            // with act: where the value BEFORE the activation goes too (same type
                         // and layout as `out`; what the activation's gradient needs), or null
   float* stats;         // EpiStats matrix [ceil(M / 128) * 4][2 * N] (tc_kernel.cuh) or null:
-                        // per-column sums and sums of squares of a row-major fp32 output
+                        // per-column sums and sums of squares of a row-major output's values as
+                        // they are stored
 };
 
 // How an M x N contraction over k_iters stages and Z batches runs: tile width, whether CTA pairs
@@ -110,8 +111,8 @@ Launch plan_launch(long long M, long long N, long long k_iters, long long Z, boo
 // iterations per split, chosen so that tiles * splits fills whole rounds of the persistent grid.
 void plan_splits(long long tiles, long long k_iters, long long min_ips, int* splits, int* ips);
 
-// fp32 tensor map; dims[0] is the contiguous dimension, strides_bytes[i] belongs to
-// dims[i+1]; box[0] must be 32 elements.  mode: K-major operand tile (128-byte swizzle of
+// Tensor map of fp32 or 16-bit elements (`operand`); dims[0] is the contiguous dimension,
+// strides_bytes[i] belongs to dims[i+1]; box[0] is 128 bytes.  mode: K-major operand tile (128-byte swizzle of
 // 16-byte chunks), MN-major operand tile (TF32 operands with a contiguous m / n index need
 // the swizzle of 32-byte chunks), or an unswizzled staging tile for TMA stores.
 // elem_strides (optional) samples every s-th element of a dimension; the box extent of that

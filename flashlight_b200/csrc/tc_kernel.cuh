@@ -375,7 +375,7 @@ tc_persistent_kernel(const __grid_constant__ CUtensorMap map_a,
               // a * b ~ a_hi * b_hi + a_lo * b_hi + a_hi * b_lo with x = x_hi + x_lo, x_hi exact
               // in TF32: fp32-grade products out of three tensor-core passes
               const uint32_t off = s * SL::kStageBytes;
-  #pragma unroll
+#pragma unroll
               for (int j = 0; j < kBK / kUmmaK; ++j) {
                 const uint64_t ah = umma_desc_advance(a_desc0, off + j * a_jstep);
                 const uint64_t bh = umma_desc_advance(b_desc0, off + j * b_jstep);
@@ -390,11 +390,11 @@ tc_persistent_kernel(const __grid_constant__ CUtensorMap map_a,
               continue;
             }
             const int kn = min(KSUB, k1 - k);
-  #pragma unroll
+#pragma unroll
             for (int sub = 0; sub < KSUB; ++sub) {
               if (sub >= kn) break;
               const uint32_t off = (s * KSUB + sub) * SL::kStageBytes;
-  #pragma unroll
+#pragma unroll
               for (int j = 0; j < kBK / kUmmaK; ++j) {
                 const uint64_t ad = umma_desc_advance(a_desc0, off + j * a_jstep);
                 const uint64_t bd = umma_desc_advance(b_desc0, off + j * b_jstep);

@@ -207,11 +207,11 @@ tc_pair_kernel(const __grid_constant__ CUtensorMap map_a,
             }
             TC_PROF_ADD(m_full, w1);
             tc_fence_after();
-  #pragma unroll
+#pragma unroll
             for (int sub = 0; sub < KSUB; ++sub) {
               if (sub >= kn) break;
               const uint32_t off = (s * KSUB + sub) * SL::kStageBytes;
-  #pragma unroll
+#pragma unroll
               for (int j = 0; j < kBK / kUmmaK; ++j) {
                 const uint64_t ad = umma_desc_advance(a_desc0, off + j * a_jstep);
                 const uint64_t bd = umma_desc_advance(b_desc0, off + j * b_jstep);

@@ -1,6 +1,6 @@
 """The persistent LSTM / GRU recurrence (one kernel for all time steps of a layer and direction, the
-recurrent weights resident in shared memory, a grid-wide barrier per step) against the fp64
-oracle and against the one-kernel-per-step path, and the bounded wait of its barrier."""
+recurrent weights resident in shared memory, states exchanged as tagged words) against the fp64
+oracle and against the one-kernel-per-step path, and the bounded wait of its exchange."""
 import ctypes as C
 import os
 import subprocess
