@@ -283,8 +283,8 @@ rnn_sequence_kernel(const __grid_constant__ Launch<SeqJob> a) {
   if (threadIdx.x == 0) {
     mbar_init(w_bar, 1);
     mbar_init(done_bar, stages);
-    mbar_init(&recv_bar[0], 1);
-    mbar_init(&recv_bar[1], 1);
+    mbar_init(&recv_bar[0], 1 + kSeqThreads / 32);  // the byte count's, the warps'
+    mbar_init(&recv_bar[1], 1 + kSeqThreads / 32);
     *failed = 0;
     fence_barrier_init();
   }
@@ -345,15 +345,8 @@ rnn_sequence_kernel(const __grid_constant__ Launch<SeqJob> a) {
         (uint32_t)owner);
     const uint32_t push_bar = mapa_u32(smem_u32(recv_bar), (uint32_t)owner);
     const uint32_t recv_bytes = (uint32_t)(kUnits * G * quads * 16);
-    // A warp that loads no tile, pushes no row and updates no pair takes no part: nobody waits for it,
-    // so it could fall two phases behind a barrier that it only follows, and miss one.
-    const bool pushes = (warp & 3) < G && (warp >> 2) * (kHalf / 4) < quads;
-    bool updates = false;
-#pragma unroll
-    for (int it = 0; it < kItems; ++it) updates = updates || live[it];
-    const bool role = warp < stages || pushes || __any_sync(0xffffffffu, updates);
 
-    for (int step = 0; role && step < a.T && waits.warp_goes_on(); ++step) {
+    for (int step = 0; step < a.T && waits.warp_goes_on(); ++step) {
       const int t = job.reverse ? a.T - 1 - step : step;
       const int slot = step & 1;
       float* g_t = job.gates + (long long)t * a.B_total * G * H + group * kUnits + rank * kOwn;
@@ -388,7 +381,7 @@ rnn_sequence_kernel(const __grid_constant__ Launch<SeqJob> a) {
         if (lane == 0) issue_tile<false, NB>(tmem_base, a_desc0, b_desc0, warp, done_bar);
         __syncwarp();
       }
-      if (pushes && waits.warp_bar<false>(done_bar, step & 1)) {
+      if ((warp & 3) < G && waits.warp_bar<false>(done_bar, step & 1)) {
         tc_fence_after();
         const uint32_t at = push_at + (uint32_t)(slot * Recv<G, NB>::kFloats * 4);
         const uint32_t bar = push_bar + (uint32_t)(slot * 8);
@@ -405,6 +398,9 @@ rnn_sequence_kernel(const __grid_constant__ Launch<SeqJob> a) {
         }
         tc_fence_before();
       }
+      // Every warp counts for the step's barrier, those too that had no tile, row or pair to care for:
+      // one that only followed could fall behind by two phases and miss one.
+      if (lane == 0) mbar_arrive(&recv_bar[slot]);
       if (!waits.warp_bar<true>(&recv_bar[slot], (step >> 1) & 1)) break;
       const float* rp = recv + slot * Recv<G, NB>::kFloats;
       uint32_t* h_x = a.xch[ji] + (long long)slot * B * H + group * kUnits + rank * kOwn;
@@ -499,7 +495,7 @@ rnn_sequence_backward_kernel(const __grid_constant__ Launch<SeqBwdJob> a) {
   if (threadIdx.x == 0) {
     mbar_init(w_bar, 1);
     mbar_init(done_bar, stages);
-    mbar_init(read_bar, 2 * min(4, (H - mt * kBM + 31) / 32));
+    mbar_init(read_bar, kSeqThreads / 32);
     *failed = 0;
     fence_barrier_init();
   }
@@ -583,17 +579,10 @@ rnn_sequence_backward_kernel(const __grid_constant__ Launch<SeqBwdJob> a) {
     const long long slot_size = (long long)a.ctas * SL * block;
     const int row = (warp & 3) * 32 + lane;  // accumulator row = output of the tile
     const bool row_live = mt * kBM + row < H;
-    const bool warp_live = mt * kBM + (warp & 3) * 32 < H;
     unsigned long long* push = a.part[ji] + tile_at + ((long long)(row / units) * SL + rank) * block + 2 * (row % units);
     const unsigned long long* pull = a.part[ji] + tile_at + (long long)rank * SL * block;
 
-    // (a warp with no part in the steps stays out of them, as in the forward kernel)
-    bool updates = false;
-#pragma unroll
-    for (int it = 0; it < kItems; ++it) updates = updates || live[it];
-    const bool role = warp < stages || warp_live || __any_sync(0xffffffffu, updates);
-
-    for (int sb = 0; role && sb < a.T && waits.warp_goes_on(); ++sb) {
+    for (int sb = 0; sb < a.T && waits.warp_goes_on(); ++sb) {
       const int step = a.T - 1 - sb;
       const int t = job.reverse ? a.T - 1 - step : step;
       const int slot = sb & 1;
@@ -650,7 +639,9 @@ rnn_sequence_backward_kernel(const __grid_constant__ Launch<SeqBwdJob> a) {
       // the operand tiles may be overwritten, and the accumulators read, once the MMAs are done
       if (!waits.warp_bar<false>(done_bar, sb & 1)) break;
       const unsigned long long stamp = (unsigned long long)(sb + 1) << 32;
-      if (warp_live) {
+      // (all warps, those too whose rows lie past the end: one that only followed done_bar could fall two
+      // steps behind it and miss a phase)
+      {
         tc_fence_after();
         unsigned long long* to = push + slot * slot_size;
 #pragma unroll
