@@ -25,7 +25,6 @@ using namespace tc;
 
 constexpr int kSliceK = 256;                // K per CTA
 constexpr int kStagesK = kSliceK / kBK;     // 8 tiles of 32 k
-static_assert(kStagesK == kRnnTiles, "one accumulator per k tile");
 constexpr int kABytes = kBM * kBK * 4;      // 16 KB per k tile
 constexpr int kBBytes = 32 * kBK * 4;       // 4 KB per k tile (32 batch rows)
 constexpr int kPartStride = 33;             // floats per partial row (bank-conflict padding)
@@ -76,7 +75,7 @@ lstm_step_kernel(const __grid_constant__ CUtensorMap map_w,
     *failed = 0;
     fence_barrier_init();
   }
-  if (warp == 1) tmem_alloc(tmem_slot, 32 * kRnnTiles);
+  if (warp == 1) tmem_alloc(tmem_slot, 32 * kRnnAccs);
   tc_fence_before();
   __syncthreads();
   tc_fence_after();
@@ -96,7 +95,7 @@ lstm_step_kernel(const __grid_constant__ CUtensorMap map_w,
       tma_load(&map_h, &full_bar[lane], b_tiles + lane * kBBytes, 2, c);
     }
   } else if (warp == 1) {
-    if (lane == 0) {
+    if (elect_one()) {
       const uint32_t idesc = umma_idesc_tf32(32, 0, 0);
       const uint64_t a_desc0 = umma_desc(smem_u32(a_tiles), 16, 1024, 2);
       const uint64_t b_desc0 = umma_desc(smem_u32(b_tiles), 16, 1024, 2);
@@ -108,8 +107,8 @@ lstm_step_kernel(const __grid_constant__ CUtensorMap map_w,
         tc_fence_after();
 #pragma unroll
         for (int j = 0; j < kBK / kUmmaK; ++j)
-          umma_tf32(tmem_base + 32 * s, umma_desc_advance(a_desc0, s * kABytes + j * 32),
-                    umma_desc_advance(b_desc0, s * kBBytes + j * 32), idesc, j ? 1u : 0u);
+          umma_tf32(tmem_base + 32 * (s % kRnnAccs), umma_desc_advance(a_desc0, s * kABytes + j * 32),
+                    umma_desc_advance(b_desc0, s * kBBytes + j * 32), idesc, s >= kRnnAccs || j ? 1u : 0u);
       }
       umma_commit(done_bar);  // arrives when every MMA issued above (possibly none) is done
     }
@@ -122,7 +121,7 @@ lstm_step_kernel(const __grid_constant__ CUtensorMap map_w,
     float v[32], w[32];
     tmem_ld32(tmem_base + ((uint32_t)(quarter * 32) << 16), v);
 #pragma unroll
-    for (int q = 1; q < kRnnTiles; ++q) {
+    for (int q = 1; q < kRnnAccs; ++q) {
       tmem_ld32(tmem_base + 32 * q + ((uint32_t)(quarter * 32) << 16), w);
 #pragma unroll
       for (int j = 0; j < 32; ++j) v[j] += w[j];
@@ -164,7 +163,7 @@ lstm_step_kernel(const __grid_constant__ CUtensorMap map_w,
   cluster_sync_all();  // nobody leaves while a peer may still read its partial tile
   if (warp == 1) {
     tc_fence_after();
-    tmem_dealloc(tmem_base, 32 * kRnnTiles);
+    tmem_dealloc(tmem_base, 32 * kRnnAccs);
   }
 }
 

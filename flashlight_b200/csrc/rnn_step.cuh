@@ -8,9 +8,9 @@
 
 namespace flb200 {
 
-// k tiles of 32 that a CTA contracts per step, each into an accumulator of its own; the epilogue
-// adds them in order (rnn_sequence.cu says why).
-constexpr int kRnnTiles = 8;
+// Accumulators of a CTA's contraction per step, of every kRnnAccs-th k tile each; the epilogue adds
+// them in order (shared with rnn_sequence.cu, whose sums are the same bits).
+constexpr int kRnnAccs = 2;
 
 // TF32 mode on sm_100, batch <= 32, hidden size a multiple of 256 up to 2048.
 bool lstm_step_supported(int math_mode, int B, int H);

@@ -123,6 +123,39 @@ def test_persistent_other_cells_match_oracle(L, dims, with_state, mode):
         assert_close_scaled(dhx, wdhx, 5e-3, "persistent cell dhx")
 
 
+@pytest.mark.parametrize("cell,I,H,B,T,bidir", [
+    (R.RNN_LSTM, 16, 1020, 5, 4, True),    # 16 k tiles a CTA, most of them in tensor memory, the last one ragged
+    (R.RNN_GRU, 16, 516, 32, 3, True),     # 9 k tiles forward: one worker has two, the others one
+    (R.RNN_LSTM, 16, 1024, 33, 3, False),  # 48 rows a job
+    (R.RNN_LSTM, 16, 1024, 49, 3, False),  # two jobs of 25 and 24 rows side by side
+    (R.RNN_TANH, 16, 68, 48, 5, True),     # backward: pieces of 32 gate rows, five of eight empty
+    (R.RNN_GRU, 16, 4, 1, 6, False),       # the smallest
+])
+def test_persistent_sizes_off_the_tiles(L, cell, I, H, B, T, bidir):
+    """Every product rounds both operands to TF32 (2^-10 relative at most, truncated); over sums of up to
+    4096 products of either sign that stays within 5e-3 of the result's scale, as in the tests above."""
+    from flashlight_b200.extension import AutogradPayload, B200AutogradExtension, RNNGradData
+    dirs = 2 if bidir else 1
+    ext = B200AutogradExtension(math_mode=L.MATH_TF32)
+    w = randn(R.rnn_num_params(I, H, 1, cell, bidir), seed=60) * (0.5 / H ** 0.5)
+    x = randn(T, B, I, seed=61)
+    payload = AutogradPayload()
+    before = L.kernel_launches()
+    y, hy, _ = ext.rnn(x.cuda(), None, None, w.cuda(), H, 1, cell, bidir, 0.0, payload)
+    assert L.kernel_launches() - before <= 8 * dirs  # not a kernel per time step
+    wy, why, _ = R.rnn(x.double(), None, None, w.double(), H, 1, cell, bidir)
+    assert_close_scaled(y, wy, 5e-3, "y")
+    assert_close_scaled(hy, why, 5e-3, "hy")
+    gy = randn(T, B, dirs * H, seed=64)
+    dx, _, _, dw = ext.rnnBackward(x.cuda(), None, None, w.cuda(), RNNGradData(gy.cuda(), None, None), y,
+                                   1, H, cell, bidir, 0.0, payload)
+    wdx, _, _, wdw = R.rnn_backward(x.double(), None, None, w.double(), H, 1, cell, bidir, gy.double(),
+                                    None, None)
+    assert_close_scaled(dx, wdx, 5e-3, "dx")
+    assert_close_scaled(dw, wdw, 5e-3, "dw")
+    assert L.lib.flb200_tc_poll_status(torch.cuda.current_stream().cuda_stream) == L.OK
+
+
 def test_persistent_equals_per_step_path(L):
     """Same arithmetic, same order: the persistent kernel reproduces the per-step kernels bit
     for bit (the other path is selected in a child process, the switch is read once)."""
