@@ -73,7 +73,7 @@ tc_pair_kernel(const __grid_constant__ CUtensorMap map_a,
   uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(tempty_bar + 2);
   volatile int* failed = reinterpret_cast<volatile int*>(tmem_slot + 1);
 
-  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const int warp = __shfl_sync(0xffffffffu, threadIdx.x >> 5, 0), lane = threadIdx.x & 31;
   const uint32_t rank = cluster_ctarank();  // 0 = leader
   const int pair = blockIdx.x >> 1, n_pairs = gridDim.x >> 1;
   constexpr uint32_t kTmemCols = 2 * BN;
@@ -163,7 +163,7 @@ tc_pair_kernel(const __grid_constant__ CUtensorMap map_a,
       }
     }
   } else if (warp == 1) {
-    if (lane == 0 && rank == 0) {
+    if (rank == 0 && elect_one()) {
       const bool half = prob.operand != kOperandTf32;
       const uint32_t idesc =
           half ? umma_idesc_f16_pair(prob.operand, BN, prob.a_mn_major, prob.b_mn_major)

@@ -110,11 +110,10 @@ struct PatchConvProblem {
   }
   __device__ __forceinline__ void load_pair(const CUtensorMap* ma, const CUtensorMap* mb,
                                             const Tile& t, LoadState& ls, uint32_t full_bar,
-                                            char* a_dst, char* b_dst, int rank, int lane) const {
-    if (lane == 0) {
+                                            char* a_dst, char* b_dst, int rank, int) const {
+    if (elect_one()) {
       int ca[4] = {ls.cc * kel, ls.aw, ls.ah, t.b0};
       tma_load_pair(ma, full_bar, a_dst, 4, ca);
-    } else if (lane == 1) {
       int cb[4] = {ls.cc * kel, t.n0 + rank * (BN / 2), ls.wtap, 0};  // this CTA's half of B
       tma_load_pair(mb, full_bar, b_dst, 3, cb);
     }
