@@ -379,7 +379,7 @@ int tc_conv_backward_data(const ConvGeo& g, const float* gy, const float* w, flo
       const uint64_t strides[2] = {(uint64_t)g.C * 4, 128};
       const uint32_t box[3] = {32, 32, (uint32_t)(L.bn / 32)};
       if (int rc = tc::make_tensor_map(&mb, w, 3, dims, strides, box, tc::kMapMnMajor)) return rc;
-      pb.rank = 3; pb.mn_dim = 2; pb.k_dim = 1; pb.mn_grouped = 1;
+      pb.rank = 3; pb.mn_dim = 2; pb.k_dim = 1; pb.mn_grouped = 5;
     } else if (int rc = map2d(&mb, w, g.C, g.Cout, g.C, 32, true)) {
       return rc;
     }

@@ -335,7 +335,8 @@ static Launch compute_launch(long long M, long long N, long long k_iters, long l
       if (k_iters < 4) continue;
     }
     double clocks = w.clocks * (x3 ? 2.5 : 1.0);
-    // issuing a TMA copy takes a producer warp ~120 clocks, and there are two of them
+    // issuing a TMA copy takes a producer warp ~120 clocks, and there are two of them (the boxes of a
+    // grouped MN-major operand are one copy; counting them so changed no choice by more than noise)
     const int copies = (a_mn_major ? kBM / box : 1) +
                        (b_mn_major ? (w.pairs ? w.bn / 2 : w.bn) / box : 1);
     if (clocks < copies * 65.0) clocks = copies * 65.0;
@@ -483,15 +484,24 @@ int build_operand(const Side& s, const void* base, long long rows, long long K, 
   const bool half = operand != tc::kOperandTf32;
   const uint32_t kstage = tc::stage_k(operand);  // elements of K per stage (128 bytes)
   const uint64_t esize = half ? 2 : 4;
-  uint64_t dims[3], strides[2];
-  uint32_t box[3];
+  uint64_t dims[4], strides[3];
+  uint32_t box[4];
   *plan = tc::OperandPlan{};
   plan->k_inner = 0;
   plan->k2_dim = -1;
+  int rank = 2;
   if (s.mn_major) {
-    dims[0] = (uint64_t)rows; dims[1] = (uint64_t)K;
     box[0] = half ? 64 : 32; box[1] = kstage;
+    dims[0] = (uint64_t)rows; dims[1] = (uint64_t)K;
     plan->mn_major = 1; plan->mn_dim = 0; plan->k_dim = 1;
+    if (rows % box[0] == 0) {
+      dims[0] = box[0]; dims[2] = (uint64_t)rows / box[0];
+      strides[1] = box[0] * esize;
+      box[2] = (uint32_t)tile_rows / box[0];
+      plan->mn_dim = 2;
+      plan->mn_grouped = half ? 6 : 5;
+      rank = 3;
+    }
   } else {
     dims[0] = (uint64_t)K; dims[1] = (uint64_t)rows;
     box[0] = kstage; box[1] = (uint32_t)tile_rows;
@@ -499,14 +509,12 @@ int build_operand(const Side& s, const void* base, long long rows, long long K, 
   }
   plan->k_elems = (int)kstage;
   strides[0] = (uint64_t)s.ld * esize;
-  int rank = 2;
   plan->z_dim = -1;
   if (batch > 1) {
-    dims[2] = (uint64_t)batch;
-    strides[1] = (uint64_t)batch_stride * esize;
-    box[2] = 1;
-    rank = 3;
-    plan->z_dim = 2;
+    dims[rank] = (uint64_t)batch;
+    strides[rank - 1] = (uint64_t)batch_stride * esize;
+    box[rank] = 1;
+    plan->z_dim = rank++;
   }
   plan->rank = rank;
   // 16-bit tiles use the plain 128-byte swizzle for both majors

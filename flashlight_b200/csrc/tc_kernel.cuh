@@ -5,10 +5,10 @@
 // One CTA per SM walks a static list of 128 x BN output tiles:
 //   warp 0   : TMA producer — issues cp.async.bulk.tensor loads (never multicast) into a
 //              STAGES-deep ring of 128-byte-swizzled shared-memory tiles and runs ahead into
-//              the next output tile while the current one drains.  Lane 0 owns the
-//              barriers; every lane issues at most one copy per stage, so the boxes of a
-//              stage go out together.  Per-stage work is a handful of multiply-adds:
-//              coordinates advance incrementally.
+//              the next output tile while the current one drains.  One elected lane owns the
+//              barriers and issues the copies; per stage it adds to the coordinates and no more,
+//              since a stage's MMAs take only 160 to 512 clocks.  (A lane per copy, coordinates
+//              by multiplication: 470 clocks per stage of two copies, 730 of four.)
 //   warp 1   : allocates TMEM (2 accumulators of BN columns); one lane issues tcgen05.mma
 //              for each ready stage and tcgen05.commit to free the stage / publish the tile
 //   warps 6-9: only in the 3xTF32 instantiation (fp32-grade products): split every landed
@@ -26,7 +26,7 @@
 //
 // A problem policy P tells the skeleton what a tile is:
 //   int  a_mn_major, b_mn_major, operand;   // operand: kOperandTf32 / kOperandBf16 / kOperandF16
-//   static constexpr bool kWarpProducer;  // load() is called by the whole warp (else lane 0)
+//   static constexpr bool kTwoProducers;  // a producer warp per operand, else one for both
 //   static constexpr int kMinBlocks;      // second argument of tc_persistent_kernel's launch
 //                                         // bounds: 1 = the register allocator may use the whole
 //                                         // file for the one resident CTA, 0 = its own choice
@@ -34,12 +34,12 @@
 //   __device__ int  num_tiles() const;
 //   __device__ void decode(int tile, Tile&) const;
 //   __device__ int  k_begin(const Tile&) const;  __device__ int k_end(const Tile&) const;
-//   __device__ void load_begin(const Tile&, LoadState&, int copy) const;   // once per tile;
-//                        // copy = index of the stage's copy this lane will issue
+//   template <int kWhich> __device__ void load_begin(const Tile&, LoadState&) const;   // once per tile
+//   __device__ uint32_t stage_bytes(const Tile&) const;   // that the copies of a stage bring
+//   template <int kWhich>
 //   __device__ void load(const CUtensorMap* a, const CUtensorMap* b, const Tile&, LoadState&,
-//                        uint64_t* bar, char* a_dst, char* b_dst, int lane) const;
-//                        // one stage, called by the whole warp: lane 0 posts the byte count,
-//                        // lane i issues copy i; every lane advances its LoadState
+//                        uint64_t* bar, char* a_dst, char* b_dst) const;
+//                        // one stage: issues the copies and advances the LoadState
 //   __device__ bool chunk_live(const Tile&, int c0) const;                // warp-uniform
 //   __device__ void store(const Tile&, int row, int c0, const float* v, float* stage,
 //                         int lane) const;   // 32 columns of row `row`; called by all 32 lanes
@@ -153,10 +153,9 @@ struct SmemLayout {
 constexpr int stages_for(int bn) { return bn >= 256 ? 4 : (bn >= 128 ? 6 : (bn >= 64 ? 8 : 10)); }
 constexpr int stages_for_x3(int bn) { return bn >= 256 ? 2 : (bn >= 128 ? 3 : (bn >= 64 ? 4 : 5)); }
 constexpr int kThreadsX3 = kThreads + 128;  // four more warps split the operands
-// Policies whose stage is several copies get a second producer warp (warp 6): issuing one TMA
-// copy costs the issuing warp ~110-130 clocks and copies issued from different lanes of one
-// warp still go out one after the other, so a stage of 5 to 12 copies took 650 to 1500 clocks
-// to issue against ~500 clocks of MMAs; two warps issue the even and the odd copies.
+// The copies of a stage: of one operand or of both.  Policies whose operands may be several boxes per
+// stage have a producer warp for each (warps 0 and 6).
+enum { kA = 0, kB = 1, kBoth = 2 };
 // Tiles of 128 or more columns get a second group of four epilogue warps (each group drains
 // every other 32-column chunk of the accumulator): with one group, shapes with a short K loop
 // and a large output (1x1 layers on 56x56 planes: 2 K blocks per 128 KB tile) were bound by the
@@ -164,12 +163,12 @@ constexpr int kThreadsX3 = kThreads + 128;  // four more warps split the operand
 template <int X3, int BN>
 constexpr int epilogue_groups() { return (X3 == 0 && BN >= 128) ? 2 : 1; }
 template <class P, int X3>
-constexpr int second_epilogue_first_warp() { return P::kWarpProducer && X3 == 0 ? 7 : 6; }
+constexpr int second_epilogue_first_warp() { return P::kTwoProducers && X3 == 0 ? 7 : 6; }
 template <class P, int X3, int BN>
 constexpr int threads_for() {
   if (X3) return kThreadsX3;
   if (epilogue_groups<X3, BN>() == 2) return (second_epilogue_first_warp<P, X3>() + 4) * 32;
-  return P::kWarpProducer ? kThreads + 32 : kThreads;
+  return P::kTwoProducers ? kThreads + 32 : kThreads;
 }
 
 __device__ __forceinline__ void mbar_arrive(uint64_t* bar) {
@@ -241,66 +240,20 @@ tc_persistent_kernel(const __grid_constant__ CUtensorMap map_a,
   tc_fence_after();
   const uint32_t tmem_base = *tmem_slot;
 
-  constexpr bool kTwoProducers = P::kWarpProducer && X3 == 0;
-  if (warp == 0 || (kTwoProducers && warp == 6)) {
-    uint32_t s = 0, round = 0;
-    typename P::Tile t;
-    typename P::LoadState ls;
-    // part / parts: this warp issues the copies whose index is congruent to part mod parts;
-    // part 0 also posts the stage's byte count
-    const int part = warp == 0 ? 0 : 1;
-    constexpr int parts = kTwoProducers ? 2 : 1;
-    if constexpr (P::kWarpProducer) {
-      // All 32 lanes walk the loop: lane 0 waits for the stage to be free and posts the byte
-      // count, then each lane issues one of the stage's copies (a single instruction for
-      // the warp), so a stage made of many boxes costs the same issue time as a small one.
-      bool live = true;
-      TC_PROF_VAR(p_wait);
-      TC_PROF_NOW(p_t0);
-      for (int tile = blockIdx.x; live && tile < n_tiles; tile += gridDim.x) {
-        int stop = 0;
-        if (lane == 0) stop = *failed;
-        if (__shfl_sync(0xffffffffu, stop, 0) != 0) break;
-        prob.decode(tile, t);
-        prob.load_begin(t, ls, lane * parts + part);  // the index of the copy this lane issues
-        const int k1 = prob.k_end(t);
-        for (int k = prob.k_begin(t); k < k1; k += KSUB) {
-          int ok = 1;
-          TC_PROF_NOW(w0);
-          if (lane == 0 && round > 0 && !mbar_wait(&empty_bar[s], (round - 1) & 1)) {
-            *failed = 1;
-            ok = 0;
-          }
-          TC_PROF_ADD(p_wait, w0);
-          if (__shfl_sync(0xffffffffu, ok, 0) == 0) {
-            live = false;
-            break;
-          }
-          const int kn = min(KSUB, k1 - k);
-#pragma unroll
-          for (int sub = 0; sub < KSUB; ++sub) {
-            if (sub >= kn) break;
-            char* a_dst = tiles + (s * KSUB + sub) * SL::kStageBytes;
-            prob.load(&map_a, &map_b, t, ls, &full_bar[s], a_dst, a_dst + SL::kABytes, lane,
-                      sub == kn - 1, part, parts);
-          }
-          if (++s == NG) { s = 0; ++round; }
-        }
-      }
-#ifdef FLB200_TC_PROFILE
-      if (lane == 0 && part == 0) { TC_PROF_PUT(0, p_wait); TC_PROF_PUT(1, clock64() - p_t0); }
-#endif
-    } else if (elect_one()) {
-      // Two copies per stage: one lane does everything and the loop has no warp exchange.  (Elected,
-      // not lane 0, like the MMA issuer: 3x3 convolutions of 256 images of 56 x 56 x 64 take 191 us
-      // instead of 227, of 8 images with 32-column tiles 18 instead of 24.  For the policies
-      // with a copy per lane, one elected lane that issues them all measured 3 to 13 % slower: their
-      // coordinates are not carried from stage to stage.)
+  constexpr bool kTwo = P::kTwoProducers && X3 == 0;
+  if (warp == 0 || (kTwo && warp == 6)) {
+    // One elected lane waits for a group of stages to be free, posts its byte count (not kB) and issues
+    // the copies: of both operands, or of one where the policy has two producers.
+    auto produce = [&](auto which) {
+      constexpr int kWhich = decltype(which)::value;
+      uint32_t s = 0, round = 0;
+      typename P::Tile t;
+      typename P::LoadState ls;
       TC_PROF_VAR(p_wait);
       TC_PROF_NOW(p_t0);
       for (int tile = blockIdx.x; tile < n_tiles && *failed == 0; tile += gridDim.x) {
         prob.decode(tile, t);
-        prob.load_begin(t, ls, 0);
+        prob.template load_begin<kWhich>(t, ls);
         const int k1 = prob.k_end(t);
         for (int k = prob.k_begin(t); k < k1; k += KSUB) {
           TC_PROF_NOW(w0);
@@ -314,15 +267,23 @@ tc_persistent_kernel(const __grid_constant__ CUtensorMap map_a,
           for (int sub = 0; sub < KSUB; ++sub) {
             if (sub >= kn) break;
             char* a_dst = tiles + (s * KSUB + sub) * SL::kStageBytes;
-            prob.load(&map_a, &map_b, t, ls, &full_bar[s], a_dst, a_dst + SL::kABytes, 0,
-                      sub == kn - 1, 0, 1);
+            if constexpr (kWhich != kB) mbar_post_tx(&full_bar[s], prob.stage_bytes(t), sub == kn - 1);
+            prob.template load<kWhich>(&map_a, &map_b, t, ls, &full_bar[s], a_dst, a_dst + SL::kABytes);
           }
           if (++s == NG) { s = 0; ++round; }
         }
       }
 #ifdef FLB200_TC_PROFILE
-      TC_PROF_PUT(0, p_wait); TC_PROF_PUT(1, clock64() - p_t0);
+      if (kWhich != kB) { TC_PROF_PUT(0, p_wait); TC_PROF_PUT(1, clock64() - p_t0); }
 #endif
+    };
+    if (elect_one()) {
+      if constexpr (kTwo) {
+        if (warp == 0) produce(std::integral_constant<int, kA>{});
+        else produce(std::integral_constant<int, kB>{});
+      } else {
+        produce(std::integral_constant<int, kBoth>{});
+      }
     }
   } else if (warp == 1) {
     if (elect_one()) {
@@ -520,7 +481,7 @@ tc_persistent_kernel(const __grid_constant__ CUtensorMap map_a,
 // together share the (large) A tile through L2.
 template <int BN>
 struct GemmProblem {
-  static constexpr bool kWarpProducer = true;
+  static constexpr bool kTwoProducers = true;
   static constexpr int kMinBlocks = 1;
   int operand;  // kOperandTf32, or 16-bit (64 elements per stage)
   OperandCoords a, b;
@@ -532,7 +493,8 @@ struct GemmProblem {
   float* partial;  // split-K scratch [z*splits + s][M][N]
 
   struct Tile { int m0, n0, z, split, k0, k1; };
-  struct LoadState { int a_lo, a_hi, b_lo, b_hi; };
+  struct Walk { int c[4], lo; };  // coordinates of an operand's first box, stage of the inner k level
+  struct LoadState { Walk a, b; };
 
   __device__ __forceinline__ int num_tiles() const { return tiles_m * tiles_n * Z * splits; }
   __device__ __forceinline__ void decode(int tile, Tile& t) const {
@@ -546,36 +508,67 @@ struct GemmProblem {
   }
   __device__ __forceinline__ int k_begin(const Tile& t) const { return t.k0; }
   __device__ __forceinline__ int k_end(const Tile& t) const { return t.k1; }
-  __device__ __forceinline__ void load_begin(const Tile& t, LoadState& ls, int) const {
-    ls.a_hi = a.k_inner > 0 ? t.k0 / a.k_inner : 0;
-    ls.a_lo = t.k0 - ls.a_hi * a.k_inner;
-    ls.b_hi = b.k_inner > 0 ? t.k0 / b.k_inner : 0;
-    ls.b_lo = t.k0 - ls.b_hi * b.k_inner;
+  static __device__ __forceinline__ void walk_begin(const OperandCoords& o, Walk& w, int mn, const Tile& t) {
+    const int hi = o.k_inner > 0 ? t.k0 / o.k_inner : 0;
+    w.lo = t.k0 - hi * o.k_inner;
+    operand_coords(o, mn, w.lo, hi, t.z, w.c);
   }
-  __device__ __forceinline__ void load(const CUtensorMap* ma, const CUtensorMap* mb,
-                                       const Tile& t, LoadState& ls, uint64_t* bar, char* a_dst,
-                                       char* b_dst, int lane, bool last, int part,
-                                       int parts) const {
-    if (lane == 0 && part == 0) mbar_post_tx(bar, (kBM + BN) * kBK * 4, last);
-    __syncwarp();
-    // a K-major operand is one box, an MN-major one a box per 32 rows: copies [0, na) are A,
-    // [na, na + nb) are B; copy i is issued by lane i / parts of producer warp i % parts
+  // Boxes [first, first + count) of an operand's stage.  A K-major operand is one box, an MN-major one a
+  // box per 32 (16-bit: 64) rows, or one copy of them all where the map is grouped.
+  template <bool kPair, int kRank, class Bar>
+  __device__ __forceinline__ void copy_boxes(const OperandCoords& o, const CUtensorMap* map, Bar bar, char* dst,
+                                             const Walk& w, int first, int count) const {
     const int box_mn = operand ? 64 : 32, box_bytes = operand ? 8192 : kBK * 128;
-    const int na = a_mn_major && !a.mn_shift ? kBM / box_mn : 1;
-    const int nb = b_mn_major && !b.mn_shift ? BN / box_mn : 1;  // grouped: one copy
-    const int copy = lane * parts + part;
-    if (copy < na) {
-      int c[4];
-      operand_coords(a, t.m0 + box_mn * copy, ls.a_lo, ls.a_hi, t.z, c);
-      tma_load(ma, bar, a_dst + copy * box_bytes, a.rank, c);
-    } else if (copy < na + nb) {
-      const int j = copy - na;
-      int c[4];
-      operand_coords(b, t.n0 + box_mn * j, ls.b_lo, ls.b_hi, t.z, c);
-      tma_load(mb, bar, b_dst + j * box_bytes, b.rank, c);
+    int c[4];
+#pragma unroll
+    for (int d = 0; d < kRank; ++d) c[d] = w.c[d] + first * box_mn * o.mn_mul[d];
+    dst += first * box_bytes;
+    for (int i = 0;;) {
+      if constexpr (kPair) tma_load_pair(map, bar, dst, kRank, c);
+      else tma_load(map, bar, dst, kRank, c);
+      if (++i >= count) break;
+      dst += box_bytes;
+#pragma unroll
+      for (int d = 0; d < kRank; ++d) c[d] += box_mn * o.mn_mul[d];
     }
-    if (++ls.a_lo == a.k_inner) { ls.a_lo = 0; ++ls.a_hi; }
-    if (++ls.b_lo == b.k_inner) { ls.b_lo = 0; ++ls.b_hi; }
+  }
+  template <bool kPair, class Bar>
+  __device__ __forceinline__ void walk_load(const OperandCoords& o, const CUtensorMap* map, Bar bar, char* dst,
+                                            Walk& w, int first, int count) const {
+    if (o.rank == 2) copy_boxes<kPair, 2>(o, map, bar, dst, w, first, count);
+    else if (o.rank == 3) copy_boxes<kPair, 3>(o, map, bar, dst, w, first, count);
+    else copy_boxes<kPair, 4>(o, map, bar, dst, w, first, count);
+#pragma unroll
+    for (int d = 0; d < 4; ++d) w.c[d] += o.k_mul[d];
+    if (++w.lo == o.k_inner) {
+      w.lo = 0;
+#pragma unroll
+      for (int d = 0; d < 4; ++d) w.c[d] += o.k2_mul[d] - o.k_inner * o.k_mul[d];
+    }
+  }
+  __device__ __forceinline__ int boxes_of(const OperandCoords& o, int rows) const {
+    return o.mn_major && !o.mn_shift ? rows / (operand ? 64 : 32) : 1;
+  }
+  // Of two producers A's takes the last boxes of B where B has more than A.
+  template <int kWhich, bool kPair, class Bar>
+  __device__ __forceinline__ void load_stage(const CUtensorMap* ma, const CUtensorMap* mb, LoadState& ls, Bar bar,
+                                             char* a_dst, char* b_dst, int b_rows) const {
+    const int na = boxes_of(a, kBM), nb = boxes_of(b, b_rows);
+    const int moved = kWhich == kBoth ? 0 : max(0, (nb - na) >> 1);
+    if constexpr (kWhich != kB) walk_load<kPair>(a, ma, bar, a_dst, ls.a, 0, na);
+    if (kWhich != kA) walk_load<kPair>(b, mb, bar, b_dst, ls.b, 0, nb - moved);
+    else if (moved > 0) walk_load<kPair>(b, mb, bar, b_dst, ls.b, nb - moved, moved);
+  }
+  template <int kWhich>
+  __device__ __forceinline__ void load_begin(const Tile& t, LoadState& ls) const {
+    if constexpr (kWhich != kB) walk_begin(a, ls.a, t.m0, t);
+    walk_begin(b, ls.b, t.n0, t);
+  }
+  __device__ __forceinline__ uint32_t stage_bytes(const Tile&) const { return (kBM + BN) * kBK * 4; }
+  template <int kWhich>
+  __device__ __forceinline__ void load(const CUtensorMap* ma, const CUtensorMap* mb, const Tile&,
+                                       LoadState& ls, uint64_t* bar, char* a_dst, char* b_dst) const {
+    load_stage<kWhich, false>(ma, mb, ls, bar, a_dst, b_dst, BN);
   }
   // CTA pairs (tc_pair.cuh): the halves of a pair tile are two consecutive 128-row blocks of
   // the same column block, batch and K slice; row blocks run fastest, then splits, columns,
@@ -600,25 +593,17 @@ struct GemmProblem {
     t.k0 = t.split * iters_per_split;
     t.k1 = min(t.k0 + iters_per_split, k_iters);
   }
-  __device__ __forceinline__ void load_pair(const CUtensorMap* ma, const CUtensorMap* mb,
-                                            const Tile& t, LoadState& ls, uint32_t full_bar,
-                                            char* a_dst, char* b_dst, int rank, int copy) const {
-    // this CTA's 128 rows of A and its BN/2 columns of B; `copy` = which of the stage's copies
-    // the calling lane issues
-    const int box_mn = operand ? 64 : 32, box_bytes = operand ? 8192 : kBK * 128;
-    const int na = a_mn_major ? kBM / box_mn : 1, nb = b_mn_major ? (BN / 2) / box_mn : 1;
-    if (copy < na) {
-      int c[4];
-      operand_coords(a, t.m0 + box_mn * copy, ls.a_lo, ls.a_hi, t.z, c);
-      tma_load_pair(ma, full_bar, a_dst + copy * box_bytes, a.rank, c);
-    } else if (copy < na + nb) {
-      const int j = copy - na;
-      int c[4];
-      operand_coords(b, t.n0 + rank * (BN / 2) + box_mn * j, ls.b_lo, ls.b_hi, t.z, c);
-      tma_load_pair(mb, full_bar, b_dst + j * box_bytes, b.rank, c);
-    }
-    if (++ls.a_lo == a.k_inner) { ls.a_lo = 0; ++ls.a_hi; }
-    if (++ls.b_lo == b.k_inner) { ls.b_lo = 0; ++ls.b_hi; }
+  // this CTA's 128 rows of A and its BN / 2 columns of B
+  template <int kWhich>
+  __device__ __forceinline__ void load_begin_pair(const Tile& t, LoadState& ls, int rank) const {
+    if constexpr (kWhich != kB) walk_begin(a, ls.a, t.m0, t);
+    walk_begin(b, ls.b, t.n0 + rank * (BN / 2), t);
+  }
+  template <int kWhich>
+  __device__ __forceinline__ void load_pair(const CUtensorMap* ma, const CUtensorMap* mb, const Tile&,
+                                            LoadState& ls, uint32_t full_bar, char* a_dst,
+                                            char* b_dst) const {
+    load_stage<kWhich, true>(ma, mb, ls, full_bar, a_dst, b_dst, BN / 2);
   }
   __device__ __forceinline__ bool chunk_live(const Tile& t, int c0) const {
     return t.n0 + c0 < N;

@@ -22,10 +22,10 @@
 // A policy used here adds to the interface of tc_kernel.cuh:
 //   __device__ int  num_pair_tiles() const;
 //   __device__ void decode_pair(int pair_tile, int rank, Tile&) const;  // this CTA's half
+//   template <int kWhich> __device__ void load_begin_pair(const Tile&, LoadState&, int rank) const;
+//   template <int kWhich>
 //   __device__ void load_pair(const CUtensorMap* a, const CUtensorMap* b, const Tile&, LoadState&,
-//                             uint32_t full_bar_cluster_addr, char* a_dst, char* b_dst,
-//                             int rank, int lane) const;
-//                             // called by the whole producer warp; lane i issues copy i.
+//                             uint32_t full_bar_cluster_addr, char* a_dst, char* b_dst) const;
 //                             // A: this CTA's 128 rows; B: rows n0 + rank * BN/2 ...
 #pragma once
 #include <cuda_runtime.h>
@@ -47,11 +47,11 @@ struct PairSmemLayout {
 };
 constexpr int pair_stages_for(int bn) { return bn >= 256 ? 6 : 8; }
 
-// Threads: the six warps of tc_kernel.cuh plus, for policies whose stage is several copies, a
-// second producer warp (warp 6) that issues every other copy.
+// Threads: the six warps of tc_kernel.cuh plus, for policies with two producers, the second one
+// (warp 6).
 // ... and a second group of four epilogue warps (see tc_kernel.cuh) behind them.
 template <class P>
-constexpr int pair_second_epilogue_first_warp() { return P::kWarpProducer ? 7 : 6; }
+constexpr int pair_second_epilogue_first_warp() { return P::kTwoProducers ? 7 : 6; }
 template <class P>
 constexpr int pair_threads_for() { return (pair_second_epilogue_first_warp<P>() + 4) * 32; }
 
@@ -98,68 +98,62 @@ tc_pair_kernel(const __grid_constant__ CUtensorMap map_a,
   tc_fence_after();
   const uint32_t tmem_base = *tmem_slot;
 
-  constexpr bool kTwoProducers = P::kWarpProducer;
-  if (warp == 0 || (kTwoProducers && warp == 6)) {
-    // The whole warp walks the loop (see tc_kernel.cuh): lane 0 owns the barriers, lane i
-    // issues copy i * parts + part of the stage; the leader's part 0 posts the byte count.
-    const int part = warp == 0 ? 0 : 1;
-    constexpr int parts = kTwoProducers ? 2 : 1;
-    uint32_t s = 0, round = 0;
-    typename P::Tile t;
-    typename P::LoadState ls;
-    bool live = true;
-    TC_PROF_VAR(p_wait);
-    TC_PROF_NOW(p_t0);
-    for (int tile = pair; live && tile < n_tiles; tile += n_pairs) {
-      int stop = 0;
-      if (lane == 0) stop = *failed;
-      if (__shfl_sync(0xffffffffu, stop, 0) != 0) {
-        live = false;
-        break;
-      }
-      prob.decode_pair(tile, (int)rank, t);
-      prob.load_begin(t, ls, lane * parts + part);
-      const int k1 = prob.k_end(t);
-      for (int k = prob.k_begin(t); k < k1; k += KSUB) {
-        const int kn = min(KSUB, k1 - k);
-        int ok = 1;
-        TC_PROF_NOW(w0);
-        if (lane == 0) {
+  constexpr bool kTwo = P::kTwoProducers;
+  if (warp == 0 || (kTwo && warp == 6)) {
+    // One elected lane per producer warp (see tc_kernel.cuh); the leader's posts the byte count of
+    // both CTAs.
+    auto produce = [&](auto which) {
+      constexpr int kWhich = decltype(which)::value;
+      uint32_t s = 0, round = 0;
+      typename P::Tile t;
+      typename P::LoadState ls;
+      const uint32_t full_leader = mapa_u32(smem_u32(&full_bar[0]), 0);
+      TC_PROF_VAR(p_wait);
+      TC_PROF_NOW(p_t0);
+      for (int tile = pair; tile < n_tiles && *failed == 0; tile += n_pairs) {
+        prob.decode_pair(tile, (int)rank, t);
+        prob.template load_begin_pair<kWhich>(t, ls, (int)rank);
+        const int k1 = prob.k_end(t);
+        for (int k = prob.k_begin(t); k < k1; k += KSUB) {
+          const int kn = min(KSUB, k1 - k);
+          TC_PROF_NOW(w0);
           if (round > 0 && !mbar_wait(&empty_bar[s], (round - 1) & 1)) {
             *failed = 1;
-            ok = 0;
-          } else if (rank == 0 && part == 0) {
-            mbar_expect_tx(&full_bar[s], kn * 2 * SL::kStageBytes);
+            break;
+          }
+          TC_PROF_ADD(p_wait, w0);
+          if (kWhich != kB && rank == 0) mbar_expect_tx(&full_bar[s], kn * 2 * SL::kStageBytes);
+#pragma unroll
+          for (int sub = 0; sub < KSUB; ++sub) {
+            if (sub >= kn) break;
+            char* a_dst = tiles + (s * KSUB + sub) * SL::kStageBytes;
+            prob.template load_pair<kWhich>(&map_a, &map_b, t, ls, full_leader + s * 8, a_dst,
+                                            a_dst + SL::kABytes);
+          }
+          if (++s == NG) { s = 0; ++round; }
+        }
+      }
+#ifdef FLB200_TC_PROFILE
+      if (kWhich != kB) { TC_PROF_PUT(0, p_wait); TC_PROF_PUT(1, clock64() - p_t0); }
+#endif
+      // The leader's last commits still arrive on this CTA's empty barriers: wait for them
+      // so that the CTA does not leave while they are in flight.
+      if (kWhich != kB && *failed == 0) {
+        for (int i = 0; i < NG; ++i) {
+          const uint32_t fills = round + (static_cast<uint32_t>(i) < s ? 1u : 0u);
+          if (fills > 0 && !mbar_wait(&empty_bar[i], (fills - 1) & 1)) {
+            *failed = 1;
+            break;
           }
         }
-        TC_PROF_ADD(p_wait, w0);
-        if (__shfl_sync(0xffffffffu, ok, 0) == 0) {
-          live = false;
-          break;
-        }
-        const uint32_t full_leader = mapa_u32(smem_u32(&full_bar[s]), 0);
-#pragma unroll
-        for (int sub = 0; sub < KSUB; ++sub) {
-          if (sub >= kn) break;
-          char* a_dst = tiles + (s * KSUB + sub) * SL::kStageBytes;
-          prob.load_pair(&map_a, &map_b, t, ls, full_leader, a_dst, a_dst + SL::kABytes,
-                         (int)rank, lane * parts + part);
-        }
-        if (++s == NG) { s = 0; ++round; }
       }
-    }
-#ifdef FLB200_TC_PROFILE
-    if (lane == 0 && part == 0) { TC_PROF_PUT(0, p_wait); TC_PROF_PUT(1, clock64() - p_t0); }
-#endif
-    // The leader's last commits still arrive on this CTA's empty barriers: wait for them
-    // so that the CTA does not leave while they are in flight.
-    if (live && lane == 0 && part == 0 && *failed == 0) {
-      for (int i = 0; i < NG; ++i) {
-        const uint32_t fills = round + (static_cast<uint32_t>(i) < s ? 1u : 0u);
-        if (fills > 0 && !mbar_wait(&empty_bar[i], (fills - 1) & 1)) {
-          *failed = 1;
-          break;
-        }
+    };
+    if (elect_one()) {
+      if constexpr (kTwo) {
+        if (warp == 0) produce(std::integral_constant<int, kA>{});
+        else produce(std::integral_constant<int, kB>{});
+      } else {
+        produce(std::integral_constant<int, kBoth>{});
       }
     }
   } else if (warp == 1) {

@@ -49,7 +49,7 @@ constexpr int kMaxPatchClasses = 4;
 
 template <int BN>
 struct PatchConvProblem {
-  static constexpr bool kWarpProducer = false;
+  static constexpr bool kTwoProducers = false;
   static constexpr int kMinBlocks = 1;
   int a_mn_major, b_mn_major;  // 0, 0
   int operand;
@@ -77,7 +77,7 @@ struct PatchConvProblem {
   float* stats;   // EpiStats matrix [pixel tiles * 4][2 * n_out] (tc_kernel.cuh), or null
 
   struct Tile { int q0, p0, b0, n0, c; };
-  struct LoadState { int i, j, cc, aw, ah, wtap, c; };
+  struct LoadState { int i, j, cc, aw, ah, wtap, c, n0; };
 
   __device__ __forceinline__ int num_tiles() const {
     return tiles_q * tiles_p * tiles_b * tiles_n * ncls;
@@ -108,15 +108,19 @@ struct PatchConvProblem {
     t.p0 = (r % tiles_p) * PH; r /= tiles_p;
     t.b0 = r * NB;
   }
+  template <int>
+  __device__ __forceinline__ void load_begin_pair(const Tile& t, LoadState& ls, int rank) const {
+    load_begin<kBoth>(t, ls);
+    ls.n0 = t.n0 + rank * (BN / 2);  // this CTA's half of B
+  }
+  template <int>
   __device__ __forceinline__ void load_pair(const CUtensorMap* ma, const CUtensorMap* mb,
                                             const Tile& t, LoadState& ls, uint32_t full_bar,
-                                            char* a_dst, char* b_dst, int rank, int) const {
-    if (elect_one()) {
-      int ca[4] = {ls.cc * kel, ls.aw, ls.ah, t.b0};
-      tma_load_pair(ma, full_bar, a_dst, 4, ca);
-      int cb[4] = {ls.cc * kel, t.n0 + rank * (BN / 2), ls.wtap, 0};  // this CTA's half of B
-      tma_load_pair(mb, full_bar, b_dst, 3, cb);
-    }
+                                            char* a_dst, char* b_dst) const {
+    int ca[4] = {ls.cc * kel, ls.aw, ls.ah, t.b0};
+    tma_load_pair(ma, full_bar, a_dst, 4, ca);
+    int cb[4] = {ls.cc * kel, ls.n0, ls.wtap, 0};
+    tma_load_pair(mb, full_bar, b_dst, 3, cb);
     advance(ls);
   }
   __device__ __forceinline__ void advance(LoadState& ls) const {
@@ -136,7 +140,9 @@ struct PatchConvProblem {
   }
   __device__ __forceinline__ int k_begin(const Tile&) const { return 0; }
   __device__ __forceinline__ int k_end(const Tile& t) const { return cls[t.c].ntaps * cchunks; }
-  __device__ __forceinline__ void load_begin(const Tile& t, LoadState& ls, int) const {
+  template <int>
+  __device__ __forceinline__ void load_begin(const Tile& t, LoadState& ls) const {
+    ls.n0 = t.n0;
     ls.i = 0;
     ls.j = 0;
     ls.cc = 0;
@@ -146,13 +152,16 @@ struct PatchConvProblem {
     ls.ah = t.p0 * a_h_mul + taps.dh0;
     ls.wtap = taps.r0 * taps.kW + taps.s0;
   }
+  __device__ __forceinline__ uint32_t stage_bytes(const Tile&) const {
+    return (kBM + BN) * kBK * 4;  // NB * PH * QW == 128 rows of 128 bytes + B tile
+  }
+  template <int>
   __device__ __forceinline__ void load(const CUtensorMap* ma, const CUtensorMap* mb,
                                        const Tile& t, LoadState& ls, uint64_t* bar, char* a_dst,
-                                       char* b_dst, int, bool last, int, int) const {
-    mbar_post_tx(bar, (kBM + BN) * kBK * 4, last);  // NB*PH*QW == 128 rows of 128 bytes + B tile
+                                       char* b_dst) const {
     int ca[4] = {ls.cc * kel, ls.aw, ls.ah, t.b0};
     tma_load(ma, bar, a_dst, 4, ca);
-    int cb[4] = {ls.cc * kel, t.n0, ls.wtap, 0};
+    int cb[4] = {ls.cc * kel, ls.n0, ls.wtap, 0};
     tma_load(mb, bar, b_dst, 3, cb);
     advance(ls);
   }
@@ -302,7 +311,7 @@ struct PatchConvProblem {
 
 template <int BN>
 struct PatchWgradProblem {
-  static constexpr bool kWarpProducer = true;
+  static constexpr bool kTwoProducers = true;
   static constexpr int kMinBlocks = 1;
   int a_mn_major, b_mn_major;  // 1, 1
   int operand;
@@ -321,7 +330,8 @@ struct PatchWgradProblem {
   float* partial;              // [split][tap][M][N]
 
   struct Tile { int m0, n0, tap0, ntap, cn_live, split, k0, k1; };
-  struct LoadState { int qi, pi, img, dw, dh; };
+  // (tr, ts): the first of the taps [tap, tap_end) that this producer loads
+  struct LoadState { int qi, pi, img, tr, ts, tap, tap_end; };
 
   __device__ __forceinline__ int num_tiles() const {
     return tiles_m * tiles_n * tap_groups * splits;
@@ -339,50 +349,62 @@ struct PatchWgradProblem {
   }
   __device__ __forceinline__ int k_begin(const Tile& t) const { return t.k0; }
   __device__ __forceinline__ int k_end(const Tile& t) const { return t.k1; }
-  __device__ __forceinline__ void load_begin(const Tile& t, LoadState& ls, int copy) const {
+  template <int kWhich>
+  __device__ __forceinline__ void load_begin(const Tile& t, LoadState& ls) const {
     int r = t.k0;
     ls.qi = r % tiles_q; r /= tiles_q;
     ls.pi = r % tiles_p; r /= tiles_p;
     ls.img = r;
-    // the first copies are dy, the others x, tap after tap
-    const int na = a_each ? a_nbox : 1;
-    const int tap = t.tap0 + (max(copy - na, 0) >> (b_each ? cn_shift : 0));
-    const int tr = tap / kW, ts = tap - tr * kW;
-    ls.dw = ts * dil_x - pad_x;
-    ls.dh = tr * dil_y - pad_y;
+    // of two producers A's takes the last taps of a tile of several
+    const int moved = kWhich == kBoth ? 0 : (t.ntap - 1) >> 1;
+    ls.tap = kWhich == kA ? t.ntap - moved : 0;
+    ls.tap_end = kWhich == kB ? t.ntap - moved : t.ntap;
+    ls.tr = (t.tap0 + ls.tap) / kW;
+    ls.ts = t.tap0 + ls.tap - ls.tr * kW;
   }
+  // 32 pixels x 32 fp32 or 64 pixels x 64 16-bit channels
+  __device__ __forceinline__ int box_bytes() const { return 128 << cb_shift; }
+  __device__ __forceinline__ uint32_t stage_bytes(const Tile& t) const {
+    return (a_nbox + (t.ntap << cn_shift)) * box_bytes();
+  }
+  // With the channel index of a map split into (32 contiguous channels, group of 32) one copy
+  // brings every 32 x 32 box of an operand: a_nbox boxes of dy, and per tap 1 << cn_shift boxes
+  // of x.  Boxes past the last channel are zero-filled or hold a neighbouring pixel's channels;
+  // they only reach accumulator rows / columns that the epilogue never stores.  Over whole
+  // channels each box is a copy of its own, zero-filled past the last channel.
+  template <int kWhich>
   __device__ __forceinline__ void load(const CUtensorMap* ma, const CUtensorMap* mb,
                                        const Tile& t, LoadState& ls, uint64_t* bar, char* a_dst,
-                                       char* b_dst, int lane, bool last, int part,
-                                       int parts) const {
+                                       char* b_dst) const {
     const int q0 = ls.qi * QW, p0 = ls.pi * PH;
-    const int copy = lane * parts + part;
-    // With the channel index of a map split into (32 contiguous channels, group of 32) one copy
-    // brings every 32 x 32 box of an operand: a_nbox boxes of dy, and per tap 1 << cn_shift boxes
-    // of x.  Boxes past the last channel are zero-filled or hold a neighbouring pixel's channels;
-    // they only reach accumulator rows / columns that the epilogue never stores.  Over whole
-    // channels each box is a copy of its own, zero-filled past the last channel.
-    const int box_bytes = 128 << cb_shift;  // 32 pixels x 32 fp32 or 64 pixels x 64 16-bit channels
-    if (lane == 0 && part == 0)
-      mbar_post_tx(bar, (a_nbox + (t.ntap << cn_shift)) * box_bytes, last);
-    __syncwarp();
-    const int na = a_each ? a_nbox : 1, j = copy - na;
-    if (j < 0) {
+    if constexpr (kWhich != kB) {
       if (a_each) {
-        int ca[5] = {t.m0 + (copy << cb_shift), q0, p0, ls.img, 0};
-        tma_load(ma, bar, a_dst + copy * box_bytes, 4, ca);
+        for (int i = 0; i < a_nbox; ++i) {
+          int ca[5] = {t.m0 + (i << cb_shift), q0, p0, ls.img, 0};
+          tma_load(ma, bar, a_dst + i * box_bytes(), 4, ca);
+        }
       } else {
         int ca[5] = {0, q0, p0, ls.img, t.m0 >> cb_shift};
         tma_load(ma, bar, a_dst, 5, ca);
       }
-    } else if (j < (b_each ? t.ntap << cn_shift : t.ntap)) {
-      const int w = q0 * b_w_mul + ls.dw, h = p0 * b_h_mul + ls.dh;
-      if (b_each) {
-        int cb[5] = {t.n0 + ((j & ((1 << cn_shift) - 1)) << cb_shift), w, h, ls.img, 0};
-        tma_load(mb, bar, b_dst + j * box_bytes, 4, cb);
-      } else {
-        int cb[5] = {0, w, h, ls.img, t.n0 >> cb_shift};
-        tma_load(mb, bar, b_dst + (j << cn_shift) * box_bytes, 5, cb);
+    }
+    if (ls.tap < ls.tap_end) {
+      const int w0 = q0 * b_w_mul - pad_x, h0 = p0 * b_h_mul - pad_y;
+      int w = w0 + ls.ts * dil_x, h = h0 + ls.tr * dil_y, ts = ls.ts;
+      for (int tap = ls.tap;;) {
+        char* dst = b_dst + (tap << cn_shift) * box_bytes();
+        if (b_each) {
+          for (int i = 0; i < 1 << cn_shift; ++i) {
+            int cb[5] = {t.n0 + (i << cb_shift), w, h, ls.img, 0};
+            tma_load(mb, bar, dst + i * box_bytes(), 4, cb);
+          }
+        } else {
+          int cb[5] = {0, w, h, ls.img, t.n0 >> cb_shift};
+          tma_load(mb, bar, dst, 5, cb);
+        }
+        if (++tap >= ls.tap_end) break;
+        w += dil_x;
+        if (++ts == kW) { ts = 0; w = w0; h += dil_y; }
       }
     }
     if (++ls.qi == tiles_q) {

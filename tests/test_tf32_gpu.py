@@ -469,3 +469,26 @@ def test_linear_bias_activation_declines_gracefully(L, fx):
     assert fx.linear_bias_act(x, w, b, True, math_mode=L.MATH_TF32) is None      # O % 32 != 0
     x2, w2, b2 = randn(8, 16, seed=127).cuda(), randn(16, 32, seed=128).cuda(), randn(32, seed=129).cuda()
     assert fx.linear_bias_act(x2, w2, b2, True, math_mode=L.MATH_STRICT_F32) is None  # fp32 FMA mode
+
+
+@pytest.mark.parametrize("batch", [1, 3])
+@pytest.mark.parametrize("dtype,tol", [(torch.float32, TF32_SCALED_TOL), (torch.bfloat16, 1.6e-2)])
+@pytest.mark.parametrize("mnk", [
+    (128, 64, 64),     # one whole tile, one copy per operand and stage
+    (320, 2112, 72),   # groups past the last row and column, a K tail
+    (712, 2056, 200),  # no multiple of a group: a copy per box, the two producers share them
+    (192, 712, 40),    # one operand of each kind
+])
+def test_matmul_mn_major_boxes(L, fx, mnk, dtype, tol, batch):
+    """Operands whose m and n are contiguous: all boxes of a stage in one copy where the extent is whole
+    groups of 32 (16-bit: 64), else a copy per box.  Bounds: of the tests above (TF32), and bf16
+    operands and result, 2^-8 relative each, on sums of random signs."""
+    m, n, k = mnk
+    a, b = randn(batch, k, m, seed=5).to(dtype), randn(batch, k, n, seed=6).to(dtype)
+    want = a.double().transpose(1, 2) @ b.double()
+    c, launched = tc_delta(L, lambda: fx.matmul(a.cuda(), b.cuda(), m=m, n=n, k=k, a_strides=(1, m),
+                                                b_strides=(n, 1), batch=batch,
+                                                batch_strides=(k * m, k * n, m * n),
+                                                math_mode=L.MATH_TF32))
+    assert launched >= 1
+    assert_close_scaled(c.reshape(batch, m, n), want, tol, f"matmul {mnk} x {batch} {dtype}")
