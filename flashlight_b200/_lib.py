@@ -110,6 +110,8 @@ SIGNATURES = {
                                                      vp, vp, vp, vp, vp, sz, vp]),
     "flb200_batchnorm_relu_backward": (C.c_int, [P(BatchnormDesc), vp, vp, vp, vp, vp, vp, vp, vp,
                                                  vp, vp, sz, vp]),
+    "flb200_batchnorm_relu_backward_sum": (C.c_int, [P(BatchnormDesc), vp, vp, vp, vp, vp, vp, vp, vp,
+                                                     vp, vp, vp, vp, sz, vp]),
     "flb200_matmul_workspace_bytes": (sz, [P(MatmulDesc)]),
     "flb200_matmul": (C.c_int, [P(MatmulDesc), vp, vp, vp, vp, sz, vp]),
     "flb200_matmul_wide": (C.c_int, [P(MatmulDesc), vp, vp, vp, vp, sz, vp]),

@@ -144,7 +144,9 @@ class Variable:
                     stack.append((inp, False))
         for node in reversed(order):
             func = node.grad_func
-            if node._grad_second is not None and node.grad_func2 is not None:
+            # (a node that is asked for its gradient afterwards needs the sum itself)
+            if (node._grad_second is not None and node.grad_func2 is not None and not retain_graph and
+                    node.grad_hook is None):
                 first, second = node._grad, node._grad_second
                 node._grad_second = None
                 node.grad_func2(node.inputs, first, second)
@@ -234,21 +236,32 @@ def batchnorm(x: Variable, weight: Optional[Variable], bias: Optional[Variable],
     xt = x.tensor
     ins = [x] + ([weight] if weight is not None else []) + ([bias] if bias is not None else [])
 
-    def grad_func(inputs, gy):
-        if relu:
-            gx, gw, gb = ext.batchnormReluBackward(gy, save_mean, save_var, xt, wt, bt, axes, train,
-                                                   epsilon, None)
-        else:
-            gx, gw, gb = ext.batchnormBackward(gy, save_mean, save_var, xt, wt, axes, train,
-                                               epsilon, None)
-        inputs[0].addGrad(gx)
+    def give(inputs, gx, gw, gb):
+        if gx is not None:
+            inputs[0].addGrad(gx)
         k = 1
         if weight is not None:
             inputs[k].addGrad(gw.reshape(wt.shape)); k += 1
         if bias is not None:
             inputs[k].addGrad(gb.reshape(bt.shape))
 
-    return Variable(y, False, ins, grad_func)
+    def grad_func(inputs, gy):
+        if relu:
+            give(inputs, *ext.batchnormReluBackward(gy, save_mean, save_var, xt, wt, bt, axes, train, epsilon,
+                                                    None, needInput=inputs[0].isCalcGrad()))
+        else:
+            give(inputs, *ext.batchnormBackward(gy, save_mean, save_var, xt, wt, axes, train, epsilon, None))
+
+    def grad_func2(inputs, ga, gb):
+        if not ext.batchnormSumSupported(xt, ga, gb, axes):
+            return grad_func(inputs, F.add(ga, gb))
+        give(inputs, *ext.batchnormReluBackward(ga, save_mean, save_var, xt, wt, bt, axes, train, epsilon,
+                                                None, gb, inputs[0].isCalcGrad()))
+
+    out = Variable(y, False, ins, grad_func)
+    if relu:
+        out.grad_func2 = grad_func2
+    return out
 
 
 def batchnorm_add_relu(x: Variable, addend: Variable, weight: Optional[Variable],

@@ -607,7 +607,7 @@ int launch_reduce(const char* name, const void* a, const void* b, float2* partia
       dim3 vgrid((unsigned)ct.col_blocks, (unsigned)splits);
       column_reduce_vec_kernel<T, NIN, F><<<vgrid, 256, 0, st>>>(
           static_cast<const T*>(a), static_cast<const T*>(b), partial, outer, channels,
-          splits, rps, ct.cq_shift, f);
+          splits, rps, ct.cq_shift, f, nullptr, nullptr);
       FLB200_AFTER_LAUNCH(name);
       *splits_out = splits;
       return FLB200_OK;
@@ -631,6 +631,20 @@ int launch_reduce(const char* name, const void* a, const void* b, float2* partia
         static_cast<const T*>(a), static_cast<const T*>(b), partial, g, f);
   FLB200_AFTER_LAUNCH(name);
   *splits_out = g.splits;
+  return FLB200_OK;
+}
+
+// The reduction over (a, b + b2) on channels-last tensors that 16-byte vectors take; sum: b + b2, or null.
+template <typename T, typename F>
+int launch_reduce_sum(const char* name, const void* a, const void* b, const void* b2, void* sum, float2* partial,
+                      long long rows, long long channels, F f, int* splits_out, cudaStream_t st) {
+  const int splits = column_splits(rows, channels, true);
+  const ColumnTiling ct = column_tiling(channels, Vec16<T>::N);
+  column_reduce_vec_kernel<T, 3, F><<<dim3((unsigned)ct.col_blocks, (unsigned)splits), 256, 0, st>>>(
+      static_cast<const T*>(a), static_cast<const T*>(b), partial, rows, channels, splits,
+      (rows + splits - 1) / splits, ct.cq_shift, f, static_cast<const T*>(b2), static_cast<T*>(sum));
+  FLB200_AFTER_LAUNCH(name);
+  *splits_out = splits;
   return FLB200_OK;
 }
 
@@ -1055,10 +1069,11 @@ static int batchnorm_backward_impl(bool relu, const uint8_t* tail_mask, const vo
                                    const float* bias,
                                    const float* save_mean, const float* save_invstd, void* grad_x,
                                    float* grad_weight, float* grad_bias, void* workspace,
-                                   size_t workspace_bytes, void* stream) {
+                                   size_t workspace_bytes, void* stream,
+                                   const void* relu_gb = nullptr, void* relu_sum = nullptr) {
   FLB200_REQUIRE(d, "batchnorm_backward: null descriptor");
   if (int st = check_geo("batchnorm_backward", d->outer, d->channels, d->inner)) return st;
-  FLB200_REQUIRE(grad_y && x && save_mean && save_invstd && grad_x && grad_weight && grad_bias,
+  FLB200_REQUIRE(grad_y && x && save_mean && save_invstd && grad_weight && grad_bias,
                  "batchnorm_backward: null tensor");
   const size_t need = flb200_batchnorm_workspace_bytes(d);
   if (!workspace || workspace_bytes < need)
@@ -1106,6 +1121,12 @@ static int batchnorm_backward_impl(bool relu, const uint8_t* tail_mask, const vo
     FLB200_AFTER_LAUNCH("batchnorm_tail_backward_reduce");
     splits = g.splits;
     grad_y = tail_sum;
+  } else if (relu_gb) {
+    BnReluBwdReduceF rf{save_mean, save_invstd, weight, bias};
+    FLB200_DISPATCH_DTYPE(d->dtype, "batchnorm_relu_backward_sum",
+                          rc = (launch_reduce_sum<T>("batchnorm_relu_backward_reduce_sum", x, grad_y, relu_gb,
+                                                     relu_sum, partial, d->outer, C, rf, &splits, st)));
+    grad_y = relu_sum;
   } else if (relu) {
     BnReluBwdReduceF rf{save_mean, save_invstd, weight, bias};
     FLB200_DISPATCH_DTYPE(d->dtype, "batchnorm_relu_backward",
@@ -1124,6 +1145,7 @@ static int batchnorm_backward_impl(bool relu, const uint8_t* tail_mask, const vo
       partial, splits, C, (double)d->outer * (double)d->inner, weight, save_mean, save_invstd,
       grad_weight, grad_bias, coef);
   FLB200_AFTER_LAUNCH("batchnorm_backward_finalize");
+  if (!grad_x) return rc;
   if (relu) {
     BnReluBwdApplyF af{coef, save_invstd, weight, bias};
     FLB200_DISPATCH_DTYPE(d->dtype, "batchnorm_relu_backward",
@@ -1143,6 +1165,7 @@ int flb200_batchnorm_backward(const flb200_batchnorm_desc* d, const void* grad_y
                               const float* save_invstd, void* grad_x, float* grad_weight,
                               float* grad_bias, void* workspace, size_t workspace_bytes,
                               void* stream) {
+  FLB200_REQUIRE(grad_x, "batchnorm_backward: null tensor");
   return batchnorm_backward_impl(false, nullptr, nullptr, nullptr, d, grad_y, x, weight, nullptr,
                                  save_mean, save_invstd,
                                  grad_x, grad_weight, grad_bias, workspace, workspace_bytes,
@@ -1153,6 +1176,7 @@ int flb200_batchnorm_relu_backward(const flb200_batchnorm_desc* d, const void* g
                                    const float* save_mean, const float* save_invstd,
                                    void* grad_x, float* grad_weight, float* grad_bias,
                                    void* workspace, size_t workspace_bytes, void* stream) {
+  FLB200_REQUIRE(grad_x, "batchnorm_backward: null tensor");
   return batchnorm_backward_impl(true, nullptr, nullptr, nullptr, d, grad_y, x, weight, bias,
                                  save_mean, save_invstd, grad_x, grad_weight, grad_bias, workspace,
                                  workspace_bytes, stream);
@@ -1164,6 +1188,7 @@ int flb200_batchnorm_add_relu_backward(const flb200_batchnorm_desc* d, const uin
                                        float* grad_weight, float* grad_bias, void* workspace,
                                        size_t workspace_bytes, void* stream) {
   FLB200_REQUIRE(d && mask && grad_y_a && grad_sum, "batchnorm_add_relu_backward: null argument");
+  FLB200_REQUIRE(grad_x, "batchnorm_backward: null tensor");
   if (!add_relu_supported(d) || !aligned16(x) ||
       !aligned16(grad_y_a) || !aligned16(grad_sum) || (grad_y_b && !aligned16(grad_y_b)))
     return fail(FLB200_UNSUPPORTED,
@@ -1172,6 +1197,24 @@ int flb200_batchnorm_add_relu_backward(const flb200_batchnorm_desc* d, const uin
   return batchnorm_backward_impl(false, mask, grad_y_b, grad_sum, d, grad_y_a, x, weight, nullptr,
                                  save_mean, save_invstd, grad_x, grad_weight, grad_bias, workspace,
                                  workspace_bytes, stream);
+}
+
+int flb200_batchnorm_relu_backward_sum(const flb200_batchnorm_desc* d, const void* grad_y_a,
+                                       const void* grad_y_b, const void* x, const float* weight,
+                                       const float* bias, const float* save_mean,
+                                       const float* save_invstd, void* grad_sum, void* grad_x,
+                                       float* grad_weight, float* grad_bias, void* workspace,
+                                       size_t workspace_bytes, void* stream) {
+  FLB200_REQUIRE(d && (!grad_y_b || !grad_x || grad_sum), "batchnorm_relu_backward_sum: null argument");
+  const int vec = d->dtype == FLB200_F32 ? 4 : 8;
+  if (grad_y_b && (d->inner != 1 || d->channels % vec != 0 || !aligned16(x) || !aligned16(grad_y_a) ||
+                   !aligned16(grad_y_b) || (grad_sum && !aligned16(grad_sum))))
+    return fail(FLB200_UNSUPPORTED,
+                "batchnorm_relu_backward_sum: two gradients are added for channels-last, 16-byte aligned "
+                "tensors of whole 16-byte vectors of channels only");
+  return batchnorm_backward_impl(true, nullptr, nullptr, nullptr, d, grad_y_a, x, weight, bias,
+                                 save_mean, save_invstd, grad_x, grad_weight, grad_bias, workspace,
+                                 workspace_bytes, stream, grad_y_b, grad_x ? grad_sum : nullptr);
 }
 
 }  // extern "C"

@@ -863,6 +863,22 @@ NATIVE(batchnorm_backward) {
                    stream()));
   return wrap({gx, gw, gb});
 }
+// relu(batch-norm): (grad_a, grad_b or None, save_mean, save_invstd, input, weight, bias, axes, need_x)
+//   -> (grad_x or None, grad_weight, grad_bias)
+NATIVE(batchnorm_relu_backward_sum) {
+  const Tensor &ga = x.tensor(0), &in = x.tensor(4);
+  const Tensor* gb = x.t(1);
+  const flb200_batchnorm_desc d = bn_desc(in, x.at(7));
+  const bool need = x.b(8);
+  Tensor gx, gs, gw = floats(d.channels, in), gb_out = floats(d.channels, in);
+  if (need) gx = empty_like(in);
+  if (need && gb) gs = empty_like(in);
+  Workspace ws(flb200_batchnorm_workspace_bytes(&d), in);
+  check(unlocked(flb200_batchnorm_relu_backward_sum, &d, P(ga), P(gb), P(in), Pf(x.t(5)), Pf(x.t(6)), Pf(x.t(2)),
+                 Pf(x.t(3)), gs.defined() ? P(gs) : nullptr, gx.defined() ? P(gx) : nullptr, Pf(&gw), Pf(&gb_out),
+                 ws.p(), ws.bytes, stream()));
+  return wrap({gx, gw, gb_out});
+}
 // (mask, grad_a, grad_b or None, save_mean, save_invstd, input, weight, axes)
 //   -> (grad_sum, grad_x, grad_weight, grad_bias)
 NATIVE(batchnorm_add_relu_backward) {
@@ -897,7 +913,7 @@ PyMethodDef methods[] = {
     ENTRY(conv2d_cache_bytes), ENTRY(conv2d), ENTRY(conv2d_backward_data),
     ENTRY(conv2d_backward_filter_bias), ENTRY(pool2d), ENTRY(pool2d_backward), ENTRY(batchnorm),
     ENTRY(batchnorm_add_relu_supported), ENTRY(batchnorm_add_relu), ENTRY(batchnorm_backward),
-    ENTRY(batchnorm_add_relu_backward), {nullptr, nullptr, 0, nullptr}};
+    ENTRY(batchnorm_add_relu_backward), ENTRY(batchnorm_relu_backward_sum), {nullptr, nullptr, 0, nullptr}};
 
 PyModuleDef module = {PyModuleDef_HEAD_INIT, "_native", nullptr, -1, methods,
                       nullptr, nullptr, nullptr, nullptr};

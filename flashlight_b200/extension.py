@@ -413,12 +413,25 @@ class B200AutogradExtension:
             raise RuntimeError("can't compute batchnorm grad when train was not specified")
         return N.batchnorm_add_relu_backward(mask, gradA, gradB, saveMean, saveVar, input, weight, axes)
 
+    @staticmethod
+    def batchnormSumSupported(input, gradA, gradB, axes) -> bool:
+        """Whether batchnormReluBackward adds two gradients itself."""
+        return (list(axes) == [2] and is_channels_last(input) and gradA.dtype == input.dtype and
+                gradB.dtype == input.dtype and same_layout(gradA, input) and same_layout(gradB, input) and
+                input.shape[1] * input.element_size() % 16 == 0 and
+                not (input.data_ptr() | gradA.data_ptr() | gradB.data_ptr()) & 15)
+
     def batchnormReluBackward(self, gradOutput, saveMean, saveVar, input, weight, bias, axes, train,
-                              epsilon, payload=None):
+                              epsilon, payload=None, gradOutput2=None, needInput=True):
         """Gradient of relu(batchnorm(x)) given the gradient of the relu output: the predicate
-        is rebuilt from the input, so no output tensor or mask is needed."""
+        is rebuilt from the input, so no output tensor or mask is needed.  gradOutput2: a second
+        consumer's gradient, added where the first is read (check batchnormSumSupported);
+        needInput=False: None in the place of the input's gradient."""
         if not train:
             raise RuntimeError("can't compute batchnorm grad when train was not specified")
+        if gradOutput2 is not None or not needInput:
+            return N.batchnorm_relu_backward_sum(gradOutput, gradOutput2, saveMean, saveVar, input, weight,
+                                                 bias, axes, needInput)
         return N.batchnorm_backward(gradOutput, saveMean, saveVar, input, weight, bias, axes, True)
 
     # ------------------------------------------------------------------ rnn

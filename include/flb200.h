@@ -303,6 +303,17 @@ int flb200_batchnorm_relu_backward(const flb200_batchnorm_desc* d, const void* g
                                    const float* save_mean, const float* save_invstd,
                                    void* grad_x, float* grad_weight, float* grad_bias,
                                    void* workspace, size_t workspace_bytes, void* stream);
+/* The same where the relu output had two consumers, whose gradients are grad_y_a and grad_y_b (NULL: one
+ * consumer), and where grad_x is not needed (NULL).  The two are added as they are read, rounded to the
+ * tensors' type; with grad_x their sum is written to grad_sum (else it may be NULL).  Two gradients:
+ * channels-last, 16-byte aligned tensors of a multiple of 4 (16-bit: 8) channels, else
+ * FLB200_UNSUPPORTED. */
+int flb200_batchnorm_relu_backward_sum(const flb200_batchnorm_desc* d, const void* grad_y_a,
+                                       const void* grad_y_b, const void* x, const float* weight,
+                                       const float* bias, const float* save_mean,
+                                       const float* save_invstd, void* grad_sum, void* grad_x,
+                                       float* grad_weight, float* grad_bias, void* workspace,
+                                       size_t workspace_bytes, void* stream);
 
 /* --------------------------------------------------------- matmul (a9) */
 /* C[m,n] = alpha * sum_k A(m,k) B(k,n) + beta * C[m,n] on ROW-MAJOR views with

@@ -1,0 +1,46 @@
+"""relu(batch-norm) whose output has two consumers, or whose input takes no gradient: the gradients are
+those of the operator chain (the consumers' gradients added by F.add first) bit for bit."""
+import pytest
+import torch
+
+from tests.parity import randn
+
+pytestmark = pytest.mark.gpu
+
+
+@pytest.mark.parametrize("dtype", [torch.float32, torch.float16, torch.bfloat16])
+@pytest.mark.parametrize("shape", [
+    (3, 8, 5, 7),      # 105 rows: whole groups of rows and a remainder
+    (2, 264, 3, 3),    # more vectors than a CTA has columns, fewer rows than it has lanes
+    (40, 64, 29, 31),  # many splits
+    (2, 12, 6, 6),     # no whole 16-bit vectors
+])
+@pytest.mark.parametrize("need_x", [False, True])
+def test_two_consumers(shape, dtype, need_x):
+    from flashlight_b200 import autograd as A
+    from flashlight_b200 import functions as F
+    from flashlight_b200.autograd import Variable
+    cl = lambda seed, s=1.0: (randn(*shape, seed=seed) * s).cuda().to(dtype).contiguous(
+        memory_format=torch.channels_last)
+    C = shape[1]
+    x, ga, gb = cl(1), cl(2, 0.1), cl(3, 0.1)
+    w, b = (randn(C, seed=4).abs() + 0.5).cuda(), randn(C, seed=5).cuda()
+
+    def run(second, need, retain=False):
+        xv, wv, bv = Variable(x, need), Variable(w, True), Variable(b, True)
+        y = A.batchnorm(xv, wv, bv, None, None, [2], True, 0.1, 1e-5, relu=True)
+        if second:
+            y.addGrad(ga)
+            y.backward(gb, retain_graph=retain)
+        else:
+            y.backward(F.add(ga, gb), retain_graph=retain)
+        return xv.grad, wv.grad, bv.grad, y.grad
+
+    got, want = run(True, need_x), run(False, True)
+    assert (got[0] is not None) == need_x
+    if need_x:
+        assert torch.equal(got[0], want[0])
+    assert torch.equal(got[1], want[1]) and torch.equal(got[2], want[2])
+    # a graph that is kept keeps the sum as the output's gradient
+    kept = run(True, need_x, retain=True)
+    assert torch.equal(kept[3], F.add(ga, gb)) and torch.equal(kept[1], want[1])
