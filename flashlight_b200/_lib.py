@@ -166,6 +166,10 @@ SIGNATURES = {
     "flb200_cce_backward": (C.c_int, [vp, vp, vp, vp, i64, i64, C.c_int, C.c_int, C.c_int, vp]),
     "flb200_log_softmax_cce_backward": (C.c_int, [vp, vp, vp, vp, vp, i64, i64, C.c_int, C.c_int,
                                                   C.c_int, vp]),
+    "flb200_scores_cce_forward": (C.c_int, [vp, vp, vp, vp, vp, vp, i64, i64, C.c_int, C.c_int, C.c_int, vp,
+                                            sz, vp]),
+    "flb200_scores_cce_backward": (C.c_int, [vp, vp, vp, vp, vp, vp, i64, i64, C.c_int, C.c_int, C.c_int,
+                                             vp]),
     "flb200_rnn_num_params": (i64, [P(RnnDesc)]),
     "flb200_rnn_reserve_bytes": (sz, [P(RnnDesc)]),
     "flb200_rnn_workspace_bytes": (sz, [P(RnnDesc), C.c_int]),

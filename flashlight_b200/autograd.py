@@ -557,8 +557,23 @@ def categorical_cross_entropy(logp: Variable, targets: torch.Tensor, reduction=L
 
 
 def log_softmax_cross_entropy(x: Variable, targets: torch.Tensor, reduction=L.REDUCE_MEAN,
-                              ignore_index=-1) -> Variable:
-    """categoricalCrossEntropy(logSoftmax(x)) with the fused gradient kernel."""
+                              ignore_index=-1, wide: bool = False) -> Variable:
+    """categoricalCrossEntropy(logSoftmax(x)) with the fused gradient kernel.  wide=True: of
+    cast(x, float32), without that copy in memory where the library can."""
+    xt = x.tensor
+    half = wide and xt.dtype in (torch.float16, torch.bfloat16)
+    if half or xt.dtype == torch.float32:
+        # (shorter rows are a warp's, and their log-probabilities a small tensor)
+        fused = F.scores_cross_entropy(xt, targets, reduction, ignore_index) if xt.shape[-1] > 1024 else None
+        if fused is not None:
+            loss, state, lse = fused
+
+            def grad_scores(inputs, gl):
+                inputs[0].addGrad(F.scores_cross_entropy_backward(xt, lse, gl, state))
+
+            return Variable(loss, False, [x], grad_scores)
+        if half:
+            x = cast(x, torch.float32)
     y = F.log_softmax(x.tensor)
     loss, state = F.categorical_cross_entropy(y, targets, reduction, ignore_index)
 

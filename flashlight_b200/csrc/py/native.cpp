@@ -503,6 +503,34 @@ NATIVE(cce_forward) {  // (logp, targets int32, reduction, ignore_index) -> (los
                            code_of(logp), ws.p(), ws.bytes, st));
   return wrap({loss, meta});
 }
+// from the scores: (x, targets int32, reduction, ignore_index) -> (loss, meta, lse), or None where the
+// library has no kernel for the rows
+NATIVE(scores_cce_forward) {
+  const Tensor &in = x.tensor(0), &tg = x.tensor(1);
+  int64_t C, X;
+  classes(in, &C, &X);
+  if (C <= 1024 || C % 4 != 0 || X < 1 || X > 65535 || !in.is_contiguous() || !aligned16(&in)) Py_RETURN_NONE;
+  const int red = x.n32(2);
+  Tensor loss = floats(red == FLB200_REDUCE_NONE ? X : 1, in), lse = floats(X, in);
+  Tensor meta = empty({2}, ScalarType::Int, in);  // [count, bad-target flag]
+  int32_t* m = static_cast<int32_t*>(meta.data_ptr());
+  void* st = stream();
+  if (unlocked(cudaMemsetAsync, m, 0, (size_t)8, static_cast<cudaStream_t>(st)) != cudaSuccess)
+    check(FLB200_LAUNCH_FAILURE);
+  Workspace ws(flb200_cce_workspace_bytes(X), in);
+  check(unlocked(flb200_scores_cce_forward, P(in), Pf(&lse), static_cast<const int32_t*>(P(tg)), Pf(&loss), m, m + 1,
+                 C, X, red, x.n32(3), code_of(in), ws.p(), ws.bytes, st));
+  return wrap({loss, meta, lse});
+}
+NATIVE(scores_cce_backward) {  // (x, lse, grad_loss, targets, meta, reduction, ignore_index)
+  const Tensor &in = x.tensor(0), &tg = x.tensor(3), &meta = x.tensor(4);
+  int64_t C, X;
+  classes(in, &C, &X);
+  Tensor gx = empty_like(in);
+  check(unlocked(flb200_scores_cce_backward, P(in), Pf(x.t(1)), Pf(x.t(2)), static_cast<const int32_t*>(P(tg)),
+                 static_cast<const int32_t*>(P(meta)), P(gx), C, X, x.n32(5), x.n32(6), code_of(in), stream()));
+  return wrap(gx);
+}
 NATIVE(cce_backward) {  // (grad_loss, targets, meta, C, reduction, ignore_index, like)
   const Tensor &tg = x.tensor(1), &meta = x.tensor(2), &like = x.tensor(6);
   Tensor gx = empty_like(like);
@@ -906,7 +934,7 @@ PyMethodDef methods[] = {
     ENTRY(dropout_apply), ENTRY(astype), ENTRY(reorder), ENTRY(bernoulli_mask), ENTRY(channel_sum),
     ENTRY(channel_bias_add), ENTRY(layernorm), ENTRY(layernorm_backward), ENTRY(linear),
     ENTRY(linear_bias_act), ENTRY(linear_backward), ENTRY(matmul), ENTRY(log_softmax),
-    ENTRY(log_softmax_backward), ENTRY(cce_forward), ENTRY(cce_backward),
+    ENTRY(log_softmax_backward), ENTRY(cce_forward), ENTRY(scores_cce_forward), ENTRY(scores_cce_backward), ENTRY(cce_backward),
     ENTRY(log_softmax_cce_backward), ENTRY(softmax), ENTRY(softmax_backward),
     ENTRY(attention_backward), ENTRY(attention_packed), ENTRY(attention_packed_backward),
     ENTRY(embedding), ENTRY(embedding_backward),

@@ -70,33 +70,70 @@ log_softmax_forward_kernel(const T* __restrict__ x, T* __restrict__ y, long long
 // maximum and the sum of exponentials taken in ONE sweep (a running maximum, the sum rescaled
 // whenever it moves), then the sweep that writes y: two reads of the row instead of three, the
 // second one out of cache.
+// Four consecutive scores as fp32.
+__device__ __forceinline__ float4 load4(const float* p) { return *reinterpret_cast<const float4*>(p); }
+template <typename T>
+__device__ __forceinline__ float4 load4(const T* p) {
+  const uint2 r = *reinterpret_cast<const uint2*>(p);
+  const T* h = reinterpret_cast<const T*>(&r);
+  return make_float4(Num<T>::to_f(h[0]), Num<T>::to_f(h[1]), Num<T>::to_f(h[2]), Num<T>::to_f(h[3]));
+}
+// log of the sum of a row's exponentials, by a CTA
+template <typename T>
+__device__ __forceinline__ float row_lse(const T* xr, long long C4, float* scratch) {
+  float m = -INFINITY, s = 0.f;
+  auto take = [&](const float4 v) {
+    const float vm = fmaxf(fmaxf(v.x, v.y), fmaxf(v.z, v.w));
+    if (vm > m) {
+      s *= expf(m - vm);  // m = -inf: s is 0 and stays 0
+      m = vm;
+    }
+    const float r = m == -INFINITY ? 0.f : m;  // nothing but -inf so far: it weighs nothing
+    s += expf(v.x - r) + expf(v.y - r) + expf(v.z - r) + expf(v.w - r);
+  };
+  long long c = threadIdx.x;
+  for (; c + 3 * kRowThreads < C4; c += 4 * kRowThreads) {  // four loads in flight
+    float4 v[4];
+#pragma unroll
+    for (int u = 0; u < 4; ++u) v[u] = load4(xr + 4 * (c + u * kRowThreads));
+#pragma unroll
+    for (int u = 0; u < 4; ++u) take(v[u]);
+  }
+  for (; c < C4; c += kRowThreads) take(load4(xr + 4 * c));
+  const float row_max = group_max<kRowThreads>(m, scratch);
+  // a thread that saw nothing (m = -inf) contributes 0, or its NaN; rows whose maximum is -inf or
+  // NaN give NaN, as the three-sweep kernel does
+  const float mine = m == -INFINITY ? s : s * expf(m - row_max);
+  const float total = group_sum<kRowThreads>(mine, scratch);
+  return row_max + logf(total);
+}
+
 __global__ void __launch_bounds__(kRowThreads)
 log_softmax_forward_vec_kernel(const float* __restrict__ x, float* __restrict__ y, long long C4,
                                long long X) {
   __shared__ float scratch[32];
   for (long long row = blockIdx.x; row < X; row += gridDim.x) {
     const float4* xr = reinterpret_cast<const float4*>(x) + row * C4;
-    float m = -INFINITY, s = 0.f;
-    for (long long c = threadIdx.x; c < C4; c += kRowThreads) {
-      const float4 v = xr[c];
-      const float vm = fmaxf(fmaxf(v.x, v.y), fmaxf(v.z, v.w));
-      if (vm > m) {
-        s *= expf(m - vm);  // m = -inf: s is 0 and stays 0
-        m = vm;
-      }
-      s += expf(v.x - m) + expf(v.y - m) + expf(v.z - m) + expf(v.w - m);
-    }
-    const float row_max = group_max<kRowThreads>(m, scratch);
-    // a thread that saw nothing (m = -inf) contributes 0; rows whose maximum is -inf or NaN
-    // give NaN, as the three-sweep kernel does
-    const float mine = m == -INFINITY ? 0.f : s * expf(m - row_max);
-    const float total = group_sum<kRowThreads>(mine, scratch);
-    const float lse = row_max + logf(total);
+    const float lse = row_lse(x + row * C4 * 4, C4, scratch);
     float4* yr = reinterpret_cast<float4*>(y) + row * C4;
     for (long long c = threadIdx.x; c < C4; c += kRowThreads) {
       const float4 v = xr[c];
       yr[c] = make_float4(v.x - lse, v.y - lse, v.z - lse, v.w - lse);
     }
+  }
+}
+
+// Loss straight from the scores: of logSoftmax only the row's lse is kept, since x - lse is recomputed where
+// it is read, with the same rounding.  4096 rows of 32000 bf16 scores: the copy to fp32, logSoftmax, its
+// fused gradient and the copy back took 154 + 251 + 194 + 122 us for 2.9 GB; now two reads and a write of the
+// scores, 0.8 GB.
+template <typename T>
+__global__ void __launch_bounds__(kRowThreads)
+row_lse_kernel(const T* __restrict__ x, float* __restrict__ lse, long long C4, long long X) {
+  __shared__ float scratch[32];
+  for (long long row = blockIdx.x; row < X; row += gridDim.x) {
+    const float v = row_lse(x + row * C4 * 4, C4, scratch);
+    if (threadIdx.x == 0) lse[row] = v;
   }
 }
 
@@ -133,12 +170,14 @@ __device__ __forceinline__ float cce_weight(const float* grad_loss, const int32_
   return grad_loss[0];
 }
 
-// partial[blockIdx] = (sum of -logp[target], number of targets kept)
+// partial[blockIdx] = (sum of -logp[target], number of targets kept).  lse: logp holds scores, logSoftmax of
+// which is taken here
 template <typename T>
 __global__ void __launch_bounds__(256)
 cce_forward_kernel(const T* __restrict__ logp, const int32_t* __restrict__ targets,
                    float* __restrict__ loss_none, float2* __restrict__ partial,
-                   int32_t* __restrict__ bad_flag, long long C, long long X, int ignore_index) {
+                   int32_t* __restrict__ bad_flag, long long C, long long X, int ignore_index,
+                   const float* __restrict__ lse) {
   __shared__ float scratch[32];
   float s = 0.f, n = 0.f;
   const long long stride = (long long)gridDim.x * blockDim.x;
@@ -150,7 +189,7 @@ cce_forward_kernel(const T* __restrict__ logp, const int32_t* __restrict__ targe
     } else if (t < 0 || t >= C) {
       if (bad_flag) atomicOr(bad_flag, 1);
     } else {
-      v = -Num<T>::to_f(logp[i * C + t]);
+      v = -(lse ? Num<T>::to_f(logp[i * C + t]) - lse[i] : Num<T>::to_f(logp[i * C + t]));
       n += 1.f;
     }
     if (loss_none) loss_none[i] = v;
@@ -216,24 +255,28 @@ lsm_cce_backward_kernel(const T* __restrict__ y, const float* __restrict__ grad_
   }
 }
 
-// The same for fp32 rows of a multiple of 4 classes (16-byte aligned): blockIdx.y = row, four
-// classes per thread, the row's target and weight read once per thread, no division.
+// The same for rows of a multiple of 4 classes (16-byte aligned): blockIdx.y = row, four classes per
+// thread, the row's target and weight read once per thread, no division.  LSE: y holds scores, lse[row] makes
+// log-probabilities of them.
+template <typename T, bool LSE>
 __global__ void __launch_bounds__(256)
-lsm_cce_backward_vec_kernel(const float* __restrict__ y, const float* __restrict__ grad_loss,
-                            const int32_t* __restrict__ targets,
-                            const int32_t* __restrict__ count, float* __restrict__ dx,
+lsm_cce_backward_vec_kernel(const T* __restrict__ y, const float* __restrict__ lse,
+                            const float* __restrict__ grad_loss, const int32_t* __restrict__ targets,
+                            const int32_t* __restrict__ count, T* __restrict__ dx,
                             long long C4, int reduction, int ignore_index) {
   const long long row = blockIdx.y;
   const int t = targets[row];
   const bool live = t != ignore_index && t >= 0 && t < 4 * C4;
   const float g = live ? cce_weight(grad_loss, count, row, reduction) : 0.f;
-  const float4* yr = reinterpret_cast<const float4*>(y) + row * C4;
-  float4* dr = reinterpret_cast<float4*>(dx) + row * C4;
+  const float z = LSE ? lse[row] : 0.f;
+  const T* yr = y + row * C4 * 4;
+  T* dr = dx + row * C4 * 4;
   for (long long c = (long long)blockIdx.x * blockDim.x + threadIdx.x; c < C4;
        c += (long long)gridDim.x * blockDim.x) {
     float4 v = make_float4(0.f, 0.f, 0.f, 0.f);
     if (live) {
-      const float4 l = yr[c];
+      float4 l = load4(yr + 4 * c);
+      if (LSE) l = make_float4(l.x - z, l.y - z, l.z - z, l.w - z);
       v = make_float4(g * expf(l.x), g * expf(l.y), g * expf(l.z), g * expf(l.w));
       if ((t >> 2) == c) {  // the one class that also gets the -1 of the one-hot target
         const int k = t & 3;
@@ -242,8 +285,28 @@ lsm_cce_backward_vec_kernel(const float* __restrict__ y, const float* __restrict
         if (k == 0) v.x = fixed; else if (k == 1) v.y = fixed; else if (k == 2) v.z = fixed; else v.w = fixed;
       }
     }
-    dr[c] = v;
+    if constexpr (sizeof(T) == 4) {
+      *reinterpret_cast<float4*>(dr + 4 * c) = v;
+    } else {
+      const T h[4] = {Num<T>::from_f(v.x), Num<T>::from_f(v.y), Num<T>::from_f(v.z), Num<T>::from_f(v.w)};
+      *reinterpret_cast<uint2*>(dr + 4 * c) = *reinterpret_cast<const uint2*>(h);
+    }
   }
+}
+template <typename T, bool LSE>
+int launch_lsm_cce_backward(const void* y, const float* lse, const float* grad_loss, const int32_t* targets,
+                            const int32_t* count, void* dx, long long C, long long X, int reduction,
+                            int ignore_index, cudaStream_t st) {
+  long long bx = (C / 4 + 255) / 256;
+  if (bx > 64) bx = 64;
+  lsm_cce_backward_vec_kernel<T, LSE><<<dim3((unsigned)bx, (unsigned)X), 256, 0, st>>>(
+      static_cast<const T*>(y), lse, grad_loss, targets, count, static_cast<T*>(dx), C / 4, reduction, ignore_index);
+  FLB200_AFTER_LAUNCH("log_softmax_cce_backward");
+  return FLB200_OK;
+}
+// Rows that a CTA reads in whole vectors (shorter ones are a warp's) and the grid of the gradient takes.
+bool scores_supported(const void* x, long long C, long long X) {
+  return C > 1024 && C % 4 == 0 && C < 0x7fffffffLL && X <= 65535 && aligned16(x);
 }
 
 constexpr int kCceParts = 1024;
@@ -324,10 +387,10 @@ size_t flb200_cce_workspace_bytes(int64_t X) {
   return (size_t)kCceParts * sizeof(float2);
 }
 
-int flb200_cce_forward(const void* logp, const int32_t* targets, float* loss, int32_t* count_out,
-                       int32_t* bad_target_flag, int64_t C, int64_t X, int reduction,
-                       int ignore_index, int dtype, void* workspace, size_t workspace_bytes,
-                       void* stream) {
+static int cce_forward_impl(const void* logp, const float* lse, const int32_t* targets, float* loss,
+                            int32_t* count_out, int32_t* bad_target_flag, int64_t C, int64_t X, int reduction,
+                            int ignore_index, int dtype, void* workspace, size_t workspace_bytes,
+                            void* stream) {
   if (int st = check_reduction("cce_forward", reduction)) return st;
   FLB200_REQUIRE(C >= 1 && X >= 1, "cce_forward: bad extents");
   FLB200_REQUIRE(logp && targets && loss, "cce_forward: null tensor");
@@ -342,17 +405,17 @@ int flb200_cce_forward(const void* logp, const int32_t* targets, float* loss, in
     case FLB200_F32:
       cce_forward_kernel<float><<<grid, 256, 0, st>>>(static_cast<const float*>(logp), targets,
                                                       loss_none, partial, bad_target_flag, C, X,
-                                                      ignore_index);
+                                                      ignore_index, lse);
       break;
     case FLB200_F16:
       cce_forward_kernel<__half><<<grid, 256, 0, st>>>(static_cast<const __half*>(logp), targets,
                                                        loss_none, partial, bad_target_flag, C, X,
-                                                       ignore_index);
+                                                       ignore_index, lse);
       break;
     case FLB200_BF16:
       cce_forward_kernel<__nv_bfloat16><<<grid, 256, 0, st>>>(
           static_cast<const __nv_bfloat16*>(logp), targets, loss_none, partial, bad_target_flag, C,
-          X, ignore_index);
+          X, ignore_index, lse);
       break;
     default:
       return fail(FLB200_UNSUPPORTED, "cce_forward: unknown dtype %d", dtype);
@@ -361,6 +424,72 @@ int flb200_cce_forward(const void* logp, const int32_t* targets, float* loss, in
   cce_finalize_kernel<<<1, 32, 0, st>>>(partial, grid, loss, count_out, reduction);
   FLB200_AFTER_LAUNCH("cce_finalize");
   return FLB200_OK;
+}
+
+int flb200_cce_forward(const void* logp, const int32_t* targets, float* loss, int32_t* count_out,
+                       int32_t* bad_target_flag, int64_t C, int64_t X, int reduction,
+                       int ignore_index, int dtype, void* workspace, size_t workspace_bytes,
+                       void* stream) {
+  return cce_forward_impl(logp, nullptr, targets, loss, count_out, bad_target_flag, C, X, reduction, ignore_index,
+                          dtype, workspace, workspace_bytes, stream);
+}
+
+int flb200_scores_cce_forward(const void* x, float* lse, const int32_t* targets, float* loss,
+                              int32_t* count_out, int32_t* bad_target_flag, int64_t C, int64_t X,
+                              int reduction, int ignore_index, int dtype, void* workspace,
+                              size_t workspace_bytes, void* stream) {
+  FLB200_REQUIRE(C >= 1 && X >= 1, "scores_cce_forward: bad extents");
+  FLB200_REQUIRE(x && lse && targets && loss, "scores_cce_forward: null tensor");
+  if (!scores_supported(x, C, X))
+    return fail(FLB200_UNSUPPORTED, "scores_cce_forward: up to 65535 16-byte aligned rows of more than 1024 "
+                                    "classes, a multiple of 4, only");
+  if (int st = check_reduction("scores_cce_forward", reduction)) return st;
+  if (!workspace || workspace_bytes < flb200_cce_workspace_bytes(X))
+    return fail(FLB200_WORKSPACE_TOO_SMALL, "scores_cce_forward: workspace too small");
+  cudaStream_t st = as_stream(stream);
+  const int grid = grid_for(X, 1);
+  switch (dtype) {
+    case FLB200_F32:
+      row_lse_kernel<<<grid, kRowThreads, 0, st>>>(static_cast<const float*>(x), lse, C / 4, X);
+      break;
+    case FLB200_F16:
+      row_lse_kernel<<<grid, kRowThreads, 0, st>>>(static_cast<const __half*>(x), lse, C / 4, X);
+      break;
+    case FLB200_BF16:
+      row_lse_kernel<<<grid, kRowThreads, 0, st>>>(static_cast<const __nv_bfloat16*>(x), lse, C / 4, X);
+      break;
+    default:
+      return fail(FLB200_UNSUPPORTED, "scores_cce_forward: unknown dtype %d", dtype);
+  }
+  FLB200_AFTER_LAUNCH("row_lse");
+  return cce_forward_impl(x, lse, targets, loss, count_out, bad_target_flag, C, X, reduction, ignore_index, dtype,
+                          workspace, workspace_bytes, stream);
+}
+
+int flb200_scores_cce_backward(const void* x, const float* lse, const float* grad_loss,
+                               const int32_t* targets, const int32_t* count, void* grad_x, int64_t C,
+                               int64_t X, int reduction, int ignore_index, int dtype, void* stream) {
+  FLB200_REQUIRE(C >= 1 && X >= 1, "scores_cce_backward: bad extents");
+  FLB200_REQUIRE(x && lse && grad_loss && targets && grad_x, "scores_cce_backward: null tensor");
+  FLB200_REQUIRE(reduction != FLB200_REDUCE_MEAN || count, "scores_cce_backward: MEAN needs count");
+  if (int st = check_reduction("scores_cce_backward", reduction)) return st;
+  if (!scores_supported(x, C, X) || !aligned16(grad_x))
+    return fail(FLB200_UNSUPPORTED, "scores_cce_backward: up to 65535 16-byte aligned rows of more than 1024 "
+                                    "classes, a multiple of 4, only");
+  cudaStream_t st = as_stream(stream);
+  switch (dtype) {
+    case FLB200_F32:
+      return launch_lsm_cce_backward<float, true>(x, lse, grad_loss, targets, count, grad_x, C, X, reduction,
+                                                  ignore_index, st);
+    case FLB200_F16:
+      return launch_lsm_cce_backward<__half, true>(x, lse, grad_loss, targets, count, grad_x, C, X, reduction,
+                                                   ignore_index, st);
+    case FLB200_BF16:
+      return launch_lsm_cce_backward<__nv_bfloat16, true>(x, lse, grad_loss, targets, count, grad_x, C, X, reduction,
+                                                          ignore_index, st);
+    default:
+      return fail(FLB200_UNSUPPORTED, "scores_cce_backward: unknown dtype %d", dtype);
+  }
 }
 
 int flb200_cce_backward(const float* grad_loss, const int32_t* targets, const int32_t* count,
@@ -406,13 +535,8 @@ int flb200_log_softmax_cce_backward(const void* y, const float* grad_loss, const
   cudaStream_t st = as_stream(stream);
   const int grid = grid_for(C * X, 256 * 4);
   if (dtype == FLB200_F32 && C % 4 == 0 && X <= 65535 && aligned16(y) && aligned16(grad_x)) {
-    long long bx = (C / 4 + 255) / 256;
-    if (bx > 64) bx = 64;
-    lsm_cce_backward_vec_kernel<<<dim3((unsigned)bx, (unsigned)X), 256, 0, st>>>(
-        static_cast<const float*>(y), grad_loss, targets, count, static_cast<float*>(grad_x),
-        C / 4, reduction, ignore_index);
-    FLB200_AFTER_LAUNCH("log_softmax_cce_backward");
-    return FLB200_OK;
+    return launch_lsm_cce_backward<float, false>(y, nullptr, grad_loss, targets, count, grad_x, C, X, reduction,
+                                                 ignore_index, st);
   }
   switch (dtype) {
     case FLB200_F32:

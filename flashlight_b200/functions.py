@@ -230,6 +230,25 @@ def log_softmax_cross_entropy_backward(y, grad_loss, state: CrossEntropyState):
                                       state.ignore_index)
 
 
+def scores_cross_entropy(x, targets, reduction: int = L.REDUCE_MEAN, ignore_index: int = -1):
+    """categoricalCrossEntropy(logSoftmax(x)) in fp32 arithmetic whatever the type of the scores, without
+    the log-probabilities in memory.  Returns (loss, state, lse), or None where the library has no kernel
+    for the rows (see flb200_scores_cce_forward)."""
+    if targets.numel() * x.shape[-1] != x.numel():
+        raise ValueError("dimension mismatch in categorical cross entropy")
+    if targets.dtype != torch.int32:
+        targets = targets.to(torch.int32)
+    out = N.scores_cce_forward(x, targets, reduction, ignore_index)
+    if out is None:
+        return None
+    return out[0], CrossEntropyState(targets, out[1], reduction, ignore_index), out[2]
+
+
+def scores_cross_entropy_backward(x, lse, grad_loss, state: CrossEntropyState):
+    return N.scores_cce_backward(x, lse, grad_loss, state.targets, state.count, state.reduction,
+                                 state.ignore_index)
+
+
 # ------------------------------------------------------------------ embedding
 def embedding(table, ids):
     """fl::embedding forward: rows of `table` (vocab, dim) picked by `ids` (any shape)."""

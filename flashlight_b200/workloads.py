@@ -253,7 +253,7 @@ class TransformerLM(nn.Module):
         # bf16 compute with fp32 master weights: parameters stay fp32; the matrices and the
         # embedding are cast to bf16 where they are used and their gradients come back as fp32
         # (autograd.cast); biases and LayerNorm parameters are used in fp32 by the kernels or
-        # cast likewise; the class scores are cast to fp32 for the loss.
+        # cast likewise; the loss is that of the class scores cast to fp32.
         self.compute_dtype = compute_dtype
         mk = lambda i, o: nn.Linear(i, o, True, gen, device)
         ones = lambda n: Variable(torch.ones(n, device=device), True)
@@ -325,5 +325,5 @@ class TransformerLM(nn.Module):
             x = A.add(x, self._attention(self._ln(x, blk["ln1"]), blk, B, T, mask))
             h = self._lin(blk["w1"], self._ln(x, blk["ln2"]), gelu=True)  # Linear + bias + GELU
             x = A.add(x, self._lin(blk["w2"], h))
-        scores = A.cast(self._lin(self.head, self._ln(x, self.ln_f)), torch.float32)
-        return A.log_softmax_cross_entropy(scores, targets)
+        scores = self._lin(self.head, self._ln(x, self.ln_f))
+        return A.log_softmax_cross_entropy(scores, targets, wide=True)

@@ -587,6 +587,19 @@ int flb200_log_softmax_cce_backward(const void* y, const float* grad_loss,
                                     const int32_t* targets, const int32_t* count,
                                     void* grad_x, int64_t C, int64_t X, int reduction,
                                     int ignore_index, int dtype, void* stream);
+/* categoricalCrossEntropy(logSoftmax(x)) and its gradient straight from the scores x [C,X] in the arithmetic
+ * of fp32 (16-bit scores as if copied to fp32 before, their gradient rounded once).  Of logSoftmax only
+ * lse [X], the log of the sum of each row's exponentials, is kept.  FLB200_UNSUPPORTED unless C is a multiple
+ * of 4 above 1024, X <= 65535 and the tensors are 16-byte aligned.  The rest as flb200_cce_forward and
+ * flb200_log_softmax_cce_backward; workspace: flb200_cce_workspace_bytes. */
+int flb200_scores_cce_forward(const void* x, float* lse, const int32_t* targets, float* loss,
+                              int32_t* count_out, int32_t* bad_target_flag, int64_t C, int64_t X,
+                              int reduction, int ignore_index, int dtype, void* workspace,
+                              size_t workspace_bytes, void* stream);
+int flb200_scores_cce_backward(const void* x, const float* lse, const float* grad_loss,
+                               const int32_t* targets, const int32_t* count, void* grad_x,
+                               int64_t C, int64_t X, int reduction, int ignore_index, int dtype,
+                               void* stream);
 
 /* ----------------------------------------------------------- rnn (a7, a8) */
 /* x [I,B,T], y [H*dirs,B,T], hx/cx/hy/cy [H,B,L*dirs]; w flat in the cuDNN
