@@ -113,6 +113,7 @@ SIGNATURES = {
     "flb200_batchnorm_relu_backward_sum": (C.c_int, [P(BatchnormDesc), vp, vp, vp, vp, vp, vp, vp, vp,
                                                      vp, vp, vp, vp, sz, vp]),
     "flb200_matmul_workspace_bytes": (sz, [P(MatmulDesc)]),
+    "flb200_matmul_call_workspace_bytes": (sz, [P(MatmulDesc), vp, vp, vp]),
     "flb200_matmul": (C.c_int, [P(MatmulDesc), vp, vp, vp, vp, sz, vp]),
     "flb200_matmul_wide": (C.c_int, [P(MatmulDesc), vp, vp, vp, vp, sz, vp]),
     "flb200_linear_workspace_bytes": (sz, [i64, i64, i64, C.c_int]),

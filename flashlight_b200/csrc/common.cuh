@@ -3,6 +3,8 @@
 
 #include <type_traits>
 #include <cuda_runtime.h>
+
+#include <cstring>
 #include <cuda_fp16.h>
 #include <cuda_bf16.h>
 
@@ -29,6 +31,36 @@ struct DeviceInfo {
   int cc_minor = 0;
 };
 const DeviceInfo& device_info();
+
+// A thread's last answers to a question that its Key (plain bytes) decides, as the scratch queries are: an
+// operator asks several, and weighing the plans behind one takes 0.3 us each, up to sixteen of them.
+template <typename Key, typename Value, int N = 256>
+class Memo {
+ public:
+  // The answer kept for `key`, or null; put() then keeps one in its place.
+  const Value* find(const Key& key) {
+    unsigned long long h = 1469598103934665603ull;
+    const unsigned char* p = reinterpret_cast<const unsigned char*>(&key);
+    for (size_t i = 0; i + 4 <= sizeof(Key); i += 4) {
+      unsigned w;
+      memcpy(&w, p + i, 4);
+      h = (h ^ w) * 1099511628211ull;
+    }
+    at_ = &entries_[(h ^ (h >> 32)) % N];
+    return at_->used && memcmp(&at_->key, &key, sizeof(Key)) == 0 ? &at_->value : nullptr;
+  }
+  const Value& put(const Key& key, const Value& value) {
+    memcpy(&at_->key, &key, sizeof(Key));
+    at_->value = value;
+    at_->used = true;
+    return at_->value;
+  }
+
+ private:
+  struct Entry { bool used; Key key; Value value; };
+  Entry entries_[N] = {};
+  Entry* at_ = nullptr;
+};
 
 inline cudaStream_t as_stream(void* s) { return reinterpret_cast<cudaStream_t>(s); }
 

@@ -578,9 +578,19 @@ int flb200_conv2d_output_dims(const flb200_conv2d_desc* d, int32_t* Wo, int32_t*
   return FLB200_OK;
 }
 
-size_t flb200_conv2d_workspace_bytes(const flb200_conv2d_desc* d, int which) {
-  ConvGeo g;
-  if (make_conv_geo("conv2d_workspace_bytes", d, &g)) return 0;
+// Key of the three queries below.  (A call with a descriptor that they refuse is not kept: it sets the
+// error text again.)
+struct ConvQuery { flb200_conv2d_desc d; int which, sm, cc, outer_x3; };
+static ConvQuery conv_query(const flb200_conv2d_desc* d, int which) {
+  ConvQuery q;
+  memset(&q, 0, sizeof(q));
+  q.d = *d;
+  const DeviceInfo& di = device_info();
+  q.which = which; q.sm = di.sm_count; q.cc = di.cc_major; q.outer_x3 = tc::x3_enabled() ? 1 : 0;
+  return q;
+}
+
+static size_t conv2d_workspace_bytes(const flb200_conv2d_desc* d, int which, ConvGeo g) {
   size_t need = 0;
   if (which == 0) {
     need = strict_scratch_bytes(g, 0) +
@@ -604,6 +614,18 @@ size_t flb200_conv2d_workspace_bytes(const flb200_conv2d_desc* d, int which) {
   return need;
 }
 
+size_t flb200_conv2d_workspace_bytes(const flb200_conv2d_desc* d, int which) {
+  static thread_local Memo<ConvQuery, size_t> memo;
+  ConvQuery q;
+  if (d) {
+    q = conv_query(d, which);
+    if (const size_t* known = memo.find(q)) return *known;
+  }
+  ConvGeo g;
+  if (make_conv_geo("conv2d_workspace_bytes", d, &g)) return 0;
+  return memo.put(q, conv2d_workspace_bytes(d, which, g));
+}
+
 int flb200_conv2d_forward(const flb200_conv2d_desc* d, const void* x, const void* w,
                           const void* bias, void* y, void* workspace, size_t workspace_bytes,
                           void* stream) {
@@ -612,10 +634,16 @@ int flb200_conv2d_forward(const flb200_conv2d_desc* d, const void* x, const void
 }
 
 size_t flb200_conv2d_cache_bytes(const flb200_conv2d_desc* d, int which) {
+  static thread_local Memo<ConvQuery, size_t> memo;
+  ConvQuery q;
+  if (d) {
+    q = conv_query(d, which);
+    if (const size_t* known = memo.find(q)) return *known;
+  }
   ConvGeo g;
   if (make_conv_geo("conv2d_cache_bytes", d, &g)) return 0;
   if (d->math_mode == FLB200_MATH_STRICT_F32 || which < 0 || which > 1) return 0;
-  return tc_conv_cache_bytes(g, which);
+  return memo.put(q, tc_conv_cache_bytes(g, which));
 }
 
 int flb200_conv2d_forward_cached(const flb200_conv2d_desc* d, const void* x, const void* w,
@@ -669,17 +697,30 @@ int flb200_conv2d_forward_cached(const flb200_conv2d_desc* d, const void* x, con
   return strict_image_pass<false>("conv2d_forward", g, xf, wf, bf, yf, workspace, workspace_bytes, st);
 }
 
-size_t flb200_conv2d_stats_bytes(const flb200_conv2d_desc* d, int64_t* groups) {
-  ConvGeo g;
-  if (groups) *groups = 0;
-  if (make_conv_geo("conv2d_stats_bytes", d, &g)) return 0;
+static long long conv2d_stats_groups(const flb200_conv2d_desc* d, ConvGeo g) {
   if (d->math_mode == FLB200_MATH_STRICT_F32 || (d->dtype != FLB200_F32 && !native16(d, &g, 0))) return 0;
   tc::X3Scope x3(g.operand == tc::kOperandTf32 && d->math_mode == FLB200_MATH_F32X3);
   const long long n = tc_conv_stats_groups(g);
-  if (n == 0 || !tc_conv_supported(g, 0, tc_conv_workspace_bytes(g, 0))) return 0;
-  if (groups) *groups = n;
+  return n == 0 || !tc_conv_supported(g, 0, tc_conv_workspace_bytes(g, 0)) ? 0 : n;
+}
+size_t flb200_conv2d_stats_bytes(const flb200_conv2d_desc* d, int64_t* groups) {
+  static thread_local Memo<ConvQuery, long long> memo;
+  if (groups) *groups = 0;
+  ConvQuery q;
+  const long long* n = nullptr;
+  if (d) {
+    q = conv_query(d, 0);
+    n = memo.find(q);
+  }
+  if (!n) {
+    ConvGeo g;
+    if (make_conv_geo("conv2d_stats_bytes", d, &g)) return 0;
+    n = &memo.put(q, conv2d_stats_groups(d, g));
+  }
+  if (*n == 0) return 0;
+  if (groups) *groups = *n;
   // CTA pairs may write one phantom tile (four all-zero rows) past the last real one
-  return (size_t)(n + 4) * 2 * g.Cout * sizeof(float);
+  return (size_t)(*n + 4) * 2 * d->Cout * sizeof(float);
 }
 
 int flb200_conv2d_forward_stats(const flb200_conv2d_desc* d, const void* x, const void* w,

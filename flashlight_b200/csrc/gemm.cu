@@ -106,9 +106,23 @@ extern "C" {
 
 size_t flb200_matmul_workspace_bytes(const flb200_matmul_desc* d) {
   if (!d || d->m <= 0 || d->n <= 0 || d->batch <= 0) return 0;
+  struct Key { long long m, n, k, batch; int mode, sm, cc, outer_x3; };
+  static thread_local Memo<Key, size_t> memo;
+  const DeviceInfo& di = device_info();
+  const Key key = {d->m, d->n, d->k, d->batch, d->math_mode, di.sm_count, di.cc_major, tc::x3_enabled() ? 1 : 0};
+  if (const size_t* known = memo.find(key)) return *known;
   size_t need = plan_simt(d->m, d->n, d->k, d->batch).workspace_bytes;
   const size_t tc = tc_gemm_workspace_bytes(d);
-  return need > tc ? need : tc;
+  return memo.put(key, need > tc ? need : tc);
+}
+
+size_t flb200_matmul_call_workspace_bytes(const flb200_matmul_desc* d, const void* a, const void* b,
+                                          const void* c) {
+  if (check_desc(d, a, b, c) || d->m == 0 || d->n == 0) return 0;
+  tc::X3Scope x3(d->dtype == FLB200_F32 && d->math_mode == FLB200_MATH_F32X3);
+  if ((d->dtype == FLB200_BF16 || d->math_mode != FLB200_MATH_STRICT_F32) && tc_gemm_supported(d, a, b, c))
+    return tc_gemm_call_workspace_bytes(d, a, b, c);
+  return flb200_matmul_workspace_bytes(d);
 }
 
 int flb200_matmul(const flb200_matmul_desc* d, const void* a, const void* b, void* c,

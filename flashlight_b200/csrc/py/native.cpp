@@ -402,7 +402,11 @@ NATIVE(linear_bias_act) {  // (x, weight, bias or None, gelu, mode) -> (y, pre) 
     Py_RETURN_NONE;
   Tensor y = rows_of(in, d.O), pre;
   if (gelu) pre = empty_like(y);
-  Workspace ws(flb200_linear_workspace_bytes(d.O, d.I, d.cols, 0), in);
+  flb200_matmul_desc m = {};  // the product that the call runs
+  m.m = d.cols; m.n = d.O; m.k = d.I; m.batch = 1;
+  m.a_row = d.I; m.a_col = 1; m.b_row = d.O; m.b_col = 1; m.c_row = d.O; m.c_col = 1;
+  m.alpha = 1.f; m.dtype = code_of(in); m.math_mode = mode;
+  Workspace ws(flb200_matmul_call_workspace_bytes(&m, P(in), P(w), P(y)), in);
   const int st = unlocked(
       flb200_linear_bias_act_forward, d.O, d.I, d.cols, P(w), P(in), Pf(bias), P(y), gelu ? P(pre) : nullptr,
       gelu ? FLB200_ACT_GELU : FLB200_ACT_NONE, code_of(in), mode, ws.p(), ws.bytes, stream());
@@ -459,7 +463,7 @@ NATIVE(matmul) {
   }
   d.alpha = (float)x.d(16); d.beta = (float)x.d(17);
   d.dtype = code_of(a); d.math_mode = x.n32(18);
-  Workspace ws(flb200_matmul_workspace_bytes(&d), a);
+  Workspace ws(flb200_matmul_call_workspace_bytes(&d, P(a), P(b), P(c)), a);
   check(wide ? unlocked(flb200_matmul_wide, &d, P(a), P(b), Pf(&c), ws.p(), ws.bytes, stream())
              : unlocked(flb200_matmul, &d, P(a), P(b), P(c), ws.p(), ws.bytes, stream()));
   return wrap(c);

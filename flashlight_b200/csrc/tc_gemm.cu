@@ -62,7 +62,7 @@ int make_tensor_map(CUtensorMap* map, const void* base, int rank, const uint64_t
     int rank, mode, operand, used;
   };
   struct Entry { Key key; CUtensorMap map; };
-  static thread_local Entry known[128] = {};
+  static thread_local Entry known[512] = {};
   Key key;
   memset(&key, 0, sizeof(key));
   key.base = base;
@@ -73,7 +73,7 @@ int make_tensor_map(CUtensorMap* map, const void* base, int rank, const uint64_t
     if (i > 0) key.gs[i - 1] = gs[i - 1];
     h = h * 31 + gd[i] + 17 * bx[i];
   }
-  Entry& e = known[(h * 0x9e3779b97f4a7c15ull) >> 57];
+  Entry& e = known[(h * 0x9e3779b97f4a7c15ull) >> 55];
   if (memcmp(&e.key, &key, sizeof(key)) == 0) {
     *map = e.map;
     return FLB200_OK;
@@ -374,14 +374,14 @@ static Launch compute_launch(long long M, long long N, long long k_iters, long l
 Launch plan_launch(long long M, long long N, long long k_iters, long long Z, bool a_mn_major,
                    bool b_mn_major, int operand, bool split_k) {
   struct Entry { long long m, n, k, z, rest; Launch plan; };
-  static thread_local Entry known[64] = {};
+  static thread_local Entry known[256] = {};
   const long long sm = device_info().sm_count > 0 ? device_info().sm_count : 148;
   const bool x3 = x3_enabled();
   if (k_iters < 1) k_iters = 1;
   const long long rest = 1 + (a_mn_major ? 2 : 0) + (b_mn_major ? 4 : 0) + (split_k ? 8 : 0) +
                          (x3 ? 16 : 0) + operand * 32LL + sm * 256;
   const unsigned long long h = ((unsigned long long)(M * 31 + N) * 31 + k_iters * 7 + Z) * 31 + rest;
-  Entry& e = known[(h * 0x9e3779b97f4a7c15ull) >> 58];
+  Entry& e = known[(h * 0x9e3779b97f4a7c15ull) >> 56];
   if (e.m != M || e.n != N || e.k != k_iters || e.z != Z || e.rest != rest)
     e = Entry{M, N, k_iters, Z, rest,
               compute_launch(M, N, k_iters, Z, a_mn_major, b_mn_major, operand, split_k, sm, x3)};
@@ -548,6 +548,16 @@ size_t tc_gemm_workspace_bytes(const flb200_matmul_desc* d) {
       }
   }
   return need;
+}
+
+size_t tc_gemm_call_workspace_bytes(const flb200_matmul_desc* d, const void* a, const void* b, const void* c) {
+  const Prepared p = prepare(d, a, b, c);
+  if (!p.ok) return 0;
+  const int operand = tc::operand_of(d->dtype);
+  const long long kstage = tc::stage_k(operand);
+  return tc::plan_launch(p.swap ? d->n : d->m, p.swap ? d->m : d->n, (d->k + kstage - 1) / kstage, d->batch,
+                         (p.swap ? p.b : p.a).mn_major, (p.swap ? p.a : p.b).mn_major, operand, true)
+      .workspace_bytes;
 }
 
 int tc_gemm_run(const flb200_matmul_desc* d, const void* a, const void* b, void* c, void* ws,

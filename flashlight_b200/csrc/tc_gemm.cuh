@@ -12,6 +12,8 @@ namespace flb200 {
 // True when the tensor-core kernel covers this problem (layout, alignment, size).
 bool tc_gemm_supported(const flb200_matmul_desc* d, const void* a, const void* b, const void* c);
 size_t tc_gemm_workspace_bytes(const flb200_matmul_desc* d);
+// The scratch that tc_gemm_run plans with for these operands (0: it would not split K).
+size_t tc_gemm_call_workspace_bytes(const flb200_matmul_desc* d, const void* a, const void* b, const void* c);
 // bias_n / act / pre: per-column bias, activation and pre-activation copy fused into the store
 // (EpiloguePlan); only for products whose result is stored row-major as the caller's C
 // (FLB200_UNSUPPORTED otherwise, so that the caller can run the operators one by one).

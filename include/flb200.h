@@ -333,6 +333,10 @@ typedef struct flb200_matmul_desc {
 } flb200_matmul_desc;
 
 size_t flb200_matmul_workspace_bytes(const flb200_matmul_desc* d);
+/* The same for a call with these operands, whose alignment decides the kernel: what it will use, 0 where it
+ * needs none (the query above answers for every alignment and operand type). */
+size_t flb200_matmul_call_workspace_bytes(const flb200_matmul_desc* d, const void* a,
+                                          const void* b, const void* c);
 int flb200_matmul(const flb200_matmul_desc* d, const void* a, const void* b, void* c,
                   void* workspace, size_t workspace_bytes, void* stream);
 /* The same with an f32 C whatever the operands' type: the gradient of fp32 master weights from bf16
