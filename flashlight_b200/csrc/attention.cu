@@ -25,7 +25,10 @@
 // operand (rows = m or n, 64 k per row) or as an MN-major operand (rows = k, 64 m or n per
 // row), so Q_i, dO_i and K_j are used as TMA delivered them, and P / dS (two 64-key halves,
 // 16 KB apart) feed both the transposed products and dS K_j.  dQ blocks of different CTAs are
-// summed with fp32 atomics into scratch and rounded to bf16 by a second small kernel.
+// summed in fp32 into scratch, a bulk reduction each, and rounded to bf16 by a second small kernel.
+// The chain from contraction to softmax to contraction bounds it, with one CTA per SM (its tiles and
+// accumulators fill both memories): so Q_i+2 and dO_i+2 are fetched behind block i, S and dP of block i + 1
+// run behind its gradients, and dQ comes first of these, its sums leaving while dV and dK are made.
 // Every mbarrier wait is bounded (tc_core.cuh): a wait that runs out raises the library's status
 // flag and the CTA finishes its loop without waiting again.
 #include <cuda_bf16.h>
@@ -50,7 +53,8 @@ using namespace tc;
 constexpr int kAttnThreads = 288;      // warps 0..7: two threads per query row (each half of the
                                        // columns); warp 8: TMA + MMA
 constexpr int kTile = 128 * 128;       // bytes of a [128 rows][64 bf16] tile
-constexpr int kAttnSmem = 4 * kTile + 2 * 2 * kTile + 1024 + 256;  // K V Q dO, P dS, align, bars
+// K V, two buffers of Q dO, P dS, dQ (fp32), align, bars
+constexpr int kAttnSmem = 2 * kTile + 4 * kTile + 2 * 2 * kTile + 2 * kTile + 1024 + 256;
 
 // element (batch b, head h, position t, d) of a tensor is at b * batch + h * head + t * row + d
 struct HeadStrides { long long batch, head, row; };
@@ -74,10 +78,13 @@ __device__ __forceinline__ uint32_t score_chunk(int r, int key0) {
          ((((uint32_t)(key0 & 63) >> 3) ^ ((uint32_t)r & 7)) << 4);
 }
 
-// four consecutive fp32 sums in one reduction instruction (16-byte aligned address)
-__device__ __forceinline__ void red_add_v4(float* p, float a, float b, float c, float d) {
-  asm volatile("red.global.add.v4.f32 [%0], {%1, %2, %3, %4};" ::"l"(p), "f"(a), "f"(b), "f"(c),
-               "f"(d)
+// Row r of a dQ block is 64 floats in 16 chunks; chunk q is kept at q ^ (r & 15), in shared memory for the sake
+// of the banks and so in the fp32 sums too (narrow_dq_kernel reads it back).
+__device__ __forceinline__ int dq_chunk(int r, int q) { return q ^ (r & 15); }
+// adds `bytes` of fp32 in shared memory to device memory, asynchronously
+__device__ __forceinline__ void bulk_add(float* dst, const void* src, uint32_t bytes) {
+  asm volatile("cp.reduce.async.bulk.global.shared::cta.bulk_group.add.f32 [%0], [%1], %2;" ::"l"(dst),
+               "r"(smem_u32(src)), "r"(bytes)
                : "memory");
 }
 
@@ -131,17 +138,19 @@ attention_backward_kernel(const __grid_constant__ CUtensorMap map_q,
                                        ~static_cast<uintptr_t>(1023));
   char* sK = base;
   char* sV = base + kTile;
-  char* sQ = base + 2 * kTile;
+  char* sQ = base + 2 * kTile;   // the second buffer of both 2 tiles further
   char* sDO = base + 3 * kTile;
-  char* sP = base + 4 * kTile;   // two 64-key halves
-  char* sDS = base + 6 * kTile;  // two 64-key halves
-  uint64_t* bars = reinterpret_cast<uint64_t*>(base + 8 * kTile);
+  char* sP = base + 6 * kTile;   // two 64-key halves
+  char* sDS = base + 8 * kTile;  // two 64-key halves
+  char* sDQ = base + 10 * kTile;
+  uint64_t* bars = reinterpret_cast<uint64_t*>(base + 12 * kTile);
   uint64_t* bar_kv = bars;      // K_j, V_j landed
-  uint64_t* bar_q = bars + 1;   // Q_i, dO_i landed
-  uint64_t* bar_s = bars + 2;   // S and dP complete
-  uint64_t* bar_o = bars + 3;   // dV, dK, dQ contractions complete
-  uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(bars + 4);
-  int* failed = reinterpret_cast<int*>(bars + 5);
+  uint64_t* bar_q = bars + 1;   // [2] Q_i, dO_i landed
+  uint64_t* bar_s = bars + 3;   // S and dP complete
+  uint64_t* bar_dq = bars + 4;  // dQ contraction complete
+  uint64_t* bar_o = bars + 5;   // dV and dK contractions complete
+  uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(bars + 6);
+  volatile int* failed = reinterpret_cast<volatile int*>(bars + 7);
 
   const int warp = __shfl_sync(0xffffffffu, threadIdx.x >> 5, 0), lane = threadIdx.x & 31;
   const int nblk = (a.T + 127) / 128;
@@ -151,10 +160,7 @@ attention_backward_kernel(const __grid_constant__ CUtensorMap map_q,
   const long long row0 = (long long)bh * a.T;  // first row of this head in lse, dsum and dq_acc
 
   if (threadIdx.x == 0) {
-    mbar_init(bar_kv, 1);
-    mbar_init(bar_q, 1);
-    mbar_init(bar_s, 1);
-    mbar_init(bar_o, 1);
+    for (int k = 0; k < 6; ++k) mbar_init(bars + k, 1);
     *failed = 0;
     fence_barrier_init();
   }
@@ -183,12 +189,47 @@ attention_backward_kernel(const __grid_constant__ CUtensorMap map_q,
   const uint32_t id_t = umma_idesc_f16(kOperandBf16, 64, 1, 1);    // dV, dK: both operands MN-major
   const uint32_t id_q = umma_idesc_f16(kOperandBf16, 64, 0, 1);    // dQ: dS K-major, K_j MN-major
 
+  auto wait = [&](uint64_t* bar, uint32_t phase, int code) {
+    if (*failed == 0 && !mbar_wait(bar, phase)) *failed = code;
+    tc_fence_after();
+  };
+  auto load_q = [&](int i, uint32_t buf) {
+    mbar_expect_tx(&bar_q[buf], 2 * kTile);
+    int c[4] = {0, i * 128, head, batch};
+    tma_load(&map_q, &bar_q[buf], sQ + buf * 2 * kTile, 4, c);
+    tma_load(&map_do, &bar_q[buf], sDO + buf * 2 * kTile, 4, c);
+  };
+  auto scores = [&](uint32_t buf, uint32_t phase) {
+    wait(&bar_q[buf], phase, 2);
+    const uint32_t off = buf * 2 * kTile;
+#pragma unroll
+    for (int kk = 0; kk < 4; ++kk)  // K = 64 d in steps of 16
+      umma_f16(tmem, umma_desc_advance(dQ_k, off + kk * 32), umma_desc_advance(dK_k, kk * 32), id_s, kk > 0);
+#pragma unroll
+    for (int kk = 0; kk < 4; ++kk)
+      umma_f16(tmem + 128, umma_desc_advance(dDO_k, off + kk * 32), umma_desc_advance(dV_k, kk * 32), id_s, kk > 0);
+    umma_commit(bar_s);
+  };
+  const int i_first = a.causal ? j : 0, blocks = nblk - i_first;
   if (warp == 8 && elect_one()) {
     mbar_expect_tx(bar_kv, 2 * kTile);
     int c[4] = {0, j * 128, head, batch};
     tma_load(&map_k, bar_kv, sK, 4, c);
+    load_q(i_first, 0);
     tma_load(&map_v, bar_kv, sV, 4, c);
+    if (blocks > 1) load_q(i_first + 1, 1);
+    wait(bar_kv, 0, 1);
+    scores(0, 0);
   }
+  float lse = 0.f, dsum = 0.f;
+  auto fetch_row = [&](int i) {
+    lse = dsum = 0.f;
+    if (row_thread && i * 128 + r < a.T) {
+      dsum = a.dsum[row0 + (long long)i * 128 + r];
+      lse = a.lse[row0 + (long long)i * 128 + r];
+    }
+  };
+  fetch_row(i_first);
 
 #ifdef FLB200_ATTN_PROFILE
   long long pc[6] = {0, 0, 0, 0, 0, 0};
@@ -197,44 +238,16 @@ attention_backward_kernel(const __grid_constant__ CUtensorMap map_q,
 #else
 #define ATTN_MARK(k, t)
 #endif
-  const int i_first = a.causal ? j : 0;
-  uint32_t it = 0;
-  for (int i = i_first; i < nblk; ++i, ++it) {
+  const uint32_t lane_addr = tmem + ((uint32_t)((warp & 3) * 32) << 16);
+  for (int it = 0; it < blocks; ++it) {
+    const int i = i_first + it;
     const uint32_t ph = it & 1;
-    const long long qrow = row0 + (long long)i * 128;
-    __syncwarp();
-    if (warp == 8 && elect_one()) {
-      mbar_expect_tx(bar_q, 2 * kTile);
-      int c[4] = {0, i * 128, head, batch};
-      tma_load(&map_q, bar_q, sQ, 4, c);
-      tma_load(&map_do, bar_q, sDO, 4, c);
-      if (it == 0 && *failed == 0 && !mbar_wait(bar_kv, 0)) *failed = 1;
-      if (*failed == 0 && !mbar_wait(bar_q, ph)) *failed = 2;
-      tc_fence_after();
-#pragma unroll
-      for (int kk = 0; kk < 4; ++kk)  // K = 64 d in steps of 16
-        umma_f16(tmem, umma_desc_advance(dQ_k, kk * 32), umma_desc_advance(dK_k, kk * 32), id_s,
-                  kk > 0);
-#pragma unroll
-      for (int kk = 0; kk < 4; ++kk)
-        umma_f16(tmem + 128, umma_desc_advance(dDO_k, kk * 32), umma_desc_advance(dV_k, kk * 32),
-                  id_s, kk > 0);
-      umma_commit(bar_s);
-    }
-    float lse = 0.f, dsum = 0.f;
     if (row_thread) {
-      if (i * 128 + r < a.T) {
-        dsum = a.dsum[qrow + r];
-        lse = a.lse[qrow + r];
-      }
-      ATTN_MARK(0, tp);
-      if (*failed == 0 && !mbar_wait(bar_s, ph)) *failed = 3;
-      tc_fence_after();
+      wait(bar_s, ph, 3);
       ATTN_MARK(1, tp);
-      const uint32_t lane_addr = tmem + ((uint32_t)((warp & 3) * 32) << 16);
       const int q_pos = i * 128 + r;
       // Keys in front of `live` count; blocks off the diagonal and the ends have no others, and the test
-      // per element is most of what such a block costs (4900 clocks of a step's 9300, now 2000).
+      // per element is most of what such a block costs (4900 clocks, without it 1750).
       const bool whole = !(a.causal && i == j) && (i + 1) * 128 <= a.T && (j + 1) * 128 <= a.T;
       const int live = q_pos >= a.T ? 0 : min(a.T, a.causal ? q_pos + 1 : a.T) - j * 128;
       const float scale2 = a.scale * kLog2e, lse2 = lse * kLog2e, dsum_s = a.scale * dsum;
@@ -256,6 +269,8 @@ attention_backward_kernel(const __grid_constant__ CUtensorMap map_q,
             dp[e] = p * fmaf(dp[e], a.scale, -dsum_s);
           }
         }
+        // the last block's dV and dK have read P and dS
+        if (it > 0 && c0 == 64 * half) wait(bar_o, ph ^ 1, 4);
 #pragma unroll
         for (int u = 0; u < 4; ++u) {
           const uint32_t off = score_chunk(r, c0 + 8 * u);
@@ -268,62 +283,76 @@ attention_backward_kernel(const __grid_constant__ CUtensorMap map_q,
         }
       }
       fence_proxy_async();  // the tensor core reads these generic-proxy writes next
+      if (threadIdx.x == 0) bulk_wait_read<0>();  // the last dQ has left its tile
       ATTN_MARK(2, tp);
     }
     tc_fence_before();
-    __syncthreads();
-    if (warp == 8 && elect_one()) {
-      tc_fence_after();
+    __syncthreads();  // P and dS are complete; S, dP and the last dQ have been read
+    if (warp == 8) {
+      if (elect_one()) {
+        const uint32_t off = ph * 2 * kTile;
+        tc_fence_after();
 #pragma unroll
-      for (int kk = 0; kk < 8; ++kk) {  // K = 128 query rows in steps of 16
-        umma_f16(tmem + 256, umma_desc_advance(dP_mn, kk * 2048),
-                  umma_desc_advance(dDO_mn, kk * 2048), id_t, (it > 0 || kk > 0) ? 1u : 0u);
-        umma_f16(tmem + 320, umma_desc_advance(dDS_mn, kk * 2048),
-                  umma_desc_advance(dQ_mn, kk * 2048), id_t, (it > 0 || kk > 0) ? 1u : 0u);
+        for (int kk = 0; kk < 8; ++kk)  // K = 128 keys: two 64-key halves of dS, 16 key rows of K_j
+          umma_f16(tmem + 384, umma_desc_advance(dDS_k, (kk >> 2) * kTile + (kk & 3) * 32),
+                   umma_desc_advance(dK_mn, kk * 2048), id_q, kk > 0);
+        umma_commit(bar_dq);
+#pragma unroll
+        for (int kk = 0; kk < 8; ++kk) {  // K = 128 query rows in steps of 16
+          umma_f16(tmem + 256, umma_desc_advance(dP_mn, kk * 2048),
+                   umma_desc_advance(dDO_mn, off + kk * 2048), id_t, (it > 0 || kk > 0) ? 1u : 0u);
+          umma_f16(tmem + 320, umma_desc_advance(dDS_mn, kk * 2048),
+                   umma_desc_advance(dQ_mn, off + kk * 2048), id_t, (it > 0 || kk > 0) ? 1u : 0u);
+        }
+        umma_commit(bar_o);
+        if (it + 1 < blocks) scores(ph ^ 1, ((it + 1) >> 1) & 1);
+        if (it + 2 < blocks) {
+          wait(bar_o, ph, 4);
+          load_q(i + 2, ph);
+        }
       }
-#pragma unroll
-      for (int kk = 0; kk < 8; ++kk)  // K = 128 keys: two 64-key halves of dS, 16 key rows of K_j
-        umma_f16(tmem + 384, umma_desc_advance(dDS_k, (kk >> 2) * kTile + (kk & 3) * 32),
-                  umma_desc_advance(dK_mn, kk * 2048), id_q, kk > 0);
-      umma_commit(bar_o);
-    }
-    if (*failed == 0 && !mbar_wait(bar_o, ph)) *failed = 4;
-    tc_fence_after();
-    if (row_thread) {
+      __syncwarp();
+    } else {
+      if (it + 1 < blocks) fetch_row(i + 1);
+      wait(bar_dq, ph, 5);
       ATTN_MARK(3, tp);
-      float* dst = a.dq_acc + (qrow + r) * 64 + 32 * half;
       float v[32];
-      tmem_ld32(tmem + ((uint32_t)((warp & 3) * 32) << 16) + 384u + 32u * half, v);
+      tmem_ld32(lane_addr + 384u + 32u * half, v);
+      float4* to = reinterpret_cast<float4*>(sDQ) + r * 16;
 #pragma unroll
       for (int e = 0; e < 32; e += 4)
-        if (i * 128 + r < a.T) red_add_v4(dst + e, v[e], v[e + 1], v[e + 2], v[e + 3]);
+        to[dq_chunk(r, 8 * half + e / 4)] = make_float4(v[e], v[e + 1], v[e + 2], v[e + 3]);
+      fence_proxy_async();
+      asm volatile("bar.sync 1, 256;" ::: "memory");  // the row threads
+      if (threadIdx.x == 0) {
+        bulk_add(a.dq_acc + (row0 + (long long)i * 128) * 64, sDQ, (uint32_t)min(128, a.T - i * 128) * 256u);
+        bulk_commit();
+      }
       ATTN_MARK(4, tp);
     }
-    // the next block's loads and contractions overwrite Q_i, dO_i, S, dP, P, dS and dQ
-    tc_fence_before();
-    __syncthreads();
-    tc_fence_after();
-#ifdef FLB200_ATTN_PROFILE
-    if (row_thread) { ATTN_MARK(5, tp); }
-#endif
   }
+  if (*failed)  // copies and contractions under way when a wait ran out have ended after this
+    for (const long long t0 = clock64(); clock64() - t0 < 100000;) {
+    }
+  if (row_thread) wait(bar_o, (blocks - 1) & 1, 4);
+  if (threadIdx.x == 0) bulk_wait<0>();
 #ifdef FLB200_ATTN_PROFILE
   if (blockIdx.x == 0 && threadIdx.x == 0)
-    printf("attention profile (CTA 0, %u blocks): D+lse %lld | wait S,dP %lld | softmax %lld | wait dV dK dQ %lld | atomics %lld | sync %lld\n",
-           it, pc[0], pc[1], pc[2], pc[3], pc[4], pc[5]);
+    printf("attention profile (CTA 0, %d blocks): wait S,dP %lld | softmax %lld | wait dQ %lld | dQ %lld\n",
+           blocks, pc[1], pc[2], pc[3], pc[4]);
 #endif
 
   if (row_thread) {
     // the first half of the row threads stores dV_j, the second dK_j
     const int key = j * 128 + r;
-    const uint32_t lane_addr = tmem + ((uint32_t)((warp & 3) * 32) << 16) + 256u + 64u * half;
+    const uint32_t from = lane_addr + 256u + 64u * half;
     __nv_bfloat16* out = (half == 0 ? a.dv : a.dk) + batch * a.gs.batch + head * a.gs.head +
                          (long long)key * a.gs.row;
 #pragma unroll 1
     for (int c0 = 0; c0 < 64; c0 += 32) {
       float v[32];
       __syncwarp();  // the lanes past the end store nothing, and are back for the next load
-      tmem_ld32(lane_addr + (uint32_t)c0, v);
+      tmem_ld32(from + (uint32_t)c0, v);
       if (key < a.T) {
 #pragma unroll
         for (int u = 0; u < 4; ++u)
@@ -375,9 +404,10 @@ __global__ void narrow_dq_kernel(const float* __restrict__ acc, __nv_bfloat16* _
                                  long long n8, int T, int heads, HeadStrides gs) {
   for (long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x; i < n8;
        i += (long long)gridDim.x * blockDim.x) {
-    const float4 lo = reinterpret_cast<const float4*>(acc)[2 * i];
-    const float4 hi = reinterpret_cast<const float4*>(acc)[2 * i + 1];
     const long long row = i >> 3, bh = row / T, b = bh / heads;
+    const int in_block = (int)(row - bh * T) & 127, q = 2 * ((int)i & 7);
+    const float4 lo = reinterpret_cast<const float4*>(acc)[row * 16 + dq_chunk(in_block, q)];
+    const float4 hi = reinterpret_cast<const float4*>(acc)[row * 16 + dq_chunk(in_block, q + 1)];
     __nv_bfloat16* to = dq + b * gs.batch + (bh - b * heads) * gs.head + (row - bh * T) * gs.row + 8 * (i & 7);
     *reinterpret_cast<uint4*>(to) = make_uint4(pack_bf16(lo.x, lo.y), pack_bf16(lo.z, lo.w),
                                                  pack_bf16(hi.x, hi.y), pack_bf16(hi.z, hi.w));
