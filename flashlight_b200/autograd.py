@@ -236,7 +236,15 @@ def batchnorm(x: Variable, weight: Optional[Variable], bias: Optional[Variable],
     xt = x.tensor
     ins = [x] + ([weight] if weight is not None else []) + ([bias] if bias is not None else [])
 
-    def give(inputs, gx, gw, gb):
+    def grad_func(inputs, gy, gy2=None):
+        if not relu:
+            gx, gw, gb = ext.batchnormBackward(gy, save_mean, save_var, xt, wt, axes, train, epsilon, None)
+        else:
+            # gy2: the second consumer's gradient (grad_func2)
+            if gy2 is not None and not ext.batchnormSumSupported(xt, gy, gy2, axes):
+                gy, gy2 = F.add(gy, gy2), None
+            gx, gw, gb = ext.batchnormReluBackward(gy, save_mean, save_var, xt, wt, bt, axes, train, epsilon,
+                                                   None, gy2, inputs[0].isCalcGrad())
         if gx is not None:
             inputs[0].addGrad(gx)
         k = 1
@@ -245,22 +253,9 @@ def batchnorm(x: Variable, weight: Optional[Variable], bias: Optional[Variable],
         if bias is not None:
             inputs[k].addGrad(gb.reshape(bt.shape))
 
-    def grad_func(inputs, gy):
-        if relu:
-            give(inputs, *ext.batchnormReluBackward(gy, save_mean, save_var, xt, wt, bt, axes, train, epsilon,
-                                                    None, needInput=inputs[0].isCalcGrad()))
-        else:
-            give(inputs, *ext.batchnormBackward(gy, save_mean, save_var, xt, wt, axes, train, epsilon, None))
-
-    def grad_func2(inputs, ga, gb):
-        if not ext.batchnormSumSupported(xt, ga, gb, axes):
-            return grad_func(inputs, F.add(ga, gb))
-        give(inputs, *ext.batchnormReluBackward(ga, save_mean, save_var, xt, wt, bt, axes, train, epsilon,
-                                                None, gb, inputs[0].isCalcGrad()))
-
     out = Variable(y, False, ins, grad_func)
     if relu:
-        out.grad_func2 = grad_func2
+        out.grad_func2 = grad_func
     return out
 
 

@@ -133,6 +133,7 @@ attention_backward_kernel(const __grid_constant__ CUtensorMap map_q,
                           const __grid_constant__ CUtensorMap map_k,
                           const __grid_constant__ CUtensorMap map_v,
                           const __grid_constant__ CUtensorMap map_do, const AttnArgs a) {
+  chain_begin();
   extern __shared__ __align__(1024) char smem_raw[];
   char* base = reinterpret_cast<char*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) &
                                        ~static_cast<uintptr_t>(1023));
@@ -377,6 +378,7 @@ __global__ void attention_dsum_kernel(const __nv_bfloat16* __restrict__ o,
                                       const __nv_bfloat16* __restrict__ d_o,
                                       float* __restrict__ dsum, long long rows, int T,
                                       int heads) {
+  chain_begin();
   const long long t = blockIdx.x * (long long)blockDim.x + threadIdx.x;
   const long long row = t >> 3;
   float acc = 0.f;
@@ -402,6 +404,7 @@ __global__ void attention_dsum_kernel(const __nv_bfloat16* __restrict__ o,
 
 __global__ void narrow_dq_kernel(const float* __restrict__ acc, __nv_bfloat16* __restrict__ dq,
                                  long long n8, int T, int heads, HeadStrides gs) {
+  chain_begin();
   for (long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x; i < n8;
        i += (long long)gridDim.x * blockDim.x) {
     const long long row = i >> 3, bh = row / T, b = bh / heads;
@@ -441,6 +444,7 @@ __global__ void __launch_bounds__(kAttnThreads, 2)
 attention_forward_kernel(const __grid_constant__ CUtensorMap map_q,
                          const __grid_constant__ CUtensorMap map_k,
                          const __grid_constant__ CUtensorMap map_v, const AttnFwdArgs a) {
+  chain_begin();
   extern __shared__ __align__(1024) char smem_raw[];
   char* base = smem_raw + ((1024 - (smem_u32(smem_raw) & 1023)) & 1023);
   char* sQ = base;
@@ -657,8 +661,9 @@ int run_attention_backward(const void* q, const void* k, const void* v, const He
   const size_t acc_bytes = (size_t)rows * 64 * sizeof(float);
   FLB200_CUDA_CHECK(cudaMemsetAsync(workspace, 0, acc_bytes, st));
   float* dsum = reinterpret_cast<float*>(static_cast<char*>(workspace) + acc_bytes);
-  attention_dsum_kernel<<<(unsigned)((rows * 8 + 255) / 256), 256, 0, st>>>(
-      static_cast<const __nv_bfloat16*>(o), static_cast<const __nv_bfloat16*>(grad_o), dsum, rows, (int)T,
+  launch_chained(attention_dsum_kernel, (unsigned)((rows * 8 + 255) / 256), 256, 0, st,
+                 static_cast<const __nv_bfloat16*>(o), static_cast<const __nv_bfloat16*>(grad_o), dsum, rows,
+                 (int)T,
       (int)heads);
   FLB200_AFTER_LAUNCH("attention_dsum");
   AttnArgs a{};
@@ -674,12 +679,12 @@ int run_attention_backward(const void* q, const void* k, const void* v, const He
   a.scale = scale;
   a.status = tc::status_ptr();
   const unsigned grid = (unsigned)(batch * heads * ((T + 127) / 128));
-  attention_backward_kernel<<<grid, kAttnThreads, kAttnSmem, st>>>(mq, mk, mv, mg, a);
+  launch_chained(attention_backward_kernel, grid, kAttnThreads, kAttnSmem, st, mq, mk, mv, mg, a);
   FLB200_AFTER_LAUNCH("attention_backward");
   tc::count_tc_launch();
   const long long n8 = rows * 64 / 8;
-  narrow_dq_kernel<<<(unsigned)std::min<long long>((n8 + 255) / 256, 148 * 8), 256, 0, st>>>(
-      a.dq_acc, static_cast<__nv_bfloat16*>(grad_q), n8, (int)T, (int)heads, gs);
+  launch_chained(narrow_dq_kernel, (unsigned)std::min<long long>((n8 + 255) / 256, 148 * 8), 256, 0, st,
+                 a.dq_acc, static_cast<__nv_bfloat16*>(grad_q), n8, (int)T, (int)heads, gs);
   FLB200_AFTER_LAUNCH("attention_narrow_dq");
   return FLB200_OK;
 }
@@ -764,7 +769,7 @@ int flb200_attention_packed_forward(const void* qkv, void* out, float* lse, int6
   a.scale = scale;
   a.status = tc::status_ptr();
   const unsigned grid = (unsigned)(batch * heads * ((seq_len + 127) / 128));
-  attention_forward_kernel<<<grid, kAttnThreads, kFwdSmem, as_stream(stream)>>>(mq, mk, mv, a);
+  launch_chained(attention_forward_kernel, grid, kAttnThreads, kFwdSmem, as_stream(stream), mq, mk, mv, a);
   FLB200_AFTER_LAUNCH("attention_forward");
   tc::count_tc_launch();
   return FLB200_OK;

@@ -21,6 +21,7 @@ template <typename T, int PER>
 __global__ void __launch_bounds__(256)
 softmax_forward_kernel(const T* __restrict__ x, T* __restrict__ y, long long rows, int cols,
                        float scale, int period, float* __restrict__ lse) {
+  chain_begin();
   const int lane = threadIdx.x & 31;
   const long long r = (long long)blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5);
   if (r >= rows) return;
@@ -57,6 +58,7 @@ template <typename T, int PER>
 __global__ void __launch_bounds__(256)
 softmax_backward_kernel(const T* __restrict__ y, const T* __restrict__ dy, T* __restrict__ dx,
                         long long rows, int cols, float scale) {
+  chain_begin();
   const int lane = threadIdx.x & 31;
   const long long r = (long long)blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5);
   if (r >= rows) return;
@@ -87,11 +89,11 @@ int launch(bool backward, const void* a, const void* b, void* out, long long row
 #define FLB200_SOFTMAX_CASE(PER)                                                              \
   if (cols <= 32 * PER) {                                                                     \
     if (backward)                                                                             \
-      softmax_backward_kernel<T, PER><<<grid, 256, 0, st>>>(                                  \
+      launch_chained(softmax_backward_kernel<T, PER>, grid, 256, 0, st, \
           static_cast<const T*>(a), static_cast<const T*>(b), static_cast<T*>(out), rows,     \
           cols, scale);                                                                       \
     else                                                                                      \
-      softmax_forward_kernel<T, PER><<<grid, 256, 0, st>>>(                                   \
+      launch_chained(softmax_forward_kernel<T, PER>, grid, 256, 0, st, \
           static_cast<const T*>(a), static_cast<T*>(out), rows, cols, scale, period, lse);    \
     return FLB200_OK;                                                                         \
   }

@@ -151,6 +151,7 @@ bn_add_relu_apply_kernel(const float* __restrict__ x, const float* __restrict__ 
                          float* __restrict__ y, uint8_t* __restrict__ mask, ChannelGeo g,
                          const float* __restrict__ mean, const BnScale scale,
                          const float* __restrict__ shift) {
+  chain_begin();
   constexpr int NV = G / 4;
   const long long c = blockIdx.x;
   const float m = mean[c], sc = scale.at(c), sh = shift ? shift[c] : 0.f;
@@ -195,6 +196,7 @@ bn_tail_backward_reduce_kernel(const float* __restrict__ x, const float* __restr
                                const float* __restrict__ gb, const uint8_t* __restrict__ mask,
                                float* __restrict__ gz, float2* __restrict__ partial, ChannelGeo g,
                                const float* __restrict__ mean) {
+  chain_begin();
   constexpr int NV = G / 4;
   __shared__ float scratch[32];
   const long long c = blockIdx.x;
@@ -238,6 +240,7 @@ bn_add_relu_apply_scalar_kernel(const float* __restrict__ x, const float* __rest
                                 float* __restrict__ y, uint8_t* __restrict__ mask, ChannelGeo g,
                                 const float* __restrict__ mean, const BnScale scale,
                                 const float* __restrict__ shift) {
+  chain_begin();
   const long long c = blockIdx.x;
   const float m = mean[c], sc = scale.at(c), sh = shift ? shift[c] : 0.f;
   long long begin = (long long)blockIdx.y * g.chunk;
@@ -256,6 +259,7 @@ bn_tail_backward_reduce_scalar_kernel(const float* __restrict__ x, const float* 
                                       const uint8_t* __restrict__ mask, float* __restrict__ gz,
                                       float2* __restrict__ partial, ChannelGeo g,
                                       const float* __restrict__ mean) {
+  chain_begin();
   __shared__ float scratch[32];
   const long long c = blockIdx.x;
   const float m = mean[c];
@@ -308,6 +312,7 @@ bn_add_relu_apply_cl_kernel(const T* __restrict__ x, const T* __restrict__ adden
                             long long channels, long long rows_per_split, int co_shift,
                             const float* __restrict__ mean, const BnScale scale,
                             const float* __restrict__ shift) {
+  chain_begin();
   const int co = 1 << co_shift, rl = 256 >> co_shift;
   const int tq = threadIdx.x & (co - 1), tr = threadIdx.x >> co_shift;
   const long long c = ((long long)blockIdx.x * co + tq) * 8;
@@ -349,8 +354,8 @@ void launch_add_relu_cl(const void* x, const void* addend, void* y, uint8_t* mas
   const long long rps = apply_rows_per_split(rows, ot.col_blocks, 256 >> ot.co_shift,
                                              sizeof(T) == 4 ? 16 : 4);  // registers: 4 per SM
   const dim3 grid((unsigned)ot.col_blocks, (unsigned)((rows + rps - 1) / rps));
-  bn_add_relu_apply_cl_kernel<T><<<grid, 256, 0, st>>>(
-      static_cast<const T*>(x), static_cast<const T*>(addend), static_cast<T*>(y), mask, rows, channels,
+  launch_chained(bn_add_relu_apply_cl_kernel<T>, grid, 256, 0, st, static_cast<const T*>(x),
+                 static_cast<const T*>(addend), static_cast<T*>(y), mask, rows, channels,
       rps, ot.co_shift, mean, scale, shift);
 }
 
@@ -362,6 +367,7 @@ bn_tail_backward_reduce_cl_kernel(const T* __restrict__ x, const T* __restrict__
                                   long long rows, long long channels, int splits,
                                   long long rows_per_split, int co_shift,
                                   const float* __restrict__ mean) {
+  chain_begin();
   __shared__ float sh0[2048];
   __shared__ float sh1[2048];
   const int co = 1 << co_shift, rl = 256 >> co_shift;
@@ -491,6 +497,7 @@ __device__ __forceinline__ bool fin_sums(const float2* __restrict__ partial, int
 
 __global__ void sum_finalize_kernel(const float2* __restrict__ partial, int splits,
                                     long long channels, float* __restrict__ out) {
+  chain_begin();
   long long c;
   double s0, s1;
   if (!fin_sums(partial, splits, channels, &c, &s0, &s1)) return;
@@ -508,6 +515,7 @@ __global__ void bn_stats_finalize_kernel(const float2* __restrict__ partial, int
                                          float* __restrict__ save_mean,
                                          float* __restrict__ save_invstd,
                                          float* __restrict__ scale) {
+  chain_begin();
   long long c;
   double s0, s1;
   if (!fin_sums(partial, splits, channels, &c, &s0, &s1)) return;
@@ -539,6 +547,7 @@ __global__ void bn_stats_finalize_matrix_kernel(const float2* __restrict__ parti
                                                 float* __restrict__ save_mean,
                                                 float* __restrict__ save_invstd,
                                                 float* __restrict__ scale) {
+  chain_begin();
   const long long c = ((long long)blockIdx.x * blockDim.x + threadIdx.x) >> 5;
   const int lane = threadIdx.x & 31;
   if (c >= channels) return;  // whole warps only
@@ -567,6 +576,7 @@ __global__ void bn_stats_finalize_matrix_kernel(const float2* __restrict__ parti
 __global__ void affine_bwd_finalize_kernel(const float2* __restrict__ partial, int splits,
                                            long long channels, float* __restrict__ grad_weight,
                                            float* __restrict__ grad_bias) {
+  chain_begin();
   long long c;
   double s0, s1;
   if (!fin_sums(partial, splits, channels, &c, &s0, &s1)) return;
@@ -582,6 +592,7 @@ __global__ void bn_bwd_finalize_kernel(const float2* __restrict__ partial, int s
                                        float* __restrict__ grad_weight,
                                        float* __restrict__ grad_bias,
                                        float4* __restrict__ coef) {
+  chain_begin();
   long long c;
   double s0, s1;
   if (!fin_sums(partial, splits, channels, &c, &s0, &s1)) return;
@@ -605,16 +616,16 @@ int launch_reduce(const char* name, const void* a, const void* b, float2* partia
     if (vec) {
       const ColumnTiling ct = column_tiling(channels, Vec16<T>::N);
       dim3 vgrid((unsigned)ct.col_blocks, (unsigned)splits);
-      column_reduce_vec_kernel<T, NIN, F><<<vgrid, 256, 0, st>>>(
-          static_cast<const T*>(a), static_cast<const T*>(b), partial, outer, channels,
+      launch_chained(column_reduce_vec_kernel<T, NIN, F>, vgrid, 256, 0, st, static_cast<const T*>(a),
+                     static_cast<const T*>(b), partial, outer, channels,
           splits, rps, ct.cq_shift, f, nullptr, nullptr);
       FLB200_AFTER_LAUNCH(name);
       *splits_out = splits;
       return FLB200_OK;
     }
     dim3 grid((unsigned)((channels + 31) / 32), (unsigned)splits);
-    column_reduce_kernel<T, NIN, F><<<grid, 256, 0, st>>>(
-        static_cast<const T*>(a), static_cast<const T*>(b), partial, outer, channels, splits, rps,
+    launch_chained(column_reduce_kernel<T, NIN, F>, grid, 256, 0, st, static_cast<const T*>(a),
+                   static_cast<const T*>(b), partial, outer, channels, splits, rps,
         f);
     FLB200_AFTER_LAUNCH(name);
     *splits_out = splits;
@@ -624,11 +635,11 @@ int launch_reduce(const char* name, const void* a, const void* b, float2* partia
   const bool vec = inner % Vec16<T>::N == 0 && aligned16(a) && (NIN == 1 || aligned16(b));
   dim3 grid((unsigned)channels, (unsigned)g.splits);
   if (vec)
-    channel_reduce_kernel<T, NIN, true, F><<<grid, kChanThreads, 0, st>>>(
-        static_cast<const T*>(a), static_cast<const T*>(b), partial, g, f);
+    launch_chained(channel_reduce_kernel<T, NIN, true, F>, grid, kChanThreads, 0, st, static_cast<const T*>(a),
+                   static_cast<const T*>(b), partial, g, f);
   else
-    channel_reduce_kernel<T, NIN, false, F><<<grid, kChanThreads, 0, st>>>(
-        static_cast<const T*>(a), static_cast<const T*>(b), partial, g, f);
+    launch_chained(channel_reduce_kernel<T, NIN, false, F>, grid, kChanThreads, 0, st, static_cast<const T*>(a),
+                   static_cast<const T*>(b), partial, g, f);
   FLB200_AFTER_LAUNCH(name);
   *splits_out = g.splits;
   return FLB200_OK;
@@ -640,8 +651,8 @@ int launch_reduce_sum(const char* name, const void* a, const void* b, const void
                       long long rows, long long channels, F f, int* splits_out, cudaStream_t st) {
   const int splits = column_splits(rows, channels, true);
   const ColumnTiling ct = column_tiling(channels, Vec16<T>::N);
-  column_reduce_vec_kernel<T, 3, F><<<dim3((unsigned)ct.col_blocks, (unsigned)splits), 256, 0, st>>>(
-      static_cast<const T*>(a), static_cast<const T*>(b), partial, rows, channels, splits,
+  launch_chained(column_reduce_vec_kernel<T, 3, F>, dim3((unsigned)ct.col_blocks, (unsigned)splits), 256, 0, st,
+                 static_cast<const T*>(a), static_cast<const T*>(b), partial, rows, channels, splits,
       (rows + splits - 1) / splits, ct.cq_shift, f, static_cast<const T*>(b2), static_cast<T*>(sum));
   FLB200_AFTER_LAUNCH(name);
   *splits_out = splits;
@@ -657,15 +668,15 @@ int launch_apply(const char* name, const void* a, const void* b, void* out, long
       const long long rps = apply_rows_per_split(outer, ct.col_blocks, 256 >> ct.cq_shift,
                                                  sizeof(T) == 4 ? 16 : 6);
       dim3 vgrid((unsigned)ct.col_blocks, (unsigned)((outer + rps - 1) / rps));
-      column_apply_vec_kernel<T, NIN, F><<<vgrid, 256, 0, st>>>(
-          static_cast<const T*>(a), static_cast<const T*>(b), static_cast<T*>(out),
+      launch_chained(column_apply_vec_kernel<T, NIN, F>, vgrid, 256, 0, st, static_cast<const T*>(a),
+                     static_cast<const T*>(b), static_cast<T*>(out),
           outer, channels, rps, ct.cq_shift, f);
       FLB200_AFTER_LAUNCH(name);
       return FLB200_OK;
     }
     const int grid = grid_for(outer * channels, 256 * 4);
-    column_apply_kernel<T, NIN, F><<<grid, 256, 0, st>>>(
-        static_cast<const T*>(a), static_cast<const T*>(b), static_cast<T*>(out), outer, channels,
+    launch_chained(column_apply_kernel<T, NIN, F>, grid, 256, 0, st, static_cast<const T*>(a),
+                   static_cast<const T*>(b), static_cast<T*>(out), outer, channels,
         f);
     FLB200_AFTER_LAUNCH(name);
     return FLB200_OK;
@@ -675,11 +686,11 @@ int launch_apply(const char* name, const void* a, const void* b, void* out, long
                    (NIN == 1 || aligned16(b));
   dim3 grid((unsigned)channels, (unsigned)g.splits);
   if (vec)
-    channel_apply_kernel<T, NIN, true, F><<<grid, kChanThreads, 0, st>>>(
-        static_cast<const T*>(a), static_cast<const T*>(b), static_cast<T*>(out), g, f);
+    launch_chained(channel_apply_kernel<T, NIN, true, F>, grid, kChanThreads, 0, st, static_cast<const T*>(a),
+                   static_cast<const T*>(b), static_cast<T*>(out), g, f);
   else
-    channel_apply_kernel<T, NIN, false, F><<<grid, kChanThreads, 0, st>>>(
-        static_cast<const T*>(a), static_cast<const T*>(b), static_cast<T*>(out), g, f);
+    launch_chained(channel_apply_kernel<T, NIN, false, F>, grid, kChanThreads, 0, st, static_cast<const T*>(a),
+                   static_cast<const T*>(b), static_cast<T*>(out), g, f);
   FLB200_AFTER_LAUNCH(name);
   return FLB200_OK;
 }
@@ -728,7 +739,7 @@ static int channel_sum_impl(const void* in, float* out, long long outer, long lo
                         rc = (launch_reduce<T, 1>("channel_sum", in, nullptr, partial, outer, channels, inner,
                                                   SumF{}, &splits, st, most_splits)));
   if (rc) return rc;
-  sum_finalize_kernel<<<fin_grid(channels), kFinThreads, 0, st>>>(partial, splits, channels, out);
+  launch_chained(sum_finalize_kernel, fin_grid(channels), kFinThreads, 0, st, partial, splits, channels, out);
   FLB200_AFTER_LAUNCH("channel_sum_finalize");
   return FLB200_OK;
 }
@@ -844,8 +855,8 @@ int flb200_layernorm_affine_backward(const void* grad_y, const void* xhat, const
                                                     partial, rows, features, 1, AffineBwdReduceF{},
                                                     &splits, st)));
     if (rc) return rc;
-    affine_bwd_finalize_kernel<<<fin_grid(features), kFinThreads, 0, st>>>(
-        partial, splits, features, grad_weight, grad_bias);
+    launch_chained(affine_bwd_finalize_kernel, fin_grid(features), kFinThreads, 0, st, partial, splits,
+                   features, grad_weight, grad_bias);
     FLB200_AFTER_LAUNCH("layernorm_affine_backward_finalize");
   }
   if (grad_xhat) {
@@ -938,8 +949,8 @@ static int batchnorm_forward_impl(bool relu, const void* addend, uint8_t* mask,
       rc = launch_reduce<float, 1>("batchnorm_stats_matrix", stats, nullptr, p2, stat_groups,
                                    2 * C, 1, SumF{}, &splits, st);
       if (rc) return rc;
-      bn_stats_finalize_matrix_kernel<<<fin_grid(C), kFinThreads, 0, st>>>(
-          p2, splits, C, (double)d->outer * (double)d->inner, weight, epsilon, momentum,
+      launch_chained(bn_stats_finalize_matrix_kernel, fin_grid(C), kFinThreads, 0, st, p2, splits, C,
+                     (double)d->outer * (double)d->inner, weight, epsilon, momentum,
           running_mean, running_var, save_mean, save_invstd, scale);
       FLB200_AFTER_LAUNCH("batchnorm_stats_finalize_matrix");
     } else {
@@ -949,8 +960,8 @@ static int batchnorm_forward_impl(bool relu, const void* addend, uint8_t* mask,
                             rc = (launch_reduce<T, 1>("batchnorm_stats", x, nullptr, partial,
                                                       d->outer, C, d->inner, sf, &splits, st)));
       if (rc) return rc;
-      bn_stats_finalize_kernel<<<fin_grid(C), kFinThreads, 0, st>>>(
-          partial, splits, C, (double)d->outer * (double)d->inner, x, d->inner, d->dtype, weight,
+      launch_chained(bn_stats_finalize_kernel, fin_grid(C), kFinThreads, 0, st, partial, splits, C,
+                     (double)d->outer * (double)d->inner, x, d->inner, d->dtype, weight,
           epsilon, momentum, running_mean, running_var, save_mean, save_invstd, scale);
       FLB200_AFTER_LAUNCH("batchnorm_stats_finalize");
     }
@@ -969,16 +980,16 @@ static int batchnorm_forward_impl(bool relu, const void* addend, uint8_t* mask,
     const ChannelGeo g = make_channel_geo(d->outer, C, d->inner);
     const dim3 grid((unsigned)C, (unsigned)g.splits);
     if (d->inner % 8 == 0)
-      bn_add_relu_apply_kernel<8><<<grid, kChanThreads, 0, st>>>(
-          static_cast<const float*>(x), static_cast<const float*>(addend), static_cast<float*>(y),
+      launch_chained(bn_add_relu_apply_kernel<8>, grid, kChanThreads, 0, st, static_cast<const float*>(x),
+                     static_cast<const float*>(addend), static_cast<float*>(y),
           mask, g, mean_ptr, bs, bias);
     else if (d->inner % 4 != 0)
-      bn_add_relu_apply_scalar_kernel<<<grid, kChanThreads, 0, st>>>(
-          static_cast<const float*>(x), static_cast<const float*>(addend), static_cast<float*>(y),
+      launch_chained(bn_add_relu_apply_scalar_kernel, grid, kChanThreads, 0, st, static_cast<const float*>(x),
+                     static_cast<const float*>(addend), static_cast<float*>(y),
           mask, g, mean_ptr, bs, bias);
     else
-      bn_add_relu_apply_kernel<4><<<grid, kChanThreads, 0, st>>>(
-          static_cast<const float*>(x), static_cast<const float*>(addend), static_cast<float*>(y),
+      launch_chained(bn_add_relu_apply_kernel<4>, grid, kChanThreads, 0, st, static_cast<const float*>(x),
+                     static_cast<const float*>(addend), static_cast<float*>(y),
           mask, g, mean_ptr, bs, bias);
     FLB200_AFTER_LAUNCH("batchnorm_add_relu_apply");
   } else if (relu) {
@@ -1093,9 +1104,9 @@ static int batchnorm_backward_impl(bool relu, const uint8_t* tail_mask, const vo
     const long long rps = (d->outer + splits - 1) / splits;
     FLB200_DISPATCH_DTYPE(
         d->dtype, "batchnorm_add_relu_backward",
-        (bn_tail_backward_reduce_cl_kernel<T>
-         <<<dim3((unsigned)ot.col_blocks, (unsigned)splits), 256, 0, st>>>(
-             static_cast<const T*>(x), static_cast<const T*>(grad_y), static_cast<const T*>(tail_gb),
+        (launch_chained(bn_tail_backward_reduce_cl_kernel<T>, dim3((unsigned)ot.col_blocks, (unsigned)splits),
+                        256, 0, st, static_cast<const T*>(x), static_cast<const T*>(grad_y),
+                        static_cast<const T*>(tail_gb),
              tail_mask, static_cast<T*>(tail_sum), partial, d->outer, C, splits, rps, ot.co_shift,
              save_mean)));
     FLB200_AFTER_LAUNCH("batchnorm_tail_backward_reduce_channels_last");
@@ -1104,18 +1115,18 @@ static int batchnorm_backward_impl(bool relu, const uint8_t* tail_mask, const vo
     const ChannelGeo g = make_channel_geo(d->outer, C, d->inner);
     const dim3 grid((unsigned)C, (unsigned)g.splits);
     if (d->inner % 8 == 0)
-      bn_tail_backward_reduce_kernel<8><<<grid, kChanThreads, 0, st>>>(
-          static_cast<const float*>(x), static_cast<const float*>(grad_y),
+      launch_chained(bn_tail_backward_reduce_kernel<8>, grid, kChanThreads, 0, st, static_cast<const float*>(x),
+                     static_cast<const float*>(grad_y),
           static_cast<const float*>(tail_gb), tail_mask, static_cast<float*>(tail_sum), partial, g,
           save_mean);
     else if (d->inner % 4 != 0)
-      bn_tail_backward_reduce_scalar_kernel<<<grid, kChanThreads, 0, st>>>(
-          static_cast<const float*>(x), static_cast<const float*>(grad_y),
+      launch_chained(bn_tail_backward_reduce_scalar_kernel, grid, kChanThreads, 0, st,
+                     static_cast<const float*>(x), static_cast<const float*>(grad_y),
           static_cast<const float*>(tail_gb), tail_mask, static_cast<float*>(tail_sum), partial, g,
           save_mean);
     else
-      bn_tail_backward_reduce_kernel<4><<<grid, kChanThreads, 0, st>>>(
-          static_cast<const float*>(x), static_cast<const float*>(grad_y),
+      launch_chained(bn_tail_backward_reduce_kernel<4>, grid, kChanThreads, 0, st, static_cast<const float*>(x),
+                     static_cast<const float*>(grad_y),
           static_cast<const float*>(tail_gb), tail_mask, static_cast<float*>(tail_sum), partial, g,
           save_mean);
     FLB200_AFTER_LAUNCH("batchnorm_tail_backward_reduce");
@@ -1141,8 +1152,8 @@ static int batchnorm_backward_impl(bool relu, const uint8_t* tail_mask, const vo
                                                     st)));
   }
   if (rc) return rc;
-  bn_bwd_finalize_kernel<<<fin_grid(C), kFinThreads, 0, st>>>(
-      partial, splits, C, (double)d->outer * (double)d->inner, weight, save_mean, save_invstd,
+  launch_chained(bn_bwd_finalize_kernel, fin_grid(C), kFinThreads, 0, st, partial, splits, C,
+                 (double)d->outer * (double)d->inner, weight, save_mean, save_invstd,
       grad_weight, grad_bias, coef);
   FLB200_AFTER_LAUNCH("batchnorm_backward_finalize");
   if (!grad_x) return rc;

@@ -72,6 +72,7 @@ template <typename T, int NIN, bool VEC, typename F>
 __global__ void __launch_bounds__(kChanThreads)
 channel_reduce_kernel(const T* __restrict__ a, const T* __restrict__ b,
                       float2* __restrict__ partial, ChannelGeo g, F f) {
+  chain_begin();
   __shared__ float scratch[32];
   const long long c = blockIdx.x;
   const int s = blockIdx.y;
@@ -122,6 +123,7 @@ template <typename T, int NIN, bool VEC, typename F>
 __global__ void __launch_bounds__(kChanThreads)
 channel_apply_kernel(const T* __restrict__ a, const T* __restrict__ b, T* __restrict__ out,
                      ChannelGeo g, F f) {
+  chain_begin();
   const long long c = blockIdx.x;
   const int s = blockIdx.y;
   const typename F::K k = f.channel(c);
@@ -171,6 +173,7 @@ __global__ void __launch_bounds__(256)
 column_reduce_kernel(const T* __restrict__ a, const T* __restrict__ b,
                      float2* __restrict__ partial, long long rows, long long channels,
                      int splits, long long rows_per_split, F f) {
+  chain_begin();
   __shared__ float sh0[8][33];
   __shared__ float sh1[8][33];
   const int tx = threadIdx.x & 31, ty = threadIdx.x >> 5;
@@ -208,6 +211,7 @@ template <typename T, int NIN, typename F>
 __global__ void __launch_bounds__(256)
 column_apply_kernel(const T* __restrict__ a, const T* __restrict__ b, T* __restrict__ out,
                     long long rows, long long channels, F f) {
+  chain_begin();
   const long long total = rows * channels;
   const long long threads = (long long)gridDim.x * blockDim.x;
   const bool fixed = threads >= channels;
@@ -256,6 +260,7 @@ column_reduce_vec_kernel(const T* __restrict__ a, const T* __restrict__ b,
                          float2* __restrict__ partial, long long rows, long long channels,
                          int splits, long long rows_per_split, int cq_shift, F f,
                          const T* __restrict__ b2, T* __restrict__ sum) {
+  chain_begin();
   constexpr int V = Vec16<T>::N;
   __shared__ float sh0[256 * V];
   __shared__ float sh1[256 * V];
@@ -360,6 +365,7 @@ __global__ void __launch_bounds__(256, sizeof(T) == 4 ? 4 : NIN == 2 ? 2 : 3)
 column_apply_vec_kernel(const T* __restrict__ a, const T* __restrict__ b,
                         T* __restrict__ out, long long rows, long long channels,
                         long long rows_per_split, int cq_shift, F f) {
+  chain_begin();
   constexpr int V = Vec16<T>::N;
   const int cq = 1 << cq_shift, rl = 256 >> cq_shift;
   const int tq = threadIdx.x & (cq - 1), tr = threadIdx.x >> cq_shift;

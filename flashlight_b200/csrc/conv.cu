@@ -478,6 +478,7 @@ __device__ __forceinline__ void widen8(const T* in, float* out) {
 // scores to fp32: 165 and 152.)
 template <typename T>
 __global__ void widen_kernel(const T* __restrict__ in, float* __restrict__ out, long long n) {
+  chain_begin();
   const long long stride = (long long)gridDim.x * blockDim.x * 8;
   long long i = ((long long)blockIdx.x * blockDim.x + threadIdx.x) * 8;
   if (((reinterpret_cast<uintptr_t>(in) | reinterpret_cast<uintptr_t>(out)) & 15) == 0) {
@@ -492,6 +493,7 @@ __global__ void widen_kernel(const T* __restrict__ in, float* __restrict__ out, 
 }
 template <typename T>
 __global__ void narrow_kernel(const float* __restrict__ in, T* __restrict__ out, long long n) {
+  chain_begin();
   const long long stride = (long long)gridDim.x * blockDim.x * 8;
   long long i = ((long long)blockIdx.x * blockDim.x + threadIdx.x) * 8;
   if (((reinterpret_cast<uintptr_t>(in) | reinterpret_cast<uintptr_t>(out)) & 15) == 0) {
@@ -514,9 +516,10 @@ int widen(const void* in, float* out, long long n, int dtype, cudaStream_t st) {
   if (n == 0 || !in) return FLB200_OK;
   const unsigned grid = (unsigned)std::min<long long>(n / 8 / 256 + 1, 16LL * device_info().sm_count);
   if (dtype == FLB200_F16)
-    widen_kernel<__half><<<grid, 256, 0, st>>>(static_cast<const __half*>(in), out, n);
+    launch_chained(widen_kernel<__half>, grid, 256, 0, st, static_cast<const __half*>(in), out, n);
   else
-    widen_kernel<__nv_bfloat16><<<grid, 256, 0, st>>>(static_cast<const __nv_bfloat16*>(in), out, n);
+    launch_chained(widen_kernel<__nv_bfloat16>, grid, 256, 0, st, static_cast<const __nv_bfloat16*>(in), out,
+                   n);
   FLB200_AFTER_LAUNCH("conv_widen");
   return FLB200_OK;
 }
@@ -524,9 +527,9 @@ int narrow(const float* in, void* out, long long n, int dtype, cudaStream_t st) 
   if (n == 0 || !out) return FLB200_OK;
   const unsigned grid = (unsigned)std::min<long long>(n / 8 / 256 + 1, 16LL * device_info().sm_count);
   if (dtype == FLB200_F16)
-    narrow_kernel<__half><<<grid, 256, 0, st>>>(in, static_cast<__half*>(out), n);
+    launch_chained(narrow_kernel<__half>, grid, 256, 0, st, in, static_cast<__half*>(out), n);
   else
-    narrow_kernel<__nv_bfloat16><<<grid, 256, 0, st>>>(in, static_cast<__nv_bfloat16*>(out), n);
+    launch_chained(narrow_kernel<__nv_bfloat16>, grid, 256, 0, st, in, static_cast<__nv_bfloat16*>(out), n);
   FLB200_AFTER_LAUNCH("conv_narrow");
   return FLB200_OK;
 }

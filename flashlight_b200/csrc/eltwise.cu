@@ -19,6 +19,7 @@ template <typename T, typename Op>
 __global__ void __launch_bounds__(kThreads) unary_vec_kernel(const T* __restrict__ a,
                                                              T* __restrict__ out, int64_t n,
                                                              Op op) {
+  chain_begin();
   constexpr int V = Vec16<T>::N;
   const int64_t nvec = n / V;
   const int64_t stride = (int64_t)gridDim.x * kThreads;
@@ -46,6 +47,7 @@ template <typename T, typename Op>
 __global__ void __launch_bounds__(kThreads) unary_scalar_kernel(const T* __restrict__ a,
                                                                 T* __restrict__ out, int64_t n,
                                                                 Op op) {
+  chain_begin();
   const int64_t stride = (int64_t)gridDim.x * kThreads;
   for (int64_t t = (int64_t)blockIdx.x * kThreads + threadIdx.x; t < n; t += stride)
     out[t] = Num<T>::from_f(op(Num<T>::to_f(a[t])));
@@ -56,6 +58,7 @@ __global__ void __launch_bounds__(kThreads) binary_vec_kernel(const T* __restric
                                                               const T* __restrict__ b,
                                                               T* __restrict__ out, int64_t n,
                                                               Op op) {
+  chain_begin();
   constexpr int V = Vec16<T>::N;
   const int64_t nvec = n / V;
   const int64_t stride = (int64_t)gridDim.x * kThreads;
@@ -88,6 +91,7 @@ __global__ void __launch_bounds__(kThreads) binary_scalar_kernel(const T* __rest
                                                                  const T* __restrict__ b,
                                                                  T* __restrict__ out, int64_t n,
                                                                  Op op) {
+  chain_begin();
   const int64_t stride = (int64_t)gridDim.x * kThreads;
   for (int64_t t = (int64_t)blockIdx.x * kThreads + threadIdx.x; t < n; t += stride)
     out[t] = Num<T>::from_f(op(Num<T>::to_f(a[t]), Num<T>::to_f(b[t])));
@@ -99,11 +103,11 @@ int launch_unary(const char* name, const void* a, void* out, int64_t n, Op op, v
   const bool vec = aligned16(a) && aligned16(out);
   const int grid = grid_for(n, kThreads * Vec16<T>::N * kUnroll);
   if (vec)
-    unary_vec_kernel<T, Op><<<grid, kThreads, 0, as_stream(stream)>>>(
-        static_cast<const T*>(a), static_cast<T*>(out), n, op);
+    launch_chained(unary_vec_kernel<T, Op>, grid, kThreads, 0, as_stream(stream), static_cast<const T*>(a),
+                   static_cast<T*>(out), n, op);
   else
-    unary_scalar_kernel<T, Op><<<grid, kThreads, 0, as_stream(stream)>>>(
-        static_cast<const T*>(a), static_cast<T*>(out), n, op);
+    launch_chained(unary_scalar_kernel<T, Op>, grid, kThreads, 0, as_stream(stream), static_cast<const T*>(a),
+                   static_cast<T*>(out), n, op);
   FLB200_AFTER_LAUNCH(name);
   return FLB200_OK;
 }
@@ -115,11 +119,11 @@ int launch_binary(const char* name, const void* a, const void* b, void* out, int
   const bool vec = aligned16(a) && aligned16(b) && aligned16(out);
   const int grid = grid_for(n, kThreads * Vec16<T>::N * kUnroll);
   if (vec)
-    binary_vec_kernel<T, Op><<<grid, kThreads, 0, as_stream(stream)>>>(
-        static_cast<const T*>(a), static_cast<const T*>(b), static_cast<T*>(out), n, op);
+    launch_chained(binary_vec_kernel<T, Op>, grid, kThreads, 0, as_stream(stream), static_cast<const T*>(a),
+                   static_cast<const T*>(b), static_cast<T*>(out), n, op);
   else
-    binary_scalar_kernel<T, Op><<<grid, kThreads, 0, as_stream(stream)>>>(
-        static_cast<const T*>(a), static_cast<const T*>(b), static_cast<T*>(out), n, op);
+    launch_chained(binary_scalar_kernel<T, Op>, grid, kThreads, 0, as_stream(stream), static_cast<const T*>(a),
+                   static_cast<const T*>(b), static_cast<T*>(out), n, op);
   FLB200_AFTER_LAUNCH(name);
   return FLB200_OK;
 }
@@ -218,6 +222,7 @@ template <bool ADD>
 __global__ void __launch_bounds__(256)
 relu_forward_mask_kernel(const float* __restrict__ x, const float* __restrict__ x2,
                          float* __restrict__ y, uint8_t* __restrict__ mask, long long n) {
+  chain_begin();
   const long long full = n >> 3;  // complete groups of 8
   const long long stride = (long long)gridDim.x * blockDim.x;
   const float4* xv = reinterpret_cast<const float4*>(x);
@@ -268,6 +273,7 @@ template <bool ADD>
 __global__ void __launch_bounds__(256)
 relu_backward_mask_kernel(const uint8_t* __restrict__ mask, const float* __restrict__ dy,
                           const float* __restrict__ dy2, float* __restrict__ dx, long long n) {
+  chain_begin();
   const long long full = n >> 3;
   const long long stride = (long long)gridDim.x * blockDim.x;
   const float4* gv = reinterpret_cast<const float4*>(dy);
@@ -308,6 +314,7 @@ relu_backward_mask_kernel(const uint8_t* __restrict__ mask, const float* __restr
 __global__ void __launch_bounds__(256)
 sgd_step_kernel(float* __restrict__ p, float* __restrict__ g, float* __restrict__ v, long long n,
                 float lr, float mu, float wd, int nesterov, float grad_scale, int grad_mode) {
+  chain_begin();
   const long long stride = (long long)gridDim.x * blockDim.x;
   const bool vec = ((reinterpret_cast<uintptr_t>(p) | reinterpret_cast<uintptr_t>(g) |
                      (v ? reinterpret_cast<uintptr_t>(v) : 0)) & 15) == 0;
@@ -349,8 +356,8 @@ int flb200_sgd_step(void* param, void* grad, void* velocity, int64_t n, float lr
   FLB200_REQUIRE(momentum == 0.f || velocity, "sgd_step: momentum needs a velocity buffer");
   if (dtype != FLB200_F32) return fail(FLB200_UNSUPPORTED, "sgd_step: f32 parameters only");
   const int grid = grid_for((n + 3) / 4, 256);
-  sgd_step_kernel<<<grid, 256, 0, as_stream(stream)>>>(
-      static_cast<float*>(param), static_cast<float*>(grad),
+  launch_chained(sgd_step_kernel, grid, 256, 0, as_stream(stream), static_cast<float*>(param),
+                 static_cast<float*>(grad),
       momentum != 0.f ? static_cast<float*>(velocity) : nullptr, n, lr, momentum, weight_decay,
       nesterov ? 1 : 0, grad_scale, zero_grad ? 1 : 0);
   FLB200_AFTER_LAUNCH("sgd_step");
@@ -367,11 +374,12 @@ int relu_mask_forward(const char* name, const void* x, const void* x2, void* y, 
     return fail(FLB200_UNSUPPORTED, "%s: f32 tensors aligned to 16 bytes only", name);
   const int grid = grid_for((n + 7) / 8, 256 * 2);
   if (x2)
-    relu_forward_mask_kernel<true><<<grid, 256, 0, as_stream(stream)>>>(
-        static_cast<const float*>(x), static_cast<const float*>(x2), static_cast<float*>(y), mask, n);
+    launch_chained(relu_forward_mask_kernel<true>, grid, 256, 0, as_stream(stream),
+                   static_cast<const float*>(x), static_cast<const float*>(x2), static_cast<float*>(y), mask,
+                   n);
   else
-    relu_forward_mask_kernel<false><<<grid, 256, 0, as_stream(stream)>>>(
-        static_cast<const float*>(x), nullptr, static_cast<float*>(y), mask, n);
+    launch_chained(relu_forward_mask_kernel<false>, grid, 256, 0, as_stream(stream),
+                   static_cast<const float*>(x), nullptr, static_cast<float*>(y), mask, n);
   FLB200_AFTER_LAUNCH(name);
   return FLB200_OK;
 }
@@ -384,12 +392,12 @@ int relu_mask_backward(const char* name, const uint8_t* mask, const void* g1, co
     return fail(FLB200_UNSUPPORTED, "%s: f32 tensors aligned to 16 bytes only", name);
   const int grid = grid_for((n + 7) / 8, 256 * 2);
   if (g2)
-    relu_backward_mask_kernel<true><<<grid, 256, 0, as_stream(stream)>>>(
-        mask, static_cast<const float*>(g1), static_cast<const float*>(g2),
+    launch_chained(relu_backward_mask_kernel<true>, grid, 256, 0, as_stream(stream), mask,
+                   static_cast<const float*>(g1), static_cast<const float*>(g2),
         static_cast<float*>(grad_x), n);
   else
-    relu_backward_mask_kernel<false><<<grid, 256, 0, as_stream(stream)>>>(
-        mask, static_cast<const float*>(g1), nullptr, static_cast<float*>(grad_x), n);
+    launch_chained(relu_backward_mask_kernel<false>, grid, 256, 0, as_stream(stream), mask,
+                   static_cast<const float*>(g1), nullptr, static_cast<float*>(grad_x), n);
   FLB200_AFTER_LAUNCH(name);
   return FLB200_OK;
 }
@@ -468,6 +476,7 @@ __device__ __forceinline__ uint4 philox4x32_10(uint4 ctr, uint2 key) {
 template <typename T>
 __global__ void bernoulli_mask_kernel(T* out, long long n, float keep, unsigned long long seed,
                                       unsigned long long offset) {
+  chain_begin();
   const long long blocks = (n + 3) / 4;
   for (long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x; i < blocks;
        i += (long long)gridDim.x * blockDim.x) {
@@ -499,16 +508,16 @@ extern "C" int flb200_bernoulli_mask(void* out, int64_t n, float keep_prob, uint
   cudaStream_t st = as_stream(stream);
   switch (dtype) {
     case FLB200_F32:
-      bernoulli_mask_kernel<float><<<grid, 256, 0, st>>>(static_cast<float*>(out), n, keep_prob,
+      launch_chained(bernoulli_mask_kernel<float>, grid, 256, 0, st, static_cast<float*>(out), n, keep_prob,
                                                          seed, offset);
       break;
     case FLB200_F16:
-      bernoulli_mask_kernel<__half><<<grid, 256, 0, st>>>(static_cast<__half*>(out), n, keep_prob,
+      launch_chained(bernoulli_mask_kernel<__half>, grid, 256, 0, st, static_cast<__half*>(out), n, keep_prob,
                                                           seed, offset);
       break;
     case FLB200_BF16:
-      bernoulli_mask_kernel<__nv_bfloat16><<<grid, 256, 0, st>>>(
-          static_cast<__nv_bfloat16*>(out), n, keep_prob, seed, offset);
+      launch_chained(bernoulli_mask_kernel<__nv_bfloat16>, grid, 256, 0, st, static_cast<__nv_bfloat16*>(out),
+                     n, keep_prob, seed, offset);
       break;
     default:
       return fail(FLB200_UNSUPPORTED, "bernoulli_mask: unsupported dtype %d", dtype);
@@ -534,6 +543,7 @@ struct ReorderGeo {
 __global__ void __launch_bounds__(256)
 reorder_runs_kernel(const uint4* __restrict__ in, uint4* __restrict__ out, ReorderGeo g,
                     long long runs) {
+  chain_begin();
   const int lanes = 1 << g.lanes_shift;
   const int sub = threadIdx.x & (lanes - 1);
   const long long per_cta = 256 >> g.lanes_shift;
@@ -578,8 +588,8 @@ extern "C" int flb200_reorder(const void* in, void* out, const int64_t* dims,
   long long grid = (runs + per_cta - 1) / per_cta;
   const long long cap = 32LL * device_info().sm_count;
   if (grid > cap) grid = cap;
-  reorder_runs_kernel<<<(unsigned)grid, 256, 0, as_stream(stream)>>>(
-      static_cast<const uint4*>(in), static_cast<uint4*>(out), g, runs);
+  launch_chained(reorder_runs_kernel, (unsigned)grid, 256, 0, as_stream(stream), static_cast<const uint4*>(in),
+                 static_cast<uint4*>(out), g, runs);
   FLB200_AFTER_LAUNCH("reorder");
   return FLB200_OK;
 }

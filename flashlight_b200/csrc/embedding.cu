@@ -27,6 +27,7 @@ template <typename T, typename I>
 __global__ void __launch_bounds__(256)
 embedding_forward_kernel(const T* __restrict__ table, const void* __restrict__ ids,
                          T* __restrict__ out, long long rows, long long dim, long long vocab) {
+  chain_begin();
   const long long total = rows * dim;
   for (long long t = (long long)blockIdx.x * blockDim.x + threadIdx.x; t < total;
        t += (long long)gridDim.x * blockDim.x) {
@@ -43,6 +44,7 @@ __global__ void __launch_bounds__(256)
 embedding_backward_kernel(const T* __restrict__ grad_out, const void* __restrict__ ids,
                           float* __restrict__ grad_table, long long rows, long long dim,
                           long long vocab) {
+  chain_begin();
   const int lane = threadIdx.x & 31;
   const long long v = (long long)blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5);
   if (v >= vocab) return;
@@ -85,6 +87,7 @@ embedding_backward_by_position_kernel(const T* __restrict__ grad_out,
                                       const void* __restrict__ ids,
                                       float* __restrict__ grad_table, long long rows,
                                       long long dim, long long vocab) {
+  chain_begin();
   const int lane = threadIdx.x & 31;
   const long long i = (long long)blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5);
   if (i >= rows) return;
@@ -127,11 +130,11 @@ int launch_fwd(const void* table, const void* ids, int ids64, void* out, long lo
                long long dim, long long vocab, cudaStream_t st) {
   const int grid = grid_for(rows * dim, 256);
   if (ids64)
-    embedding_forward_kernel<T, long long><<<grid, 256, 0, st>>>(
-        static_cast<const T*>(table), ids, static_cast<T*>(out), rows, dim, vocab);
+    launch_chained(embedding_forward_kernel<T, long long>, grid, 256, 0, st, static_cast<const T*>(table), ids,
+                   static_cast<T*>(out), rows, dim, vocab);
   else
-    embedding_forward_kernel<T, int><<<grid, 256, 0, st>>>(
-        static_cast<const T*>(table), ids, static_cast<T*>(out), rows, dim, vocab);
+    launch_chained(embedding_forward_kernel<T, int>, grid, 256, 0, st, static_cast<const T*>(table), ids,
+                   static_cast<T*>(out), rows, dim, vocab);
   return FLB200_OK;
 }
 template <typename T>
@@ -142,20 +145,20 @@ int launch_bwd(const void* grad_out, const void* ids, int ids64, float* grad_tab
     if (rows == 0) return FLB200_OK;
     const unsigned pgrid = (unsigned)((rows + 7) / 8);
     if (ids64)
-      embedding_backward_by_position_kernel<T, long long><<<pgrid, 256, 0, st>>>(
-          static_cast<const T*>(grad_out), ids, grad_table, rows, dim, vocab);
+      launch_chained(embedding_backward_by_position_kernel<T, long long>, pgrid, 256, 0, st,
+                     static_cast<const T*>(grad_out), ids, grad_table, rows, dim, vocab);
     else
-      embedding_backward_by_position_kernel<T, int><<<pgrid, 256, 0, st>>>(
-          static_cast<const T*>(grad_out), ids, grad_table, rows, dim, vocab);
+      launch_chained(embedding_backward_by_position_kernel<T, int>, pgrid, 256, 0, st,
+                     static_cast<const T*>(grad_out), ids, grad_table, rows, dim, vocab);
     return FLB200_OK;
   }
   const unsigned grid = (unsigned)((vocab + 7) / 8);
   if (ids64)
-    embedding_backward_kernel<T, long long><<<grid, 256, 0, st>>>(
-        static_cast<const T*>(grad_out), ids, grad_table, rows, dim, vocab);
+    launch_chained(embedding_backward_kernel<T, long long>, grid, 256, 0, st, static_cast<const T*>(grad_out),
+                   ids, grad_table, rows, dim, vocab);
   else
-    embedding_backward_kernel<T, int><<<grid, 256, 0, st>>>(
-        static_cast<const T*>(grad_out), ids, grad_table, rows, dim, vocab);
+    launch_chained(embedding_backward_kernel<T, int>, grid, 256, 0, st, static_cast<const T*>(grad_out), ids,
+                   grad_table, rows, dim, vocab);
   return FLB200_OK;
 }
 

@@ -23,6 +23,7 @@ template <typename T>
 __global__ void __launch_bounds__(256)
 filter_permute_kernel(const T* __restrict__ w, T* __restrict__ out, int Cout, int C, int RS,
                       unsigned rs_magic, int ci_shift, long long s_tap, long long s_co, long long s_ci, int pad) {
+  chain_begin();
   extern __shared__ char permute_smem[];
   T* tile = reinterpret_cast<T*>(permute_smem);
   const int ci_run = 1 << ci_shift;
@@ -81,7 +82,8 @@ int filter_permute(const T* w, T* out, int Cout, int C, int RS, long long s_tap,
             (unsigned)groups);
   FLB200_REQUIRE(grid.y <= 65535 && groups <= 65535, "filter_permute: too many channels");
   const unsigned magic = RS == 1 ? 0u : (unsigned)(((1ull << 32) + RS - 1) / RS);
-  filter_permute_kernel<T><<<grid, 256, smem, st>>>(w, out, Cout, C, RS, magic, shift, s_tap, s_co, s_ci, pad);
+  launch_chained(filter_permute_kernel<T>, grid, 256, smem, st, w, out, Cout, C, RS, magic, shift, s_tap, s_co,
+                 s_ci, pad);
   FLB200_AFTER_LAUNCH("filter_permute");
   return FLB200_OK;
 }

@@ -31,6 +31,7 @@ layernorm_forward_kernel(const T* __restrict__ x, const float* __restrict__ weig
                          const float* __restrict__ bias, T* __restrict__ y,
                          T* __restrict__ xhat, float* __restrict__ mean_out,
                          float* __restrict__ invstd_out, long long rows, int features, float eps) {
+  chain_begin();
   const int lane = threadIdx.x & 31;
   const long long r = (long long)blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5);
   if (r >= rows) return;
@@ -75,6 +76,7 @@ __global__ void __launch_bounds__(256)
 layernorm_backward_kernel(const T* __restrict__ dy, const T* __restrict__ xhat,
                           const float* __restrict__ weight, const float* __restrict__ invstd,
                           T* __restrict__ dx, long long rows, int features) {
+  chain_begin();
   const int lane = threadIdx.x & 31;
   const long long r = (long long)blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5);
   if (r >= rows) return;
@@ -127,6 +129,7 @@ layernorm_forward_vec_kernel(const T* __restrict__ x, const float* __restrict__ 
                              T* __restrict__ xhat, float* __restrict__ mean_out,
                              float* __restrict__ invstd_out, long long rows, int features,
                              float eps) {
+  chain_begin();
   constexpr int V = 16 / sizeof(T);
   const int lane = threadIdx.x & 31;
   const long long r = (long long)blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5);
@@ -187,6 +190,7 @@ __global__ void __launch_bounds__(256)
 layernorm_backward_vec_kernel(const T* __restrict__ dy, const T* __restrict__ xhat,
                               const float* __restrict__ weight, const float* __restrict__ invstd,
                               T* __restrict__ dx, long long rows, int features) {
+  chain_begin();
   constexpr int V = 16 / sizeof(T);
   const int lane = threadIdx.x & 31;
   const long long r = (long long)blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5);
@@ -242,7 +246,7 @@ int launch_forward(const void* x, const float* w, const float* b, void* y, void*
     constexpr int V = 16 / sizeof(T);
 #define FLB200_LN_VEC(PERV)                                                                       \
   if (features <= 32 * V * PERV) {                                                                \
-    layernorm_forward_vec_kernel<T, PERV><<<grid, 256, 0, st>>>(                                  \
+    launch_chained(layernorm_forward_vec_kernel<T, PERV>, grid, 256, 0, st, \
         static_cast<const T*>(x), w, b, static_cast<T*>(y), static_cast<T*>(xhat), mean, invstd,  \
         rows, features, eps);                                                                     \
     return FLB200_OK;                                                                             \
@@ -257,7 +261,7 @@ int launch_forward(const void* x, const float* w, const float* b, void* y, void*
   }
 #define FLB200_LN_CASE(PER)                                                                       \
   if (features <= 32 * PER) {                                                                     \
-    layernorm_forward_kernel<T, PER><<<grid, 256, 0, st>>>(                                       \
+    launch_chained(layernorm_forward_kernel<T, PER>, grid, 256, 0, st, \
         static_cast<const T*>(x), w, b, static_cast<T*>(y), static_cast<T*>(xhat), mean, invstd,  \
         rows, features, eps);                                                                     \
     return FLB200_OK;                                                                             \
@@ -280,7 +284,7 @@ int launch_backward(const void* dy, const void* xhat, const float* w, const floa
     constexpr int V = 16 / sizeof(T);
 #define FLB200_LN_VEC(PERV)                                                                   \
   if (features <= 32 * V * PERV) {                                                            \
-    layernorm_backward_vec_kernel<T, PERV><<<grid, 256, 0, st>>>(                             \
+    launch_chained(layernorm_backward_vec_kernel<T, PERV>, grid, 256, 0, st, \
         static_cast<const T*>(dy), static_cast<const T*>(xhat), w, invstd, static_cast<T*>(dx), \
         rows, features);                                                                      \
     return FLB200_OK;                                                                         \
@@ -295,7 +299,7 @@ int launch_backward(const void* dy, const void* xhat, const float* w, const floa
   }
 #define FLB200_LN_CASE(PER)                                                                   \
   if (features <= 32 * PER) {                                                                 \
-    layernorm_backward_kernel<T, PER><<<grid, 256, 0, st>>>(                                  \
+    launch_chained(layernorm_backward_kernel<T, PER>, grid, 256, 0, st, \
         static_cast<const T*>(dy), static_cast<const T*>(xhat), w, invstd, static_cast<T*>(dx), \
         rows, features);                                                                      \
     return FLB200_OK;                                                                         \

@@ -64,6 +64,7 @@ __global__ void __launch_bounds__(256) pool_forward_kernel(const T* __restrict__
                                                            T* __restrict__ y,
                                                            uint8_t* __restrict__ argmax,
                                                            PoolGeo g) {
+  chain_begin();
   const long long out_plane = (long long)g.Ho * g.Wo;
   const long long total = g.planes * out_plane;
   const long long stride = (long long)gridDim.x * blockDim.x;
@@ -103,6 +104,7 @@ __global__ void __launch_bounds__(256) pool_backward_kernel(const T* __restrict_
                                                             const T* __restrict__ x,
                                                             const uint8_t* __restrict__ argmax,
                                                             T* __restrict__ dx, PoolGeo g) {
+  chain_begin();
   const long long in_plane = (long long)g.H * g.W;
   const long long out_plane = (long long)g.Ho * g.Wo;
   const long long total = g.planes * in_plane;
@@ -153,6 +155,7 @@ template <int WX, int WY, int SX, int SY>
 __global__ void __launch_bounds__(256)
 pool_forward_max_tile_kernel(const float* __restrict__ x, float* __restrict__ y,
                              uint8_t* __restrict__ argmax, PoolGeo g, int band_rows, int nbands) {
+  chain_begin();
   extern __shared__ float tile[];
   const int wx = WX ? WX : g.wx, wy = WY ? WY : g.wy, sx = SX ? SX : g.sx, sy = SY ? SY : g.sy;
   const long long plane = blockIdx.x / nbands;
@@ -228,6 +231,7 @@ __global__ void __launch_bounds__(256)
 pool_backward_max_tile_kernel(const float* __restrict__ dy, const uint8_t* __restrict__ argmax,
                               float* __restrict__ dx, PoolGeo g, int band_rows, int nbands,
                               int max_out_rows) {
+  chain_begin();
   extern __shared__ float tile[];  // [max_out_rows][Wo] dy, then the argmax bytes
   const int wx = WX ? WX : g.wx, wy = WY ? WY : g.wy, sx = SX ? SX : g.sx, sy = SY ? SY : g.sy;
   uint8_t* sel = reinterpret_cast<uint8_t*>(tile + (size_t)max_out_rows * g.Wo);
@@ -290,6 +294,7 @@ pool_backward_max_tile_kernel(const float* __restrict__ dy, const uint8_t* __res
 __global__ void __launch_bounds__(256)
 pool_backward_global_avg_kernel(const float* __restrict__ dy, float* __restrict__ dx,
                                 long long planes, int hw) {
+  chain_begin();
   const long long total = planes * hw;
   const float div = (float)hw;  // divided, not multiplied by the reciprocal: same bits as the generic kernel
   const long long stride = (long long)gridDim.x * blockDim.x;
@@ -300,14 +305,14 @@ pool_backward_global_avg_kernel(const float* __restrict__ dy, float* __restrict_
 template <int WX, int WY, int SX, int SY>
 void launch_pool_fwd_tile(const float* x, float* y, uint8_t* argmax, const PoolGeo& g, int band,
                           int nbands, size_t smem, cudaStream_t st) {
-  pool_forward_max_tile_kernel<WX, WY, SX, SY><<<(unsigned)(g.planes * nbands), 256, smem, st>>>(
-      x, y, argmax, g, band, nbands);
+  launch_chained(pool_forward_max_tile_kernel<WX, WY, SX, SY>, (unsigned)(g.planes * nbands), 256, smem, st, x,
+                 y, argmax, g, band, nbands);
 }
 template <int WX, int WY, int SX, int SY>
 void launch_pool_bwd_tile(const float* dy, const uint8_t* argmax, float* dx, const PoolGeo& g,
                           int band, int nbands, int out_rows, size_t smem, cudaStream_t st) {
-  pool_backward_max_tile_kernel<WX, WY, SX, SY>
-      <<<(unsigned)(g.planes * nbands), 256, smem, st>>>(dy, argmax, dx, g, band, nbands, out_rows);
+  launch_chained(pool_backward_max_tile_kernel<WX, WY, SX, SY>, (unsigned)(g.planes * nbands), 256, smem, st,
+                 dy, argmax, dx, g, band, nbands, out_rows);
 }
 bool is_window(const PoolGeo& g, int wx, int wy, int sx, int sy) {
   return g.wx == wx && g.wy == wy && g.sx == sx && g.sy == sy;
@@ -342,6 +347,7 @@ template <typename T>
 __global__ void __launch_bounds__(256)
 pool_backward_max_strip_kernel(const T* __restrict__ dy, const uint8_t* __restrict__ argmax,
                                T* __restrict__ dx, PoolGeo g) {
+  chain_begin();
   const int strips_w = (g.W + 3) >> 2;
   const int strips = strips_w * g.H;
   const int in_plane = g.H * g.W, out_plane = g.Ho * g.Wo;
@@ -396,6 +402,7 @@ template <typename T, int V>
 __global__ void __launch_bounds__(256)
 pool_forward_cl_kernel(const T* __restrict__ x, T* __restrict__ y, uint8_t* __restrict__ argmax,
                        PoolGeo g, int C, int per_image) {
+  chain_begin();
   // blockIdx.y = image; the index inside an image fits 32 bits (checked by the launcher)
   const unsigned cv = C / V;
   const long long n = blockIdx.y;
@@ -465,6 +472,7 @@ __global__ void __launch_bounds__(256)
 pool_backward_cl_kernel(const T* __restrict__ dy, const T* __restrict__ x,
                         const uint8_t* __restrict__ argmax, T* __restrict__ dx, PoolGeo g, int C,
                         int per_image) {
+  chain_begin();
   const unsigned cv = C / V;
   const long long n = blockIdx.y;
   for (unsigned t = blockIdx.x * blockDim.x + threadIdx.x; t < (unsigned)per_image;
@@ -551,6 +559,7 @@ __global__ void __launch_bounds__(256)
 pool_forward_max_cl_fixed_kernel(const float* __restrict__ x, float* __restrict__ y,
                                  uint8_t* __restrict__ argmax, PoolGeo g, int C, int cv_shift,
                                  int per_image) {
+  chain_begin();
   const long long n = blockIdx.y;
   const unsigned cv = (unsigned)C >> 2;
   for (unsigned t = blockIdx.x * blockDim.x + threadIdx.x; t < (unsigned)per_image;
@@ -600,6 +609,7 @@ __global__ void __launch_bounds__(256)
 pool_backward_max_cl_fixed_kernel(const float* __restrict__ dy, const uint8_t* __restrict__ argmax,
                                   float* __restrict__ dx, PoolGeo g, int C, int cv_shift,
                                   int per_image) {
+  chain_begin();
   constexpr int NW = (WIN + S - 1) / S;  // windows per axis that can cover a pixel
   const long long n = blockIdx.y;
   const unsigned cv = (unsigned)C >> 2;
@@ -643,6 +653,7 @@ __global__ void __launch_bounds__(256)
 pool_backward_max_cl_cell_kernel(const float* __restrict__ dy, const uint8_t* __restrict__ argmax,
                                  float* __restrict__ dx, PoolGeo g, int C, int cv_shift,
                                  int cells_w, int per_image) {
+  chain_begin();
   const long long n = blockIdx.y;
   const unsigned cv = (unsigned)C >> 2;
   for (unsigned t = blockIdx.x * blockDim.x + threadIdx.x; t < (unsigned)per_image;
@@ -721,20 +732,20 @@ int launch_pool_cl(bool backward, const PoolGeo& g, int C, int N, const void* a,
         int shift = -1;
         if ((cvv & (cvv - 1)) == 0) { shift = 0; while ((1u << shift) < cvv) ++shift; }
         if (g.wx == 3)
-          pool_forward_max_cl_fixed_kernel<3, 2><<<grid, 256, 0, st>>>(
-              static_cast<const float*>(a), static_cast<float*>(out), argmax_out, g, C, shift, pi);
+          launch_chained(pool_forward_max_cl_fixed_kernel<3, 2>, grid, 256, 0, st, static_cast<const float*>(a),
+                         static_cast<float*>(out), argmax_out, g, C, shift, pi);
         else
-          pool_forward_max_cl_fixed_kernel<2, 2><<<grid, 256, 0, st>>>(
-              static_cast<const float*>(a), static_cast<float*>(out), argmax_out, g, C, shift, pi);
+          launch_chained(pool_forward_max_cl_fixed_kernel<2, 2>, grid, 256, 0, st, static_cast<const float*>(a),
+                         static_cast<float*>(out), argmax_out, g, C, shift, pi);
         FLB200_AFTER_LAUNCH("pool2d_forward_max_channels_last");
         return FLB200_OK;
       }
     }
     if (vec)
-      pool_forward_cl_kernel<T, V><<<grid, 256, 0, st>>>(static_cast<const T*>(a),
+      launch_chained(pool_forward_cl_kernel<T, V>, grid, 256, 0, st, static_cast<const T*>(a),
                                                          static_cast<T*>(out), argmax_out, g, C, pi);
     else
-      pool_forward_cl_kernel<T, 1><<<grid, 256, 0, st>>>(static_cast<const T*>(a),
+      launch_chained(pool_forward_cl_kernel<T, 1>, grid, 256, 0, st, static_cast<const T*>(a),
                                                          static_cast<T*>(out), argmax_out, g, C, pi);
     FLB200_AFTER_LAUNCH("pool2d_forward_channels_last");
   } else {
@@ -752,33 +763,33 @@ int launch_pool_cl(bool backward, const PoolGeo& g, int C, int N, const void* a,
           if (cbx > 4096) cbx = 4096;
           const dim3 cgrid((unsigned)cbx, (unsigned)N);
           if (g.wx == 3)
-            pool_backward_max_cl_cell_kernel<3><<<cgrid, 256, 0, st>>>(
-                static_cast<const float*>(a), argmax_in, static_cast<float*>(out), g, C, shift,
+            launch_chained(pool_backward_max_cl_cell_kernel<3>, cgrid, 256, 0, st, static_cast<const float*>(a),
+                           argmax_in, static_cast<float*>(out), g, C, shift,
                 (int)cells_w, (int)per_cells);
           else
-            pool_backward_max_cl_cell_kernel<2><<<cgrid, 256, 0, st>>>(
-                static_cast<const float*>(a), argmax_in, static_cast<float*>(out), g, C, shift,
+            launch_chained(pool_backward_max_cl_cell_kernel<2>, cgrid, 256, 0, st, static_cast<const float*>(a),
+                           argmax_in, static_cast<float*>(out), g, C, shift,
                 (int)cells_w, (int)per_cells);
           FLB200_AFTER_LAUNCH("pool2d_backward_max_channels_last");
           return FLB200_OK;
         }
         if (g.wx == 3)
-          pool_backward_max_cl_fixed_kernel<3, 2><<<grid, 256, 0, st>>>(
-              static_cast<const float*>(a), argmax_in, static_cast<float*>(out), g, C, shift, pi);
+          launch_chained(pool_backward_max_cl_fixed_kernel<3, 2>, grid, 256, 0, st,
+                         static_cast<const float*>(a), argmax_in, static_cast<float*>(out), g, C, shift, pi);
         else
-          pool_backward_max_cl_fixed_kernel<2, 2><<<grid, 256, 0, st>>>(
-              static_cast<const float*>(a), argmax_in, static_cast<float*>(out), g, C, shift, pi);
+          launch_chained(pool_backward_max_cl_fixed_kernel<2, 2>, grid, 256, 0, st,
+                         static_cast<const float*>(a), argmax_in, static_cast<float*>(out), g, C, shift, pi);
         FLB200_AFTER_LAUNCH("pool2d_backward_max_channels_last");
         return FLB200_OK;
       }
     }
     if (vec)
-      pool_backward_cl_kernel<T, V><<<grid, 256, 0, st>>>(
-          static_cast<const T*>(a), static_cast<const T*>(x), argmax_in, static_cast<T*>(out), g, C,
+      launch_chained(pool_backward_cl_kernel<T, V>, grid, 256, 0, st, static_cast<const T*>(a),
+                     static_cast<const T*>(x), argmax_in, static_cast<T*>(out), g, C,
           pi);
     else
-      pool_backward_cl_kernel<T, 1><<<grid, 256, 0, st>>>(
-          static_cast<const T*>(a), static_cast<const T*>(x), argmax_in, static_cast<T*>(out), g, C,
+      launch_chained(pool_backward_cl_kernel<T, 1>, grid, 256, 0, st, static_cast<const T*>(a),
+                     static_cast<const T*>(x), argmax_in, static_cast<T*>(out), g, C,
           pi);
     FLB200_AFTER_LAUNCH("pool2d_backward_channels_last");
   }
@@ -868,16 +879,16 @@ int flb200_pool2d_forward(const flb200_pool2d_desc* d, const void* x, void* y, u
   }
   switch (d->dtype) {
     case FLB200_F32:
-      pool_forward_kernel<float><<<grid, 256, 0, st>>>(static_cast<const float*>(x),
+      launch_chained(pool_forward_kernel<float>, grid, 256, 0, st, static_cast<const float*>(x),
                                                        static_cast<float*>(y), argmax, g);
       break;
     case FLB200_F16:
-      pool_forward_kernel<__half><<<grid, 256, 0, st>>>(static_cast<const __half*>(x),
+      launch_chained(pool_forward_kernel<__half>, grid, 256, 0, st, static_cast<const __half*>(x),
                                                         static_cast<__half*>(y), argmax, g);
       break;
     case FLB200_BF16:
-      pool_forward_kernel<__nv_bfloat16><<<grid, 256, 0, st>>>(
-          static_cast<const __nv_bfloat16*>(x), static_cast<__nv_bfloat16*>(y), argmax, g);
+      launch_chained(pool_forward_kernel<__nv_bfloat16>, grid, 256, 0, st, static_cast<const __nv_bfloat16*>(x),
+                     static_cast<__nv_bfloat16*>(y), argmax, g);
       break;
     default:
       return fail(FLB200_UNSUPPORTED, "pool2d_forward: unknown dtype %d", d->dtype);
@@ -917,32 +928,32 @@ int flb200_pool2d_backward(const flb200_pool2d_desc* d, const void* grad_y, cons
     }
     const int strips = ((g.W + 3) / 4) * g.H;
     dim3 sgrid((unsigned)((strips + 255) / 256), (unsigned)(g.planes < 32768 ? g.planes : 32768));
-    pool_backward_max_strip_kernel<float><<<sgrid, 256, 0, st>>>(
-        static_cast<const float*>(grad_y), argmax, static_cast<float*>(grad_x), g);
+    launch_chained(pool_backward_max_strip_kernel<float>, sgrid, 256, 0, st, static_cast<const float*>(grad_y),
+                   argmax, static_cast<float*>(grad_x), g);
     FLB200_AFTER_LAUNCH("pool2d_backward_max");
     return FLB200_OK;
   }
   if (d->mode != FLB200_POOL_MAX && d->dtype == FLB200_F32 && g.Ho == 1 && g.Wo == 1 &&
       g.px == 0 && g.py == 0 && g.wx == g.W && g.wy == g.H && g.H * g.W < (1 << 20)) {
-    pool_backward_global_avg_kernel<<<grid, 256, 0, st>>>(
-        static_cast<const float*>(grad_y), static_cast<float*>(grad_x), g.planes, g.H * g.W);
+    launch_chained(pool_backward_global_avg_kernel, grid, 256, 0, st, static_cast<const float*>(grad_y),
+                   static_cast<float*>(grad_x), g.planes, g.H * g.W);
     FLB200_AFTER_LAUNCH("pool2d_backward_global_avg");
     return FLB200_OK;
   }
   switch (d->dtype) {
     case FLB200_F32:
-      pool_backward_kernel<float><<<grid, 256, 0, st>>>(static_cast<const float*>(grad_y),
+      launch_chained(pool_backward_kernel<float>, grid, 256, 0, st, static_cast<const float*>(grad_y),
                                                         static_cast<const float*>(x), argmax,
                                                         static_cast<float*>(grad_x), g);
       break;
     case FLB200_F16:
-      pool_backward_kernel<__half><<<grid, 256, 0, st>>>(static_cast<const __half*>(grad_y),
+      launch_chained(pool_backward_kernel<__half>, grid, 256, 0, st, static_cast<const __half*>(grad_y),
                                                          static_cast<const __half*>(x), argmax,
                                                          static_cast<__half*>(grad_x), g);
       break;
     case FLB200_BF16:
-      pool_backward_kernel<__nv_bfloat16><<<grid, 256, 0, st>>>(
-          static_cast<const __nv_bfloat16*>(grad_y), static_cast<const __nv_bfloat16*>(x), argmax,
+      launch_chained(pool_backward_kernel<__nv_bfloat16>, grid, 256, 0, st,
+                     static_cast<const __nv_bfloat16*>(grad_y), static_cast<const __nv_bfloat16*>(x), argmax,
           static_cast<__nv_bfloat16*>(grad_x), g);
       break;
     default:

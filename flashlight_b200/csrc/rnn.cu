@@ -138,6 +138,7 @@ __device__ __forceinline__ float sigmoidf_(float v) { return 1.f / (1.f + expf(-
 // bias_comb[j] = b_ih[j] + b_hh[j], except the GRU candidate gate keeps b_ih only.
 __global__ void combine_bias_kernel(const float* __restrict__ b_ih, const float* __restrict__ b_hh,
                                     float* __restrict__ out, int H, int G, int mode) {
+  chain_begin();
   const int j = blockIdx.x * blockDim.x + threadIdx.x;
   if (j >= G * H) return;
   const bool cand = mode == FLB200_RNN_GRU && j >= 2 * H;
@@ -152,6 +153,7 @@ cell_forward_kernel(float* __restrict__ gates, const float* __restrict__ gh,
                     long long hp_stride, const float* __restrict__ c_prev, long long cp_stride,
                     float* __restrict__ c_out, float* __restrict__ q_out, float* __restrict__ h_out,
                     long long ho_stride, int B, int H, int mode) {
+  chain_begin();
   const int idx = blockIdx.x * blockDim.x + threadIdx.x;
   if (idx >= B * H) return;
   const int b = idx / H, j = idx - b * H;
@@ -194,6 +196,7 @@ cell_backward_kernel(const float* __restrict__ gates, const float* __restrict__ 
                      long long hp_stride, const float* __restrict__ dy, long long dy_stride,
                      float* __restrict__ dh, float* __restrict__ dc, float* __restrict__ dgx,
                      float* __restrict__ dgh, int B, int H, int mode) {
+  chain_begin();
   const int idx = blockIdx.x * blockDim.x + threadIdx.x;
   if (idx >= B * H) return;
   const int b = idx / H, j = idx - b * H;
@@ -235,6 +238,7 @@ cell_backward_kernel(const float* __restrict__ gates, const float* __restrict__ 
 // dst[b][j] = src ? src[b*src_stride + j] : 0
 __global__ void copy_rows_kernel(const float* __restrict__ src, long long src_stride,
                                  float* __restrict__ dst, long long dst_stride, int B, int H) {
+  chain_begin();
   const int idx = blockIdx.x * blockDim.x + threadIdx.x;
   if (idx >= B * H) return;
   const int b = idx / H, j = idx - b * H;
@@ -407,7 +411,7 @@ static int rnn_forward_impl(const flb200_rnn_desc* d, const void* x, const void*
       float* gates = reinterpret_cast<float*>(rs + RL.per_p * (size_t)p);
       float* cells = reinterpret_cast<float*>(rs + RL.per_p * (size_t)p + RL.cell_off);
       float* qbuf = reinterpret_cast<float*>(rs + RL.per_p * (size_t)p + RL.q_off);
-      combine_bias_kernel<<<(unsigned)((GH + 255) / 256), 256, 0, st>>>(wf + po.b_ih, wf + po.b_hh,
+      launch_chained(combine_bias_kernel, (unsigned)((GH + 255) / 256), 256, 0, st, wf + po.b_ih, wf + po.b_hh,
                                                                         bias, H, r.G, r.mode);
       FLB200_AFTER_LAUNCH("rnn_combine_bias");
       // all input projections of this pseudo-layer
@@ -470,8 +474,8 @@ static int rnn_forward_impl(const flb200_rnn_desc* d, const void* x, const void*
                           GH, 1.f, mmws, mmws_bytes, stream))
             return rc;
         }
-        cell_forward_kernel<<<cell_grid, 256, 0, st>>>(
-            g_t, gh, wf + po.b_hh, h_prev, hp_stride, c_prev, H, cells + (long long)t * BH,
+        launch_chained(cell_forward_kernel, cell_grid, 256, 0, st, g_t, gh, wf + po.b_hh, h_prev, hp_stride,
+                       c_prev, H, cells + (long long)t * BH,
             qbuf + (long long)t * BH, h_t, out_stride, B, H, r.mode);
         FLB200_AFTER_LAUNCH("rnn_cell_forward");
         h_prev = h_t;
@@ -479,13 +483,13 @@ static int rnn_forward_impl(const flb200_rnn_desc* d, const void* x, const void*
         c_prev = cells + (long long)t * BH;
       }
       if (hy) {
-        copy_rows_kernel<<<cell_grid, 256, 0, st>>>(h_prev, hp_stride,
+        launch_chained(copy_rows_kernel, cell_grid, 256, 0, st, h_prev, hp_stride,
                                                     static_cast<float*>(hy) + (long long)p * BH, H,
                                                     B, H);
         FLB200_AFTER_LAUNCH("rnn_copy_hy");
       }
       if (cy && r.mode == FLB200_RNN_LSTM) {
-        copy_rows_kernel<<<cell_grid, 256, 0, st>>>(c_prev, H,
+        launch_chained(copy_rows_kernel, cell_grid, 256, 0, st, c_prev, H,
                                                     static_cast<float*>(cy) + (long long)p * BH, H,
                                                     B, H);
         FLB200_AFTER_LAUNCH("rnn_copy_cy");
@@ -603,12 +607,11 @@ static int rnn_backward_impl(const flb200_rnn_desc* d, const void* x, const void
       float* dh = reinterpret_cast<float*>(ws + W.dh + W.h_stride * dir);
       float* dc = reinterpret_cast<float*>(ws + W.dc + W.h_stride * dir);
       if (!persistent) {
-      copy_rows_kernel<<<cell_grid, 256, 0, st>>>(
-          grad_hy ? static_cast<const float*>(grad_hy) + (long long)p * BH : nullptr, H, dh, H, B,
+      launch_chained(copy_rows_kernel, cell_grid, 256, 0, st,
+                     grad_hy ? static_cast<const float*>(grad_hy) + (long long)p * BH : nullptr, H, dh, H, B,
           H);
       FLB200_AFTER_LAUNCH("rnn_init_dh");
-      copy_rows_kernel<<<cell_grid, 256, 0, st>>>(
-          grad_cy && r.mode == FLB200_RNN_LSTM
+      launch_chained(copy_rows_kernel, cell_grid, 256, 0, st, grad_cy && r.mode == FLB200_RNN_LSTM
               ? static_cast<const float*>(grad_cy) + (long long)p * BH
               : nullptr,
           H, dc, H, B, H);
@@ -623,8 +626,8 @@ static int rnn_backward_impl(const flb200_rnn_desc* d, const void* x, const void
         const long long hp_stride = first ? H : ys;
         const float* c_prev = first ? (cxf ? cxf + (long long)p * BH : zero)
                                     : cells + (long long)t_prev * BH;
-        cell_backward_kernel<<<cell_grid, 256, 0, st>>>(
-            gates + (long long)t * B * GH, cells + (long long)t * BH, c_prev, H,
+        launch_chained(cell_backward_kernel, cell_grid, 256, 0, st, gates + (long long)t * B * GH,
+                       cells + (long long)t * BH, c_prev, H,
             qbuf + (long long)t * BH, h_prev, hp_stride,
             dy_l ? dy_l + (long long)t * B * ys + (long long)dir * H : nullptr, ys, dh, dc,
             dgx + (long long)t * B * GH, dgh + (long long)t * B * GH, B, H, r.mode);
@@ -636,13 +639,13 @@ static int rnn_backward_impl(const flb200_rnn_desc* d, const void* x, const void
       }
       }  // !persistent
       if (grad_hx) {
-        copy_rows_kernel<<<cell_grid, 256, 0, st>>>(
-            dh, H, static_cast<float*>(grad_hx) + (long long)p * BH, H, B, H);
+        launch_chained(copy_rows_kernel, cell_grid, 256, 0, st, dh, H,
+                       static_cast<float*>(grad_hx) + (long long)p * BH, H, B, H);
         FLB200_AFTER_LAUNCH("rnn_copy_dhx");
       }
       if (grad_cx && r.mode == FLB200_RNN_LSTM) {
-        copy_rows_kernel<<<cell_grid, 256, 0, st>>>(
-            dc, H, static_cast<float*>(grad_cx) + (long long)p * BH, H, B, H);
+        launch_chained(copy_rows_kernel, cell_grid, 256, 0, st, dc, H,
+                       static_cast<float*>(grad_cx) + (long long)p * BH, H, B, H);
         FLB200_AFTER_LAUNCH("rnn_copy_dcx");
       }
       // dW_ih[GH][In] = dgx^T * in   (K = T*B)

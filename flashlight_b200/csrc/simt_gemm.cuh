@@ -223,6 +223,7 @@ template <class T, class AL, class BL, class EP>
 __global__ void __launch_bounds__(T::kThreads, T::kMinBlocks)
 ffma_gemm_kernel(const AL al, const BL bl, const EP ep, int M, int N, int K, int tiles_n,
                  int csplits, int psplits, int k_per_split, float* __restrict__ partial) {
+  chain_begin();
   constexpr int BM = T::BM, BN = T::BN, TM = T::TM, TN = T::TN, TX = T::TX, TY = T::TY;
   constexpr bool AK = k_layout(AL::kKind), BK = k_layout(BL::kKind);
   using S = FfmaSmem<T, AL, BL>;
@@ -482,6 +483,7 @@ ffma_gemm_kernel(const AL al, const BL bl, const EP ep, int M, int N, int K, int
 template <class EP>
 __global__ void __launch_bounds__(256)
 ffma_reduce_kernel(const float* __restrict__ partial, const EP ep, int M, int N, int Z, int psplits) {
+  chain_begin();
   const long long mn = (long long)M * N;
   const long long total = mn * Z;
   const long long stride = (long long)gridDim.x * blockDim.x;
@@ -602,13 +604,15 @@ int launch_ffma(const char* name, const AL& al, const BL& bl, const EP& ep, long
   cfg.blockDim = dim3(T::kThreads);
   cfg.dynamicSmemBytes = S::kTotal;
   cfg.stream = st;
-  cudaLaunchAttribute attr[1];
-  attr[0].id = cudaLaunchAttributeClusterDimension;
-  attr[0].val.clusterDim.x = 1;
-  attr[0].val.clusterDim.y = 1;
-  attr[0].val.clusterDim.z = (unsigned)p.csplits;
+  cudaLaunchAttribute attr[2];
+  attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;  // (launch_chained)
+  attr[0].val.programmaticStreamSerializationAllowed = 1;
+  attr[1].id = cudaLaunchAttributeClusterDimension;
+  attr[1].val.clusterDim.x = 1;
+  attr[1].val.clusterDim.y = 1;
+  attr[1].val.clusterDim.z = (unsigned)p.csplits;
   cfg.attrs = attr;
-  cfg.numAttrs = p.csplits > 1 ? 1 : 0;
+  cfg.numAttrs = p.csplits > 1 ? 2 : 1;
   FLB200_CUDA_CHECK(cudaLaunchKernelEx(&cfg, kernel, al, bl, ep, (int)M, (int)N, (int)K, (int)tiles_n,
                                        p.csplits, p.psplits, p.k_per_split, partial));
   FLB200_AFTER_LAUNCH(name);
@@ -657,7 +661,7 @@ int launch_simt_gemm(const char* name, const AL& al, const BL& bl, const EP& ep,
   }
   if (rc) return rc;
   if (p.psplits > 1) {
-    ffma_reduce_kernel<EP><<<grid_for(M * N * Z, 256), 256, 0, st>>>(partial, ep, (int)M, (int)N,
+    launch_chained(ffma_reduce_kernel<EP>, grid_for(M * N * Z, 256), 256, 0, st, partial, ep, (int)M, (int)N,
                                                                       (int)Z, p.psplits);
     FLB200_AFTER_LAUNCH("ffma_reduce");
   }

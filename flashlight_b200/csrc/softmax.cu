@@ -39,6 +39,7 @@ __device__ __forceinline__ float group_max(float v, float* scratch) {
 template <typename T, int GROUP>
 __global__ void __launch_bounds__(kRowThreads)
 log_softmax_forward_kernel(const T* __restrict__ x, T* __restrict__ y, long long C, long long X) {
+  chain_begin();
   __shared__ float scratch[32];
   const int rows_per_cta = kRowThreads / GROUP;
   const int lane = threadIdx.x % GROUP;
@@ -111,6 +112,7 @@ __device__ __forceinline__ float row_lse(const T* xr, long long C4, float* scrat
 __global__ void __launch_bounds__(kRowThreads)
 log_softmax_forward_vec_kernel(const float* __restrict__ x, float* __restrict__ y, long long C4,
                                long long X) {
+  chain_begin();
   __shared__ float scratch[32];
   for (long long row = blockIdx.x; row < X; row += gridDim.x) {
     const float4* xr = reinterpret_cast<const float4*>(x) + row * C4;
@@ -130,6 +132,7 @@ log_softmax_forward_vec_kernel(const float* __restrict__ x, float* __restrict__ 
 template <typename T>
 __global__ void __launch_bounds__(kRowThreads)
 row_lse_kernel(const T* __restrict__ x, float* __restrict__ lse, long long C4, long long X) {
+  chain_begin();
   __shared__ float scratch[32];
   for (long long row = blockIdx.x; row < X; row += gridDim.x) {
     const float v = row_lse(x + row * C4 * 4, C4, scratch);
@@ -142,6 +145,7 @@ template <typename T, int GROUP>
 __global__ void __launch_bounds__(kRowThreads)
 log_softmax_backward_kernel(const T* __restrict__ y, const T* __restrict__ dy,
                             T* __restrict__ dx, long long C, long long X) {
+  chain_begin();
   __shared__ float scratch[32];
   const int rows_per_cta = kRowThreads / GROUP;
   const int lane = threadIdx.x % GROUP;
@@ -178,6 +182,7 @@ cce_forward_kernel(const T* __restrict__ logp, const int32_t* __restrict__ targe
                    float* __restrict__ loss_none, float2* __restrict__ partial,
                    int32_t* __restrict__ bad_flag, long long C, long long X, int ignore_index,
                    const float* __restrict__ lse) {
+  chain_begin();
   __shared__ float scratch[32];
   float s = 0.f, n = 0.f;
   const long long stride = (long long)gridDim.x * blockDim.x;
@@ -203,6 +208,7 @@ cce_forward_kernel(const T* __restrict__ logp, const int32_t* __restrict__ targe
 __global__ void cce_finalize_kernel(const float2* __restrict__ partial, int nparts,
                                     float* __restrict__ loss, int32_t* __restrict__ count_out,
                                     int reduction) {
+  chain_begin();
   double s = 0.0, n = 0.0;
   for (int i = threadIdx.x; i < nparts; i += 32) {
     s += (double)partial[i].x;
@@ -222,6 +228,7 @@ __global__ void __launch_bounds__(256)
 cce_backward_kernel(const float* __restrict__ grad_loss, const int32_t* __restrict__ targets,
                     const int32_t* __restrict__ count, T* __restrict__ grad_logp, long long C,
                     long long X, int reduction, int ignore_index) {
+  chain_begin();
   const long long total = C * X;
   const long long stride = (long long)gridDim.x * blockDim.x;
   for (long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x; i < total; i += stride) {
@@ -240,6 +247,7 @@ lsm_cce_backward_kernel(const T* __restrict__ y, const float* __restrict__ grad_
                         const int32_t* __restrict__ targets, const int32_t* __restrict__ count,
                         T* __restrict__ dx, long long C, long long X, int reduction,
                         int ignore_index) {
+  chain_begin();
   const long long total = C * X;
   const long long stride = (long long)gridDim.x * blockDim.x;
   for (long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x; i < total; i += stride) {
@@ -264,6 +272,7 @@ lsm_cce_backward_vec_kernel(const T* __restrict__ y, const float* __restrict__ l
                             const float* __restrict__ grad_loss, const int32_t* __restrict__ targets,
                             const int32_t* __restrict__ count, T* __restrict__ dx,
                             long long C4, int reduction, int ignore_index) {
+  chain_begin();
   const long long row = blockIdx.y;
   const int t = targets[row];
   const bool live = t != ignore_index && t >= 0 && t < 4 * C4;
@@ -299,8 +308,9 @@ int launch_lsm_cce_backward(const void* y, const float* lse, const float* grad_l
                             int ignore_index, cudaStream_t st) {
   long long bx = (C / 4 + 255) / 256;
   if (bx > 64) bx = 64;
-  lsm_cce_backward_vec_kernel<T, LSE><<<dim3((unsigned)bx, (unsigned)X), 256, 0, st>>>(
-      static_cast<const T*>(y), lse, grad_loss, targets, count, static_cast<T*>(dx), C / 4, reduction, ignore_index);
+  launch_chained(lsm_cce_backward_vec_kernel<T, LSE>, dim3((unsigned)bx, (unsigned)X), 256, 0, st,
+                 static_cast<const T*>(y), lse, grad_loss, targets, count, static_cast<T*>(dx), C / 4,
+                 reduction, ignore_index);
   FLB200_AFTER_LAUNCH("log_softmax_cce_backward");
   return FLB200_OK;
 }
@@ -317,27 +327,27 @@ int lsm_launch(bool backward, const void* a, const void* b, void* out, long long
   if (C <= 1024) {
     const int grid = grid_for(X, kRowThreads / 32);
     if (backward)
-      log_softmax_backward_kernel<T, 32><<<grid, kRowThreads, 0, st>>>(
-          static_cast<const T*>(a), static_cast<const T*>(b), static_cast<T*>(out), C, X);
+      launch_chained(log_softmax_backward_kernel<T, 32>, grid, kRowThreads, 0, st, static_cast<const T*>(a),
+                     static_cast<const T*>(b), static_cast<T*>(out), C, X);
     else
-      log_softmax_forward_kernel<T, 32><<<grid, kRowThreads, 0, st>>>(
-          static_cast<const T*>(a), static_cast<T*>(out), C, X);
+      launch_chained(log_softmax_forward_kernel<T, 32>, grid, kRowThreads, 0, st, static_cast<const T*>(a),
+                     static_cast<T*>(out), C, X);
   } else {
     const int grid = grid_for(X, 1);
     if constexpr (std::is_same<T, float>::value) {
       if (!backward && C % 4 == 0 && aligned16(a) && aligned16(out)) {
-        log_softmax_forward_vec_kernel<<<grid, kRowThreads, 0, st>>>(
-            static_cast<const float*>(a), static_cast<float*>(out), C / 4, X);
+        launch_chained(log_softmax_forward_vec_kernel, grid, kRowThreads, 0, st, static_cast<const float*>(a),
+                       static_cast<float*>(out), C / 4, X);
         FLB200_AFTER_LAUNCH("log_softmax_forward");
         return FLB200_OK;
       }
     }
     if (backward)
-      log_softmax_backward_kernel<T, kRowThreads><<<grid, kRowThreads, 0, st>>>(
-          static_cast<const T*>(a), static_cast<const T*>(b), static_cast<T*>(out), C, X);
+      launch_chained(log_softmax_backward_kernel<T, kRowThreads>, grid, kRowThreads, 0, st,
+                     static_cast<const T*>(a), static_cast<const T*>(b), static_cast<T*>(out), C, X);
     else
-      log_softmax_forward_kernel<T, kRowThreads><<<grid, kRowThreads, 0, st>>>(
-          static_cast<const T*>(a), static_cast<T*>(out), C, X);
+      launch_chained(log_softmax_forward_kernel<T, kRowThreads>, grid, kRowThreads, 0, st,
+                     static_cast<const T*>(a), static_cast<T*>(out), C, X);
   }
   FLB200_AFTER_LAUNCH(backward ? "log_softmax_backward" : "log_softmax_forward");
   return FLB200_OK;
@@ -403,25 +413,25 @@ static int cce_forward_impl(const void* logp, const float* lse, const int32_t* t
   float* loss_none = reduction == FLB200_REDUCE_NONE ? loss : nullptr;
   switch (dtype) {
     case FLB200_F32:
-      cce_forward_kernel<float><<<grid, 256, 0, st>>>(static_cast<const float*>(logp), targets,
+      launch_chained(cce_forward_kernel<float>, grid, 256, 0, st, static_cast<const float*>(logp), targets,
                                                       loss_none, partial, bad_target_flag, C, X,
                                                       ignore_index, lse);
       break;
     case FLB200_F16:
-      cce_forward_kernel<__half><<<grid, 256, 0, st>>>(static_cast<const __half*>(logp), targets,
+      launch_chained(cce_forward_kernel<__half>, grid, 256, 0, st, static_cast<const __half*>(logp), targets,
                                                        loss_none, partial, bad_target_flag, C, X,
                                                        ignore_index, lse);
       break;
     case FLB200_BF16:
-      cce_forward_kernel<__nv_bfloat16><<<grid, 256, 0, st>>>(
-          static_cast<const __nv_bfloat16*>(logp), targets, loss_none, partial, bad_target_flag, C,
+      launch_chained(cce_forward_kernel<__nv_bfloat16>, grid, 256, 0, st,
+                     static_cast<const __nv_bfloat16*>(logp), targets, loss_none, partial, bad_target_flag, C,
           X, ignore_index, lse);
       break;
     default:
       return fail(FLB200_UNSUPPORTED, "cce_forward: unknown dtype %d", dtype);
   }
   FLB200_AFTER_LAUNCH("cce_forward");
-  cce_finalize_kernel<<<1, 32, 0, st>>>(partial, grid, loss, count_out, reduction);
+  launch_chained(cce_finalize_kernel, 1, 32, 0, st, partial, grid, loss, count_out, reduction);
   FLB200_AFTER_LAUNCH("cce_finalize");
   return FLB200_OK;
 }
@@ -450,13 +460,16 @@ int flb200_scores_cce_forward(const void* x, float* lse, const int32_t* targets,
   const int grid = grid_for(X, 1);
   switch (dtype) {
     case FLB200_F32:
-      row_lse_kernel<<<grid, kRowThreads, 0, st>>>(static_cast<const float*>(x), lse, C / 4, X);
+      launch_chained(row_lse_kernel<float>, grid, kRowThreads, 0, st, static_cast<const float*>(x), lse, C / 4,
+                     X);
       break;
     case FLB200_F16:
-      row_lse_kernel<<<grid, kRowThreads, 0, st>>>(static_cast<const __half*>(x), lse, C / 4, X);
+      launch_chained(row_lse_kernel<__half>, grid, kRowThreads, 0, st, static_cast<const __half*>(x), lse,
+                     C / 4, X);
       break;
     case FLB200_BF16:
-      row_lse_kernel<<<grid, kRowThreads, 0, st>>>(static_cast<const __nv_bfloat16*>(x), lse, C / 4, X);
+      launch_chained(row_lse_kernel<__nv_bfloat16>, grid, kRowThreads, 0, st,
+                     static_cast<const __nv_bfloat16*>(x), lse, C / 4, X);
       break;
     default:
       return fail(FLB200_UNSUPPORTED, "scores_cce_forward: unknown dtype %d", dtype);
@@ -503,18 +516,18 @@ int flb200_cce_backward(const float* grad_loss, const int32_t* targets, const in
   const int grid = grid_for(C * X, 256 * 4);
   switch (dtype) {
     case FLB200_F32:
-      cce_backward_kernel<float><<<grid, 256, 0, st>>>(grad_loss, targets, count,
+      launch_chained(cce_backward_kernel<float>, grid, 256, 0, st, grad_loss, targets, count,
                                                        static_cast<float*>(grad_logp), C, X,
                                                        reduction, ignore_index);
       break;
     case FLB200_F16:
-      cce_backward_kernel<__half><<<grid, 256, 0, st>>>(grad_loss, targets, count,
+      launch_chained(cce_backward_kernel<__half>, grid, 256, 0, st, grad_loss, targets, count,
                                                         static_cast<__half*>(grad_logp), C, X,
                                                         reduction, ignore_index);
       break;
     case FLB200_BF16:
-      cce_backward_kernel<__nv_bfloat16><<<grid, 256, 0, st>>>(
-          grad_loss, targets, count, static_cast<__nv_bfloat16*>(grad_logp), C, X, reduction,
+      launch_chained(cce_backward_kernel<__nv_bfloat16>, grid, 256, 0, st, grad_loss, targets, count,
+                     static_cast<__nv_bfloat16*>(grad_logp), C, X, reduction,
           ignore_index);
       break;
     default:
@@ -540,18 +553,18 @@ int flb200_log_softmax_cce_backward(const void* y, const float* grad_loss, const
   }
   switch (dtype) {
     case FLB200_F32:
-      lsm_cce_backward_kernel<float><<<grid, 256, 0, st>>>(
-          static_cast<const float*>(y), grad_loss, targets, count, static_cast<float*>(grad_x), C,
+      launch_chained(lsm_cce_backward_kernel<float>, grid, 256, 0, st, static_cast<const float*>(y), grad_loss,
+                     targets, count, static_cast<float*>(grad_x), C,
           X, reduction, ignore_index);
       break;
     case FLB200_F16:
-      lsm_cce_backward_kernel<__half><<<grid, 256, 0, st>>>(
-          static_cast<const __half*>(y), grad_loss, targets, count, static_cast<__half*>(grad_x),
+      launch_chained(lsm_cce_backward_kernel<__half>, grid, 256, 0, st, static_cast<const __half*>(y),
+                     grad_loss, targets, count, static_cast<__half*>(grad_x),
           C, X, reduction, ignore_index);
       break;
     case FLB200_BF16:
-      lsm_cce_backward_kernel<__nv_bfloat16><<<grid, 256, 0, st>>>(
-          static_cast<const __nv_bfloat16*>(y), grad_loss, targets, count,
+      launch_chained(lsm_cce_backward_kernel<__nv_bfloat16>, grid, 256, 0, st,
+                     static_cast<const __nv_bfloat16*>(y), grad_loss, targets, count,
           static_cast<__nv_bfloat16*>(grad_x), C, X, reduction, ignore_index);
       break;
     default:

@@ -40,6 +40,7 @@ inline long long up4(long long v) { return (v + 3) / 4 * 4; }
 __global__ void __launch_bounds__(256)
 im2col_kernel(const float* __restrict__ x, float* __restrict__ col, ConvGeo g, int hwp,
               long long ld) {
+  chain_begin();
   const int k = blockIdx.y;
   const int ci = k / g.RS, rs = k - ci * g.RS;
   const int r = rs / g.kW, s = rs - r * g.kW;
@@ -64,6 +65,7 @@ im2col_kernel(const float* __restrict__ x, float* __restrict__ col, ConvGeo g, i
 __global__ void __launch_bounds__(256)
 dgrad_gather_kernel(const float* __restrict__ gy, float* __restrict__ col, ConvGeo g, int hwp,
                     long long ld) {
+  chain_begin();
   const int k = blockIdx.y;
   const int co = k / g.RS, rs = k - co * g.RS;
   const int r = rs / g.kW, s = rs - r * g.kW;
@@ -89,6 +91,7 @@ dgrad_gather_kernel(const float* __restrict__ gy, float* __restrict__ col, ConvG
 __global__ void __launch_bounds__(256)
 planes_to_rows_kernel(const float* __restrict__ src, float* __restrict__ dst, int channels,
                       int hw_count, int hwp, long long ld) {
+  chain_begin();
   const int c = blockIdx.y;
   float* out = dst + (long long)c * ld;
   for (long long t = (long long)blockIdx.x * blockDim.x + threadIdx.x; t < ld;
@@ -101,6 +104,7 @@ planes_to_rows_kernel(const float* __restrict__ src, float* __restrict__ dst, in
 // wp[co][kp] = w[co][k] for k < kc: same values, row stride padded to a multiple of 4.
 __global__ void pad_rows_kernel(const float* __restrict__ w, float* __restrict__ wp, int rows,
                                 int kc, int kp) {
+  chain_begin();
   const long long total = (long long)rows * kp;
   for (long long t = (long long)blockIdx.x * blockDim.x + threadIdx.x; t < total;
        t += (long long)gridDim.x * blockDim.x) {
@@ -112,6 +116,7 @@ __global__ void pad_rows_kernel(const float* __restrict__ w, float* __restrict__
 // wt[ci][(co, rs)] = w[co][ci][rs], row stride k2p.
 __global__ void transpose_filter_kernel(const float* __restrict__ w, float* __restrict__ wt,
                                         ConvGeo g, int k2p) {
+  chain_begin();
   const long long total = (long long)g.C * k2p;
   const int k2 = g.Cout * g.RS;
   for (long long t = (long long)blockIdx.x * blockDim.x + threadIdx.x; t < total;
@@ -318,11 +323,11 @@ int tc_conv_forward(const ConvGeo& g, const float* x, const float* w, const floa
   size_t off = up256((size_t)s.kc * s.ld_out * 4);
   float* wp = reinterpret_cast<float*>(base + off);
   off += up256((size_t)g.Cout * s.kp * 4);
-  im2col_kernel<<<gather_grid(s.ld_out, s.kc), 256, 0, st>>>(x, col, g, s.hwp_out, s.ld_out);
+  launch_chained(im2col_kernel, gather_grid(s.ld_out, s.kc), 256, 0, st, x, col, g, s.hwp_out, s.ld_out);
   FLB200_AFTER_LAUNCH("im2col");
   const float* wsrc = w;
   if (s.kp != s.kc) {
-    pad_rows_kernel<<<grid_for((long long)g.Cout * s.kp, 256), 256, 0, st>>>(w, wp, g.Cout, s.kc,
+    launch_chained(pad_rows_kernel, grid_for((long long)g.Cout * s.kp, 256), 256, 0, st, w, wp, g.Cout, s.kc,
                                                                             s.kp);
     FLB200_AFTER_LAUNCH("pad_filter_rows");
     wsrc = wp;
@@ -396,9 +401,9 @@ int tc_conv_backward_data(const ConvGeo& g, const float* gy, const float* w, flo
   size_t off = up256((size_t)s.k2 * s.ld_in * 4);
   float* wt = reinterpret_cast<float*>(base + off);
   off += up256((size_t)g.C * s.k2p * 4);
-  dgrad_gather_kernel<<<gather_grid(s.ld_in, s.k2), 256, 0, st>>>(gy, col, g, s.hwp_in, s.ld_in);
+  launch_chained(dgrad_gather_kernel, gather_grid(s.ld_in, s.k2), 256, 0, st, gy, col, g, s.hwp_in, s.ld_in);
   FLB200_AFTER_LAUNCH("dgrad_gather");
-  transpose_filter_kernel<<<grid_for((long long)g.C * s.k2p, 256), 256, 0, st>>>(w, wt, g, s.k2p);
+  launch_chained(transpose_filter_kernel, grid_for((long long)g.C * s.k2p, 256), 256, 0, st, w, wt, g, s.k2p);
   FLB200_AFTER_LAUNCH("transpose_filter");
   if (int rc = map2d(&ma, col, s.ld_in, s.k2, s.ld_in, 32, true)) return rc;
   const long long k_iters = (s.k2 + tc::kBK - 1) / tc::kBK;
@@ -445,9 +450,9 @@ int tc_conv_backward_filter(const ConvGeo& g, const float* gy, const float* x, f
   size_t off = up256((size_t)s.kc * s.ld_out * 4);
   float* dyt = reinterpret_cast<float*>(base + off);
   off += up256((size_t)g.Cout * s.ld_out * 4);
-  im2col_kernel<<<gather_grid(s.ld_out, s.kc), 256, 0, st>>>(x, col, g, s.hwp_out, s.ld_out);
+  launch_chained(im2col_kernel, gather_grid(s.ld_out, s.kc), 256, 0, st, x, col, g, s.hwp_out, s.ld_out);
   FLB200_AFTER_LAUNCH("im2col");
-  planes_to_rows_kernel<<<gather_grid(s.ld_out, g.Cout), 256, 0, st>>>(gy, dyt, g.Cout, g.HoWo,
+  launch_chained(planes_to_rows_kernel, gather_grid(s.ld_out, g.Cout), 256, 0, st, gy, dyt, g.Cout, g.HoWo,
                                                                       s.hwp_out, s.ld_out);
   FLB200_AFTER_LAUNCH("planes_to_rows");
   if (int rc = map2d(&ma, dyt, s.ld_out, g.Cout, s.ld_out, tc::kBM, false)) return rc;

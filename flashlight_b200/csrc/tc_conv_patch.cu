@@ -37,6 +37,7 @@ ClSlot cl_slot(flb200_conv2d_cache* c, int which, size_t bytes, float* fallback)
 __global__ void __launch_bounds__(256)
 nchw_to_nhwc_kernel(const float* __restrict__ src, float* __restrict__ dst, int C, int cp,
                     int HW) {
+  chain_begin();
   __shared__ float tile[32][33];
   const int tx = threadIdx.x & 31, ty = threadIdx.x >> 5;
   const int hw0 = blockIdx.x * 32, c0 = blockIdx.y * 32;
@@ -59,6 +60,7 @@ nchw_to_nhwc_kernel(const float* __restrict__ src, float* __restrict__ dst, int 
 __global__ void __launch_bounds__(256)
 nchw_to_nhwc_vec_kernel(const float* __restrict__ src, float* __restrict__ dst, int C, int cp,
                         int HW) {
+  chain_begin();
   __shared__ float tile[64][65];
   const int hw0 = blockIdx.x * 64, c0 = blockIdx.y * 64;
   const long long n = blockIdx.z;
@@ -89,13 +91,13 @@ int to_nhwc(const float* src, float* dst, int N, int C, int cp, int HW, cudaStre
   if ((HW & 3) == 0 && (cp & 3) == 0 && ((reinterpret_cast<uintptr_t>(src) | reinterpret_cast<uintptr_t>(dst)) & 15) == 0) {
     dim3 vgrid((unsigned)((HW + 63) / 64), (unsigned)((cp + 63) / 64), (unsigned)N);
     FLB200_REQUIRE(vgrid.y <= 65535 && vgrid.z <= 65535, "nchw_to_nhwc: extent out of range");
-    nchw_to_nhwc_vec_kernel<<<vgrid, 256, 0, st>>>(src, dst, C, cp, HW);
+    launch_chained(nchw_to_nhwc_vec_kernel, vgrid, 256, 0, st, src, dst, C, cp, HW);
     FLB200_AFTER_LAUNCH("nchw_to_nhwc_vec");
     return FLB200_OK;
   }
   dim3 grid((unsigned)((HW + 31) / 32), (unsigned)((cp + 31) / 32), (unsigned)N);
   FLB200_REQUIRE(grid.y <= 65535 && grid.z <= 65535, "nchw_to_nhwc: extent out of range");
-  nchw_to_nhwc_kernel<<<grid, 256, 0, st>>>(src, dst, C, cp, HW);
+  launch_chained(nchw_to_nhwc_kernel, grid, 256, 0, st, src, dst, C, cp, HW);
   FLB200_AFTER_LAUNCH("nchw_to_nhwc");
   return FLB200_OK;
 }
@@ -104,6 +106,7 @@ int to_nhwc(const float* src, float* dst, int N, int C, int cp, int HW, cudaStre
 __global__ void __launch_bounds__(256)
 nchw_to_nhwc_sampled_kernel(const float* __restrict__ src, float* __restrict__ dst, int C, int cp,
                             int HW, int W, int Wo, int HoWo, int sx, int sy) {
+  chain_begin();
   __shared__ float tile[32][33];
   const int tx = threadIdx.x & 31, ty = threadIdx.x >> 5;
   const int hw0 = blockIdx.x * 32, c0 = blockIdx.y * 32;
@@ -158,7 +161,7 @@ int x_to_nhwc(const ConvGeo& g, const float* x, float* xt, int cp, cudaStream_t 
   if (!samples_input(g)) return to_nhwc(x, xt, g.N, g.C, cp, g.HW, st);
   dim3 grid((unsigned)((g.HoWo + 31) / 32), (unsigned)((cp + 31) / 32), (unsigned)g.N);
   FLB200_REQUIRE(grid.y <= 65535 && grid.z <= 65535, "nchw_to_nhwc: extent out of range");
-  nchw_to_nhwc_sampled_kernel<<<grid, 256, 0, st>>>(x, xt, g.C, cp, g.HW, g.W, g.Wo, g.HoWo, g.sx,
+  launch_chained(nchw_to_nhwc_sampled_kernel, grid, 256, 0, st, x, xt, g.C, cp, g.HW, g.W, g.Wo, g.HoWo, g.sx,
                                                    g.sy);
   FLB200_AFTER_LAUNCH("nchw_to_nhwc_sampled");
   return FLB200_OK;
@@ -181,6 +184,7 @@ int pack_filter(const ConvGeo& g, const float* w, float* out, int kp, bool rows_
 template <typename T>
 __global__ void wgrad_reduce_kernel(const float* __restrict__ partial, T* __restrict__ gw,
                                     int Cout, int C, int RS, int splits) {
+  chain_begin();
   const long long per_split = (long long)RS * Cout * C;
   for (long long t = (long long)blockIdx.x * blockDim.x + threadIdx.x; t < per_split;
        t += (long long)gridDim.x * blockDim.x) {
@@ -198,6 +202,7 @@ __global__ void wgrad_reduce_kernel(const float* __restrict__ partial, T* __rest
 template <typename T>
 __global__ void __launch_bounds__(256)
 wgrad_reduce_flat_kernel(const float4* __restrict__ partial, T* __restrict__ gw, long long n4, int splits) {
+  chain_begin();
   for (long long t = (long long)blockIdx.x * blockDim.x + threadIdx.x; t < n4;
        t += (long long)gridDim.x * blockDim.x) {
     float4 s = make_float4(0.f, 0.f, 0.f, 0.f);
@@ -216,6 +221,7 @@ template <typename T>
 __global__ void __launch_bounds__(256)
 wgrad_reduce_vec_kernel(const float4* __restrict__ partial, T* __restrict__ gw, int Cout, int C4,
                         int RS, int splits) {
+  chain_begin();
   extern __shared__ float red_tile[];  // [tap][32 channels + 1]
   const int q0 = blockIdx.x * 8, co = blockIdx.y;
   const int nq = min(8, C4 - q0);
@@ -245,14 +251,13 @@ int wgrad_reduce(const float* partial, T* gw, const ConvGeo& g, int splits, cuda
   const float4* p4 = reinterpret_cast<const float4*>(partial);
   const long long n4 = (long long)g.Cout * g.C / 4;
   if (vec && g.RS == 1 && (reinterpret_cast<uintptr_t>(gw) & (4 * sizeof(T) - 1)) == 0)
-    wgrad_reduce_flat_kernel<T><<<grid_for(n4, 256), 256, 0, st>>>(p4, gw, n4, splits);
+    launch_chained(wgrad_reduce_flat_kernel<T>, grid_for(n4, 256), 256, 0, st, p4, gw, n4, splits);
   else if (vec && g.Cout <= 65535 && smem <= 48 * 1024)
-    wgrad_reduce_vec_kernel<T><<<dim3((unsigned)((g.C / 4 + 7) / 8), (unsigned)g.Cout),
-                                 std::min(256, (g.RS * 8 + 31) / 32 * 32), smem, st>>>(
-        p4, gw, g.Cout, g.C / 4, g.RS, splits);
+    launch_chained(wgrad_reduce_vec_kernel<T>, dim3((unsigned)((g.C / 4 + 7) / 8), (unsigned)g.Cout),
+                   std::min(256, (g.RS * 8 + 31) / 32 * 32), smem, st, p4, gw, g.Cout, g.C / 4, g.RS, splits);
   else
-    wgrad_reduce_kernel<T><<<grid_for((long long)g.RS * g.Cout * g.C, 256), 256, 0, st>>>(
-        partial, gw, g.Cout, g.C, g.RS, splits);
+    launch_chained(wgrad_reduce_kernel<T>, grid_for((long long)g.RS * g.Cout * g.C, 256), 256, 0, st, partial,
+                   gw, g.Cout, g.C, g.RS, splits);
   FLB200_AFTER_LAUNCH("wgrad_reduce");
   return FLB200_OK;
 }
@@ -523,6 +528,7 @@ constexpr int kWinPixels = 8;  // 32 floats / 4 channels
 __global__ void __launch_bounds__(256)
 nchw_to_nhwc4_pad_kernel(const float* __restrict__ x, float4* __restrict__ dst, int N, int C, int H,
                          int W, int Hp, int Wp, int py, int px, long long total) {
+  chain_begin();
   for (long long t = (long long)blockIdx.x * blockDim.x + threadIdx.x; t < total;
        t += (long long)gridDim.x * blockDim.x) {
     const int wp = (int)(t % Wp);
@@ -541,6 +547,7 @@ nchw_to_nhwc4_pad_kernel(const float* __restrict__ x, float4* __restrict__ dst, 
 // wr[r][co][s*4 + c] = w[co][c][r][s], zero elsewhere (32 floats per row).
 __global__ void pack_filter_rows_kernel(const float* __restrict__ w, float* __restrict__ wr,
                                         int Cout, int C, int kH, int kW) {
+  chain_begin();
   const int total = kH * Cout * 32;
   for (int t = blockIdx.x * blockDim.x + threadIdx.x; t < total; t += gridDim.x * blockDim.x) {
     const int j = t & 31, co = (t >> 5) % Cout, r = (t >> 5) / Cout;
@@ -553,6 +560,7 @@ __global__ void pack_filter_rows_kernel(const float* __restrict__ w, float* __re
 __global__ void window_wgrad_reduce_kernel(const float* __restrict__ partial,
                                            float* __restrict__ gw, int Cout, int C, int kH, int kW,
                                            int splits) {
+  chain_begin();
   const int total = Cout * C * kH * kW;
   const long long per_split = (long long)kH * Cout * 32;
   for (int t = blockIdx.x * blockDim.x + threadIdx.x; t < total; t += gridDim.x * blockDim.x) {
@@ -911,12 +919,12 @@ int window_conv_forward(const ConvGeo& g, const float* x, const float* w, const 
   if (int rc = filter_map(&mb, wr, g.operand, 32, 32, g.Cout, g.kH, filter_box_rows(bn))) return rc;
   if (!xs.valid) {
     const long long total = window_pixels(g, wg);
-    nchw_to_nhwc4_pad_kernel<<<grid_for(total, 256), 256, 0, st>>>(
-        x, reinterpret_cast<float4*>(xtp), g.N, g.C, g.H, g.W, wg.Hp, wg.Wp, g.py, g.px, total);
+    launch_chained(nchw_to_nhwc4_pad_kernel, grid_for(total, 256), 256, 0, st, x,
+                   reinterpret_cast<float4*>(xtp), g.N, g.C, g.H, g.W, wg.Hp, wg.Wp, g.py, g.px, total);
     FLB200_AFTER_LAUNCH("nchw_to_nhwc4_pad");
     if (xs.flag) *xs.flag = 1;
   }
-  pack_filter_rows_kernel<<<grid_for(g.kH * g.Cout * 32, 256), 256, 0, st>>>(w, wr, g.Cout, g.C,
+  launch_chained(pack_filter_rows_kernel, grid_for(g.kH * g.Cout * 32, 256), 256, 0, st, w, wr, g.Cout, g.C,
                                                                             g.kH, g.kW);
   FLB200_AFTER_LAUNCH("pack_filter_rows");
   a.pix_w = g.Wo; a.pix_h = g.Ho; a.images = g.N; a.n_out = g.Cout;
@@ -961,8 +969,8 @@ int window_conv_backward_filter(const ConvGeo& g, const float* gy, const float* 
     return rc;
   if (!xs.valid) {
     const long long total = window_pixels(g, wg);
-    nchw_to_nhwc4_pad_kernel<<<grid_for(total, 256), 256, 0, st>>>(
-        x, reinterpret_cast<float4*>(xtp), g.N, g.C, g.H, g.W, wg.Hp, wg.Wp, g.py, g.px, total);
+    launch_chained(nchw_to_nhwc4_pad_kernel, grid_for(total, 256), 256, 0, st, x,
+                   reinterpret_cast<float4*>(xtp), g.N, g.C, g.H, g.W, wg.Hp, wg.Wp, g.py, g.px, total);
     FLB200_AFTER_LAUNCH("nchw_to_nhwc4_pad");
     if (xs.flag) *xs.flag = 1;
   }
@@ -972,8 +980,8 @@ int window_conv_backward_filter(const ConvGeo& g, const float* gy, const float* 
   // the channel groups of the view, so the launch has a single tap at offset zero.
   const WgradTaps tp{32 * g.kH, 1, 1, 1, 1, 0, 0};
   if (int rc = run_wgrad_any(ma, mb, a_each, 0, g, tp, wp, partial, st)) return rc;
-  window_wgrad_reduce_kernel<<<grid_for((long long)g.Cout * g.C * g.RS, 256), 256, 0, st>>>(
-      partial, gw, g.Cout, g.C, g.kH, g.kW, wp.splits);
+  launch_chained(window_wgrad_reduce_kernel, grid_for((long long)g.Cout * g.C * g.RS, 256), 256, 0, st, partial,
+                 gw, g.Cout, g.C, g.kH, g.kW, wp.splits);
   FLB200_AFTER_LAUNCH("window_wgrad_reduce");
   return FLB200_OK;
 }

@@ -130,6 +130,7 @@ int* status_ptr() {
 static __global__ void __launch_bounds__(256)
 tc_splitk_reduce_kernel(const float* __restrict__ partial, EpiloguePlan ep, int M, int N, int Z,
                         int splits) {
+  chain_begin();
   const long long mn = (long long)M * N;
   const long long total = mn * Z;
   const long long stride = (long long)gridDim.x * blockDim.x;
@@ -168,6 +169,7 @@ template <typename T, int G>
 static __global__ void __launch_bounds__(256)
 tc_splitk_reduce_vec_kernel(const float4* __restrict__ partial, EpiloguePlan ep, int M, int N4,
                             int Z, int splits) {
+  chain_begin();
   constexpr int kItems = 256 / G;
   __shared__ float4 shared_sum[G > 1 ? 256 : 1];
   const int item = threadIdx.x % kItems, g = threadIdx.x / kItems;
@@ -224,9 +226,11 @@ static void launch_reduce_vec(const float4* partial, const EpiloguePlan& ep, lon
                               int splits, cudaStream_t st) {
   const long long total = M * N4 * Z;
   if (splits >= 16 && total < 148 * 256)
-    tc_splitk_reduce_vec_kernel<T, 8><<<grid_for(total, 32), 256, 0, st>>>(partial, ep, (int)M, (int)N4, (int)Z, splits);
+    launch_chained(tc_splitk_reduce_vec_kernel<T, 8>, grid_for(total, 32), 256, 0, st, partial, ep, (int)M,
+                   (int)N4, (int)Z, splits);
   else
-    tc_splitk_reduce_vec_kernel<T, 1><<<grid_for(total, 256), 256, 0, st>>>(partial, ep, (int)M, (int)N4, (int)Z, splits);
+    launch_chained(tc_splitk_reduce_vec_kernel<T, 1>, grid_for(total, 256), 256, 0, st, partial, ep, (int)M,
+                   (int)N4, (int)Z, splits);
 }
 
 static long long env_ll(const char* name, long long dflt) {
@@ -421,7 +425,7 @@ int run(const CUtensorMap& ma, const CUtensorMap& mb, const OperandPlan& pa, con
       else launch_reduce_vec<float>(p4, ep, M, N / 4, Z, L.splits, st);
     } else {
       const int rgrid = grid_for(M * N * Z, 256);
-      tc_splitk_reduce_kernel<<<rgrid, 256, 0, st>>>(partial, ep, (int)M, (int)N, (int)Z,
+      launch_chained(tc_splitk_reduce_kernel, rgrid, 256, 0, st, partial, ep, (int)M, (int)N, (int)Z,
                                                      L.splits);
     }
     FLB200_AFTER_LAUNCH("tc_splitk_reduce");

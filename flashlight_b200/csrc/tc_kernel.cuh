@@ -196,6 +196,7 @@ template <class P, int BN, int STAGES, int X3 = 0, int KSUB = 1>
 __global__ void __launch_bounds__(threads_for<P, X3, BN>(), P::kMinBlocks)
 tc_persistent_kernel(const __grid_constant__ CUtensorMap map_a,
                      const __grid_constant__ CUtensorMap map_b, const P prob, int* status) {
+  chain_begin();
   using SL = SmemLayout<BN, STAGES, X3>;
   // The ring's STAGES sub-stages (one 128-byte-wide K block of both operands each) are handed
   // over in groups of KSUB: one pair of barriers, one wait and one commit per group.  A
@@ -823,8 +824,8 @@ int launch_problem_as(const char* name, const CUtensorMap& ma, const CUtensorMap
   }
   const long long sms = device_info().sm_count;
   const unsigned grid = (unsigned)(tiles < sms ? tiles : sms);
-  tc_persistent_kernel<P, BN, STAGES, X3, KSUB><<<grid, threads_for<P, X3, BN>(), SL::kTotal, st>>>(
-      ma, mb, prob, status_ptr());
+  launch_chained(tc_persistent_kernel<P, BN, STAGES, X3, KSUB>, grid, threads_for<P, X3, BN>(), SL::kTotal, st,
+                 ma, mb, prob, status_ptr());
   FLB200_AFTER_LAUNCH(name);
   count_tc_launch();
 #ifdef FLB200_TC_PROFILE

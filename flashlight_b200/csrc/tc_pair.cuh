@@ -59,6 +59,7 @@ template <class P, int BN, int STAGES, int KSUB = 2>
 __global__ void __launch_bounds__(pair_threads_for<P>(), 1)
 tc_pair_kernel(const __grid_constant__ CUtensorMap map_a,
                const __grid_constant__ CUtensorMap map_b, const P prob, int* status) {
+  chain_begin();
   using SL = PairSmemLayout<BN, STAGES>;
   static_assert(BN >= 64 && BN % 64 == 0, "each CTA holds BN/2 columns in 32-column boxes");
   // the ring's sub-stages change hands in groups of KSUB (see tc_kernel.cuh)
@@ -307,13 +308,15 @@ int launch_pair_problem(const char* name, const CUtensorMap& ma, const CUtensorM
   cfg.blockDim = dim3(pair_threads_for<P>());
   cfg.dynamicSmemBytes = SL::kTotal;
   cfg.stream = st;
-  cudaLaunchAttribute attr[1];
+  cudaLaunchAttribute attr[2];
   attr[0].id = cudaLaunchAttributeClusterDimension;
   attr[0].val.clusterDim.x = 2;
   attr[0].val.clusterDim.y = 1;
   attr[0].val.clusterDim.z = 1;
+  attr[1].id = cudaLaunchAttributeProgrammaticStreamSerialization;  // (launch_chained)
+  attr[1].val.programmaticStreamSerializationAllowed = 1;
   cfg.attrs = attr;
-  cfg.numAttrs = 1;
+  cfg.numAttrs = 2;
   FLB200_CUDA_CHECK(cudaLaunchKernelEx(&cfg, tc_pair_kernel<P, BN, STAGES, KSUB>, ma, mb, prob,
                                        status_ptr()));
   FLB200_AFTER_LAUNCH(name);
