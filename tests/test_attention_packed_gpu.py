@@ -53,6 +53,22 @@ def test_attention_packed_infinite_scores(causal):
     assert_close_scaled(lse.reshape(B, h, T)[:, :, first:], torch.logsumexp(s, -1)[:, :, first:], 1e-3, "attention lse")
 
 
+def test_attention_packed_large_scores():
+    """The softmax of a single key is 1 and its lse the score, whatever the score: 0.125 * 64 * 110 * 111 = 97680,
+    exact in every step, and nothing between the score and its exponential may round by the score's size."""
+    from flashlight_b200 import functions as F
+    B, T, h = 3, 1, 2
+    qkv = randn(B, 3, h, 64, seed=4).bfloat16()
+    qkv[:, 0], qkv[:, 1] = 110.0, 111.0
+    qkv = qkv.reshape(B, 3 * h * 64).cuda()
+    go = randn(B, h * 64, seed=5).bfloat16().cuda()
+    out, lse = F.attention_packed(qkv, B, T, h, 0.125, True)
+    g = F.attention_packed_backward(qkv, out, go, lse, B, T, h, 0.125, True)
+    assert torch.equal(lse, torch.full_like(lse, 97680.0))
+    assert torch.equal(out, qkv.reshape(B, 3, h * 64)[:, 2])
+    assert torch.equal(g.reshape(B, 3, h * 64)[:, 2], go)
+
+
 def test_attention_packed_declines_what_it_is_not_built_for():
     from flashlight_b200 import functions as F
     assert F.attention_packed(randn(8, 96, seed=1).bfloat16().cuda(), 1, 8, 1, 1.0, True) is None
