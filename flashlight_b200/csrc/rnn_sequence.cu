@@ -1,5 +1,5 @@
 // The recurrence of a layer as one persistent kernel: all T steps, with the recurrent weights
-// resident in shared memory, and both directions (or several parts of a large batch) side by side
+// resident in tensor memory and shared memory, and both directions (or several parts of a large batch) side by side
 // as jobs of one launch where the device holds them.
 //
 // What bounds a step is latency: between two steps every unit's new state has to reach all CTAs.
@@ -10,9 +10,9 @@
 // step s + 2 once everybody has consumed step s, which the data dependence itself ensures (each state
 // needs all states of the step before).
 //
-// Both directions of a 1024-unit LSTM are 32 MB of weights, as much as the shared memory of all SMs; half
-// of it lies in tensor memory instead, as the A operand of the MMAs, which is also the faster place to read
-// it from.  So they run side by side: 32 rows of the batch take 4.4 us per step forward and 5.1 backward,
+// Both directions of a 1024-unit LSTM are 32 MB of weights, as much as the shared memory of all SMs; of a CTA's
+// 16 k tiles 8 (forward) or 12 (backward) lie in tensor memory instead, beside the accumulators, as the A
+// operand of the MMAs, which is also the faster place to read them from.  So they run side by side: 32 rows of the batch take 4.4 us per step forward and 5.1 backward,
 // where one direction after the other took 2 x 3.9 and 2 x 6.6 (weights in shared memory only, words
 // fetched by the threads that polled them, the backward pass with a second exchange through L2 for its
 // partial sums).  Of a backward step of 9600 clocks about 1000 are the cell gradient, 1700 until its words
@@ -46,7 +46,7 @@ constexpr int kABytes = kBM * kBK * 4;      // 16 KB: one 32-wide k tile of the 
 constexpr int kWorkers = 8;                 // warps that bring tiles, move sums and update states
 constexpr int kWorkThreads = 32 * kWorkers;
 constexpr int kMaxTiles = 2 * kWorkers;     // k tiles a CTA keeps at most
-constexpr int kIssuers = kRnnAccs;          // warps that only issue MMAs, an accumulator each
+constexpr int kIssuers = 2;                 // warps that only issue MMAs, of every other k tile
 constexpr int kSeqThreads = kWorkThreads + 32 * kIssuers;
 constexpr int kTmemColumns = 512;
 constexpr uint32_t kTagMask = 0x1fff;       // bits of an fp32 word that a TF32 operand ignores
@@ -267,14 +267,16 @@ __device__ __forceinline__ void tmem_st8(uint32_t addr, const float* v) {
                "r"(__float_as_uint(v[6])), "r"(__float_as_uint(v[7]))
                : "memory");
 }
-// All MMAs of one step, by one lane of an issuing warp: of every kIssuers-th tile as it becomes whole.
+// All MMAs of one step, by one lane of an issuing warp: of every kIssuers-th tile as it becomes whole, tile s
+// into accumulator s % accs (a power of two, at least kIssuers).
 template <bool kAMajorMn, int N>
-__device__ __forceinline__ bool issue_step(uint32_t d, uint64_t a_desc0, uint32_t a_tmem, int in_smem,
+__device__ __forceinline__ bool issue_step(uint32_t d, uint32_t acc_stride, int accs, uint64_t a_desc0, uint32_t a_tmem, int in_smem,
                                            uint64_t b_desc0, int first, int stages, uint32_t parity,
                                            uint64_t* full_bar, uint64_t* done_bar, const Waits& w) {
   for (int s = first; s < stages; s += kIssuers) {
     if (!w.bar<false>(&full_bar[s], parity)) return false;
-    issue_tile<kAMajorMn, N>(d, a_desc0, a_tmem, in_smem, b_desc0, s, s == first);
+    issue_tile<kAMajorMn, N>(d + (uint32_t)(s & (accs - 1)) * acc_stride, a_desc0, a_tmem, in_smem, b_desc0, s,
+                             s < accs);
   }
   umma_commit(done_bar);
   return true;
@@ -301,21 +303,28 @@ __device__ __forceinline__ void tmem_ld_async(uint32_t addr, uint32_t* r) {
         : "r"(addr)
         : "memory");
 }
-// N columns of this warp's rows: `accs` accumulators kStride columns apart, loaded together, added in order
-template <int kAccs, uint32_t kStride, int N>
+// N columns of this warp's rows: `accs` accumulators kStride columns apart, added in order.  Four are loaded
+// together: eight take registers that the states of the batch need.
+template <uint32_t kStride, int N>
 __device__ __forceinline__ void read_sums(uint32_t at, int accs, float* v) {
-  uint32_t r[kAccs][N];
+  constexpr int kTogether = 4;
 #pragma unroll
-  for (int q = 0; q < kAccs; ++q)
-    if (q < accs) tmem_ld_async<N>(at + q * kStride, r[q]);
-  asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
+  for (int q0 = 0; q0 < kRnnAccs; q0 += kTogether) {
+    if (q0 >= accs) break;
+    uint32_t r[kTogether][N];
 #pragma unroll
-  for (int q = 0; q < kAccs; ++q) {
+    for (int q = 0; q < kTogether; ++q)
+      if (q0 + q < accs) tmem_ld_async<N>(at + (q0 + q) * kStride, r[q]);
+    asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
 #pragma unroll
-    for (int j = 0; j < N; ++j) asm volatile("" : "+r"(r[q][j]));  // read only after the wait
-    if (q < accs) {
+    for (int q = 0; q < kTogether; ++q) {
 #pragma unroll
-      for (int j = 0; j < N; ++j) v[j] = q == 0 ? __uint_as_float(r[0][j]) : v[j] + __uint_as_float(r[q][j]);
+      for (int j = 0; j < N; ++j) asm volatile("" : "+r"(r[q][j]));  // read only after the wait
+      if (q0 + q < accs) {
+#pragma unroll
+        for (int j = 0; j < N; ++j)
+          v[j] = q0 + q == 0 ? __uint_as_float(r[0][j]) : v[j] + __uint_as_float(r[q][j]);
+      }
     }
   }
 }
@@ -333,6 +342,7 @@ struct Launch {
   int slice;    // states / gate rows of a CTA's k slice
   int stages;   // k tiles of a CTA, of 32 states or of P x 32 gate rows
   int in_smem;  // those whose weights are in shared memory; the others' are in tensor memory
+  int accs;     // accumulators, of every accs-th k tile each
   int ctas;     // of one job
   int absent_cta;
 };
@@ -356,7 +366,7 @@ inline size_t seq_smem(int in_smem, int stages, int cols, int recv) {
 // A cluster owns 32 hidden units, all gates of them = up to 128 rows of one UMMA tile (gate-major;
 // the rows of absent gates are zeros); its KS CTAs split K = H into slices of at most 256, or 512 with the
 // weights of half the tiles in tensor memory.  Worker s brings the 32 states of k tile s (and of s + 8), two
-// warps issue the MMAs (M = 128, N = batch), each of every other tile into its own accumulator, the
+// warps issue the MMAs (M = 128, N = batch), each of every other tile; tiles s and s + 8 share an accumulator.  The
 // workers push the partial sums of each unit from tensor memory straight into the shared memory of the CTA
 // that updates it (st.async: one trip, no cluster barrier), and every thread updates the same (unit,
 // batch) pairs in all steps, with the cell state in a register.  What a step leaves for the backward pass is
@@ -410,7 +420,7 @@ rnn_sequence_kernel(const __grid_constant__ Launch<SeqJob> a) {
   tc_fence_before();
   __syncthreads();
   tc_fence_after();
-  const uint32_t tmem_base = *tmem_slot, a_tmem = tmem_base + kIssuers * kAccStride;
+  const uint32_t tmem_base = *tmem_slot, a_tmem = tmem_base + a.accs * kAccStride;
 
   if (warp == 0) {  // the resident slice of W_hh
     if (lane == 0) mbar_expect_tx(w_bar, in_smem * G * (32 * 128));
@@ -471,7 +481,7 @@ rnn_sequence_kernel(const __grid_constant__ Launch<SeqJob> a) {
       const uint64_t a_desc0 = umma_desc(smem_u32(a_tiles), 16, 1024, 2);
       const uint64_t b_desc0 = umma_desc(smem_u32(b_tiles), 16, 1024, 2);
       for (int step = 0; step < a.T; ++step)
-        if (!issue_step<false, NB>(tmem_base + q * kAccStride, a_desc0, a_tmem, in_smem, b_desc0, q, stages,
+        if (!issue_step<false, NB>(tmem_base, kAccStride, a.accs, a_desc0, a_tmem, in_smem, b_desc0, q, stages,
                                    step & 1, full_bar, done_bar, waits))
           break;
     }
@@ -556,7 +566,8 @@ rnn_sequence_kernel(const __grid_constant__ Launch<SeqJob> a) {
         for (int i = 0; i < kHalf; i += kChunk) {
           const int c0 = (warp >> 2) * kHalf + i;  // warps w and w + 4 share the rows of tensor memory
           float v[kChunk];
-          read_sums<kIssuers, kAccStride, kChunk>(tmem_base + ((uint32_t)((warp & 3) * 32) << 16) + c0, stages, v);
+          read_sums<kAccStride, kChunk>(tmem_base + ((uint32_t)((warp & 3) * 32) << 16) + c0,
+                                                  min(stages, a.accs), v);
 #pragma unroll
           for (int j = 0; j < kChunk / 4; ++j)
             if (c0 / 4 + j < quads)
@@ -577,7 +588,7 @@ rnn_sequence_kernel(const __grid_constant__ Launch<SeqJob> a) {
 #pragma unroll
         for (int g = 0; g < G; ++g) pre[g] = 0.f;
 #pragma unroll
-        for (int q = 0; q < KS; ++q)  // same order as lstm_step_kernel: bit-identical sums
+        for (int q = 0; q < KS; ++q)  // slices of 256: the order of lstm_step_kernel, the same bits
 #pragma unroll
           for (int g = 0; g < G; ++g) pre[g] += rp[(((q * G + g) * (NB / 4) + (b >> 2)) * kOwn + u) * 4 + (b & 3)];
         float h;
@@ -700,7 +711,7 @@ rnn_sequence_backward_kernel(const __grid_constant__ Launch<SeqBwdJob> a) {
   // this warp's rows of the accumulator, and of the tiles in tensor memory: a part, 32 outputs of it
   const int part = (warp & 3) * 32 / kOut;
   const uint32_t lanes = (uint32_t)((warp & 3) * 32) << 16;
-  const uint32_t a_tmem = tmem_base + kIssuers * kAccStride;
+  const uint32_t a_tmem = tmem_base + a.accs * kAccStride;
   if (warp < kWorkers) {
     const int j = group * kOut + (warp & 3) * 32 % kOut + lane;
     for (int s = in_smem + (warp >> 2); s < stages; s += 2) {
@@ -727,7 +738,7 @@ rnn_sequence_backward_kernel(const __grid_constant__ Launch<SeqBwdJob> a) {
       const uint64_t a_desc0 = umma_desc(smem_u32(a_tiles), kBK * 128, 512, 1);
       const uint64_t b_desc0 = umma_desc(smem_u32(b_tiles), 16, 1024, 2);
       for (int sb = 0; sb < a.T; ++sb)
-        if (!issue_step<true, kCols>(tmem_base + q * kAccStride, a_desc0, a_tmem, in_smem, b_desc0, q, stages,
+        if (!issue_step<true, kCols>(tmem_base, kAccStride, a.accs, a_desc0, a_tmem, in_smem, b_desc0, q, stages,
                                      sb & 1, full_bar, done_bar, waits))
           break;
     }
@@ -851,7 +862,7 @@ rnn_sequence_backward_kernel(const __grid_constant__ Launch<SeqBwdJob> a) {
         for (int i = 0; i < kHalf; i += kChunk) {
           const int c0 = (warp >> 2) * kHalf + i;  // warps w and w + 4 share the rows of tensor memory
           float v[kChunk];
-          read_sums<kIssuers, kAccStride, kChunk>(tmem_base + lanes + part * NB + c0, stages, v);
+          read_sums<kAccStride, kChunk>(tmem_base + lanes + part * NB + c0, min(stages, a.accs), v);
 #pragma unroll
           for (int j = 0; j < kChunk / 4; ++j)
             if (c0 / 4 + j < quads)
@@ -901,7 +912,7 @@ typedef void (*BwdKernel)(const Launch<SeqBwdJob>);
 // One way to run a job: `rows` of the batch, a cluster of CTAs per group of units or outputs.
 struct Plan {
   int rows;  // of the batch per job; 0: not possible
-  int nb, cluster, slice, stages, in_smem, ctas;
+  int nb, cluster, slice, stages, in_smem, accs, ctas;
   size_t smem;
   const void* kernel;
 };
@@ -912,11 +923,21 @@ void set_rows(Plan* p, int B, int nb) {
 }
 bool wants_48(int B) { return B > 32 && B <= 48; }  // where 48 rows save a second job
 
-// k tiles whose weights tensor memory does not hold beside the accumulators, `cols` wide.  An MMA of 32 / 64
-// columns takes 28 / 41 clocks with A in tensor memory, 49 / 57 with A in shared memory.
-int tiles_in_smem(int cols, int stages) {
-  const int fit = (kTmemColumns - kIssuers * ((cols + 31) / 32 * 32)) / kBK;
-  return std::max(0, stages - fit);
+// Accumulators, `cols` wide: one per k tile up to kRnnAccs.  Beside them tensor memory takes what it holds of the
+// weights (an MMA of 32 / 64 columns takes 28 / 41 clocks with A in tensor memory, 49 / 57 with A in shared
+// memory), shared memory the rest; where that is too much, half as many accumulators, of chains twice as long.
+// Sums of positive products are 5.9e-7 too small in chains of 128 products, below 2.2e-7 in chains of 32.
+// (Two accumulators everywhere, and all the weights that fit in tensor memory: 61 steps of a 320-unit GRU 337
+// us, so 354; 3 layers of both directions of a 1024-unit LSTM, 500 steps, with gradients 21.6 ms, so 22.0.)
+void place_tiles(Plan* p, int cols, int recv) {
+  p->accs = kIssuers;
+  while (p->accs < std::min(p->stages, kRnnAccs)) p->accs *= 2;
+  for (;; p->accs /= 2) {
+    const int fit = (kTmemColumns - p->accs * ((cols + 31) / 32 * 32)) / kBK;
+    p->in_smem = std::max(0, p->stages - fit);
+    p->smem = seq_smem(p->in_smem, p->stages, cols, recv);
+    if (p->smem <= kMostSmem || p->accs == kIssuers) return;
+  }
 }
 
 template <int G, int NB>
@@ -934,8 +955,7 @@ Plan forward_plan(int B, int H, int G, int nb, bool wide) {
   p.slice = ((H + p.cluster - 1) / p.cluster + kBK - 1) / kBK * kBK;
   p.ctas = (H + kUnits - 1) / kUnits * p.cluster;
   p.stages = p.slice / kBK;
-  p.in_smem = tiles_in_smem(nb, p.stages);
-  p.smem = seq_smem(p.in_smem, p.stages, nb, kUnits * G * nb);
+  place_tiles(&p, nb, kUnits * G * nb);
   if (p.smem > kMostSmem) return p;
   set_rows(&p, B, nb);
   if (nb == 32)
@@ -954,8 +974,7 @@ Plan backward_plan(int B, int H, int G) {
   p.slice = sub * P;
   p.ctas = (H + out - 1) / out * KC;
   p.stages = sub / kBK;
-  p.in_smem = tiles_in_smem(P * NB, p.stages);
-  p.smem = seq_smem(p.in_smem, p.stages, P * NB, kBM * NB);
+  place_tiles(&p, P * NB, kBM * NB);
   if (p.stages > kMaxTiles || p.smem > kMostSmem) return p;
   set_rows(&p, B, NB);
   p.kernel = reinterpret_cast<const void*>(G == 1   ? rnn_sequence_backward_kernel<KC, P, 1, NB>
@@ -1070,7 +1089,7 @@ int launch(const char* name, const SeqShape& s, const Plan& p, const Job* jobs, 
     a.out_stride = s.out_stride;
     a.dy_stride = s.dy_stride;
     a.T = s.T; a.B_total = s.B; a.H = s.H; a.act = s.act;
-    a.slice = p.slice; a.stages = p.stages; a.in_smem = p.in_smem; a.ctas = p.ctas;
+    a.slice = p.slice; a.stages = p.stages; a.in_smem = p.in_smem; a.accs = p.accs; a.ctas = p.ctas;
     a.absent_cta = absent_cta;
     cudaLaunchConfig_t cfg{};
     cfg.gridDim = dim3((unsigned)(m * p.ctas));

@@ -25,6 +25,7 @@ using namespace tc;
 
 constexpr int kSliceK = 256;                // K per CTA
 constexpr int kStagesK = kSliceK / kBK;     // 8 tiles of 32 k
+static_assert(kStagesK == kRnnAccs, "one accumulator per k tile");
 constexpr int kABytes = kBM * kBK * 4;      // 16 KB per k tile
 constexpr int kBBytes = 32 * kBK * 4;       // 4 KB per k tile (32 batch rows)
 constexpr int kPartStride = 33;             // floats per partial row (bank-conflict padding)
@@ -107,8 +108,8 @@ lstm_step_kernel(const __grid_constant__ CUtensorMap map_w,
         tc_fence_after();
 #pragma unroll
         for (int j = 0; j < kBK / kUmmaK; ++j)
-          umma_tf32(tmem_base + 32 * (s % kRnnAccs), umma_desc_advance(a_desc0, s * kABytes + j * 32),
-                    umma_desc_advance(b_desc0, s * kBBytes + j * 32), idesc, s >= kRnnAccs || j ? 1u : 0u);
+          umma_tf32(tmem_base + 32 * s, umma_desc_advance(a_desc0, s * kABytes + j * 32),
+                    umma_desc_advance(b_desc0, s * kBBytes + j * 32), idesc, j ? 1u : 0u);
       }
       umma_commit(done_bar);  // arrives when every MMA issued above (possibly none) is done
     }

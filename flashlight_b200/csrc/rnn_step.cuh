@@ -9,8 +9,9 @@
 namespace flb200 {
 
 // Accumulators of a CTA's contraction per step, of every kRnnAccs-th k tile each; the epilogue adds
-// them in order (shared with rnn_sequence.cu, whose sums are the same bits).
-constexpr int kRnnAccs = 2;
+// them in order.  The tensor core does not round the sums that it carries on, so a chain is kept short:
+// in a slice of 256 states every tile of 32 has an accumulator of its own.
+constexpr int kRnnAccs = 8;
 
 // TF32 mode on sm_100, batch <= 32, hidden size a multiple of 256 up to 2048.
 bool lstm_step_supported(int math_mode, int B, int H);

@@ -185,6 +185,57 @@ torch.save([y.cpu(), hy.cpu(), cy.cpu()], sys.argv[1])
         assert torch.equal(a, b)
 
 
+@pytest.mark.parametrize("H", [256, 512, 1024])
+def test_recurrent_sums_are_not_biased(L, H):
+    """Sums of H positive products of operands that TF32 holds exactly.  The tensor core cuts off what it
+    carries from one MMA (8 products) to the next: at most 2^-23 of the sum so far, half of it on average.  In
+    chains of 32 products that is three times, at 2/4, 3/4 and all of the sum, an average of 0.75 * 0.72 (a unit
+    is 2^-23 to 2^-24 of a value): 1.0e-7 of the sum, and in chains of 128 products 3.4e-7."""
+    from flashlight_b200.extension import AutogradPayload, B200AutogradExtension
+    ext = B200AutogradExtension(math_mode=L.MATH_TF32)
+    I, B, T = 8, 8, 2
+    cut = lambda t: (t.view(torch.int32) & -8192).view(torch.float32)
+    g = torch.Generator().manual_seed(70 + H)
+    w = torch.zeros(R.rnn_num_params(I, H, 1, R.RNN_RELU, False))
+    w_hh = R.rnn_unpack(w, I, H, 1, R.RNN_RELU, False)[0][1]
+    w_hh.copy_(cut(torch.rand(H, H, generator=g) * 0.5 + 0.5))
+    h0 = cut(torch.rand(1, B, H, generator=g) * 0.5 + 0.5)
+    y, _, _ = ext.rnn(torch.zeros(T, B, I).cuda(), h0.cuda(), None, w.cuda(), H, 1, R.RNN_RELU, False, 0.0,
+                      AutogradPayload())
+    want = h0[0].double() @ w_hh.double().t()
+    bias = float(((y[0].cpu().double() - want) / want).mean())
+    assert abs(bias) < 2.2e-7, bias
+
+
+def test_persistent_equals_per_step_path_1024(L):
+    """As above for slices of 256 of 1024 states: one direction (both together take slices of 512, whose sums
+    are associated in another way)."""
+    code = r"""
+import sys, torch
+sys.path.insert(0, %r)
+from flashlight_b200 import _lib as L
+from flashlight_b200.extension import AutogradPayload, B200AutogradExtension
+from oracle import flref as R
+from tests.parity import randn
+ext = B200AutogradExtension(math_mode=L.MATH_TF32)
+I, H, B, T = 32, 1024, 19, 5
+w = randn(R.rnn_num_params(I, H, 1, R.RNN_LSTM, False), seed=50) * (0.5 / H ** 0.5)
+x = randn(T, B, I, seed=51)
+y, hy, cy = ext.rnn(x.cuda(), None, None, w.cuda(), H, 1, R.RNN_LSTM, False, 0.0, AutogradPayload())
+torch.save([y.cpu(), hy.cpu(), cy.cpu()], sys.argv[1])
+""" % str(ROOT)
+    outs = []
+    for flag in ("1", "0"):
+        path = f"/tmp/flb200_rnn_persistent_1024_{flag}.pt"
+        env = dict(os.environ, FLB200_RNN_PERSISTENT=flag)
+        res = subprocess.run([sys.executable, "-c", code, path], env=env, capture_output=True,
+                             text=True, timeout=600)
+        assert res.returncode == 0, res.stderr[-2000:]
+        outs.append(torch.load(path))
+    for a, b in zip(*outs):
+        assert torch.equal(a, b)
+
+
 def test_barrier_wait_is_bounded(L):
     """One thread block never arrives at the per-step grid barrier: the others give up after
     the budget, the kernel ends by itself, the status flag reads FLB200_TIMEOUT once and the
