@@ -123,7 +123,9 @@ __device__ __forceinline__ void ln_store(T* p, const float* f) {
 }
 
 // V consecutive parameters (null: `fill`), whole vectors where their address allows.  (One float at a time a
-// warp's load touches 32 sectors for 128 bytes: forward of 4096 rows of 768 bf16 features 10.3 us, so 7.0.)
+// warp's load touches 32 sectors for 128 bytes: forward of 65536 rows of 768 bf16 features 117 us, so 59; of
+// 4096 rows 16 and 10.)  They are read where they are used: in flight during the row's reductions they hold
+// registers that keep other rows from the SM (98 us; 256 fp32 features 43 against 37).
 template <int V>
 __device__ __forceinline__ void ln_params(const float* p, int c, bool vec, float fill, float* f) {
   if (p && vec) {
@@ -155,8 +157,6 @@ layernorm_forward_vec_kernel(const T* __restrict__ x, const float* __restrict__ 
   if (r >= rows) return;
   const T* xr = x + r * features;
   const bool wvec = ln_params_vec(weight), bvec = ln_params_vec(bias);
-  constexpr bool kEarly = PERV <= 3;  // the parameters in flight during the row's reductions
-  float w[kEarly ? PERV : 1][V], b[kEarly ? PERV : 1][V];
   float v[PERV][V];
   float s = 0.f;
 #pragma unroll
@@ -164,10 +164,6 @@ layernorm_forward_vec_kernel(const T* __restrict__ x, const float* __restrict__ 
     const int c = (j * 32 + lane) * V;
     if (c < features) {
       ln_load<T, V>(xr + c, v[j]);
-      if constexpr (kEarly) {
-        ln_params<V>(weight, c, wvec, 1.f, w[j]);
-        ln_params<V>(bias, c, bvec, 0.f, b[j]);
-      }
 #pragma unroll
       for (int k = 0; k < V; ++k) s += v[j][k];
     } else {
@@ -199,17 +195,13 @@ layernorm_forward_vec_kernel(const T* __restrict__ x, const float* __restrict__ 
   for (int j = 0; j < PERV; ++j) {
     const int c = (j * 32 + lane) * V;
     if (c >= features) continue;
-    constexpr bool kLate = !kEarly;
-    float(&wj)[V] = w[kLate ? 0 : j], (&bj)[V] = b[kLate ? 0 : j];
-    if constexpr (kLate) {
-      ln_params<V>(weight, c, wvec, 1.f, wj);
-      ln_params<V>(bias, c, bvec, 0.f, bj);
-    }
-    float h[V], o[V];
+    float h[V], o[V], w[V], b[V];
+    ln_params<V>(weight, c, wvec, 1.f, w);
+    ln_params<V>(bias, c, bvec, 0.f, b);
 #pragma unroll
     for (int k = 0; k < V; ++k) {
       h[k] = (v[j][k] - mean) * invstd;
-      o[k] = weight ? fmaf(h[k], wj[k], bj[k]) : h[k] + bj[k];
+      o[k] = weight ? fmaf(h[k], w[k], b[k]) : h[k] + b[k];
     }
     if (hr) ln_store<T, V>(hr + c, h);
     ln_store<T, V>(yr + c, o);
