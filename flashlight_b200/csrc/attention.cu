@@ -428,9 +428,10 @@ __global__ void narrow_dq_kernel(const float* __restrict__ acc, __nv_bfloat16* _
 // output in fp32 registers, rescaled by exp(m_old - m) per block.  K_{j+1} is fetched while the
 // probabilities of block j are computed, S_{j+1} runs behind O_j.  What bounds it is that chain from
 // contraction to contraction, not the tensor pipe: two CTAs share an SM and fill each other's waits.
-// 8 x 12 heads of 512 positions: 39 us; scores, softmax and context as three operators with a
-// reordering copy before and after were five launches, three T x T passes and about 90 us.  A pass of
-// 12 layers over 128 positions went from 2.1 to 1.4 ms with the 48 launches that are gone.
+// 8 x 12 heads of 512 positions: 24.5 us (39 with a mask test per element); scores, softmax and context
+// as three operators with a reordering copy before and after were five launches, three T x T passes and
+// about 90 us.  A pass of 12 layers over 128 positions went from 2.1 to 1.4 ms with the 48 launches that
+// are gone.
 constexpr int kFwdSmem = 5 * kTile + 1024 + 1024 + 256;  // Q K V P(2), row exchange, align, bars
 struct AttnFwdArgs {
   __nv_bfloat16* out;
@@ -661,8 +662,7 @@ int run_attention_backward(const void* q, const void* k, const void* v, const He
   float* dsum = reinterpret_cast<float*>(static_cast<char*>(workspace) + acc_bytes);
   launch_chained(attention_dsum_kernel, (unsigned)((rows * 8 + 255) / 256), 256, 0, st,
                  static_cast<const __nv_bfloat16*>(o), static_cast<const __nv_bfloat16*>(grad_o), dsum, rows,
-                 (int)T,
-      (int)heads);
+                 (int)T, (int)heads);
   FLB200_AFTER_LAUNCH("attention_dsum");
   AttnArgs a{};
   a.gs = gs;

@@ -401,7 +401,7 @@ static int rnn_forward_impl(const flb200_rnn_desc* d, const void* x, const void*
                                                          RL.inner_y_stride * (size_t)l);
     const long long out_stride = (long long)H * r.dirs;
     // TF32 mode, where the device can hold it: the recurrences of the layer's directions in one
-    // persistent kernel for all T steps, W_hh resident in shared memory
+    // persistent kernel for all T steps, W_hh resident on the SMs
     SeqShape shape = seq_shape(r);
     int rows = persistent_off() ? 0 : B;
     std::vector<SeqJob> jobs;

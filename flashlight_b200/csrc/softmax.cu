@@ -67,10 +67,6 @@ log_softmax_forward_kernel(const T* __restrict__ x, T* __restrict__ y, long long
   }
 }
 
-// Long fp32 rows (C a multiple of 4, 16-byte aligned): a CTA per row, 16-byte accesses, the
-// maximum and the sum of exponentials taken in ONE sweep (a running maximum, the sum rescaled
-// whenever it moves), then the sweep that writes y: two reads of the row instead of three, the
-// second one out of cache.
 // Four consecutive scores as fp32.
 __device__ __forceinline__ float4 load4(const float* p) { return *reinterpret_cast<const float4*>(p); }
 template <typename T>
@@ -79,7 +75,9 @@ __device__ __forceinline__ float4 load4(const T* p) {
   const T* h = reinterpret_cast<const T*>(&r);
   return make_float4(Num<T>::to_f(h[0]), Num<T>::to_f(h[1]), Num<T>::to_f(h[2]), Num<T>::to_f(h[3]));
 }
-// log of the sum of a row's exponentials, by a CTA
+// log of the sum of a row's exponentials (C a multiple of 4, in whole vectors), by a CTA: the maximum and the
+// sum taken in ONE sweep, a running maximum, the sum rescaled whenever it moves.  Scores of -inf weigh
+// nothing; a row of nothing else, or with a NaN or +inf, gives NaN probabilities.
 template <typename T>
 __device__ __forceinline__ float row_lse(const T* xr, long long C4, float* scratch) {
   float m = -INFINITY, s = 0.f;
@@ -109,6 +107,8 @@ __device__ __forceinline__ float row_lse(const T* xr, long long C4, float* scrat
   return row_max + logf(total);
 }
 
+// Long fp32 rows (C a multiple of 4, 16-byte aligned): a CTA per row, 16-byte accesses, row_lse, then the
+// sweep that writes y: two reads of the row instead of three, the second one out of cache.
 __global__ void __launch_bounds__(kRowThreads)
 log_softmax_forward_vec_kernel(const float* __restrict__ x, float* __restrict__ y, long long C4,
                                long long X) {
@@ -127,7 +127,7 @@ log_softmax_forward_vec_kernel(const float* __restrict__ x, float* __restrict__ 
 
 // Loss straight from the scores: of logSoftmax only the row's lse is kept, since x - lse is recomputed where
 // it is read, with the same rounding.  4096 rows of 32000 bf16 scores: the copy to fp32, logSoftmax, its
-// fused gradient and the copy back took 154 + 251 + 194 + 122 us for 2.9 GB; now two reads and a write of the
+// fused gradient and the copy back took 154 + 251 + 194 + 122 us for 3.7 GB; now two reads and a write of the
 // scores, 0.8 GB.
 template <typename T>
 __global__ void __launch_bounds__(kRowThreads)

@@ -311,7 +311,8 @@ void plan_splits(long long tiles, long long k_iters, long long min_ips, int* spl
 }
 
 // The launch lasts `rounds` tiles per CTA (or CTA pair), so the plan weighs the clocks of a tile
-// against how evenly the tiles fill the 148 SMs.  Clocks of one stage (128 bytes of K), measured:
+// against how evenly the tiles fill the 148 SMs.  Clocks of one stage (128 bytes of K), measured
+// before a lane of the producers and issuers did nothing but add, and kept since (their order decides):
 // a tile sits at the shared-memory port, 2 x (16 KB + BN x 128 B) per stage at 128 B/clock, and
 // above ~420 of barrier hand-over; a pair halves the B half of that and runs at the tensor
 // pipe's own 512.  A small product wants narrow tiles and a split of K for the sake of the
@@ -333,14 +334,15 @@ static Launch compute_launch(long long M, long long N, long long k_iters, long l
     if (operand != kOperandTf32 && b_mn_major && w.bn < box) continue;  // one box at least
     if (w.pairs) {
       if (x3 || M <= kBM) continue;
-      // TF32 pairs, measured: both operands MN-major (12 copies a stage) win nothing, and a
-      // short K loop loses more to the cross-CTA hand-offs than it gains
+      // TF32 pairs, measured: both operands MN-major win 4 % on the largest products and lose on others, and
+      // a short K loop loses more to the cross-CTA hand-offs than it gains
       if (operand == kOperandTf32 && (b_mn_major || k_iters < (a_mn_major ? 8 : 4))) continue;
       if (k_iters < 4) continue;
     }
     double clocks = w.clocks * (x3 ? 2.5 : 1.0);
-    // issuing a TMA copy takes a producer warp ~120 clocks, and there are two of them (the boxes of a
-    // grouped MN-major operand are one copy; counting them so changed no choice by more than noise)
+    // issuing a TMA copy took a producer warp ~120 clocks, and there are two of them.  (The boxes of a grouped
+    // MN-major operand are one copy now, which counts as its boxes here still: counting it so changed no time
+    // by more than noise.)
     const int copies = (a_mn_major ? kBM / box : 1) +
                        (b_mn_major ? (w.pairs ? w.bn / 2 : w.bn) / box : 1);
     if (clocks < copies * 65.0) clocks = copies * 65.0;
