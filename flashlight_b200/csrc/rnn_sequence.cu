@@ -148,14 +148,18 @@ struct Feed {
 // The tag stays in the operand: the tensor core does not read those bits.  meanwhile() runs while the
 // second tile, or the MMAs of the first, are in flight (before the first and after the second it costs 0.1
 // to 0.8 us a step).
-// kWhole: tiles whose words past the batch's rows and past K are zeros from the start; of up to four rows they are
+// kWhole: tiles whose words past the batch's rows and past K are zeros from the start; of up to eight rows they are
 // stored by the lanes that polled them, without the copy and the second look at every word.  (One row of 1024
-// units, 40 steps forward: 172 us by copies, 134 so; the backward pass, whose tiles start undefined, copies.)
+// units, 40 steps forward: 172 us by copies, 136 so; eight rows of a 320-unit GRU 114; nine rows are copied, 138.
+// The backward pass, whose tiles start undefined, copies.)
 template <bool kWhole, int P, int NB, typename Meanwhile>
 __device__ __forceinline__ void bring_tiles(Feed& f, int slot, uint32_t tag, int warp, int lane,
                                             const Waits& w, int code, Meanwhile&& meanwhile) {
   constexpr int kTiles = kMaxTiles / kWorkers, kStep = kWorkers * kBK, kBytes = P * NB * 128;
-  const int q = 4 * (lane & 7), row = (lane >> 3) * ((f.B + 3) / 4);
+  // kWhole, up to eight rows: the samples are all there is, and they are stored from where they are
+  constexpr int kLoads = kTiles * P, kSets = kWhole ? 2 : 1;
+  const bool direct = kWhole && f.B <= 4 * kSets;
+  const int q = 4 * (lane & 7), row = (lane >> 3) * (direct ? 1 : (f.B + 3) / 4);
   const uint32_t* from = f.x + ((long long)slot * f.B + row) * f.K + f.k0 + q;
   auto copy = [&](int i) {
     const int s = warp + i * kWorkers;
@@ -171,37 +175,41 @@ __device__ __forceinline__ void bring_tiles(Feed& f, int slot, uint32_t tag, int
     __syncwarp();
   };
   uint32_t pending = 0, to_copy = 0;
-  uint4 v[kTiles * P];
+  uint4 v[kSets * kLoads];  // the second set: four rows further down
 #pragma unroll
   for (int i = 0; i < kTiles; ++i) {
     if (warp + i * kWorkers < f.stages) to_copy |= 1u << i;
 #pragma unroll
     for (int p = 0; p < P; ++p)
-      if (warp + i * kWorkers < f.stages && row < f.B && f.k0 + q + i * kStep + p * f.sub < f.K)
-        pending |= 1u << (i * P + p);
+#pragma unroll
+      for (int h = 0; h < kSets; ++h)
+        if (warp + i * kWorkers < f.stages && row + 4 * h < f.B && (h == 0 || direct) &&
+            f.k0 + q + i * kStep + p * f.sub < f.K)
+          pending |= 1u << (h * kLoads + i * P + p);
   }
   const uint32_t mine = to_copy, chunks = pending;
-  // kWhole, up to four rows: the samples are all there is, and they are stored from where they are
-  const bool direct = kWhole && f.B <= 4;
   int spins = 0;
   long long t0 = clock64();
   while (to_copy && w.warp_goes_on()) {
 #pragma unroll
-    for (int u = 0; u < kTiles * P; ++u)
-      if (pending >> u & 1) v[u] = ld_relaxed_v4(from + (u / P) * kStep + (u % P) * f.sub);
+    for (int u = 0; u < kSets * kLoads; ++u)
+      if (pending >> u & 1)
+        v[u] = ld_relaxed_v4(from + (u / kLoads) * 4 * f.K + (u % kLoads / P) * kStep + (u % P) * f.sub);
 #pragma unroll
-    for (int u = 0; u < kTiles * P; ++u)
+    for (int u = 0; u < kSets * kLoads; ++u)
       if ((pending >> u & 1) && is_tagged(v[u], tag)) pending &= ~(1u << u);
 #pragma unroll
     for (int i = 0; i < kTiles; ++i)
-      if ((to_copy >> i & 1) && !__any_sync(0xffffffffu, pending >> (i * P) & ((1u << P) - 1))) {
+      if ((to_copy >> i & 1) && !__any_sync(0xffffffffu, (pending | pending >> kLoads) >> (i * P) & ((1u << P) - 1))) {
         if (direct) {
           const int s = warp + i * kWorkers;
 #pragma unroll
-          for (int p = 0; p < P; ++p)
-            if (chunks >> (i * P + p) & 1)
-              *reinterpret_cast<uint4*>(f.b_tiles + s * kBytes + p * (NB * 128) + row * 128 +
-                                        (((lane & 7) ^ (row & 7)) << 4)) = v[i * P + p];
+          for (int u = 0; u < kSets * P; ++u) {
+            const int h = u / P, p = u % P, b = row + 4 * h;
+            if (chunks >> (h * kLoads + i * P + p) & 1)
+              *reinterpret_cast<uint4*>(f.b_tiles + s * kBytes + p * (NB * 128) + b * 128 +
+                                        (((lane & 7) ^ (b & 7)) << 4)) = v[h * kLoads + i * P + p];
+          }
           fence_proxy_async();  // every lane's stores, before the MMAs read
           __syncwarp();
           if (lane == 0) mbar_arrive(&f.full_bar[s]);
@@ -953,7 +961,7 @@ bool wants_48(int B) { return B > 32 && B <= 48; }  // where 48 rows save a seco
 // memory), shared memory the rest; where that is too much, half as many accumulators, of chains twice as long.
 // Sums of positive products are 5.9e-7 too small in chains of 128 products, below 2.2e-7 in chains of 32.
 // (Two accumulators everywhere, and all the weights that fit in tensor memory: 61 steps of a 320-unit GRU 337
-// us, so 354; 3 layers of both directions of a 1024-unit LSTM, 500 steps, with gradients 21.6 ms, so 22.0.)
+// us, so 354, with tiles of few rows stored by those who poll 301; 3 layers of both directions of a 1024-unit LSTM, 500 steps, with gradients 21.6 ms, so 22.0.)
 void place_tiles(Plan* p, int cols, int recv) {
   p->accs = kIssuers;
   while (p->accs < std::min(p->stages, kRnnAccs)) p->accs *= 2;

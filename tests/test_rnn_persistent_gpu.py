@@ -210,19 +210,19 @@ def test_recurrent_sums_are_not_biased(L, H):
 @pytest.mark.parametrize("cell,H", [(R.RNN_LSTM, 1024), (R.RNN_GRU, 700), (R.RNN_TANH, 36), (R.RNN_LSTM, 320)])
 @pytest.mark.parametrize("bidir", [False, True])
 def test_few_rows_equal_rows_of_a_batch(L, cell, H, bidir):
-    """Tiles of up to four rows of the batch reach the tensor core another way than those of more: the same
+    """Tiles of up to eight rows of the batch reach the tensor core another way than those of more: the same
     bits.  (Of inputs that are zeros: the projection of a few other inputs has routes of its own, with other
     roundings.)"""
     from flashlight_b200.extension import AutogradPayload, B200AutogradExtension
     ext = B200AutogradExtension(math_mode=L.MATH_TF32)
     I, T = 8, 11
     w = (randn(R.rnn_num_params(I, H, 1, cell, bidir), seed=60) * (0.5 / H ** 0.5)).cuda()
-    hx = randn(2 if bidir else 1, 5, H, seed=61).cuda()
+    hx = randn(2 if bidir else 1, 9, H, seed=61).cuda()
     run = lambda h: ext.rnn(torch.zeros(T, h.shape[1], I, device="cuda"), h.contiguous(),
                             h.contiguous() if cell == R.RNN_LSTM else None, w, H, 1, cell, bidir, 0.0,
                             AutogradPayload())[0]
     want = run(hx)
-    for B in (1, 3, 4):
+    for B in (1, 3, 4, 5, 8):
         assert torch.equal(run(hx[:, :B]), want[:, :B]), f"batch {B}"
     assert L.lib.flb200_tc_poll_status(torch.cuda.current_stream().cuda_stream) == L.OK
 
